@@ -107,6 +107,12 @@ bool uses_tile_kernels(const Args* a) {
   return a->backend == MF_BACKEND_AUTO && simplicial_sm100_packs_heads(a->tokens, a->heads);
 }
 
+// Molecules of at most 32 tokens run on the warp-level kernels, with and without the factorized bias.
+template <typename Args>
+bool uses_small_kernels(const Args* a) {
+  return (a->backend == MF_BACKEND_AUTO || a->backend == MF_BACKEND_TCGEN05_TILES) && a->tokens <= kSmallTokens;
+}
+
 }  // namespace
 }  // namespace mf
 
@@ -129,7 +135,7 @@ extern "C" int mf_feature_flags(void) { return tensor_maps_available() ? MF_FEAT
 extern "C" size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* a) {
   if (!a) return 0;
   int rc;
-  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd")) return simplicial_sm100_fwd_workspace_bytes(*a);
+  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd") && !uses_small_kernels(a)) return simplicial_sm100_fwd_workspace_bytes(*a);
   return 0;
 }
 
@@ -137,7 +143,7 @@ extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a
   if (!a) return 0;
   int rc;
   if (wants_tcgen05(a, &rc, "mf_simplicial_bwd"))
-    return uses_tile_kernels(a) ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
+    return uses_small_kernels(a) ? 0 : uses_tile_kernels(a) ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
   return simplicial_generic_bwd_workspace_bytes(*a);
 }
 
@@ -179,6 +185,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
   if (!tc) return simplicial_generic_fwd(*a, s);
+  if (uses_small_kernels(a)) return simplicial_small_fwd(*a, nullptr, s);
   return uses_tile_kernels(a) ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
 }
 
@@ -200,6 +207,7 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
   if (!tc) return simplicial_generic_bwd(*a, s);
+  if (uses_small_kernels(a)) return simplicial_small_bwd(*a, nullptr, s);
   return uses_tile_kernels(a) ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
 }
 

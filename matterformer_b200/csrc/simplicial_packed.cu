@@ -6,7 +6,7 @@
 // points take the GEMM's output as it is -- rows of q, k1, v1, k2, v2 are slices of the packed tensor, addressed
 // with strides -- apply the query scale on load, write the attention output as (B,N,H*D) and the five gradients
 // straight into one (B,N,5,H,D) tensor, so neither pass over the activations exists any more.  They run the
-// packed-heads tile kernels (simplicial_sm100.cu, simplicial_sm100_bwd.cu) and therefore serve molecules of at most
+// warp-level kernels (simplicial_small_fwd.cu, simplicial_small_bwd.cu) and therefore serve molecules of at most
 // 32 tokens with a multiple of four heads of 64 channels in bf16: the trunk's shape.
 #include "common.cuh"
 #include "simplicial.cuh"
@@ -84,40 +84,22 @@ MfSimplicialBwdArgs as_bwd(const MfSimplicialPackedArgs* a) {
 
 using namespace mf;
 
-extern "C" size_t mf_simplicial_packed_fwd_workspace_bytes(const MfSimplicialPackedArgs* a) {
-  if (!a || a->batch <= 0) return 0;
-  const MfSimplicialFwdArgs f = as_fwd(a);
-  return simplicial_sm100_fwd_workspace_bytes(f);
-}
-
-extern "C" size_t mf_simplicial_packed_bwd_workspace_bytes(const MfSimplicialPackedArgs* a) {
-  if (!a || a->batch <= 0) return 0;
-  const MfSimplicialBwdArgs r = as_bwd(a);
-  return simplicial_sm100_bwd_workspace_bytes(r);
-}
+// The kernels these calls run on need no workspace; the functions stay for callers that ask.
+extern "C" size_t mf_simplicial_packed_fwd_workspace_bytes(const MfSimplicialPackedArgs*) { return 0; }
+extern "C" size_t mf_simplicial_packed_bwd_workspace_bytes(const MfSimplicialPackedArgs*) { return 0; }
 
 extern "C" int mf_simplicial_packed_fwd(const MfSimplicialPackedArgs* a, void* stream) {
   int rc = check_packed(a, "mf_simplicial_packed_fwd", false);
   if (rc != MF_OK || a->batch == 0 || a->heads == 0 || a->tokens == 0) return rc;
   const MfSimplicialFwdArgs f = as_fwd(a);
-  const size_t need = simplicial_sm100_fwd_workspace_bytes(f);
-  if (!a->workspace || a->workspace_bytes < need) {
-    set_error("mf_simplicial_packed_fwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
-    return MF_ERR_WORKSPACE_TOO_SMALL;
-  }
   const TileLayouts l = packed_layouts(a);
-  return simplicial_sm100_fwd_layouts(f, &l, static_cast<cudaStream_t>(stream));
+  return simplicial_small_fwd(f, &l, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mf_simplicial_packed_bwd(const MfSimplicialPackedArgs* a, void* stream) {
   int rc = check_packed(a, "mf_simplicial_packed_bwd", true);
   if (rc != MF_OK || a->batch == 0 || a->heads == 0 || a->tokens == 0) return rc;
   const MfSimplicialBwdArgs r = as_bwd(a);
-  const size_t need = simplicial_sm100_bwd_workspace_bytes(r);
-  if (!a->workspace || a->workspace_bytes < need) {
-    set_error("mf_simplicial_packed_bwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
-    return MF_ERR_WORKSPACE_TOO_SMALL;
-  }
   const TileLayouts l = packed_layouts(a);
-  return simplicial_sm100_bwd_layouts(r, &l, static_cast<cudaStream_t>(stream));
+  return simplicial_small_bwd(r, &l, static_cast<cudaStream_t>(stream));
 }

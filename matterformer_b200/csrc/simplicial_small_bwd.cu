@@ -1,0 +1,558 @@
+// 2-simplicial attention, backward, for molecules of at most 32 tokens in bf16 (see simplicial_warp.cuh).
+//
+// For one query i every gradient is a product of 32 x 32 matrices that a warp holds in registers: S_i = (K1 o q_i) K2^T and
+// P_i as in the forward pass, dP_i = (V1 o dO_i) V2^T, dS_i = P_i o (dP_i - delta_i), and with U_i = dS_i K2, W_i = P_i V2
+//
+//   dq_i = sum_j k1_j o U_i[j]     dk1_j += q_i o U_i[j]      dk2 += dS_i^T (K1 o q_i)
+//                                  dv1_j += dO_i o W_i[j]     dv2 += P_i^T (V1 o dO_i)
+//
+// Four accumulators of 32 x 64 do not fit one warp, so the queries are walked twice: the V side (P: dv1, dv2), then the K side
+// (dS: dq, dk1, dk2 and the bias gradients), which forms S_i and P_i again; 64 + 64 accumulator registers each, no barrier
+// and no shared-memory exchange during a walk.  The warps of a CTA share one (batch, head), split its queries and are added
+// up in a fixed order.  The products over the keys k take P and dS as the logit product left them (U^T = K2^T dS^T has dS
+// as its B operand), those over j an 8x8 transposition in registers.  delta_i = dO_i . out_i is formed on load.
+// Every output has one writer: no atomics, no workspace, nothing to zero beforehand.
+//
+// What bounds it: latency at two warps per scheduler (255 registers; the mma.sync pipe is 38 % busy, shared memory 50 %).
+// Measured at 1024 molecules of 9-29 atoms x 8 heads: 547 us, against 980 + 39 us for the tcgen05 tile kernel and its delta
+// pass; with the two sides on two warps of a pair 613 us (the V side waits for the K side, and two code paths share the
+// instruction cache).
+#include "common.cuh"
+#include "simplicial.cuh"
+#include "simplicial_warp.cuh"
+
+namespace mf {
+namespace {
+
+struct SmallBwdParams {
+  const __nv_bfloat16* grad_out;
+  const __nv_bfloat16* q;
+  const __nv_bfloat16* k1;
+  const __nv_bfloat16* v1;
+  const __nv_bfloat16* k2;
+  const __nv_bfloat16* v2;
+  const float* out;
+  const float* lse;
+  const uint8_t* query_valid;
+  const uint8_t* key_valid;
+  const uint8_t* pair_valid;
+  const float* u;
+  const float* v_bias;
+  const float* w;
+  const float* gate;
+  float* du;
+  float* dv_bias;
+  float* dw;
+  float* dgate;
+  __nv_bfloat16* dq;
+  __nv_bfloat16* dk1;
+  __nv_bfloat16* dv1;
+  __nv_bfloat16* dk2;
+  __nv_bfloat16* dv2;
+  int H, N;
+  float q_scale;
+  RowLayout in, act;
+};
+
+constexpr int kAccStride = kD + 4;  // fp32 rows of the gradient stage
+
+template <bool kBias>
+struct SmallBwdShared {
+  __align__(128) uint8_t tile[6][kSmallTile];  // q, k1, v1, k2, v2, grad_out
+  __nv_bfloat16 dq[kSmallRows][kD];
+  union {
+    float acc[2][kSmallRows][kAccStride];      // sums of the side just walked: first-key and second-key gradient
+    float4 dw[4][8][32];                       // K side walk: the warps' dw_jk as the fragments of the logits hold it
+  };
+  float lse2[kSmallRows], delta[kSmallRows];
+  uint32_t visible[kSmallRows];                // bit k of word j: the pair (j, k) counts
+  float4 w[kBias ? 8 : 1][32];                 // bias w_jk as the fragments of the logits hold it
+};
+
+constexpr int kTq = 0, kTk1 = kSmallTile, kTv1 = 2 * kSmallTile, kTk2 = 3 * kSmallTile, kTv2 = 4 * kSmallTile, kTgo = 5 * kSmallTile;
+
+// c (16 x 8 tiles, rows j, columns k) = (X o x_i) Y^T for two key-major tiles X, Y and the row x_i
+template <int MT, int NT>
+__device__ __forceinline__ void pair_product(float (&c)[MT][NT][4], const FragBase& fb, int x, int y, const uint32_t (&row)[8]) {
+#pragma unroll
+  for (int kp = 0; kp < 2; ++kp) {
+    uint32_t b[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) load_b(b[nt], fb, y, nt, kp);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int ks = 2 * kp + k;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        uint32_t a[4];
+        load_a(a, fb, x, mt, ks);
+        a[0] = mul_bf16x2(a[0], row[2 * ks]);
+        a[1] = mul_bf16x2(a[1], row[2 * ks]);
+        a[2] = mul_bf16x2(a[2], row[2 * ks + 1]);
+        a[3] = mul_bf16x2(a[3], row[2 * ks + 1]);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          if (ks == 0) mma16_first(c[mt][nt], a, b[nt][2 * k], b[nt][2 * k + 1]);
+          else mma16(c[mt][nt], a, b[nt][2 * k], b[nt][2 * k + 1]);
+        }
+      }
+    }
+  }
+}
+
+// One walk; warp w takes the queries w, w + kWarps, ....  Leaves the two sums in sm.acc and all warps at a barrier.
+template <int MT, int NT, bool kHoles, bool kBias, int kWarps, bool kKeySide>
+__device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwdShared<kBias>& sm, int bh, int n,
+                                               uint32_t qmask) {
+  constexpr int KS = (NT + 1) / 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
+  const uint32_t qt = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
+  const FragBase fb(qt, lane);
+  constexpr int x1 = kKeySide ? kTk1 : kTv1, x2 = kKeySide ? kTk2 : kTv2, xr = kKeySide ? kTq : kTgo;
+  uint32_t vis[MT][2];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh)
+      vis[mt][hh] = kHoles ? sm.visible[mt * 16 + hh * 8 + row8] >> (2 * quad) : (mt * 16 + hh * 8 + row8 < n ? ~0u : 0u);
+
+  float a1[4][2 * MT][4], a2[KS][8][4];  // first-key gradient [channels][j], second-key gradient [k][channels]
+#pragma unroll
+  for (int dt = 0; dt < 4; ++dt)
+#pragma unroll
+    for (int jt = 0; jt < 2 * MT; ++jt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a1[dt][jt][e] = 0.f;
+#pragma unroll
+  for (int kt = 0; kt < KS; ++kt)
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a2[kt][t][e] = 0.f;
+  if constexpr (kBias && kKeySide) {
+#pragma unroll
+    for (int f = 0; f < 8; ++f) sm.dw[warp][f][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+
+  const int nq = 32 - __clz(qmask);
+  for (int i = warp; i < nq; i += kWarps) {
+    if (!((qmask >> i) & 1u)) continue;
+    float s[MT][NT][4];
+    {
+      uint32_t qf[8];
+      load_row_pairs(qf, qt, i, lane);
+      pair_product<MT, NT>(s, fb, kTk1, kTk2, qf);
+    }
+    float ul = 0.f, vl = 0.f, g = 0.f;  // bias: u_i,lane, v_i,lane
+    if constexpr (kBias) {
+      const size_t at = ((size_t)bh * p.N + i) * p.N + lane;
+      ul = lane < n ? p.u[at] : 0.f;
+      vl = lane < n ? p.v_bias[at] : 0.f;
+      g = p.gate[(size_t)bh * p.N + i];
+      float ur[MT][2];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) ur[mt][hh] = __shfl_sync(0xffffffffu, ul, mt * 16 + hh * 8 + row8);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const float va = __shfl_sync(0xffffffffu, vl, nt * 8 + 2 * quad), vb = __shfl_sync(0xffffffffu, vl, nt * 8 + 2 * quad + 1);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const float4 w = sm.w[mt * 4 + nt][lane];
+          s[mt][nt][0] = fmaf(g, (ur[mt][0] + va) + w.x, s[mt][nt][0]);
+          s[mt][nt][1] = fmaf(g, (ur[mt][0] + vb) + w.y, s[mt][nt][1]);
+          s[mt][nt][2] = fmaf(g, (ur[mt][1] + va) + w.z, s[mt][nt][2]);
+          s[mt][nt][3] = fmaf(g, (ur[mt][1] + vb) + w.w, s[mt][nt][3]);
+        }
+      }
+    }
+    const float lse2 = sm.lse2[i];
+    const float2 le = make_float2(kLog2e, kLog2e);
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const float c = vis[mt][hh] ? -lse2 : -INFINITY;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          float2 x = fma2(make_float2(s[mt][nt][2 * hh], s[mt][nt][2 * hh + 1]), le, make_float2(c, c));
+          x.x = fast_exp2(x.x);
+          x.y = fast_exp2(x.y);
+          if (kHoles) {
+            if (!((vis[mt][hh] >> (nt * 8)) & 1u)) x.x = 0.f;
+            if (!((vis[mt][hh] >> (nt * 8 + 1)) & 1u)) x.y = 0.f;
+          } else if (nt == NT - 1 || MT == 1) {  // MT == 1 serves 1 to 16 keys
+            if (nt * 8 + 2 * quad >= n) x.x = 0.f;
+            if (nt * 8 + 2 * quad + 1 >= n) x.y = 0.f;
+          }
+          s[mt][nt][2 * hh] = x.x, s[mt][nt][2 * hh + 1] = x.y;
+        }
+      }
+    if constexpr (kKeySide) {
+      float dp[MT][NT][4];
+      {
+        uint32_t gf[8];
+        load_row_pairs(gf, qt + kTgo, i, lane);
+        pair_product<MT, NT>(dp, fb, kTv1, kTv2, gf);
+      }
+      const float nd = -sm.delta[i];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const float2 d = add2(make_float2(dp[mt][nt][2 * hh], dp[mt][nt][2 * hh + 1]), make_float2(nd, nd));
+            const float2 x = mul2(make_float2(s[mt][nt][2 * hh], s[mt][nt][2 * hh + 1]), d);
+            s[mt][nt][2 * hh] = x.x, s[mt][nt][2 * hh + 1] = x.y;
+          }
+      if constexpr (kBias) {
+        float rs[MT][2], cs[8], wsum = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) cs[e] = 0.f;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          rs[mt][0] = rs[mt][1] = 0.f;
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            const float(&x)[4] = s[mt][nt];
+            rs[mt][0] += x[0] + x[1];
+            rs[mt][1] += x[2] + x[3];
+            cs[2 * nt] += x[0] + x[2];
+            cs[2 * nt + 1] += x[1] + x[3];
+            const float4 w = sm.w[mt * 4 + nt][lane];
+            wsum = fmaf(x[0], w.x, fmaf(x[1], w.y, fmaf(x[2], w.z, fmaf(x[3], w.w, wsum))));
+            float4& dw = sm.dw[warp][mt * 4 + nt][lane];
+            float4 t = dw;
+            t.x = fmaf(g, x[0], t.x), t.y = fmaf(g, x[1], t.y), t.z = fmaf(g, x[2], t.z), t.w = fmaf(g, x[3], t.w);
+            dw = t;
+          }
+        }
+        // row sums over the quad, column sums over the eight row groups; lane l ends up with row l and with column l
+        float r4[4] = {rs[0][0], rs[0][1], MT > 1 ? rs[MT - 1][0] : 0.f, MT > 1 ? rs[MT - 1][1] : 0.f};
+        const bool q0 = quad & 1, q1 = quad >> 1;
+        float ra = (q0 ? r4[2] : r4[0]) + __shfl_xor_sync(0xffffffffu, q0 ? r4[0] : r4[2], 1);
+        float rb = (q0 ? r4[3] : r4[1]) + __shfl_xor_sync(0xffffffffu, q0 ? r4[1] : r4[3], 1);
+        float rsum = (q1 ? rb : ra) + __shfl_xor_sync(0xffffffffu, q1 ? ra : rb, 2);  // row 16 q0 + 8 q1 + row8
+        const bool c0 = row8 & 1, c1 = (row8 >> 1) & 1, c2 = row8 >> 2;
+        float t4[4], t2[2];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) t4[e] = (c0 ? cs[4 + e] : cs[e]) + __shfl_xor_sync(0xffffffffu, c0 ? cs[e] : cs[4 + e], 4);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) t2[e] = (c1 ? t4[2 + e] : t4[e]) + __shfl_xor_sync(0xffffffffu, c1 ? t4[e] : t4[2 + e], 8);
+        float csum = (c2 ? t2[1] : t2[0]) + __shfl_xor_sync(0xffffffffu, c2 ? t2[0] : t2[1], 16);
+        const int rrow = 16 * (int)q0 + 8 * (int)q1 + row8;                             // row of rsum
+        const int ccol = 8 * (2 * (int)c0 + (int)c1) + 2 * quad + (int)c2;              // column of csum
+        const size_t at = ((size_t)bh * p.N + i) * p.N;
+        if (p.du && rrow < p.N) p.du[at + rrow] = g * rsum;
+        if (p.dv_bias && ccol < p.N) p.dv_bias[at + ccol] = g * csum;
+        if (p.dgate) {
+          // sum dS (u + v + w), the common offset of u and v taken out first
+          const float off = __shfl_sync(0xffffffffu, ul, 0);
+          const float uo = __shfl_sync(0xffffffffu, ul, rrow) - off, vo = __shfl_sync(0xffffffffu, vl, ccol) + off;
+          const float tot = warp_sum((rrow < n ? uo * rsum : 0.f) + (ccol < n ? vo * csum : 0.f) + wsum);
+          if (lane == 0) p.dgate[(size_t)bh * p.N + i] = tot;
+        }
+      }
+    }
+    // P or dS in bf16: pk[mt][nt][hh] = two keys k of one row j; at = its transpose, the A operand over j
+    uint32_t pk[MT][2 * KS][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 2 * KS; ++nt)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) pk[mt][nt][hh] = nt < NT ? pack2_bf16(s[mt][nt < NT ? nt : 0][2 * hh], s[mt][nt < NT ? nt : 0][2 * hh + 1]) : 0u;
+    uint32_t at[KS][MT][4];
+#pragma unroll
+    for (int kt = 0; kt < KS; ++kt)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        at[kt][mt][0] = transpose8x8(pk[mt][2 * kt][0]);
+        at[kt][mt][1] = 2 * kt + 1 < NT ? transpose8x8(pk[mt][2 * kt + 1][0]) : 0u;
+        at[kt][mt][2] = transpose8x8(pk[mt][2 * kt][1]);
+        at[kt][mt][3] = 2 * kt + 1 < NT ? transpose8x8(pk[mt][2 * kt + 1][1]) : 0u;
+      }
+    uint32_t xd[8];
+    load_row_dup(xd, qt + xr, i, lane);
+    float dq[8];
+#pragma unroll
+    for (int dt = 0; dt < 4; ++dt) {
+      float c[2 * MT][4];
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        uint32_t a[4];
+        load_t(a, fb, x2, dt, ks);
+#pragma unroll
+        for (int jt = 0; jt < 2 * MT; ++jt) {
+          const uint32_t b0 = pk[jt >> 1][2 * ks][jt & 1], b1 = pk[jt >> 1][2 * ks + 1][jt & 1];
+          if (ks == 0) mma16_first(c[jt], a, b0, b1);
+          else mma16(c[jt], a, b0, b1);
+        }
+      }
+      const float xa = bf16_hi(xd[2 * dt]), xb = bf16_hi(xd[2 * dt + 1]);
+      float2 lo = make_float2(0.f, 0.f), hi = lo;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        uint32_t kf[4];
+        load_t(kf, fb, x1, dt, mt);
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const int jt = 2 * mt + jj;
+          const float2 ca = make_float2(c[jt][0], c[jt][1]), cb = make_float2(c[jt][2], c[jt][3]);
+          float(&acc)[4] = a1[dt][jt];
+          const float2 na = fma2(ca, make_float2(xa, xa), make_float2(acc[0], acc[1]));
+          const float2 nb = fma2(cb, make_float2(xb, xb), make_float2(acc[2], acc[3]));
+          acc[0] = na.x, acc[1] = na.y, acc[2] = nb.x, acc[3] = nb.y;
+          if constexpr (kKeySide) {
+            lo = fma2(ca, make_float2(bf16_lo(kf[2 * jj]), bf16_hi(kf[2 * jj])), lo);
+            hi = fma2(cb, make_float2(bf16_lo(kf[2 * jj + 1]), bf16_hi(kf[2 * jj + 1])), hi);
+          }
+        }
+        const uint32_t b0 = mul_bf16x2(kf[0], xd[2 * dt]), b1 = mul_bf16x2(kf[2], xd[2 * dt]);
+        const uint32_t b2 = mul_bf16x2(kf[1], xd[2 * dt + 1]), b3 = mul_bf16x2(kf[3], xd[2 * dt + 1]);
+#pragma unroll
+        for (int kt = 0; kt < KS; ++kt) {
+          mma16(a2[kt][2 * dt], at[kt][mt], b0, b1);
+          mma16(a2[kt][2 * dt + 1], at[kt][mt], b2, b3);
+        }
+      }
+      if constexpr (kKeySide) dq[2 * dt] = lo.x + lo.y, dq[2 * dt + 1] = hi.x + hi.y;
+    }
+    if constexpr (kKeySide) {
+      quad_sum8(dq, lane);
+      const int d0 = (4 * (quad & 1) + 2 * (quad >> 1)) * 8 + row8;
+      sm.dq[i][d0] = __float2bfloat16_rn(dq[0] * p.q_scale);
+      sm.dq[i][d0 + 8] = __float2bfloat16_rn(dq[1] * p.q_scale);
+    }
+  }
+
+  if constexpr (kBias && kKeySide) {
+    __syncthreads();
+    if (p.dw) {
+      float* dw = p.dw + (size_t)bh * p.N * p.N;
+      for (int idx = threadIdx.x; idx < p.N * p.N; idx += 32 * kWarps) {
+        const int j = idx / p.N, k = idx - j * p.N;
+        float v = 0.f;
+        if (j < n && k < n) {
+          const int f = (j >> 4) * 4 + (k >> 3), ln = 4 * (j & 7) + ((k & 7) >> 1), e = 2 * ((j >> 3) & 1) + (k & 1);
+#pragma unroll
+          for (int q = 0; q < kWarps; ++q) v += reinterpret_cast<const float*>(&sm.dw[q][f][ln])[e];
+        }
+        dw[idx] = v;
+      }
+    }
+  }
+#pragma unroll 1
+  for (int q = 0; q < kWarps; ++q) {
+    __syncthreads();
+    if (q != warp) continue;
+#pragma unroll
+    for (int dt = 0; dt < 4; ++dt)
+#pragma unroll
+      for (int jt = 0; jt < 2 * MT; ++jt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float& o = sm.acc[0][jt * 8 + 2 * quad + (e & 1)][dt * 16 + (e >> 1) * 8 + row8];
+          o = (q ? o : 0.f) + a1[dt][jt][e];
+        }
+#pragma unroll
+    for (int kt = 0; kt < KS; ++kt)
+#pragma unroll
+      for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          float2& o = *reinterpret_cast<float2*>(&sm.acc[1][kt * 16 + hh * 8 + row8][8 * t + 2 * quad]);
+          const float2 old = q ? o : make_float2(0.f, 0.f);
+          o = make_float2(old.x + a2[kt][t][2 * hh], old.y + a2[kt][t][2 * hh + 1]);
+        }
+  }
+  __syncthreads();
+}
+
+// Both walks and the gradient rows; a lane writes eight channels.
+template <int MT, int NT, bool kHoles, bool kBias, int kWarps>
+__device__ __forceinline__ void small_bwd_walks(const SmallBwdParams& p, SmallBwdShared<kBias>& sm, int b, int h, int n,
+                                                uint32_t kmask, uint32_t qmask) {
+  const int bh = b * p.H + h;
+  auto store_rows = [&](__nv_bfloat16* g1, __nv_bfloat16* g2) {
+    for (int idx = threadIdx.x; idx < 16 * p.N; idx += 32 * kWarps) {
+      const int t = idx & 1, r = idx >> 4, c = (idx >> 1) & 7;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (r < n && ((kmask >> r) & 1u)) {
+        const float4 x = *reinterpret_cast<const float4*>(&sm.acc[t][r][8 * c]), y = *reinterpret_cast<const float4*>(&sm.acc[t][r][8 * c + 4]);
+        v.x = pack2_bf16(x.x, x.y), v.y = pack2_bf16(x.z, x.w), v.z = pack2_bf16(y.x, y.y), v.w = pack2_bf16(y.z, y.w);
+      }
+      *reinterpret_cast<uint4*>((t ? g2 : g1) + p.in.at(b, h, r) + 8 * c) = v;
+    }
+  };
+  small_bwd_side<MT, NT, kHoles, kBias, kWarps, false>(p, sm, bh, n, qmask);
+  store_rows(p.dv1, p.dv2);
+  __syncthreads();
+  small_bwd_side<MT, NT, kHoles, kBias, kWarps, true>(p, sm, bh, n, qmask);
+  store_rows(p.dk1, p.dk2);
+}
+
+template <bool kBias, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_kernel(const __grid_constant__ SmallBwdParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  SmallBwdShared<kBias>& sm = *reinterpret_cast<SmallBwdShared<kBias>*>(smem);
+  constexpr int kThreads = 32 * kWarps;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int N = p.N, bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
+  const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
+  const uint32_t qmask = __ballot_sync(0xffffffffu, lane < N && p.query_valid[(size_t)b * N + min(lane, N - 1)] > 0);
+  const int n = qmask ? 32 - __clz(kmask) : 0, nq = n ? 32 - __clz(qmask) : 0;
+  if (n > 0) {
+    const __nv_bfloat16* src[6] = {p.q, p.k1, p.v1, p.k2, p.v2, p.grad_out};
+    const uint32_t t0 = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
+    // a hole in a mask takes the full-size variant, which reads all rows
+    const int key_rows = (p.pair_valid || (kmask & (kmask + 1)) != 0u) ? kSmallRows : (n + 15) & ~15;
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      const bool query = t == 0 || t == 5;
+      const uint32_t mask = query ? qmask : kmask;
+      for (int idx = tid; idx < 8 * (query ? nq : key_rows); idx += kThreads) {
+        const int r = idx >> 3, c = idx & 7;
+        const bool ok = (mask >> r) & 1u;
+        cp_async16(row_chunk(t0 + t * kSmallTile, r, c), src[t] + (t == 5 ? p.act : p.in).at(b, h, ok ? r : 0) + c * 8, ok);
+      }
+    }
+    cp_async_commit();
+  }
+  bool hole = (kmask & (kmask + 1)) != 0u;
+  for (int j = tid >> 5; j < kSmallRows; j += kWarps) {
+    uint32_t word = (j < N && ((kmask >> j) & 1u)) ? kmask : 0u;
+    if (p.pair_valid && word != 0u) {
+      const uint32_t pv = __ballot_sync(0xffffffffu, lane < N && p.pair_valid[((size_t)b * N + j) * N + min(lane, N - 1)] > 0);
+      hole |= (pv & kmask) != kmask;
+      word &= pv;
+    }
+    if (lane == 0) sm.visible[j] = word;
+  }
+  for (int idx = tid; idx < kSmallRows * kD / 8; idx += kThreads) reinterpret_cast<float4*>(sm.dq)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (kBias) {
+    for (int idx = tid; idx < 8 * 32; idx += kThreads) {
+      const int f = idx >> 5, ln = idx & 31, j = (f >> 2) * 16 + (ln >> 2), k = (f & 3) * 8 + 2 * (ln & 3);
+      const float* w = p.w + (size_t)bh * N * N;
+      float4 v;
+      v.x = (j < n && k < n) ? w[j * N + k] : 0.f;
+      v.y = (j < n && k + 1 < n) ? w[j * N + k + 1] : 0.f;
+      v.z = (j + 8 < n && k < n) ? w[(j + 8) * N + k] : 0.f;
+      v.w = (j + 8 < n && k + 1 < n) ? w[(j + 8) * N + k + 1] : 0.f;
+      sm.w[f][ln] = v;
+    }
+  }
+  // delta_i = dO_i . out_i, eight lanes per query
+  for (int idx = tid; idx < ((8 * nq + 31) & ~31); idx += kThreads) {
+    const int i = idx >> 3, c = idx & 7;
+    float d = 0.f;
+    if (i < nq && ((qmask >> i) & 1u)) {
+      const float4* o = reinterpret_cast<const float4*>(p.out + ((size_t)bh * N + i) * kD + c * 8);
+      const uint4 g = *reinterpret_cast<const uint4*>(p.grad_out + p.act.at(b, h, i) + c * 8);
+      const float4 x = o[0], y = o[1];
+      d = fmaf(x.x, bf16_lo(g.x), fmaf(x.y, bf16_hi(g.x), fmaf(x.z, bf16_lo(g.y), x.w * bf16_hi(g.y))));
+      d = fmaf(y.x, bf16_lo(g.z), fmaf(y.y, bf16_hi(g.z), fmaf(y.z, bf16_lo(g.w), fmaf(y.w, bf16_hi(g.w), d))));
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    if (c == 0 && i < nq) {
+      sm.delta[i] = d;
+      sm.lse2[i] = p.lse[(size_t)bh * N + i] * kLog2e;
+    }
+  }
+  cp_async_wait<0>();
+  hole = __syncthreads_or(hole) != 0;
+  if (n > 0 && p.q_scale != 1.f) {  // a power of two: exact
+    const uint32_t scale2 = pack2_bf16(p.q_scale, p.q_scale);
+    uint4* q = reinterpret_cast<uint4*>(sm.tile[0]);
+    for (int idx = tid; idx < 8 * nq; idx += kThreads) {
+      uint4 v = q[idx];
+      v.x = mul_bf16x2(v.x, scale2), v.y = mul_bf16x2(v.y, scale2), v.z = mul_bf16x2(v.z, scale2), v.w = mul_bf16x2(v.w, scale2);
+      q[idx] = v;
+    }
+    __syncthreads();
+  }
+  if (n > 0) {
+    if (hole) small_bwd_walks<2, 4, true, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else if (n <= 16) small_bwd_walks<1, 2, false, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else if (n <= 24) small_bwd_walks<2, 3, false, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else small_bwd_walks<2, 4, false, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
+  }
+  // the rows of dq, and everything when the molecule has no valid query or key
+  __nv_bfloat16* dst[5] = {p.dq, p.dk1, p.dv1, p.dk2, p.dv2};
+  for (int idx = tid; idx < (n > 0 ? 1 : 5) * 8 * N; idx += kThreads) {
+    const int t = idx / (8 * N), rem = idx - t * 8 * N, r = rem >> 3, c = rem & 7;
+    *reinterpret_cast<uint4*>(dst[t] + p.in.at(b, h, r) + 8 * c) =
+        t == 0 ? *reinterpret_cast<const uint4*>(&sm.dq[r][8 * c]) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  if constexpr (kBias) {
+    if (n == 0 && p.dw)
+      for (int idx = tid; idx < N * N; idx += kThreads) p.dw[(size_t)bh * N * N + idx] = 0.f;
+    // rows of du, dv and dgate that no query wrote
+    for (int i = tid >> 5; i < N; i += kWarps)
+      if (i >= nq || !((qmask >> i) & 1u)) {
+        const size_t at = ((size_t)bh * N + i) * N;
+        if (lane < N) {
+          if (p.du) p.du[at + lane] = 0.f;
+          if (p.dv_bias) p.dv_bias[at + lane] = 0.f;
+        }
+        if (p.dgate && lane == 0) p.dgate[(size_t)bh * N + i] = 0.f;
+      }
+  }
+}
+
+}  // namespace
+
+int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream) {
+  SmallBwdParams p{};
+  p.grad_out = static_cast<const __nv_bfloat16*>(a.grad_out);
+  p.q = static_cast<const __nv_bfloat16*>(a.q);
+  p.k1 = static_cast<const __nv_bfloat16*>(a.k1);
+  p.v1 = static_cast<const __nv_bfloat16*>(a.v1);
+  p.k2 = static_cast<const __nv_bfloat16*>(a.k2);
+  p.v2 = static_cast<const __nv_bfloat16*>(a.v2);
+  p.out = a.out;
+  p.lse = a.lse;
+  p.query_valid = a.query_valid;
+  p.key_valid = a.pair_key_valid;
+  p.pair_valid = a.pair_valid;
+  p.u = a.u, p.v_bias = a.v_bias, p.w = a.w, p.gate = a.gate;
+  p.du = a.du, p.dv_bias = a.dv_bias, p.dw = a.dw, p.dgate = a.dgate;
+  p.dq = static_cast<__nv_bfloat16*>(a.dq);
+  p.dk1 = static_cast<__nv_bfloat16*>(a.dk1);
+  p.dv1 = static_cast<__nv_bfloat16*>(a.dv1);
+  p.dk2 = static_cast<__nv_bfloat16*>(a.dk2);
+  p.dv2 = static_cast<__nv_bfloat16*>(a.dv2);
+  p.H = a.heads;
+  p.N = a.tokens;
+  p.q_scale = layouts ? layouts->q_scale : 1.f;
+  p.in = layouts ? layouts->in : contiguous_rows(a.heads, a.tokens);
+  p.act = layouts ? layouts->act : contiguous_rows(a.heads, a.tokens);
+  const int bh = a.batch * a.heads;
+  // Eight warps of 255 registers fill an SM: four (batch, head)s of two warps each, or two of four.
+  const int warps = bh >= 1024 ? 2 : 4;
+  profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
+  cudaError_t e = cudaSuccess;
+#define MF_LAUNCH(BIAS, S)                                                                                             \
+  do {                                                                                                                 \
+    constexpr int bytes = (int)sizeof(SmallBwdShared<BIAS>);                                                        \
+    e = cudaFuncSetAttribute(simplicial_small_bwd_kernel<BIAS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
+    if (e == cudaSuccess) simplicial_small_bwd_kernel<BIAS, S><<<bh, 32 * S, bytes, stream>>>(p);                      \
+  } while (0)
+  if (a.u) {
+    if (warps == 2) MF_LAUNCH(true, 2);
+    else MF_LAUNCH(true, 4);
+  } else {
+    if (warps == 2) MF_LAUNCH(false, 2);
+    else MF_LAUNCH(false, 4);
+  }
+#undef MF_LAUNCH
+  if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_small_bwd_kernel)");
+  profile_mark(MF_PROFILE_SIMPLICIAL_BWD, false, stream);
+  MF_CHECK_LAUNCH("simplicial_small_bwd_kernel");
+  return MF_OK;
+}
+
+}  // namespace mf

@@ -62,7 +62,8 @@ def set_check_status(on: bool) -> bool:
 
 def _remember_status(ws: Optional[torch.Tensor]) -> None:
     global _LAST_STATUS
-    if ws is None or ws.numel() < 4:
+    if ws is None:  # a kernel without device-side waits: nothing can expire
+        _LAST_STATUS = None
         return
     _LAST_STATUS = ws[:4].view(torch.int32).clone()
     if _CHECK_STATUS and not torch.cuda.is_current_stream_capturing():
@@ -344,8 +345,8 @@ def cuda_simplicial_attention_backward(
         )
     L = _lib.lib()
     need = L.mf_simplicial_bwd_workspace_bytes(ctypes.byref(a))
-    ws = torch.empty(max(need, 1), device=q.device, dtype=torch.uint8)
-    a.workspace = ws.data_ptr()
+    ws = torch.empty(need, device=q.device, dtype=torch.uint8) if need else None
+    a.workspace = ws.data_ptr() if ws is not None else None
     a.workspace_bytes = need
     with torch.cuda.device(q.device):
         _lib.check(L.mf_simplicial_bwd(ctypes.byref(a), _stream(q.device)))
@@ -465,13 +466,9 @@ class _PackedSimplicialAttention(torch.autograd.Function):
                                         proj=proj.data_ptr(), query_valid=qv.data_ptr(), pair_key_valid=kv.data_ptr(),
                                         pair_valid=pv.data_ptr() if pv is not None else None, out32=out32.data_ptr(),
                                         lse=lse.data_ptr(), out=out.data_ptr())  # fmt: skip
-        L = _lib.lib()
-        need = int(L.mf_simplicial_packed_fwd_workspace_bytes(ctypes.byref(a)))
-        ws = torch.empty(max(need, 16), device=proj.device, dtype=torch.uint8)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), need
         with torch.cuda.device(proj.device):
-            _lib.check(L.mf_simplicial_packed_fwd(ctypes.byref(a), _stream(proj.device)))
-        _remember_status(ws)
+            _lib.check(_lib.lib().mf_simplicial_packed_fwd(ctypes.byref(a), _stream(proj.device)))
+        _remember_status(None)
         ctx.save_for_backward(proj, qv, kv, pv, out32, lse)
         ctx.meta = (heads, float(q_scale))
         return out
@@ -489,13 +486,9 @@ class _PackedSimplicialAttention(torch.autograd.Function):
                                         pair_valid=pv.data_ptr() if pv is not None else None, out32=out32.data_ptr(),
                                         lse=lse.data_ptr(), grad_out=grad_out.data_ptr(),
                                         grad_proj=grad_proj.data_ptr())  # fmt: skip
-        L = _lib.lib()
-        need = int(L.mf_simplicial_packed_bwd_workspace_bytes(ctypes.byref(a)))
-        ws = torch.empty(max(need, 16), device=proj.device, dtype=torch.uint8)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), need
         with torch.cuda.device(proj.device):
-            _lib.check(L.mf_simplicial_packed_bwd(ctypes.byref(a), _stream(proj.device)))
-        _remember_status(ws)
+            _lib.check(_lib.lib().mf_simplicial_packed_bwd(ctypes.byref(a), _stream(proj.device)))
+        _remember_status(None)
         return grad_proj, None, None, None, None, None
 
 
