@@ -280,6 +280,13 @@ size_t mf_knn_cells_workspace_bytes(int32_t batch, int32_t n_max);
 int mf_knn_topk_cells(const float* frac, const float* cell, const int32_t* num_atoms, const int32_t* grid_dims,
                       const float* bounds, int32_t batch, int32_t n_max, int32_t k, int32_t include_self,
                       int32_t* idx, float* dist2, void* workspace, size_t workspace_bytes, void* stream);
+/*
+ * The same from what a model holds: `lattice` is (B,6) fp32 latents, or (B,3,3) cells when `lattice_is_cell` (see
+ * mf_radius_blocks below); the search grid is chosen as mf_knn_search_grid does.  Workspace as for mf_knn_topk_cells.
+ */
+int mf_knn_topk_lattice(const float* frac, const float* lattice, int32_t lattice_is_cell, const int32_t* num_atoms,
+                        int32_t batch, int32_t n_max, int32_t k, int32_t include_self, int32_t* idx, float* dist2,
+                        void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * Cell sort + radius block list.
@@ -300,6 +307,14 @@ int mf_cell_sort_blocklist(const float* frac, const float* cell, const int32_t* 
                            int32_t batch, int32_t n_max, float cutoff, int32_t* perm, int32_t* block_count,
                            int32_t* block_cols, uint32_t* block_mask, void* workspace, size_t workspace_bytes,
                            void* stream);
+/*
+ * The same from what a model holds: `lattice` is (B,6) fp32 latents [log a, log b, log c, cos alpha, cos beta, cos gamma]
+ * (ref: lattice_latent_to_lower_triangular, src/matterformer/geometry/lattice.py:12-47), or (B,3,3) cells when
+ * `lattice_is_cell`; the grid has floor(perpendicular width / cutoff) cells per axis, between 1 and 64.
+ */
+int mf_radius_blocks(const float* frac, const float* lattice, int32_t lattice_is_cell, const int32_t* num_atoms,
+                     int32_t batch, int32_t n_max, double cutoff, int32_t* perm, int32_t* block_count, int32_t* block_cols,
+                     uint32_t* block_mask, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------- */
 /* Radius block-sparse attention and local-window attention                   */

@@ -7,8 +7,10 @@ fails loudly instead of silently computing somewhere else.
 from __future__ import annotations
 
 import ctypes
-from ctypes import POINTER, Structure, c_char_p, c_float, c_int32, c_size_t, c_void_p
+from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int32, c_size_t, c_void_p
 from pathlib import Path
+
+import torch
 
 LIB_PATH = Path(__file__).resolve().parent / "libmatterformer_b200.so"
 
@@ -40,8 +42,10 @@ EXPORTED_SYMBOLS = (
     "mf_knn_search_grid",
     "mf_knn_cells_workspace_bytes",
     "mf_knn_topk_cells",
+    "mf_knn_topk_lattice",
     "mf_radius_blocks_workspace_bytes",
     "mf_cell_sort_blocklist",
+    "mf_radius_blocks",
     "mf_sparse_attn_bwd_workspace_bytes",
     "mf_radius_attn_fwd",
     "mf_radius_attn_bwd",
@@ -310,6 +314,12 @@ def lib() -> ctypes.CDLL:
         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p,
     ]  # fmt: skip
     L.mf_cell_sort_blocklist.restype = c_int32
+    L.mf_knn_topk_lattice.argtypes = [c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p,
+                                      c_void_p, c_size_t, c_void_p]  # fmt: skip
+    L.mf_knn_topk_lattice.restype = c_int32
+    L.mf_radius_blocks.argtypes = [c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int32, c_double, c_void_p, c_void_p, c_void_p,
+                                   c_void_p, c_void_p, c_size_t, c_void_p]  # fmt: skip
+    L.mf_radius_blocks.restype = c_int32
     L.mf_sparse_attn_bwd_workspace_bytes.argtypes = [POINTER(MfSparseAttnArgs)]
     L.mf_sparse_attn_bwd_workspace_bytes.restype = c_size_t
     for name in ("mf_radius_attn_fwd", "mf_radius_attn_bwd", "mf_local_attn_fwd", "mf_local_attn_bwd"):
@@ -404,6 +414,18 @@ def check(rc: int) -> None:
     if rc == MF_ERR_INVALID_ARGUMENT:
         raise ValueError(msg)
     raise RuntimeError(msg)
+
+
+def launch(fn, device: torch.device, *args) -> None:
+    """``fn(*args, stream)`` on the current stream of ``device``, with that device current, errors raised."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    if index == torch.cuda.current_device():
+        rc = fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    else:
+        with torch.cuda.device(index):
+            rc = fn(*args, torch._C._cuda_getCurrentRawStream(index))
+    if rc != MF_OK:
+        check(rc)
 
 
 def simplicial_row_plan(n_queries: int, valid_keys: int) -> tuple[int, int, int, int]:

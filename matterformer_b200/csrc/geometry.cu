@@ -95,90 +95,178 @@ __global__ void __launch_bounds__(128) knn_kernel(const float* __restrict__ frac
 }
 
 // ---------------------------------------------------------------------------
-// cell sort
+// cell sort and block list: two launches
+//
+// Bound by launches and the host: 8 structures of 300-500 atoms took 443 us as 54 launches (the cell and the grid as chains
+// of element-wise operations, keys, ranks, one CTA per pair of tiles, compaction) of 132 us on the device, and take 27 us
+// as two.
 // ---------------------------------------------------------------------------
-__global__ void cell_key_kernel(const float* __restrict__ frac, const int32_t* __restrict__ num_atoms,
-                                const int32_t* __restrict__ grid_dims, int n_max, int32_t* __restrict__ keys) {
-  const int b = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_max) return;
-  const int n = min(num_atoms[b], n_max);
-  int key = INT32_MAX;
-  if (i < n) {
-    const float* p = frac + ((size_t)b * n_max + i) * 3;
-    const int gx = grid_dims[3 * b + 0], gy = grid_dims[3 * b + 1], gz = grid_dims[3 * b + 2];
-    key = (cell_coord(p[0], gx) * gy + cell_coord(p[1], gy)) * gz + cell_coord(p[2], gz);
+// What the second kernel needs of a structure: its cell and the perpendicular widths.
+struct StructureInfo {
+  float cell[9];
+  float width[3];
+};
+
+constexpr int kRankAtoms = 64;   // atoms per CTA
+constexpr int kRankTile = 2048;  // keys in shared memory at a time
+
+// Grid cell of every atom and its rank = number of atoms with a smaller (cell, index); padded atoms keep their place.
+// The cell comes from `lattice` (latents) or `cell`, the grid from `grid_dims` or from the widths and the cutoff; every CTA
+// of a structure works both out again, which costs less than a launch.  16 threads share an atom's comparisons.
+__global__ void __launch_bounds__(1024) cell_rank_kernel(const float* __restrict__ frac, const float* __restrict__ lattice,
+                                                         const float* __restrict__ cell, const int32_t* __restrict__ num_atoms,
+                                                         const int32_t* __restrict__ grid_dims, double cutoff, int n_max,
+                                                         StructureInfo* __restrict__ info, int32_t* __restrict__ perm) {
+  __shared__ int32_t keys[kRankTile];
+  __shared__ float sc[9];
+  __shared__ int grid[3];
+  const int b = blockIdx.y, tid = threadIdx.x, n = min(num_atoms[b], n_max);
+  const int i0 = blockIdx.x * kRankAtoms;
+  if (tid < 32) {
+    if (lattice) {
+      if (tid == 0) cell_from_latent(lattice + (size_t)b * 6, sc);
+    } else if (tid < 9) {
+      sc[tid] = cell[(size_t)b * 9 + tid];
+    }
+    __syncwarp();
+    if (tid < 3) {
+      double vol;
+      const double w = axis_width(sc, tid, &vol);
+      grid[tid] = grid_dims ? grid_dims[3 * b + tid] : (int)fmin(fmax(floor(w / fmax(cutoff, 1e-12)), 1.0), 64.0);
+      if (blockIdx.x == 0) info[b].width[tid] = (float)w;
+    }
+    if (blockIdx.x == 0 && tid < 9) info[b].cell[tid] = sc[tid];
   }
-  keys[(size_t)b * n_max + i] = key;
+  __syncthreads();
+  const int gx = grid[0], gy = grid[1], gz = grid[2];
+  auto key_of = [&](int i) {
+    const float* p = frac + ((size_t)b * n_max + i) * 3;
+    return (cell_coord(p[0], gx) * gy + cell_coord(p[1], gy)) * gz + cell_coord(p[2], gz);
+  };
+  const int i = i0 + (tid >> 4), part = tid & 15;
+  const int ki = i < n ? key_of(i) : 0;
+  int rank = 0;
+  for (int j0 = 0; j0 < n && i0 < n; j0 += kRankTile) {
+    const int cnt = min(kRankTile, n - j0);
+    __syncthreads();
+    for (int t = tid; t < cnt; t += 1024) keys[t] = key_of(j0 + t);
+    __syncthreads();
+#pragma unroll 4
+    for (int t = part; t < cnt; t += 16) rank += keys[t] < ki + (j0 + t < i ? 1 : 0);  // ties: the lower index first
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+  if (part == 0 && i < n_max) perm[(size_t)b * n_max + (i < n ? rank : i)] = i;
 }
 
-// rank of atom i = number of atoms with a smaller (key, index); padded atoms keep their place.
-__global__ void __launch_bounds__(256) cell_rank_kernel(const int32_t* __restrict__ keys,
-                                                        const int32_t* __restrict__ num_atoms, int n_max,
-                                                        int32_t* __restrict__ perm) {
-  __shared__ int32_t sk[256];
-  const int b = blockIdx.y;
-  const int n = min(num_atoms[b], n_max);
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  const int32_t* kb = keys + (size_t)b * n_max;
-  const int32_t ki = (i < n) ? kb[i] : INT32_MAX;
-  int rank = 0;
-  for (int j0 = 0; j0 < n; j0 += 256) {
-    __syncthreads();
-    if (j0 + threadIdx.x < n) sk[threadIdx.x] = kb[j0 + threadIdx.x];
-    __syncthreads();
-    const int cnt = min(256, n - j0);
-    if (i < n) {
-      for (int t = 0; t < cnt; ++t) {
-        const int32_t kj = sk[t];
-        rank += (kj < ki) || (kj == ki && (j0 + t) < i);
+// Whether one of the 27 images of the pair is within the cutoff: the images that min_image_d2 would minimise over, less
+// those that lie farther than the cutoff by their distance along one axis alone.  That bound carries a margin for the
+// rounding of the distances it stands for, so the answer is the same bit.
+__device__ __forceinline__ bool within_cutoff(float xi, float yi, float zi, float xj, float yj, float zj, const Cell& c,
+                                              const float* width, float cutoff, float margin) {
+  const float dx = __fsub_rn(xi, xj), dy = __fsub_rn(yi, yj), dz = __fsub_rn(zi, zj);
+  const float limit = fmaf(margin, fabsf(dx) + fabsf(dy) + fabsf(dz) + 3.f, cutoff * 1.0001f);
+  bool hit = false;
+#pragma unroll 1
+  for (int ox = -1; ox <= 1; ++ox) {
+    const float ax = __fadd_rn(dx, (float)ox);
+    if (fabsf(ax) * width[0] > limit) continue;
+#pragma unroll 1
+    for (int oy = -1; oy <= 1; ++oy) {
+      const float ay = __fadd_rn(dy, (float)oy);
+      if (fabsf(ay) * width[1] > limit) continue;
+#pragma unroll
+      for (int oz = -1; oz <= 1; ++oz) {
+        const float az = __fadd_rn(dz, (float)oz);
+        if (fabsf(az) * width[2] > limit) continue;
+        const float d2 = image_d2(dx, dy, dz, (float)ox, (float)oy, (float)oz, c);
+        hit |= __fsqrt_rn(d2) <= cutoff;
       }
     }
   }
-  if (i < n)
-    perm[(size_t)b * n_max + rank] = i;
-  else if (i < n_max)
-    perm[(size_t)b * n_max + i] = i;
+  return hit;
 }
 
-// one block per (column tile J, row tile I, batch); warp r = row of the tile, lane c = column
-__global__ void __launch_bounds__(1024) block_mask_kernel(const float* __restrict__ frac,
-                                                          const float* __restrict__ cell,
-                                                          const int32_t* __restrict__ num_atoms,
-                                                          const int32_t* __restrict__ perm, int n_max, int tiles,
-                                                          float cutoff, uint32_t* __restrict__ block_mask,
-                                                          int32_t* __restrict__ active) {
-  const int J = blockIdx.x, I = blockIdx.y, b = blockIdx.z;
-  const int r = threadIdx.x >> 5, cidx = threadIdx.x & 31;
+// One CTA per row tile I; warp r = row of the tile, lane = column of the column tile J.  The active column tiles are
+// collected in shared memory and listed at the end.
+__global__ void __launch_bounds__(1024) block_list_kernel(const float* __restrict__ frac, const StructureInfo* __restrict__ info,
+                                                          const int32_t* __restrict__ num_atoms, const int32_t* __restrict__ perm,
+                                                          int n_max, int tiles, float cutoff, uint32_t* __restrict__ block_mask,
+                                                          int32_t* __restrict__ block_count, int32_t* __restrict__ block_cols) {
+  extern __shared__ uint32_t active[];  // bit J
+  const int I = blockIdx.x, b = blockIdx.y;
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = min(num_atoms[b], n_max);
-  const int si = 32 * I + r, sj = 32 * J + cidx;
   const float* pos = frac + (size_t)b * n_max * 3;
   const int32_t* pb = perm + (size_t)b * n_max;
-  bool hit = false;
-  if (si < n && sj < n) {
-    const Cell c = load_cell(cell + (size_t)b * 9);
-    const int ai = pb[si], aj = pb[sj];
-    const float d2 = min_image_d2(pos[3 * ai], pos[3 * ai + 1], pos[3 * ai + 2], pos[3 * aj], pos[3 * aj + 1],
-                                  pos[3 * aj + 2], c);
-    hit = __fsqrt_rn(d2) <= cutoff;
+  const int words = (tiles + 31) / 32;
+  for (int t = threadIdx.x; t < words; t += 1024) active[t] = 0u;
+  const Cell c = load_cell(info[b].cell);
+  const float width[3] = {info[b].width[0], info[b].width[1], info[b].width[2]};
+  float sum = 0.f;
+#pragma unroll
+  for (int t = 0; t < 9; ++t) sum += fabsf(info[b].cell[t]);
+  const float margin = 4e-6f * sum;
+  const int si = 32 * I + r;
+  float xi = 0.f, yi = 0.f, zi = 0.f;
+  if (si < n) {
+    const int ai = pb[si];
+    xi = pos[3 * ai], yi = pos[3 * ai + 1], zi = pos[3 * ai + 2];
   }
-  const uint32_t word = __ballot_sync(0xffffffffu, hit);
-  if (cidx == 0) block_mask[(((size_t)b * tiles + I) * tiles + J) * 32 + r] = word;
-  const int any = __syncthreads_or(hit);
-  if (threadIdx.x == 0) active[((size_t)b * tiles + I) * tiles + J] = any;
+  __syncthreads();
+  uint32_t* mask = block_mask + ((size_t)b * tiles + I) * tiles * 32 + r;
+  int aj = lane < n ? pb[lane] : 0;
+  for (int J = 0; J < tiles; ++J) {
+    const int sj = 32 * J + lane, nj = sj + 32;
+    const float xj = pos[3 * aj], yj = pos[3 * aj + 1], zj = pos[3 * aj + 2];
+    aj = nj < n ? pb[nj] : 0;  // of the next column tile
+    const bool hit = si < n && sj < n && within_cutoff(xi, yi, zi, xj, yj, zj, c, width, cutoff, margin);
+    const uint32_t word = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) {
+      mask[(size_t)J * 32] = word;
+      if (word) atomicOr(&active[J >> 5], 1u << (J & 31));
+    }
+  }
+  __syncthreads();
+  if (r == 0) {
+    int32_t* cols = block_cols + ((size_t)b * tiles + I) * tiles;
+    int count = 0;
+    for (int w = 0; w < words; ++w) {
+      const uint32_t bits = active[w];
+      if ((bits >> lane) & 1u) cols[count + __popc(bits & ((1u << lane) - 1u))] = 32 * w + lane;
+      count += __popc(bits);
+    }
+    for (int t = count + lane; t < tiles; t += 32) cols[t] = -1;
+    if (lane == 0) block_count[(size_t)b * tiles + I] = count;
+  }
 }
 
-__global__ void block_compact_kernel(const int32_t* __restrict__ active, int tiles, int total_rows,
-                                     int32_t* __restrict__ block_count, int32_t* __restrict__ block_cols) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;  // flattened (b, I)
-  if (row >= total_rows) return;
-  const int32_t* a = active + (size_t)row * tiles;
-  int32_t* cols = block_cols + (size_t)row * tiles;
-  int cnt = 0;
-  for (int J = 0; J < tiles; ++J)
-    if (a[J]) cols[cnt++] = J;
-  block_count[row] = cnt;
-  for (int t = cnt; t < tiles; ++t) cols[t] = -1;
+int radius_blocks(const float* frac, const float* lattice, const float* cell, const int32_t* num_atoms,
+                  const int32_t* grid_dims, int32_t batch, int32_t n_max, double cutoff, int32_t* perm, int32_t* block_count,
+                  int32_t* block_cols, uint32_t* block_mask, void* workspace, size_t workspace_bytes, const char* name,
+                  cudaStream_t s) {
+  MF_CHECK_ARG(batch >= 0 && n_max >= 0, "%s: negative size", name);
+  MF_CHECK_ARG(cutoff >= 0.0, "%s: cutoff must be non-negative", name);
+  if (batch == 0 || n_max == 0) return MF_OK;
+  MF_CHECK_ARG(frac && (lattice || cell) && num_atoms && perm && block_count && block_cols && block_mask,
+               "%s: null pointer argument", name);
+  const size_t need = mf_radius_blocks_workspace_bytes(batch, n_max);
+  if (!workspace || workspace_bytes < need) {
+    set_error("%s: workspace of %zu bytes needed, %zu given", name, need, workspace_bytes);
+    return MF_ERR_WORKSPACE_TOO_SMALL;
+  }
+  MF_CHECK_ARG(batch <= 65535, "%s: batch above 65535", name);
+  const int tiles = (n_max + 31) / 32;
+  const size_t words = (size_t)(tiles + 31) / 32 * 4;
+  MF_CHECK_ARG(words <= 48 * 1024, "%s: %d tokens are too many", name, (int)n_max);  // 12 million
+  StructureInfo* info = static_cast<StructureInfo*>(workspace);
+  cell_rank_kernel<<<dim3((n_max + kRankAtoms - 1) / kRankAtoms, batch), 1024, 0, s>>>(frac, lattice, cell, num_atoms, grid_dims,
+                                                                                       cutoff, n_max, info, perm);
+  MF_CHECK_LAUNCH("cell_rank_kernel");
+  block_list_kernel<<<dim3(tiles, batch), 1024, words, s>>>(frac, info, num_atoms, perm, n_max, tiles, (float)cutoff, block_mask,
+                                                            block_count, block_cols);
+  MF_CHECK_LAUNCH("block_list_kernel");
+  return MF_OK;
 }
 
 }  // namespace
@@ -203,40 +291,24 @@ extern "C" int mf_knn_topk(const float* frac, const float* cell, const int32_t* 
   return MF_OK;
 }
 
-extern "C" size_t mf_radius_blocks_workspace_bytes(int32_t batch, int32_t n_max) {
-  const size_t tiles = (size_t)(n_max + 31) / 32;
-  return align_up((size_t)batch * n_max * sizeof(int32_t), 256) + align_up((size_t)batch * tiles * tiles * 4, 256);
+extern "C" size_t mf_radius_blocks_workspace_bytes(int32_t batch, int32_t) {
+  return align_up((size_t)batch * sizeof(StructureInfo), 256);
 }
 
 extern "C" int mf_cell_sort_blocklist(const float* frac, const float* cell, const int32_t* num_atoms,
                                       const int32_t* grid_dims, int32_t batch, int32_t n_max, float cutoff,
                                       int32_t* perm, int32_t* block_count, int32_t* block_cols,
                                       uint32_t* block_mask, void* workspace, size_t workspace_bytes, void* stream) {
-  MF_CHECK_ARG(batch >= 0 && n_max >= 0, "mf_cell_sort_blocklist: negative size");
-  MF_CHECK_ARG(cutoff >= 0.f, "mf_cell_sort_blocklist: cutoff must be non-negative");
-  if (batch == 0 || n_max == 0) return MF_OK;
-  MF_CHECK_ARG(frac && cell && num_atoms && grid_dims && perm && block_count && block_cols && block_mask,
-               "mf_cell_sort_blocklist: null pointer argument");
-  const size_t need = mf_radius_blocks_workspace_bytes(batch, n_max);
-  if (!workspace || workspace_bytes < need) {
-    set_error("mf_cell_sort_blocklist: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-    return MF_ERR_WORKSPACE_TOO_SMALL;
-  }
-  MF_CHECK_ARG(batch <= 65535, "mf_cell_sort_blocklist: batch above 65535");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int tiles = (n_max + 31) / 32;
-  int32_t* keys = static_cast<int32_t*>(workspace);
-  int32_t* active = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) +
-                                               align_up((size_t)batch * n_max * sizeof(int32_t), 256));
-  cell_key_kernel<<<dim3((n_max + 255) / 256, batch), 256, 0, s>>>(frac, num_atoms, grid_dims, n_max, keys);
-  MF_CHECK_LAUNCH("cell_key_kernel");
-  cell_rank_kernel<<<dim3((n_max + 255) / 256, batch), 256, 0, s>>>(keys, num_atoms, n_max, perm);
-  MF_CHECK_LAUNCH("cell_rank_kernel");
-  block_mask_kernel<<<dim3(tiles, tiles, batch), 1024, 0, s>>>(frac, cell, num_atoms, perm, n_max, tiles, cutoff,
-                                                               block_mask, active);
-  MF_CHECK_LAUNCH("block_mask_kernel");
-  const int rows = batch * tiles;
-  block_compact_kernel<<<(rows + 127) / 128, 128, 0, s>>>(active, tiles, rows, block_count, block_cols);
-  MF_CHECK_LAUNCH("block_compact_kernel");
-  return MF_OK;
+  MF_CHECK_ARG(grid_dims || batch <= 0 || n_max <= 0, "mf_cell_sort_blocklist: null pointer argument");
+  return radius_blocks(frac, nullptr, cell, num_atoms, grid_dims, batch, n_max, cutoff, perm, block_count, block_cols,
+                       block_mask, workspace, workspace_bytes, "mf_cell_sort_blocklist", static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mf_radius_blocks(const float* frac, const float* lattice, int32_t lattice_is_cell, const int32_t* num_atoms,
+                                int32_t batch, int32_t n_max, double cutoff, int32_t* perm, int32_t* block_count,
+                                int32_t* block_cols, uint32_t* block_mask, void* workspace, size_t workspace_bytes,
+                                void* stream) {
+  return radius_blocks(frac, lattice_is_cell ? nullptr : lattice, lattice_is_cell ? lattice : nullptr, num_atoms, nullptr, batch,
+                       n_max, cutoff, perm, block_count, block_cols, block_mask, workspace, workspace_bytes, "mf_radius_blocks",
+                       static_cast<cudaStream_t>(stream));
 }

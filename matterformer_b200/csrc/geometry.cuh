@@ -67,4 +67,31 @@ __device__ __forceinline__ int cell_coord(float f, int g) {
   return min(max(c, 0), g - 1);
 }
 
+// The lower-triangular cell (nine floats, rows = lattice vectors) of the latent [log a, log b, log c, cos alpha, cos beta,
+// cos gamma]: operation for operation what the host-side formula does in fp32 (lattice_latent_to_cell), clamps included.
+__device__ __forceinline__ void cell_from_latent(const float* lat, float* cell) {
+  auto clamp = [](float x, float lo, float hi) { return x != x ? x : fminf(fmaxf(x, lo), hi); };  // NaN stays NaN
+  const float a = expf(clamp(lat[0], -5.f, 5.f)), b = expf(clamp(lat[1], -5.f, 5.f)), c = expf(clamp(lat[2], -5.f, 5.f));
+  const float ca = clamp(lat[3], -0.9999f, 0.9999f), cb = clamp(lat[4], -0.9999f, 0.9999f), cg = clamp(lat[5], -0.9999f, 0.9999f);
+  const float sg = __fsqrt_rn(clamp(__fsub_rn(1.f, __fmul_rn(cg, cg)), 1e-8f, INFINITY));
+  const float c20 = __fmul_rn(c, cb), c21 = __fdiv_rn(__fmul_rn(c, __fsub_rn(ca, __fmul_rn(cb, cg))), sg);
+  const float c22 = __fsqrt_rn(__fsub_rn(__fsub_rn(__fmul_rn(c, c), __fmul_rn(c20, c20)), __fmul_rn(c21, c21)));
+  cell[0] = a, cell[1] = 0.f, cell[2] = 0.f;
+  cell[3] = __fmul_rn(b, cg), cell[4] = __fmul_rn(b, sg), cell[5] = 0.f;
+  cell[6] = c20, cell[7] = c21, cell[8] = clamp(c22, 1e-8f, INFINITY);
+}
+
+// Volume and the perpendicular width along one axis of a cell, in double precision.
+__device__ __forceinline__ double axis_width(const float* c, int axis, double* volume) {
+  const double r[3][3] = {{c[0], c[1], c[2]}, {c[3], c[4], c[5]}, {c[6], c[7], c[8]}};
+  const double bc[3] = {r[1][1] * r[2][2] - r[1][2] * r[2][1], r[1][2] * r[2][0] - r[1][0] * r[2][2],
+                        r[1][0] * r[2][1] - r[1][1] * r[2][0]};
+  const double vol = fabs(r[0][0] * bc[0] + r[0][1] * bc[1] + r[0][2] * bc[2]);
+  const int u = (axis + 1) % 3, v = (axis + 2) % 3;
+  const double x0 = r[u][1] * r[v][2] - r[u][2] * r[v][1], x1 = r[u][2] * r[v][0] - r[u][0] * r[v][2],
+               x2 = r[u][0] * r[v][1] - r[u][1] * r[v][0];
+  *volume = vol;
+  return vol / fmax(sqrt(x0 * x0 + x1 * x1 + x2 * x2), 1e-12);
+}
+
 }  // namespace mf

@@ -32,6 +32,9 @@ struct KnnWorkspace {
   int32_t* keys;     // (B, N) bin of every atom
   int32_t* flags;    // (B) 1 when a coordinate lies outside [0,1)
   float4* sorted;    // (B, N) x, y, z, original index (as int bits), grouped by bin
+  float* cell;       // (B, 3, 3) cells, (B, 3) bins per axis and (B, 2) bounds when the setup kernel worked them out
+  int32_t* grid;
+  float* bounds;
 };
 
 __global__ void knn_zero_kernel(int32_t* counts, int32_t* flags, int B) {
@@ -98,34 +101,127 @@ __global__ void knn_fill_kernel(const float* __restrict__ frac, const int32_t* _
   w.sorted[(size_t)b * n_max + slot] = make_float4(p[0], p[1], p[2], __int_as_float(i));
 }
 
-// Bins per axis and the two distance bounds of the search, one thread per structure (double precision; the
-// bounds are rounded down because they serve as lower bounds on distances to atoms that were not visited).
+// Bins along one axis of a structure and what that axis contributes to the two distance bounds of the search (double
+// precision; the bounds are rounded down because they serve as lower bounds on distances to atoms that were not visited).
+__device__ __forceinline__ int search_bins(const float* c, int axis, int n, int k, double* width) {
+  double vol;
+  const double w = axis_width(c, axis, &vol);
+  vol = fmax(vol, 1e-12);
+  // bin edge ~ 1.25 x the radius of a sphere holding k atoms at the mean density
+  const double r_est = 1.25 * cbrt(3.0 * k * vol / (4.0 * 3.14159265358979323846 * fmax((double)n, 1.0)));
+  *width = w;
+  return (int)fmin(fmax(floor(w / r_est), 1.0), (double)kMaxBinsPerAxis);
+}
+__device__ __forceinline__ void search_bounds(const double (&w)[3], const int (&g)[3], float* bounds) {
+  double h = 1e300, wmin = 1e300;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    h = fmin(h, w[a] / g[a]);
+    wmin = fmin(wmin, w[a]);
+  }
+  bounds[0] = __double2float_rd(h * (1.0 - 1e-6));
+  bounds[1] = __double2float_rd(0.5 * wmin * (1.0 - 1e-6));
+}
+
 __global__ void knn_grid_kernel(const float* __restrict__ cell, const int32_t* __restrict__ num_atoms, int B, int n_max,
                                 int k, int32_t* __restrict__ grid_dims, float* __restrict__ bounds) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
-  const float* c = cell + (size_t)b * 9;
-  const double a0 = c[0], a1 = c[1], a2 = c[2], b0 = c[3], b1 = c[4], b2 = c[5], c0 = c[6], c1 = c[7], c2 = c[8];
-  // cross products b x c, c x a, a x b
-  const double bc0 = b1 * c2 - b2 * c1, bc1 = b2 * c0 - b0 * c2, bc2 = b0 * c1 - b1 * c0;
-  const double ca0 = c1 * a2 - c2 * a1, ca1 = c2 * a0 - c0 * a2, ca2 = c0 * a1 - c1 * a0;
-  const double ab0 = a1 * b2 - a2 * b1, ab1 = a2 * b0 - a0 * b2, ab2 = a0 * b1 - a1 * b0;
-  const double vol = fmax(fabs(a0 * bc0 + a1 * bc1 + a2 * bc2), 1e-12);
-  const double w[3] = {vol / fmax(sqrt(bc0 * bc0 + bc1 * bc1 + bc2 * bc2), 1e-12),
-                       vol / fmax(sqrt(ca0 * ca0 + ca1 * ca1 + ca2 * ca2), 1e-12),
-                       vol / fmax(sqrt(ab0 * ab0 + ab1 * ab1 + ab2 * ab2), 1e-12)};
-  const double n = fmax((double)min(num_atoms[b], n_max), 1.0);
-  // bin edge ~ 1.25 x the radius of a sphere holding k atoms at the mean density
-  const double r_est = 1.25 * cbrt(3.0 * k * vol / (4.0 * 3.14159265358979323846 * n));
-  double h = 1e300, wmin = 1e300;
+  double w[3];
+  int g[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const int g = (int)fmin(fmax(floor(w[a] / r_est), 1.0), (double)kMaxBinsPerAxis);
-    grid_dims[3 * b + a] = g;
-    h = fmin(h, w[a] / g);
-    wmin = fmin(wmin, w[a]);
+    g[a] = search_bins(cell + (size_t)b * 9, a, min(num_atoms[b], n_max), k, &w[a]);
+    grid_dims[3 * b + a] = g[a];
   }
-  bounds[2 * b] = __double2float_rd(h * (1.0 - 1e-6));
-  bounds[2 * b + 1] = __double2float_rd(0.5 * wmin * (1.0 - 1e-6));
+  search_bounds(w, g, bounds + 2 * b);
+}
+
+// Everything before the search in one launch, one CTA per structure: cell, grid, bounds, bin sizes and starts (counted and
+// scanned in shared memory), atoms grouped by bin, empty rows of the padding.  Replaces seven launches (cell and grid, zero,
+// count, scan, fill, padding), which take longer than the work they do for structures of a few thousand atoms; beyond
+// kSetupAtoms one CTA would be slower than the separate kernels.
+constexpr int kSetupAtoms = 16384;
+__global__ void __launch_bounds__(1024) knn_setup_kernel(const float* __restrict__ frac, const float* __restrict__ lattice,
+                                                         const float* __restrict__ cell, const int32_t* __restrict__ num_atoms,
+                                                         int n_max, int k, KnnWorkspace w, int32_t* __restrict__ idx,
+                                                         float* __restrict__ dist2) {
+  __shared__ int32_t bins[kMaxBins];
+  __shared__ int32_t part[32];
+  __shared__ float sc[9];
+  __shared__ double sw[3];
+  __shared__ int sg[3];
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, n = min(num_atoms[b], n_max);
+  if (tid < 32) {
+    if (lattice) {
+      if (tid == 0) cell_from_latent(lattice + (size_t)b * 6, sc);
+    } else if (tid < 9) {
+      sc[tid] = cell[(size_t)b * 9 + tid];
+    }
+    __syncwarp();
+    if (tid < 3) sg[tid] = search_bins(sc, tid, n, k, &sw[tid]);
+    if (tid < 9) w.cell[(size_t)b * 9 + tid] = sc[tid];
+    __syncwarp();
+    if (tid == 0) search_bounds({sw[0], sw[1], sw[2]}, {sg[0], sg[1], sg[2]}, w.bounds + 2 * b);
+    if (tid < 3) w.grid[3 * b + tid] = sg[tid];
+  } else {
+    for (int t = tid - 32; t < kMaxBins; t += 992) bins[t] = 0;
+  }
+  __syncthreads();
+  const int gx = sg[0], gy = sg[1], gz = sg[2];
+  const float* pos = frac + (size_t)b * n_max * 3;
+  bool outside = false;
+  for (int i = tid; i < n; i += 1024) {
+    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
+    outside |= !(x >= 0.f && x < 1.f && y >= 0.f && y < 1.f && z >= 0.f && z < 1.f);
+    atomicAdd(&bins[(cell_coord(x, gx) * gy + cell_coord(y, gy)) * gz + cell_coord(z, gz)], 1);
+  }
+  outside = __syncthreads_or(outside) != 0;
+  if (tid == 0) w.flags[b] = outside;
+  // exclusive scan, four bins per thread
+  int c[4], sum = 0;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    c[t] = bins[4 * tid + t];
+    sum += c[t];
+  }
+  int run = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += v;
+  }
+  if (lane == 31) part[tid >> 5] = run;
+  __syncthreads();
+  if (tid < 32) {
+    int v = part[tid];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    part[tid] = v;
+  }
+  __syncthreads();
+  run += (tid >= 32 ? part[(tid >> 5) - 1] : 0) - sum;
+  int32_t* start = w.counts + (size_t)b * (kMaxBins + 1);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    bins[4 * tid + t] = run;
+    start[4 * tid + t] = run;
+    run += c[t];
+  }
+  if (tid == 1023) start[kMaxBins] = run;
+  __syncthreads();
+  for (int i = tid; i < n; i += 1024) {
+    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
+    const int slot = atomicAdd(&bins[(cell_coord(x, gx) * gy + cell_coord(y, gy)) * gz + cell_coord(z, gz)], 1);
+    w.sorted[(size_t)b * n_max + slot] = make_float4(x, y, z, __int_as_float(i));
+  }
+  for (long long t = tid + (long long)n * k; t < (long long)n_max * k; t += 1024) {
+    idx[(size_t)b * n_max * k + t] = -1;
+    if (dist2) dist2[(size_t)b * n_max * k + t] = INFINITY;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -403,6 +499,10 @@ KnnWorkspace carve(void* ws, int B, int N) {
   w.flags = reinterpret_cast<int32_t*>(p);
   p += align_up((size_t)B * 4, 256);
   w.sorted = reinterpret_cast<float4*>(p);
+  p += align_up((size_t)B * N * sizeof(float4), 256);
+  w.cell = reinterpret_cast<float*>(p);
+  w.grid = reinterpret_cast<int32_t*>(w.cell + 9 * (size_t)B);
+  w.bounds = reinterpret_cast<float*>(w.grid + 3 * (size_t)B);
   return w;
 }
 
@@ -414,7 +514,7 @@ using namespace mf;
 extern "C" size_t mf_knn_cells_workspace_bytes(int32_t batch, int32_t n_max) {
   const size_t B = batch, N = n_max;
   return align_up(B * (kMaxBins + 1) * 4, 256) + align_up(B * kMaxBins * 4, 256) + align_up(B * N * 4, 256) +
-         align_up(B * 4, 256) + align_up(B * N * sizeof(float4), 256);
+         align_up(B * 4, 256) + align_up(B * N * sizeof(float4), 256) + align_up(B * 14 * 4, 256);
 }
 
 extern "C" int mf_knn_search_grid(const float* cell, const int32_t* num_atoms, int32_t batch, int32_t n_max, int32_t k,
@@ -428,22 +528,39 @@ extern "C" int mf_knn_search_grid(const float* cell, const int32_t* num_atoms, i
   return MF_OK;
 }
 
-extern "C" int mf_knn_topk_cells(const float* frac, const float* cell, const int32_t* num_atoms,
-                                 const int32_t* grid_dims, const float* bounds, int32_t batch, int32_t n_max,
-                                 int32_t k, int32_t include_self, int32_t* idx, float* dist2, void* workspace,
-                                 size_t workspace_bytes, void* stream) {
-  MF_CHECK_ARG(batch >= 0 && n_max >= 0, "mf_knn_topk_cells: negative size");
-  MF_CHECK_ARG(k >= 1 && k <= 32, "mf_knn_topk_cells: k must be in [1, 32], got %d", (int)k);
+namespace mf {
+namespace {
+
+int knn_check(const void* frac, const void* cell, const void* num_atoms, int batch, int n_max, int k, const void* idx,
+              const void* workspace, size_t workspace_bytes, const char* name) {
+  MF_CHECK_ARG(batch >= 0 && n_max >= 0, "%s: negative size", name);
+  MF_CHECK_ARG(k >= 1 && k <= 32, "%s: k must be in [1, 32], got %d", name, k);
   if (batch == 0 || n_max == 0) return MF_OK;
-  MF_CHECK_ARG(frac && cell && num_atoms && grid_dims && bounds && idx, "mf_knn_topk_cells: null pointer argument");
-  MF_CHECK_ARG(batch <= 65535, "mf_knn_topk_cells: batch above 65535");
+  MF_CHECK_ARG(frac && cell && num_atoms && idx, "%s: null pointer argument", name);
+  MF_CHECK_ARG(batch <= 65535, "%s: batch above 65535", name);
   const size_t need = mf_knn_cells_workspace_bytes(batch, n_max);
   if (!workspace || workspace_bytes < need) {
-    set_error("mf_knn_topk_cells: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+    set_error("%s: workspace of %zu bytes needed, %zu given", name, need, workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  KnnWorkspace w = carve(workspace, batch, n_max);
+  return MF_OK;
+}
+
+int knn_search(const float* cell, const int32_t* num_atoms, const int32_t* grid_dims, const float* bounds, int batch, int n_max,
+               int k, int include_self, const KnnWorkspace& w, int32_t* idx, float* dist2, cudaStream_t s) {
+  dim3 grid(64, batch);  // 256 warps per structure, each taking every 256th bin
+  if (k <= 16)
+    knn_warp_kernel<16><<<grid, 128, 0, s>>>(cell, num_atoms, grid_dims, bounds, n_max, k, include_self, w, idx, dist2);
+  else
+    knn_warp_kernel<32><<<grid, 128, 0, s>>>(cell, num_atoms, grid_dims, bounds, n_max, k, include_self, w, idx, dist2);
+  MF_CHECK_LAUNCH("knn_warp_kernel");
+  return MF_OK;
+}
+
+// Binning and search on a grid that already exists, without the setup kernel: structures of any size.
+int knn_binned(const float* frac, const float* cell, const int32_t* num_atoms, const int32_t* grid_dims, const float* bounds,
+               int batch, int n_max, int k, int include_self, const KnnWorkspace& w, int32_t* idx, float* dist2,
+               cudaStream_t s) {
   const int zero_n = batch * (kMaxBins + 1);
   knn_zero_kernel<<<(zero_n + 255) / 256, 256, 0, s>>>(w.counts, w.flags, batch);
   MF_CHECK_LAUNCH("knn_zero_kernel");
@@ -454,14 +571,50 @@ extern "C" int mf_knn_topk_cells(const float* frac, const float* cell, const int
   MF_CHECK_LAUNCH("knn_scan_kernel");
   knn_fill_kernel<<<per_atom, 256, 0, s>>>(frac, num_atoms, n_max, w);
   MF_CHECK_LAUNCH("knn_fill_kernel");
-  dim3 grid(64, batch);  // 256 warps per structure, each taking every 256th bin
-  if (k <= 16)
-    knn_warp_kernel<16><<<grid, 128, 0, s>>>(cell, num_atoms, grid_dims, bounds, n_max, k, include_self, w, idx, dist2);
-  else
-    knn_warp_kernel<32><<<grid, 128, 0, s>>>(cell, num_atoms, grid_dims, bounds, n_max, k, include_self, w, idx, dist2);
-  MF_CHECK_LAUNCH("knn_warp_kernel");
+  const int rc = knn_search(cell, num_atoms, grid_dims, bounds, batch, n_max, k, include_self, w, idx, dist2, s);
+  if (rc != MF_OK) return rc;
   const long long pad = (long long)n_max * k;
   knn_pad_rows_kernel<<<dim3((unsigned)((pad + 255) / 256), batch), 256, 0, s>>>(num_atoms, n_max, k, idx, dist2);
   MF_CHECK_LAUNCH("knn_pad_rows_kernel");
   return MF_OK;
+}
+
+__global__ void knn_cell_kernel(const float* __restrict__ lattice, int B, float* __restrict__ cell) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < B) cell_from_latent(lattice + (size_t)b * 6, cell + (size_t)b * 9);
+}
+
+}  // namespace
+}  // namespace mf
+
+extern "C" int mf_knn_topk_cells(const float* frac, const float* cell, const int32_t* num_atoms,
+                                 const int32_t* grid_dims, const float* bounds, int32_t batch, int32_t n_max,
+                                 int32_t k, int32_t include_self, int32_t* idx, float* dist2, void* workspace,
+                                 size_t workspace_bytes, void* stream) {
+  const int rc = knn_check(frac, cell, num_atoms, batch, n_max, k, idx, workspace, workspace_bytes, "mf_knn_topk_cells");
+  if (rc != MF_OK || batch == 0 || n_max == 0) return rc;
+  MF_CHECK_ARG(grid_dims && bounds, "mf_knn_topk_cells: null pointer argument");
+  return knn_binned(frac, cell, num_atoms, grid_dims, bounds, batch, n_max, k, include_self, carve(workspace, batch, n_max), idx,
+                    dist2, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mf_knn_topk_lattice(const float* frac, const float* lattice, int32_t lattice_is_cell, const int32_t* num_atoms,
+                                   int32_t batch, int32_t n_max, int32_t k, int32_t include_self, int32_t* idx, float* dist2,
+                                   void* workspace, size_t workspace_bytes, void* stream) {
+  int rc = knn_check(frac, lattice, num_atoms, batch, n_max, k, idx, workspace, workspace_bytes, "mf_knn_topk_lattice");
+  if (rc != MF_OK || batch == 0 || n_max == 0) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const KnnWorkspace w = carve(workspace, batch, n_max);
+  if (n_max <= kSetupAtoms) {
+    knn_setup_kernel<<<batch, 1024, 0, s>>>(frac, lattice_is_cell ? nullptr : lattice, lattice, num_atoms, n_max, k, w, idx, dist2);
+    MF_CHECK_LAUNCH("knn_setup_kernel");
+    return knn_search(w.cell, num_atoms, w.grid, w.bounds, batch, n_max, k, include_self, w, idx, dist2, s);
+  }
+  if (!lattice_is_cell) {
+    knn_cell_kernel<<<(batch + 127) / 128, 128, 0, s>>>(lattice, batch, w.cell);
+    MF_CHECK_LAUNCH("knn_cell_kernel");
+  }
+  const float* cell = lattice_is_cell ? lattice : w.cell;
+  if ((rc = mf_knn_search_grid(cell, num_atoms, batch, n_max, k, w.grid, w.bounds, stream)) != MF_OK) return rc;
+  return knn_binned(frac, cell, num_atoms, w.grid, w.bounds, batch, n_max, k, include_self, w, idx, dist2, s);
 }

@@ -53,6 +53,14 @@ def _as_cell(lattice_or_cell: torch.Tensor) -> torch.Tensor:
     return lattice_latent_to_cell(lattice_or_cell).contiguous()
 
 
+def _lattice_operand(lattice: torch.Tensor, device: torch.device) -> tuple[torch.Tensor, int]:
+    """The lattice as the kernels take it, fp32 on ``device``, and whether it holds cells.  Latents stay latents: the kernels
+    form the cell, with the operations of :func:`lattice_latent_to_cell`, instead of some twenty launches here."""
+    if lattice.device == device and lattice.ndim == 2 and lattice.shape[-1] == 6:
+        return lattice.detach().float().contiguous(), 0
+    return _as_cell(lattice.detach()).to(device), 1
+
+
 def cell_grid_dims(cell: torch.Tensor, cutoff: float, max_per_axis: int = 64) -> torch.Tensor:
     """Cells per axis = floor(perpendicular width / cutoff), clamped to [1, max_per_axis]. (B,3) int32."""
     c = cell.double()
@@ -109,22 +117,20 @@ def knn_topk(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Optional[torch
         raise ValueError(f"method must be 'cells' or 'pairs', got {method!r}")
     B, N, _ = pos.shape
     frac = pos.float().contiguous()
-    cell = _as_cell(lattice).to(pos.device)
     na = _num_atoms(num_atoms, B, N, pos.device)
     idx = torch.empty((B, N, k), device=pos.device, dtype=torch.int32)
     d2 = torch.empty((B, N, k), device=pos.device, dtype=torch.float32)
     L = _lib.lib()
-    with torch.cuda.device(pos.device):
-        if method == "pairs":
-            _lib.check(L.mf_knn_topk(frac.data_ptr(), cell.data_ptr(), na.data_ptr(), B, N, int(k),
-                                     int(bool(include_self)), idx.data_ptr(), d2.data_ptr(), _stream(pos.device)))  # fmt: skip
-        else:
-            gd, bounds = knn_search_grid(cell, na, int(k))
-            need = L.mf_knn_cells_workspace_bytes(B, N)
-            ws = torch.empty(max(need, 1), device=pos.device, dtype=torch.uint8)
-            _lib.check(L.mf_knn_topk_cells(frac.data_ptr(), cell.data_ptr(), na.data_ptr(), gd.data_ptr(),
-                                           bounds.data_ptr(), B, N, int(k), int(bool(include_self)), idx.data_ptr(),
-                                           d2.data_ptr(), ws.data_ptr(), need, _stream(pos.device)))  # fmt: skip
+    if method == "pairs":
+        cell = _as_cell(lattice).to(pos.device)
+        _lib.launch(L.mf_knn_topk, pos.device, frac.data_ptr(), cell.data_ptr(), na.data_ptr(), B, N, int(k),
+                    int(bool(include_self)), idx.data_ptr(), d2.data_ptr())  # fmt: skip
+    else:
+        lat, is_cell = _lattice_operand(lattice, pos.device)
+        need = L.mf_knn_cells_workspace_bytes(B, N)
+        ws = torch.empty(max(need, 1), device=pos.device, dtype=torch.uint8)
+        _lib.launch(L.mf_knn_topk_lattice, pos.device, frac.data_ptr(), lat.data_ptr(), is_cell, na.data_ptr(), B, N, int(k),
+                    int(bool(include_self)), idx.data_ptr(), d2.data_ptr(), ws.data_ptr(), need)  # fmt: skip
     return idx, d2
 
 
@@ -159,9 +165,7 @@ def build_radius_blocks(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Opt
     T = (N + 31) // 32
     dev = pos.device
     frac = pos.float().contiguous()
-    cell = _as_cell(lattice).to(dev)
     na = _num_atoms(num_atoms, B, N, dev)
-    gd = (cell_grid_dims(cell, cutoff) if grid_dims is None else grid_dims.to(device=dev, dtype=torch.int32)).contiguous()
     perm = torch.empty((B, N), device=dev, dtype=torch.int32)
     count = torch.empty((B, T), device=dev, dtype=torch.int32)
     cols = torch.empty((B, T, T), device=dev, dtype=torch.int32)
@@ -169,10 +173,15 @@ def build_radius_blocks(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Opt
     L = _lib.lib()
     need = L.mf_radius_blocks_workspace_bytes(B, N)
     ws = torch.empty(max(need, 1), device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
-        _lib.check(L.mf_cell_sort_blocklist(frac.data_ptr(), cell.data_ptr(), na.data_ptr(), gd.data_ptr(), B, N,
-                                            float(cutoff), perm.data_ptr(), count.data_ptr(), cols.data_ptr(),
-                                            mask.data_ptr(), ws.data_ptr(), need, _stream(dev)))  # fmt: skip
+    out = (perm.data_ptr(), count.data_ptr(), cols.data_ptr(), mask.data_ptr(), ws.data_ptr(), need)
+    if grid_dims is None:
+        lat, is_cell = _lattice_operand(lattice, dev)
+        _lib.launch(L.mf_radius_blocks, dev, frac.data_ptr(), lat.data_ptr(), is_cell, na.data_ptr(), B, N, float(cutoff), *out)
+    else:
+        cell = _as_cell(lattice).to(dev)
+        gd = grid_dims.to(device=dev, dtype=torch.int32).contiguous()
+        _lib.launch(L.mf_cell_sort_blocklist, dev, frac.data_ptr(), cell.data_ptr(), na.data_ptr(), gd.data_ptr(), B, N,
+                    float(cutoff), *out)  # fmt: skip
     return RadiusBlocks(perm=perm, block_count=count, block_cols=cols, block_mask=mask, num_atoms=na,
                         cutoff=float(cutoff))  # fmt: skip
 
