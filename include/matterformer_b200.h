@@ -186,6 +186,9 @@ size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* args);
  * in the reference.)  Only the tensor-core kernels leave a status word at the start of the workspace. */
 int mf_simplicial_fwd_backend(const MfSimplicialFwdArgs* args);
 int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* args);
+/* 1 when the gradients of bias and residual operands have to be zero-filled before this call, 0 when the kernels that would
+ * serve it write every element themselves (molecules of at most 32 tokens on the tensor cores). */
+int mf_simplicial_bwd_needs_zeros(const MfSimplicialBwdArgs* args);
 
 /* How the row-packed tensor-core kernels lay a molecule with `n_queries` queries (1 + index of the last valid
  * one) and `valid_keys` valid keys onto 128-row tiles: plan[0] = query ranges, plan[1] = queries per range,

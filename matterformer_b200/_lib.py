@@ -29,6 +29,7 @@ MF_SPARSE_BACKEND = {"auto": 0, "mma": 1, "tcgen05": 2}
 # Every symbol include/matterformer_b200.h declares.
 EXPORTED_SYMBOLS = (
     "mf_simplicial_fwd_backend",
+    "mf_simplicial_bwd_needs_zeros",
     "mf_simplicial_bwd_backend",
     "mf_simplicial_row_plan",
     "mf_simplicial_fwd_workspace_bytes",
@@ -381,6 +382,8 @@ def lib() -> ctypes.CDLL:
     L.mf_simplicial_fwd_backend.restype = c_int32
     L.mf_simplicial_bwd_backend.argtypes = [POINTER(MfSimplicialBwdArgs)]
     L.mf_simplicial_bwd_backend.restype = c_int32
+    L.mf_simplicial_bwd_needs_zeros.argtypes = [POINTER(MfSimplicialBwdArgs)]
+    L.mf_simplicial_bwd_needs_zeros.restype = c_int32
     L.mf_profile_enable.argtypes = [c_int32]
     L.mf_profile_enable.restype = c_int32
     L.mf_profile_read.argtypes = [c_int32, POINTER(ctypes.c_double), POINTER(c_int32)]

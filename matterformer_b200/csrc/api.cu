@@ -63,12 +63,12 @@ int check_bias(const Args* a, const char* name) {
 
 inline bool vectors_aligned(const MfSimplicialFwdArgs* a) {
   return aligned16(a->q) && aligned16(a->k1) && aligned16(a->v1) && aligned16(a->k2) && aligned16(a->v2) &&
-         aligned16(a->out) && aligned16(a->out_cast);
+         aligned16(a->out) && aligned16(a->out_cast) && aligned16(a->message_basis);
 }
 inline bool vectors_aligned(const MfSimplicialBwdArgs* a) {
   return aligned16(a->q) && aligned16(a->k1) && aligned16(a->v1) && aligned16(a->k2) && aligned16(a->v2) &&
          aligned16(a->grad_out) && aligned16(a->out) && aligned16(a->dq) && aligned16(a->dk1) && aligned16(a->dv1) &&
-         aligned16(a->dk2) && aligned16(a->dv2);
+         aligned16(a->dk2) && aligned16(a->dv2) && aligned16(a->message_basis);
 }
 
 template <typename Args>
@@ -79,10 +79,11 @@ bool has_factorized_bias(const Args* a) {
 template <typename Args>
 bool wants_tcgen05(const Args* a, int* rc, const char* name) {
   *rc = MF_OK;
-  // The factorized bias is built into the tile kernels, not into the row-packed ones; the low-rank residuals run on the
-  // CUDA-core kernel.
+  // The factorized bias is built into the tile and the warp-level kernels, not into the row-packed ones; the low-rank
+  // residuals into the warp-level ones (at most 32 tokens), else they run on the CUDA-core kernel.
   const bool has_residual = a->angle_left || a->message_left;
-  const bool bias_ok = !has_residual && (!has_factorized_bias(a) || a->backend != MF_BACKEND_TCGEN05);
+  const bool bias_ok = (!has_residual || (a->backend == MF_BACKEND_AUTO && a->tokens <= kSmallTokens)) &&
+                       (!has_factorized_bias(a) || a->backend != MF_BACKEND_TCGEN05);
   // the tensor-core kernels move rows with 16-byte vector accesses; tensors that do not start on a 16-byte boundary
   // (a view into the middle of another tensor) go to the CUDA-core kernel, which loads element by element
   const bool ok = bias_ok && simplicial_sm100_supports(a->dtype, a->precision, a->tokens, a->head_dim) &&
@@ -159,6 +160,12 @@ extern "C" int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* a) {
   return wants_tcgen05(a, &rc, "mf_simplicial_bwd_backend") ? MF_BACKEND_TCGEN05 : MF_BACKEND_GENERIC;
 }
 
+extern "C" int mf_simplicial_bwd_needs_zeros(const MfSimplicialBwdArgs* a) {
+  if (!a) return 1;
+  int rc;
+  return !(wants_tcgen05(a, &rc, "mf_simplicial_bwd_needs_zeros") && uses_small_kernels(a));
+}
+
 extern "C" int mf_simplicial_row_plan(int32_t n_queries, int32_t valid_keys, int32_t plan[4]) {
   MF_CHECK_ARG(plan != nullptr, "mf_simplicial_row_plan: null output pointer");
   MF_CHECK_ARG(n_queries >= 0 && valid_keys >= 0, "mf_simplicial_row_plan: negative count");
@@ -185,7 +192,8 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
   if (!tc) return simplicial_generic_fwd(*a, s);
-  if (uses_small_kernels(a)) return simplicial_small_fwd(*a, nullptr, s);
+  if (uses_small_kernels(a))
+    return a->angle_left || a->message_left ? simplicial_small_res_fwd(*a, s) : simplicial_small_fwd(*a, nullptr, s);
   return uses_tile_kernels(a) ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
 }
 

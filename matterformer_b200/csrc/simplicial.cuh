@@ -25,10 +25,11 @@ int simplicial_sm100_bwd_layouts(const MfSimplicialBwdArgs& a, const TileLayouts
 size_t simplicial_sm100_fwd_workspace_bytes(const MfSimplicialFwdArgs& a);
 size_t simplicial_sm100_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 
-// warp-level kernels for molecules of at most 32 tokens (simplicial_small_fwd.cu, simplicial_small_bwd.cu)
+// warp-level kernels for molecules of at most 32 tokens (simplicial_small_fwd.cu, simplicial_small_res_fwd.cu, simplicial_small_bwd.cu)
 constexpr int kSmallTokens = 32;
 int simplicial_small_fwd(const MfSimplicialFwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
 int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
+int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);  // with the low-rank residuals
 
 // row-packed tcgen05 kernels (simplicial_rows_fwd.cu, simplicial_rows_bwd.cu); same problems as the kernels above
 int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);

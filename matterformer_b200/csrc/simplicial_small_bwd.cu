@@ -44,6 +44,20 @@ struct SmallBwdParams {
   float* dv_bias;
   float* dw;
   float* dgate;
+  // low-rank residuals and their gradients (RK > 0)
+  const float* al;
+  const float* ar;
+  const float* agate;
+  const float* ml;
+  const float* mr;
+  const float* basis;
+  float* dal;
+  float* dar;
+  float* dagate;
+  float* dml;
+  float* dmr;
+  float* mcoef;  // rm^-1/2 sum_jk P ml mr, from which the caller forms the gradient of basis
+  int ra, rm;
   __nv_bfloat16* dq;
   __nv_bfloat16* dk1;
   __nv_bfloat16* dv1;
@@ -56,7 +70,7 @@ struct SmallBwdParams {
 
 constexpr int kAccStride = kD + 4;  // fp32 rows of the gradient stage
 
-template <bool kBias>
+template <bool kBias, int RK = 0, int kWarps = 1>
 struct SmallBwdShared {
   __align__(128) uint8_t tile[6][kSmallTile];  // q, k1, v1, k2, v2, grad_out
   __nv_bfloat16 dq[kSmallRows][kD];
@@ -67,42 +81,16 @@ struct SmallBwdShared {
   float lse2[kSmallRows], delta[kSmallRows];
   uint32_t visible[kSmallRows];                // bit k of word j: the pair (j, k) counts
   float4 w[kBias ? 8 : 1][32];                 // bias w_jk as the fragments of the logits hold it
+  // RK > 0: rm^-1/2 dO_i . basis_r, and the residual factors of the query that each warp works on
+  float dc[RK ? kSmallRows : 1][RK ? 16 * RK : 1];
+  __align__(128) uint8_t factor[RK ? kWarps : 1][4][RK ? 2 * RankTile<RK ? RK : 1>::kTile : 16];
 };
 
 constexpr int kTq = 0, kTk1 = kSmallTile, kTv1 = 2 * kSmallTile, kTk2 = 3 * kSmallTile, kTv2 = 4 * kSmallTile, kTgo = 5 * kSmallTile;
 
-// c (16 x 8 tiles, rows j, columns k) = (X o x_i) Y^T for two key-major tiles X, Y and the row x_i
-template <int MT, int NT>
-__device__ __forceinline__ void pair_product(float (&c)[MT][NT][4], const FragBase& fb, int x, int y, const uint32_t (&row)[8]) {
-#pragma unroll
-  for (int kp = 0; kp < 2; ++kp) {
-    uint32_t b[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) load_b(b[nt], fb, y, nt, kp);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int ks = 2 * kp + k;
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        uint32_t a[4];
-        load_a(a, fb, x, mt, ks);
-        a[0] = mul_bf16x2(a[0], row[2 * ks]);
-        a[1] = mul_bf16x2(a[1], row[2 * ks]);
-        a[2] = mul_bf16x2(a[2], row[2 * ks + 1]);
-        a[3] = mul_bf16x2(a[3], row[2 * ks + 1]);
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          if (ks == 0) mma16_first(c[mt][nt], a, b[nt][2 * k], b[nt][2 * k + 1]);
-          else mma16(c[mt][nt], a, b[nt][2 * k], b[nt][2 * k + 1]);
-        }
-      }
-    }
-  }
-}
-
 // One walk; warp w takes the queries w, w + kWarps, ....  Leaves the two sums in sm.acc and all warps at a barrier.
-template <int MT, int NT, bool kHoles, bool kBias, int kWarps, bool kKeySide>
-__device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwdShared<kBias>& sm, int bh, int n,
+template <int MT, int NT, bool kHoles, bool kBias, int RK, int kWarps, bool kKeySide, typename Shared>
+__device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, Shared& sm, int bh, int n, uint32_t kmask,
                                                uint32_t qmask) {
   constexpr int KS = (NT + 1) / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
@@ -129,7 +117,12 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
     for (int t = 0; t < 8; ++t)
 #pragma unroll
       for (int e = 0; e < 4; ++e) a2[kt][t][e] = 0.f;
-  if constexpr (kBias && kKeySide) {
+  const bool bias = kBias && (RK == 0 || p.u != nullptr);
+  using Factor = RankTile<RK ? RK : 1>;
+  const uint32_t f0 = (uint32_t)__cvta_generic_to_shared(sm.factor[RK ? warp : 0][0]);
+  const Factor left{f0}, right{f0 + 2 * Factor::kTile}, mleft{f0 + 4 * Factor::kTile}, mright{f0 + 6 * Factor::kTile};
+  const float a_scale = RK ? rsqrtf((float)p.ra) : 0.f, m_scale = RK ? rsqrtf((float)p.rm) : 0.f;
+  if (bias && kKeySide) {
 #pragma unroll
     for (int f = 0; f < 8; ++f) sm.dw[warp][f][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -143,8 +136,39 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
       load_row_pairs(qf, qt, i, lane);
       pair_product<MT, NT>(s, fb, kTk1, kTk2, qf);
     }
+    float ga = 0.f;  // gate and scale of the angle residual
+    if constexpr (RK > 0) {
+      const size_t qi = (size_t)bh * p.N + i;
+      __syncwarp();
+      if (p.al) {
+        stage_factor(left, p.al + qi * p.N * p.ra, n, p.ra, kmask, nullptr, lane);
+        stage_factor(right, p.ar + qi * p.N * p.ra, n, p.ra, kmask, nullptr, lane);
+      }
+      if (p.ml) {  // K side: only ML_r (dO_i . basis_r) enters dP
+        stage_factor(mleft, p.ml + qi * p.N * p.rm, n, p.rm, kmask, kKeySide ? sm.dc[i] : nullptr, lane);
+        stage_factor(mright, p.mr + qi * p.N * p.rm, n, p.rm, kmask, nullptr, lane);
+      }
+      __syncwarp();
+      if (p.al) {
+        ga = p.agate[qi] * a_scale;
+        float ad[MT][NT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ad[mt][nt][e] = 0.f;
+        add_rank_product<MT, NT>(ad, left, right, lane);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[mt][nt][e] = fmaf(ga, ad[mt][nt][e], s[mt][nt][e]);
+      }
+    }
     float ul = 0.f, vl = 0.f, g = 0.f;  // bias: u_i,lane, v_i,lane
-    if constexpr (kBias) {
+    if (bias) {
       const size_t at = ((size_t)bh * p.N + i) * p.N + lane;
       ul = lane < n ? p.u[at] : 0.f;
       vl = lane < n ? p.v_bias[at] : 0.f;
@@ -195,6 +219,9 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
         uint32_t gf[8];
         load_row_pairs(gf, qt + kTgo, i, lane);
         pair_product<MT, NT>(dp, fb, kTv1, kTv2, gf);
+        if constexpr (RK > 0) {
+          if (p.ml) add_rank_product<MT, NT>(dp, mleft, mright, lane);
+        }
       }
       const float nd = -sm.delta[i];
 #pragma unroll
@@ -207,7 +234,7 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
             const float2 x = mul2(make_float2(s[mt][nt][2 * hh], s[mt][nt][2 * hh + 1]), d);
             s[mt][nt][2 * hh] = x.x, s[mt][nt][2 * hh + 1] = x.y;
           }
-      if constexpr (kBias) {
+      if (bias) {
         float rs[MT][2], cs[8], wsum = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) cs[e] = 0.f;
@@ -274,6 +301,80 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
         at[kt][mt][2] = transpose8x8(pk[mt][2 * kt][1]);
         at[kt][mt][3] = 2 * kt + 1 < NT ? transpose8x8(pk[mt][2 * kt + 1][1]) : 0u;
       }
+    if constexpr (RK > 0) {
+      // K side: X = dS R_i and dS^T L_i give dL, dR and the gate; V side: T = P MR_i and P^T ML_i give dML, dMR and the
+      // coefficients of the basis
+      const Factor &fl = kKeySide ? left : mleft, &fr = kKeySide ? right : mright;
+      const int rank = kKeySide ? p.ra : p.rm;
+      const size_t qi = (size_t)bh * p.N + i;
+      float *gl = kKeySide ? p.dal : p.dml, *gr = kKeySide ? p.dar : p.dmr, gate_sum = 0.f;
+      if (kKeySide ? p.al != nullptr : p.ml != nullptr) {
+#pragma unroll
+        for (int rk = 0; rk < RK; ++rk) {
+          float t[2 * MT][4], lo = 0.f, hi = 0.f;
+          rank_sums<MT>(t, fr, pk, rk, lane);
+          float c[KS][2][4];
+#pragma unroll
+          for (int kt = 0; kt < KS; ++kt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[kt][0][e] = c[kt][1][e] = 0.f;
+          const int ra = 16 * rk + row8, rb = ra + 8;
+          const float sa = kKeySide ? ga : sm.dc[i][ra], sb = kKeySide ? ga : sm.dc[i][rb];
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            uint32_t h[4], l[4];
+            fl.load_t(h, 0, rk, mt, lane);
+            fl.load_t(l, 1, rk, mt, lane);
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              const float* x = t[2 * mt + jj];
+              lo = fmaf(x[0], bf16_lo(h[2 * jj]) + bf16_lo(l[2 * jj]), fmaf(x[1], bf16_hi(h[2 * jj]) + bf16_hi(l[2 * jj]), lo));
+              hi = fmaf(x[2], bf16_lo(h[2 * jj + 1]) + bf16_lo(l[2 * jj + 1]),
+                        fmaf(x[3], bf16_hi(h[2 * jj + 1]) + bf16_hi(l[2 * jj + 1]), hi));
+              if (gl) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const int j = (2 * mt + jj) * 8 + 2 * quad + (e & 1), r = e < 2 ? ra : rb;
+                  if (j < p.N && r < rank) gl[(qi * p.N + j) * rank + r] = (e < 2 ? sa : sb) * x[e];
+                }
+              }
+            }
+#pragma unroll
+            for (int kt = 0; kt < KS; ++kt) {
+              mma16(c[kt][0], at[kt][mt], h[0], h[2]);
+              mma16(c[kt][0], at[kt][mt], l[0], l[2]);
+              mma16(c[kt][1], at[kt][mt], h[1], h[3]);
+              mma16(c[kt][1], at[kt][mt], l[1], l[3]);
+            }
+          }
+          if (gr) {
+#pragma unroll
+            for (int kt = 0; kt < KS; ++kt)
+#pragma unroll
+              for (int t8 = 0; t8 < 2; ++t8)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const int k = kt * 16 + (e >> 1) * 8 + row8, r = 16 * rk + 8 * t8 + 2 * quad + (e & 1);
+                  if (k < p.N && r < rank) gr[(qi * p.N + k) * rank + r] = (kKeySide ? ga : sm.dc[i][r]) * c[kt][t8][e];
+                }
+          }
+          if (kKeySide) {
+            gate_sum += lo + hi;
+          } else {
+            quad_reduce(lo);
+            quad_reduce(hi);
+            if (p.mcoef && quad == 0) {
+              if (ra < rank) p.mcoef[qi * rank + ra] = m_scale * lo;
+              if (rb < rank) p.mcoef[qi * rank + rb] = m_scale * hi;
+            }
+          }
+        }
+        if (kKeySide && p.dagate) {
+          gate_sum = warp_sum(gate_sum);
+          if (lane == 0) p.dagate[qi] = a_scale * gate_sum;
+        }
+      }
+    }
     uint32_t xd[8];
     load_row_dup(xd, qt + xr, i, lane);
     float dq[8];
@@ -328,7 +429,7 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
     }
   }
 
-  if constexpr (kBias && kKeySide) {
+  if (bias && kKeySide) {
     __syncthreads();
     if (p.dw) {
       float* dw = p.dw + (size_t)bh * p.N * p.N;
@@ -372,8 +473,8 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, SmallBwd
 }
 
 // Both walks and the gradient rows; a lane writes eight channels.
-template <int MT, int NT, bool kHoles, bool kBias, int kWarps>
-__device__ __forceinline__ void small_bwd_walks(const SmallBwdParams& p, SmallBwdShared<kBias>& sm, int b, int h, int n,
+template <int MT, int NT, bool kHoles, bool kBias, int RK, int kWarps, typename Shared>
+__device__ __forceinline__ void small_bwd_walks(const SmallBwdParams& p, Shared& sm, int b, int h, int n,
                                                 uint32_t kmask, uint32_t qmask) {
   const int bh = b * p.H + h;
   auto store_rows = [&](__nv_bfloat16* g1, __nv_bfloat16* g2) {
@@ -387,17 +488,19 @@ __device__ __forceinline__ void small_bwd_walks(const SmallBwdParams& p, SmallBw
       *reinterpret_cast<uint4*>((t ? g2 : g1) + p.in.at(b, h, r) + 8 * c) = v;
     }
   };
-  small_bwd_side<MT, NT, kHoles, kBias, kWarps, false>(p, sm, bh, n, qmask);
+  small_bwd_side<MT, NT, kHoles, kBias, RK, kWarps, false>(p, sm, bh, n, kmask, qmask);
   store_rows(p.dv1, p.dv2);
   __syncthreads();
-  small_bwd_side<MT, NT, kHoles, kBias, kWarps, true>(p, sm, bh, n, qmask);
+  small_bwd_side<MT, NT, kHoles, kBias, RK, kWarps, true>(p, sm, bh, n, kmask, qmask);
   store_rows(p.dk1, p.dk2);
 }
 
-template <bool kBias, int kWarps>
+template <bool kBias, int RK, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_kernel(const __grid_constant__ SmallBwdParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
-  SmallBwdShared<kBias>& sm = *reinterpret_cast<SmallBwdShared<kBias>*>(smem);
+  using Shared = SmallBwdShared<kBias, RK, kWarps>;
+  Shared& sm = *reinterpret_cast<Shared*>(smem);
+  const bool bias = kBias && (RK == 0 || p.u != nullptr);
   constexpr int kThreads = 32 * kWarps;
   const int tid = threadIdx.x, lane = tid & 31;
   const int N = p.N, bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
@@ -408,7 +511,7 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
     const __nv_bfloat16* src[6] = {p.q, p.k1, p.v1, p.k2, p.v2, p.grad_out};
     const uint32_t t0 = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
     // a hole in a mask takes the full-size variant, which reads all rows
-    const int key_rows = (p.pair_valid || (kmask & (kmask + 1)) != 0u) ? kSmallRows : (n + 15) & ~15;
+    const int key_rows = (RK > 0 || p.pair_valid || (kmask & (kmask + 1)) != 0u) ? kSmallRows : (n + 15) & ~15;
 #pragma unroll
     for (int t = 0; t < 6; ++t) {
       const bool query = t == 0 || t == 5;
@@ -432,7 +535,11 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
     if (lane == 0) sm.visible[j] = word;
   }
   for (int idx = tid; idx < kSmallRows * kD / 8; idx += kThreads) reinterpret_cast<float4*>(sm.dq)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
-  if constexpr (kBias) {
+  if constexpr (RK > 0) {
+    for (int idx = tid; idx < (int)sizeof(sm.factor) / 16; idx += kThreads)
+      reinterpret_cast<float4*>(sm.factor)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (bias) {
     for (int idx = tid; idx < 8 * 32; idx += kThreads) {
       const int f = idx >> 5, ln = idx & 31, j = (f >> 2) * 16 + (ln >> 2), k = (f & 3) * 8 + 2 * (ln & 3);
       const float* w = p.w + (size_t)bh * N * N;
@@ -474,11 +581,32 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
     }
     __syncthreads();
   }
-  if (n > 0) {
-    if (hole) small_bwd_walks<2, 4, true, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
-    else if (n <= 16) small_bwd_walks<1, 2, false, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
-    else if (n <= 24) small_bwd_walks<2, 3, false, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
-    else small_bwd_walks<2, 4, false, kBias, kWarps>(p, sm, b, h, n, kmask, qmask);
+  if constexpr (RK > 0) {
+    if (n > 0 && p.ml) {
+      const uint32_t go = (uint32_t)__cvta_generic_to_shared(sm.tile[5]);
+      const float m_scale = rsqrtf((float)p.rm);
+      for (int idx = tid; idx < nq * p.rm; idx += kThreads) {
+        const int i = idx / p.rm, r = idx - i * p.rm;
+        const float4* bs = reinterpret_cast<const float4*>(p.basis + ((size_t)h * p.rm + r) * kD);
+        float d = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint4 x;
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(row_chunk(go, i, c)));
+          const float4 y = bs[2 * c], z = bs[2 * c + 1];
+          d = fmaf(bf16_lo(x.x), y.x, fmaf(bf16_hi(x.x), y.y, fmaf(bf16_lo(x.y), y.z, fmaf(bf16_hi(x.y), y.w, d))));
+          d = fmaf(bf16_lo(x.z), z.x, fmaf(bf16_hi(x.z), z.y, fmaf(bf16_lo(x.w), z.z, fmaf(bf16_hi(x.w), z.w, d))));
+        }
+        sm.dc[i][r] = m_scale * d;
+      }
+      __syncthreads();
+    }
+    if (n > 0) small_bwd_walks<2, 4, true, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
+  } else if (n > 0) {
+    if (hole) small_bwd_walks<2, 4, true, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else if (n <= 16) small_bwd_walks<1, 2, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else if (n <= 24) small_bwd_walks<2, 3, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else small_bwd_walks<2, 4, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
   }
   // the rows of dq, and everything when the molecule has no valid query or key
   __nv_bfloat16* dst[5] = {p.dq, p.dk1, p.dv1, p.dk2, p.dv2};
@@ -487,7 +615,18 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
     *reinterpret_cast<uint4*>(dst[t] + p.in.at(b, h, r) + 8 * c) =
         t == 0 ? *reinterpret_cast<const uint4*>(&sm.dq[r][8 * c]) : make_uint4(0u, 0u, 0u, 0u);
   }
-  if constexpr (kBias) {
+  if constexpr (RK > 0) {  // residual gradients of queries that no warp took
+    float* rows[6] = {p.dal, p.dar, p.dml, p.dmr, p.dagate, p.mcoef};
+    const int len[6] = {N * p.ra, N * p.ra, N * p.rm, N * p.rm, 1, p.rm};
+    for (int i = tid >> 5; i < N; i += kWarps)
+      if (i >= nq || !((qmask >> i) & 1u)) {
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+          if (rows[t])
+            for (int x = lane; x < len[t]; x += 32) rows[t][((size_t)bh * N + i) * len[t] + x] = 0.f;
+      }
+  }
+  if (bias) {
     if (n == 0 && p.dw)
       for (int idx = tid; idx < N * N; idx += kThreads) p.dw[(size_t)bh * N * N + idx] = 0.f;
     // rows of du, dv and dgate that no query wrote
@@ -520,6 +659,11 @@ int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layout
   p.pair_valid = a.pair_valid;
   p.u = a.u, p.v_bias = a.v_bias, p.w = a.w, p.gate = a.gate;
   p.du = a.du, p.dv_bias = a.dv_bias, p.dw = a.dw, p.dgate = a.dgate;
+  p.al = a.angle_left, p.ar = a.angle_right, p.agate = a.angle_gate;
+  p.ml = a.message_left, p.mr = a.message_right, p.basis = a.message_basis;
+  p.dal = a.dangle_left, p.dar = a.dangle_right, p.dagate = a.dangle_gate;
+  p.dml = a.dmessage_left, p.dmr = a.dmessage_right, p.mcoef = a.message_coeff;
+  p.ra = a.angle_left ? a.angle_rank : 1, p.rm = a.message_left ? a.message_rank : 1;
   p.dq = static_cast<__nv_bfloat16*>(a.dq);
   p.dk1 = static_cast<__nv_bfloat16*>(a.dk1);
   p.dv1 = static_cast<__nv_bfloat16*>(a.dv1);
@@ -535,18 +679,21 @@ int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layout
   const int warps = bh >= 1024 ? 2 : 4;
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
   cudaError_t e = cudaSuccess;
-#define MF_LAUNCH(BIAS, S)                                                                                             \
+#define MF_LAUNCH(BIAS, RK, S)                                                                                             \
   do {                                                                                                                 \
-    constexpr int bytes = (int)sizeof(SmallBwdShared<BIAS>);                                                        \
-    e = cudaFuncSetAttribute(simplicial_small_bwd_kernel<BIAS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
-    if (e == cudaSuccess) simplicial_small_bwd_kernel<BIAS, S><<<bh, 32 * S, bytes, stream>>>(p);                      \
+    constexpr int bytes = (int)sizeof(SmallBwdShared<BIAS, RK, S>);                                                        \
+    e = cudaFuncSetAttribute(simplicial_small_bwd_kernel<BIAS, RK, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
+    if (e == cudaSuccess) simplicial_small_bwd_kernel<BIAS, RK, S><<<bh, 32 * S, bytes, stream>>>(p);                      \
   } while (0)
-  if (a.u) {
-    if (warps == 2) MF_LAUNCH(true, 2);
-    else MF_LAUNCH(true, 4);
+  if (a.angle_left || a.message_left) {
+    if (max(p.ra, p.rm) <= 16) MF_LAUNCH(true, 1, 4);
+    else MF_LAUNCH(true, 2, 4);
+  } else if (a.u) {
+    if (warps == 2) MF_LAUNCH(true, 0, 2);
+    else MF_LAUNCH(true, 0, 4);
   } else {
-    if (warps == 2) MF_LAUNCH(false, 2);
-    else MF_LAUNCH(false, 4);
+    if (warps == 2) MF_LAUNCH(false, 0, 2);
+    else MF_LAUNCH(false, 0, 4);
   }
 #undef MF_LAUNCH
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_small_bwd_kernel)");

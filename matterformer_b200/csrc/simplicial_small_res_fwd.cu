@@ -1,0 +1,289 @@
+// 2-simplicial attention, forward, for molecules of at most 32 tokens in bf16 with the low-rank residuals
+// (angle: logits += agate_i ra^-1/2 L_i R_i^T, message: out_i += sum_r c_ir basis_r; with or without the factorized bias).
+//
+// The residual factors belong to one query, L_i and R_i are (keys x rank): for a fixed query both residuals are matrix
+// products like the attention itself, so this kernel walks query by query (the kernel without residuals walks over first
+// keys, where the factors would be different for every row).  A warp takes a query: 32 x 32 logits in registers, factors
+// staged in its own shared memory as hi + lo bf16 (see RankTile), exact maximum, P as the B operand of W^T = V2^T P^T and
+// of T^T = MR^T P^T, c_ir = sum_j ML_jr T_jr.
+#include "common.cuh"
+#include "simplicial.cuh"
+#include "simplicial_warp.cuh"
+
+namespace mf {
+namespace {
+
+struct ResFwdParams {
+  const __nv_bfloat16* q;
+  const __nv_bfloat16* k1;
+  const __nv_bfloat16* v1;
+  const __nv_bfloat16* k2;
+  const __nv_bfloat16* v2;
+  const uint8_t* query_valid;
+  const uint8_t* key_valid;
+  const uint8_t* pair_valid;
+  const float* u;
+  const float* v_bias;
+  const float* w;
+  const float* gate;
+  const float* al;
+  const float* ar;
+  const float* agate;
+  const float* ml;
+  const float* mr;
+  const float* basis;
+  int ra, rm;
+  float* out;
+  float* lse;
+  __nv_bfloat16* out_cast;
+  int H, N;
+};
+
+constexpr int kResWarps = 4;
+
+template <int RK>
+struct ResFwdShared {
+  __align__(128) uint8_t tile[5][kSmallTile];                            // q, k1, v1, k2, v2
+  __align__(128) uint8_t factor[kResWarps][4][2 * RankTile<RK>::kTile];  // L, R, ML, MR of the warp's query
+  uint32_t visible[kSmallRows];
+};
+
+template <int RK>
+__global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_kernel(const __grid_constant__ ResFwdParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  ResFwdShared<RK>& sm = *reinterpret_cast<ResFwdShared<RK>*>(smem);
+  constexpr int kThreads = 32 * kResWarps, MT = 2, NT = 4;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = lane & 3, row8 = lane >> 2;
+  const int N = p.N, bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
+  const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
+  const uint32_t qmask = __ballot_sync(0xffffffffu, lane < N && p.query_valid[(size_t)b * N + min(lane, N - 1)] > 0);
+  const int n = 32 - __clz(kmask);
+  const RowLayout rows{(long long)p.H * N * kD, (long long)N * kD, kD};
+  {
+    const __nv_bfloat16* src[5] = {p.q, p.k1, p.v1, p.k2, p.v2};
+    const uint32_t t0 = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
+#pragma unroll
+    for (int t = 0; t < 5; ++t)
+      for (int idx = tid; idx < 8 * kSmallRows; idx += kThreads) {
+        const int r = idx >> 3, c = idx & 7;
+        const bool ok = ((t == 0 ? qmask : kmask) >> r) & 1u;
+        cp_async16(row_chunk(t0 + t * kSmallTile, r, c), src[t] + rows.at(b, h, ok ? r : 0) + c * 8, ok);
+      }
+    cp_async_commit();
+  }
+  for (int idx = tid; idx < (int)sizeof(sm.factor) / 16; idx += kThreads) reinterpret_cast<float4*>(sm.factor)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j = warp; j < kSmallRows; j += kResWarps) {
+    uint32_t word = (j < N && ((kmask >> j) & 1u)) ? kmask : 0u;
+    if (p.pair_valid && word != 0u)
+      word &= __ballot_sync(0xffffffffu, lane < N && p.pair_valid[((size_t)b * N + j) * N + min(lane, N - 1)] > 0);
+    if (lane == 0) sm.visible[j] = word;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+
+  const uint32_t qt = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
+  const FragBase fb(qt, lane);
+  constexpr int kTk1 = kSmallTile, kTv1 = 2 * kSmallTile, kTk2 = 3 * kSmallTile, kTv2 = 4 * kSmallTile;
+  const uint32_t f0 = (uint32_t)__cvta_generic_to_shared(sm.factor[warp][0]);
+  const RankTile<RK> left{f0}, right{f0 + 2 * RankTile<RK>::kTile}, mleft{f0 + 4 * RankTile<RK>::kTile}, mright{f0 + 6 * RankTile<RK>::kTile};
+  uint32_t vis[MT][2];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) vis[mt][hh] = sm.visible[mt * 16 + hh * 8 + row8] >> (2 * quad);
+
+  for (int i = warp; i < N; i += kResWarps) {
+    const size_t qi = (size_t)bh * N + i;
+    bool have = ((qmask >> i) & 1u) && n > 0;
+    float l = 0.f, m = -INFINITY, o[8];
+    float coef[2 * RK];  // message coefficients of ranks 8 e + row8
+    if (have) {
+      __syncwarp();
+      if (p.al) {
+        stage_factor(left, p.al + qi * N * p.ra, n, p.ra, kmask, nullptr, lane);
+        stage_factor(right, p.ar + qi * N * p.ra, n, p.ra, kmask, nullptr, lane);
+      }
+      if (p.ml) {
+        stage_factor(mleft, p.ml + qi * N * p.rm, n, p.rm, kmask, nullptr, lane);
+        stage_factor(mright, p.mr + qi * N * p.rm, n, p.rm, kmask, nullptr, lane);
+      }
+      __syncwarp();
+      float s[MT][NT][4];
+      {
+        uint32_t qf[8];
+        load_row_pairs(qf, qt, i, lane);
+        pair_product<MT, NT>(s, fb, kTk1, kTk2, qf);
+      }
+      if (p.u) {
+        const size_t row = qi * N + lane;
+        const float ul = lane < n ? p.u[row] : 0.f, vl = lane < n ? p.v_bias[row] : 0.f, g = p.gate[qi];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int j = mt * 16 + (e >> 1) * 8 + row8, k = nt * 8 + 2 * quad + (e & 1);
+              const float uv = __shfl_sync(0xffffffffu, ul, j) + __shfl_sync(0xffffffffu, vl, k);
+              const float w = (j < n && k < n) ? p.w[((size_t)bh * N + j) * N + k] : 0.f;
+              s[mt][nt][e] = fmaf(g, uv + w, s[mt][nt][e]);
+            }
+      }
+      if (p.al) {
+        float ad[MT][NT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ad[mt][nt][e] = 0.f;
+        add_rank_product<MT, NT, RK>(ad, left, right, lane);
+        const float g = p.agate[qi] * rsqrtf((float)p.ra);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[mt][nt][e] = fmaf(g, ad[mt][nt][e], s[mt][nt][e]);
+      }
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (!((vis[mt][e >> 1] >> (nt * 8 + (e & 1))) & 1u)) s[mt][nt][e] = -INFINITY;
+            m = fmaxf(m, s[mt][nt][e]);
+          }
+      m = warp_max(m);
+      have = m > -INFINITY;
+      const float m2 = have ? m * kLog2e : 0.f;
+      uint32_t pk[MT][NT][2];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const float a = fast_exp2(fmaf(s[mt][nt][2 * hh], kLog2e, -m2)), c = fast_exp2(fmaf(s[mt][nt][2 * hh + 1], kLog2e, -m2));
+            l += a + c;
+            pk[mt][nt][hh] = pack2_bf16(a, c);
+          }
+      l = warp_sum(l);
+#pragma unroll
+      for (int dt = 0; dt < 4; ++dt) {
+        float w[2 * MT][4];
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          uint32_t a[4];
+          load_t(a, fb, kTv2, dt, ks);
+#pragma unroll
+          for (int jt = 0; jt < 2 * MT; ++jt) {
+            const uint32_t b0 = pk[jt >> 1][2 * ks][jt & 1], b1 = pk[jt >> 1][2 * ks + 1][jt & 1];
+            if (ks == 0) mma16_first(w[jt], a, b0, b1);
+            else mma16(w[jt], a, b0, b1);
+          }
+        }
+        float lo = 0.f, hi = 0.f;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          uint32_t v[4];
+          load_t(v, fb, kTv1, dt, mt);
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj) {
+            const float* c = w[2 * mt + jj];
+            lo = fmaf(c[0], bf16_lo(v[2 * jj]), fmaf(c[1], bf16_hi(v[2 * jj]), lo));
+            hi = fmaf(c[2], bf16_lo(v[2 * jj + 1]), fmaf(c[3], bf16_hi(v[2 * jj + 1]), hi));
+          }
+        }
+        o[2 * dt] = lo, o[2 * dt + 1] = hi;
+      }
+      quad_sum8(o, lane);
+      if (p.ml) {
+        // T^T (ranks x j) = MR^T P^T, c_r = sum_j ML_jr T_jr
+#pragma unroll
+        for (int rk = 0; rk < RK; ++rk) {
+          float t[2 * MT][4], lo = 0.f, hi = 0.f;
+          rank_sums<MT, NT, RK>(t, mright, pk, rk, lane);
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            uint32_t mh[4], mo[4];
+            mleft.load_t(mh, 0, rk, mt, lane);
+            mleft.load_t(mo, 1, rk, mt, lane);
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              const float* c = t[2 * mt + jj];
+              const uint32_t a0 = mh[2 * jj], a1 = mo[2 * jj], b0 = mh[2 * jj + 1], b1 = mo[2 * jj + 1];
+              lo = fmaf(c[0], bf16_lo(a0) + bf16_lo(a1), fmaf(c[1], bf16_hi(a0) + bf16_hi(a1), lo));
+              hi = fmaf(c[2], bf16_lo(b0) + bf16_lo(b1), fmaf(c[3], bf16_hi(b0) + bf16_hi(b1), hi));
+            }
+          }
+#pragma unroll
+          for (int x = 1; x < 4; x <<= 1) {
+            lo += __shfl_xor_sync(0xffffffffu, lo, x);
+            hi += __shfl_xor_sync(0xffffffffu, hi, x);
+          }
+          coef[2 * rk] = lo, coef[2 * rk + 1] = hi;
+        }
+      }
+    }
+    const int d0 = (4 * (quad & 1) + 2 * (quad >> 1)) * 8 + row8;  // the lane's two channels: d0 and d0 + 8
+    float x0 = have ? o[0] : 0.f, x1 = have ? o[1] : 0.f;
+    if (p.ml && have) {
+      const float scale = rsqrtf((float)p.rm);
+#pragma unroll
+      for (int e = 0; e < 2 * RK; ++e)
+#pragma unroll
+        for (int r8 = 0; r8 < 8; ++r8) {
+          const float c = __shfl_sync(0xffffffffu, coef[e], 4 * r8) * scale;
+          const int r = 8 * e + r8;
+          if (r < p.rm) {
+            const float* bs = p.basis + ((size_t)h * p.rm + r) * kD + d0;
+            x0 = fmaf(c, bs[0], x0);
+            x1 = fmaf(c, bs[8], x1);
+          }
+        }
+    }
+    const float inv = have ? 1.f / l : 0.f;
+    x0 *= inv, x1 *= inv;
+    float* out = p.out + qi * kD + d0;
+    out[0] = x0, out[8] = x1;
+    if (p.out_cast) {
+      __nv_bfloat16* oc = p.out_cast + qi * kD + d0;
+      oc[0] = __float2bfloat16_rn(x0), oc[8] = __float2bfloat16_rn(x1);
+    }
+    if (lane == 0) p.lse[qi] = have ? m + logf(l) : 0.f;
+  }
+}
+
+}  // namespace
+
+int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
+  ResFwdParams p{};
+  p.q = static_cast<const __nv_bfloat16*>(a.q);
+  p.k1 = static_cast<const __nv_bfloat16*>(a.k1);
+  p.v1 = static_cast<const __nv_bfloat16*>(a.v1);
+  p.k2 = static_cast<const __nv_bfloat16*>(a.k2);
+  p.v2 = static_cast<const __nv_bfloat16*>(a.v2);
+  p.query_valid = a.query_valid, p.key_valid = a.pair_key_valid, p.pair_valid = a.pair_valid;
+  p.u = a.u, p.v_bias = a.v_bias, p.w = a.w, p.gate = a.gate;
+  p.al = a.angle_left, p.ar = a.angle_right, p.agate = a.angle_gate;
+  p.ml = a.message_left, p.mr = a.message_right, p.basis = a.message_basis;
+  p.ra = a.angle_left ? a.angle_rank : 1, p.rm = a.message_left ? a.message_rank : 1;
+  p.out = a.out, p.lse = a.lse, p.out_cast = static_cast<__nv_bfloat16*>(a.out_cast);
+  p.H = a.heads, p.N = a.tokens;
+  auto launch = [&](auto kernel, int bytes) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) kernel<<<a.batch * a.heads, 32 * kResWarps, bytes, stream>>>(p);
+    return e;
+  };
+  profile_mark(MF_PROFILE_SIMPLICIAL_FWD, true, stream);
+  const cudaError_t e = max(p.ra, p.rm) <= 16 ? launch(simplicial_small_res_fwd_kernel<1>, (int)sizeof(ResFwdShared<1>))
+                                              : launch(simplicial_small_res_fwd_kernel<2>, (int)sizeof(ResFwdShared<2>));
+  if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_small_res_fwd_kernel)");
+  profile_mark(MF_PROFILE_SIMPLICIAL_FWD, false, stream);
+  MF_CHECK_LAUNCH("simplicial_small_res_fwd_kernel");
+  return MF_OK;
+}
+
+}  // namespace mf

@@ -116,6 +116,10 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return r;
 }
 
+__device__ __forceinline__ void quad_reduce(float& v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+}
 // Sums of the eight values over the four lanes of a quad; every lane keeps two of them: v[0], v[1] = values e0, e0 + 1
 // with e0 = 4 (lane & 1) + 2 ((lane >> 1) & 1).
 __device__ __forceinline__ void quad_sum8(float (&v)[8], int lane) {
@@ -130,6 +134,149 @@ __device__ __forceinline__ void quad_sum8(float (&v)[8], int lane) {
   for (int e = 0; e < 2; ++e) {
     const float keep = upper ? t[2 + e] : t[e], give = upper ? t[e] : t[2 + e];
     v[e] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+  }
+}
+
+// c (16 x 8 tiles, rows j, columns k) = (X o x_i) Y^T for two key-major tiles X, Y and the row x_i
+template <int MT, int NT>
+__device__ __forceinline__ void pair_product(float (&c)[MT][NT][4], const FragBase& fb, int x, int y, const uint32_t (&row)[8]) {
+#pragma unroll
+  for (int kp = 0; kp < 2; ++kp) {
+    uint32_t b[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) load_b(b[nt], fb, y, nt, kp);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int ks = 2 * kp + k;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        uint32_t a[4];
+        load_a(a, fb, x, mt, ks);
+        a[0] = mul_bf16x2(a[0], row[2 * ks]);
+        a[1] = mul_bf16x2(a[1], row[2 * ks]);
+        a[2] = mul_bf16x2(a[2], row[2 * ks + 1]);
+        a[3] = mul_bf16x2(a[3], row[2 * ks + 1]);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          if (ks == 0) mma16_first(c[mt][nt], a, b[nt][2 * k], b[nt][2 * k + 1]);
+          else mma16(c[mt][nt], a, b[nt][2 * k], b[nt][2 * k + 1]);
+        }
+      }
+    }
+  }
+}
+
+// ---- low-rank residuals (simplicial_small_res_fwd.cu, simplicial_small_bwd.cu) ------------------------------------------
+// For one query i, angle logits L_i R_i^T and message sums are products over the rank as well.  The fp32 factors of a query,
+// (n x rank) each, are staged in shared memory as two bf16 tiles, x = hi + lo, and a product is hi hi + hi lo + lo hi: the
+// dropped lo lo term is 2^-16 of it.  Rows of RK x 16 ranks, zero beyond the rank and beyond the last key.
+template <int RK>
+struct RankTile {
+  static constexpr int kRow = RK * 32;                // bytes
+  static constexpr int kTile = kSmallRows * kRow;     // one of hi / lo
+  uint32_t base;                                      // hi at base, lo behind it
+
+  // chunks of 16 bytes, swizzled so that eight consecutive rows fall into different banks
+  __device__ __forceinline__ uint32_t at(int row, int chunk) const {
+    return base + row * kRow + ((chunk ^ (RK == 1 ? (row >> 2) & 1 : (row >> 1) & 3)) << 4);
+  }
+  // A operand over ranks (rows 16*mt x ranks 16*rk), B operand over ranks (rows 16*np, +8: two row tiles at once)
+  __device__ __forceinline__ void load_a(uint32_t (&r)[4], int lo, int mt, int rk, int lane) const {
+    ldmatrix_x4(r, at(mt * 16 + (lane & 15), 2 * rk + (lane >> 4)) + lo * kTile);
+  }
+  __device__ __forceinline__ void load_b2(uint32_t (&r)[4], int lo, int np, int rk, int lane) const {
+    ldmatrix_x4(r, at(np * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * rk + ((lane >> 3) & 1)) + lo * kTile);
+  }
+  // Transposed: ranks 16*rk as rows x tile rows 16*js as columns (A operand over the tile's rows); r[0], r[2] / r[1], r[3]
+  // are the B operands (tile rows 16*js, ranks 16*rk / 16*rk + 8)
+  __device__ __forceinline__ void load_t(uint32_t (&r)[4], int lo, int rk, int js, int lane) const {
+    ldmatrix_x4_trans(r, at(js * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * rk + ((lane >> 3) & 1)) + lo * kTile);
+  }
+};
+
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
+  hi = pack2_bf16(x, y);
+  lo = pack2_bf16(x - bf16_lo(hi), y - bf16_hi(hi));
+}
+
+__device__ __forceinline__ void store_shared64(uint32_t addr, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+
+// Stages rows [0, n) of one query's factor (row-major, `rank` floats each) by one warp, column r times rank_scale[r] when
+// given; rows of hidden keys become zeros.
+template <int RK>
+__device__ __forceinline__ void stage_factor(const RankTile<RK>& t, const float* __restrict__ src, int n, int rank, uint32_t kmask,
+                                             const float* rank_scale, int lane) {
+  if ((rank & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    const int q = rank >> 2, total = n * q;
+    for (int idx = lane; idx < total; idx += 32) {
+      const int row = idx / q, c = idx - row * q;
+      float4 x = reinterpret_cast<const float4*>(src)[idx];
+      if (!((kmask >> row) & 1u)) x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (rank_scale) x.x *= rank_scale[4 * c], x.y *= rank_scale[4 * c + 1], x.z *= rank_scale[4 * c + 2], x.w *= rank_scale[4 * c + 3];
+      uint32_t h0, l0, h1, l1;
+      split_bf16(x.x, x.y, h0, l0);
+      split_bf16(x.z, x.w, h1, l1);
+      const uint32_t a = t.at(row, c >> 1) + (c & 1) * 8;
+      store_shared64(a, h0, h1);
+      store_shared64(a + RankTile<RK>::kTile, l0, l1);
+    }
+  } else {
+    for (int idx = lane; idx < n * rank; idx += 32) {
+      const int row = idx / rank, r = idx - row * rank;
+      const float x = ((kmask >> row) & 1u) ? src[idx] * (rank_scale ? rank_scale[r] : 1.f) : 0.f;
+      uint32_t h, l;
+      split_bf16(x, 0.f, h, l);
+      const uint32_t a = t.at(row, r >> 3) + (r & 7) * 2;
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)h) : "memory");
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + RankTile<RK>::kTile), "h"((uint16_t)l) : "memory");
+    }
+  }
+}
+
+// c[mt][nt] += L_i R_i^T over the rank
+template <int MT, int NT, int RK>
+__device__ __forceinline__ void add_rank_product(float (&c)[MT][NT][4], const RankTile<RK>& left, const RankTile<RK>& right, int lane) {
+#pragma unroll
+  for (int rk = 0; rk < RK; ++rk)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      uint32_t ah[4], al[4];
+      left.load_a(ah, 0, mt, rk, lane);
+      left.load_a(al, 1, mt, rk, lane);
+#pragma unroll
+      for (int np = 0; np < (NT + 1) / 2; ++np) {
+        uint32_t bh[4], bl[4];
+        right.load_b2(bh, 0, np, rk, lane);
+        right.load_b2(bl, 1, np, rk, lane);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (2 * np + t < NT) {
+            float(&d)[4] = c[mt][2 * np + t < NT ? 2 * np + t : 0];
+            mma16(d, ah, bh[2 * t], bh[2 * t + 1]);
+            mma16(d, ah, bl[2 * t], bl[2 * t + 1]);
+            mma16(d, al, bh[2 * t], bh[2 * t + 1]);
+          }
+      }
+    }
+}
+
+// t (ranks 16*rk x j, as W^T) = F^T P^T for a factor F (keys x rank) and P (or dS) as pk[mt][nt][hh] holds it
+template <int MT, int NK, int RK>
+__device__ __forceinline__ void rank_sums(float (&t)[2 * MT][4], const RankTile<RK>& f, const uint32_t (&pk)[MT][NK][2], int rk, int lane) {
+#pragma unroll
+  for (int ks = 0; ks < NK / 2; ++ks) {
+    uint32_t h[4], l[4];
+    f.load_t(h, 0, rk, ks, lane);
+    f.load_t(l, 1, rk, ks, lane);
+#pragma unroll
+    for (int jt = 0; jt < 2 * MT; ++jt) {
+      const uint32_t b0 = pk[jt >> 1][2 * ks][jt & 1], b1 = pk[jt >> 1][2 * ks + 1][jt & 1];
+      if (ks == 0) mma16_first(t[jt], h, b0, b1);
+      else mma16(t[jt], h, b0, b1);
+      mma16(t[jt], l, b0, b1);
+    }
   }
 }
 

@@ -65,9 +65,9 @@ def _remember_status(ws: Optional[torch.Tensor]) -> None:
     if ws is None:  # a kernel without device-side waits: nothing can expire
         _LAST_STATUS = None
         return
-    _LAST_STATUS = ws[:4].view(torch.int32).clone()
+    _LAST_STATUS = torch.narrow_copy(ws, 0, 0, 4)
     if _CHECK_STATUS and not torch.cuda.is_current_stream_capturing():
-        code = int(_LAST_STATUS.item())
+        code = device_status()
         if code != 0:
             raise RuntimeError(f"a device-side wait of the tensor-core simplicial kernel expired (status {code}); "
                                "the outputs of this call are zeros")  # fmt: skip
@@ -82,7 +82,7 @@ def device_status() -> int:
     """
     if _LAST_STATUS is None:
         return 0
-    return int(_LAST_STATUS.item())
+    return int(_LAST_STATUS.view(torch.int32).item())
 
 
 def _stream(device: torch.device):
@@ -231,14 +231,15 @@ def cuda_simplicial_attention_forward(
         a.message_left, a.message_right, a.message_basis = (t.data_ptr() for t in message[0])
         a.message_rank = message[1]
     L = _lib.lib()
-    need = L.mf_simplicial_fwd_workspace_bytes(ctypes.byref(a))
-    ws = torch.empty(max(need, 1), device=q.device, dtype=torch.uint8) if need else None
-    a.workspace = ws.data_ptr() if ws is not None else None
-    a.workspace_bytes = need
-    with torch.cuda.device(q.device):
-        _lib.check(L.mf_simplicial_fwd(ctypes.byref(a), _stream(q.device)))
-    if L.mf_simplicial_fwd_backend(ctypes.byref(a)) == _lib.MF_BACKEND["tcgen05"]:
-        _remember_status(ws)  # only the tensor-core kernels keep a status word there
+    ref = ctypes.byref(a)
+    need = L.mf_simplicial_fwd_workspace_bytes(ref)
+    ws = torch.empty(need, device=q.device, dtype=torch.uint8) if need else None
+    if ws is not None:
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    _lib.launch(L.mf_simplicial_fwd, q.device, ref)
+    # only the tensor-core kernels keep a status word in their workspace
+    if (ws is not None or _LAST_STATUS is not None) and L.mf_simplicial_fwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
+        _remember_status(ws)
     return out, lse, out32
 
 
@@ -294,30 +295,9 @@ def cuda_simplicial_attention_backward(
     qv = _mask_bytes(query_valid, (B, N), "query_valid")
     kv = _mask_bytes(pair_key_valid, (B, N), "pair_key_valid")
     pv = _mask_bytes(pair_valid, (B, N, N), "pair_valid") if pair_valid is not None else None
-    grads = [torch.empty_like(q) for _ in range(5)]
     bias = _factorized_bias(u, v_bias, w, gate, B, H, N)
-    bias_grads = [None, None, None, None]
-    if bias is not None:
-        for slot, (need_it, like) in enumerate(zip((need_du, need_dv_bias, need_dw, need_dgate), bias)):
-            if need_it:
-                bias_grads[slot] = torch.zeros_like(like)
-
     angle = _angle_group(angle_left, angle_right, angle_gate, B, H, N)
     message = _message_group(message_left, message_right, message_basis, B, H, N, D)
-    angle_grads = [None, None, None]
-    message_grads = [None, None, None]  # left, right, coefficients (the basis gradient is formed from them below)
-    if angle is not None:
-        for slot, (need_it, like) in enumerate(zip((need_dangle_left, need_dangle_right, need_dangle_gate), angle[0])):
-            if need_it:
-                angle_grads[slot] = torch.zeros_like(like)
-    if message is not None:
-        ml32, mr32, _ = message[0]
-        if need_dmessage_left:
-            message_grads[0] = torch.zeros_like(ml32)
-        if need_dmessage_right:
-            message_grads[1] = torch.zeros_like(mr32)
-        if need_dmessage_basis:
-            message_grads[2] = torch.zeros((B, H, N, message[1]), device=q.device, dtype=torch.float32)
 
     a = _lib.MfSimplicialBwdArgs()
     a.batch, a.heads, a.tokens, a.head_dim = B, H, N, D
@@ -329,29 +309,47 @@ def cuda_simplicial_attention_backward(
     a.out, a.lse = out.data_ptr(), lse.data_ptr()
     a.query_valid, a.pair_key_valid = qv.data_ptr(), kv.data_ptr()
     a.pair_valid = pv.data_ptr() if pv is not None else None
+    grads = [torch.empty_like(q) for _ in range(5)]
     a.dq, a.dk1, a.dv1, a.dk2, a.dv2 = (g.data_ptr() for g in grads)
+    L = _lib.lib()
+    ref = ctypes.byref(a)
     if bias is not None:
         a.u, a.v_bias, a.w, a.gate = (t.data_ptr() for t in bias)
-        a.du, a.dv_bias, a.dw, a.dgate = (g.data_ptr() if g is not None else None for g in bias_grads)
     if angle is not None:
         a.angle_left, a.angle_right, a.angle_gate = (t.data_ptr() for t in angle[0])
         a.angle_rank = angle[1]
-        a.dangle_left, a.dangle_right, a.dangle_gate = (g.data_ptr() if g is not None else None for g in angle_grads)
     if message is not None:
         a.message_left, a.message_right, a.message_basis = (t.data_ptr() for t in message[0])
         a.message_rank = message[1]
-        a.dmessage_left, a.dmessage_right, a.message_coeff = (
-            g.data_ptr() if g is not None else None for g in message_grads
-        )
-    L = _lib.lib()
-    need = L.mf_simplicial_bwd_workspace_bytes(ctypes.byref(a))
+    bias_grads = [None, None, None, None]
+    angle_grads = [None, None, None]
+    message_grads = [None, None, None]  # left, right, coefficients (the basis gradient is formed from them below)
+    if bias is not None or angle is not None or message is not None:
+        # most kernels add to these gradients, or skip what is hidden; those for small molecules write every element
+        new = torch.zeros_like if L.mf_simplicial_bwd_needs_zeros(ref) else torch.empty_like
+        if bias is not None:
+            bias_grads = [new(t) if need_it else None
+                          for need_it, t in zip((need_du, need_dv_bias, need_dw, need_dgate), bias)]  # fmt: skip
+            a.du, a.dv_bias, a.dw, a.dgate = (g.data_ptr() if g is not None else None for g in bias_grads)
+        if angle is not None:
+            angle_grads = [new(t) if need_it else None
+                           for need_it, t in zip((need_dangle_left, need_dangle_right, need_dangle_gate), angle[0])]  # fmt: skip
+            a.dangle_left, a.dangle_right, a.dangle_gate = (g.data_ptr() if g is not None else None for g in angle_grads)
+        if message is not None:
+            ml32, mr32, _ = message[0]
+            message_grads = [new(ml32) if need_dmessage_left else None, new(mr32) if need_dmessage_right else None,
+                             new(ml32[:, :, :, 0]) if need_dmessage_basis else None]  # fmt: skip
+            a.dmessage_left, a.dmessage_right, a.message_coeff = (
+                g.data_ptr() if g is not None else None for g in message_grads
+            )
+    need = L.mf_simplicial_bwd_workspace_bytes(ref)
     ws = torch.empty(need, device=q.device, dtype=torch.uint8) if need else None
-    a.workspace = ws.data_ptr() if ws is not None else None
-    a.workspace_bytes = need
-    with torch.cuda.device(q.device):
-        _lib.check(L.mf_simplicial_bwd(ctypes.byref(a), _stream(q.device)))
-    if L.mf_simplicial_bwd_backend(ctypes.byref(a)) == _lib.MF_BACKEND["tcgen05"]:
-        _remember_status(ws)  # only the tensor-core kernels keep a status word there
+    if ws is not None:
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    _lib.launch(L.mf_simplicial_bwd, q.device, ref)
+    # only the tensor-core kernels keep a status word in their workspace
+    if (ws is not None or _LAST_STATUS is not None) and L.mf_simplicial_bwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
+        _remember_status(ws)
     if bias is not None:  # the reference returns each bias gradient in the dtype of its operand (:1155-1160)
         bias_grads = [g.to(t.dtype) if g is not None else None for g, t in zip(bias_grads, (u, v_bias, w, gate))]
     if angle is not None:
@@ -466,8 +464,7 @@ class _PackedSimplicialAttention(torch.autograd.Function):
                                         proj=proj.data_ptr(), query_valid=qv.data_ptr(), pair_key_valid=kv.data_ptr(),
                                         pair_valid=pv.data_ptr() if pv is not None else None, out32=out32.data_ptr(),
                                         lse=lse.data_ptr(), out=out.data_ptr())  # fmt: skip
-        with torch.cuda.device(proj.device):
-            _lib.check(_lib.lib().mf_simplicial_packed_fwd(ctypes.byref(a), _stream(proj.device)))
+        _lib.launch(_lib.lib().mf_simplicial_packed_fwd, proj.device, ctypes.byref(a))
         _remember_status(None)
         ctx.save_for_backward(proj, qv, kv, pv, out32, lse)
         ctx.meta = (heads, float(q_scale))
@@ -486,8 +483,7 @@ class _PackedSimplicialAttention(torch.autograd.Function):
                                         pair_valid=pv.data_ptr() if pv is not None else None, out32=out32.data_ptr(),
                                         lse=lse.data_ptr(), grad_out=grad_out.data_ptr(),
                                         grad_proj=grad_proj.data_ptr())  # fmt: skip
-        with torch.cuda.device(proj.device):
-            _lib.check(_lib.lib().mf_simplicial_packed_bwd(ctypes.byref(a), _stream(proj.device)))
+        _lib.launch(_lib.lib().mf_simplicial_packed_bwd, proj.device, ctypes.byref(a))
         _remember_status(None)
         return grad_proj, None, None, None, None, None
 
