@@ -140,13 +140,14 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, Shared& 
     if constexpr (RK > 0) {
       const size_t qi = (size_t)bh * p.N + i;
       __syncwarp();
-      if (p.al) {
-        stage_factor(left, p.al + qi * p.N * p.ra, n, p.ra, kmask, nullptr, lane);
-        stage_factor(right, p.ar + qi * p.N * p.ra, n, p.ra, kmask, nullptr, lane);
-      }
-      if (p.ml) {  // K side: only ML_r (dO_i . basis_r) enters dP
-        stage_factor(mleft, p.ml + qi * p.N * p.rm, n, p.rm, kmask, kKeySide ? sm.dc[i] : nullptr, lane);
-        stage_factor(mright, p.mr + qi * p.N * p.rm, n, p.rm, kmask, nullptr, lane);
+      const size_t qa = qi * p.N * p.ra, qm = qi * p.N * p.rm;
+      if (p.al) stage_factors<2>({left, right}, {p.al + qa, p.ar + qa}, n, p.ra, kmask, nullptr, lane);
+      if (p.ml)  // K side: only ML_r (dO_i . basis_r) enters dP
+        stage_factors<2>({mleft, mright}, {p.ml + qm, p.mr + qm}, n, p.rm, kmask, kKeySide ? sm.dc[i] : nullptr, lane);
+      if (i + kWarps < nq) {
+        const size_t next = (size_t)kWarps * p.N;
+        if (p.al) prefetch_l2(p.al + qa + next * p.ra, n * p.ra * 4, lane), prefetch_l2(p.ar + qa + next * p.ra, n * p.ra * 4, lane);
+        if (p.ml) prefetch_l2(p.ml + qm + next * p.rm, n * p.rm * 4, lane), prefetch_l2(p.mr + qm + next * p.rm, n * p.rm * 4, lane);
       }
       __syncwarp();
       if (p.al) {

@@ -99,13 +99,17 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
     float coef[2 * RK];  // message coefficients of ranks 8 e + row8
     if (have) {
       __syncwarp();
-      if (p.al) {
-        stage_factor(left, p.al + qi * N * p.ra, n, p.ra, kmask, nullptr, lane);
-        stage_factor(right, p.ar + qi * N * p.ra, n, p.ra, kmask, nullptr, lane);
+      const size_t qa = qi * N * p.ra, qm = qi * N * p.rm;
+      if (p.al && p.ml && p.ra == p.rm) {
+        stage_factors<4, RK>({left, right, mleft, mright}, {p.al + qa, p.ar + qa, p.ml + qm, p.mr + qm}, n, p.ra, kmask, nullptr, lane);
+      } else {
+        if (p.al) stage_factors<2, RK>({left, right}, {p.al + qa, p.ar + qa}, n, p.ra, kmask, nullptr, lane);
+        if (p.ml) stage_factors<2, RK>({mleft, mright}, {p.ml + qm, p.mr + qm}, n, p.rm, kmask, nullptr, lane);
       }
-      if (p.ml) {
-        stage_factor(mleft, p.ml + qi * N * p.rm, n, p.rm, kmask, nullptr, lane);
-        stage_factor(mright, p.mr + qi * N * p.rm, n, p.rm, kmask, nullptr, lane);
+      if (i + kResWarps < N) {
+        const size_t next = (size_t)kResWarps * N;
+        if (p.al) prefetch_l2(p.al + qa + next * p.ra, n * p.ra * 4, lane), prefetch_l2(p.ar + qa + next * p.ra, n * p.ra * 4, lane);
+        if (p.ml) prefetch_l2(p.ml + qm + next * p.rm, n * p.rm * 4, lane), prefetch_l2(p.mr + qm + next * p.rm, n * p.rm * 4, lane);
       }
       __syncwarp();
       float s[MT][NT][4];

@@ -203,36 +203,60 @@ __device__ __forceinline__ void store_shared64(uint32_t addr, uint32_t a, uint32
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
 
-// Stages rows [0, n) of one query's factor (row-major, `rank` floats each) by one warp, column r times rank_scale[r] when
-// given; rows of hidden keys become zeros.
-template <int RK>
-__device__ __forceinline__ void stage_factor(const RankTile<RK>& t, const float* __restrict__ src, int n, int rank, uint32_t kmask,
-                                             const float* rank_scale, int lane) {
-  if ((rank & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+// Stages rows [0, n) of F factors of one query (row-major, `rank` floats each) by one warp, column r of the first
+// one times scale0[r] when given; rows of hidden keys become zeros.  All loads are issued before the first value is used: a query's factors come from DRAM.
+template <int F, int RK>
+__device__ __forceinline__ void stage_factors(const RankTile<RK> (&t)[F], const float* const (&src)[F], int n, int rank, uint32_t kmask,
+                                              const float* scale0, int lane) {
+  bool fast = (rank & 3) == 0;
+#pragma unroll
+  for (int f = 0; f < F; ++f) fast = fast && (reinterpret_cast<uintptr_t>(src[f]) & 15) == 0;
+  if (fast) {
     const int q = rank >> 2, total = n * q;
-    for (int idx = lane; idx < total; idx += 32) {
-      const int row = idx / q, c = idx - row * q;
-      float4 x = reinterpret_cast<const float4*>(src)[idx];
-      if (!((kmask >> row) & 1u)) x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (rank_scale) x.x *= rank_scale[4 * c], x.y *= rank_scale[4 * c + 1], x.z *= rank_scale[4 * c + 2], x.w *= rank_scale[4 * c + 3];
-      uint32_t h0, l0, h1, l1;
-      split_bf16(x.x, x.y, h0, l0);
-      split_bf16(x.z, x.w, h1, l1);
-      const uint32_t a = t.at(row, c >> 1) + (c & 1) * 8;
-      store_shared64(a, h0, h1);
-      store_shared64(a + RankTile<RK>::kTile, l0, l1);
+    float4 x[F][4 * RK];
+#pragma unroll
+    for (int f = 0; f < F; ++f)
+#pragma unroll
+      for (int s = 0; s < 4 * RK; ++s) {
+        const int idx = lane + 32 * s;
+        x[f][s] = idx < total ? __ldg(reinterpret_cast<const float4*>(src[f]) + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+    for (int s = 0; s < 4 * RK; ++s) {
+      const int idx = lane + 32 * s;
+      if (idx < total) {
+        const int row = idx / q, c = idx - row * q;
+        const bool ok = (kmask >> row) & 1u;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+          float4 v = ok ? x[f][s] : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (f == 0 && scale0) v.x *= scale0[4 * c], v.y *= scale0[4 * c + 1], v.z *= scale0[4 * c + 2], v.w *= scale0[4 * c + 3];
+          uint32_t h0, l0, h1, l1;
+          split_bf16(v.x, v.y, h0, l0);
+          split_bf16(v.z, v.w, h1, l1);
+          const uint32_t a = t[f].at(row, c >> 1) + (c & 1) * 8;
+          store_shared64(a, h0, h1);
+          store_shared64(a + RankTile<RK>::kTile, l0, l1);
+        }
+      }
     }
   } else {
     for (int idx = lane; idx < n * rank; idx += 32) {
       const int row = idx / rank, r = idx - row * rank;
-      const float x = ((kmask >> row) & 1u) ? src[idx] * (rank_scale ? rank_scale[r] : 1.f) : 0.f;
-      uint32_t h, l;
-      split_bf16(x, 0.f, h, l);
-      const uint32_t a = t.at(row, r >> 3) + (r & 7) * 2;
-      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)h) : "memory");
-      asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + RankTile<RK>::kTile), "h"((uint16_t)l) : "memory");
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        uint32_t h, l;
+        split_bf16(((kmask >> row) & 1u) ? src[f][idx] * (f == 0 && scale0 ? scale0[r] : 1.f) : 0.f, 0.f, h, l);
+        const uint32_t a = t[f].at(row, r >> 3) + (r & 7) * 2;
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)h) : "memory");
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + RankTile<RK>::kTile), "h"((uint16_t)l) : "memory");
+      }
     }
   }
+}
+// Brings `bytes` from `p` on into L2 (one line per lane and step): the factors of the query that comes next
+__device__ __forceinline__ void prefetch_l2(const float* p, int bytes, int lane) {
+  for (int o = lane * 128; o < bytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p) + o));
 }
 
 // c[mt][nt] += L_i R_i^T over the rank
