@@ -186,6 +186,10 @@ size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* args);
  * in the reference.)  Only the tensor-core kernels leave a status word at the start of the workspace. */
 int mf_simplicial_fwd_backend(const MfSimplicialFwdArgs* args);
 int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* args);
+/* The gradient of message_basis from MfSimplicialBwdArgs.message_coeff: out[h,r,:] = sum_{b,i} coeff[b,h,i,r] grad_out[b,h,i,:]
+ * (coeff (B,H,N,R) fp32, grad_out (B,H,N,D) in `dtype`, out (H,R,D) fp32; fixed order of additions). */
+int mf_simplicial_basis_grad(const float* coeff, const void* grad_out, int32_t dtype, int32_t batch, int32_t heads,
+                             int32_t tokens, int32_t rank, int32_t head_dim, float* out, void* stream);
 /* 1 when the gradients of bias and residual operands have to be zero-filled before this call, 0 when the kernels that would
  * serve it write every element themselves (molecules of at most 32 tokens on the tensor cores). */
 int mf_simplicial_bwd_needs_zeros(const MfSimplicialBwdArgs* args);

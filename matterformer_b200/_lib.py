@@ -7,6 +7,7 @@ fails loudly instead of silently computing somewhere else.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int32, c_size_t, c_void_p
 from pathlib import Path
 
@@ -30,6 +31,7 @@ MF_SPARSE_BACKEND = {"auto": 0, "mma": 1, "tcgen05": 2}
 EXPORTED_SYMBOLS = (
     "mf_simplicial_fwd_backend",
     "mf_simplicial_bwd_needs_zeros",
+    "mf_simplicial_basis_grad",
     "mf_simplicial_bwd_backend",
     "mf_simplicial_row_plan",
     "mf_simplicial_fwd_workspace_bytes",
@@ -384,12 +386,33 @@ def lib() -> ctypes.CDLL:
     L.mf_simplicial_bwd_backend.restype = c_int32
     L.mf_simplicial_bwd_needs_zeros.argtypes = [POINTER(MfSimplicialBwdArgs)]
     L.mf_simplicial_bwd_needs_zeros.restype = c_int32
+    L.mf_simplicial_basis_grad.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p,
+                                           c_void_p]  # fmt: skip
+    L.mf_simplicial_basis_grad.restype = c_int32
     L.mf_profile_enable.argtypes = [c_int32]
     L.mf_profile_enable.restype = c_int32
     L.mf_profile_read.argtypes = [c_int32, POINTER(ctypes.c_double), POINTER(c_int32)]
     L.mf_profile_read.restype = c_int32
     _LIB = L
     return L
+
+
+_NATIVE: list = []
+
+
+def native():
+    """The operators' host path in C++ (``csrc/torch_binding.cpp``), or None where it has not been built: the Python path
+    then serves every call."""
+    if not _NATIVE:
+        path = LIB_PATH.parent / "_mf_torch.so"
+        module = None
+        if path.exists():
+            lib()  # the symbols the binding links against, from the file next to it
+            spec = importlib.util.spec_from_file_location("_mf_torch", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+        _NATIVE.append(module)
+    return _NATIVE[0]
 
 
 def last_error() -> str:

@@ -17,6 +17,7 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 OBJ_DIR = PKG_DIR / "build"
 LIB_PATH = PKG_DIR / "libmatterformer_b200.so"
+TORCH_BINDING = PKG_DIR / "_mf_torch.so"
 
 NVCC_FLAGS = [
     "-gencode",
@@ -73,7 +74,31 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_torch_binding(force)
     return LIB_PATH
+
+
+def _build_torch_binding(force: bool) -> None:
+    """The operators' host path for torch (csrc/torch_binding.cpp), linked against the library next to it."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    src = CSRC / "torch_binding.cpp"
+    if not force and TORCH_BINDING.exists() and TORCH_BINDING.stat().st_mtime > max(
+        src.stat().st_mtime, _newest([PKG_DIR.parent / "include" / "matterformer_b200.h"])
+    ):
+        return
+    includes = [*cpp_extension.include_paths(device_type="cuda"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{p}" for p in includes), "-DTORCH_EXTENSION_NAME=_mf_torch",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", str(src), "-o", str(TORCH_BINDING),
+           f"-L{PKG_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN",
+           *(f"-L{p}" for p in cpp_extension.library_paths(device_type="cuda")),
+           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]  # fmt: skip
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src.name}:\n{res.stdout}\n{res.stderr}")
 
 
 if __name__ == "__main__":

@@ -662,4 +662,46 @@ int simplicial_generic_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   return MF_OK;
 }
 
+namespace {
+// d basis[h,r,:] = sum over (b,i) of coeff[b,h,i,r] grad_out[b,h,i,:]; one CTA per (h,r), sixteen row groups of 64 lanes, added
+// up in a fixed order.  (As a batched matrix-vector product behind a cast it took 53 us at 64 x 29 rows.)
+template <typename T>
+__global__ void __launch_bounds__(1024) basis_grad_kernel(const float* __restrict__ coeff, const T* __restrict__ grad_out, int B,
+                                                          int H, int N, int R, int D, float* __restrict__ out) {
+  __shared__ float part[16][128];
+  const int h = blockIdx.x, r = blockIdx.y, g = threadIdx.x >> 6, l = threadIdx.x & 63;
+  float a0 = 0.f, a1 = 0.f;
+  const bool in0 = l < D, in1 = l + 64 < D;
+#pragma unroll 8
+  for (int row = g; row < B * N; row += 16) {
+    const size_t at = ((size_t)(row / N) * H + h) * N + row % N;
+    const float c = coeff[at * R + r];
+    if (in0) a0 = fmaf(c, to_f32<T>(grad_out[at * D + l]), a0);
+    if (in1) a1 = fmaf(c, to_f32<T>(grad_out[at * D + l + 64]), a1);
+  }
+  part[g][l] = a0;
+  part[g][l + 64] = a1;
+  __syncthreads();
+  if (threadIdx.x < D) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) s += part[q][threadIdx.x];
+    out[((size_t)h * R + r) * D + threadIdx.x] = s;
+  }
+}
+}  // namespace
+
 }  // namespace mf
+
+extern "C" int mf_simplicial_basis_grad(const float* coeff, const void* grad_out, int32_t dtype, int32_t batch, int32_t heads,
+                                        int32_t tokens, int32_t rank, int32_t head_dim, float* out, void* stream) {
+  using namespace mf;
+  MF_CHECK_ARG(batch >= 0 && heads >= 0 && tokens >= 0 && rank >= 1 && rank <= 32 && head_dim >= 1 && head_dim <= 128,
+               "mf_simplicial_basis_grad: bad size");
+  if (heads == 0) return MF_OK;
+  MF_CHECK_ARG(out && ((coeff && grad_out) || batch == 0 || tokens == 0), "mf_simplicial_basis_grad: null pointer argument");
+  MF_DISPATCH_DTYPE(dtype, T, (basis_grad_kernel<T><<<dim3(heads, rank), 1024, 0, static_cast<cudaStream_t>(stream)>>>(
+                                  coeff, static_cast<const T*>(grad_out), batch, heads, tokens, rank, head_dim, out)));
+  MF_CHECK_LAUNCH("basis_grad_kernel");
+  return MF_OK;
+}

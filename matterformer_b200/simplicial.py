@@ -62,10 +62,13 @@ def set_check_status(on: bool) -> bool:
 
 def _remember_status(ws: Optional[torch.Tensor]) -> None:
     global _LAST_STATUS
-    if ws is None:  # a kernel without device-side waits: nothing can expire
-        _LAST_STATUS = None
+    native = _lib.native()
+    if native is not None:  # which also remembers the calls it serves itself
+        native.remember_status(ws)
+    else:  # a kernel without device-side waits leaves no workspace: nothing can expire
+        _LAST_STATUS = torch.narrow_copy(ws, 0, 0, 4) if ws is not None else None
+    if ws is None:
         return
-    _LAST_STATUS = torch.narrow_copy(ws, 0, 0, 4)
     if _CHECK_STATUS and not torch.cuda.is_current_stream_capturing():
         code = device_status()
         if code != 0:
@@ -80,9 +83,9 @@ def device_status() -> int:
     expired, the kernel gave up cleanly and the affected outputs are zeros (the backward pass then
     writes every gradient as zeros).  Reading it synchronises.
     """
-    if _LAST_STATUS is None:
-        return 0
-    return int(_LAST_STATUS.view(torch.int32).item())
+    native = _lib.native()
+    status = native.last_status() if native is not None else _LAST_STATUS
+    return 0 if status is None else int(status.view(torch.int32).item())
 
 
 def _stream(device: torch.device):
@@ -238,7 +241,7 @@ def cuda_simplicial_attention_forward(
         a.workspace, a.workspace_bytes = ws.data_ptr(), need
     _lib.launch(L.mf_simplicial_fwd, q.device, ref)
     # only the tensor-core kernels keep a status word in their workspace
-    if (ws is not None or _LAST_STATUS is not None) and L.mf_simplicial_fwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
+    if L.mf_simplicial_fwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
         _remember_status(ws)
     return out, lse, out32
 
@@ -348,7 +351,7 @@ def cuda_simplicial_attention_backward(
         a.workspace, a.workspace_bytes = ws.data_ptr(), need
     _lib.launch(L.mf_simplicial_bwd, q.device, ref)
     # only the tensor-core kernels keep a status word in their workspace
-    if (ws is not None or _LAST_STATUS is not None) and L.mf_simplicial_bwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
+    if L.mf_simplicial_bwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
         _remember_status(ws)
     if bias is not None:  # the reference returns each bias gradient in the dtype of its operand (:1155-1160)
         bias_grads = [g.to(t.dtype) if g is not None else None for g, t in zip(bias_grads, (u, v_bias, w, gate))]
@@ -357,7 +360,10 @@ def cuda_simplicial_attention_backward(
                        for g, t in zip(angle_grads, (angle_left, angle_right, angle_gate))]  # fmt: skip
     if message is not None:
         if message_grads[2] is not None:  # d basis[h,r,:] = sum_{b,i} coeff[b,h,i,r] grad_out[b,h,i,:]
-            message_grads[2] = torch.einsum("bhir,bhid->hrd", message_grads[2], grad_out.float()).to(message_basis.dtype)
+            coeff, message_grads[2] = message_grads[2], torch.empty_like(message[0][2])
+            _lib.launch(L.mf_simplicial_basis_grad, q.device, coeff.data_ptr(), grad_out.data_ptr(), a.dtype, B, H, N, message[1],
+                        D, message_grads[2].data_ptr())  # fmt: skip
+            message_grads[2] = message_grads[2].to(message_basis.dtype)
         message_grads[0] = message_grads[0].to(message_left.dtype) if message_grads[0] is not None else None
         message_grads[1] = message_grads[1].to(message_right.dtype) if message_grads[1] is not None else None
     return (*grads, *bias_grads, *angle_grads, *message_grads)
@@ -441,6 +447,9 @@ class CudaTwoSimplicialAttentionFunction(torch.autograd.Function):
 
 
 
+_KERNEL_CALLS = (cuda_simplicial_attention_forward, cuda_simplicial_attention_backward)
+
+
 def packed_projection_applies(proj: torch.Tensor, heads: int, head_dim: int) -> bool:
     """Whether :func:`simplicial_attention_packed` serves this projection: CUDA bf16 (B, N, 5*H*64) with at most 32
     tokens and a multiple of four heads (the kernels that pack four heads into one tile)."""
@@ -511,6 +520,16 @@ def simplicial_attention_cuda(q, k1, v1, k2, v2, *, query_valid, pair_key_valid,
     ``angle_residual`` an optional ``(left, right, gate)`` tuple and ``message_residual`` an optional
     ``(left, right, basis)`` tuple of the low-rank residuals (simplicial_attention.py:50-104).
     """
+    native = _lib.native()
+    if native is not None and not _CHECK_STATUS and _KERNEL_CALLS == (cuda_simplicial_attention_forward,
+                                                                      cuda_simplicial_attention_backward):  # fmt: skip
+        # (checks, launch and autograd node in C++; None when an operand needs converting, or an error message)
+        out = native.simplicial_attention(q, k1, v1, k2, v2, query_valid, pair_key_valid, pair_valid,
+                                          factorized_bias or (), angle_residual or (), message_residual or (),
+                                          _lib.MF_PRECISION[normalize_simplicial_precision(precision)], _lib.MF_BACKEND[_BACKEND],
+                                          MAX_RESIDUAL_RANK)  # fmt: skip
+        if out is not None:
+            return out
     empty_f = q.new_empty(0)
     empty_b = torch.empty(0, device=q.device, dtype=torch.bool)
     u, v, w, gate = factorized_bias if factorized_bias is not None else (empty_f,) * 4

@@ -234,6 +234,17 @@ def _check_qkv(name, q, k, v):
         raise ValueError(f"{name}: head_dim must be 32, 64 or 128, got {q.shape[-1]}")
 
 
+def _sparse_attention(q, k, v, num_atoms, window, scale, count, cols, mask):
+    """Radius (``window`` 0) or band attention: checks, launch and autograd node in C++ where that is built and the operands
+    are ready, else :class:`_SparseAttention`."""
+    native = _lib.native()
+    if native is not None:
+        out = native.sparse_attention(q, k, v, num_atoms, count, cols, mask, window, scale, _lib.MF_SPARSE_BACKEND[_SPARSE_BACKEND])
+        if out is not None:
+            return out
+    return _SparseAttention.apply(q, k, v, num_atoms, "local" if window else "radius", window, scale, count, cols, mask)
+
+
 class _SparseAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, num_atoms, kind, window, scale, block_count, block_cols, block_mask):
@@ -290,8 +301,7 @@ def radius_block_sparse_attention(q, k, v, blocks: RadiusBlocks, *, scale: Optio
     if not sorted_inputs:
         idx = blocks.perm.long()[:, None, :, None].expand_as(q)
         q, k, v = (torch.gather(t, 2, idx) for t in (q, k, v))
-    out = _SparseAttention.apply(q, k, v, blocks.num_atoms, "radius", 0, scale, blocks.block_count,
-                                 blocks.block_cols, blocks.block_mask)  # fmt: skip
+    out = _sparse_attention(q, k, v, blocks.num_atoms, 0, scale, blocks.block_count, blocks.block_cols, blocks.block_mask)
     if not sorted_inputs:
         inv = blocks.inverse_perm.long()[:, None, :, None].expand_as(out)
         out = torch.gather(out, 2, inv)
@@ -308,7 +318,7 @@ def local_window_attention(q, k, v, num_atoms: Optional[torch.Tensor] = None, wi
     na = _num_atoms(num_atoms, B, N, q.device)
     scale = D**-0.5 if scale is None else float(scale)
     empty = torch.empty(0, device=q.device, dtype=torch.int32)
-    return _SparseAttention.apply(q, k, v, na, "local", int(window), scale, empty, empty, empty)
+    return _sparse_attention(q, k, v, na, int(window), scale, empty, empty, empty)
 
 
 class _LocalAttentionPacked(torch.autograd.Function):
