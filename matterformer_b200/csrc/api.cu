@@ -114,6 +114,13 @@ bool uses_small_kernels(const Args* a) {
   return (a->backend == MF_BACKEND_AUTO || a->backend == MF_BACKEND_TCGEN05_TILES) && a->tokens <= kSmallTokens;
 }
 
+// fp32 molecules of at most 64 tokens (two keys per lane would not fit the registers), plain attention, aligned rows.
+template <typename Args>
+bool uses_f32_kernels(const Args* a) {
+  return a->backend == MF_BACKEND_AUTO && a->dtype == MF_DTYPE_F32 && a->tokens <= 64 && (a->head_dim == 32 || a->head_dim == 64) &&
+         !has_factorized_bias(a) && !a->angle_left && !a->message_left && vectors_aligned(a);
+}
+
 }  // namespace
 }  // namespace mf
 
@@ -145,7 +152,7 @@ extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a
   int rc;
   if (wants_tcgen05(a, &rc, "mf_simplicial_bwd"))
     return uses_small_kernels(a) ? 0 : uses_tile_kernels(a) ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
-  return simplicial_generic_bwd_workspace_bytes(*a);
+  return uses_f32_kernels(a) ? 0 : simplicial_generic_bwd_workspace_bytes(*a);
 }
 
 extern "C" int mf_simplicial_fwd_backend(const MfSimplicialFwdArgs* a) {
@@ -191,7 +198,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
     set_error("mf_simplicial_fwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
-  if (!tc) return simplicial_generic_fwd(*a, s);
+  if (!tc) return uses_f32_kernels(a) ? simplicial_f32_fwd(*a, s) : simplicial_generic_fwd(*a, s);
   if (uses_small_kernels(a))
     return a->angle_left || a->message_left ? simplicial_small_res_fwd(*a, s) : simplicial_small_fwd(*a, nullptr, s);
   return uses_tile_kernels(a) ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
@@ -214,7 +221,7 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
     set_error("mf_simplicial_bwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
-  if (!tc) return simplicial_generic_bwd(*a, s);
+  if (!tc) return uses_f32_kernels(a) ? simplicial_f32_bwd(*a, s) : simplicial_generic_bwd(*a, s);
   if (uses_small_kernels(a)) return simplicial_small_bwd(*a, nullptr, s);
   return uses_tile_kernels(a) ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
 }

@@ -12,6 +12,10 @@ int simplicial_generic_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 int simplicial_generic_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
 size_t simplicial_generic_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 
+// fp32 CUDA-core kernels for small molecules without geometry operands (simplicial_f32.cu)
+int simplicial_f32_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
+int simplicial_f32_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
+
 // tcgen05 tensor-core kernels (simplicial_sm100.cu)
 bool simplicial_sm100_supports(int dtype, int precision, int tokens, int head_dim);
 // Molecules of at most 32 tokens: four heads share one 128-row tile (needs a multiple of four heads).

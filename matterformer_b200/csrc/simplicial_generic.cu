@@ -663,31 +663,74 @@ int simplicial_generic_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
 }
 
 namespace {
-// d basis[h,r,:] = sum over (b,i) of coeff[b,h,i,r] grad_out[b,h,i,:]; one CTA per (h,r), sixteen row groups of 64 lanes, added
-// up in a fixed order.  (As a batched matrix-vector product behind a cast it took 53 us at 64 x 29 rows.)
+// d basis[h,r,:] = sum over (b,i) of coeff[b,h,i,r] grad_out[b,h,i,:].  A cluster of eight CTAs per head, each with an eighth
+// of the rows staged through shared memory; the partial sums are added up over the cluster in rank order, so the result
+// does not depend on the schedule.  (As a batched matrix-vector product behind a cast it took 53 us at 64 x 29 rows.)
+constexpr int kBasisRows = 32;
 template <typename T>
-__global__ void __launch_bounds__(1024) basis_grad_kernel(const float* __restrict__ coeff, const T* __restrict__ grad_out, int B,
-                                                          int H, int N, int R, int D, float* __restrict__ out) {
-  __shared__ float part[16][128];
-  const int h = blockIdx.x, r = blockIdx.y, g = threadIdx.x >> 6, l = threadIdx.x & 63;
-  float a0 = 0.f, a1 = 0.f;
-  const bool in0 = l < D, in1 = l + 64 < D;
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256) basis_grad_kernel(const float* __restrict__ coeff,
+                                                                                   const T* __restrict__ grad_out, int B, int H,
+                                                                                   int N, int R, int D, float* __restrict__ out) {
+  __shared__ float sc[kBasisRows][33], sg[kBasisRows][128], part[32 * 128];
+  const int h = blockIdx.y, tid = threadIdx.x, rows = B * N;
+  unsigned rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  float acc[16];  // outputs tid, tid + 256, ... of the R x D matrix
+#pragma unroll
+  for (int t = 0; t < 16; ++t) acc[t] = 0.f;
+  const int per = (rows + 7) / 8, lo = rank * per, hi = min(lo + per, rows);
+  for (int r0 = lo; r0 < hi; r0 += kBasisRows) {
+    __syncthreads();
+    // all of a thread's loads before the first store: the kernel is bound by their latency
+    float x[kBasisRows * 32 / 256], y[kBasisRows * 128 / 256];
+#pragma unroll
+    for (int t = 0; t < kBasisRows * 32 / 256; ++t) {
+      const int idx = tid + 256 * t, row = r0 + idx / R;
+      x[t] = (idx < kBasisRows * R && row < hi) ? coeff[(((size_t)(row / N) * H + h) * N + row % N) * R + idx % R] : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < kBasisRows * 128 / 256; ++t) {
+      const int idx = tid + 256 * t, row = r0 + idx / D;
+      y[t] = (idx < kBasisRows * D && row < hi) ? to_f32<T>(grad_out[(((size_t)(row / N) * H + h) * N + row % N) * D + idx % D]) : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < kBasisRows * 32 / 256; ++t) {
+      const int idx = tid + 256 * t;
+      if (idx < kBasisRows * R) sc[idx / R][idx % R] = x[t];
+    }
+#pragma unroll
+    for (int t = 0; t < kBasisRows * 128 / 256; ++t) {
+      const int idx = tid + 256 * t;
+      if (idx < kBasisRows * D) sg[idx / D][idx % D] = y[t];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      const int o = tid + 256 * t;
+      if (o < R * D) {
+        const int r = o / D, d = o % D;
 #pragma unroll 8
-  for (int row = g; row < B * N; row += 16) {
-    const size_t at = ((size_t)(row / N) * H + h) * N + row % N;
-    const float c = coeff[at * R + r];
-    if (in0) a0 = fmaf(c, to_f32<T>(grad_out[at * D + l]), a0);
-    if (in1) a1 = fmaf(c, to_f32<T>(grad_out[at * D + l + 64]), a1);
+        for (int row = 0; row < kBasisRows; ++row) acc[t] = fmaf(sc[row][r], sg[row][d], acc[t]);
+      }
+    }
   }
-  part[g][l] = a0;
-  part[g][l + 64] = a1;
-  __syncthreads();
-  if (threadIdx.x < D) {
+#pragma unroll
+  for (int t = 0; t < 16; ++t) part[tid + 256 * t] = acc[t];
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(part);
+  for (int o = rank * 256 + tid; o < R * D; o += 8 * 256) {
     float s = 0.f;
 #pragma unroll
-    for (int q = 0; q < 16; ++q) s += part[q][threadIdx.x];
-    out[((size_t)h * R + r) * D + threadIdx.x] = s;
+    for (int q = 0; q < 8; ++q) {
+      uint32_t addr;
+      float v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(mine + 4 * o), "r"(q));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+      s += v;
+    }
+    out[(size_t)h * R * D + o] = s;
   }
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // part stays until all have read
 }
 }  // namespace
 
@@ -700,7 +743,7 @@ extern "C" int mf_simplicial_basis_grad(const float* coeff, const void* grad_out
                "mf_simplicial_basis_grad: bad size");
   if (heads == 0) return MF_OK;
   MF_CHECK_ARG(out && ((coeff && grad_out) || batch == 0 || tokens == 0), "mf_simplicial_basis_grad: null pointer argument");
-  MF_DISPATCH_DTYPE(dtype, T, (basis_grad_kernel<T><<<dim3(heads, rank), 1024, 0, static_cast<cudaStream_t>(stream)>>>(
+  MF_DISPATCH_DTYPE(dtype, T, (basis_grad_kernel<T><<<dim3(8, heads), 256, 0, static_cast<cudaStream_t>(stream)>>>(
                                   coeff, static_cast<const T*>(grad_out), batch, heads, tokens, rank, head_dim, out)));
   MF_CHECK_LAUNCH("basis_grad_kernel");
   return MF_OK;
