@@ -259,10 +259,13 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
   const float4* sorted = w.sorted + (size_t)b * n_max;
   const int32_t* start = w.counts + (size_t)b * (kMaxBins + 1);
   const Cell c = load_cell(cell + (size_t)b * 9);
-  // the grid has a fixed number of warps per structure; each takes every (warps per structure)-th bin
-  for (int bin = blockIdx.x * 4 + warp; bin < gx * gy * gz; bin += gridDim.x * 4) {
-  const int q0 = start[bin], q1 = start[bin + 1];
-  if (q0 == q1) continue;
+  // the grid has a fixed number of warps per structure; each takes every (warps per structure)-th bin, and where there are
+  // more warps than bins (a few small structures) several of them share the queries of a bin
+  const int bins = gx * gy * gz, warps = gridDim.x * 4, parts = max(1, min(32, warps / bins));
+  for (int item = blockIdx.x * 4 + warp; item < bins * parts; item += warps) {
+  const int bin = item % bins, part = item / bins;
+  const int q0 = start[bin] + part, q1 = start[bin + 1];
+  if (q0 >= q1) continue;
   const float h = bounds[2 * b];           // min over axes of width / bins, rounded down
   const float half_w = bounds[2 * b + 1];  // half the smallest perpendicular width, rounded down
   const float fast_limit2 = half_w * half_w * (1.f - 1e-4f);
@@ -277,7 +280,17 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
   const bool covers_all = exhaustive || (gx <= 3 && gy <= 3 && gz <= 3);
   int n_cand = 0;
   bool in_smem = ordered;
+  bool inner = false;  // no neighbour bin is reached across the cell boundary: the zero image is the rounded one
+  if (!ordered && n <= kWarpCand) {
+    // a structure that fits the list: all its atoms, instead of a search bin by bin with a handful of atoms each
+    for (int e = lane; e < n; e += 32) cand[e] = __ldg(sorted + e);
+    n_cand = n;
+    in_smem = true;
+    __syncwarp();
+  }
+  const bool covers = covers_all || (!ordered && in_smem);
   if (ordered) {
+    inner = gx >= 5 && gy >= 5 && gz >= 5 && cx > 0 && cx < gx - 1 && cy > 0 && cy < gy - 1 && cz > 0 && cz < gz - 1;
     // lane t < 27 looks up the extent of neighbour bin t; one prefix sum places every bin's atoms in the list, and the
     // copies of the 27 bins are independent loads (two round trips to memory instead of one per bin)
     int e0 = 0, cnt = 0;
@@ -309,11 +322,13 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
   }
 
   // the list of the k best, entry t on lane t
-  float d = INFINITY;
-  int id = 0x7fffffff;
+  // entries are 64-bit keys, the bits of d2 (never negative) above the index: one comparison orders by (d2, index)
+  constexpr unsigned long long kNone = ((unsigned long long)0x7f800000u << 32) | 0x7fffffffu;
+  unsigned long long key = kNone;
+  auto key_of = [](float d2, int i) { return ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)i; };
+  auto dist_of = [](unsigned long long k) { return __uint_as_float((unsigned)(k >> 32)); };
   int my_id = -1;
   float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto before = [](float cd, int ci, float ed, int ei) { return cd < ed || (cd == ed && ci < ei); };
   // A shell that does not cover every bin only counts if the k-th distance ends up below its reach (else the
   // search is repeated with a wider shell), so candidates at or beyond the reach can be dropped unseen.
   float keep_below = INFINITY;
@@ -325,6 +340,13 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
     if (ok && (include_self || __float_as_int(o.w) != my_id)) {
       if (!exhaustive) {
         const float dx = __fsub_rn(me.x, o.x), dy = __fsub_rn(me.y, o.y), dz = __fsub_rn(me.z, o.z);
+        if (inner) {  // |delta| < 0.5 on every axis: (0, 0, 0) is the offset the comparisons below would find
+          const float rx = __fmaf_rn(dz, c.l20, __fmaf_rn(dy, c.l10, __fmul_rn(dx, c.l00)));
+          const float ry = __fmaf_rn(dz, c.l21, __fmul_rn(dy, c.l11)), rz = __fmul_rn(dz, c.l22);
+          d2 = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx)));
+          if (d2 >= fast_limit2 && far_kept >= fast_limit2) d2 = min_image_d2(me.x, me.y, me.z, o.x, o.y, o.z, c);
+          return d2;
+        }
         // -rint(delta) for |delta| < 1 (ties at +-0.5 go to 0), by comparison: cheaper than three conversions
         const float ox = dx > 0.5f ? -1.f : (dx < -0.5f ? 1.f : 0.f), oy = dy > 0.5f ? -1.f : (dy < -0.5f ? 1.f : 0.f),
                     oz = dz > 0.5f ? -1.f : (dz < -0.5f ? 1.f : 0.f);
@@ -336,48 +358,37 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
     }
     return d2;
   };
-  // the lanes' candidates (d2, oid) that beat the current last entry, inserted one at a time
-  auto insert_batch = [&](float d2, int oid, float worst_d, int worst_i) {
-    uint32_t pass = __ballot_sync(0xffffffffu, d2 < keep_below && before(d2, oid, worst_d, worst_i));
+  // the lanes' candidates that beat the current last entry, inserted one at a time
+  auto insert_batch = [&](float d2, int oid) {
+    const unsigned long long mine = key_of(d2, oid);
+    const unsigned long long last = __shfl_sync(0xffffffffu, key, KMAX - 1);
+    uint32_t pass = __ballot_sync(0xffffffffu, d2 < keep_below && mine < last);
     while (pass) {
       const int src = __ffs(pass) - 1;
       pass &= pass - 1;
-      const float cd = __shfl_sync(0xffffffffu, d2, src);
-      const int ci = __shfl_sync(0xffffffffu, oid, src);
-      const uint32_t bal = __ballot_sync(0xffffffffu, lane < KMAX && before(cd, ci, d, id));
-      const float pd = __shfl_up_sync(0xffffffffu, d, 1);
-      const int pi = __shfl_up_sync(0xffffffffu, id, 1);
+      const unsigned long long ck = __shfl_sync(0xffffffffu, mine, src);
+      const uint32_t bal = __ballot_sync(0xffffffffu, lane < KMAX && ck < key);
+      const unsigned long long pk = __shfl_up_sync(0xffffffffu, key, 1);
       if (bal == 0u) continue;  // earlier insertions of this batch pushed it out
       const int pos = __ffs(bal) - 1;
-      if (lane == pos) {
-        d = cd;
-        id = ci;
-      } else if (lane > pos && lane < KMAX) {
-        d = pd;
-        id = pi;
-      }
+      if (lane == pos) key = ck;
+      else if (lane > pos && lane < KMAX) key = pk;
     }
   };
   // 32 candidates, one per lane (valid where `ok`)
   auto consider = [&](float4 o, bool ok) {
-    const float worst_d = __shfl_sync(0xffffffffu, d, KMAX - 1);
-    const int worst_i = __shfl_sync(0xffffffffu, id, KMAX - 1);
-    insert_batch(distance(o, ok, fminf(worst_d, keep_below)), __float_as_int(o.w), worst_d, worst_i);
+    const float worst = dist_of(__shfl_sync(0xffffffffu, key, KMAX - 1));
+    insert_batch(distance(o, ok, fminf(worst, keep_below)), __float_as_int(o.w));
   };
-  // the lanes' 32 entries sorted ascending by (d2, index) across the warp (bitonic network, 15 exchanges)
+  // the lanes' 32 entries sorted ascending across the warp (bitonic network, 15 exchanges)
   auto sort_lanes = [&]() {
 #pragma unroll
     for (int k2 = 2; k2 <= 32; k2 <<= 1) {
 #pragma unroll
       for (int j = k2 >> 1; j > 0; j >>= 1) {
-        const float pd = __shfl_xor_sync(0xffffffffu, d, j);
-        const int pi = __shfl_xor_sync(0xffffffffu, id, j);
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
         const bool keep_min = ((lane & j) == 0) == ((lane & k2) == 0);
-        const bool take = keep_min ? before(pd, pi, d, id) : before(d, id, pd, pi);
-        if (take) {
-          d = pd;
-          id = pi;
-        }
+        if ((other < key) == keep_min) key = other;
       }
     }
   };
@@ -405,15 +416,27 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
   };
 
   const int s_max = max(max(gx, gy), gz);
-  for (int q = q0; q < q1; ++q) {
+  for (int q = q0; q < q1; q += parts) {
     me = __ldg(sorted + q);
     my_id = __float_as_int(me.w);
-    d = INFINITY;
-    id = 0x7fffffff;
+    key = kNone;
     int s = 1;
     bool all_bins;
-    keep_below = (covers_all || exhaustive || s_max <= 1) ? INFINITY : h * h * (1.f - 2e-5f);
-    if (in_smem) {
+    keep_below = (covers || s_max <= 1) ? INFINITY : h * h * (1.f - 2e-5f);
+    if (in_smem && !ordered) {
+      // the first 32 atoms sorted in one go, the others inserted while they beat the last entry (which also spares most of
+      // the far ones the 27-image search)
+      const float4 o = lane < n_cand ? cand[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float d2 = distance(o, lane < n_cand, INFINITY);
+      if (d2 < INFINITY) key = key_of(d2, __float_as_int(o.w));
+      sort_lanes();
+      if (lane >= KMAX) key = kNone;
+      for (int c0 = 32; c0 < n_cand; c0 += 32) {
+        const bool ok = c0 + lane < n_cand;
+        consider(ok ? cand[c0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f), ok);
+      }
+      all_bins = true;
+    } else if (in_smem) {
       // first every candidate's distance, keeping those within the shell's reach; then the first 32 survivors are
       // sorted across the lanes in one go and become the list, the rest (few) are inserted one at a time
       int m = 0;
@@ -429,20 +452,14 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
       __syncwarp();
       if (lane < m) {
         const float2 sv = surv[lane];
-        d = sv.x;
-        id = __float_as_int(sv.y);
+        key = key_of(sv.x, __float_as_int(sv.y));
       }
       sort_lanes();
-      if (lane >= KMAX) {
-        d = INFINITY;
-        id = 0x7fffffff;
-      }
+      if (lane >= KMAX) key = kNone;
       for (int c0 = 32; c0 < m; c0 += 32) {
         const bool ok = c0 + lane < m;
         const float2 sv = ok ? surv[c0 + lane] : make_float2(INFINITY, __int_as_float(0x7fffffff));
-        const float worst_d = __shfl_sync(0xffffffffu, d, KMAX - 1);
-        const int worst_i = __shfl_sync(0xffffffffu, id, KMAX - 1);
-        insert_batch(sv.x, __float_as_int(sv.y), worst_d, worst_i);
+        insert_batch(sv.x, __float_as_int(sv.y));
       }
       __syncwarp();  // the survivor buffer is rewritten for the next query
       all_bins = covers_all;
@@ -452,11 +469,10 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
     // complete when the needed neighbours are known and the farthest of them is inside the searched shell
     while (!all_bins && !exhaustive) {
       const float reach = (float)s * h;
-      const float kth = need >= 1 ? __shfl_sync(0xffffffffu, d, need - 1) : 0.f;
+      const float kth = need >= 1 ? dist_of(__shfl_sync(0xffffffffu, key, need - 1)) : 0.f;
       if (kth < reach * reach * (1.f - 2e-5f) || s >= s_max) break;
       ++s;
-      d = INFINITY;
-      id = 0x7fffffff;
+      key = kNone;
       {  // the reach of the new shell, unless it is the last one (every bin, or the largest half-width)
         const bool last = (2 * s + 1 >= gx && 2 * s + 1 >= gy && 2 * s + 1 >= gz) || s >= s_max;
         const float reach_s = (float)s * h;
@@ -465,9 +481,9 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
       all_bins = scan_shell(s);
     }
     if (lane < k) {
-      const bool have = d < INFINITY;
-      idx[((size_t)b * n_max + my_id) * k + lane] = have ? id : -1;
-      if (dist2) dist2[((size_t)b * n_max + my_id) * k + lane] = have ? d : INFINITY;
+      const bool have = dist_of(key) < INFINITY;
+      idx[((size_t)b * n_max + my_id) * k + lane] = have ? (int)(unsigned)key : -1;
+      if (dist2) dist2[((size_t)b * n_max + my_id) * k + lane] = have ? dist_of(key) : INFINITY;
     }
   }
   __syncwarp();  // the shared-memory list is refilled for the next bin
@@ -548,7 +564,9 @@ int knn_check(const void* frac, const void* cell, const void* num_atoms, int bat
 
 int knn_search(const float* cell, const int32_t* num_atoms, const int32_t* grid_dims, const float* bounds, int batch, int n_max,
                int k, int include_self, const KnnWorkspace& w, int32_t* idx, float* dist2, cudaStream_t s) {
-  dim3 grid(64, batch);  // 256 warps per structure, each taking every 256th bin
+  // at least 256 warps per structure, more when there are few structures: about 4700 (four per scheduler and SM twice over)
+  const int wanted = (1184 + batch - 1) / batch;
+  dim3 grid(wanted > 64 ? wanted : 64, batch);
   if (k <= 16)
     knn_warp_kernel<16><<<grid, 128, 0, s>>>(cell, num_atoms, grid_dims, bounds, n_max, k, include_self, w, idx, dist2);
   else

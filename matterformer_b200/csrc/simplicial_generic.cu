@@ -671,51 +671,46 @@ template <typename T>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256) basis_grad_kernel(const float* __restrict__ coeff,
                                                                                    const T* __restrict__ grad_out, int B, int H,
                                                                                    int N, int R, int D, float* __restrict__ out) {
-  __shared__ float sc[kBasisRows][33], sg[kBasisRows][128], part[32 * 128];
+  __shared__ float sc[kBasisRows][32], sg[kBasisRows][128], part[32 * 128];
   const int h = blockIdx.y, tid = threadIdx.x, rows = B * N;
   unsigned rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  float acc[16];  // outputs tid, tid + 256, ... of the R x D matrix
+  // loading: eight threads per row; summing: channels d and d + 64, ranks rg, rg + 4, ...
+  const int lr = tid >> 3, lc = tid & 7, d = tid & 63, rg = tid >> 6;
+  float acc[8][2];
 #pragma unroll
-  for (int t = 0; t < 16; ++t) acc[t] = 0.f;
+  for (int t = 0; t < 8; ++t) acc[t][0] = acc[t][1] = 0.f;
   const int per = (rows + 7) / 8, lo = rank * per, hi = min(lo + per, rows);
   for (int r0 = lo; r0 < hi; r0 += kBasisRows) {
-    __syncthreads();
-    // all of a thread's loads before the first store: the kernel is bound by their latency
-    float x[kBasisRows * 32 / 256], y[kBasisRows * 128 / 256];
+    const int row = r0 + lr;
+    const size_t at = row < hi ? ((size_t)(row / N) * H + h) * N + row % N : 0;
+    float x[4], y[16];  // all loads before the first store: the kernel is bound by their latency
 #pragma unroll
-    for (int t = 0; t < kBasisRows * 32 / 256; ++t) {
-      const int idx = tid + 256 * t, row = r0 + idx / R;
-      x[t] = (idx < kBasisRows * R && row < hi) ? coeff[(((size_t)(row / N) * H + h) * N + row % N) * R + idx % R] : 0.f;
-    }
+    for (int t = 0; t < 4; ++t) x[t] = (row < hi && lc + 8 * t < R) ? coeff[at * R + lc + 8 * t] : 0.f;
 #pragma unroll
-    for (int t = 0; t < kBasisRows * 128 / 256; ++t) {
-      const int idx = tid + 256 * t, row = r0 + idx / D;
-      y[t] = (idx < kBasisRows * D && row < hi) ? to_f32<T>(grad_out[(((size_t)(row / N) * H + h) * N + row % N) * D + idx % D]) : 0.f;
-    }
-#pragma unroll
-    for (int t = 0; t < kBasisRows * 32 / 256; ++t) {
-      const int idx = tid + 256 * t;
-      if (idx < kBasisRows * R) sc[idx / R][idx % R] = x[t];
-    }
-#pragma unroll
-    for (int t = 0; t < kBasisRows * 128 / 256; ++t) {
-      const int idx = tid + 256 * t;
-      if (idx < kBasisRows * D) sg[idx / D][idx % D] = y[t];
-    }
+    for (int t = 0; t < 16; ++t) y[t] = (row < hi && lc + 8 * t < D) ? to_f32<T>(grad_out[at * D + lc + 8 * t]) : 0.f;
     __syncthreads();
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      const int o = tid + 256 * t;
-      if (o < R * D) {
-        const int r = o / D, d = o % D;
-#pragma unroll 8
-        for (int row = 0; row < kBasisRows; ++row) acc[t] = fmaf(sc[row][r], sg[row][d], acc[t]);
+    for (int t = 0; t < 4; ++t) sc[lr][lc + 8 * t] = x[t];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) sg[lr][lc + 8 * t] = y[t];
+    __syncthreads();
+#pragma unroll 4
+    for (int q = 0; q < kBasisRows; ++q) {
+      const float g0 = sg[q][d], g1 = sg[q][d + 64];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const float c = sc[q][rg + 4 * t];
+        acc[t][0] = fmaf(c, g0, acc[t][0]);
+        acc[t][1] = fmaf(c, g1, acc[t][1]);
       }
     }
   }
 #pragma unroll
-  for (int t = 0; t < 16; ++t) part[tid + 256 * t] = acc[t];
+  for (int t = 0; t < 8; ++t)
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (rg + 4 * t < R && d + 64 * u < D) part[(rg + 4 * t) * D + d + 64 * u] = acc[t][u];
   asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
   const uint32_t mine = (uint32_t)__cvta_generic_to_shared(part);
   for (int o = rank * 256 + tid; o < R * D; o += 8 * 256) {
