@@ -1,0 +1,396 @@
+// Local-window attention, bf16, head_dim 64, windows of 32, 64 and 128: query i sees keys i - w/2 .. i + w/2 - 1
+// (same operator as sparse_attn_mma.cu, which serves the other shapes).
+//
+// A band is short, so a tile's whole neighbourhood fits shared memory: a CTA owns kRows rows and loads them with the w/2 rows
+// before and after, once.  A warp owns 16 rows; the w + 16 partner rows that they can see are w/16 + 1 chunks of 16 with a
+// fixed pattern: the first and the last chunk are triangles, everything between is visible, so no bitmaps, no walk and no
+// masks except at the ends of a structure.  Forward: no running maximum (the softmax shift is 0 unless a row's sum leaves
+// 2^-60 .. 2^60; then the warp looks for its maxima and starts over).  Backward: one launch; the warp's 16 rows first as
+// queries (dq), then as keys (dk, dv), from the same shared rows; delta = dO . out is formed on load.  Every output row has
+// one owner: no atomics, bit-identical reruns.
+#include "common.cuh"
+#include "simplicial_warp.cuh"
+
+namespace mf {
+namespace {
+
+struct BandParams {
+  const __nv_bfloat16* q;
+  const __nv_bfloat16* k;
+  const __nv_bfloat16* v;
+  const __nv_bfloat16* grad_out;
+  const int32_t* num_atoms;
+  __nv_bfloat16* out;  // backward: read
+  float* lse;
+  __nv_bfloat16* dq;
+  __nv_bfloat16* dk;
+  __nv_bfloat16* dv;
+  int H, N;
+  float scale;
+  RowLayout in, act;  // rows of q, k, v and their gradients; rows of out and grad_out
+};
+
+constexpr float kBandLow = 8.6736174e-19f, kBandHigh = 1.1529215e18f;  // 2^-60, 2^60
+
+// rows [first, first + rows) of one head into a swizzled tile; rows outside [0, n) become zeros
+template <int kThreads>
+__device__ __forceinline__ void load_band(uint32_t tile, const __nv_bfloat16* src, long long stride, int first, int rows, int n) {
+  for (int idx = threadIdx.x; idx < rows * 8; idx += kThreads) {
+    const int r = idx >> 3, c = idx & 7, row = first + r;
+    const bool ok = row >= 0 && row < n;
+    cp_async16(row_chunk(tile, r, c), src + (ok ? row : 0) * stride + c * 8, ok);
+  }
+}
+
+// c (16 x 16) = A (16 x 64, fragments) . 16 rows of the tile from byte offset `at`
+__device__ __forceinline__ void chunk_product(float (&c)[2][4], const uint32_t (&a)[4][4], const FragBase& fb, int at) {
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int kp = 0; kp < 2; ++kp) {
+      uint32_t b[4];
+      load_b(b, fb, at, nt, kp);
+      if (kp == 0) mma16_first(c[nt], a[0], b[0], b[1]);
+      else mma16(c[nt], a[2], b[0], b[1]);
+      mma16(c[nt], a[2 * kp + 1], b[2], b[3]);
+    }
+}
+// acc (16 x 64) += P (16 x 16, packed as an A operand) . rows of the chunk
+__device__ __forceinline__ void chunk_accumulate(float (&acc)[8][4], const uint32_t (&p)[4], const FragBase& fb, int at) {
+#pragma unroll
+  for (int dp = 0; dp < 4; ++dp) {
+    uint32_t b[4];
+    load_t2(b, fb, at, dp, 0);
+    mma16(acc[2 * dp], p, b[0], b[1]);
+    mma16(acc[2 * dp + 1], p, b[2], b[3]);
+  }
+}
+__device__ __forceinline__ void pack_chunk(uint32_t (&p)[4], const float (&s)[2][4]) {
+  p[0] = pack2_bf16(s[0][0], s[0][1]);
+  p[1] = pack2_bf16(s[0][2], s[0][3]);
+  p[2] = pack2_bf16(s[1][0], s[1][1]);
+  p[3] = pack2_bf16(s[1][2], s[1][3]);
+}
+// 16 x 64 accumulator to bf16 rows; rows at or beyond N are skipped.  The four lanes of a row exchange their words first (a
+// 4 x 4 transposition), so that a lane stores 16 bytes: stored as they are, every instruction touches eight rows in pieces
+// of 16 bytes, and these pieces, not the arithmetic, filled the load/store pipe.
+__device__ __forceinline__ void store_rows(__nv_bfloat16* dst, long long stride, const float (&acc)[8][4], int row, int N, float lo,
+                                           float hi) {
+  const int quad = threadIdx.x & 3;
+  const bool q0 = quad & 1, q1 = quad >> 1;
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const float mul = hh ? hi : lo;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t w[4];  // tiles 4 half + t; after the exchange: tile 4 half + quad, columns 2 t, 2 t + 1
+#pragma unroll
+      for (int t = 0; t < 4; ++t) w[t] = pack2_bf16(acc[4 * half + t][2 * hh] * mul, acc[4 * half + t][2 * hh + 1] * mul);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {  // across quad bit 0: tiles 2 t and 2 t + 1
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, q0 ? w[2 * t] : w[2 * t + 1], 1);
+        if (q0) w[2 * t] = other; else w[2 * t + 1] = other;
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {  // across quad bit 1: tiles t and t + 2
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, q1 ? w[t] : w[t + 2], 2);
+        if (q1) w[t] = other; else w[t + 2] = other;
+      }
+      if (row + 8 * hh < N)
+        *reinterpret_cast<uint4*>(dst + (row + 8 * hh) * stride + 32 * half + 8 * quad) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+template <int W, int kRows>
+__global__ void __launch_bounds__(kRows * 2, W == 128 ? (kRows == 128 ? 2 : 4) : (kRows == 128 ? 3 : 6)) band_fwd_kernel(const __grid_constant__ BandParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = W / 16 + 1;
+  constexpr int kTv = kHalo * kRowBytes, kTq = 2 * kTv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
+  const int t0 = blockIdx.x * kRows, bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H, N = p.N;
+  const int n = min(p.num_atoms[b], N);
+  const uint32_t tile = (uint32_t)__cvta_generic_to_shared(smem);
+  const long long in0 = p.in.at(b, h, 0), act0 = p.act.at(b, h, 0);
+  if (t0 < n) {
+    load_band<kThreads>(tile, p.k + in0, p.in.token, t0 - kHalf, kHalo, n);
+    load_band<kThreads>(tile + kTq, p.q + in0, p.in.token, t0, kRows, n);
+    load_band<kThreads>(tile + kTv, p.v + in0, p.in.token, t0 - kHalf, kHalo, n);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+  const int i0 = t0 + warp * 16, row = i0 + row8;  // the lane's rows: row and row + 8
+  if (i0 >= N) return;
+  const FragBase fb(tile, lane);
+  float o[8][4], l[2] = {0.f, 0.f}, shift[2] = {0.f, 0.f};
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
+  if (i0 < n) {
+    uint32_t q[4][4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) load_a(q[ks], fb, kTq + warp * 16 * kRowBytes, 0, ks);
+    const float sc2 = p.scale * kLog2e;
+    // hidden pairs of chunk c: the two triangles, and keys outside the structure
+    auto logits = [&](float(&s)[2][4], int c) {
+      chunk_product(s, q, fb, (warp + c) * 16 * kRowBytes);
+      const int key0 = i0 - kHalf + 16 * c;
+      const bool ends = key0 < 0 || key0 + 16 > n;
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
+          bool seen = true;
+          if (c == 0) seen = rel >= r;
+          if (c == kChunks - 1) seen = rel < r;
+          if (ends) seen = seen && key0 + rel >= 0 && key0 + rel < n;
+          s[nt][e] = seen ? s[nt][e] * sc2 : -INFINITY;
+        }
+    };
+    for (bool exact = false;; exact = true) {
+      if (exact) {
+        float m[2] = {-INFINITY, -INFINITY};
+#pragma unroll 1
+        for (int c = 0; c < kChunks; ++c) {
+          float s[2][4];
+          logits(s, c);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m[e >> 1] = fmaxf(m[e >> 1], s[nt][e]);
+        }
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          m[hh] = fmaxf(m[hh], __shfl_xor_sync(0xffffffffu, m[hh], 1));
+          m[hh] = fmaxf(m[hh], __shfl_xor_sync(0xffffffffu, m[hh], 2));
+          shift[hh] = m[hh] > -INFINITY ? m[hh] : 0.f;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
+      }
+      float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
+        float s[2][4];
+        logits(s, c);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            float2 x = add2(make_float2(s[nt][2 * hh], s[nt][2 * hh + 1]), make_float2(-shift[hh], -shift[hh]));
+            x.x = fast_exp2(x.x);
+            x.y = fast_exp2(x.y);
+            l2[hh] = add2(l2[hh], x);
+            s[nt][2 * hh] = x.x, s[nt][2 * hh + 1] = x.y;
+          }
+        uint32_t pk[4];
+        pack_chunk(pk, s);
+        chunk_accumulate(o, pk, fb, kTv + (warp + c) * 16 * kRowBytes);
+      }
+      bool fine = true;
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        l[hh] = l2[hh].x + l2[hh].y;
+        quad_reduce(l[hh]);
+        if (row + 8 * hh < n) fine = fine && l[hh] >= kBandLow && l[hh] <= kBandHigh;
+      }
+      if (exact || __all_sync(0xffffffffu, fine)) break;
+    }
+  }
+  float inv[2];
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const bool have = row + 8 * hh < n && l[hh] != 0.f;
+    inv[hh] = have ? 1.f / l[hh] : 0.f;
+    if (quad == 0 && row + 8 * hh < N) p.lse[(size_t)bh * N + row + 8 * hh] = have ? (shift[hh] + log2f(l[hh])) * kLn2 : 0.f;
+  }
+  store_rows(p.out + act0, p.act.token, o, row, N, inv[0], inv[1]);
+}
+
+template <int W, int kRows>
+__global__ void __launch_bounds__(kRows * 2, kRows == 128 ? (W == 128 ? 1 : 2) : (W == 128 ? 2 : 3)) band_bwd_kernel(const __grid_constant__ BandParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = W / 16 + 1;
+  constexpr int kTk = kHalo * kRowBytes, kTv = 2 * kTk, kTg = 3 * kTk;  // q, k, v, grad_out
+  float* lse = reinterpret_cast<float*>(smem + 4 * kTk);  // of the halo rows, in the log2 domain
+  float* delta = lse + kHalo;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
+  const int t0 = blockIdx.x * kRows, first = t0 - kHalf, bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H, N = p.N;
+  const int n = min(p.num_atoms[b], N);
+  const uint32_t tile = (uint32_t)__cvta_generic_to_shared(smem);
+  const long long in0 = p.in.at(b, h, 0), act0 = p.act.at(b, h, 0);
+  if (t0 < n) {
+    load_band<kThreads>(tile + kTg, p.grad_out + act0, p.act.token, first, kHalo, n);
+    load_band<kThreads>(tile, p.q + in0, p.in.token, first, kHalo, n);
+    load_band<kThreads>(tile + kTk, p.k + in0, p.in.token, first, kHalo, n);
+    load_band<kThreads>(tile + kTv, p.v + in0, p.in.token, first, kHalo, n);
+    cp_async_commit();
+    // delta of the halo rows, eight lanes per row (their own loads of dO, while the copies are in flight), all loads first
+    constexpr int kSteps = kHalo * 8 / kThreads;
+    static_assert(kHalo * 8 % kThreads == 0, "whole steps");
+    uint4 x[kSteps], g[kSteps];
+    float ls[kSteps];
+    const int r0 = threadIdx.x >> 3, c = threadIdx.x & 7;
+#pragma unroll
+    for (int t = 0; t < kSteps; ++t) {
+      const int row = first + r0 + t * (kThreads / 8);
+      x[t] = g[t] = make_uint4(0u, 0u, 0u, 0u);
+      ls[t] = INFINITY;  // no weight for rows outside the structure
+      if (row >= 0 && row < n) {
+        x[t] = *reinterpret_cast<const uint4*>(p.out + act0 + row * p.act.token + c * 8);
+        g[t] = *reinterpret_cast<const uint4*>(p.grad_out + act0 + row * p.act.token + c * 8);
+        if (c == 0) ls[t] = p.lse[(size_t)bh * N + row] * kLog2e;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < kSteps; ++t) {
+      float d = fmaf(bf16_lo(x[t].x), bf16_lo(g[t].x), bf16_hi(x[t].x) * bf16_hi(g[t].x));
+      d = fmaf(bf16_lo(x[t].y), bf16_lo(g[t].y), fmaf(bf16_hi(x[t].y), bf16_hi(g[t].y), d));
+      d = fmaf(bf16_lo(x[t].z), bf16_lo(g[t].z), fmaf(bf16_hi(x[t].z), bf16_hi(g[t].z), d));
+      d = fmaf(bf16_lo(x[t].w), bf16_lo(g[t].w), fmaf(bf16_hi(x[t].w), bf16_hi(g[t].w), d));
+      d += __shfl_xor_sync(0xffffffffu, d, 1);
+      d += __shfl_xor_sync(0xffffffffu, d, 2);
+      d += __shfl_xor_sync(0xffffffffu, d, 4);
+      if (c == 0) {
+        delta[r0 + t * (kThreads / 8)] = d;
+        lse[r0 + t * (kThreads / 8)] = ls[t];
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+  const int i0 = t0 + warp * 16, row = i0 + row8;
+  if (i0 >= N) return;
+  const FragBase fb(tile, lane);
+  const int own = (warp * 16 + kHalf) * kRowBytes;  // the warp's rows inside the halo
+  const float sc2 = p.scale * kLog2e;
+  uint32_t a[4][4], g[4][4];
+  float acc0[8][4], acc1[8][4];
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc0[t][e] = 0.f;
+  if (i0 < n) {  // ---- the rows as queries.  (Keys outside the structure have zero rows: whatever weight they get meets zeros.)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) load_a(a[ks], fb, own, 0, ks), load_a(g[ks], fb, kTg + own, 0, ks);
+    const int r0 = warp * 16 + kHalf + row8;
+    const float la = lse[r0], lb = lse[r0 + 8], da = delta[r0], db = delta[r0 + 8];
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+      const int at = (warp + c) * 16 * kRowBytes;
+      float s[2][4], dp[2][4];
+      chunk_product(s, a, fb, kTk + at);
+      chunk_product(dp, g, fb, kTv + at);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
+          // a logit of 0 against zero rows may give a huge weight where the row's log-sum-exp is very negative: bounded, so
+          // that it stays finite and 0 . weight = 0
+          float pr = fast_exp2(fminf(fmaf(s[nt][e], sc2, -(e < 2 ? la : lb)), 100.f));
+          if (c == 0 && rel < r) pr = 0.f;
+          if (c == kChunks - 1 && rel >= r) pr = 0.f;
+          s[nt][e] = pr * (dp[nt][e] - (e < 2 ? da : db)) * p.scale;
+        }
+      uint32_t pk[4];
+      pack_chunk(pk, s);
+      chunk_accumulate(acc0, pk, fb, kTk + at);
+    }
+  }
+  store_rows(p.dq + in0, p.in.token, acc0, row, N, row < n ? 1.f : 0.f, row + 8 < n ? 1.f : 0.f);
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc0[t][e] = acc1[t][e] = 0.f;
+  if (i0 < n) {  // ---- the rows as keys: key j is seen by queries j - w/2 + 1 .. j + w/2
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) load_a(a[ks], fb, kTk + own, 0, ks), load_a(g[ks], fb, kTv + own, 0, ks);
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+      const int at = (warp + c) * 16 * kRowBytes;
+      float s[2][4], dp[2][4];
+      chunk_product(s, a, fb, at);
+      chunk_product(dp, g, fb, kTg + at);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const int q0 = (warp + c) * 16 + nt * 8 + 2 * quad;
+        const float2 l = *reinterpret_cast<const float2*>(&lse[q0]), d = *reinterpret_cast<const float2*>(&delta[q0]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
+          float pr = fast_exp2(fmaf(s[nt][e], sc2, -((e & 1) ? l.y : l.x)));
+          if (c == 0 && rel <= r) pr = 0.f;
+          if (c == kChunks - 1 && rel > r) pr = 0.f;
+          s[nt][e] = pr;
+          dp[nt][e] = pr * (dp[nt][e] - ((e & 1) ? d.y : d.x)) * p.scale;
+        }
+      }
+      uint32_t pk[4];
+      pack_chunk(pk, s);
+      chunk_accumulate(acc1, pk, fb, kTg + at);  // dv += P^T dO
+      pack_chunk(pk, dp);
+      chunk_accumulate(acc0, pk, fb, at);        // dk += dS^T Q
+    }
+  }
+  const bool lo = row < n, hi = row + 8 < n;
+#pragma unroll
+  for (int t = 0; t < 8; ++t)  // (selected, not multiplied: a row beyond the structure may have met an infinite weight)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (!(e < 2 ? lo : hi)) acc0[t][e] = acc1[t][e] = 0.f;
+  store_rows(p.dk + in0, p.in.token, acc0, row, N, 1.f, 1.f);
+  store_rows(p.dv + in0, p.in.token, acc1, row, N, 1.f, 1.f);
+}
+
+template <int W, int kRows>
+int launch_band(const BandParams& p, int BH, bool backward, cudaStream_t s) {
+  constexpr int halo = (kRows + W) * kRowBytes;
+  const int bytes = backward ? 4 * halo + (kRows + W) * 8 : 2 * halo + kRows * kRowBytes;
+  auto kernel = backward ? band_bwd_kernel<W, kRows> : band_fwd_kernel<W, kRows>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(band_attn_kernel)");
+  kernel<<<dim3((p.N + kRows - 1) / kRows, BH), kRows * 2, bytes, s>>>(p);
+  MF_CHECK_LAUNCH("band_attn_kernel");
+  return MF_OK;
+}
+
+}  // namespace
+
+// Windows whose chunks are whole, structures long enough that a tile is not mostly halo; shorter ones (a trunk's molecules)
+// stay on the 32-row walk.
+bool band_attn_applies(const MfSparseAttnArgs& a) {
+  return a.dtype == MF_DTYPE_BF16 && a.head_dim == 64 && (a.window == 32 || a.window == 64 || a.window == 128) && a.tokens >= 96;
+}
+
+int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream) {
+  BandParams p{};
+  p.q = static_cast<const __nv_bfloat16*>(a.q);
+  p.k = static_cast<const __nv_bfloat16*>(a.k);
+  p.v = static_cast<const __nv_bfloat16*>(a.v);
+  p.grad_out = static_cast<const __nv_bfloat16*>(a.grad_out);
+  p.num_atoms = a.num_atoms;
+  p.out = static_cast<__nv_bfloat16*>(a.out);
+  p.lse = a.lse;
+  p.dq = static_cast<__nv_bfloat16*>(a.dq);
+  p.dk = static_cast<__nv_bfloat16*>(a.dk);
+  p.dv = static_cast<__nv_bfloat16*>(a.dv);
+  p.H = a.heads, p.N = a.tokens, p.scale = a.scale;
+  p.in = layouts ? layouts[0] : contiguous_rows(a.heads, a.tokens);
+  p.act = layouts ? layouts[1] : contiguous_rows(a.heads, a.tokens);
+  const int BH = a.batch * a.heads;
+  // 128-row tiles re-read half as much halo; 64-row ones spread a small call over twice as many CTAs
+  const bool wide = (long long)BH * ((a.tokens + 127) / 128) >= 592;
+  switch (a.window) {
+    case 32: return wide ? launch_band<32, 128>(p, BH, backward, stream) : launch_band<32, 64>(p, BH, backward, stream);
+    case 64: return wide ? launch_band<64, 128>(p, BH, backward, stream) : launch_band<64, 64>(p, BH, backward, stream);
+    default: return wide ? launch_band<128, 128>(p, BH, backward, stream) : launch_band<128, 64>(p, BH, backward, stream);
+  }
+}
+
+}  // namespace mf

@@ -355,6 +355,7 @@ int run_sparse(const MfSparseAttnArgs* a, bool backward, void* stream, const cha
                  "aligned tensors and the driver's tensor-map encoder", name);
     const bool tc = a->backend == MF_SPARSE_BACKEND_TCGEN05 ||
                     (a->backend == MF_SPARSE_BACKEND_AUTO && fits && kRadius && a->tokens >= 256);
+    if (!kRadius && a->backend == MF_SPARSE_BACKEND_AUTO && band_attn_applies(*a)) return band_attn(*a, nullptr, backward, s);
     if (tc) return backward ? sparse_attn_sm100_bwd(*a, kRadius, s) : sparse_attn_sm100_fwd(*a, kRadius, s);
     return backward ? sparse_attn_mma_bwd(*a, kRadius, s) : sparse_attn_mma_fwd(*a, kRadius, s);
   }
@@ -433,6 +434,10 @@ int run_local_packed(const MfLocalAttnPackedArgs* a, bool backward, void* stream
   }
   const RowLayout in{(long long)a->tokens * 3 * hd, (long long)a->head_dim, 3 * hd};  // a group's rows in (B,N,3,H,D)
   const RowLayout act{(long long)a->tokens * hd, (long long)a->head_dim, hd};          // (B,N,H,D)
+  if (band_attn_applies(s)) {
+    const RowLayout layouts[2] = {in, act};
+    return band_attn(s, layouts, backward, static_cast<cudaStream_t>(stream));
+  }
   return local_attn_mma_layouts(s, in, act, backward, static_cast<cudaStream_t>(stream));
 }
 }  // namespace

@@ -18,6 +18,10 @@ struct RowLayout;
 int local_attn_mma_layouts(const MfSparseAttnArgs& a, const RowLayout& in, const RowLayout& act, bool backward,
                            cudaStream_t stream);
 
+// Bands of 32, 64 or 128 tokens at head_dim 64 (band_attn.cu); `layouts` as above, or null for contiguous rows.
+bool band_attn_applies(const MfSparseAttnArgs& a);
+int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream);
+
 // ---- warp-level tensor-core helpers (m16n8k16, bf16 operands, fp32 accumulate) ---------------------------
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem_addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
