@@ -63,16 +63,19 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
   const float* sc = scale + (size_t)b * C;
   const int nvec = C >> 3;
   const float inv_c = 1.f / (float)C;
-  for (int n = warp; n < N; n += kAdaWarps) {
+  // a warp's rows are spread over gridDim.y CTAs: with a molecule per CTA, a small batch left the chip to its latency
+  for (int n = blockIdx.y * kAdaWarps + warp; n < N; n += kAdaWarps * gridDim.y) {
     const size_t row = (size_t)b * N + n;
     const TX* xr = x + row * C;
-    float xv[VEC][8];
+    float xv[VEC][8], scv[VEC][8], shv[VEC][8];
     float s = 0.f;
 #pragma unroll
     for (int t = 0; t < VEC; ++t) {
       const int v = lane + 32 * t;
       if (v < nvec) {
         ld8<TX>(xr + 8 * v, xv[t]);
+        ld8<float>(sc + 8 * v, scv[t]);
+        ld8<float>(sh + 8 * v, shv[t]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) s += xv[t][e];
       }
@@ -94,11 +97,9 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
     for (int t = 0; t < VEC; ++t) {
       const int v = lane + 32 * t;
       if (v < nvec) {
-        float scv[8], shv[8], out[8];
-        ld8<float>(sc + 8 * v, scv);
-        ld8<float>(sh + 8 * v, shv);
+        float out[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) out[e] = fmaf((xv[t][e] - mean) * rstd, 1.f + scv[e], shv[e]);
+        for (int e = 0; e < 8; ++e) out[e] = fmaf((xv[t][e] - mean) * rstd, 1.f + scv[t][e], shv[t][e]);
         st8<TH>(h + row * C + 8 * v, out);
       }
     }
@@ -323,9 +324,12 @@ extern "C" int mf_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* s
   MF_CHECK_ARG(x && shift && scale && h && mean && rstd, "mf_ln_modulate_fwd: null pointer argument");
   MF_CHECK_ALIGNED("mf_ln_modulate_fwd", x, shift, scale, h);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // enough CTAs for four per SM, at most one row per warp
+  const int rows = (tokens + kAdaWarps - 1) / kAdaWarps, wanted = (592 + batch - 1) / batch;
+  const dim3 grid(batch, rows < wanted ? (rows > 0 ? rows : 1) : wanted);
   MF_ADA_DISPATCH(x_dtype, h_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
-                             (ln_modulate_fwd_kernel<TX, TH, VEC><<<batch, kAdaWarps * 32, 0, s>>>(
+                             (ln_modulate_fwd_kernel<TX, TH, VEC><<<grid, kAdaWarps * 32, 0, s>>>(
                                  static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
                                  rstd))));
   MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");

@@ -279,7 +279,7 @@ __device__ __forceinline__ void small_fwd_rows(const SmallFwdParams& p, SmallFwd
 }
 
 template <bool kBias, int kWarps>
-__global__ void __launch_bounds__(32 * kWarps, (kBias ? 12 : 14) / kWarps) simplicial_small_fwd_kernel(const __grid_constant__ SmallFwdParams p) {
+__global__ void __launch_bounds__(32 * kWarps, kBias ? 12 / kWarps : (kWarps == 4 ? 4 : 14 / kWarps)) simplicial_small_fwd_kernel(const __grid_constant__ SmallFwdParams p) {
   __shared__ SmallFwdShared<kBias> sm;
   const int tid = threadIdx.x, lane = tid & 31;
   const int N = p.N, bh = blockIdx.x, b = bh / p.H, h = bh % p.H;

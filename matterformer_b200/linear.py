@@ -10,7 +10,7 @@ gradient, fixed order of additions).  The GEMMs themselves stay library calls (c
 """
 from __future__ import annotations
 
-from typing import Iterable, Optional
+from typing import Iterable, Optional, Sequence
 
 import torch
 import torch.nn.functional as F
@@ -54,6 +54,10 @@ def bf16_copy(p: torch.Tensor) -> torch.Tensor:
     return copy
 
 
+def has_bf16_copy(p: torch.Tensor) -> bool:
+    return getattr(p, _SHADOW, None) is not None
+
+
 def refresh_bf16_copies(params: Iterable[torch.Tensor], *, force: bool = False) -> None:
     """Bring the bf16 copies of ``params`` up to date with one multi-tensor copy.  ``force`` copies even when the version
     counters say nothing changed: a step captured in a CUDA graph must contain the copy, because a replay updates the
@@ -75,6 +79,80 @@ def refresh_bf16_copies(params: Iterable[torch.Tensor], *, force: bool = False) 
     if stale_dst:
         with torch.no_grad():
             torch._foreach_copy_(stale_dst, stale_src)
+
+
+_REFRESH_IN_CAPTURE = True
+
+
+class no_refresh_in_capture:
+    """For a captured evaluation whose owner brings the bf16 copies up to date itself, before each replay."""
+
+    def __enter__(self):
+        global _REFRESH_IN_CAPTURE
+        self._before, _REFRESH_IN_CAPTURE = _REFRESH_IN_CAPTURE, False
+
+    def __exit__(self, *exc):
+        global _REFRESH_IN_CAPTURE
+        _REFRESH_IN_CAPTURE = self._before
+
+
+def refresh_must_be_captured() -> bool:
+    return _REFRESH_IN_CAPTURE and torch.cuda.is_current_stream_capturing()
+
+
+def stacked_bf16_copies(params: Sequence[torch.Tensor], stack: Optional[torch.Tensor]) -> torch.Tensor:
+    """The bf16 copies of equally shaped parameters as one contiguous tensor, (len(params) * rows, ...): each parameter's
+    copy is a view of it, so refreshing the copies refreshes the stack.  ``stack`` is returned as it is while it still holds
+    them.  Freshly placed copies are filled by the next :func:`refresh_bf16_copies`, or here where that does not follow."""
+    rows, first = params[0].shape[0], params[0]
+    if stack is not None and stack.device == first.device:
+        for i, p in enumerate(params):
+            entry = getattr(p, _SHADOW, None)
+            if entry is None or entry[0].data_ptr() != stack[i * rows :].data_ptr() or entry[0].shape != p.shape:
+                break
+        else:
+            return stack
+    with torch.no_grad():
+        stack = torch.cat([p.detach().to(torch.bfloat16) for p in params])
+    for i, p in enumerate(params):
+        setattr(p, _SHADOW, (stack[i * rows : (i + 1) * rows], p._version))
+    return stack
+
+
+class _StackedModulation(torch.autograd.Function):
+    """The adaptive-LayerNorm modulations of all layers from the one conditioning vector they share: one GEMM forward, three
+    products backward, instead of those per layer.  ``params``: the layers' weights, then their biases."""
+
+    @staticmethod
+    def forward(ctx, x, weights, biases, layers, *params):
+        with torch.autocast("cuda", enabled=False):
+            mod = F.linear(x, weights, biases)
+        B, C = x.shape[0], mod.shape[1] // (6 * layers)
+        out = torch.empty((6 * layers, B, C), device=x.device, dtype=torch.float32)
+        out.copy_(mod.view(B, 6 * layers, C).transpose(0, 1))
+        ctx.save_for_backward(x, weights)
+        ctx.layers = layers
+        return tuple(out.unbind(0))
+
+    @staticmethod
+    def backward(ctx, *grads):
+        x, weights = ctx.saved_tensors
+        like = next(g for g in grads if g is not None)
+        g = torch.stack([t if t is not None else torch.zeros_like(like) for t in grads], dim=1)  # (B, 6 L, C) fp32
+        g = g.reshape(g.shape[0], -1).to(torch.bfloat16)
+        with torch.autocast("cuda", enabled=False):
+            dx = torch.mm(g, weights) if ctx.needs_input_grad[0] else None
+            dw = _mm_f32(g.t(), x)
+        db = column_sums(g) if column_sums_applies(g) else g.sum(0, dtype=torch.float32)
+        return (dx, None, None, None, *dw.chunk(ctx.layers), *db.chunk(ctx.layers))
+
+
+def stacked_modulation(x: torch.Tensor, weights: torch.Tensor, biases: torch.Tensor, params: Sequence[torch.Tensor],
+                       layers: int) -> list:  # fmt: skip
+    """Per layer the six fp32 (B, C) tensors ``shift_a, scale_a, gate_a, shift_m, scale_m, gate_m``; ``weights`` / ``biases``
+    are the stacked bf16 copies of ``params``."""
+    out = _StackedModulation.apply(x, weights, biases, layers, *params)
+    return [out[6 * i : 6 * i + 6] for i in range(layers)]
 
 
 _MM_OUT_DTYPE = True  # torch.mm(..., out_dtype=) exists; cleared on the first refusal

@@ -30,7 +30,8 @@ from torch import nn
 from . import fused
 from .fused import (fused_applies, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
                     split_modulation)
-from .linear import linear_bf16, linear_gelu_bf16, refresh_bf16_copies
+from .linear import (linear_bf16, linear_gelu_bf16, refresh_bf16_copies, refresh_must_be_captured, stacked_bf16_copies,
+                     stacked_modulation)  # fmt: skip
 from .simplicial import (normalize_simplicial_precision, packed_projection_applies, simplicial_attention_cuda,
                          simplicial_attention_packed)  # fmt: skip
 
@@ -258,7 +259,8 @@ class RegularAttention(nn.Module):
         return self.attn.out_proj(merge_heads(core))
 
     def forward(self, x: torch.Tensor, *, key_padding_mask: Optional[torch.Tensor] = None,
-                sparse_plan: Optional[SparseAttentionPlan] = None) -> torch.Tensor:  # fmt: skip
+                sparse_plan: Optional[SparseAttentionPlan] = None, num_atoms: Optional[torch.Tensor] = None) -> torch.Tensor:  # fmt: skip
+        """``num_atoms``: the (B,) int32 counts of real tokens when the caller has already formed them."""
         if sparse_plan is not None:
             if not x.is_cuda:
                 raise RuntimeError("sparse attention plans need CUDA tensors (there is no CPU fallback)")
@@ -273,7 +275,8 @@ class RegularAttention(nn.Module):
         B, N, C = x.shape
         H = self.attn.num_heads
         qkv = linear_bf16(x, self.attn.in_proj_weight, self.attn.in_proj_bias).to(torch.bfloat16)
-        num_atoms = (~key_padding_mask).sum(dim=1).to(torch.int32)
+        if num_atoms is None:
+            num_atoms = (~key_padding_mask).sum(dim=1).to(torch.int32)
         # with at most 32 tokens the window-64 band covers every real token: dense attention, straight on the projection
         core = local_window_attention_packed(qkv, H, num_atoms, window=64)
         return linear_bf16(core, self.attn.out_proj.weight, self.attn.out_proj.bias)
@@ -334,14 +337,18 @@ class AdaLNBlock(nn.Module):
         self.fused_elementwise = True  # CUDA fp32 residual stream: fused norm+modulate and gated-residual kernels
 
     def forward(self, x, cond_emb, *, pad_mask=None, simplicial_attention_mask=None, sparse_plan=None,
-                zero_padding: bool = False, cond_act=None):
+                zero_padding: bool = False, cond_act=None, modulation=None, num_atoms=None):
         """``zero_padding``: return the block's output with its padded rows cleared (the ``masked_fill`` the trunk
         applies before the next block), folded into the last fused pass when the fused kernels run.  ``cond_act``:
-        ``SiLU(cond_emb)`` when the caller has already formed it (it is the same for every block of a trunk)."""
-        mod = linear_bf16(cond_act if cond_act is not None else self.ada_ln[0](cond_emb), self.ada_ln[-1].weight,
-                          self.ada_ln[-1].bias)  # fmt: skip
+        ``SiLU(cond_emb)`` when the caller has already formed it (it is the same for every block of a trunk).
+        ``modulation``: the six modulation tensors, formed by the trunk for all its blocks at once; ``num_atoms``: counts of
+        real tokens for the attention layer."""
         fused = self.fused_elementwise and fused_applies(x)
-        shift_a, scale_a, gate_a, shift_m, scale_m, gate_m = split_modulation(mod) if fused else mod.chunk(6, dim=-1)
+        mod = None if modulation is not None else linear_bf16(cond_act if cond_act is not None else self.ada_ln[0](cond_emb), self.ada_ln[-1].weight,
+                          self.ada_ln[-1].bias)  # fmt: skip
+        if modulation is None:
+            modulation = split_modulation(mod) if fused else mod.chunk(6, dim=-1)
+        shift_a, scale_a, gate_a, shift_m, scale_m, gate_m = modulation
         if fused:
             # one pass each for norm + modulate and for the gated residual; under bf16 autocast the modulated
             # activations are written in bf16, which is what the Linear layers that consume them cast to anyway
@@ -351,7 +358,7 @@ class AdaLNBlock(nn.Module):
         else:
             h = _modulate(self.norm1(x), shift_a, scale_a)
         if self.attn_type == "mha":
-            attn_out = self.attn(h, key_padding_mask=pad_mask, sparse_plan=sparse_plan)
+            attn_out = self.attn(h, key_padding_mask=pad_mask, sparse_plan=sparse_plan, num_atoms=num_atoms)
         else:
             attn_out = self.attn(h, key_padding_mask=pad_mask, attention_mask=simplicial_attention_mask)
         if fused:
@@ -399,12 +406,20 @@ class TransformerTrunk(nn.Module):
         b, n, _ = x.shape
         if pad_mask is not None:
             pad_mask = pad_mask.bool()
-        if x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16:
+        bf16 = x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
+        layers = [block.ada_ln[-1] for block in self.blocks]
+        stacked = bf16 and fused_applies(x) and cond_emb.ndim == 2 and all(
+            block.fused_elementwise and m.weight.dtype == torch.float32 and m.bias is not None for block, m in zip(self.blocks, layers)
+        )
+        if stacked:
+            self._modulation_w16 = stacked_bf16_copies([m.weight for m in layers], getattr(self, "_modulation_w16", None))
+            self._modulation_b16 = stacked_bf16_copies([m.bias for m in layers], getattr(self, "_modulation_b16", None))
+        if bf16:
             # the bf16 copies the blocks' Linear layers compute with: all of them in one multi-tensor copy; a step that is
             # being captured into a CUDA graph always contains the copy (its replays change the parameters)
-            refresh_bf16_copies(self._linear_parameters(), force=torch.cuda.is_current_stream_capturing())
+            refresh_bf16_copies(self._linear_parameters(), force=refresh_must_be_captured())
         sim_mask = SimplicialAttentionMask.from_key_padding_mask(pad_mask, batch_size=b, num_tokens=n, device=x.device)
-        if self.emit_pair_valid:
+        if self.emit_pair_valid and not x.is_cuda:  # (the kernels take the padding from the key mask: the same pairs)
             v = sim_mask.pair_key_valid
             sim_mask = SimplicialAttentionMask(sim_mask.query_valid, v, v[:, :, None] & v[:, None, :])
         # the reference clears the padded rows before every block (transformer.py, the loop of TransformerTrunk.forward);
@@ -414,11 +429,16 @@ class TransformerTrunk(nn.Module):
             x = x.masked_fill(pad_mask[..., None], 0.0)
         # every block starts its modulation with the same SiLU(cond_emb): formed (and cast for the bf16 Linear) once
         cond_act = F.silu(cond_emb)
-        if x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16:
+        if bf16:
             cond_act = cond_act.to(torch.bfloat16)
-        for block in self.blocks:
+        modulation = [None] * len(self.blocks)
+        if stacked:
+            modulation = stacked_modulation(cond_act, self._modulation_w16, self._modulation_b16,
+                                            [m.weight for m in layers] + [m.bias for m in layers], len(layers))  # fmt: skip
+        num_atoms = (~pad_mask).sum(dim=1).to(torch.int32) if x.is_cuda and pad_mask is not None else None
+        for block, six in zip(self.blocks, modulation):
             x = block(x, cond_emb, pad_mask=pad_mask, simplicial_attention_mask=sim_mask, sparse_plan=sparse_plan,
-                      zero_padding=pad_mask is not None, cond_act=cond_act)
+                      zero_padding=pad_mask is not None, cond_act=cond_act, modulation=six, num_atoms=num_atoms)
         x = layer_norm(x, self.norm_out)
         if pad_mask is not None:
             x = x.masked_fill(pad_mask[..., None], 0.0)
