@@ -114,6 +114,11 @@ bool uses_small_kernels(const Args* a) {
   return (a->backend == MF_BACKEND_AUTO || a->backend == MF_BACKEND_TCGEN05_TILES) && a->tokens <= kSmallTokens;
 }
 
+// Larger molecules: the forward pass runs on the warp-level kernel, unless a tcgen05 family is asked for.
+inline bool uses_warp_forward(const MfSimplicialFwdArgs* a) {
+  return a->backend == MF_BACKEND_AUTO && a->tokens > kSmallTokens;
+}
+
 // fp32 molecules of at most 64 tokens (two keys per lane would not fit the registers), plain attention, aligned rows.
 template <typename Args>
 bool uses_f32_kernels(const Args* a) {
@@ -143,7 +148,7 @@ extern "C" int mf_feature_flags(void) { return tensor_maps_available() ? MF_FEAT
 extern "C" size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* a) {
   if (!a) return 0;
   int rc;
-  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd") && !uses_small_kernels(a)) return simplicial_sm100_fwd_workspace_bytes(*a);
+  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd") && !uses_small_kernels(a) && !uses_warp_forward(a)) return simplicial_sm100_fwd_workspace_bytes(*a);
   return 0;
 }
 
@@ -201,6 +206,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
   if (!tc) return uses_f32_kernels(a) ? simplicial_f32_fwd(*a, s) : simplicial_generic_fwd(*a, s);
   if (uses_small_kernels(a))
     return a->angle_left || a->message_left ? simplicial_small_res_fwd(*a, s) : simplicial_small_fwd(*a, nullptr, s);
+  if (uses_warp_forward(a)) return simplicial_warp_fwd(*a, s);
   return uses_tile_kernels(a) ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
 }
 

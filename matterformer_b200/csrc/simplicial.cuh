@@ -35,6 +35,9 @@ int simplicial_small_fwd(const MfSimplicialFwdArgs& a, const TileLayouts* layout
 int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
 int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);  // with the low-rank residuals
 
+// warp-level forward kernel for 33 to 192 tokens (simplicial_warp_fwd.cu)
+int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
+
 // row-packed tcgen05 kernels (simplicial_rows_fwd.cu, simplicial_rows_bwd.cu); same problems as the kernels above
 int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);

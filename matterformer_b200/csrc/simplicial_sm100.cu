@@ -712,7 +712,7 @@ extern "C" int mf_simplicial_fwd_noalloc(const MfSimplicialFwdArgs* args, void* 
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
   // (kernels that keep no status word leave the one of an earlier call behind)
-  if (a.tokens <= kSmallTokens && (e = cudaMemsetAsync(scratch, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream))) != cudaSuccess)
+  if (mf_simplicial_fwd_workspace_bytes(&a) == 0 && (e = cudaMemsetAsync(scratch, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream))) != cudaSuccess)
     return cuda_error(e, "mf_simplicial_fwd_noalloc: cudaMemsetAsync");
   // Same validation and launch as the allocating entry point; the status word at the start of the scratch is
   // cleared by the first kernel of every call, nothing else has to start at zero.
