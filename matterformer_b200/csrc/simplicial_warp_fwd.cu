@@ -5,6 +5,8 @@
 // warp keeps the block row's K1 o q_i and W^T in registers and needs no barrier and no exchange with other warps.  The
 // softmax shift is 0 unless the query's sum leaves 2^-60 .. 2^60, in which case it is done again with its exact maximum.
 // Blocks in which every pair counts take no masks.
+#include <type_traits>
+
 #include "common.cuh"
 #include "simplicial.cuh"
 #include "simplicial_warp.cuh"
@@ -50,16 +52,15 @@ struct QueryState {
   float m;  // exact pass: running maximum
 };
 
-template <bool kBias, bool kMaxPass>
+template <bool kBias, bool kMaxPass, int MT>
 __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdHeader& hd, const FragBase& fb, int tile_bytes,
                                           const uint32_t (&qf)[8], int bh, int i, int jb, int n, float shift, QueryState<kBias>& st) {
   const int lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
   const int tk2 = tile_bytes, tv1 = 2 * tile_bytes, tv2 = 3 * tile_bytes;
   const int nb = (n + 31) >> 5;
-  const bool two = n - 32 * jb > 16;  // both 16-row halves hold keys
-  uint32_t a[2][4][4];
+  uint32_t a[MT][4][4];
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       load_a(a[mt][ks], fb, jb * 32 * kRowBytes, mt, ks);
@@ -68,38 +69,38 @@ __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdH
       a[mt][ks][2] = mul_bf16x2(a[mt][ks][2], qf[2 * ks + 1]);
       a[mt][ks][3] = mul_bf16x2(a[mt][ks][3], qf[2 * ks + 1]);
     }
-  float ur[2][2], g = 0.f;
+  float ur[MT][2], g = 0.f;
   const size_t row = ((size_t)bh * p.N + i) * p.N;
   if constexpr (kBias) {
     g = p.gate[(size_t)bh * p.N + i];
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int j = 32 * jb + 16 * mt + 8 * hh + row8;
         ur[mt][hh] = j < n ? p.u[row + j] : 0.f;
       }
   }
-  float w[4][4][4];  // W^T: channels 16 dt x j tiles
+  float w[4][2 * MT][4];  // W^T: channels 16 dt x j tiles
 #pragma unroll
   for (int dt = 0; dt < 4; ++dt)
 #pragma unroll
-    for (int jt = 0; jt < 4; ++jt)
+    for (int jt = 0; jt < 2 * MT; ++jt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) w[dt][jt][e] = 0.f;
-#pragma unroll 1
-  for (int kb = 0; kb < nb; ++kb) {
+  auto block = [&](int kb, auto tiles) {  // 32 x 32, or 16 wide where the molecule ends in the first half
+    constexpr int NT = decltype(tiles)::value;
     const bool full = hd.full[jb][kb];
     const int at2 = kb * 32 * kRowBytes;
-    float s[2][4][4];
+    float s[MT][NT][4];
 #pragma unroll
     for (int kp = 0; kp < 2; ++kp)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
+      for (int nt = 0; nt < NT; ++nt) {
         uint32_t b[4];
         load_b(b, fb, tk2 + at2, nt, kp);
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
+        for (int mt = 0; mt < MT; ++mt) {
           if (kp == 0) mma16_first(s[mt][nt], a[mt][0], b[0], b[1]);
           else mma16(s[mt][nt], a[mt][2], b[0], b[1]);
           mma16(s[mt][nt], a[mt][2 * kp + 1], b[2], b[3]);
@@ -107,11 +108,11 @@ __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdH
       }
     if constexpr (kBias) {
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
+      for (int nt = 0; nt < NT; ++nt) {
         const int k = 32 * kb + 8 * nt + 2 * quad;
         const float va = k < n ? p.v_bias[row + k] : 0.f, vb = k + 1 < n ? p.v_bias[row + k + 1] : 0.f;
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
             const int j = 32 * jb + 16 * mt + 8 * hh + row8;
@@ -124,12 +125,12 @@ __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdH
     }
     if (!full) {
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const uint32_t vis = hd.visible[32 * jb + 16 * mt + 8 * hh + row8][kb] >> (2 * quad);
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt) {
+          for (int nt = 0; nt < NT; ++nt) {
             if (!((vis >> (8 * nt)) & 1u)) s[mt][nt][2 * hh] = -INFINITY;
             if (!((vis >> (8 * nt + 1)) & 1u)) s[mt][nt][2 * hh + 1] = -INFINITY;
           }
@@ -137,21 +138,21 @@ __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdH
     }
     if constexpr (kMaxPass) {
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int e = 0; e < 4; ++e) st.m = fmaxf(st.m, s[mt][nt][e]);
-      continue;
+      return;
     }
-    uint32_t pk[2][4][2];
+    uint32_t pk[MT][NT][2];
     const float2 le = make_float2(kLog2e, kLog2e), c = make_float2(-shift, -shift);
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
+        for (int nt = 0; nt < NT; ++nt) {
           float2 x = fma2(make_float2(s[mt][nt][2 * hh], s[mt][nt][2 * hh + 1]), le, c);
           x.x = fast_exp2(x.x);
           x.y = fast_exp2(x.y);
@@ -161,20 +162,23 @@ __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdH
 #pragma unroll
     for (int dt = 0; dt < 4; ++dt)
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
+      for (int ks = 0; ks < NT / 2; ++ks) {
         uint32_t v[4];
         load_t(v, fb, tv2 + at2, dt, ks);
 #pragma unroll
-        for (int jt = 0; jt < 4; ++jt)
-          if (jt < 2 || two) mma16(w[dt][jt], v, pk[jt >> 1][2 * ks][jt & 1], pk[jt >> 1][2 * ks + 1][jt & 1]);
+        for (int jt = 0; jt < 2 * MT; ++jt) mma16(w[dt][jt], v, pk[jt >> 1][2 * ks][jt & 1], pk[jt >> 1][2 * ks + 1][jt & 1]);
       }
-  }
+  };
+  const int last = n - 32 * (nb - 1);
+#pragma unroll 1
+  for (int kb = 0; kb < nb - (last <= 16); ++kb) block(kb, std::integral_constant<int, 4>{});
+  if (last <= 16) block(nb - 1, std::integral_constant<int, 2>{});
   if constexpr (!kMaxPass) {
 #pragma unroll
     for (int dt = 0; dt < 4; ++dt) {
       float2 lo = make_float2(0.f, 0.f), hi = lo;
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         uint32_t v[4];
         load_t(v, fb, tv1 + jb * 32 * kRowBytes, dt, mt);
 #pragma unroll
@@ -252,6 +256,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) simplicial_warp_fwd_kernel(con
   __syncthreads();
 
   const FragBase fb(tile0, lane);
+  const int half = n - 32 * (nb - 1) <= 16;  // the last block row holds keys in its first 16 rows only
   for (int i = i0 + warp; i < min(i1, nq); i += kFwdWarps) {
     const bool valid = (hd.qmask[i >> 5] >> (i & 31)) & 1u;
     QueryState<kBias> st;
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) simplicial_warp_fwd_kernel(con
         if (exact) {
           st.m = -INFINITY;
 #pragma unroll 1
-          for (int jb = 0; jb < nb; ++jb) block_row<kBias, true>(p, hd, fb, tile_bytes, qf, bh, i, jb, n, 0.f, st);
+          for (int jb = 0; jb < nb; ++jb) block_row<kBias, true, 2>(p, hd, fb, tile_bytes, qf, bh, i, jb, n, 0.f, st);
           const float m = warp_max(st.m);
           shift = m > -INFINITY ? m * kLog2e : 0.f;
         }
@@ -273,7 +278,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) simplicial_warp_fwd_kernel(con
 #pragma unroll
         for (int e = 0; e < 8; ++e) st.o[e] = 0.f;
 #pragma unroll 1
-        for (int jb = 0; jb < nb; ++jb) block_row<kBias, false>(p, hd, fb, tile_bytes, qf, bh, i, jb, n, shift, st);
+        for (int jb = 0; jb < nb - half; ++jb) block_row<kBias, false, 2>(p, hd, fb, tile_bytes, qf, bh, i, jb, n, shift, st);
+        if (half) block_row<kBias, false, 1>(p, hd, fb, tile_bytes, qf, bh, i, nb - 1, n, shift, st);
         l = warp_sum(st.l.x + st.l.y);
         if (exact || (l >= kWarpLow && l <= kWarpHigh)) break;
       }
