@@ -31,6 +31,7 @@ struct WarpFwdParams {
   float* lse;
   __nv_bfloat16* out_cast;
   int H, N, chunk;  // chunk: queries per CTA
+  int even;         // rows of v_bias and w start on 8-byte boundaries
 };
 
 constexpr int kFwdWarps = 12;                  // 168 registers each fill the register file
@@ -107,20 +108,39 @@ __device__ __forceinline__ void block_row(const WarpFwdParams& p, const WarpFwdH
         }
       }
     if constexpr (kBias) {
+      const int k0 = 32 * kb + 2 * quad, j0 = 32 * jb + row8;
+      const float* vr = p.v_bias + row + k0;
+      const float* wr = p.w + ((size_t)bh * p.N + j0) * p.N + k0;
+      if (full && p.even) {  // whole pairs of keys on 8-byte boundaries
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const int k = 32 * kb + 8 * nt + 2 * quad;
-        const float va = k < n ? p.v_bias[row + k] : 0.f, vb = k + 1 < n ? p.v_bias[row + k + 1] : 0.f;
+        for (int nt = 0; nt < NT; ++nt) {
+          const float2 v = *reinterpret_cast<const float2*>(vr + 8 * nt);
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+          for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int j = 32 * jb + 16 * mt + 8 * hh + row8;
-            const float* wr = p.w + ((size_t)bh * p.N + j) * p.N + k;
-            const float wa = (j < n && k < n) ? wr[0] : 0.f, wb = (j < n && k + 1 < n) ? wr[1] : 0.f;
-            s[mt][nt][2 * hh] = fmaf(g, (ur[mt][hh] + va) + wa, s[mt][nt][2 * hh]);
-            s[mt][nt][2 * hh + 1] = fmaf(g, (ur[mt][hh] + vb) + wb, s[mt][nt][2 * hh + 1]);
-          }
+            for (int hh = 0; hh < 2; ++hh) {
+              const float2 x = add2(add2(make_float2(ur[mt][hh], ur[mt][hh]), v),
+                                    *reinterpret_cast<const float2*>(wr + (16 * mt + 8 * hh) * p.N + 8 * nt));
+              const float2 y = fma2(make_float2(g, g), x, make_float2(s[mt][nt][2 * hh], s[mt][nt][2 * hh + 1]));
+              s[mt][nt][2 * hh] = y.x, s[mt][nt][2 * hh + 1] = y.y;
+            }
+        }
+      } else {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          const bool ka = k0 + 8 * nt < n, kc = k0 + 8 * nt + 1 < n;
+          const float va = ka ? vr[8 * nt] : 0.f, vb = kc ? vr[8 * nt + 1] : 0.f;
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              const bool jin = j0 + 16 * mt + 8 * hh < n;
+              const float* x = wr + (16 * mt + 8 * hh) * p.N + 8 * nt;
+              const float wa = (jin && ka) ? x[0] : 0.f, wb = (jin && kc) ? x[1] : 0.f;
+              s[mt][nt][2 * hh] = fmaf(g, (ur[mt][hh] + va) + wa, s[mt][nt][2 * hh]);
+              s[mt][nt][2 * hh + 1] = fmaf(g, (ur[mt][hh] + vb) + wb, s[mt][nt][2 * hh + 1]);
+            }
+        }
       }
     }
     if (!full) {
@@ -310,6 +330,7 @@ int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   p.u = a.u, p.v_bias = a.v_bias, p.w = a.w, p.gate = a.gate;
   p.out = a.out, p.lse = a.lse, p.out_cast = static_cast<__nv_bfloat16*>(a.out_cast);
   p.H = a.heads, p.N = a.tokens;
+  p.even = a.tokens % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.v_bias) | reinterpret_cast<uintptr_t>(a.w)) & 7) == 0;
   // Queries per CTA: two per warp keep the last wave short on large molecules (a CTA of 24 queries against 36 blocks runs 50
   // times as long as its loads take); smaller molecules need more to pay for their loads, small batches fewer to fill the chip.
   const int bh = a.batch * a.heads;
