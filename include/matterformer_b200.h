@@ -56,7 +56,8 @@ extern "C" {
 #define MF_BACKEND_AUTO 0    /* tensor-core (tcgen05) kernel when the problem qualifies, else the fp32 CUDA-core kernel */
 #define MF_BACKEND_GENERIC 1 /* always the fp32 CUDA-core kernel */
 #define MF_BACKEND_TCGEN05 2 /* tensor-core kernel (row-packed) or MF_ERR_UNSUPPORTED */
-#define MF_BACKEND_TCGEN05_TILES 3 /* tensor-core kernels with one query per tile row, or MF_ERR_UNSUPPORTED */
+#define MF_BACKEND_TCGEN05_TILES 3 /* tensor-core kernels with one query per tile row (warp-level ones up to 32 tokens and
+                                    * with the factorized bias), or MF_ERR_UNSUPPORTED */
 
 /* ------------------------------------------------------------------------- */
 /* 2-simplicial attention                                                     */
@@ -502,8 +503,7 @@ int mf_merge_heads(void* const* ins, const float* scales, void* packed, int32_t 
  * call, all five gradients into grad_proj (B,N,5,H,D) bf16, the gradient of the unscaled projection.  out32 (B,H,N,D)
  * fp32 and lse (B,H,N) fp32 are written by the forward call and read by the backward call, as in mf_simplicial_fwd /
  * mf_simplicial_bwd, whose semantics (masks, zero rows, reproducibility) apply.  Served shapes: head_dim 64, at most 32
- * tokens, heads a multiple of four (the kernels that pack four heads into one 128-row tile); MF_ERR_UNSUPPORTED
- * otherwise.  16-byte aligned tensors; workspaces from the two *_workspace_bytes functions.
+ * tokens, heads a multiple of four; MF_ERR_UNSUPPORTED otherwise.  16-byte aligned tensors; workspaces from the two *_workspace_bytes functions.
  */
 typedef struct MfSimplicialPackedArgs {
   int32_t batch, heads, tokens, head_dim;

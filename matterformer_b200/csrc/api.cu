@@ -79,8 +79,8 @@ bool has_factorized_bias(const Args* a) {
 template <typename Args>
 bool wants_tcgen05(const Args* a, int* rc, const char* name) {
   *rc = MF_OK;
-  // The factorized bias is built into the tile and the warp-level kernels, not into the row-packed ones; the low-rank
-  // residuals into the warp-level ones (at most 32 tokens), else they run on the CUDA-core kernel.
+  // The factorized bias is built into the warp-level kernels, not into the row-packed ones; the low-rank residuals into the
+  // warp-level ones of at most 32 tokens, else they run on the CUDA-core kernel.
   const bool has_residual = a->angle_left || a->message_left;
   const bool bias_ok = (!has_residual || (a->backend == MF_BACKEND_AUTO && a->tokens <= kSmallTokens)) &&
                        (!has_factorized_bias(a) || a->backend != MF_BACKEND_TCGEN05);
@@ -91,21 +91,12 @@ bool wants_tcgen05(const Args* a, int* rc, const char* name) {
   if (a->backend == MF_BACKEND_GENERIC) return false;
   if ((a->backend == MF_BACKEND_TCGEN05 || a->backend == MF_BACKEND_TCGEN05_TILES) && !ok) {
     set_error("%s: the tcgen05 kernels need bf16 inputs with precision bf16_tc, head_dim 64, tokens <= 192, tensors "
-              "that start on 16-byte boundaries and no residual operands; the factorized bias is built into the tile "
-              "kernels only", name);
+              "that start on 16-byte boundaries and no residual operands; the factorized bias does not run on the "
+              "row-packed ones", name);
     *rc = MF_ERR_UNSUPPORTED;
     return false;
   }
   return ok;
-}
-
-// Which of the two tensor-core kernel families serves a qualifying call.  Molecules of at most 32 tokens with a
-// multiple of four heads run fastest with four heads sharing one tile (measured on B200 at 1024 molecules of up to 29
-// atoms: 0.39 / 0.94 ms forward / backward against 0.93 / 1.25 ms row-packed); everything else is row-packed.
-template <typename Args>
-bool uses_tile_kernels(const Args* a) {
-  if (a->backend == MF_BACKEND_TCGEN05_TILES || has_factorized_bias(a)) return true;
-  return a->backend == MF_BACKEND_AUTO && simplicial_sm100_packs_heads(a->tokens, a->heads);
 }
 
 // Molecules of at most 32 tokens run on the warp-level kernels, with and without the factorized bias.
@@ -161,7 +152,9 @@ extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a
   if (!a) return 0;
   int rc;
   if (wants_tcgen05(a, &rc, "mf_simplicial_bwd"))
-    return uses_small_kernels(a) ? 0 : uses_warp_backward(a) ? simplicial_warp_bwd_workspace_bytes(*a) : uses_tile_kernels(a) ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
+    return uses_small_kernels(a)   ? 0
+           : uses_warp_backward(a) ? simplicial_warp_bwd_workspace_bytes(*a)
+           : a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
   return uses_f32_kernels(a) ? 0 : simplicial_generic_bwd_workspace_bytes(*a);
 }
 
@@ -212,7 +205,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
   if (uses_small_kernels(a))
     return a->angle_left || a->message_left ? simplicial_small_res_fwd(*a, s) : simplicial_small_fwd(*a, nullptr, s);
   if (uses_warp_forward(a)) return simplicial_warp_fwd(*a, s);
-  return uses_tile_kernels(a) ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
+  return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
 }
 
 extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
@@ -235,7 +228,7 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
   if (!tc) return uses_f32_kernels(a) ? simplicial_f32_bwd(*a, s) : simplicial_generic_bwd(*a, s);
   if (uses_small_kernels(a)) return simplicial_small_bwd(*a, nullptr, s);
   if (uses_warp_backward(a)) return simplicial_warp_bwd(*a, s);
-  return uses_tile_kernels(a) ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
+  return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -18,18 +18,14 @@ int simplicial_f32_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
 
 // tcgen05 tensor-core kernels (simplicial_sm100.cu)
 bool simplicial_sm100_supports(int dtype, int precision, int tokens, int head_dim);
-// Molecules of at most 32 tokens: four heads share one 128-row tile (needs a multiple of four heads).
-inline bool simplicial_sm100_packs_heads(int tokens, int heads) { return tokens <= 32 && heads % 4 == 0; }
 int simplicial_sm100_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 int simplicial_sm100_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
-// Same kernels with rows that are not (B,H,N,D) contiguous (NULL = contiguous); see RowLayout.
-struct TileLayouts;
-int simplicial_sm100_bwd_layouts(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
-int simplicial_sm100_fwd_layouts(const MfSimplicialFwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
 size_t simplicial_sm100_fwd_workspace_bytes(const MfSimplicialFwdArgs& a);
 size_t simplicial_sm100_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 
-// warp-level kernels for molecules of at most 32 tokens (simplicial_small_fwd.cu, simplicial_small_res_fwd.cu, simplicial_small_bwd.cu)
+// warp-level kernels for molecules of at most 32 tokens (simplicial_small_fwd.cu, simplicial_small_res_fwd.cu, simplicial_small_bwd.cu);
+// rows that are not (B,H,N,D) contiguous by `layouts` (NULL = contiguous), see RowLayout
+struct TileLayouts;
 constexpr int kSmallTokens = 32;
 int simplicial_small_fwd(const MfSimplicialFwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
 int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);

@@ -98,16 +98,7 @@ struct FwdParams {
   const BatchInfo* info;
   const int32_t* order;
   int32_t* status;
-  // factorized logit bias gate_i * ((u_ij + v_ik) + w_jk), fp32, (B,H,N,N) x 3 and (B,H,N); packed-heads kernel only
-  const float* u;
-  const float* v_bias;
-  const float* w;
-  const float* gate;
-  int bias_vec4;       // rows of v_bias and w start on 16-byte boundaries
   int H, N, q_tiles;
-  RowLayout in;        // rows of q, k1, v1, k2, v2
-  RowLayout act;       // rows of out_cast
-  float q_scale;       // applied to q on load; 1 or another power of two (exact in bf16)
   int use_tma;         // K2 / V2 tiles arrive through the tensor maps below (else plain loads)
   CUtensorMap tm_k2;   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle
   CUtensorMap tm_v2;
@@ -121,16 +112,6 @@ constexpr int kSmemPv = kSmemA + kTileM * 128;            // [192][6] pair_valid
 constexpr int kSmemFwdBytes = kSmemPv + kMaxKeys * 6 * 4;
 constexpr int kSmemFwdAlloc = kSmemFwdBytes + 1024;       // slack for the manual 1024-byte alignment
 
-// kPacked: molecules of at most 32 tokens.  One CTA then serves four heads of a molecule: warp w holds the 32
-// query rows of head 4g+w, the K2 / V2 tiles stack the four heads' keys (row 32w'+k = key k of head 4g+w'), the
-// logit GEMM computes all 128 x 128 head combinations and only the diagonal 32 x 32 blocks are used: each row
-// reads the 32 columns of its own head and writes zeros as the probabilities of the other heads' keys.
-// kBias: the factorized geometry bias of the reference kernel (triton_simplicial_attention.py:244-262) is added to the
-// logits in fp32 before the softmax: gate_i * ((u_ij + v_ik) + w_jk), the three terms summed first, as the reference sums
-// them.  u_ij is one value per row and step, the rows v_i. and w_j. are read through the caches.  One head per tile: the
-// biased logits of the maximum pass are written back over the logits in tensor memory, so that the exponential pass reads
-// them instead of forming the bias again.
-template <bool kPacked, bool kBias = false>
 __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __grid_constant__ FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -140,19 +121,16 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // heaviest molecules first
-  const int per_b = kPacked ? p.H / 4 : p.H * p.q_tiles;
+  const int per_b = p.H * p.q_tiles;
   const int b = p.order[blockIdx.x / per_b];
-  const int bh0 = kPacked ? b * p.H + 4 * (int)(blockIdx.x % per_b) : 0;  // packed: first of the CTA's four heads
-  const int h = kPacked ? 4 * (int)(blockIdx.x % per_b) + warp : (int)(blockIdx.x % per_b) / p.q_tiles;
-  const int qt = kPacked ? 0 : blockIdx.x % p.q_tiles;
+  const int h = (int)(blockIdx.x % per_b) / p.q_tiles;
+  const int qt = blockIdx.x % p.q_tiles;
   const int N = p.N;
   const int bh = b * p.H + h;
-  const size_t base = (size_t)bh * N * kD;           // fp32 out and lse: always (B,H,N,D)
-  const long long in_base = p.in.at(b, h, 0);         // this head's rows of q, k1, v1, k2, v2
-  const long long act_base = p.act.at(b, h, 0);       // ... of out_cast
+  const size_t base = (size_t)bh * N * kD;           // (B,H,N,D)
   const int n_keys = p.info[b].n_keys;
   const int n_queries = p.info[b].n_queries;
-  const int row = kPacked ? lane : qt * kTileM + tid;  // this thread's query
+  const int row = qt * kTileM + tid;  // this thread's query
   const bool row_in = row < N;
   const bool row_ok = row_in && p.query_valid[(size_t)b * N + row] > 0;
 
@@ -163,7 +141,7 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
 #pragma unroll
       for (int c = 0; c < kD / 4; ++c) o[c] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (p.out_cast) {
-        uint4* oc = reinterpret_cast<uint4*>(p.out_cast + act_base + row * p.act.token);
+        uint4* oc = reinterpret_cast<uint4*>(p.out_cast + base + (size_t)row * kD);
 #pragma unroll
         for (int c = 0; c < kD / 8; ++c) oc[c] = make_uint4(0, 0, 0, 0);
       }
@@ -171,9 +149,9 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
     }
     return;
   }
-  const int nk_pad = kPacked ? 128 : (n_keys + 15) & ~15;  // MMA N (multiple of 16)
+  const int nk_pad = (n_keys + 15) & ~15;  // MMA N (multiple of 16)
   const int n_chunks = (nk_pad + 31) >> 5;
-  const bool warp_live = kPacked || qt * kTileM + warp * 32 < n_queries;
+  const bool warp_live = qt * kTileM + warp * 32 < n_queries;
 
   // ---- set-up: barriers, tensor memory, key masks, operand tiles
   if (tid == 0) {
@@ -216,8 +194,8 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
     if (p.use_tma) {
       if (tid == 0) {
         mbar_arrive_expect_tx(&bar_kv, (uint32_t)n_chunks * 2u * kTmaBoxRows * 128u);
-        for (int c = 0; c < n_chunks; ++c) {  // packed: box c = the (at most 32) keys of head c of the CTA
-          const int row0 = kPacked ? 0 : c * kTmaBoxRows, mat = kPacked ? bh0 + c : bh;
+        for (int c = 0; c < n_chunks; ++c) {
+          const int row0 = c * kTmaBoxRows, mat = bh;
           tma_load_rows(smem + kSmemK2 + c * kTmaBoxRows * 128, &p.tm_k2, row0, mat, &bar_kv);
           tma_load_rows(smem + kSmemV2 + c * kTmaBoxRows * 128, &p.tm_v2, row0, mat, &bar_kv);
         }
@@ -225,9 +203,8 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
     } else {
       for (int idx = tid; idx < nk_pad * 8; idx += 128) {
         const int r = idx >> 3, c = idx & 7;
-        const int key = kPacked ? (r & 31) : r;  // packed: tile row 32w'+k holds key k of head w'
-        // packed: row r of the tile belongs to head 4g + (r >> 5), the CTA's heads being bh0 % H .. bh0 % H + 3
-        const long long src = kPacked ? p.in.at(b, (bh0 - b * p.H) + (r >> 5), key) : in_base + r * p.in.token;
+        const int key = r;
+        const size_t src = base + (size_t)r * kD;
         uint4 vk = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
         if ((kmask[key >> 5] >> (key & 31)) & 1u) {
           vk = __ldg(reinterpret_cast<const uint4*>(p.k2 + src) + c);
@@ -242,7 +219,7 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
   // this thread's query row as 32 bf16x2 words
   uint32_t qreg[32];
   {
-    const uint4* qp = reinterpret_cast<const uint4*>(p.q + in_base + row * p.in.token);
+    const uint4* qp = reinterpret_cast<const uint4*>(p.q + base + (size_t)row * kD);
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       uint4 v = make_uint4(0, 0, 0, 0);
@@ -252,14 +229,6 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
       qreg[4 * c + 2] = v.z;
       qreg[4 * c + 3] = v.w;
     }
-    if (p.q_scale != 1.f) {
-      const __nv_bfloat162 sc = __float2bfloat162_rn(p.q_scale);
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const __nv_bfloat162 t = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&qreg[c]), sc);
-        qreg[c] = *reinterpret_cast<const uint32_t*>(&t);
-      }
-    }
   }
   bool bad = false;
   if (p.use_tma) {
@@ -267,7 +236,7 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
     if (!bad)  // rows of invalid keys must be zero whatever the padded tokens hold
       for (int idx = tid; idx < nk_pad * 8; idx += 128) {
         const int r = idx >> 3, c = idx & 7;
-        const int key = kPacked ? (r & 31) : r;
+        const int key = r;
         if (!((kmask[key >> 5] >> (key & 31)) & 1u)) {
           const uint32_t off = r * 128 + ((c ^ (r & 7)) << 4);
           *reinterpret_cast<uint4*>(smem + kSmemK2 + off) = make_uint4(0, 0, 0, 0);
@@ -298,18 +267,11 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
   float l_run = 0.f;
   uint32_t phase = 0;
 
-  // bias operands of this thread's row (kBias): the gate, and the rows of u and v_bias
-  const size_t nn = (size_t)N * N;
-  const float gate_i = (kBias && row_ok) ? p.gate[(size_t)bh * N + row] : 0.f;
-  const float* u_row = kBias ? p.u + (size_t)bh * nn + (size_t)(row_ok ? row : 0) * N : nullptr;
-  const float* v_row = kBias ? p.v_bias + (size_t)bh * nn + (size_t)(row_ok ? row : 0) * N : nullptr;
-
   for (int j = 0; j < n_keys; ++j) {
     if (!((kmask[j >> 5] >> (j & 31)) & 1u)) continue;  // uniform
-    const float u_ij = kBias ? __ldg(u_row + j) : 0.f;
     // ---- A_j = Q o k1_j  (one row per thread)
     {
-      const uint4* kp = reinterpret_cast<const uint4*>(p.k1 + in_base + j * p.in.token);
+      const uint4* kp = reinterpret_cast<const uint4*>(p.k1 + base + (size_t)j * kD);
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const uint4 kk = __ldg(kp + c);
@@ -330,8 +292,8 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
       int jn = j + 1;
       while (jn < n_keys && !((kmask[jn >> 5] >> (jn & 31)) & 1u)) ++jn;
       if (lane == 0 && jn < n_keys) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.k1 + in_base + jn * p.in.token));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.v1 + in_base + jn * p.in.token));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.k1 + base + (size_t)jn * kD));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.v1 + base + (size_t)jn * kD));
       }
     }
     fence_smem_to_async_proxy();
@@ -366,65 +328,20 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
           mx4[e & 3] = fmaxf(mx4[e & 3], ((word >> e) & 1u) ? __uint_as_float(s[e]) : -INFINITY);
       }
     };
-    // packed heads: the row has one chunk, the 32 columns of its own head; it stays in registers for pass 2
-    const uint32_t tmem_srow = tmem_row + (kPacked ? 32 * warp : 0);
-    const int row_chunks = kPacked ? 1 : n_chunks;
+    const uint32_t tmem_srow = tmem_row;
     uint32_t sa[32], sb[32];
     tmem_ld32(tmem_srow, sa);
-    if constexpr (kBias && kPacked) {  // the row's one chunk: logits += gate_i * ((u_ij + v_ik) + w_jk) for its head's keys
-      const float* w_row = p.w + (size_t)bh * nn + (size_t)j * N;
-      float bsum[32];
-#pragma unroll
-      for (int e = 0; e < 32; ++e) bsum[e] = e < N ? (u_ij + __ldg(v_row + e)) + __ldg(w_row + e) : 0.f;
+    for (int c = 0; c < n_chunks; c += 2) {
       tmem_ld_wait();
-#pragma unroll
-      for (int e = 0; e < 32; ++e) sa[e] = __float_as_uint(fmaf(gate_i, bsum[e], __uint_as_float(sa[e])));
-    }
-    // one head per tile with the bias: add it to chunk c and put the chunk back for pass 2
-    auto bias_chunk = [&](uint32_t (&s)[32], int c) {
-      if constexpr (kBias && !kPacked) {
-        const float* w_row = p.w + (size_t)bh * nn + (size_t)j * N;
-        if (p.bias_vec4) {  // rows of v_bias and w start on 16-byte boundaries: four keys per load
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const int k = 32 * c + e;
-            if (k < N) {
-              const float4 vv = __ldg(reinterpret_cast<const float4*>(v_row + k));
-              const float4 ww = __ldg(reinterpret_cast<const float4*>(w_row + k));
-              s[e] = __float_as_uint(fmaf(gate_i, (u_ij + vv.x) + ww.x, __uint_as_float(s[e])));
-              s[e + 1] = __float_as_uint(fmaf(gate_i, (u_ij + vv.y) + ww.y, __uint_as_float(s[e + 1])));
-              s[e + 2] = __float_as_uint(fmaf(gate_i, (u_ij + vv.z) + ww.z, __uint_as_float(s[e + 2])));
-              s[e + 3] = __float_as_uint(fmaf(gate_i, (u_ij + vv.w) + ww.w, __uint_as_float(s[e + 3])));
-            }
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int k = 32 * c + e;
-            if (k < N) {
-              const float bsum = (u_ij + __ldg(v_row + k)) + __ldg(w_row + k);
-              s[e] = __float_as_uint(fmaf(gate_i, bsum, __uint_as_float(s[e])));
-            }
-          }
-        }
-        tmem_st16(tmem_srow + 32 * c, reinterpret_cast<const uint32_t(&)[16]>(s[0]));
-        tmem_st16(tmem_srow + 32 * c + 16, reinterpret_cast<const uint32_t(&)[16]>(s[16]));
-      }
-    };
-    for (int c = 0; c < row_chunks; c += 2) {
-      tmem_ld_wait();
-      if (c + 1 < row_chunks) tmem_ld32(tmem_srow + 32 * (c + 1), sb);
-      bias_chunk(sa, c);
+      if (c + 1 < n_chunks) tmem_ld32(tmem_srow + 32 * (c + 1), sb);
       max_chunk(sa, c);
-      if (c + 1 < row_chunks) {
+      if (c + 1 < n_chunks) {
         tmem_ld_wait();
-        if (c + 2 < row_chunks) tmem_ld32(tmem_srow + 32 * (c + 2), sa);
-        bias_chunk(sb, c + 1);
+        if (c + 2 < n_chunks) tmem_ld32(tmem_srow + 32 * (c + 2), sa);
         max_chunk(sb, c + 1);
       }
     }
-    if constexpr (kBias && !kPacked) tmem_st_wait();  // the biased logits are in tensor memory before they are read again
-    if (!kPacked) tmem_ld32(tmem_srow, sa);  // first chunk of pass 2
+    tmem_ld32(tmem_srow, sa);  // first chunk of pass 2
     const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
     const float m_new = fmaxf(m_run, mx * kLog2e);
     const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
@@ -448,25 +365,17 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
         ps4[(e >> 1) & 3] += p0 + p1;
         pk[e >> 1] = pack_bf16x2(p0, p1);
       }
-      tmem_st16(tmem_row + 16 * (kPacked ? warp : c), pk);
+      tmem_st16(tmem_row + 16 * c, pk);
     };
-    for (int c = 0; c < row_chunks; c += 2) {
+    for (int c = 0; c < n_chunks; c += 2) {
       tmem_ld_wait();
-      if (c + 1 < row_chunks) tmem_ld32(tmem_srow + 32 * (c + 1), sb);
+      if (c + 1 < n_chunks) tmem_ld32(tmem_srow + 32 * (c + 1), sb);
       exp_chunk(sa, c);
-      if (c + 1 < row_chunks) {
+      if (c + 1 < n_chunks) {
         tmem_ld_wait();
-        if (c + 2 < row_chunks) tmem_ld32(tmem_srow + 32 * (c + 2), sa);
+        if (c + 2 < n_chunks) tmem_ld32(tmem_srow + 32 * (c + 2), sa);
         exp_chunk(sb, c + 1);
       }
-    }
-    if (kPacked) {  // probabilities of the other heads' keys: zeros over the cross-head logits
-      uint32_t zero16[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) zero16[e] = 0u;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (c != warp) tmem_st16(tmem_row + 16 * c, zero16);
     }
     const float psum = (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
     l_run = l_run * alpha + psum;
@@ -488,7 +397,7 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
     // v1_j while the MMA runs
     uint4 v1w[8];
     {
-      const uint4* vp = reinterpret_cast<const uint4*>(p.v1 + in_base + j * p.in.token);
+      const uint4* vp = reinterpret_cast<const uint4*>(p.v1 + base + (size_t)j * kD);
 #pragma unroll
       for (int c = 0; c < 8; ++c) v1w[c] = __ldg(vp + c);
     }
@@ -529,7 +438,7 @@ __global__ void __launch_bounds__(128, 2) simplicial_fwd_sm100_kernel(const __gr
     for (int c = 0; c < kD / 4; ++c)
       o[c] = make_float4(o_acc[4 * c] * inv, o_acc[4 * c + 1] * inv, o_acc[4 * c + 2] * inv, o_acc[4 * c + 3] * inv);
     if (p.out_cast) {
-      uint4* oc = reinterpret_cast<uint4*>(p.out_cast + act_base + row * p.act.token);
+      uint4* oc = reinterpret_cast<uint4*>(p.out_cast + base + (size_t)row * kD);
 #pragma unroll
       for (int c = 0; c < kD / 8; ++c) {
         uint4 v;
@@ -588,10 +497,6 @@ size_t simplicial_sm100_fwd_workspace_bytes(const MfSimplicialFwdArgs& a) {
 }
 
 int simplicial_sm100_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
-  return simplicial_sm100_fwd_layouts(a, nullptr, stream);
-}
-
-int simplicial_sm100_fwd_layouts(const MfSimplicialFwdArgs& a, const TileLayouts* layouts, cudaStream_t stream) {
   size_t info_off, order_off;
   simplicial_schedule_layout(a.batch, &info_off, &order_off);
   char* ws = static_cast<char*>(a.workspace);
@@ -615,30 +520,17 @@ int simplicial_sm100_fwd_layouts(const MfSimplicialFwdArgs& a, const TileLayouts
   p.H = a.heads;
   p.N = a.tokens;
   p.q_tiles = (a.tokens + kTileM - 1) / kTileM;
-  p.u = a.u, p.v_bias = a.v_bias, p.w = a.w, p.gate = a.gate;
-  p.bias_vec4 = a.tokens % 4 == 0 && reinterpret_cast<uintptr_t>(a.v_bias) % 16 == 0 && reinterpret_cast<uintptr_t>(a.w) % 16 == 0;
-  p.in = p.act = contiguous_rows(a.heads, a.tokens);
-  p.q_scale = 1.f;
-  if (layouts) {  // rows that are not (B,H,N,D) contiguous come by plain loads: the tensor maps describe that form only
-    p.in = layouts->in, p.act = layouts->act, p.q_scale = layouts->q_scale;
-    p.use_tma = 0;
-  } else {
-    p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, a.batch * a.heads) &&
-                make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, a.batch * a.heads);
-  }
+  p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, a.batch * a.heads) &&
+              make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, a.batch * a.heads);
   int rc = launch_schedule(a.query_valid, a.pair_key_valid, a.batch, a.tokens, info, order, p.status, stream);
   if (rc != MF_OK) return rc;
-  const bool packed = simplicial_sm100_packs_heads(a.tokens, a.heads);
-  const bool bias = a.u != nullptr;
-  auto kern = bias ? (packed ? simplicial_fwd_sm100_kernel<true, true> : simplicial_fwd_sm100_kernel<false, true>)
-                   : (packed ? simplicial_fwd_sm100_kernel<true, false> : simplicial_fwd_sm100_kernel<false, false>);
   {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFwdAlloc);
+    cudaError_t e = cudaFuncSetAttribute(simplicial_fwd_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemFwdAlloc);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_fwd_sm100_kernel)");
   }
-  const long long blocks = packed ? (long long)a.batch * (a.heads / 4) : (long long)a.batch * a.heads * p.q_tiles;
+  const long long blocks = (long long)a.batch * a.heads * p.q_tiles;
   profile_mark(MF_PROFILE_SIMPLICIAL_FWD, true, stream);
-  kern<<<(unsigned)blocks, 128, kSmemFwdAlloc, stream>>>(p);
+  simplicial_fwd_sm100_kernel<<<(unsigned)blocks, 128, kSmemFwdAlloc, stream>>>(p);
   profile_mark(MF_PROFILE_SIMPLICIAL_FWD, false, stream);
   MF_CHECK_LAUNCH("simplicial_fwd_sm100_kernel");
   return MF_OK;

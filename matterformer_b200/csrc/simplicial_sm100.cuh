@@ -41,7 +41,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
 int launch_schedule(const uint8_t* query_valid, const uint8_t* key_valid, int B, int N, BatchInfo* info,
                     int32_t* order, int32_t* status, cudaStream_t stream);
 
-struct TileLayouts {   // non-default row layouts of a tile-kernel call (see RowLayout)
+struct TileLayouts {   // non-default row layouts of a call of the small kernels (see RowLayout)
   RowLayout in;        // q, k1, v1, k2, v2 and their gradients
   RowLayout act;       // out_cast (forward), grad_out (backward)
   float q_scale;       // q is multiplied by this on load (a power of two), dq on store

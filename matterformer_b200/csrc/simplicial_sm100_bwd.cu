@@ -62,18 +62,6 @@ constexpr int kOffPv = kOffDS + 2 * kTileM * 128;  // [192][6] pair_valid bit ro
 constexpr int kOffRed = kOffPv + kMaxKeys * kMaskWords * 4;  // 2 x [8 warps][64] column-sum partials
 constexpr int kSmemBwdBytes = kOffRed + 2 * 8 * 64 * 4;
 constexpr int kSmemBwdAlloc = kSmemBwdBytes + 1024;
-// with the factorized bias, four heads per tile: per row the running sum over the steps of dS (the gradient of v_bias),
-// [128][33] fp32
-constexpr int kOffDvb = kSmemBwdBytes;
-constexpr int kDvbStride = 33;  // odd: the rows of a warp fall into different banks
-// with the factorized bias, one head per tile: the four row groups' column sums of gate_i dS of a step (the gradient of
-// w), 2 steps x [4][128] fp32, and the column halves' row sums of dS (the gradient of u) and of dS x bias (the
-// gradient of the gate), 2 steps x [128] fp32
-constexpr int kOffDwRed = kSmemBwdBytes;
-constexpr int kOffDuRed = kOffDwRed + 2 * 4 * kSlab * 4;
-static_assert(kOffDuRed + 2 * kTileM * 4 <= kOffDvb + kTileM * kDvbStride * 4, "the bias scratch of both variants fits one size");
-constexpr int kSmemBwdBiasAlloc = kOffDvb + kTileM * kDvbStride * 4 + 1024;
-
 struct BwdParams {
   const __nv_bfloat16* grad_out;
   const __nv_bfloat16* q;
@@ -97,69 +85,21 @@ struct BwdParams {
   int32_t* status;
   int H, N, q_tiles, slabs;
   size_t part_stride;  // BH * N * 64
-  // factorized logit bias gate_i * ((u_ij + v_ik) + w_jk) and its gradients, fp32, (B,H,N,N) x 3 and (B,H,N);
-  // packed-heads kernel only
-  const float* u;
-  const float* v_bias;
-  const float* w;
-  const float* gate;
-  float* du;
-  float* dv_bias;
-  float* dw;
-  float* dgate;
-  int dv_vec4;         // rows of dv_bias start on 16-byte boundaries: four keys per reduction
-  int bias_vec4;       // likewise the rows of v_bias and w: four keys per load
-  // four heads per tile: one CTA holds every contribution to its heads' gradients and writes them itself, in bf16
-  __nv_bfloat16* gq;
-  __nv_bfloat16* gk1;
-  __nv_bfloat16* gv1;
-  __nv_bfloat16* gk2;
-  __nv_bfloat16* gv2;
-  RowLayout in;        // rows of q, k1, v1, k2, v2 and of the five gradients
-  RowLayout act;       // rows of grad_out
-  float q_scale;       // applied to q on load and to dq on store; 1 or another power of two
   int use_tma;         // K2 / V2 slabs arrive through the tensor maps below (else plain loads)
   CUtensorMap tm_k2;   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle
   CUtensorMap tm_v2;
 };
 
-template <typename T>
-__global__ void delta_bf16_kernel(const __nv_bfloat16* __restrict__ grad_out, RowLayout go, int H, int N,
-                                  const float* __restrict__ out, float* __restrict__ delta, int rows) {
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // (b, h, n) in the order of out and delta
+__global__ void delta_bf16_kernel(const __nv_bfloat16* __restrict__ grad_out, const float* __restrict__ out,
+                                  float* __restrict__ delta, int rows) {
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // (b, h, n)
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
-  const int n = row % N, bh = row / N;
-  const __nv_bfloat162 g = reinterpret_cast<const __nv_bfloat162*>(grad_out + go.at(bh / H, bh % H, n))[lane];
+  const __nv_bfloat162 g = reinterpret_cast<const __nv_bfloat162*>(grad_out + (size_t)row * kD)[lane];
   const float2 o = reinterpret_cast<const float2*>(out + (size_t)row * kD)[lane];
   float s = fmaf(__bfloat162float(g.x), o.x, __bfloat162float(g.y) * o.y);
   s = warp_sum(s);
   if (lane == 0) delta[row] = s;
-}
-
-// Additions to global memory that return nothing (the thread does not wait for them).  Additions of one thread to one
-// address take effect in program order, so a location with a single writer accumulates in a fixed order.
-__device__ __forceinline__ void red_add(float* addr, float v) {
-  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void red_add4(float* addr, float a, float b, float c, float d) {  // 16-byte aligned
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
-// Sum over the 32 lanes of a warp of a 32-vector held by every lane: lane l returns the total of column l.
-// Fixed exchange pattern -> deterministic.
-__device__ __forceinline__ float warp_column_sums32(float (&v)[32], int lane) {
-#pragma unroll
-  for (int off = 16, n = 16; off >= 1; off >>= 1, n >>= 1) {
-    const bool upper = (lane & off) != 0;
-#pragma unroll
-    for (int t = 0; t < n; ++t) {
-      const float send = upper ? v[t] : v[t + n];
-      const float keep = upper ? v[t + n] : v[t];
-      v[t] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  return v[0];
 }
 
 // Sum over the 32 lanes of a warp of a 64-vector held by every lane.  Returns in (r0, r1) the
@@ -182,22 +122,6 @@ __device__ __forceinline__ void warp_column_sums(float (&v)[64], int lane, float
 constexpr int kBwdThreads = 384;   // 8 worker warps + one warp group that holds the issuing warp
 constexpr int kIssuerThread = 256;
 
-// kPacked: molecules of at most 32 tokens.  One CTA serves four heads of a molecule: tile row 32w+i is query i
-// of head 4g+w, slab row 32w+k is key k of the same head.  The logit GEMMs compute all 128 x 128 combinations;
-// a row uses the 32 columns of its own head and its probabilities for the other heads' keys are written as
-// zeros, which keeps the four products that follow block-diagonal.
-// kBias: the factorized geometry bias of the reference kernel enters the recomputed logits, and its four gradients leave
-// the same element-wise pass (triton_simplicial_attention.py:660-682): du_ij = gate_i sum_k dS, dv_ik = gate_i sum_j dS,
-// dw_jk = sum_i gate_i dS, dgate_i = sum_jk dS ((u_ij + v_ik) + w_jk).
-// Four heads per tile: a row's 32 live logits of a step are all in one thread and the 32 rows of a head are the lanes of
-// one warp, so every sum is local or one shuffle tree; dv accumulates over the steps in a shared-memory row private to
-// the thread, and every gradient element has one writer.
-// One head per tile: a (row, key) pair belongs to one thread of one CTA, which adds gate_i dS to dv_bias in global
-// memory step by step (one writer per address: fixed order).  The sums over a row's keys are combined between the two
-// column halves of the CTA through shared memory and between the (at most two) key slabs by an atomic addition; the
-// sums over the rows go warp -> four row groups (shared memory) -> the (at most two) query tiles (atomic addition).
-// Two addends commute, so the results do not depend on the order in which the CTAs run.
-template <bool kPacked, bool kBias = false>
 __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_constant__ BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -211,40 +135,26 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
   const bool is_worker = tid < 256;
   const int grp = (tid >> 7) & 1;  // 0: q side, 1: dO side
   const int r = tid & 127;         // row of the tile
-  const int per_b = kPacked ? p.H / 4 : p.H * p.q_tiles * p.slabs;
+  const int per_b = p.H * p.q_tiles * p.slabs;
   const int b = p.order[blockIdx.x / per_b];
   int rem = blockIdx.x % per_b;
-  const int hh = r >> 5;                                       // packed: which of the CTA's four heads this row is
-  const int bh0 = kPacked ? b * p.H + 4 * rem : 0;             // packed: first of the CTA's four heads
-  const int h = kPacked ? 4 * rem + hh : rem / (p.q_tiles * p.slabs);
+  const int h = rem / (p.q_tiles * p.slabs);
   rem %= p.q_tiles * p.slabs;
-  const int qt = kPacked ? 0 : rem / p.slabs;
-  const int slab = kPacked ? 0 : rem % p.slabs;
+  const int qt = rem / p.slabs;
+  const int slab = rem % p.slabs;
   const int N = p.N;
   const int bh = b * p.H + h;
   const size_t base = (size_t)bh * N * kD;      // partial planes, lse, delta: always (B,H,N,D)
-  const long long in_base = p.in.at(b, h, 0);    // this head's rows of q, k1, v1, k2, v2
   const int n_keys = p.info[b].n_keys;
   const int n_queries = p.info[b].n_queries;
   if (qt * kTileM >= n_queries || slab * kSlab >= n_keys) {  // nothing to attend to (uniform per CTA)
-    if constexpr (kPacked) {  // the gradients of the CTA's four heads are zeros
-      for (int idx = tid; idx < 4 * N * 8; idx += kBwdThreads) {
-        const long long off = p.in.at(b, bh0 - b * p.H + idx / (N * 8), (idx >> 3) % N) + 8 * (idx & 7);
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(p.gq + off) = z;
-        *reinterpret_cast<uint4*>(p.gk1 + off) = z;
-        *reinterpret_cast<uint4*>(p.gv1 + off) = z;
-        *reinterpret_cast<uint4*>(p.gk2 + off) = z;
-        *reinterpret_cast<uint4*>(p.gv2 + off) = z;
-      }
-    }
     return;  // one head per tile: the finalize kernel never reads this CTA's partials
   }
 
   const int k0 = slab * kSlab;                                  // first key of the slab
   const int nk_slab = min(kSlab, n_keys - k0);                  // keys in the slab
-  const int nk_pad = kPacked ? kSlab : (nk_slab + 15) & ~15;    // MMA N of the logit GEMMs
-  const int row = kPacked ? (r & 31) : qt * kTileM + r;
+  const int nk_pad = (nk_slab + 15) & ~15;    // MMA N of the logit GEMMs
+  const int row = qt * kTileM + r;
   const bool row_ok = is_worker && row < N && p.query_valid[(size_t)b * N + row] > 0;
 
   if (tid == 0) {
@@ -293,8 +203,8 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     if (p.use_tma) {
       if (tid == 0) {
         mbar_arrive_expect_tx(&bar_kv, (uint32_t)(kSlab / kTmaBoxRows) * 2u * kTmaBoxRows * 128u);
-        for (int c = 0; c < kSlab / kTmaBoxRows; ++c) {  // packed: box c = the keys of head c of the CTA
-          const int row0 = kPacked ? 0 : k0 + c * kTmaBoxRows, mat = kPacked ? bh0 + c : bh;
+        for (int c = 0; c < kSlab / kTmaBoxRows; ++c) {
+          const int row0 = k0 + c * kTmaBoxRows, mat = bh;
           tma_load_rows(smem + kOffK2 + c * kTmaBoxRows * 128, &p.tm_k2, row0, mat, &bar_kv);
           tma_load_rows(smem + kOffV2 + c * kTmaBoxRows * 128, &p.tm_v2, row0, mat, &bar_kv);
         }
@@ -302,8 +212,8 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     } else {
       for (int idx = tid; idx < kSlab * 8; idx += kBwdThreads) {
         const int rr = idx >> 3, c = idx & 7;
-        const int k = kPacked ? (rr & 31) : k0 + rr;  // packed: slab row 32w'+k holds key k of head w'
-        const long long src = kPacked ? p.in.at(b, (bh0 - b * p.H) + (rr >> 5), k) : in_base + k * p.in.token;
+        const int k = k0 + rr;
+        const size_t src = base + (size_t)k * kD;
         uint4 vk = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
         if (k < n_keys && ((kmask[k >> 5] >> (k & 31)) & 1u)) {
           vk = __ldg(reinterpret_cast<const uint4*>(p.k2 + src) + c);
@@ -318,10 +228,6 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     // because the transposed products read all 128 key rows of the slab
     for (int idx = tid; idx < 4 * kTileM * 8; idx += kBwdThreads)
       *reinterpret_cast<uint4*>(smem + kOffP + idx * 16) = make_uint4(0, 0, 0, 0);
-    if constexpr (kBias && !kPacked) {  // column-sum slots of warps and column halves without work stay zero
-      for (int idx = tid; idx < 2 * 4 * kSlab + 2 * kTileM; idx += kBwdThreads)
-        reinterpret_cast<float*>(smem + kOffDwRed)[idx] = 0.f;
-    }
   }
   // Row data of the workers; loaded inside the worker branch so that it is not live where the roles split.
   uint32_t xreg[32];
@@ -332,7 +238,7 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     if (kv_ok)
       for (int idx = tid; idx < kSlab * 8; idx += kBwdThreads) {
         const int rr = idx >> 3, c = idx & 7;
-        const int k = kPacked ? (rr & 31) : k0 + rr;
+        const int k = k0 + rr;
         if (!(k < n_keys && ((kmask[k >> 5] >> (k & 31)) & 1u))) {
           const uint32_t off = rr * 128 + ((c ^ (rr & 7)) << 4);
           *reinterpret_cast<uint4*>(smem + kOffK2 + off) = make_uint4(0, 0, 0, 0);
@@ -355,12 +261,11 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
   const uint32_t idesc_acc = make_idesc_bf16(kTileM, kD, true, true);     // A MN-major (transposed), B MN-major
   // 32-column chunks this thread handles; warps whose 32 rows all lie beyond the last valid query have no
   // row work at all (their rows of P and dS stay at the zeros written during set-up)
-  const bool warp_live = kPacked || qt * kTileM + (warp & 3) * 32 < n_queries;
+  const bool warp_live = qt * kTileM + (warp & 3) * 32 < n_queries;
   const int nk_x = min(64, nk_pad), nk_y = nk_pad - nk_x;  // logit columns of the two halves of the slab
   const int ks_x = nk_x / 16, ks_y = nk_y / 16;
-  // packed: the row's own head occupies column block hh = 2*half + group of exactly one (half, group) pair
-  const bool live_x = kPacked ? (hh == grp) : (warp_live && 32 * grp < nk_x);
-  const bool live_y = kPacked ? (hh == 2 + grp) : (warp_live && 32 * grp < nk_y);
+  const bool live_x = warp_live && 32 * grp < nk_x;
+  const bool live_y = warp_live && 32 * grp < nk_y;
   const uint32_t idesc_x = make_idesc_bf16(kTileM, nk_x, false, false);
   const uint32_t idesc_y = make_idesc_bf16(kTileM, nk_y > 0 ? nk_y : 16, false, false);
 
@@ -368,7 +273,7 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
 
   // builds this group's scaled operand for step j into stage `st`
   auto build_operand = [&](int j, int st) {
-    const __nv_bfloat16* src = (grp == 0 ? p.k1 : p.v1) + in_base + j * p.in.token;
+    const __nv_bfloat16* src = (grp == 0 ? p.k1 : p.v1) + base + (size_t)j * kD;
     const uint4* kp = reinterpret_cast<const uint4*>(src);
     uint8_t* dst = smem + (grp == 0 ? kOffA1 : kOffA2) + st * (kTileM * 128) + r * 128;
 #pragma unroll
@@ -429,68 +334,17 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
   int step = 0;     // parity selects the `red` buffer
   // one half of the element-wise pass: P and dS of 32 columns as bf16 into shared memory (operands of the
   // transposed products) and, packed, over the S / dP columns just read (A operands of U and W)
-  // bias operands and gradient sums of this thread's row (kBias)
-  const size_t nn = (size_t)p.N * p.N;
-  const float gate_i = (kBias && row_ok) ? p.gate[(size_t)bh * N + row] : 0.f;
-  const float* u_row = kBias ? p.u + (size_t)bh * nn + (size_t)(row_ok ? row : 0) * N : nullptr;
-  const float* v_row = kBias ? p.v_bias + (size_t)bh * nn + (size_t)(row_ok ? row : 0) * N : nullptr;
-  float* dvb_row = reinterpret_cast<float*>(smem + kOffDvb) + r * kDvbStride;  // sum over the steps of dS of this row
-  float* dwred = reinterpret_cast<float*>(smem + kOffDwRed);                   // [2][4][128], zeroed during set-up
-  float* dured = reinterpret_cast<float*>(smem + kOffDuRed);                   // [2][128]
-  float dgate_acc = 0.f;
-  float du_step = 0.f;  // one head per tile: this thread's part of sum_k dS of the current step
-  if constexpr (kBias && kPacked) {
-    if (is_worker && (live_x || live_y)) {  // the thread that will form this row's dS
-#pragma unroll
-      for (int e = 0; e < 32; ++e) dvb_row[e] = 0.f;
-    }
-  }
-  // the bias of this thread's 32 columns of one half of step jj: (u_ij + v_ik) + w_jk.  It does not depend on the
-  // products, so it is fetched before the wait for the logits and is in registers when they arrive.
-  float bsum[kBias ? 32 : 1];
-  auto load_bias = [&](int half, int jj) {
-    if constexpr (kBias) {
-      const int col = 64 * half + 32 * grp;
-      const float* w_row = p.w + (size_t)bh * nn + (size_t)jj * N;
-      const float u_ij = __ldg(u_row + jj);
-      const int kb = kPacked ? 0 : k0 + col;  // first key of this thread's 32 columns
-      if (!kPacked && p.bias_vec4) {  // rows of v_bias and w start on 16-byte boundaries: four keys per load
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float4 vv = make_float4(0.f, 0.f, 0.f, 0.f), ww = vv;
-          const bool in = kb + e < N;
-          if (in) {
-            vv = __ldg(reinterpret_cast<const float4*>(v_row + kb + e));
-            ww = __ldg(reinterpret_cast<const float4*>(w_row + kb + e));
-          }
-          bsum[e] = in ? (u_ij + vv.x) + ww.x : 0.f;
-          bsum[e + 1] = in ? (u_ij + vv.y) + ww.y : 0.f;
-          bsum[e + 2] = in ? (u_ij + vv.z) + ww.z : 0.f;
-          bsum[e + 3] = in ? (u_ij + vv.w) + ww.w : 0.f;
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) bsum[e] = kb + e < N ? (u_ij + __ldg(v_row + kb + e)) + __ldg(w_row + kb + e) : 0.f;
-      }
-    }
-  };
   auto half_pass = [&](int half, int jj) {
     const int col = 64 * half + 32 * grp;  // column inside the slab
     uint32_t s[32], dp[32];
     tmem_ld32(tmem_row + kColS + col, s);
     tmem_ld32(tmem_row + kColDP + col, dp);
     tmem_ld_wait();
-    if constexpr (kBias) {
-#pragma unroll
-      for (int e = 0; e < 32; ++e) s[e] = __float_as_uint(fmaf(gate_i, bsum[e], __uint_as_float(s[e])));
-    }
-    const int wi = kPacked ? 0 : (k0 + col) >> 5;  // packed: the block's 32 columns are keys 0..31 of the row's head
+    const int wi = (k0 + col) >> 5;
     const uint32_t word = kmask[MF_IDX(wi, kMaskWords, p.status)] & pvbits[MF_IDX(jj * kMaskWords + wi, kMaxKeys * kMaskWords, p.status)];
     uint8_t* prow = smem + kOffP + half * (kTileM * 128) + r * 128;
     uint8_t* dsrow = smem + kOffDS + half * (kTileM * 128) + r * 128;
     uint32_t pk[16], dk[16];
-    float dsum = 0.f;                  // kBias: sum_k dS of the row (du_ij)
-    float gds[kBias ? 32 : 1];         // kBias: gate_i dS per key, for the column sums over the head's rows (dw_jk)
 #pragma unroll
     for (int q4 = 0; q4 < 4; ++q4) {  // 8 columns = one 16-byte chunk at a time
       uint32_t* pw = pk + 4 * q4;
@@ -506,16 +360,6 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
         }
         const float d0 = p0 * (__uint_as_float(dp[e]) - delta);
         const float d1 = p1 * (__uint_as_float(dp[e + 1]) - delta);
-        if constexpr (kBias) {
-          dsum += d0 + d1;
-          dgate_acc = fmaf(d0, bsum[e], fmaf(d1, bsum[e + 1], dgate_acc));
-          if constexpr (kPacked) {
-            dvb_row[e] += d0;
-            dvb_row[e + 1] += d1;
-          }
-          gds[e] = gate_i * d0;
-          gds[e + 1] = gate_i * d1;
-        }
         pw[t] = pack_bf16x2(p0, p1);
         dw[t] = pack_bf16x2(d0, d1);
       }
@@ -526,39 +370,6 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     }
     tmem_st16(tmem_row + kColS + col, pk);
     tmem_st16(tmem_row + kColDP + col, dk);
-    if constexpr (kBias && kPacked) {
-      if (row_ok && p.du) p.du[(size_t)bh * nn + (size_t)row * N + jj] = gate_i * dsum;
-      const float tot = warp_column_sums32(gds, lane);  // the warp's lanes are the 32 queries of this head
-      if (lane < N && p.dw) p.dw[(size_t)bh * nn + (size_t)jj * N + lane] = tot;
-    }
-    if constexpr (kBias && !kPacked) {
-      du_step += dsum;
-      const int kb = k0 + col;
-      if (row_ok && p.dv_bias) {  // dv_bias[i, k] += gate_i dS: this thread is the only writer of its 32 addresses
-        float* dst = p.dv_bias + (size_t)bh * nn + (size_t)row * N + kb;
-        if (p.dv_vec4) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 4)
-            if (kb + e < N) red_add4(dst + e, gds[e], gds[e + 1], gds[e + 2], gds[e + 3]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (kb + e < N) red_add(dst + e, gds[e]);
-        }
-      }
-      const float tot = warp_column_sums32(gds, lane);  // over the warp's 32 rows; lane = column
-      dwred[(step & 1) * 512 + (warp & 3) * kSlab + col + lane] = tot;
-    }
-  };
-  // packed: the 32 columns of another head in this row: zero probabilities over the cross-head logits (the
-  // shared-memory copies of P and dS keep the zeros written during set-up)
-  auto zero_pass = [&](int half) {
-    const int col = 64 * half + 32 * grp;
-    uint32_t zero16[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) zero16[e] = 0u;
-    tmem_st16(tmem_row + kColS + col, zero16);
-    tmem_st16(tmem_row + kColDP + col, zero16);
   };
   // U += dS.K2 and W += P.V2 over the keys of one half; A operands from tensor memory
   auto issue_uw = [&](int half, int ks_count) {
@@ -575,14 +386,7 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
   };
   // the column sums of step jj wait in red[buf]; 64 threads of each group add the four warp partials
   auto store_column_sums = [&](int jj, int buf) {
-    if (kPacked) {  // one head per warp: nothing to add, two of the 4 x 64 sums per thread
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int w = (r >> 6) + 2 * t, d = r & 63;
-        const float tot = red[MF_IDX((buf & 1) * 512 + (grp * 4 + w) * 64 + d, 1024, p.status)];
-        (grp == 0 ? p.gk1 : p.gv1)[p.in.at(b, bh0 - b * p.H + w, jj) + d] = __float2bfloat16_rn(tot);
-      }
-    } else if (r < 64) {
+    if (r < 64) {
       const float* rp = red + (buf & 1) * 512 + (grp * 4) * 64 + r;
       const float tot = (rp[0] + rp[64]) + (rp[128] + rp[192]);
       float* dst = (grp == 0 ? p.dk1_part : p.dv1_part) + (size_t)(qt * p.slabs + slab) * p.part_stride + base +
@@ -646,7 +450,7 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     // this thread's row of q (group 0) or dO (group 1) as 32 bf16x2 words
     {
-      const __nv_bfloat16* src = grp == 0 ? p.q + in_base + row * p.in.token : p.grad_out + p.act.at(b, h, row);
+      const __nv_bfloat16* src = grp == 0 ? p.q + base + (size_t)row * kD : p.grad_out + base + (size_t)row * kD;
       const uint4* xp = reinterpret_cast<const uint4*>(src);
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -656,14 +460,6 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
         xreg[4 * c + 1] = v.y;
         xreg[4 * c + 2] = v.z;
         xreg[4 * c + 3] = v.w;
-      }
-      if (grp == 0 && p.q_scale != 1.f) {
-        const __nv_bfloat162 sc = __float2bfloat162_rn(p.q_scale);
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const __nv_bfloat162 t = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&xreg[c]), sc);
-          xreg[c] = *reinterpret_cast<const uint32_t*>(&t);
-        }
       }
     }
     // exp2(S log2e - lse log2e); an invalid row keeps +inf so that every probability is 0
@@ -683,31 +479,20 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
       int jn = j + 1;
       while (jn < n_keys && !((kmask[jn >> 5] >> (jn & 31)) & 1u)) ++jn;
       if (lane == 0 && jn < n_keys) {  // the rows scaled into the next operands: one 128-byte line each
-        const __nv_bfloat16* nxt = (grp == 0 ? p.k1 : p.v1) + in_base + jn * p.in.token;
+        const __nv_bfloat16* nxt = (grp == 0 ? p.k1 : p.v1) + base + (size_t)jn * kD;
         asm volatile("prefetch.global.L1 [%0];" ::"l"(nxt));
       }
-      if (live_x) load_bias(0, j);
       wait_on(&bar_sx, phase);
       tc_fence_after_sync();
-      du_step = 0.f;
       if (live_x) half_pass(0, j);
-      else if (kPacked) zero_pass(0);
-      if constexpr (kBias && !kPacked) {  // the other column half's part of du_ij, read after this step's arrivals
-        if (grp == 1) dured[(step & 1) * kTileM + r] = du_step;
-      }
       tmem_st_wait();
       fence_smem_to_async_proxy();
       tc_fence_before_sync();  // also orders the previous drain's reads of U, W before the products issued next
       mbar_arrive(&bar_px);
       if (nk_y > 0) {
-        if (live_y) load_bias(1, j);
         wait_on(&bar_sy, phase);
         tc_fence_after_sync();
         if (live_y) half_pass(1, j);
-        else if (kPacked) zero_pass(1);
-        if constexpr (kBias && !kPacked) {
-          if (grp == 1) dured[(step & 1) * kTileM + r] = du_step;
-        }
         tmem_st_wait();
         fence_smem_to_async_proxy();
         tc_fence_before_sync();
@@ -719,23 +504,13 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
         tc_fence_before_sync();
         mbar_arrive(&bar_a);
       }
-      const uint4* k1p = reinterpret_cast<const uint4*>(p.k1 + in_base + j * p.in.token);
+      const uint4* k1p = reinterpret_cast<const uint4*>(p.k1 + base + (size_t)j * kD);
       wait_on(&bar_uw, phase);
       tc_fence_after_sync();
       phase ^= 1u;
       // U, W of this step exist, so every worker has passed its arrivals of this step and thereby finished the
       // previous drain: the previous step's column sums are complete in `red` (other buffer than this step's)
       if (j_prev >= 0) store_column_sums(j_prev, step ^ 1);
-      if constexpr (kBias && !kPacked) {
-        // likewise this step's sums of dS: every worker wrote its parts before the arrivals that U and W waited for
-        if (grp == 0) {
-          const float* dr = dwred + (step & 1) * 512 + r;
-          const float tot = (dr[0] + dr[kSlab]) + (dr[2 * kSlab] + dr[3 * kSlab]);
-          if (k0 + r < N && p.dw) atomicAdd(p.dw + (size_t)bh * nn + (size_t)j * N + k0 + r, tot);  // <= 2 query tiles
-          const float du_ij = du_step + dured[(step & 1) * kTileM + r];
-          if (row_ok && p.du) atomicAdd(p.du + (size_t)bh * nn + (size_t)row * N + j, gate_i * du_ij);  // <= 2 key slabs
-        }
-      }
       // ---- drain: group 0 reads U (dq, dk1_j), group 1 reads W (dv1_j)
       float* red_j = red + (step & 1) * 512;
       if (!warp_live) {
@@ -786,70 +561,23 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     // ---- epilogue: the last step's accumulated products are still in flight (the issuer committed bar_fin)
     wait_on(&bar_fin, 0);
     tc_fence_after_sync();
-    if constexpr (kBias && !kPacked) {  // the two column halves' parts of dgate_i meet in shared memory
-      if (grp == 1) dured[r] = dgate_acc;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-    }
     if (bad) {
       atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
     } else {
-      if constexpr (kBias && !kPacked) {
-        if (grp == 0 && row_ok && p.dgate) atomicAdd(p.dgate + (size_t)bh * N + row, dgate_acc + dured[r]);  // <= 2 key slabs
-      }
-      if constexpr (kBias && kPacked) {
-        if ((live_x || live_y) && row_ok) {  // the thread that formed this row's dS
-          if (p.dv_bias)
-            for (int e = 0; e < N && e < 32; ++e) p.dv_bias[(size_t)bh * nn + (size_t)row * N + e] = gate_i * dvb_row[e];
-          if (p.dgate) p.dgate[(size_t)bh * N + row] = dgate_acc;
-        }
-      }
-      if constexpr (kPacked) {
-        // rows of first keys that no step visited: zeros (same thread-to-element mapping as store_column_sums)
-        for (int jj = 0; jj < N; ++jj) {
-          if ((kmask[jj >> 5] >> (jj & 31)) & 1u) continue;  // uniform
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-            (grp == 0 ? p.gk1 : p.gv1)[p.in.at(b, bh0 - b * p.H + (r >> 6) + 2 * t, jj) + (r & 63)] = __float2bfloat16_rn(0.f);
-        }
-        if (grp == 0 && row < N) {
-          const float sc = row_ok ? p.q_scale : 0.f;
-          uint4* dst = reinterpret_cast<uint4*>(p.gq + p.in.at(b, h, row));
-#pragma unroll
-          for (int c = 0; c < kD / 8; ++c)
-            dst[c] = make_uint4(pack_bf16x2(dq_acc[8 * c] * sc, dq_acc[8 * c + 1] * sc),
-                                pack_bf16x2(dq_acc[8 * c + 2] * sc, dq_acc[8 * c + 3] * sc),
-                                pack_bf16x2(dq_acc[8 * c + 4] * sc, dq_acc[8 * c + 5] * sc),
-                                pack_bf16x2(dq_acc[8 * c + 6] * sc, dq_acc[8 * c + 7] * sc));
-        }
-      } else if (grp == 0 && row < N) {
+      if (grp == 0 && row < N) {
         float4* dst = reinterpret_cast<float4*>(p.dq_part + (size_t)slab * p.part_stride + base + (size_t)row * kD);
 #pragma unroll
         for (int c = 0; c < kD / 4; ++c)
           dst[c] = make_float4(dq_acc[4 * c], dq_acc[4 * c + 1], dq_acc[4 * c + 2], dq_acc[4 * c + 3]);
       }
       // accumulators: lane r of tensor memory = key k0 + r; group 0 stores dK2, group 1 dV2
-      const int k = kPacked ? (r & 31) : k0 + r;  // packed: lane 32w+k = key k of head w, this thread's own head
+      const int k = k0 + r;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t w[32];
         tmem_ld32(tmem_row + (grp == 0 ? kColDK2 : kColDV2) + 32 * half, w);
         tmem_ld_wait();
-        if constexpr (kPacked) {
-          if (k < N) {
-            const bool live = !first && k < n_keys && ((kmask[k >> 5] >> (k & 31)) & 1u);
-            uint4* dst = reinterpret_cast<uint4*>((grp == 0 ? p.gk2 : p.gv2) + p.in.at(b, h, k) + 32 * half);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint4 o = make_uint4(0, 0, 0, 0);
-              if (live)
-                o = make_uint4(pack_bf16x2(__uint_as_float(w[8 * c]), __uint_as_float(w[8 * c + 1])),
-                               pack_bf16x2(__uint_as_float(w[8 * c + 2]), __uint_as_float(w[8 * c + 3])),
-                               pack_bf16x2(__uint_as_float(w[8 * c + 4]), __uint_as_float(w[8 * c + 5])),
-                               pack_bf16x2(__uint_as_float(w[8 * c + 6]), __uint_as_float(w[8 * c + 7])));
-              dst[c] = o;
-            }
-          }
-        } else if (k < n_keys && !first) {
+        if (k < n_keys && !first) {
           float4* dst = reinterpret_cast<float4*>((grp == 0 ? p.dk2_part : p.dv2_part) + (size_t)qt * p.part_stride +
                                                   base + (size_t)k * kD + 32 * half);
 #pragma unroll
@@ -864,22 +592,6 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kBwdTmemCols);
-}
-
-// Four heads per tile: the gradients are final when the main kernel ends; only after an expired device-side wait
-// (status word set) are they all overwritten with zeros, as the finalize kernel does for the other shapes.
-__global__ void simplicial_bwd_zero_on_error_kernel(BwdParams p, int BH) {
-  if (p.status[0] == 0) return;
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // one thread per 8 elements
-  if (idx >= (long long)BH * p.N * (kD / 8)) return;
-  const int row = (int)((idx / (kD / 8)) % p.N), bh = (int)(idx / ((long long)(kD / 8) * p.N));
-  const long long off = p.in.at(bh / p.H, bh % p.H, row) + 8 * (idx % (kD / 8));
-  const uint4 z = make_uint4(0, 0, 0, 0);
-  *reinterpret_cast<uint4*>(p.gq + off) = z;
-  *reinterpret_cast<uint4*>(p.gk1 + off) = z;
-  *reinterpret_cast<uint4*>(p.gv1 + off) = z;
-  *reinterpret_cast<uint4*>(p.gk2 + off) = z;
-  *reinterpret_cast<uint4*>(p.gv2 + off) = z;
 }
 
 // Sums the partials in a fixed order and writes the five gradients in bf16; rows of padded
@@ -897,8 +609,7 @@ __global__ void simplicial_bwd_finalize_kernel(BwdParams p, __nv_bfloat16* __res
   const int b = bh / p.H;
   const int n_keys = p.info[b].n_keys, n_queries = p.info[b].n_queries;
   const int nqt = (n_queries + kTileM - 1) / kTileM, nsl = (n_keys + kSlab - 1) / kSlab;
-  const size_t off = ((size_t)bh * p.N + row) * kD + 4 * d4;             // in the partial planes
-  const long long dst = p.in.at(b, bh - b * p.H, row) + 4 * d4;          // in the gradient tensors
+  const size_t off = ((size_t)bh * p.N + row) * kD + 4 * d4;
   const bool sane = p.status[0] == 0;  // after an expired device-side wait every gradient is written as zeros
   const bool q_ok = sane && row < n_queries && p.query_valid[(size_t)b * p.N + row] > 0 && n_keys > 0;
   const bool k_ok = sane && row < n_keys && p.key_valid[(size_t)b * p.N + row] > 0 && n_queries > 0;
@@ -917,8 +628,7 @@ __global__ void simplicial_bwd_finalize_kernel(BwdParams p, __nv_bfloat16* __res
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
   if (q_ok)
     for (int s = 0; s < nsl; ++s) add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)s * p.part_stride + off));
-  a.x *= p.q_scale, a.y *= p.q_scale, a.z *= p.q_scale, a.w *= p.q_scale;
-  store4(dq + dst, a);
+  store4(dq + off, a);
   float4 k2v = make_float4(0.f, 0.f, 0.f, 0.f), v2v = k2v, k1v = k2v, v1v = k2v;
   if (k_ok) {
     for (int t = 0; t < nqt; ++t) {
@@ -930,10 +640,10 @@ __global__ void simplicial_bwd_finalize_kernel(BwdParams p, __nv_bfloat16* __res
       }
     }
   }
-  store4(dk2 + dst, k2v);
-  store4(dv2 + dst, v2v);
-  store4(dk1 + dst, k1v);
-  store4(dv1 + dst, v1v);
+  store4(dk2 + off, k2v);
+  store4(dv2 + off, v2v);
+  store4(dk1 + off, k1v);
+  store4(dv1 + off, v1v);
 }
 
 struct BwdLayout {
@@ -972,10 +682,6 @@ size_t simplicial_sm100_bwd_workspace_bytes(const MfSimplicialBwdArgs& a) {
 }
 
 int simplicial_sm100_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
-  return simplicial_sm100_bwd_layouts(a, nullptr, stream);
-}
-
-int simplicial_sm100_bwd_layouts(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream) {
   const BwdLayout l = bwd_layout(a.batch, a.heads, a.tokens);
   char* ws = static_cast<char*>(a.workspace);
   const int BH = a.batch * a.heads;
@@ -991,19 +697,7 @@ int simplicial_sm100_bwd_layouts(const MfSimplicialBwdArgs& a, const TileLayouts
   p.key_valid = a.pair_key_valid;
   p.pair_valid = a.pair_valid;
   p.status = reinterpret_cast<int32_t*>(ws);
-  p.in = p.act = contiguous_rows(a.heads, a.tokens);
-  p.q_scale = 1.f;
-  p.u = a.u, p.v_bias = a.v_bias, p.w = a.w, p.gate = a.gate;
-  p.du = a.du, p.dv_bias = a.dv_bias, p.dw = a.dw, p.dgate = a.dgate;
-  p.gq = static_cast<__nv_bfloat16*>(a.dq), p.gk1 = static_cast<__nv_bfloat16*>(a.dk1);
-  p.gv1 = static_cast<__nv_bfloat16*>(a.dv1), p.gk2 = static_cast<__nv_bfloat16*>(a.dk2);
-  p.gv2 = static_cast<__nv_bfloat16*>(a.dv2);
-  if (layouts) {  // rows that are not (B,H,N,D) contiguous come by plain loads: the tensor maps describe that form only
-    p.in = layouts->in, p.act = layouts->act, p.q_scale = layouts->q_scale;
-    p.use_tma = 0;
-  } else {
-    p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, BH) && make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, BH);
-  }
+  p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, BH) && make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, BH);
   BatchInfo* info = reinterpret_cast<BatchInfo*>(ws + l.info);
   int32_t* order = reinterpret_cast<int32_t*>(ws + l.order);
   float* delta = reinterpret_cast<float*>(ws + l.delta);
@@ -1024,31 +718,17 @@ int simplicial_sm100_bwd_layouts(const MfSimplicialBwdArgs& a, const TileLayouts
   int rc = launch_schedule(a.query_valid, a.pair_key_valid, a.batch, a.tokens, info, order, p.status, stream);
   if (rc != MF_OK) return rc;
   const int rows = BH * a.tokens;
-  delta_bf16_kernel<float><<<(rows + 7) / 8, 256, 0, stream>>>(p.grad_out, p.act, a.heads, a.tokens, a.out, delta, rows);
+  delta_bf16_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p.grad_out, a.out, delta, rows);
   MF_CHECK_LAUNCH("delta_bf16_kernel");
-  const bool packed = simplicial_sm100_packs_heads(a.tokens, a.heads);
-  const bool bias = a.u != nullptr;
-  p.dv_vec4 = bias && a.dv_bias && a.tokens % 4 == 0 && reinterpret_cast<uintptr_t>(a.dv_bias) % 16 == 0;
-  p.bias_vec4 = bias && a.tokens % 4 == 0 && reinterpret_cast<uintptr_t>(a.v_bias) % 16 == 0 &&
-                reinterpret_cast<uintptr_t>(a.w) % 16 == 0;
-  auto kern = bias ? (packed ? simplicial_bwd_sm100_kernel<true, true> : simplicial_bwd_sm100_kernel<false, true>)
-                   : (packed ? simplicial_bwd_sm100_kernel<true, false> : simplicial_bwd_sm100_kernel<false, false>);
-  const int smem_alloc = bias ? kSmemBwdBiasAlloc : kSmemBwdAlloc;
   {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_alloc);
+    cudaError_t e = cudaFuncSetAttribute(simplicial_bwd_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBwdAlloc);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_bwd_sm100_kernel)");
   }
-  const long long blocks = packed ? (long long)a.batch * (a.heads / 4) : (long long)BH * p.q_tiles * p.slabs;
+  const long long blocks = (long long)BH * p.q_tiles * p.slabs;
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
-  kern<<<(unsigned)blocks, kBwdThreads, smem_alloc, stream>>>(p);
+  simplicial_bwd_sm100_kernel<<<(unsigned)blocks, kBwdThreads, kSmemBwdAlloc, stream>>>(p);
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, false, stream);
   MF_CHECK_LAUNCH("simplicial_bwd_sm100_kernel");
-  if (packed) {
-    const long long total8 = (long long)rows * (kD / 8);
-    simplicial_bwd_zero_on_error_kernel<<<(unsigned)((total8 + 255) / 256), 256, 0, stream>>>(p, BH);
-    MF_CHECK_LAUNCH("simplicial_bwd_zero_on_error_kernel");
-    return MF_OK;
-  }
   const long long total4 = (long long)rows * (kD / 4);
   simplicial_bwd_finalize_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, stream>>>(
       p, static_cast<__nv_bfloat16*>(a.dq), static_cast<__nv_bfloat16*>(a.dk1), static_cast<__nv_bfloat16*>(a.dv1),
