@@ -1,7 +1,7 @@
 // 2-simplicial attention with the factorized bias, backward, 33 to 192 tokens in bf16 (see simplicial_warp.cuh).
 //
 // First key by first key: for one j the logits over all queries and second keys are a matrix product, and with
-//   S_j = (Q o k1_j) K2^T + bias,  dP_j = dO (V2 o v1_j)^T,  P = exp(S - lse),  dS = P o (dP - delta)
+//   S_j = (Q o k1_j) K2^T + bias,  dP_j = (dO o v1_j) V2^T,  P = exp(S - lse),  dS = P o (dP - delta)
 // five products give all five gradients (query by query it takes six):
 //   T_j = dS_j^T Q  -> dk2 += k1_j o T_j, dk1_j = colsum(K2 o T_j)        R_j = P_j^T dO -> dv2 += v1_j o R_j, dv1_j = colsum(V2 o R_j)
 //   U_j = dS_j K2   -> dq += k1_j o U_j
@@ -298,15 +298,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) simplicial_warp_bwd_kernel(con
           for (int kp = 0; kp < 2; ++kp) {
             uint32_t a[2][4];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              load_a(a[k], fb, tv2 + atk, 0, 2 * kp + k);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) a[k][e] = mul_bf16x2(a[k][e], row2[4 * kp + 2 * k + (e >> 1)]);
-            }
+            for (int k = 0; k < 2; ++k) load_a(a[k], fb, tv2 + atk, 0, 2 * kp + k);
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
               uint32_t x[4];
               load_b(x, fb, tg + ati, nt, kp);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) x[e] = mul_bf16x2(x[e], row2[4 * kp + e]);
               if (kp == 0) mma16_first(dp[nt], a[0], x[0], x[1]);
               else mma16(dp[nt], a[0], x[0], x[1]);
               mma16(dp[nt], a[1], x[2], x[3]);
