@@ -458,6 +458,27 @@ int mf_gated_residual_bwd(const void* dy, int32_t dy_dtype, const float* gate, c
                           float* dgate, void* stream);
 
 /*
+ * out = a_b x + c_b (y - z) + k (p - q) over (B,N,C) fp32, zeros where pad (B,N) is non-zero, and with `center` (C = 3)
+ * minus its mean over the molecule's real rows: the updates of coordinates and atom features in EDMPreconditioner and
+ * edm_sampler with recenter_coordinates, tasks/edm.py:34-81, 153-233.  y, z, p with q may be NULL (z only with y); a and c
+ * are (B) device arrays, or NULL for the values a_value, c_value.
+ */
+typedef struct MfMaskedSumArgs {
+  int32_t batch, tokens, channels, center;
+  const float* x;
+  const float* y;
+  const float* z;
+  const float* p;
+  const float* q;
+  const float* a;
+  const float* c;
+  const uint8_t* pad;
+  float* out;
+  float a_value, c_value, k, reserved0;
+} MfMaskedSumArgs;
+int mf_masked_sum(const MfMaskedSumArgs* args, void* stream);
+
+/*
  * out[c] = sum_r x[r, c]: the bias gradient of a Linear layer (the sum of its output gradient over all tokens), which
  * autograd forms for every Linear of AdaLNBlock.forward, transformer.py:228-316.  x (rows, cols) row-major fp32 or
  * bf16, starting on a 16-byte boundary, cols a multiple of 8; out (cols) fp32; fp32 accumulation in a fixed order

@@ -63,6 +63,7 @@ EXPORTED_SYMBOLS = (
     "mf_feature_flags",
     "mf_ln_modulate_fwd",
     "mf_ln_modulate_bwd",
+    "mf_masked_sum",
     "mf_gated_residual_fwd",
     "mf_gated_residual_bwd",
     "mf_column_sums_workspace_bytes",
@@ -243,6 +244,12 @@ class MfSimplicialPackedArgs(Structure):
     ]
 
 
+class MfMaskedSumArgs(Structure):
+    _fields_ = [(n, c_int32) for n in ("batch", "tokens", "channels", "center")] + \
+               [(n, c_void_p) for n in ("x", "y", "z", "p", "q", "a", "c", "pad", "out")] + \
+               [(n, c_float) for n in ("a_value", "c_value", "k", "reserved0")]  # fmt: skip
+
+
 class MfPairHeadArgs(Structure):
     _fields_ = [
         ("batch", c_int32),
@@ -377,6 +384,8 @@ def lib() -> ctypes.CDLL:
     L.mf_sparse_attn_status.restype = c_int32
     L.mf_pair_head_bwd_workspace_bytes.argtypes = [POINTER(MfPairHeadArgs)]
     L.mf_pair_head_bwd_workspace_bytes.restype = c_size_t
+    L.mf_masked_sum.argtypes = [POINTER(MfMaskedSumArgs), c_void_p]
+    L.mf_masked_sum.restype = c_int32
     for fn in (L.mf_pair_head_fwd, L.mf_pair_head_bwd):
         fn.argtypes = [POINTER(MfPairHeadArgs), c_void_p]
         fn.restype = c_int32

@@ -348,3 +348,52 @@ def equivariant_pair_head(a: torch.Tensor, b: torch.Tensor, coords: torch.Tensor
     Gradients flow to ``a``, ``b``, ``w_rbf``, ``w_out`` and ``b_out``; the coordinates are treated as data.
     """
     return _PairHead.apply(a, b, coords, valid, w_rbf, w_out, b_out, centers, gamma)
+
+
+def masked_sum_applies(x: torch.Tensor, pad_mask: torch.Tensor, *others) -> bool:
+    """CUDA fp32 (B, N, C) tensors of one shape and a (B, N) bool mask."""
+    return (x.is_cuda and x.ndim == 3 and pad_mask.is_cuda and pad_mask.dtype == torch.bool and tuple(pad_mask.shape) == tuple(x.shape[:2])
+            and all(t.dtype == torch.float32 and t.shape == x.shape and t.device == x.device for t in (x, *others)))  # fmt: skip
+
+
+def masked_update(pad_mask, x, a=1.0, y=None, z=None, c=1.0, p=None, q=None, k=0.0, center=False) -> torch.Tensor:
+    B, N, C = x.shape
+    pad_mask = pad_mask.contiguous()
+    x, y, z, p, q = (t.contiguous() if t is not None else None for t in (x, y, z, p, q))
+    out = torch.empty_like(x)
+    at = lambda t: t.data_ptr() if isinstance(t, torch.Tensor) else None  # noqa: E731
+    value = lambda t: 0.0 if isinstance(t, torch.Tensor) else float(t)  # noqa: E731
+    args = _lib.MfMaskedSumArgs(B, N, C, int(center), at(x), at(y), at(z), at(p), at(q), at(a), at(c), at(pad_mask), at(out),
+                                value(a), value(c), float(k))  # fmt: skip
+    _lib.launch(_lib.lib().mf_masked_sum, x.device, ctypes.byref(args))
+    return out
+
+
+class _MaskedSum(torch.autograd.Function):
+    """Mask and centring are one symmetric projection, which the gradient passes through as well."""
+
+    @staticmethod
+    def forward(ctx, pad_mask, x, a, y, z, c, center):
+        ctx.save_for_backward(pad_mask, *(t for t in (a, c) if isinstance(t, torch.Tensor)))
+        ctx.scales = tuple(None if isinstance(t, torch.Tensor) else t for t in (a, c))
+        ctx.center = center
+        return masked_update(pad_mask, x, a, y, z, c, center=center)
+
+    @staticmethod
+    def backward(ctx, grad):
+        pad_mask, *arrays = ctx.saved_tensors
+        a, c = (arrays.pop(0) if t is None else t for t in ctx.scales)
+        need = ctx.needs_input_grad
+        dx = masked_update(pad_mask, grad, a, center=ctx.center) if need[1] else None
+        dy = masked_update(pad_mask, grad, c, center=ctx.center) if need[3] or need[4] else None
+        return None, dx, None, dy if need[3] else None, -dy if need[4] else None, None, None
+
+
+def masked_sum(pad_mask: torch.Tensor, x: torch.Tensor, *, a=1.0, y: Optional[torch.Tensor] = None, z: Optional[torch.Tensor] = None,
+               c=1.0, center: bool = False) -> torch.Tensor:  # fmt: skip
+    """``a x + c (y - z)`` in one pass, zeros on padded rows, with ``center`` minus its mean over the molecule's real rows (see
+    :func:`masked_sum_applies`).  ``a``, ``c``: numbers or contiguous fp32 (B,) tensors without gradient; differentiable in
+    ``x``, ``y`` and ``z``."""
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, y, z)):
+        return _MaskedSum.apply(pad_mask, x, a, y, z, c, center)
+    return masked_update(pad_mask, x, a, y, z, c, center=center)

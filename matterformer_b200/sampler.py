@@ -19,6 +19,7 @@ from typing import Optional
 import torch
 
 from .linear import has_bf16_copy, no_refresh_in_capture, refresh_bf16_copies
+from . import fused
 from .trunk import recenter_coordinates
 
 
@@ -124,6 +125,20 @@ def edm_sample(net, num_atoms: torch.Tensor, *, atom_channels: int = 6, lattice:
         gamma = churn if s_min <= float(t_cur) <= s_max else 0.0
         t_hat = t_cur + gamma * t_cur
         extra = torch.sqrt(t_hat.square() - t_cur.square()) * s_noise
+        if device.type == "cuda":  # the same updates, one launch each
+            extra, dt = float(extra), t_next - t_hat
+            atoms_hat = fused.masked_sum(pad_mask, atoms, y=torch.randn_like(atoms), c=extra)
+            coords_hat = fused.masked_sum(pad_mask, coords, y=torch.randn_like(coords), c=extra, center=True)
+            den_a, den_c = denoise(atoms_hat, coords_hat, float(t_hat))
+            ratio = float(dt / t_hat)
+            atoms = fused.masked_sum(pad_mask, atoms_hat, y=atoms_hat, z=den_a, c=ratio)
+            coords = fused.masked_sum(pad_mask, coords_hat, y=coords_hat, z=den_c, c=ratio, center=True)
+            if step < num_steps - 1:  # half of the first step, half of the slope at the new point
+                den_a, den_c = denoise(atoms, coords, float(t_next))
+                half = 0.5 * float(dt / t_next.clamp_min(1e-8))
+                atoms = fused.masked_update(pad_mask, atoms_hat, y=atoms, z=atoms_hat, c=0.5, p=atoms, q=den_a, k=half)
+                coords = fused.masked_update(pad_mask, coords_hat, y=coords, z=coords_hat, c=0.5, p=coords, q=den_c, k=half, center=True)
+            continue
         atoms_hat = (atoms + extra * torch.randn_like(atoms)).masked_fill(hole, 0.0)
         coords_hat = recenter_coordinates(coords + extra * torch.randn_like(coords), pad_mask)
 

@@ -30,7 +30,7 @@ from torch import nn
 from . import fused
 from .fused import (fused_applies, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
                     split_modulation)
-from .linear import (linear_bf16, linear_gelu_bf16, refresh_bf16_copies, refresh_must_be_captured, stacked_bf16_copies,
+from .linear import (linear_bf16, linear_bf16_applies, linear_gelu_bf16, refresh_bf16_copies, refresh_must_be_captured, stacked_bf16_copies,
                      stacked_modulation)  # fmt: skip
 from .simplicial import (normalize_simplicial_precision, packed_projection_applies, simplicial_attention_cuda,
                          simplicial_attention_packed)  # fmt: skip
@@ -445,6 +445,12 @@ class TransformerTrunk(nn.Module):
         return x
 
 
+def _two_layers(layers: nn.Sequential, x: torch.Tensor) -> torch.Tensor:
+    """Linear -> SiLU -> Linear with the parameters' bf16 copies under bf16 autocast."""
+    first, act, second = layers
+    return linear_bf16(act(linear_bf16(x, first.weight, first.bias)), second.weight, second.bias)
+
+
 class TimeEmbedder(nn.Module):
     def __init__(self, d_model: int, freq_dim: int = 256) -> None:
         super().__init__()
@@ -458,7 +464,7 @@ class TimeEmbedder(nn.Module):
         return torch.cat([torch.cos(args), torch.sin(args)], dim=-1)
 
     def forward(self, t_global: torch.Tensor, t_atomic: torch.Tensor) -> torch.Tensor:
-        return self.mlp(torch.cat([self._embed(t_global), self._embed(t_atomic)], dim=-1))
+        return _two_layers(self.mlp, torch.cat([self._embed(t_global), self._embed(t_atomic)], dim=-1))
 
 
 def _masked_mean(coords: torch.Tensor, pad_mask: torch.Tensor) -> torch.Tensor:
@@ -467,6 +473,8 @@ def _masked_mean(coords: torch.Tensor, pad_mask: torch.Tensor) -> torch.Tensor:
 
 
 def recenter_coordinates(coords: torch.Tensor, pad_mask: torch.Tensor) -> torch.Tensor:
+    if fused.masked_sum_applies(coords, pad_mask) and coords.shape[-1] == 3:
+        return fused.masked_sum(pad_mask, coords, center=True)
     coords = coords.masked_fill(pad_mask[..., None], 0.0)
     return (coords - _masked_mean(coords, pad_mask)).masked_fill(pad_mask[..., None], 0.0)
 
@@ -542,11 +550,14 @@ class EDMModel(nn.Module):
         if sigma.ndim == 2:
             sigma = sigma[:, 0]
         sigma_cond = torch.log(sigma.clamp_min(1e-8)) / 4.0
+        if linear_bf16_applies(atom_noisy, self.atom_proj.weight):  # (the trunk brings its own copies up to date)
+            layers = [self.atom_proj, self.conditioning.mlp[0], self.conditioning.mlp[2], self.atom_head[1], self.atom_head[3]]
+            refresh_bf16_copies([p for m in layers for p in (m.weight, m.bias)], force=refresh_must_be_captured())
         feat = sigma_cond[:, None, None].expand(-1, atom_noisy.shape[1], 1).masked_fill(pad_mask[..., None], 0.0)
-        tokens = self.atom_proj(torch.cat([atom_noisy, feat], dim=-1))
+        tokens = linear_bf16(torch.cat([atom_noisy, feat], dim=-1), self.atom_proj.weight, self.atom_proj.bias)
         cond = self.conditioning(sigma_cond, sigma_cond)
         trunk_out = self.trunk(tokens, cond, pad_mask=pad_mask)
-        atom_delta = self.atom_head[1:](layer_norm(trunk_out, self.atom_head[0])).masked_fill(pad_mask[..., None], 0.0)
+        atom_delta = _two_layers(self.atom_head[1:], layer_norm(trunk_out, self.atom_head[0])).masked_fill(pad_mask[..., None], 0.0)
         return atom_delta, self._coord_delta(trunk_out, coords_noisy, pad_mask)
 
 
@@ -567,8 +578,14 @@ class EDMPreconditioner(nn.Module):
         c_out = sigma * self.sigma_data / torch.sqrt(sigma.square() + sd2)
         c_in = 1.0 / torch.sqrt(sd2 + sigma.square())
         atom_in = atom_noisy * c_in[:, None, None]
-        coords_in = recenter_coordinates(coords_noisy * c_in[:, None, None], pad_mask)
+        fits = not sigma.requires_grad and fused.masked_sum_applies(coords_noisy, pad_mask) and \
+            fused.masked_sum_applies(atom_noisy, pad_mask)  # fmt: skip
+        coords_in = fused.masked_sum(pad_mask, coords_noisy, a=c_in, center=True) if fits else \
+            recenter_coordinates(coords_noisy * c_in[:, None, None], pad_mask)  # fmt: skip
         atom_delta, coord_delta = self.model(atom_in, coords_in, pad_mask, sigma, lattice=lattice)
+        if fits:  # (centring coords_in - coord_delta first would change nothing: the sum is centred itself)
+            return (fused.masked_sum(pad_mask, atom_noisy, a=c_skip, y=atom_in, z=atom_delta.float(), c=c_out),
+                    fused.masked_sum(pad_mask, coords_noisy, a=c_skip, y=coords_in, z=coord_delta.float(), c=c_out, center=True))  # fmt: skip
         atom_clean = atom_in - atom_delta
         coord_clean = recenter_coordinates(coords_in - coord_delta, pad_mask)
         atom_den = (c_skip[:, None, None] * atom_noisy + c_out[:, None, None] * atom_clean).masked_fill(pad_mask[..., None], 0.0)
