@@ -24,6 +24,12 @@ def _stream(device):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+def _bytes(mask: torch.Tensor) -> torch.Tensor:
+    """A mask as the bytes the kernels read: a bool tensor's own, without a copy."""
+    mask = mask.contiguous()
+    return mask.view(torch.uint8) if mask.dtype == torch.bool else mask.to(torch.uint8)
+
+
 def fused_applies(x: torch.Tensor) -> bool:
     """The kernels take a CUDA fp32 / bf16 (B, N, C) residual stream; C a multiple of 8, at most ``MAX_CHANNELS``."""
     return x.is_cuda and x.dtype in _CODE and x.ndim == 3 and x.shape[-1] <= MAX_CHANNELS and x.shape[-1] % 8 == 0
@@ -71,7 +77,7 @@ class _GatedResidual(torch.autograd.Function):
         if a.dtype not in _CODE:
             a = a.float()
         a = a.contiguous()
-        pad = pad.to(torch.uint8).contiguous() if pad is not None else None
+        pad = _bytes(pad) if pad is not None else None
         B, N, C = x.shape
         y = torch.empty_like(x)
         with torch.cuda.device(x.device):
@@ -295,7 +301,7 @@ class _PairHead(torch.autograd.Function):
         a = a.contiguous()
         b = b.to(a.dtype).contiguous()
         coords = coords.detach().float().contiguous()
-        valid = valid.to(torch.uint8).contiguous()
+        valid = _bytes(valid)
         w_rbf, w_out = w_rbf.detach().float().contiguous(), w_out.detach().float().reshape(-1).contiguous()
         b_out, centers = b_out.detach().float().reshape(-1).contiguous(), centers.detach().float().contiguous()
         B, N, _ = a.shape
