@@ -442,6 +442,18 @@ int mf_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* shift, const
 int mf_ln_modulate_bwd(const void* dh, int32_t dh_dtype, const void* x, int32_t x_dtype, const float* scale,
                        const float* mean, const float* rstd, int32_t batch, int32_t tokens, int32_t channels, void* dx,
                        float* dshift, float* dscale, void* stream);
+/*
+ * The gated residual (below) and the norm behind it in one pass: y = x + gate[b,:] * a, zeros where pad (NULL or (B,N) bytes)
+ * says so, in x's type, then h = LayerNorm(y) * (1 + scale) + shift; a and h share a type (h_dtype).  The backward call is
+ * mf_ln_modulate_add_bwd, which adds `add` (NULL or (B,N,C) in x's type), the gradient that reaches y past the norm, to dx,
+ * followed by mf_gated_residual_bwd.
+ */
+int mf_gated_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* gate, const void* a, const uint8_t* pad,
+                             const float* shift, const float* scale, int32_t batch, int32_t tokens, int32_t channels, float eps,
+                             int32_t h_dtype, void* y, void* h, float* mean, float* rstd, void* stream);
+int mf_ln_modulate_add_bwd(const void* dh, int32_t dh_dtype, const void* x, int32_t x_dtype, const float* scale,
+                           const float* mean, const float* rstd, const void* add, int32_t batch, int32_t tokens,
+                           int32_t channels, void* dx, float* dshift, float* dscale, void* stream);
 
 /*
  * y = x + gate[b,:] * a, the gated residual of AdaLNBlock.forward, transformer.py:308-316.  x, y (B,N,C) fp32 or bf16

@@ -63,6 +63,8 @@ EXPORTED_SYMBOLS = (
     "mf_feature_flags",
     "mf_ln_modulate_fwd",
     "mf_ln_modulate_bwd",
+    "mf_gated_ln_modulate_fwd",
+    "mf_ln_modulate_add_bwd",
     "mf_masked_sum",
     "mf_gated_residual_fwd",
     "mf_gated_residual_bwd",
@@ -348,6 +350,12 @@ def lib() -> ctypes.CDLL:
     L.mf_ln_modulate_bwd.argtypes = [c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_int32,
                                      c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p]  # fmt: skip
     L.mf_ln_modulate_bwd.restype = c_int32
+    L.mf_gated_ln_modulate_fwd.argtypes = [c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
+                                           c_int32, ctypes.c_float, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]  # fmt: skip
+    L.mf_gated_ln_modulate_fwd.restype = c_int32
+    L.mf_ln_modulate_add_bwd.argtypes = [c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
+                                         c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p]  # fmt: skip
+    L.mf_ln_modulate_add_bwd.restype = c_int32
     L.mf_gated_residual_fwd.argtypes = [c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int32,
                                         c_int32, c_void_p, c_void_p]  # fmt: skip
     L.mf_gated_residual_fwd.restype = c_int32

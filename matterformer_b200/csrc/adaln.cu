@@ -51,13 +51,26 @@ __device__ __forceinline__ void st8<__nv_bfloat16>(__nv_bfloat16* p, const float
   *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-template <typename TX, typename TH, int VEC>
+// The gated residual in front of the norm (the block's previous sub-layer): x + gate_b * a, zeros where `pad` says so,
+// written to y in x's type and normalised from there.
+template <typename TX, typename TA>
+struct GatedInput {
+  const float* gate;
+  const TA* a;
+  const uint8_t* pad;
+  TX* y;
+};
+
+// kGated: one pass for the gated residual and the norm behind it (bound by HBM: x is not read again; 33 -> 22 us for 29 696 rows
+// of 512 in bf16, and a launch less, which is what counts for a small batch).
+template <typename TX, typename TH, int VEC, bool kGated = false>
 __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const TX* __restrict__ x,
                                                                          const float* __restrict__ shift,
                                                                          const float* __restrict__ scale, int N, int C,
                                                                          float eps, TH* __restrict__ h,
                                                                          float* __restrict__ mean_out,
-                                                                         float* __restrict__ rstd_out) {
+                                                                         float* __restrict__ rstd_out,
+                                                                         GatedInput<TX, TH> in = {}) {
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* sh = shift + (size_t)b * C;
   const float* sc = scale + (size_t)b * C;
@@ -74,6 +87,18 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
       const int v = lane + 32 * t;
       if (v < nvec) {
         ld8<TX>(xr + 8 * v, xv[t]);
+        if constexpr (kGated) {
+          float av[8], gv[8];
+          ld8<TH>(in.a + row * C + 8 * v, av);
+          ld8<float>(in.gate + (size_t)b * C + 8 * v, gv);
+          const bool hidden = in.pad && in.pad[row];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            xv[t][e] = hidden ? 0.f : fmaf(gv[e], av[e], xv[t][e]);
+            if constexpr (sizeof(TX) == 2) xv[t][e] = __bfloat162float(__float2bfloat16_rn(xv[t][e]));  // what is stored is what is normalised
+          }
+          st8<TX>(in.y + row * C + 8 * v, xv[t]);
+        }
         ld8<float>(sc + 8 * v, scv[t]);
         ld8<float>(sh + 8 * v, shv[t]);
 #pragma unroll
@@ -132,7 +157,7 @@ __device__ __forceinline__ void molecule_column_sums(float* part, const float (&
 
 // dx, and per molecule dshift[c] = sum_n dh, dscale[c] = sum_n dh * xhat.  One sweep: the row's dh and xhat stay in
 // registers between the two row sums and the store.
-template <typename TX, typename TH, int VEC>
+template <typename TX, typename TH, int VEC, bool kAdd>
 __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const TH* __restrict__ dh,
                                                                          const TX* __restrict__ x,
                                                                          const float* __restrict__ scale,
@@ -140,7 +165,8 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
                                                                          const float* __restrict__ rstd_in, int N, int C,
                                                                          TX* __restrict__ dx,
                                                                          float* __restrict__ dshift,
-                                                                         float* __restrict__ dscale) {
+                                                                         float* __restrict__ dscale,
+                                                                         const TX* __restrict__ add) {
   extern __shared__ __align__(16) float part[];  // [kAdaWarps][C]
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* sc = scale + (size_t)b * C;
@@ -161,7 +187,7 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
   for (int n = warp; n < N; n += kAdaWarps) {
     const size_t row = (size_t)b * N + n;
     const float mean = mean_in[row], rstd = rstd_in[row];
-    float g[VEC][8], xh[VEC][8];
+    float g[VEC][8], xh[VEC][8], more[kAdd ? VEC : 1][8];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int t = 0; t < VEC; ++t) {
@@ -169,6 +195,7 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
       if (v < nvec) {
         ld8<TH>(dh + row * C + 8 * v, g[t]);
         ld8<TX>(x + row * C + 8 * v, xh[t]);
+        if constexpr (kAdd) ld8<TX>(add + row * C + 8 * v, more[t]);  // the gradient that reaches x past the norm
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           xh[t][e] = (xh[t][e] - mean) * rstd;
@@ -189,6 +216,10 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
         float out[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) out[e] = rstd * (g[t][e] - s1 - xh[t][e] * s2);
+        if constexpr (kAdd) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) out[e] += more[t][e];
+        }
         st8<TX>(dx + row * C + 8 * v, out);
       }
     }
@@ -272,6 +303,12 @@ int check_sizes(const char* name, int batch, int tokens, int channels, int half_
   return MF_OK;
 }
 
+// forward norms: enough CTAs for four per SM, at most one row per warp
+dim3 rows_grid(int batch, int tokens) {
+  const int rows = (tokens + kAdaWarps - 1) / kAdaWarps, wanted = (592 + batch - 1) / batch;
+  return dim3(batch, rows < wanted ? (rows > 0 ? rows : 1) : wanted);
+}
+
 }  // namespace
 }  // namespace mf
 
@@ -324,9 +361,7 @@ extern "C" int mf_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* s
   MF_CHECK_ARG(x && shift && scale && h && mean && rstd, "mf_ln_modulate_fwd: null pointer argument");
   MF_CHECK_ALIGNED("mf_ln_modulate_fwd", x, shift, scale, h);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // enough CTAs for four per SM, at most one row per warp
-  const int rows = (tokens + kAdaWarps - 1) / kAdaWarps, wanted = (592 + batch - 1) / batch;
-  const dim3 grid(batch, rows < wanted ? (rows > 0 ? rows : 1) : wanted);
+  const dim3 grid = rows_grid(batch, tokens);
   MF_ADA_DISPATCH(x_dtype, h_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
                              (ln_modulate_fwd_kernel<TX, TH, VEC><<<grid, kAdaWarps * 32, 0, s>>>(
@@ -336,24 +371,52 @@ extern "C" int mf_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* s
   return MF_OK;
 }
 
-extern "C" int mf_ln_modulate_bwd(const void* dh, int32_t dh_dtype, const void* x, int32_t x_dtype, const float* scale,
-                                  const float* mean, const float* rstd, int32_t batch, int32_t tokens, int32_t channels,
-                                  void* dx, float* dshift, float* dscale, void* stream) {
+extern "C" int mf_gated_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* gate, const void* a, const uint8_t* pad,
+                                        const float* shift, const float* scale, int32_t batch, int32_t tokens, int32_t channels,
+                                        float eps, int32_t h_dtype, void* y, void* h, float* mean, float* rstd, void* stream) {
+  int rc = check_sizes("mf_gated_ln_modulate_fwd", batch, tokens, channels, h_dtype);
+  if (rc == MF_OK) rc = check_sizes("mf_gated_ln_modulate_fwd", batch, tokens, channels, x_dtype);
+  if (rc != MF_OK) return rc;
+  if (batch == 0 || tokens == 0) return MF_OK;
+  MF_CHECK_ARG(x && gate && a && shift && scale && y && h && mean && rstd, "mf_gated_ln_modulate_fwd: null pointer argument");
+  MF_CHECK_ALIGNED("mf_gated_ln_modulate_fwd", x, gate, a, shift, scale, y, h);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const dim3 grid = rows_grid(batch, tokens);
+  MF_ADA_DISPATCH(x_dtype, h_dtype, TX, TH,
+                  MF_ADA_VEC(channels, VEC,
+                             (ln_modulate_fwd_kernel<TX, TH, VEC, true><<<grid, kAdaWarps * 32, 0, s>>>(
+                                 static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
+                                 rstd, GatedInput<TX, TH>{gate, static_cast<const TH*>(a), pad, static_cast<TX*>(y)}))));
+  MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
+  return MF_OK;
+}
+
+extern "C" int mf_ln_modulate_add_bwd(const void* dh, int32_t dh_dtype, const void* x, int32_t x_dtype, const float* scale,
+                                      const float* mean, const float* rstd, const void* add, int32_t batch, int32_t tokens,
+                                      int32_t channels, void* dx, float* dshift, float* dscale, void* stream) {
   int rc = check_sizes("mf_ln_modulate_bwd", batch, tokens, channels, dh_dtype);
   if (rc == MF_OK) rc = check_sizes("mf_ln_modulate_bwd", batch, tokens, channels, x_dtype);
   if (rc != MF_OK) return rc;
   if (batch == 0) return MF_OK;
   MF_CHECK_ARG(dh && x && scale && mean && rstd && dx && dshift && dscale, "mf_ln_modulate_bwd: null pointer argument");
-  MF_CHECK_ALIGNED("mf_ln_modulate_bwd", dh, x, scale, dx, dshift, dscale);
+  MF_CHECK_ALIGNED("mf_ln_modulate_bwd", dh, x, scale, add, dx, dshift, dscale);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t smem = (size_t)kAdaWarps * channels * sizeof(float);
   MF_ADA_DISPATCH(x_dtype, dh_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
-                             (ln_modulate_bwd_kernel<TX, TH, VEC><<<batch, kAdaWarps * 32, smem, s>>>(
+                             auto kernel = add ? ln_modulate_bwd_kernel<TX, TH, VEC, true> : ln_modulate_bwd_kernel<TX, TH, VEC, false>;
+                             kernel<<<batch, kAdaWarps * 32, smem, s>>>(
                                  static_cast<const TH*>(dh), static_cast<const TX*>(x), scale, mean, rstd, tokens, channels,
-                                 static_cast<TX*>(dx), dshift, dscale))));
+                                 static_cast<TX*>(dx), dshift, dscale, static_cast<const TX*>(add))));
   MF_CHECK_LAUNCH("ln_modulate_bwd_kernel");
   return MF_OK;
+}
+
+extern "C" int mf_ln_modulate_bwd(const void* dh, int32_t dh_dtype, const void* x, int32_t x_dtype, const float* scale,
+                                  const float* mean, const float* rstd, int32_t batch, int32_t tokens, int32_t channels,
+                                  void* dx, float* dshift, float* dscale, void* stream) {
+  return mf_ln_modulate_add_bwd(dh, dh_dtype, x, x_dtype, scale, mean, rstd, nullptr, batch, tokens, channels, dx, dshift, dscale,
+                                stream);
 }
 
 extern "C" int mf_gated_residual_fwd(const void* x, int32_t x_dtype, const float* gate, const void* a, int32_t a_dtype,

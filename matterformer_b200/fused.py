@@ -118,6 +118,49 @@ def gated_residual(x: torch.Tensor, gate: torch.Tensor, a: torch.Tensor,
     return _GatedResidual.apply(x, gate, a, pad_mask)
 
 
+class _GatedLnModulate(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, gate, a, pad, shift, scale, eps):
+        x, a = x.contiguous(), a.contiguous()
+        gate, shift, scale = gate.contiguous(), shift.contiguous(), scale.contiguous()
+        pad = _bytes(pad) if pad is not None else None
+        B, N, C = x.shape
+        y, h = torch.empty_like(x), torch.empty_like(a)
+        mean = torch.empty((B, N), device=x.device, dtype=torch.float32)
+        rstd = torch.empty_like(mean)
+        _lib.launch(_lib.lib().mf_gated_ln_modulate_fwd, x.device, x.data_ptr(), _CODE[x.dtype], gate.data_ptr(), a.data_ptr(),
+                    pad.data_ptr() if pad is not None else None, shift.data_ptr(), scale.data_ptr(), B, N, C, float(eps),
+                    _CODE[a.dtype], y.data_ptr(), h.data_ptr(), mean.data_ptr(), rstd.data_ptr())  # fmt: skip
+        ctx.save_for_backward(gate, a, pad, scale, y, mean, rstd)
+        return y, h
+
+    @staticmethod
+    def backward(ctx, dy, dh):
+        gate, a, pad, scale, y, mean, rstd = ctx.saved_tensors
+        B, N, C = y.shape
+        dy, dh = dy.to(y.dtype).contiguous(), dh.to(a.dtype).contiguous()
+        total, da = torch.empty_like(y), torch.empty_like(a)
+        dx = torch.empty_like(y) if pad is not None else None
+        dgate, dshift, dscale = torch.empty((3, B, C), device=y.device, dtype=torch.float32).unbind(0)
+        _lib.launch(_lib.lib().mf_ln_modulate_add_bwd, y.device, dh.data_ptr(), _CODE[dh.dtype], y.data_ptr(), _CODE[y.dtype],
+                    scale.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dy.data_ptr(), B, N, C, total.data_ptr(),
+                    dshift.data_ptr(), dscale.data_ptr())  # fmt: skip
+        _lib.launch(_lib.lib().mf_gated_residual_bwd, y.device, total.data_ptr(), _CODE[total.dtype], gate.data_ptr(), a.data_ptr(),
+                    _CODE[a.dtype], pad.data_ptr() if pad is not None else None, B, N, C, da.data_ptr(),
+                    dx.data_ptr() if dx is not None else None, dgate.data_ptr())  # fmt: skip
+        return total if dx is None else dx, dgate, da, None, dshift, dscale, None
+
+
+def gated_ln_modulate(x: torch.Tensor, gate: torch.Tensor, a: torch.Tensor, pad_mask: Optional[torch.Tensor], shift: torch.Tensor,
+                      scale: torch.Tensor, *, eps: float, out_dtype: torch.dtype) -> tuple:  # fmt: skip
+    """``y = gated_residual(x, gate, a, pad_mask)`` and ``ln_modulate(y, shift, scale)``; one pass where ``a`` already has
+    ``out_dtype`` and the modulation is fp32, the two operators otherwise."""
+    if a.dtype == out_dtype and a.dtype in _CODE and all(t.dtype == torch.float32 for t in (gate, shift, scale)):
+        return _GatedLnModulate.apply(x, gate, a, pad_mask, shift, scale, eps)
+    y = gated_residual(x, gate, a, pad_mask)
+    return y, ln_modulate(y, shift, scale, eps=eps, out_dtype=out_dtype)
+
+
 class _SplitModulation(torch.autograd.Function):
     """(B, 6 C) -> six contiguous fp32 (B, C) tensors in one copy; the backward pass gathers the six gradients in one
     concatenation and one cast."""

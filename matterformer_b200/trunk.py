@@ -28,7 +28,7 @@ import torch.nn.functional as F
 from torch import nn
 
 from . import fused
-from .fused import (fused_applies, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
+from .fused import (fused_applies, gated_ln_modulate, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
                     split_modulation)
 from .linear import (linear_bf16, linear_bf16_applies, linear_gelu_bf16, refresh_bf16_copies, refresh_must_be_captured, stacked_bf16_copies,
                      stacked_modulation)  # fmt: skip
@@ -337,12 +337,13 @@ class AdaLNBlock(nn.Module):
         self.fused_elementwise = True  # CUDA fp32 residual stream: fused norm+modulate and gated-residual kernels
 
     def forward(self, x, cond_emb, *, pad_mask=None, simplicial_attention_mask=None, sparse_plan=None,
-                zero_padding: bool = False, cond_act=None, modulation=None, num_atoms=None):
+                zero_padding: bool = False, cond_act=None, modulation=None, num_atoms=None, h=None, following=None):
         """``zero_padding``: return the block's output with its padded rows cleared (the ``masked_fill`` the trunk
         applies before the next block), folded into the last fused pass when the fused kernels run.  ``cond_act``:
         ``SiLU(cond_emb)`` when the caller has already formed it (it is the same for every block of a trunk).
         ``modulation``: the six modulation tensors, formed by the trunk for all its blocks at once; ``num_atoms``: counts of
-        real tokens for the attention layer."""
+        real tokens for the attention layer.  ``following``: (shift, scale, eps) of the norm that opens the next block; the
+        block then returns its output and that norm's, formed in one pass, and the next block takes the latter as ``h``."""
         fused = self.fused_elementwise and fused_applies(x)
         mod = None if modulation is not None else linear_bf16(cond_act if cond_act is not None else self.ada_ln[0](cond_emb), self.ada_ln[-1].weight,
                           self.ada_ln[-1].bias)  # fmt: skip
@@ -354,7 +355,8 @@ class AdaLNBlock(nn.Module):
             # activations are written in bf16, which is what the Linear layers that consume them cast to anyway
             low = torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
             h_dtype = torch.bfloat16 if (low or x.dtype == torch.bfloat16) else torch.float32
-            h = ln_modulate(x, shift_a, scale_a, eps=self.norm1.eps, out_dtype=h_dtype)
+            if h is None:
+                h = ln_modulate(x, shift_a, scale_a, eps=self.norm1.eps, out_dtype=h_dtype)
         else:
             h = _modulate(self.norm1(x), shift_a, scale_a)
         if self.attn_type == "mha":
@@ -362,9 +364,12 @@ class AdaLNBlock(nn.Module):
         else:
             attn_out = self.attn(h, key_padding_mask=pad_mask, attention_mask=simplicial_attention_mask)
         if fused:
-            x = gated_residual(x, gate_a, attn_out)
-            h = ln_modulate(x, shift_m, scale_m, eps=self.norm2.eps, out_dtype=h_dtype)
-            return gated_residual(x, gate_m, self.mlp(h), pad_mask if zero_padding else None)
+            x, h = gated_ln_modulate(x, gate_a, attn_out, None, shift_m, scale_m, eps=self.norm2.eps, out_dtype=h_dtype)
+            pad = pad_mask if zero_padding else None
+            if following is not None:
+                shift, scale, eps = following
+                return gated_ln_modulate(x, gate_m, self.mlp(h), pad, shift, scale, eps=eps, out_dtype=h_dtype)
+            return gated_residual(x, gate_m, self.mlp(h), pad)
         x = x + gate_a[:, None, :] * attn_out
         h = _modulate(self.norm2(x), shift_m, scale_m)
         x = x + gate_m[:, None, :] * self.mlp(h)
@@ -436,9 +441,14 @@ class TransformerTrunk(nn.Module):
             modulation = stacked_modulation(cond_act, self._modulation_w16, self._modulation_b16,
                                             [m.weight for m in layers] + [m.bias for m in layers], len(layers))  # fmt: skip
         num_atoms = (~pad_mask).sum(dim=1).to(torch.int32) if x.is_cuda and pad_mask is not None else None
-        for block, six in zip(self.blocks, modulation):
+        h = None
+        for i, (block, six) in enumerate(zip(self.blocks, modulation)):
+            chain = stacked and i + 1 < len(self.blocks)  # the next block's first norm in one pass with this one's output
+            following = (*modulation[i + 1][:2], self.blocks[i + 1].norm1.eps) if chain else None
             x = block(x, cond_emb, pad_mask=pad_mask, simplicial_attention_mask=sim_mask, sparse_plan=sparse_plan,
-                      zero_padding=pad_mask is not None, cond_act=cond_act, modulation=six, num_atoms=num_atoms)
+                      zero_padding=pad_mask is not None, cond_act=cond_act, modulation=six, num_atoms=num_atoms, h=h,
+                      following=following)
+            x, h = x if chain else (x, None)
         x = layer_norm(x, self.norm_out)
         if pad_mask is not None:
             x = x.masked_fill(pad_mask[..., None], 0.0)
