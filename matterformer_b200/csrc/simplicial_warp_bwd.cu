@@ -13,8 +13,8 @@
 // meets in shared memory and is added up in a fixed order, so results are bit-identical from run to run.
 //
 // Bound by latency: two warps per scheduler (255 registers) issue an instruction in every third cycle, the tensor pipe is busy
-// for a fifth of the time.  64 molecules of 20-181 atoms, 8 heads: 5.65 ms, against 7.81 ms of 128-query tcgen05 tiles, which
-// waited for the bias and for the sums over rows and columns of every tile; 32 molecules of 20-64 atoms 0.26 against 0.43 ms.
+// for a fifth of the time.  64 molecules of 20-181 atoms, 8 heads: 5.91 ms, against 7.81 ms of 128-query tcgen05 tiles, which
+// waited for the bias and for the sums over rows and columns of every tile; 32 molecules of 20-64 atoms 0.27 against 0.43 ms.
 // Without a bias those tiles have little to wait for, and row-packed ones (simplicial_rows_bwd.cu) are the faster kernel: 1.97
 // against 3.8 ms.
 #include "common.cuh"
