@@ -41,9 +41,9 @@ if str(ROOT) not in sys.path:
 NAMES = ("q", "k1", "v1", "k2", "v2")
 METRIC = "2-simplicial attn fwd+bwd TFLOP/s"
 L2_FLUSH_BYTES = 512 << 20
-# Kernels this library launches per forward + backward pass of the headline workload (row-packed path): forward =
-# extents, launch order, main; backward = extents, launch order, delta, main, finalize.
-SIMPLICIAL_LAUNCHES_PER_STEP = 3 + 5
+# Kernels this library launches per forward + backward pass of the headline workload: forward = one; backward
+# (row-packed path) = extents, launch order, delta, main, finalize.
+SIMPLICIAL_LAUNCHES_PER_STEP = 1 + 5
 # DRAM bytes (read + written) of ONE launch of the backward kernel on the headline workload, from an ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum); None when no capture of the current kernel exists.
 BWD_KERNEL_DRAM_BYTES = 67_346_432  # 45 445 632 read + 21 900 800 written, captured on this workload
@@ -470,7 +470,7 @@ def run_simplicial(args, world, rank, local) -> dict:
         "roofline": {"bound": "tensor", "achieved": bwd_tflops, "peak": peaks["tflops"], "unit": "TFLOP/s",
                      "frac": (bwd_tflops / peaks["tflops"]) if bwd_tflops else None, "traffic": BWD_KERNEL_DRAM_BYTES,
                      "kernel": "simplicial_rows_bwd_kernel", "peak_source": peaks["source"] + " (burst)",
-                     "kernel_ms": bwd_ms / max(bwd_n, 1), "fwd_kernel": "simplicial_rows_fwd_kernel",
+                     "kernel_ms": bwd_ms / max(bwd_n, 1), "fwd_kernel": "simplicial_warp_fwd_kernel",
                      "fwd_kernel_tflops": fwd_tflops, "fwd_kernel_ms": fwd_ms / max(fwd_n, 1),
                      "fwd_frac": (fwd_tflops / peaks["tflops"]) if fwd_tflops else None},
         "e2e": {"value": e2e_value, "unit": "TFLOP/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
@@ -501,7 +501,7 @@ def run_sparse(workload: str, steps: int, warmup: int, world, rank, local, with_
         step = lambda: mfb.knn_topk(pos, cell, na, k=16)  # noqa: E731
         units = pos.shape[0] * pos.shape[1]
         bytes_alg = units * (12 + 16 * 4 + 16 * 4)
-        metric, unit, name, launches = "periodic kNN k=16 points/s", "points/s", "knn_B32_N4096_k16", 7
+        metric, unit, name, launches = "periodic kNN k=16 points/s", "points/s", "knn_B32_N4096_k16", 2  # set-up, search
         host_out = [torch.empty(*pos.shape[:2], 16, dtype=torch.int32).pin_memory(),
                     torch.empty(*pos.shape[:2], 16, dtype=torch.float32).pin_memory()]  # fmt: skip
 
@@ -537,7 +537,7 @@ def run_sparse(workload: str, steps: int, warmup: int, world, rank, local, with_
             name = "local_attn_fwd_bwd_B32_N4096_H8_D64_w64"
             kn = "k_"
             pairs = None
-            extra["kernels"] = "tcgen05, 128-row tiles" if mfb.sparse._SPARSE_BACKEND == "tcgen05" else "mma.sync, 32-row tiles"
+            extra["kernels"] = "tcgen05, 128-row tiles" if mfb.sparse._SPARSE_BACKEND == "tcgen05" else "mma.sync, one load of the band"
         go = t["grad_out"].to(dev)
 
         def step():
@@ -547,7 +547,7 @@ def run_sparse(workload: str, steps: int, warmup: int, world, rank, local, with_
         units = q.shape[0] * q.shape[2]
         nbytes = q.numel() * 2
         bytes_alg = 4 * nbytes + 8 * nbytes  # fwd: q,k,v,o; bwd: q,k,v,o,do + dq,dk,dv
-        metric, unit, launches = f"{workload} attention fwd+bwd atoms/s", "atoms/s", 3  # forward, dq (+ delta), dk+dv
+        metric, unit, launches = f"{workload} attention fwd+bwd atoms/s", "atoms/s", 3 if workload == "radius" else 2  # forward, backward (radius: dq, dk + dv)
         host_in = [t[n].pin_memory() for n in ("q", kn, "v", "grad_out")]
         host_out = [torch.empty_like(t["q"]).pin_memory() for _ in range(4)]
 
@@ -618,9 +618,9 @@ def run_sparse(workload: str, steps: int, warmup: int, world, rank, local, with_
 
 def run_bias(steps: int, warmup: int, world, rank, local, shape: str = "small", with_reference_kernels: bool = True) -> dict:
     """2-simplicial attention with the factorized geometry bias (the reference model's default geometry mode,
-    models/qm9.py:261), forward + backward on the tcgen05 tile kernels, which add the bias to the logits in fp32 and
+    models/qm9.py:261), forward + backward on the warp-level kernels, which add the bias to the logits in fp32 and
     form its four gradients in the backward kernel's element-wise pass.  ``shape`` "small": 256 molecules of 9..29
-    atoms, four heads per tile; "config2": the benchmark batch (64 molecules of 128..192 atoms), one head per tile."""
+    atoms; "config2": the benchmark batch."""
     import matterformer_b200 as mfb
     from matterformer_b200 import synthetic
 
@@ -655,8 +655,7 @@ def run_bias(steps: int, warmup: int, world, rank, local, shape: str = "small", 
     return {
         "metric": METRIC, "value": tf, "unit": "TFLOP/s", "ms_per_step": ms / steps, "scaling": "weak", "dtype": "bf16",
         "config": {"workload": f"simplicial_fwd_bwd_factorized_bias_B{B}_N{N}_H{H}_D{D}",
-                   "kernels": "tcgen05 tile kernels, %s, bias added in fp32" % ("one head per tile" if shape == "config2"
-                                                                                else "four heads per tile"),
+                   "kernels": "warp-level mma.sync kernels, bias added in fp32",
                    "gradients": "q, k1, v1, k2, v2, u, v_bias, w, gate", "kernel_to_beat": k2b},
         "roofline": {"bound": "tensor", "achieved": tf, "peak": peaks["tflops"], "unit": "TFLOP/s",
                      "frac": tf / peaks["tflops"], "peak_source": peaks["source"],
