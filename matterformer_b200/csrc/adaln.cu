@@ -33,6 +33,27 @@ __device__ __forceinline__ void ld8<__nv_bfloat16>(const __nv_bfloat16* p, float
 #pragma unroll
   for (int e = 0; e < 4; ++e) v[2 * e] = __uint_as_float(w[e] << 16), v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
 }
+// Eight channels as they are in memory, to be unpacked when they are used
+template <typename T>
+struct Raw8 {
+  uint4 w[sizeof(T) / 2];
+  __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) w[i] = reinterpret_cast<const uint4*>(p)[i];
+  }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    const uint32_t u[4] = {w[0].x, w[0].y, w[0].z, w[0].w};
+    if constexpr (sizeof(T) == 2) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[2 * e] = __uint_as_float(u[e] << 16), v[2 * e + 1] = __uint_as_float(u[e] & 0xffff0000u);
+    } else {
+      const uint4 h = w[1];
+      const uint32_t t[8] = {u[0], u[1], u[2], u[3], h.x, h.y, h.z, h.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(t[e]);
+    }
+  }
+};
 template <typename T>
 __device__ __forceinline__ void st8(T* p, const float (&v)[8]);
 template <>
@@ -172,36 +193,58 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
   const float* sc = scale + (size_t)b * C;
   const int nvec = C >> 3;
   const float inv_c = 1.f / (float)C;
-  float a_shift[VEC][8], a_scale[VEC][8], one_plus[VEC][8];
+  float* one_plus = part + kAdaWarps * C;  // 1 + scale
+  for (int c = threadIdx.x; c < C; c += kAdaWarps * 32) one_plus[c] = 1.f + sc[c];
+  __syncthreads();
+  float a_shift[VEC][8], a_scale[VEC][8];
 #pragma unroll
-  for (int t = 0; t < VEC; ++t) {
-    const int v = lane + 32 * t;
+  for (int t = 0; t < VEC; ++t)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a_shift[t][e] = 0.f, a_scale[t][e] = 0.f, one_plus[t][e] = 1.f;
-    if (v < nvec) {
-      ld8<float>(sc + 8 * v, one_plus[t]);
+    for (int e = 0; e < 8; ++e) a_shift[t][e] = 0.f, a_scale[t][e] = 0.f;
+  // the next row is on its way while this one goes through its sums (a row took 2.7 us, most of it the wait for its loads)
+  Raw8<TH> next_g[VEC];
+  Raw8<TX> next_x[VEC], next_more[kAdd ? VEC : 1];
+  float next_mean = 0.f, next_rstd = 0.f;
+  auto fetch = [&](int n) {
+    if (n >= N) return;
+    const size_t row = (size_t)b * N + n;
+    next_mean = mean_in[row], next_rstd = rstd_in[row];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) one_plus[t][e] += 1.f;
+    for (int t = 0; t < VEC; ++t) {
+      const int v = lane + 32 * t;
+      if (v < nvec) {
+        next_g[t].load(dh + row * C + 8 * v);
+        next_x[t].load(x + row * C + 8 * v);
+        if constexpr (kAdd) next_more[t].load(add + row * C + 8 * v);  // the gradient that reaches x past the norm
+      }
     }
-  }
+  };
+  fetch(warp);
   for (int n = warp; n < N; n += kAdaWarps) {
     const size_t row = (size_t)b * N + n;
-    const float mean = mean_in[row], rstd = rstd_in[row];
-    float g[VEC][8], xh[VEC][8], more[kAdd ? VEC : 1][8];
+    const float mean = next_mean, rstd = next_rstd;
+    float g[VEC][8], xh[VEC][8];
+    Raw8<TX> more[kAdd ? VEC : 1];
+#pragma unroll
+    for (int t = 0; t < VEC; ++t) {
+      next_g[t].get(g[t]);
+      next_x[t].get(xh[t]);
+      if constexpr (kAdd) more[t] = next_more[t];
+    }
+    fetch(n + kAdaWarps);
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int t = 0; t < VEC; ++t) {
       const int v = lane + 32 * t;
       if (v < nvec) {
-        ld8<TH>(dh + row * C + 8 * v, g[t]);
-        ld8<TX>(x + row * C + 8 * v, xh[t]);
-        if constexpr (kAdd) ld8<TX>(add + row * C + 8 * v, more[t]);  // the gradient that reaches x past the norm
+        float scaled[8];
+        ld8<float>(one_plus + 8 * v, scaled);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           xh[t][e] = (xh[t][e] - mean) * rstd;
           a_shift[t][e] += g[t][e];
           a_scale[t][e] = fmaf(g[t][e], xh[t][e], a_scale[t][e]);
-          g[t][e] *= one_plus[t][e];  // gradient of the normalised row
+          g[t][e] *= scaled[e];  // gradient of the normalised row
           s1 += g[t][e];
           s2 = fmaf(g[t][e], xh[t][e], s2);
         }
@@ -217,8 +260,10 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
 #pragma unroll
         for (int e = 0; e < 8; ++e) out[e] = rstd * (g[t][e] - s1 - xh[t][e] * s2);
         if constexpr (kAdd) {
+          float past[8];
+          more[t].get(past);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) out[e] += more[t][e];
+          for (int e = 0; e < 8; ++e) out[e] += past[e];
         }
         st8<TX>(dx + row * C + 8 * v, out);
       }
@@ -402,7 +447,7 @@ extern "C" int mf_ln_modulate_add_bwd(const void* dh, int32_t dh_dtype, const vo
   MF_CHECK_ARG(dh && x && scale && mean && rstd && dx && dshift && dscale, "mf_ln_modulate_bwd: null pointer argument");
   MF_CHECK_ALIGNED("mf_ln_modulate_bwd", dh, x, scale, add, dx, dshift, dscale);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t smem = (size_t)kAdaWarps * channels * sizeof(float);
+  const size_t smem = (size_t)(kAdaWarps + 1) * channels * sizeof(float);
   MF_ADA_DISPATCH(x_dtype, dh_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
                              auto kernel = add ? ln_modulate_bwd_kernel<TX, TH, VEC, true> : ln_modulate_bwd_kernel<TX, TH, VEC, false>;
