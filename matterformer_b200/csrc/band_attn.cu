@@ -9,6 +9,10 @@
 // queries (dq), then as keys (dk, dv), from the same shared rows; delta = dO . out is formed on load.  Every output row has
 // one owner: no atomics, bit-identical reruns.
 //
+// W = 0: structures of at most 32 tokens under a window that reaches every pair (a trunk's molecules).  The halo is the tile itself,
+// a warp sees two chunks, and nothing but the structure's end is masked.  1 024 molecules of 9 - 29 tokens x 8
+// heads: forward 37 -> 25 us, backward 104 -> 53 us (two launches of the 32-row walk before).
+//
 // What bounds it: shared memory, 66 % of its bandwidth (operand fragments, at 16 rows per warp), while a CTA's loads overlap
 // only with the other CTAs of the SM.  32 cells of 4096 tokens x 8 heads, window 64: forward 144 us, backward 382 us (HBM
 // floors 82 and 164 us), against 219 and 311 + 322 us for the 32-row walk with its three passes.
@@ -107,9 +111,10 @@ __device__ __forceinline__ void store_rows(__nv_bfloat16* dst, long long stride,
 }
 
 template <int W, int kRows>
-__global__ void __launch_bounds__(kRows * 2, W == 128 ? (kRows == 128 ? 2 : 4) : (kRows == 128 ? 3 : 6)) band_fwd_kernel(const __grid_constant__ BandParams p) {
+__global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 128 ? 2 : 4) : (kRows == 128 ? 3 : 6)) band_fwd_kernel(const __grid_constant__ BandParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
-  constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = W / 16 + 1;
+  constexpr bool kDense = W == 0;
+  constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = kDense ? kRows / 16 : W / 16 + 1;
   constexpr int kTv = kHalo * kRowBytes, kTq = 2 * kTv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
   const int t0 = blockIdx.x * kRows, bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H, N = p.N;
@@ -126,7 +131,9 @@ __global__ void __launch_bounds__(kRows * 2, W == 128 ? (kRows == 128 ? 2 : 4) :
   }
   const int i0 = t0 + warp * 16, row = i0 + row8;  // the lane's rows: row and row + 8
   if (i0 >= N) return;
-  const FragBase fb(tile + warp * 16 * kRowBytes, lane);  // everything a warp reads lies at fixed offsets from its rows
+  // everything a warp reads lies at fixed offsets from its rows (dense: from the structure's first)
+  const FragBase fb(tile + (kDense ? 0 : warp * 16 * kRowBytes), lane);
+  const int mine = kDense ? warp * 16 * kRowBytes : 0;
   float o[8][4], l[2] = {0.f, 0.f}, shift[2] = {0.f, 0.f};
 #pragma unroll
   for (int t = 0; t < 8; ++t)
@@ -135,12 +142,12 @@ __global__ void __launch_bounds__(kRows * 2, W == 128 ? (kRows == 128 ? 2 : 4) :
   if (i0 < n) {
     uint32_t q[4][4];
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) load_a(q[ks], fb, kTq, 0, ks);
+    for (int ks = 0; ks < 4; ++ks) load_a(q[ks], fb, kTq + mine, 0, ks);
     const float sc2 = p.scale * kLog2e;
     // hidden pairs of chunk c: the two triangles, and keys outside the structure
     auto logits = [&](float(&s)[2][4], int c) {
       chunk_product(s, q, fb, c * 16 * kRowBytes);
-      const int key0 = i0 - kHalf + 16 * c;
+      const int key0 = kDense ? 16 * c : i0 - kHalf + 16 * c;
       const bool ends = key0 < 0 || key0 + 16 > n;
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
@@ -148,8 +155,8 @@ __global__ void __launch_bounds__(kRows * 2, W == 128 ? (kRows == 128 ? 2 : 4) :
         for (int e = 0; e < 4; ++e) {
           const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
           bool seen = true;
-          if (c == 0) seen = rel >= r;
-          if (c == kChunks - 1) seen = rel < r;
+          if (!kDense && c == 0) seen = rel >= r;
+          if (!kDense && c == kChunks - 1) seen = rel < r;
           if (ends) seen = seen && key0 + rel >= 0 && key0 + rel < n;
           s[nt][e] = seen ? s[nt][e] * sc2 : -INFINITY;
         }
@@ -217,9 +224,10 @@ __global__ void __launch_bounds__(kRows * 2, W == 128 ? (kRows == 128 ? 2 : 4) :
 }
 
 template <int W, int kRows>
-__global__ void __launch_bounds__(kRows * 2, kRows == 128 ? (W == 128 ? 1 : 2) : (W == 128 ? 2 : 3)) band_bwd_kernel(const __grid_constant__ BandParams p) {
+__global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 128 ? 1 : 2) : (W == 128 ? 2 : 3)) band_bwd_kernel(const __grid_constant__ BandParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
-  constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = W / 16 + 1;
+  constexpr bool kDense = W == 0;
+  constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = kDense ? kRows / 16 : W / 16 + 1;
   constexpr int kTk = kHalo * kRowBytes, kTv = 2 * kTk, kTg = 3 * kTk;  // q, k, v, grad_out
   float* lse = reinterpret_cast<float*>(smem + 4 * kTk);  // of the halo rows, in the log2 domain
   float* delta = lse + kHalo;
@@ -270,8 +278,10 @@ __global__ void __launch_bounds__(kRows * 2, kRows == 128 ? (W == 128 ? 1 : 2) :
   }
   const int i0 = t0 + warp * 16, row = i0 + row8;
   if (i0 >= N) return;
-  const FragBase fb(tile + warp * 16 * kRowBytes, lane);  // everything a warp reads lies at fixed offsets from its rows
-  constexpr int own = kHalf * kRowBytes;  // the warp's rows inside the halo
+  // everything a warp reads lies at fixed offsets from its rows (dense: from the structure's first)
+  const FragBase fb(tile + (kDense ? 0 : warp * 16 * kRowBytes), lane);
+  const int mine = kDense ? warp * 16 * kRowBytes : 0;
+  const int own = kHalf * kRowBytes + mine;  // the warp's rows inside the halo
   const float sc2 = p.scale * kLog2e;
   uint32_t a[4][4], g[4][4];
   float acc0[8][4], acc1[8][4];
@@ -298,8 +308,8 @@ __global__ void __launch_bounds__(kRows * 2, kRows == 128 ? (W == 128 ? 1 : 2) :
           // a logit of 0 against zero rows may give a huge weight where the row's log-sum-exp is very negative: bounded, so
           // that it stays finite and 0 . weight = 0
           float pr = fast_exp2(fminf(fmaf(s[nt][e], sc2, -(e < 2 ? la : lb)), 100.f));
-          if (c == 0 && rel < r) pr = 0.f;
-          if (c == kChunks - 1 && rel >= r) pr = 0.f;
+          if (!kDense && c == 0 && rel < r) pr = 0.f;
+          if (!kDense && c == kChunks - 1 && rel >= r) pr = 0.f;
           s[nt][e] = pr * (dp[nt][e] - (e < 2 ? da : db)) * p.scale;
         }
       uint32_t pk[4];
@@ -323,14 +333,14 @@ __global__ void __launch_bounds__(kRows * 2, kRows == 128 ? (W == 128 ? 1 : 2) :
       chunk_product(dp, g, fb, kTg + at);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
-        const int q0 = (warp + c) * 16 + nt * 8 + 2 * quad;
+        const int q0 = ((kDense ? 0 : warp) + c) * 16 + nt * 8 + 2 * quad;
         const float2 l = *reinterpret_cast<const float2*>(&lse[q0]), d = *reinterpret_cast<const float2*>(&delta[q0]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
           float pr = fast_exp2(fmaf(s[nt][e], sc2, -((e & 1) ? l.y : l.x)));
-          if (c == 0 && rel <= r) pr = 0.f;
-          if (c == kChunks - 1 && rel > r) pr = 0.f;
+          if (!kDense && c == 0 && rel <= r) pr = 0.f;
+          if (!kDense && c == kChunks - 1 && rel > r) pr = 0.f;
           s[nt][e] = pr;
           dp[nt][e] = pr * (dp[nt][e] - ((e & 1) ? d.y : d.x)) * p.scale;
         }
@@ -366,10 +376,13 @@ int launch_band(const BandParams& p, int BH, bool backward, cudaStream_t s) {
 
 }  // namespace
 
-// Windows whose chunks are whole, structures long enough that a tile is not mostly halo; shorter ones (a trunk's molecules)
-// stay on the 32-row walk.
+// Windows whose chunks are whole, structures long enough that a tile is not mostly halo, or short enough that the window
+// reaches every pair of a 32-row tile; those between stay on the 32-row walk.
+constexpr int kDenseTokens = 32;  // under windows of 64 and 128
 bool band_attn_applies(const MfSparseAttnArgs& a) {
-  return a.dtype == MF_DTYPE_BF16 && a.head_dim == 64 && (a.window == 32 || a.window == 64 || a.window == 128) && a.tokens >= 96;
+  if (a.dtype != MF_DTYPE_BF16 || a.head_dim != 64) return false;
+  if (a.tokens <= kDenseTokens) return a.window == 64 || a.window == 128;
+  return (a.window == 32 || a.window == 64 || a.window == 128) && a.tokens >= 96;
 }
 
 int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream) {
@@ -388,6 +401,7 @@ int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward
   p.in = layouts ? layouts[0] : contiguous_rows(a.heads, a.tokens);
   p.act = layouts ? layouts[1] : contiguous_rows(a.heads, a.tokens);
   const int BH = a.batch * a.heads;
+  if (a.tokens <= kDenseTokens) return launch_band<0, kDenseTokens>(p, BH, backward, stream);
   // 128-row tiles re-read half as much halo; 64-row ones spread a small call over twice as many CTAs
   const bool wide = (long long)BH * ((a.tokens + 127) / 128) >= 592;
   switch (a.window) {

@@ -355,7 +355,9 @@ int run_sparse(const MfSparseAttnArgs* a, bool backward, void* stream, const cha
                  "aligned tensors and the driver's tensor-map encoder", name);
     const bool tc = a->backend == MF_SPARSE_BACKEND_TCGEN05 ||
                     (a->backend == MF_SPARSE_BACKEND_AUTO && fits && kRadius && a->tokens >= 256);
-    if (!kRadius && a->backend == MF_SPARSE_BACKEND_AUTO && band_attn_applies(*a)) return band_attn(*a, nullptr, backward, s);
+    // (structures of one 32-row tile have one mma.sync kernel, whichever way they are asked for)
+    const bool band = a->backend == MF_SPARSE_BACKEND_AUTO || (a->backend == MF_SPARSE_BACKEND_MMA && a->tokens <= 32);
+    if (!kRadius && band && band_attn_applies(*a)) return band_attn(*a, nullptr, backward, s);
     if (tc) return backward ? sparse_attn_sm100_bwd(*a, kRadius, s) : sparse_attn_sm100_fwd(*a, kRadius, s);
     return backward ? sparse_attn_mma_bwd(*a, kRadius, s) : sparse_attn_mma_fwd(*a, kRadius, s);
   }

@@ -11,10 +11,11 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("B,H,N,window,sharp", [(2, 2, 96, 64, 1.0), (2, 2, 129, 64, 1.0), (3, 1, 255, 32, 1.0), (1, 2, 257, 128, 1.0),
-                                                (2, 2, 100, 128, 1.0), (90, 8, 130, 64, 1.0), (2, 2, 200, 64, 900.0)])  # fmt: skip
+                                                (2, 2, 100, 128, 1.0), (90, 8, 130, 64, 1.0), (2, 2, 200, 64, 900.0), (3, 2, 2, 64, 1.0),
+                                                (5, 3, 16, 64, 1.0), (4, 2, 17, 128, 1.0), (40, 8, 32, 64, 1.0), (3, 2, 32, 64, 900.0)])  # fmt: skip
 def test_band_attention_vs_oracle(B, H, N, window, sharp):
     """Both tile heights, tile remainders, structures that end inside a tile, an empty and a one-token structure, and logits
-    whose exponentials leave the range in which no maximum is needed."""
+    whose exponentials leave the range in which no maximum is needed; structures that fit one tile."""
     g = torch.Generator().manual_seed(N + window)
     q, k, v, go = (torch.randn(B, H, N, 64, generator=g).bfloat16() for _ in range(4))
     q = (q.float() * sharp / 8).bfloat16()
