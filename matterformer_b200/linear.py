@@ -3,13 +3,19 @@
 ``torch.autocast`` casts every fp32 weight and bias to bf16 inside each ``F.linear`` call and casts every weight /
 bias gradient back to fp32 afterwards: for the trunk of the reference (``AdaLNBlock``, models/transformer.py:228-316,
 five Linear layers per block) that is some 600 small cast kernels per training step, a quarter of all launches once the
-batch is split over eight GPUs.  Here each parameter keeps a bf16 copy that is refreshed for all layers at once at the
-start of a forward pass (one multi-tensor copy), and the backward pass writes the weight gradient in fp32 straight out of
-the GEMM and the bias gradient comes from this library's column-sum kernels (``mf_column_sums``: one read of the output
-gradient, fixed order of additions).  The GEMMs themselves stay library calls (cuBLAS).
+batch is split over eight GPUs.  Here a forward pass makes the bf16 copies of all its layers at once (one multi-tensor
+copy, :func:`bf16_copies`), and the backward pass writes the weight gradient in fp32 straight out of the GEMM and the
+bias gradient comes from this library's column-sum kernels (``mf_column_sums``: one read of the output gradient, fixed
+order of additions).  The GEMMs themselves stay library calls (cuBLAS).
+
+The copies belong to the pass that made them.  They are not kept for the next one: a parameter's version counter does not
+see every change (a replayed CUDA graph, a write through ``.data`` or through a flat buffer that the parameter is a view
+of), so a copy that outlived its pass could not be told from a stale one.
 """
 from __future__ import annotations
 
+import contextlib
+import threading
 from typing import Iterable, Optional, Sequence
 
 import torch
@@ -17,7 +23,7 @@ import torch.nn.functional as F
 
 from .fused import column_sums, column_sums_applies, gelu_tanh_applies, gelu_tanh_backward, gelu_tanh_forward
 
-_SHADOW = "_mf_bf16_copy"  # attribute on the parameter: (bf16 tensor, parameter version it was made from)
+_COPY = "_mf_bf16_copy"  # attribute on a parameter given to refresh_bf16_copies: (bf16 tensor, version it was made from)
 
 
 def _bf16_autocast() -> bool:
@@ -29,94 +35,129 @@ def linear_bf16_applies(x: torch.Tensor, weight: torch.Tensor) -> bool:
     return x.is_cuda and weight.is_cuda and weight.dtype == torch.float32 and (x.dtype == torch.bfloat16 or _bf16_autocast())
 
 
-def _current(p: torch.Tensor) -> Optional[torch.Tensor]:
-    entry = getattr(p, _SHADOW, None)
-    if entry is None:
-        return None
-    copy, version = entry
-    if version != p._version or copy.device != p.device or copy.shape != p.shape:
-        return None
-    return copy
+class _Pass(threading.local):
+    """What the forward pass that this thread is in computes with."""
+
+    copies: dict = {}  # id of a parameter -> (the parameter, its bf16 copy)
+    kept: Optional["KeptBf16Copies"] = None
+
+
+_PASS = _Pass()
+
+
+def _takes_copy(p: Optional[torch.Tensor]) -> bool:
+    return p is not None and p.is_cuda and p.dtype == torch.float32
+
+
+class _CopySet:
+    """bf16 copies of ``params`` and of the parameters of ``stacks``, made on construction and again by :meth:`refresh`.  They
+    share one buffer, on 256-byte boundaries; a stack's lie one behind the other and are one matrix."""
+
+    def __init__(self, params: Sequence[torch.Tensor], stacks: Sequence[Sequence[torch.Tensor]]) -> None:
+        stacked = {id(p) for stack in stacks for p in stack}
+        single = [p for p in params if _takes_copy(p) and id(p) not in stacked]
+        device = next((p.device for p in (*single, *(stack[0] for stack in stacks))), None)
+        whole = [p for p in single if p.numel() % 128 == 0 and p.device == device]
+        other = [p for p in single if not (p.numel() % 128 == 0 and p.device == device)]
+        self.params = [*whole, *other, *(p for stack in stacks for p in stack)]
+        at = sum(p.numel() for p in whole)
+        sizes = [sum(p.numel() for p in stack) for stack in stacks]
+        with torch.no_grad():
+            self.buffers = [torch.empty(p.shape, device=p.device, dtype=torch.bfloat16) for p in other]
+            flat = torch.empty(at + sum(-(-n // 128) * 128 for n in sizes), device=device, dtype=torch.bfloat16)
+            self.copies = [*torch._utils._unflatten_dense_tensors(flat[:at], whole), *self.buffers] if whole else list(self.buffers)
+            self.buffers.append(flat)
+            self.stacks = []
+            for stack, n in zip(stacks, sizes):
+                self.stacks.append(flat[at : at + n].view(-1, *stack[0].shape[1:]))
+                self.copies += self.stacks[-1].split(stack[0].shape[0])
+                at += -(-n // 128) * 128
+        self.entries = {id(p): (p, c) for p, c in zip(self.params, self.copies)}
+        self.refresh()
+
+    def refresh(self) -> None:
+        if self.params:
+            with torch.no_grad():
+                torch._foreach_copy_(self.copies, self.params)
+
+
+class KeptBf16Copies:
+    """Copies that outlive a pass, for the owner of a CUDA graph: ``with kept.in_use():`` around the warm-up and the capture of an
+    evaluation makes its passes use (and on the first one make) the copies held here, and :meth:`refresh` brings them up to
+    date before a replay, once for as many replays as the parameters stay as they are."""
+
+    def __init__(self) -> None:
+        self._sets: dict = {}
+
+    def provide(self, params, stacks) -> _CopySet:
+        key = (tuple(map(id, params)), tuple(tuple(map(id, stack)) for stack in stacks))
+        if key not in self._sets:
+            new = _CopySet(params, stacks)
+            if torch.cuda.is_current_stream_capturing() or not all(isinstance(p, torch.nn.Parameter) for p in new.params):
+                return new  # computed afresh by every pass, captured ones included
+            self._sets[key] = new
+        return self._sets[key]
+
+    def refresh(self) -> None:
+        for made in self._sets.values():
+            made.refresh()
+            for buffer in made.buffers:  # (allocated on the stream of the warm-up, read by the replays on this one)
+                if buffer.is_cuda:
+                    buffer.record_stream(torch.cuda.current_stream(buffer.device))
+
+    @contextlib.contextmanager
+    def in_use(self):
+        outer, _PASS.kept = _PASS.kept, self
+        try:
+            yield
+        finally:
+            _PASS.kept = outer
+
+
+@contextlib.contextmanager
+def bf16_copies(params: Iterable[torch.Tensor], stacks: Sequence[Sequence[torch.Tensor]] = ()):
+    """``with bf16_copies(params, stacks) as stacked:`` makes the bf16 copies that the :func:`linear_bf16` calls inside compute
+    with.  ``stacks``: groups of equally shaped parameters whose copies are wanted as one matrix each, returned in ``stacked``.
+    Seen by this thread alone, and by nothing after the block; what autograd saves keeps its own copies alive."""
+    params, kept, outer = list(params), _PASS.kept, _PASS.copies
+    made = kept.provide(params, stacks) if kept is not None else _CopySet(params, stacks)
+    _PASS.copies = {**outer, **made.entries}
+    try:
+        yield made.stacks
+    finally:
+        _PASS.copies = outer
 
 
 def bf16_copy(p: torch.Tensor) -> torch.Tensor:
-    """The parameter's bf16 copy, refreshed if the parameter changed since it was made."""
-    copy = _current(p)
-    if copy is None:
-        entry = getattr(p, _SHADOW, None)
-        copy = entry[0] if entry is not None and entry[0].device == p.device and entry[0].shape == p.shape else None
-        with torch.no_grad():
-            if copy is None:
-                copy = p.detach().to(torch.bfloat16)
-            else:
-                copy.copy_(p.detach())
-        setattr(p, _SHADOW, (copy, p._version))
-    return copy
-
-
-def has_bf16_copy(p: torch.Tensor) -> bool:
-    return getattr(p, _SHADOW, None) is not None
+    """The parameter in bf16: the enclosing pass's copy, else the one its owner refreshes, else a cast."""
+    entry = _PASS.copies.get(id(p))
+    if entry is not None and entry[0] is p:
+        return entry[1]
+    copy, version = getattr(p, _COPY, (None, None))
+    if copy is not None and version == p._version and copy.device == p.device and copy.shape == p.shape:
+        return copy
+    return p.detach().to(torch.bfloat16)
 
 
 def refresh_bf16_copies(params: Iterable[torch.Tensor], *, force: bool = False) -> None:
-    """Bring the bf16 copies of ``params`` up to date with one multi-tensor copy.  ``force`` copies even when the version
-    counters say nothing changed: a step captured in a CUDA graph must contain the copy, because a replay updates the
-    parameters without running this Python code again."""
+    """For callers of :func:`linear_bf16` with layers of their own: give ``params`` bf16 copies that stay with them, all made
+    or brought up to date by one multi-tensor copy.  The caller vouches for them: without ``force`` only the parameters whose
+    version counter has moved are copied, which misses changes made by a graph's replay or through ``.data``, and a step
+    captured in a CUDA graph must contain a forced call.  (The trunk does not use these; see :func:`bf16_copies`.)"""
     stale_dst, stale_src = [], []
     for p in params:
-        if p is None or not p.is_cuda or p.dtype != torch.float32:
+        if not _takes_copy(p):
             continue
-        entry = getattr(p, _SHADOW, None)
-        if entry is None or entry[0].device != p.device or entry[0].shape != p.shape:
-            bf16_copy(p)  # first use: allocates
-            if not force:
-                continue
-            entry = getattr(p, _SHADOW)
-        if force or entry[1] != p._version:
-            stale_dst.append(entry[0])
+        copy, version = getattr(p, _COPY, (None, None))
+        if copy is None or copy.device != p.device or copy.shape != p.shape:
+            copy, version = torch.empty(p.shape, device=p.device, dtype=torch.bfloat16), None
+        if force or version != p._version:
+            stale_dst.append(copy)
             stale_src.append(p.detach())
-            setattr(p, _SHADOW, (entry[0], p._version))
+            setattr(p, _COPY, (copy, p._version))
     if stale_dst:
         with torch.no_grad():
             torch._foreach_copy_(stale_dst, stale_src)
-
-
-_REFRESH_IN_CAPTURE = True
-
-
-class no_refresh_in_capture:
-    """For a captured evaluation whose owner brings the bf16 copies up to date itself, before each replay."""
-
-    def __enter__(self):
-        global _REFRESH_IN_CAPTURE
-        self._before, _REFRESH_IN_CAPTURE = _REFRESH_IN_CAPTURE, False
-
-    def __exit__(self, *exc):
-        global _REFRESH_IN_CAPTURE
-        _REFRESH_IN_CAPTURE = self._before
-
-
-def refresh_must_be_captured() -> bool:
-    return _REFRESH_IN_CAPTURE and torch.cuda.is_current_stream_capturing()
-
-
-def stacked_bf16_copies(params: Sequence[torch.Tensor], stack: Optional[torch.Tensor]) -> torch.Tensor:
-    """The bf16 copies of equally shaped parameters as one contiguous tensor, (len(params) * rows, ...): each parameter's
-    copy is a view of it, so refreshing the copies refreshes the stack.  ``stack`` is returned as it is while it still holds
-    them.  Freshly placed copies are filled by the next :func:`refresh_bf16_copies`, or here where that does not follow."""
-    rows, first = params[0].shape[0], params[0]
-    if stack is not None and stack.device == first.device:
-        for i, p in enumerate(params):
-            entry = getattr(p, _SHADOW, None)
-            if entry is None or entry[0].data_ptr() != stack[i * rows :].data_ptr() or entry[0].shape != p.shape:
-                break
-        else:
-            return stack
-    with torch.no_grad():
-        stack = torch.cat([p.detach().to(torch.bfloat16) for p in params])
-    for i, p in enumerate(params):
-        setattr(p, _SHADOW, (stack[i * rows : (i + 1) * rows], p._version))
-    return stack
 
 
 class _StackedModulation(torch.autograd.Function):
@@ -199,9 +240,8 @@ class _LinearBf16(torch.autograd.Function):
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> torch.Tensor:
     """``F.linear`` in bf16 on fp32 parameters (what autocast computes), returning bf16.  Falls back to ``F.linear``
-    where :func:`linear_bf16_applies` says no.  A step that is captured into a CUDA graph and updates the parameters
-    must call ``refresh_bf16_copies(params, force=True)`` inside the captured region before its first layer (the trunk
-    does): the version counters this function checks do not advance during replays."""
+    where :func:`linear_bf16_applies` says no.  Casts the parameters unless the enclosing :func:`bf16_copies` or an
+    earlier :func:`refresh_bf16_copies` has done so."""
     if not linear_bf16_applies(x, weight):
         return F.linear(x, weight, bias)
     if x.dtype != torch.bfloat16:

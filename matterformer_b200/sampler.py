@@ -18,7 +18,7 @@ from typing import Optional
 
 import torch
 
-from .linear import has_bf16_copy, no_refresh_in_capture, refresh_bf16_copies
+from .linear import KeptBf16Copies
 from . import fused
 from .trunk import recenter_coordinates
 
@@ -42,43 +42,45 @@ class GraphedDenoiser:
     """One captured evaluation of ``net`` on fixed-shape buffers, replayed for every noise level.
 
     Capturing costs a few evaluations; an instance can be handed to several :func:`edm_sample` calls of the same
-    batch shape and padding mask (``denoiser=``).
+    batch shape and padding mask (``denoiser=``); every run computes with the parameters as they are when it starts.
     """
 
     def __init__(self, net, atoms, coords, pad_mask, lattice, autocast_dtype):
         self.atoms, self.coords = atoms.clone(), coords.clone()
         self.sigma = torch.ones(atoms.shape[0], device=atoms.device)
         self.pad_mask, self.lattice, self.net, self.autocast_dtype = pad_mask, lattice, net, autocast_dtype
+        # the bf16 copies of the parameters are not part of the captured evaluation (a tenth of its time): a run brings them up to
+        # date once, whether or not a parameter can be seen to have changed, and replays the graph for every noise level
+        self.copies = KeptBf16Copies()
         side = torch.cuda.Stream(atoms.device)
         side.wait_stream(torch.cuda.current_stream(atoms.device))
-        with torch.cuda.stream(side):  # warm-up outside the capture (lazy initialisation, autotuning)
+        with torch.cuda.stream(side), self.copies.in_use():  # warm-up outside the capture (lazy initialisation, autotuning)
             for _ in range(2):
                 self._eval()
         torch.cuda.current_stream(atoms.device).wait_stream(side)
-        # the bf16 copies of the parameters are not part of the captured evaluation (a tenth of its time): a call brings them
-        # up to date first if a parameter has changed since the last one
-        self.params = [p for p in net.parameters() if has_bf16_copy(p)]
-        self.versions = self._versions()
         self.graph = torch.cuda.CUDAGraph()
-        with no_refresh_in_capture(), torch.cuda.graph(self.graph):
+        with self.copies.in_use(), torch.cuda.graph(self.graph):
             self.out_atoms, self.out_coords = self._eval()
-
-    def _versions(self):
-        return [(p._version, p.data_ptr()) for p in self.params]
 
     def _eval(self):
         with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None):
             return self.net(self.atoms, self.coords, self.pad_mask, self.sigma, lattice=self.lattice)
 
-    def __call__(self, atoms, coords, sigma: float):
+    def refresh(self) -> None:
+        """Take over the parameters as they are now."""
+        self.copies.refresh()
+
+    def replay(self, atoms, coords, sigma: float):
+        """One evaluation with the parameters of the last :meth:`refresh`."""
         self.atoms.copy_(atoms)
         self.coords.copy_(coords)
         self.sigma.fill_(sigma)
-        if (versions := self._versions()) != self.versions:
-            refresh_bf16_copies(self.params, force=True)
-            self.versions = versions
         self.graph.replay()
         return self.out_atoms.float(), self.out_coords.float()
+
+    def __call__(self, atoms, coords, sigma: float):
+        self.refresh()
+        return self.replay(atoms, coords, sigma)
 
 
 @torch.no_grad()
@@ -97,6 +99,9 @@ def edm_sample(net, num_atoms: torch.Tensor, *, atom_channels: int = 6, lattice:
     pad_mask = build_pad_mask(num_atoms).to(device)
     batch, max_atoms = pad_mask.shape
     hole = pad_mask[..., None]
+    kept = type(denoiser) is GraphedDenoiser
+    if kept:  # first of all: the copy runs while the host prepares the noise
+        denoiser.refresh()
 
     atoms = torch.randn(batch, max_atoms, atom_channels, device=device).masked_fill(hole, 0.0)
     coords = recenter_coordinates(torch.randn(batch, max_atoms, 3, device=device), pad_mask)
@@ -109,9 +114,9 @@ def edm_sample(net, num_atoms: torch.Tensor, *, atom_channels: int = 6, lattice:
     if use_cuda_graph is None:  # large batches keep the GPU busy without it (measured: no gain at 1024 molecules)
         use_cuda_graph = device.type == "cuda" and batch <= 256
     if denoiser is not None:
-        denoise = denoiser
+        denoise = denoiser.replay if kept else denoiser
     elif use_cuda_graph:
-        denoise = GraphedDenoiser(net, atoms, coords, pad_mask, lattice, autocast_dtype)
+        denoise = GraphedDenoiser(net, atoms, coords, pad_mask, lattice, autocast_dtype).replay
     else:
         def denoise(a, c, sigma):
             s = torch.full((batch,), sigma, device=device)

@@ -30,8 +30,7 @@ from torch import nn
 from . import fused
 from .fused import (fused_applies, gated_ln_modulate, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
                     split_modulation)
-from .linear import (linear_bf16, linear_bf16_applies, linear_gelu_bf16, refresh_bf16_copies, refresh_must_be_captured, stacked_bf16_copies,
-                     stacked_modulation)  # fmt: skip
+from .linear import bf16_copies, linear_bf16, linear_bf16_applies, linear_gelu_bf16, stacked_modulation
 from .simplicial import (normalize_simplicial_precision, packed_projection_applies, simplicial_attention_cuda,
                          simplicial_attention_packed)  # fmt: skip
 
@@ -408,21 +407,24 @@ class TransformerTrunk(nn.Module):
                 sparse_plan: Optional[SparseAttentionPlan] = None) -> torch.Tensor:  # fmt: skip
         """``sparse_plan`` (see :func:`plan_sparse_attention`) makes every MHA layer attend over the plan's
         neighbourhoods instead of all tokens: the periodic-crystal mode of the trunk."""
-        b, n, _ = x.shape
-        if pad_mask is not None:
-            pad_mask = pad_mask.bool()
         bf16 = x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
         layers = [block.ada_ln[-1] for block in self.blocks]
         stacked = bf16 and fused_applies(x) and cond_emb.ndim == 2 and all(
             block.fused_elementwise and m.weight.dtype == torch.float32 and m.bias is not None for block, m in zip(self.blocks, layers)
         )
-        if stacked:
-            self._modulation_w16 = stacked_bf16_copies([m.weight for m in layers], getattr(self, "_modulation_w16", None))
-            self._modulation_b16 = stacked_bf16_copies([m.bias for m in layers], getattr(self, "_modulation_b16", None))
-        if bf16:
-            # the bf16 copies the blocks' Linear layers compute with: all of them in one multi-tensor copy; a step that is
-            # being captured into a CUDA graph always contains the copy (its replays change the parameters)
-            refresh_bf16_copies(self._linear_parameters(), force=refresh_must_be_captured())
+        if not (bf16 or (x.is_cuda and x.dtype == torch.bfloat16)):
+            return self._forward(x, cond_emb, pad_mask, sparse_plan, None)
+        # the bf16 copies the blocks' Linear layers compute with: all of them in one multi-tensor copy
+        stacks = ([m.weight for m in layers], [m.bias for m in layers]) if stacked else ()
+        with bf16_copies(self._linear_parameters(), stacks) as made:
+            return self._forward(x, cond_emb, pad_mask, sparse_plan, made if stacked else None)
+
+    def _forward(self, x, cond_emb, pad_mask, sparse_plan, modulation_copies):
+        """``modulation_copies``: stacked bf16 weights and biases of the modulation layers, where one GEMM serves them all."""
+        b, n, _ = x.shape
+        if pad_mask is not None:
+            pad_mask = pad_mask.bool()
+        stacked = modulation_copies is not None
         sim_mask = SimplicialAttentionMask.from_key_padding_mask(pad_mask, batch_size=b, num_tokens=n, device=x.device)
         if self.emit_pair_valid and not x.is_cuda:  # (the kernels take the padding from the key mask: the same pairs)
             v = sim_mask.pair_key_valid
@@ -434,12 +436,13 @@ class TransformerTrunk(nn.Module):
             x = x.masked_fill(pad_mask[..., None], 0.0)
         # every block starts its modulation with the same SiLU(cond_emb): formed (and cast for the bf16 Linear) once
         cond_act = F.silu(cond_emb)
-        if bf16:
+        if x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16:
             cond_act = cond_act.to(torch.bfloat16)
         modulation = [None] * len(self.blocks)
         if stacked:
-            modulation = stacked_modulation(cond_act, self._modulation_w16, self._modulation_b16,
-                                            [m.weight for m in layers] + [m.bias for m in layers], len(layers))  # fmt: skip
+            layers = [block.ada_ln[-1] for block in self.blocks]
+            modulation = stacked_modulation(cond_act, *modulation_copies, [m.weight for m in layers] + [m.bias for m in layers],
+                                            len(layers))  # fmt: skip
         num_atoms = (~pad_mask).sum(dim=1).to(torch.int32) if x.is_cuda and pad_mask is not None else None
         h = None
         for i, (block, six) in enumerate(zip(self.blocks, modulation)):
@@ -560,9 +563,13 @@ class EDMModel(nn.Module):
         if sigma.ndim == 2:
             sigma = sigma[:, 0]
         sigma_cond = torch.log(sigma.clamp_min(1e-8)) / 4.0
-        if linear_bf16_applies(atom_noisy, self.atom_proj.weight):  # (the trunk brings its own copies up to date)
-            layers = [self.atom_proj, self.conditioning.mlp[0], self.conditioning.mlp[2], self.atom_head[1], self.atom_head[3]]
-            refresh_bf16_copies([p for m in layers for p in (m.weight, m.bias)], force=refresh_must_be_captured())
+        if not linear_bf16_applies(atom_noisy, self.atom_proj.weight):
+            return self._forward(atom_noisy, coords_noisy, pad_mask, sigma_cond)
+        layers = [self.atom_proj, self.conditioning.mlp[0], self.conditioning.mlp[2], self.atom_head[1], self.atom_head[3]]
+        with bf16_copies(p for m in layers for p in (m.weight, m.bias)):  # (the trunk makes its own)
+            return self._forward(atom_noisy, coords_noisy, pad_mask, sigma_cond)
+
+    def _forward(self, atom_noisy, coords_noisy, pad_mask, sigma_cond):
         feat = sigma_cond[:, None, None].expand(-1, atom_noisy.shape[1], 1).masked_fill(pad_mask[..., None], 0.0)
         tokens = linear_bf16(torch.cat([atom_noisy, feat], dim=-1), self.atom_proj.weight, self.atom_proj.bias)
         cond = self.conditioning(sigma_cond, sigma_cond)
