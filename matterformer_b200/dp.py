@@ -65,10 +65,12 @@ class GraphedTrainStep:
     all-reduce, clipping, AdamW) and replayed.  Inputs live in static buffers that :meth:`__call__` refreshes.
     Needs an optimizer built with ``capturable=True``; with more than one rank the DDP wrapper must have run at
     least 11 eager steps on the capture stream first (PyTorch's requirement for capturing NCCL collectives).
+    The graph reads and writes the parameters and the optimizer's state where they are, so the step keeps both alive.
     """
 
     def __init__(self, net: nn.Module, loss_fn: EDMLoss, optimizer: torch.optim.Optimizer, example: dict, *,
                  autocast_dtype: Optional[torch.dtype] = torch.bfloat16, clip: float = 1.0, warmup: int = 11) -> None:  # fmt: skip
+        self.net, self.optimizer = net, optimizer
         self.static = {k: v.clone() for k, v in example.items()}
         self.stream = torch.cuda.Stream()
         self.stream.wait_stream(torch.cuda.current_stream())

@@ -476,6 +476,29 @@ def test_trunk_bf16_step_runs_and_learns():
     assert used == {"cuda"}
 
 
+@pytest.mark.gpu
+def test_captured_step_keeps_what_it_writes_alive():
+    """The optimizer's moments are written by every replay: a caller that keeps the step alone must not lose them."""
+    import gc
+    import weakref
+
+    from matterformer_b200.dp import GraphedTrainStep
+
+    dev = torch.device("cuda:0")
+    net = build_edm_net(d_model=128, n_heads=2, n_layers=2, seed=0).to(dev)
+    opt = torch.optim.AdamW(net.parameters(), lr=1e-3, fused=True, capturable=True)
+    batch = {k: v.to(dev) for k, v in config5_batch(8, seed=1).items() if k != "num_atoms"}
+    step = GraphedTrainStep(net, EDMLoss(sigma_data=1.0), opt, batch, warmup=3)
+    alive = [weakref.ref(net), weakref.ref(opt)]
+    state = opt.state[next(net.parameters())]["exp_avg"]
+    before = state.clone()
+    del net, opt
+    gc.collect()
+    assert all(r() is not None for r in alive)  # (replayed only when they are)
+    step()
+    assert not torch.equal(state, before)
+
+
 def _dp_worker(rank, world, port, out):
     os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
     dist.init_process_group("gloo", rank=rank, world_size=world)
