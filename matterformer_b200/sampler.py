@@ -14,6 +14,7 @@ coordinates), so a CPU run with the same global seed reproduces the reference's 
 from __future__ import annotations
 
 import math
+from itertools import chain
 from typing import Optional
 
 import torch
@@ -49,26 +50,40 @@ class GraphedDenoiser:
         self.atoms, self.coords = atoms.clone(), coords.clone()
         self.sigma = torch.ones(atoms.shape[0], device=atoms.device)
         self.pad_mask, self.lattice, self.net, self.autocast_dtype = pad_mask, lattice, net, autocast_dtype
+        self._capture()
+
+    def _capture(self) -> None:
         # the bf16 copies of the parameters are not part of the captured evaluation (a tenth of its time): a run brings them up to
         # date once, whether or not a parameter can be seen to have changed, and replays the graph for every noise level
         self.copies = KeptBf16Copies()
-        side = torch.cuda.Stream(atoms.device)
-        side.wait_stream(torch.cuda.current_stream(atoms.device))
+        device = self.atoms.device
+        side = torch.cuda.Stream(device)
+        side.wait_stream(torch.cuda.current_stream(device))
         with torch.cuda.stream(side), self.copies.in_use():  # warm-up outside the capture (lazy initialisation, autotuning)
             for _ in range(2):
                 self._eval()
-        torch.cuda.current_stream(atoms.device).wait_stream(side)
+        torch.cuda.current_stream(device).wait_stream(side)
         self.graph = torch.cuda.CUDAGraph()
         with self.copies.in_use(), torch.cuda.graph(self.graph):
             self.out_atoms, self.out_coords = self._eval()
+        self.tables = [t for m in self.net.modules() for t in (m._modules, m._parameters, m._buffers) if t]
+        self.tensors = [*self.net.parameters(), *self.net.buffers()]
+        self.layout = self._layout()
+
+    def _layout(self) -> list:
+        """The network's layers and tensors, and where the tensors lie; the graph reads those that have no copy in place."""
+        return [*map(id, chain.from_iterable(map(dict.values, self.tables))), *[t.data_ptr() for t in self.tensors]]
 
     def _eval(self):
         with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None):
             return self.net(self.atoms, self.coords, self.pad_mask, self.sigma, lattice=self.lattice)
 
     def refresh(self) -> None:
-        """Take over the parameters as they are now."""
+        """Take over the parameters as they are now; where they have moved, or layers were replaced, the evaluation is captured
+        anew."""
         self.copies.refresh()
+        if self._layout() != self.layout:
+            self._capture()
 
     def replay(self, atoms, coords, sigma: float):
         """One evaluation with the parameters of the last :meth:`refresh`."""

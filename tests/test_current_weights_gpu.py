@@ -213,3 +213,27 @@ def test_stacked_copies_and_odd_sizes():
             assert bf16_copy(p).data_ptr() % 16 == 0
         for m, stack in zip(made, stacks):
             assert m.data_ptr() % 256 == 0 and torch.equal(m, torch.cat([p.detach().bfloat16() for p in stack]))
+
+
+@pytest.mark.parametrize("how", ["data", "assign", "layer"])
+def test_a_kept_denoiser_follows_parameters_that_move(how):
+    """Parameters placed in new memory (a swap of ``.data``, a loaded checkpoint that is assigned, a replaced layer): the captured
+    evaluation reads some of them in place and has to be captured anew."""
+    net, n = _net(), torch.tensor(COUNTS, device=DEV)
+    denoiser = _denoiser(net, n)
+    before = _sample(net, n, denoiser)
+    if how == "data":
+        for p in net.parameters():
+            p.data = p.data * 1.5
+    elif how == "assign":
+        net.load_state_dict({k: v * 1.5 for k, v in net.state_dict().items()}, assign=True)
+    else:
+        old = net.model.pair_head[2]
+        net.model.pair_head[2] = torch.nn.Linear(old.in_features, 1).to(DEV)
+        net.model.atom_head[3] = torch.nn.Linear(128, 6).to(DEV)
+    filler = [torch.full((1 << 20,), float("nan"), device=DEV) for _ in range(4)]  # what was freed is written over
+    after = _sample(net, n, denoiser)
+    expect = _sample(_twin(net), n)
+    del filler
+    assert (expect - before).abs().max() > 1e-2
+    torch.testing.assert_close(after, expect, atol=1e-5, rtol=1e-5)
