@@ -75,7 +75,8 @@ class GraphedDenoiser:
         return [*map(id, chain.from_iterable(map(dict.values, self.tables))), *[t.data_ptr() for t in self.tensors]]
 
     def _eval(self):
-        with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None):
+        # (an enclosing autocast region may hold casts of the weights, which would go into the graph as they are now)
+        with torch.autocast("cuda", dtype=self.autocast_dtype, enabled=self.autocast_dtype is not None, cache_enabled=False):
             return self.net(self.atoms, self.coords, self.pad_mask, self.sigma, lattice=self.lattice)
 
     def refresh(self) -> None:

@@ -237,3 +237,17 @@ def test_a_kept_denoiser_follows_parameters_that_move(how):
     del filler
     assert (expect - before).abs().max() > 1e-2
     torch.testing.assert_close(after, expect, atol=1e-5, rtol=1e-5)
+
+
+def test_a_capture_inside_an_autocast_region_takes_no_casts_from_it():
+    """Above 32 tokens the MHA layers are torch's, whose weights autocast casts and keeps until its outermost region ends: casts
+    made before the capture would stay in the graph."""
+    net, n = _net(), torch.tensor([40, 33], device=DEV)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        denoiser = _denoiser(net, n)
+        before = _sample(net, n, denoiser)
+        for p in net.parameters():
+            p.data.mul_(1.5)
+        after, expect = _sample(net, n, denoiser), _sample(_twin(net), n)
+    assert (expect - before).abs().max() > 1e-2
+    torch.testing.assert_close(after, expect, atol=1e-5, rtol=1e-5)
