@@ -189,6 +189,14 @@ def plan_sparse_attention(frac: torch.Tensor, lattice: torch.Tensor, pad_mask: O
     return SparseAttentionPlan(kind=kind, blocks=blocks, num_atoms=num_atoms, window=int(window))
 
 
+def _padding_is_suffix(module: nn.Module, mask: torch.Tensor) -> bool:
+    """Whether every row of the (B, N) mask is unpadded tokens followed by padded ones.  Read from the device each time: an
+    answer kept for a mask would outlive its contents.  ``module`` remembers it for a capture that follows."""
+    if not torch.cuda.is_current_stream_capturing():
+        module._suffix_before_capture = bool((mask[:, 1:] | ~mask[:, :-1]).all().item())
+    return getattr(module, "_suffix_before_capture", True)
+
+
 class RegularAttention(nn.Module):
     """Standard multi-head self-attention (``position_mode="none"`` of the reference wrapper,
     regular_attention.py:275-338); parameters are those of ``nn.MultiheadAttention``.
@@ -197,9 +205,9 @@ class RegularAttention(nn.Module):
     same computation: CUDA, bf16 (autocast or bf16 input), at most 32 tokens (a window of 64 then
     covers every pair), head size 32/64/128, no active dropout, and a key-padding mask that marks a
     suffix of every row (how the reference's collate functions pad, data/qm9.py:119-166).  The suffix
-    property is verified on the device once per mask tensor (one read-back, remembered for the other
-    layers of the step; a mask first seen while a CUDA graph is being captured cannot be read back
-    and is taken to be the one checked during the eager warm-up steps).  A mask with holes goes to
+    property is read back from the device by every call, once for all layers of a trunk; while a CUDA
+    graph is being captured nothing can be read, and the answer of the last call before counts (the
+    warm-up's, so replays must stay with masks of that kind).  A mask with holes goes to
     ``nn.MultiheadAttention`` like everything else this kernel does not cover.  Rows of padded tokens
     return zeros on the kernel path instead of the reference's average over the real keys; the trunk
     discards those rows.  ``impl="torch"`` always uses ``nn.MultiheadAttention``.
@@ -213,20 +221,8 @@ class RegularAttention(nn.Module):
         self.impl = impl
         self._last_core_used: Optional[str] = None
 
-    _suffix_cache: tuple = (None, True)  # (identity of the last mask checked, result); shared by all layers
-
-    @classmethod
-    def _padding_is_a_suffix(cls, mask: torch.Tensor) -> bool:
-        key = (mask.data_ptr(), mask._version, tuple(mask.shape))
-        if cls._suffix_cache[0] == key:
-            return cls._suffix_cache[1]
-        if torch.cuda.is_current_stream_capturing():
-            return True
-        ok = bool((mask[:, 1:] | ~mask[:, :-1]).all().item()) if mask.shape[1] > 1 else True
-        cls._suffix_cache = (key, ok)
-        return ok
-
-    def _cuda_core_applies(self, x: torch.Tensor, key_padding_mask: Optional[torch.Tensor]) -> bool:
+    def _core_fits(self, x: torch.Tensor, key_padding_mask: Optional[torch.Tensor]) -> bool:
+        """Everything but the form of the padding."""
         if self.impl == "torch" or not x.is_cuda or key_padding_mask is None or x.shape[1] > 32:
             return False
         if self.training and self.attn.dropout > 0.0:
@@ -234,9 +230,7 @@ class RegularAttention(nn.Module):
         bf16 = x.dtype == torch.bfloat16 or (
             torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
         )
-        if not (bf16 and (self.attn.embed_dim // self.attn.num_heads) in (32, 64, 128)):
-            return False
-        return self._padding_is_a_suffix(key_padding_mask)
+        return bf16 and (self.attn.embed_dim // self.attn.num_heads) in (32, 64, 128)
 
     def _sparse_forward(self, x: torch.Tensor, plan: SparseAttentionPlan) -> torch.Tensor:
         """The layer with its core on the radius block-sparse or the local-window kernel.  Same parameters and
@@ -258,13 +252,17 @@ class RegularAttention(nn.Module):
         return self.attn.out_proj(merge_heads(core))
 
     def forward(self, x: torch.Tensor, *, key_padding_mask: Optional[torch.Tensor] = None,
-                sparse_plan: Optional[SparseAttentionPlan] = None, num_atoms: Optional[torch.Tensor] = None) -> torch.Tensor:  # fmt: skip
-        """``num_atoms``: the (B,) int32 counts of real tokens when the caller has already formed them."""
+                sparse_plan: Optional[SparseAttentionPlan] = None, num_atoms: Optional[torch.Tensor] = None,
+                padding_is_suffix: Optional[bool] = None) -> torch.Tensor:  # fmt: skip
+        """``num_atoms``: the (B,) int32 counts of real tokens, ``padding_is_suffix``: the form of the mask, when the caller
+        has already found them."""
         if sparse_plan is not None:
             if not x.is_cuda:
                 raise RuntimeError("sparse attention plans need CUDA tensors (there is no CPU fallback)")
             return self._sparse_forward(x, sparse_plan)
-        if not self._cuda_core_applies(x, key_padding_mask):
+        if not self._core_fits(x, key_padding_mask) or not (
+            _padding_is_suffix(self, key_padding_mask) if padding_is_suffix is None else padding_is_suffix
+        ):
             self._last_core_used = "torch"
             out, _ = self.attn(x, x, x, key_padding_mask=key_padding_mask, need_weights=False)
             return out
@@ -336,13 +334,15 @@ class AdaLNBlock(nn.Module):
         self.fused_elementwise = True  # CUDA fp32 residual stream: fused norm+modulate and gated-residual kernels
 
     def forward(self, x, cond_emb, *, pad_mask=None, simplicial_attention_mask=None, sparse_plan=None,
-                zero_padding: bool = False, cond_act=None, modulation=None, num_atoms=None, h=None, following=None):
+                zero_padding: bool = False, cond_act=None, modulation=None, num_atoms=None, h=None, following=None,
+                padding_is_suffix=None):
         """``zero_padding``: return the block's output with its padded rows cleared (the ``masked_fill`` the trunk
         applies before the next block), folded into the last fused pass when the fused kernels run.  ``cond_act``:
         ``SiLU(cond_emb)`` when the caller has already formed it (it is the same for every block of a trunk).
         ``modulation``: the six modulation tensors, formed by the trunk for all its blocks at once; ``num_atoms``: counts of
-        real tokens for the attention layer.  ``following``: (shift, scale, eps) of the norm that opens the next block; the
-        block then returns its output and that norm's, formed in one pass, and the next block takes the latter as ``h``."""
+        real tokens for the attention layer, ``padding_is_suffix``: whether they come first in every row.  ``following``:
+        (shift, scale, eps) of the norm that opens the next block; the block then returns its output and that norm's, formed in
+        one pass, and the next block takes the latter as ``h``."""
         fused = self.fused_elementwise and fused_applies(x)
         mod = None if modulation is not None else linear_bf16(cond_act if cond_act is not None else self.ada_ln[0](cond_emb), self.ada_ln[-1].weight,
                           self.ada_ln[-1].bias)  # fmt: skip
@@ -359,7 +359,8 @@ class AdaLNBlock(nn.Module):
         else:
             h = _modulate(self.norm1(x), shift_a, scale_a)
         if self.attn_type == "mha":
-            attn_out = self.attn(h, key_padding_mask=pad_mask, sparse_plan=sparse_plan, num_atoms=num_atoms)
+            attn_out = self.attn(h, key_padding_mask=pad_mask, sparse_plan=sparse_plan, num_atoms=num_atoms,
+                                 padding_is_suffix=padding_is_suffix)  # fmt: skip
         else:
             attn_out = self.attn(h, key_padding_mask=pad_mask, attention_mask=simplicial_attention_mask)
         if fused:
@@ -444,13 +445,16 @@ class TransformerTrunk(nn.Module):
             modulation = stacked_modulation(cond_act, *modulation_copies, [m.weight for m in layers] + [m.bias for m in layers],
                                             len(layers))  # fmt: skip
         num_atoms = (~pad_mask).sum(dim=1).to(torch.int32) if x.is_cuda and pad_mask is not None else None
+        mha = [block.attn for block in self.blocks if isinstance(block.attn, RegularAttention)]
+        reads = sparse_plan is None and any(attn._core_fits(x, pad_mask) for attn in mha)
+        suffix = _padding_is_suffix(self, pad_mask) if reads else None  # one read-back for all layers
         h = None
         for i, (block, six) in enumerate(zip(self.blocks, modulation)):
             chain = stacked and i + 1 < len(self.blocks)  # the next block's first norm in one pass with this one's output
             following = (*modulation[i + 1][:2], self.blocks[i + 1].norm1.eps) if chain else None
             x = block(x, cond_emb, pad_mask=pad_mask, simplicial_attention_mask=sim_mask, sparse_plan=sparse_plan,
                       zero_padding=pad_mask is not None, cond_act=cond_act, modulation=six, num_atoms=num_atoms, h=h,
-                      following=following)
+                      following=following, padding_is_suffix=suffix)  # fmt: skip
             x, h = x if chain else (x, None)
         x = layer_norm(x, self.norm_out)
         if pad_mask is not None:
