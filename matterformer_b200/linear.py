@@ -196,18 +196,9 @@ def stacked_modulation(x: torch.Tensor, weights: torch.Tensor, biases: torch.Ten
     return [out[6 * i : 6 * i + 6] for i in range(layers)]
 
 
-_MM_OUT_DTYPE = True  # torch.mm(..., out_dtype=) exists; cleared on the first refusal
-
-
 def _mm_f32(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """a @ b for bf16 operands with the fp32 accumulator written out unrounded."""
-    global _MM_OUT_DTYPE
-    if _MM_OUT_DTYPE:
-        try:
-            return torch.mm(a, b, out_dtype=torch.float32)
-        except (TypeError, RuntimeError):
-            _MM_OUT_DTYPE = False
-    return torch.mm(a, b).float()
+    return torch.mm(a, b, out_dtype=torch.float32)
 
 
 class _LinearBf16(torch.autograd.Function):

@@ -128,3 +128,23 @@ def test_attention_cost_batch_sampler_matches_reference_batches(golden):
         assert len(batch) == 1 or sum(simplicial_tile_steps(int(g["num_atoms"][i])) for i in batch) <= 1500
     with pytest.raises(ValueError, match="At least one batch budget"):
         AttentionCostBatchSampler(num_atoms, max_examples_per_batch=4)
+
+
+def test_a_failed_product_does_not_change_the_precision_of_later_ones(monkeypatch):
+    """Weight gradients leave the GEMM in fp32.  An error in one product (memory, say) is the caller's to see."""
+    import matterformer_b200.linear as L
+
+    asked = []
+
+    def mm(a, b, **kw):
+        asked.append(kw)
+        if len(asked) == 1:
+            raise torch.OutOfMemoryError("out of memory")
+        return (a.float() @ b.float()).to(kw.get("out_dtype", a.dtype))
+
+    monkeypatch.setattr(torch, "mm", mm)
+    a, b = torch.randn(4, 8).bfloat16(), torch.randn(8, 4).bfloat16()
+    with pytest.raises(torch.OutOfMemoryError):
+        L._mm_f32(a, b)
+    assert torch.equal(L._mm_f32(a, b), a.float() @ b.float())
+    assert all(kw == {"out_dtype": torch.float32} for kw in asked)
