@@ -537,7 +537,7 @@ int mf_merge_heads(void* const* ins, const float* scales, void* packed, int32_t 
  * call, all five gradients into grad_proj (B,N,5,H,D) bf16, the gradient of the unscaled projection.  out32 (B,H,N,D)
  * fp32 and lse (B,H,N) fp32 are written by the forward call and read by the backward call, as in mf_simplicial_fwd /
  * mf_simplicial_bwd, whose semantics (masks, zero rows, reproducibility) apply.  Served shapes: head_dim 64, at most 32
- * tokens, heads a multiple of four; MF_ERR_UNSUPPORTED otherwise.  16-byte aligned tensors; workspaces from the two *_workspace_bytes functions.
+ * tokens; MF_ERR_UNSUPPORTED otherwise.  16-byte aligned tensors; workspaces from the two *_workspace_bytes functions.
  */
 typedef struct MfSimplicialPackedArgs {
   int32_t batch, heads, tokens, head_dim;

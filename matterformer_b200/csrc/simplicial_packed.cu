@@ -7,7 +7,7 @@
 // with strides -- apply the query scale on load, write the attention output as (B,N,H*D) and the five gradients
 // straight into one (B,N,5,H,D) tensor, so neither pass over the activations exists any more.  They run the
 // warp-level kernels (simplicial_small_fwd.cu, simplicial_small_bwd.cu) and therefore serve molecules of at most
-// 32 tokens with a multiple of four heads of 64 channels in bf16: the trunk's shape.
+// 32 tokens with any number of heads of 64 channels in bf16: the trunk's shape.
 #include "common.cuh"
 #include "simplicial.cuh"
 #include "simplicial_sm100.cuh"
@@ -18,10 +18,9 @@ namespace {
 int check_packed(const MfSimplicialPackedArgs* a, const char* name, bool backward) {
   MF_CHECK_ARG(a != nullptr, "%s: null argument struct", name);
   MF_CHECK_ARG(a->batch >= 0 && a->heads >= 0 && a->tokens >= 0, "%s: negative size", name);
-  if (a->head_dim != kD || a->tokens > 32 || a->heads % 4 != 0) {
-    set_error("%s: serves head_dim 64, at most 32 tokens and a multiple of four heads (got head_dim %d, %d tokens, %d heads); "
-              "split the heads and call mf_simplicial_fwd / mf_simplicial_bwd otherwise", name, (int)a->head_dim,
-              (int)a->tokens, (int)a->heads);
+  if (a->head_dim != kD || a->tokens > 32) {
+    set_error("%s: serves head_dim 64 and at most 32 tokens (got head_dim %d, %d tokens); "
+              "split the heads and call mf_simplicial_fwd / mf_simplicial_bwd otherwise", name, (int)a->head_dim, (int)a->tokens);
     return MF_ERR_UNSUPPORTED;
   }
   if (a->batch == 0 || a->heads == 0 || a->tokens == 0) return MF_OK;

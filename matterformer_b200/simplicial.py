@@ -452,8 +452,8 @@ _KERNEL_CALLS = (cuda_simplicial_attention_forward, cuda_simplicial_attention_ba
 
 def packed_projection_applies(proj: torch.Tensor, heads: int, head_dim: int) -> bool:
     """Whether :func:`simplicial_attention_packed` serves this projection: CUDA bf16 (B, N, 5*H*64) with at most 32
-    tokens and a multiple of four heads."""
-    return (proj.is_cuda and proj.dtype == torch.bfloat16 and proj.ndim == 3 and head_dim == 64 and heads % 4 == 0
+    tokens."""
+    return (proj.is_cuda and proj.dtype == torch.bfloat16 and proj.ndim == 3 and head_dim == 64
             and proj.shape[1] <= 32 and proj.shape[2] == 5 * heads * head_dim and _BACKEND in ("auto", "tcgen05_tiles"))  # fmt: skip
 
 

@@ -51,3 +51,12 @@ def test_small_molecules_with_bias_against_oracle(B, H, N):
     assert_rel(y, out_ref, 2e-2, "out")
     for n in NAMES + BIAS_NAMES:
         assert_rel(grads[n], g_ref[n], 2.5e-2, f"d{n}")
+
+
+@pytest.mark.parametrize("B,H,N,holes", [(3, 1, 9, False), (2, 6, 29, True), (5, 3, 17, False), (171, 6, 8, False)])
+def test_packed_projection_serves_any_number_of_heads(B, H, N, holes):
+    from matterformer_b200.simplicial import packed_projection_applies
+    from test_simplicial_gpu import test_packed_projection_matches_the_head_major_call as compare
+
+    assert packed_projection_applies(torch.empty(B, N, 5 * H * 64, device="cuda:0", dtype=torch.bfloat16), H, 64)
+    compare(B, H, N, holes)
