@@ -447,9 +447,6 @@ class CudaTwoSimplicialAttentionFunction(torch.autograd.Function):
 
 
 
-_KERNEL_CALLS = (cuda_simplicial_attention_forward, cuda_simplicial_attention_backward)
-
-
 def packed_projection_applies(proj: torch.Tensor, heads: int, head_dim: int) -> bool:
     """Whether :func:`simplicial_attention_packed` serves this projection: CUDA bf16 (B, N, 5*H*64) with at most 32
     tokens."""
@@ -520,9 +517,8 @@ def simplicial_attention_cuda(q, k1, v1, k2, v2, *, query_valid, pair_key_valid,
     ``angle_residual`` an optional ``(left, right, gate)`` tuple and ``message_residual`` an optional
     ``(left, right, basis)`` tuple of the low-rank residuals (simplicial_attention.py:50-104).
     """
-    native = _lib.native()
-    if native is not None and not _CHECK_STATUS and _KERNEL_CALLS == (cuda_simplicial_attention_forward,
-                                                                      cuda_simplicial_attention_backward):  # fmt: skip
+    native = _lib.native() if q.is_cuda and not _CHECK_STATUS else None
+    if native is not None:
         # (checks, launch and autograd node in C++; None when an operand needs converting, or an error message)
         out = native.simplicial_attention(q, k1, v1, k2, v2, query_valid, pair_key_valid, pair_valid,
                                           factorized_bias or (), angle_residual or (), message_residual or (),
