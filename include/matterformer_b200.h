@@ -53,11 +53,12 @@ extern "C" {
 #define MF_PRECISION_IEEE_FP32 2
 
 /* Which implementation a simplicial call is allowed to use. */
-#define MF_BACKEND_AUTO 0    /* tensor-core (tcgen05) kernel when the problem qualifies, else the fp32 CUDA-core kernel */
+#define MF_BACKEND_AUTO 0    /* the fastest: a tensor-core kernel (warp-level mma.sync, or tcgen05 for the backward pass without
+                              * a bias above 32 tokens) when the problem qualifies, else the fp32 CUDA-core kernels */
 #define MF_BACKEND_GENERIC 1 /* always the fp32 CUDA-core kernel */
-#define MF_BACKEND_TCGEN05 2 /* tensor-core kernel (row-packed) or MF_ERR_UNSUPPORTED */
-#define MF_BACKEND_TCGEN05_TILES 3 /* tensor-core kernels with one query per tile row (warp-level ones up to 32 tokens and
-                                    * with the factorized bias), or MF_ERR_UNSUPPORTED */
+#define MF_BACKEND_TCGEN05 2 /* the row-packed tcgen05 kernels or MF_ERR_UNSUPPORTED */
+#define MF_BACKEND_TCGEN05_TILES 3 /* the tcgen05 kernels with one query per tile row; the warp-level mma.sync ones up to 32
+                                    * tokens and with the factorized bias, which those do not serve; or MF_ERR_UNSUPPORTED */
 
 /* ------------------------------------------------------------------------- */
 /* 2-simplicial attention                                                     */
@@ -184,8 +185,9 @@ typedef struct MfSimplicialBwdArgs {
 size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* args);
 size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* args);
 
-/* Which kernel family a call with these arguments runs on: MF_BACKEND_TCGEN05 or MF_BACKEND_GENERIC.  (No counterpart
- * in the reference.)  Only the tensor-core kernels leave a status word at the start of the workspace. */
+/* Whether a call with these arguments runs on tensor-core kernels (MF_BACKEND_TCGEN05, also where these are the warp-level
+ * mma.sync ones) or on CUDA cores (MF_BACKEND_GENERIC).  (No counterpart in the reference.)  Tensor-core kernels that take a
+ * workspace leave a status word at its start. */
 int mf_simplicial_fwd_backend(const MfSimplicialFwdArgs* args);
 int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* args);
 /* The gradient of message_basis from MfSimplicialBwdArgs.message_coeff: out[h,r,:] = sum_{b,i} coeff[b,h,i,r] grad_out[b,h,i,:]
@@ -214,17 +216,17 @@ int mf_simplicial_bwd(const MfSimplicialBwdArgs* args, void* stream);
  * For callers that cannot hand the library scratch memory because they cannot allocate any: code embedded in
  * another runtime's memory pool, loops that must stay off the allocator once they are running, or hosts whose
  * allocator has been shut down or frozen.  They pass inputs and outputs only; `workspace` / `workspace_bytes`
- * of the struct are ignored.  The scratch the tensor-core kernel needs (status word, per-molecule extents, launch
- * order) lives in an array that is part of the library image on every GPU that loads it, sized for at most 4096
- * molecules per call; a larger `batch` is rejected with MF_ERR_INVALID_ARGUMENT.  Only problems the tensor-core
- * forward kernel takes are accepted (bf16, precision bf16_tc, head_dim 64, tokens <= 192; otherwise
- * MF_ERR_UNSUPPORTED -- such problems need no scratch in mf_simplicial_fwd anyway).
+ * of the struct are ignored.  What scratch a kernel needs (status word, per-molecule extents, launch order) lives in an
+ * array that is part of the library image on every GPU that loads it, sized for at most 4096 molecules per call; a larger
+ * `batch` is rejected with MF_ERR_INVALID_ARGUMENT.  Only problems the tensor-core forward kernels take are accepted
+ * (bf16, precision bf16_tc, head_dim 64, tokens <= 192, no geometry operands; otherwise MF_ERR_UNSUPPORTED -- such problems
+ * need no scratch in mf_simplicial_fwd anyway).
  *
  * The first call on each device looks up the array's device address, so make that first call outside any stream
- * capture.  All calls on a device share the one array: calls whose kernels may overlap on the GPU (different
- * streams, different host threads) race on it and must be serialised by the caller.  The array keeps the previous
- * call's contents; the only part that must start at zero, the status word, is cleared by the call itself.
- * Results are identical to mf_simplicial_fwd.
+ * capture.  The kernels of MF_BACKEND_AUTO use none of the array (the call clears its status word): such calls may overlap.
+ * Calls that ask for a tcgen05 family above 32 tokens share the array: where their kernels may overlap on the GPU
+ * (different streams, different host threads) they race on it and must be serialised by the caller.  Results are
+ * identical to mf_simplicial_fwd.
  */
 int mf_simplicial_fwd_noalloc(const MfSimplicialFwdArgs* args, void* stream);
 

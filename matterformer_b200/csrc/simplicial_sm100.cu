@@ -541,9 +541,9 @@ int simplicial_sm100_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
 // ---------------------------------------------------------------------------
 // Forward pass for callers that cannot allocate device memory
 // ---------------------------------------------------------------------------
-// The tensor-core forward kernel needs a little scratch (status word, per-molecule extents, launch
-// order).  mf_simplicial_fwd takes it from the caller; this variant keeps it in the library image
-// instead, so a caller that only holds its input and output buffers -- a plugin running inside someone
+// The tcgen05 forward kernels need a little scratch (status word, per-molecule extents, launch order;
+// the warp-level ones of the default backend need none).  mf_simplicial_fwd takes it from the caller; this
+// variant keeps it in the library image instead, so a caller that only holds its input and output buffers -- a plugin running inside someone
 // else's memory pool, a real-time loop that may not touch the allocator, code that runs after the
 // framework's allocator has been frozen -- can still launch the kernel.  Every GPU that loads the
 // library carries the array (about 80 KB) until the process exits.
