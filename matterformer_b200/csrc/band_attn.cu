@@ -38,8 +38,6 @@ struct BandParams {
   RowLayout in, act;  // rows of q, k, v and their gradients; rows of out and grad_out
 };
 
-constexpr float kBandLow = 8.6736174e-19f, kBandHigh = 1.1529215e18f;  // 2^-60, 2^60
-
 // rows [first, first + rows) of one head into a swizzled tile; rows outside [0, n) become zeros
 template <int kThreads>
 __device__ __forceinline__ void load_band(uint32_t tile, const __nv_bfloat16* src, long long stride, int first, int rows, int n) {
@@ -208,7 +206,7 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
       for (int hh = 0; hh < 2; ++hh) {
         l[hh] = l2[hh].x + l2[hh].y;
         quad_reduce(l[hh]);
-        if (row + 8 * hh < n) fine = fine && l[hh] >= kBandLow && l[hh] <= kBandHigh;
+        if (row + 8 * hh < n) fine = fine && l[hh] >= kSumLow && l[hh] <= kSumHigh;
       }
       if (exact || __all_sync(0xffffffffu, fine)) break;
     }

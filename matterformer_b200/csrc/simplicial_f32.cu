@@ -39,15 +39,6 @@ struct F32Params {
   int H, N;
 };
 
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("{ .reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mov.b64 rc, {%6, %7}; "
-      "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0, %1}, rd; }"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
-}
-
 // rows [0, rows) of a (N, D) matrix into shared memory with `stride` floats per row; rows with `mask` clear become zeros
 template <int D>
 __device__ __forceinline__ void load_rows(float* dst, int stride, const float* src, int rows, uint64_t mask) {
@@ -77,8 +68,8 @@ __device__ __forceinline__ void dot4(float (&x)[4], const float* w, const float4
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const float4 y = *reinterpret_cast<const float4*>(w + t * D + 4 * c);
-      a[t] = ffma2(make_float2(y.x, y.y), make_float2(own[c].x, own[c].y), a[t]);
-      a[t] = ffma2(make_float2(y.z, y.w), make_float2(own[c].z, own[c].w), a[t]);
+      a[t] = fma2(make_float2(y.x, y.y), make_float2(own[c].x, own[c].y), a[t]);
+      a[t] = fma2(make_float2(y.z, y.w), make_float2(own[c].z, own[c].w), a[t]);
     }
 #pragma unroll
   for (int t = 0; t < 4; ++t) x[t] = a[t].x + a[t].y;
@@ -95,8 +86,8 @@ __device__ __forceinline__ void dot4_row(float (&x)[4], const float* w, const fl
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const float4 y = *reinterpret_cast<const float4*>(w + t * D + 4 * c);
-      a[t] = ffma2(make_float2(y.x, y.y), make_float2(o.x, o.y), a[t]);
-      a[t] = ffma2(make_float2(y.z, y.w), make_float2(o.z, o.w), a[t]);
+      a[t] = fma2(make_float2(y.x, y.y), make_float2(o.x, o.y), a[t]);
+      a[t] = fma2(make_float2(y.z, y.w), make_float2(o.z, o.w), a[t]);
     }
   }
 #pragma unroll
@@ -109,8 +100,8 @@ __device__ __forceinline__ void axpy(float4 (&sum)[D / 4], float c, const float*
 #pragma unroll
   for (int t = 0; t < D / 4; ++t) {
     const float4 y = *reinterpret_cast<const float4*>(row + 4 * t);
-    const float2 lo = ffma2(cc, make_float2(y.x, y.y), make_float2(sum[t].x, sum[t].y));
-    const float2 hi = ffma2(cc, make_float2(y.z, y.w), make_float2(sum[t].z, sum[t].w));
+    const float2 lo = fma2(cc, make_float2(y.x, y.y), make_float2(sum[t].x, sum[t].y));
+    const float2 hi = fma2(cc, make_float2(y.z, y.w), make_float2(sum[t].z, sum[t].w));
     sum[t] = make_float4(lo.x, lo.y, hi.x, hi.y);
   }
 }
@@ -326,8 +317,8 @@ __device__ __forceinline__ void f32_bwd_side(const F32Params& p, BwdShared<D>& s
 #pragma unroll
         for (int c = 0; c < D / 4; ++c) {
           const float4 y = *reinterpret_cast<const float4*>(&sm.row[warp][4 * c]);
-          const float2 lo = ffma2(make_float2(a[c].x, a[c].y), make_float2(y.x, y.y), make_float2(g2[c].x, g2[c].y));
-          const float2 hi = ffma2(make_float2(a[c].z, a[c].w), make_float2(y.z, y.w), make_float2(g2[c].z, g2[c].w));
+          const float2 lo = fma2(make_float2(a[c].x, a[c].y), make_float2(y.x, y.y), make_float2(g2[c].x, g2[c].y));
+          const float2 hi = fma2(make_float2(a[c].z, a[c].w), make_float2(y.z, y.w), make_float2(g2[c].z, g2[c].w));
           g2[c] = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
         float v[D], o[D / 32];

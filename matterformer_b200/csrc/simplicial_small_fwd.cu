@@ -46,11 +46,6 @@ struct SmallFwdShared {
   uint32_t visible[kSmallRows];                 // bit k of word j: the pair (j, k) counts
 };
 
-// The softmax is shifted by a value that need not be the maximum: as long as the shifted sum stays within 2^-60 .. 2^60,
-// nothing overflows and nothing that matters underflows.  The shift is 0; a warp with a row whose sum leaves that range
-// looks for the exact maxima and does its rows again.
-constexpr float kSumLow = 8.6736174e-19f, kSumHigh = 1.1529215e18f;
-
 // What a warp keeps over the walk: its 16 queries and all second keys, as operands of the logit product.
 template <int NT, bool kBias>
 struct SmallFwdRows {
@@ -212,7 +207,7 @@ __device__ __forceinline__ void small_fwd_rows(const SmallFwdParams& p, SmallFwd
     for (int hh = 0; hh < 2; ++hh)
       if ((qmask >> (hh ? ib : ia)) & 1u) fine &= ls[hh] >= kSumLow && ls[hh] <= kSumHigh;
     // every warp of the CTA takes part in the decision: the warps of one row tile are added up with one shift
-    if (exact || (kWarps > 1 ? __syncthreads_and(fine || js >= JS) : __all_sync(0xffffffffu, fine))) break;
+    if (exact || __syncthreads_and(fine || js >= JS)) break;
     exact = true;
     float m[2] = {-INFINITY, -INFINITY};
     for (int j = 0; j < n; ++j) {
@@ -232,7 +227,7 @@ __device__ __forceinline__ void small_fwd_rows(const SmallFwdParams& p, SmallFwd
       shift[hh] = m[hh] > -INFINITY ? m[hh] * kLog2e : 0.f;
     }
   }
-  if (kWarps > 1 && JS > 1) {  // the other warps of the row tile, in a fixed order, through the place of the tiles
+  if (JS > 1) {  // the other warps of the row tile, in a fixed order, through the place of the tiles
     constexpr int kStride = 34;  // o (32) and l (2) of a lane
     float(*part)[kStride][32] = reinterpret_cast<float(*)[kStride][32]>(sm.tile[0]);
     static_assert((kWarps - 1) * kStride * 32 * 4 <= 5 * kSmallTile, "partial rows of all but one warp fit the tiles");

@@ -11,6 +11,11 @@
 
 namespace mf {
 
+// The softmax is shifted by a value that need not be the maximum: as long as the shifted sum stays within 2^-60 .. 2^60,
+// nothing overflows and nothing that matters underflows.  The forward kernels take shift 0 and do the queries whose sum leaves
+// that range again, with their exact maxima.
+constexpr float kSumLow = 8.6736174e-19f, kSumHigh = 1.1529215e18f;
+
 constexpr int kRowBytes = kD * 2;            // one 64-channel bf16 row in shared memory
 constexpr int kSmallRows = 32;               // keys / queries of a small molecule
 constexpr int kSmallTile = kSmallRows * kRowBytes;
@@ -91,31 +96,6 @@ __device__ __forceinline__ void mma16_first(float (&d)[4], const uint32_t (&a)[4
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
-// two fp32 operations per instruction
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("{ .reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mov.b64 rc, {%6, %7}; "
-      "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0, %1}, rd; }"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("{ .reg .b64 ra, rb, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; add.rn.f32x2 rd, ra, rb; mov.b64 {%0, %1}, rd; }"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 r;
-  asm("{ .reg .b64 ra, rb, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mul.rn.f32x2 rd, ra, rb; mov.b64 {%0, %1}, rd; }"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-
 __device__ __forceinline__ void quad_reduce(float& v) {
   v += __shfl_xor_sync(0xffffffffu, v, 1);
   v += __shfl_xor_sync(0xffffffffu, v, 2);

@@ -40,7 +40,6 @@ struct WarpFwdParams {
 constexpr int kFwdWarps = 12;                  // 168 registers each fill the register file
 constexpr int kFwdThreads = 32 * kFwdWarps;
 constexpr int kBlocks = kMaxKeys / 32;
-constexpr float kWarpLow = 8.6736174e-19f, kWarpHigh = 1.1529215e18f;  // 2^-60, 2^60
 
 struct WarpFwdHeader {
   uint32_t visible[kMaxKeys][kBlocks];  // bit k of word (j, kb): the pair (j, 32 kb + k) counts
@@ -304,7 +303,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) simplicial_warp_fwd_kernel(con
         for (int jb = 0; jb < nb - half; ++jb) block_row<kBias, false, 2>(p, hd, fb, tile_bytes, qf, bh, i, jb, n, shift, st);
         if (half) block_row<kBias, false, 1>(p, hd, fb, tile_bytes, qf, bh, i, nb - 1, n, shift, st);
         l = warp_sum(st.l.x + st.l.y);
-        if (exact || (l >= kWarpLow && l <= kWarpHigh)) break;
+        if (exact || (l >= kSumLow && l <= kSumHigh)) break;
       }
       quad_sum8(st.o, lane);
     }
