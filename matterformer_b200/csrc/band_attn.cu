@@ -375,12 +375,17 @@ int launch_band(const BandParams& p, int BH, bool backward, cudaStream_t s) {
 }  // namespace
 
 // Windows whose chunks are whole, structures long enough that a tile is not mostly halo, or short enough that the window
-// reaches every pair of a 32-row tile; those between stay on the 32-row walk.
+// reaches every pair of a 32-row tile; those between stay on the 32-row walk.  Forward + backward of 64 structures x 8 heads,
+// walk | band: 96 tokens 42 | 33 us (window 32), 44 | 44 (64), 49 | 66 (128).  Under a window of 128 a tile is mostly halo up
+// to 192 tokens: 87 | 100 us at 160, 107 | 106 at 192, 145 | 126 at 256; there the band serves calls whose tiles are all
+// resident at once, two to an SM (4 structures of 160: 23 | 17), where the walk's three launches cost more than the halo.
 constexpr int kDenseTokens = 32;  // under windows of 64 and 128
 bool band_attn_applies(const MfSparseAttnArgs& a) {
   if (a.dtype != MF_DTYPE_BF16 || a.head_dim != 64) return false;
   if (a.tokens <= kDenseTokens) return a.window == 64 || a.window == 128;
-  return (a.window == 32 || a.window == 64 || a.window == 128) && a.tokens >= 96;
+  if (a.tokens < 96) return false;
+  if (a.window == 128) return a.tokens >= 192 || (long long)a.batch * a.heads * ((a.tokens + 63) / 64) <= 2 * 148;
+  return a.window == 32 || a.window == 64;
 }
 
 int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream) {
@@ -400,8 +405,10 @@ int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward
   p.act = layouts ? layouts[1] : contiguous_rows(a.heads, a.tokens);
   const int BH = a.batch * a.heads;
   if (a.tokens <= kDenseTokens) return launch_band<0, kDenseTokens>(p, BH, backward, stream);
-  // 128-row tiles re-read half as much halo; 64-row ones spread a small call over twice as many CTAs
-  const bool wide = (long long)BH * ((a.tokens + 127) / 128) >= 592;
+  // 128-row tiles re-read half as much halo; 64-row ones spread a call over twice as many CTAs, which pays while the wide ones
+  // would not cover the chip.  Forward + backward at window 64, 64 | 128 rows: 8 structures of 128 tokens (64 wide tiles) 14.7 |
+  // 16.3 us, 128 tiles 17.3 | 16.4, 256 tiles 29.1 | 22.5, 576 tiles 50.4 | 42.2; windows 32 and 128 turn at the same place.
+  const bool wide = (long long)BH * ((a.tokens + 127) / 128) >= 128;
   switch (a.window) {
     case 32: return wide ? launch_band<32, 128>(p, BH, backward, stream) : launch_band<32, 64>(p, BH, backward, stream);
     case 64: return wide ? launch_band<64, 128>(p, BH, backward, stream) : launch_band<64, 64>(p, BH, backward, stream);

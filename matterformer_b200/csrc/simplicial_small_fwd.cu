@@ -356,8 +356,10 @@ int simplicial_small_fwd(const MfSimplicialFwdArgs& a, const TileLayouts* layout
   p.in = layouts ? layouts->in : contiguous_rows(a.heads, a.tokens);
   p.act = layouts ? layouts->act : contiguous_rows(a.heads, a.tokens);
   const int bh = a.batch * a.heads;
-  // One warp per (batch, head) once that fills the chip several times over; fewer molecules are split over more warps.
-  const int warps = bh >= 1024 ? 2 : 4;
+  // Two warps per (batch, head), one for each row tile, once that fills the chip several times over; fewer molecules are split
+  // over four.  9-29 atoms x 8 heads, 2 | 4 warps: 64 molecules 20.2 | 15.8 us, 256 45.7 | 42.7, 512 76.4 | 77.6, 1024 140 |
+  // 148; with the bias 23.9 | 23.3, 57.2 | 56.9, 119 | 123, 222 | 239.
+  const int warps = bh >= 4096 ? 2 : 4;
   profile_mark(MF_PROFILE_SIMPLICIAL_FWD, true, stream);
 #define MF_LAUNCH(BIAS, W) simplicial_small_fwd_kernel<BIAS, W><<<bh, 32 * W, 0, stream>>>(p)
   if (a.u) {

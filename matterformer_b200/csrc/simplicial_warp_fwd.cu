@@ -335,8 +335,11 @@ int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   p.even = a.tokens % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.v_bias) | reinterpret_cast<uintptr_t>(a.w)) & 7) == 0;
   // Queries per CTA: two per warp keep the last wave short on large molecules (a CTA of 24 queries against 36 blocks runs 50
   // times as long as its loads take); smaller molecules need more to pay for their loads, small batches fewer to fill the chip.
+  // 64 molecules x 8 heads, 24 | 48 | 96 queries: up to 64 tokens 107 | 102 | 95 us, 96 215 | 207 | 222, 127 392 | 378 | 408,
+  // 128 401 | 384 | 410, 192 1 004 | 977 | 1 035; with the bias 176 | 173 | 166, 387 | 382 | 401, 833 | 831 | 891, 773 | 775 |
+  // 839, 2 076 | 2 131 | 2 296.  Halved below two CTAs per SM: 2 molecules of up to 192 tokens, 12 | 24 | 48: 62 | 101 | 183 us.
   const int bh = a.batch * a.heads;
-  int chunk = a.tokens >= 128 ? 24 : a.tokens >= 64 ? 48 : 96;
+  int chunk = a.tokens >= 128 ? 24 : a.tokens > 64 ? 48 : 96;
   while (chunk > 12 && (long long)bh * ((a.tokens + chunk - 1) / chunk) < 296) chunk >>= 1;
   p.chunk = chunk;
   const int rows = (a.tokens + 31) & ~31, bytes = (int)((sizeof(WarpFwdHeader) + 127) / 128 * 128) + 4 * rows * kRowBytes;

@@ -50,3 +50,11 @@ def test_packed_projection_takes_the_same_kernels():
     grads = torch.autograd.grad(y, parts, go.view(B, N, H, 64).transpose(1, 2).contiguous())
     assert torch.equal(out.view(B, N, H, 64).transpose(1, 2), y)
     assert torch.equal(gp, torch.cat([x.transpose(1, 2).reshape(B, N, -1) for x in grads], dim=-1))
+
+
+@pytest.mark.parametrize("B,H,N,window", [(37, 4, 128, 128), (25, 6, 127, 128), (13, 8, 191, 128), (13, 8, 192, 128), (16, 8, 65, 64),
+                                          (16, 8, 130, 64), (127, 1, 97, 32)])  # fmt: skip
+def test_both_sides_of_the_selection_rules(B, H, N, window):
+    """One wave of tiles and one tile more under a window of 128 below 192 tokens (band or walk), and both tile heights around
+    128 wide tiles: every choice is the same operator."""
+    test_band_attention_vs_oracle(B, H, N, window, 1.0)
