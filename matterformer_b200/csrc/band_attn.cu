@@ -13,8 +13,8 @@
 // a warp sees two chunks, and nothing but the structure's end is masked.  1 024 molecules of 9 - 29 tokens x 8
 // heads: forward 37 -> 25 us, backward 104 -> 53 us (two launches of the 32-row walk before).
 //
-// What bounds it: shared memory, 66 % of its bandwidth (operand fragments, at 16 rows per warp), while a CTA's loads overlap
-// only with the other CTAs of the SM.  32 cells of 4096 tokens x 8 heads, window 64: forward 144 us, backward 382 us (HBM
+// What bounds it: the L1 / shared-memory path, 62 % (forward) and 69 % (backward) of its throughput (operand fragments, at 16
+// rows per warp), while a CTA's loads overlap only with the other CTAs of the SM.  32 cells of 4096 tokens x 8 heads, window 64: forward 144 us, backward 382 us (HBM
 // floors 82 and 164 us), against 219 and 311 + 322 us for the 32-row walk with its three passes.
 #include "common.cuh"
 #include "simplicial_warp.cuh"

@@ -13,7 +13,7 @@
 // as its B operand), those over j an 8x8 transposition in registers.  delta_i = dO_i . out_i is formed on load.
 // Every output has one writer: no atomics, no workspace, nothing to zero beforehand.
 //
-// What bounds it: latency at two warps per scheduler (255 registers; the mma.sync pipe is 38 % busy, shared memory 50 %).
+// What bounds it: latency at two warps per scheduler (255 registers; the mma.sync pipe is 38 % busy, shared memory 46 %).
 // Measured at 1024 molecules of 9-29 atoms x 8 heads: 547 us, against 980 + 39 us for the tcgen05 tile kernel and its delta
 // pass; with the two sides on two warps of a pair 613 us (the V side waits for the K side, and two code paths share the
 // instruction cache).

@@ -6,7 +6,7 @@
 // needed (see kSumLow), so a step has no cross-lane operation and no barrier.  Small batches give a row tile to several
 // warps, which take every second or fourth j and are added up in a fixed order.
 //
-// What bounds it: instruction issue of the softmax next to the mma.sync pipe (42 % busy at 1024 molecules of 9-29 atoms x 8
+// What bounds it: instruction issue of the softmax next to the mma.sync pipe (43 % busy at 1024 molecules of 9-29 atoms x 8
 // heads).  Measured there: 140 us, against 358 us for tcgen05 tiles that put four heads on the 128 rows of a tile (every
 // row then meets the keys of all four heads, and a step passes through tensor memory with four barrier waits); one query per
 // step with the keys on both sides of the product (so that sums need shuffles in every step) took 195 us.
