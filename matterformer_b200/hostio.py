@@ -36,6 +36,8 @@ class HostPipelinedSimplicial:
         self._slots = [dict(inputs=None, results=None, ev_in=torch.cuda.Event(), ev_compute=torch.cuda.Event(),
                             ev_out=torch.cuda.Event(), used=False) for _ in range(self.depth)]  # fmt: skip
         self._next = 0
+        # the masks are read on the compute stream; whatever fills them has been enqueued on the caller's
+        self.s_compute.wait_stream(torch.cuda.current_stream(self.device))
 
     def submit(self, host_inputs: Sequence[torch.Tensor], host_outputs: Sequence[torch.Tensor]) -> None:
         slot = self._slots[self._next]

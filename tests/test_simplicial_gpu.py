@@ -295,6 +295,30 @@ def test_host_pipeline_gives_the_direct_results():
             assert torch.equal(got, want.cpu())
 
 
+def test_host_buffer_pipeline_waits_for_the_masks():
+    """The masks may still be on their way on the caller's stream when the pipeline is made."""
+    g = torch.Generator().manual_seed(0)
+    host_in = [(torch.randn(2, 2, 40, 64, generator=g) / 8).bfloat16().pin_memory() for _ in range(6)]
+    valid = torch.arange(40)[None, :] < torch.tensor([40, 23])[:, None]
+    results = []
+    for late in (False, True):
+        host_out = [torch.zeros_like(h).pin_memory() for h in host_in]
+        source, mask = valid.to(DEV), torch.zeros(2, 40, dtype=torch.bool, device=DEV)
+        torch.cuda.synchronize()
+        if late:
+            torch.cuda._sleep(200_000_000)  # a tenth of a second of other work
+        mask.copy_(source)
+        pipe = mfb.HostPipelinedSimplicial(torch.device(DEV), query_valid=mask, pair_key_valid=mask)
+        if not late:
+            torch.cuda.synchronize()
+        pipe.submit(host_in, host_out)
+        pipe.finish()
+        results.append(host_out)
+    assert results[0][0].abs().max() > 0
+    for x, y in zip(*results):
+        assert torch.equal(x, y)
+
+
 def test_status_word_is_read_from_tensor_core_calls_only():
     """The CUDA-core kernels keep no status word: their scratch must not be mistaken for one."""
     inp, go = _random_case(2, 4, 40, 64, seed=3, scale=1 / 8.0, lo=30)
