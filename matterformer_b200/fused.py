@@ -406,7 +406,13 @@ def masked_sum_applies(x: torch.Tensor, pad_mask: torch.Tensor, *others) -> bool
 
 
 def masked_update(pad_mask, x, a=1.0, y=None, z=None, c=1.0, p=None, q=None, k=0.0, center=False) -> torch.Tensor:
+    """``a x + c (y - z) + k (p - q)``, masked and centred as :func:`masked_sum` says; no autograd."""
+    if not masked_sum_applies(x, pad_mask, *(t for t in (y, z, p, q) if t is not None)) or pad_mask.device != x.device:
+        raise ValueError("masked sums take CUDA fp32 (B, N, C) tensors of one shape and a (B, N) bool mask, on one device")
     B, N, C = x.shape
+    for t in (a, c):
+        if isinstance(t, torch.Tensor) and not (t.shape == (B,) and t.dtype == torch.float32 and t.device == x.device and t.is_contiguous()):
+            raise ValueError("masked sums take numbers or contiguous fp32 (B,) tensors as factors")
     pad_mask = pad_mask.contiguous()
     x, y, z, p, q = (t.contiguous() if t is not None else None for t in (x, y, z, p, q))
     out = torch.empty_like(x)

@@ -140,22 +140,28 @@ def edm_sample(net, num_atoms: torch.Tensor, *, atom_channels: int = 6, lattice:
                 da, dc = net(a, c, pad_mask, s, lattice=lattice)
             return da.float(), dc.float()
 
+    fast = fused.masked_sum_applies(atoms, pad_mask) and coords.dtype == torch.float32
+
+    def evaluate(a, c, t):  # the fused updates read fp32 tensors of the sample's shape, whatever a caller's denoiser returns
+        da, dc = denoise(a, c, float(t))
+        return (da.float().expand_as(a), dc.float().expand_as(c)) if fast else (da, dc)
+
     churn = min(s_churn / max(num_steps, 1), math.sqrt(2.0) - 1.0)
     for step in range(num_steps):
         t_cur, t_next = t_steps[step], t_steps[step + 1]
         gamma = churn if s_min <= float(t_cur) <= s_max else 0.0
         t_hat = t_cur + gamma * t_cur
         extra = torch.sqrt(t_hat.square() - t_cur.square()) * s_noise
-        if device.type == "cuda":  # the same updates, one launch each
+        if fast:  # the same updates, one launch each
             extra, dt = float(extra), t_next - t_hat
             atoms_hat = fused.masked_sum(pad_mask, atoms, y=torch.randn_like(atoms), c=extra)
             coords_hat = fused.masked_sum(pad_mask, coords, y=torch.randn_like(coords), c=extra, center=True)
-            den_a, den_c = denoise(atoms_hat, coords_hat, float(t_hat))
+            den_a, den_c = evaluate(atoms_hat, coords_hat, t_hat)
             ratio = float(dt / t_hat)
             atoms = fused.masked_sum(pad_mask, atoms_hat, y=atoms_hat, z=den_a, c=ratio)
             coords = fused.masked_sum(pad_mask, coords_hat, y=coords_hat, z=den_c, c=ratio, center=True)
             if step < num_steps - 1:  # half of the first step, half of the slope at the new point
-                den_a, den_c = denoise(atoms, coords, float(t_next))
+                den_a, den_c = evaluate(atoms, coords, t_next)
                 half = 0.5 * float(dt / t_next.clamp_min(1e-8))
                 atoms = fused.masked_update(pad_mask, atoms_hat, y=atoms, z=atoms_hat, c=0.5, p=atoms, q=den_a, k=half)
                 coords = fused.masked_update(pad_mask, coords_hat, y=coords, z=coords_hat, c=0.5, p=coords, q=den_c, k=half, center=True)
@@ -163,12 +169,12 @@ def edm_sample(net, num_atoms: torch.Tensor, *, atom_channels: int = 6, lattice:
         atoms_hat = (atoms + extra * torch.randn_like(atoms)).masked_fill(hole, 0.0)
         coords_hat = recenter_coordinates(coords + extra * torch.randn_like(coords), pad_mask)
 
-        den_a, den_c = denoise(atoms_hat, coords_hat, float(t_hat))
+        den_a, den_c = evaluate(atoms_hat, coords_hat, t_hat)
         d_a, d_c = (atoms_hat - den_a) / t_hat, (coords_hat - den_c) / t_hat
         atoms = atoms_hat + (t_next - t_hat) * d_a
         coords = recenter_coordinates(coords_hat + (t_next - t_hat) * d_c, pad_mask)
         if step < num_steps - 1:  # trapezoidal correction with the slope at the new point
-            den_a, den_c = denoise(atoms, coords, float(t_next))
+            den_a, den_c = evaluate(atoms, coords, t_next)
             t_safe = t_next.clamp_min(1e-8)
             dp_a, dp_c = (atoms - den_a) / t_safe, (coords - den_c) / t_safe
             atoms = atoms_hat + (t_next - t_hat) * 0.5 * (d_a + dp_a)

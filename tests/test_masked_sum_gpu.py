@@ -31,3 +31,16 @@ def test_masked_sum_against_torch(B, N, C, center):
     with torch.no_grad():
         want = ref(0.5 * x + 0.25 * y - 3.0 * (p - q))
         torch.testing.assert_close(fused.masked_update(pad, x, 0.5, y, None, 0.25, p, q, -3.0, center), want, atol=2e-6, rtol=1e-5)
+
+
+def test_operands_of_other_types_shapes_and_places_are_refused():
+    """The kernel reads them as they lie: a narrower type, a shorter factor or a host tensor would be read beyond its end."""
+    x, pad = torch.zeros(4, 5, 3, device="cuda"), torch.zeros(4, 5, dtype=torch.bool, device="cuda")
+    for bad in (dict(y=x.bfloat16()), dict(y=x[:1]), dict(y=x.cpu()), dict(y=x, z=x[:, :4]), dict(p=x, q=x.half(), k=1.0),
+                dict(a=torch.ones(1, device="cuda")), dict(a=torch.ones(4, device="cuda", dtype=torch.float64)),
+                dict(y=x, c=torch.ones(8, device="cuda")[::2]), dict(a=torch.ones(4))):  # fmt: skip
+        with pytest.raises(ValueError, match="masked sums take"):
+            fused.masked_update(pad, x, **bad)
+    for args in ((pad.cpu(), x), (pad.float(), x), (pad[:, :4], x), (pad, x.cpu()), (pad, x.double())):
+        with pytest.raises(ValueError, match="masked sums take"):
+            fused.masked_update(*args)

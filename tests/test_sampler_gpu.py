@@ -48,6 +48,19 @@ def test_updates_on_cuda_equal_those_on_the_cpu(monkeypatch, kw):
         assert (x - y).abs().max() <= 2e-5 * max(1.0, x.abs().max().item(), kw.get("sigma_max", 10.0))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_a_denoiser_may_return_other_types_and_broadcast_shapes(dtype):
+    """Its outputs enter the updates by value, as in element-wise operations."""
+    n = torch.tensor([9, 6, 1, 4])
+    outs = []
+    for convert in (lambda t: t, lambda t: t.float()):
+        torch.manual_seed(4)
+        low = lambda a, c, sigma: (convert((0.5 * a[:1]).to(dtype)), convert((0.5 * c).to(dtype)))  # noqa: B023, E731
+        outs.append(edm_sample(_Net("cuda:0"), n, denoiser=low, num_steps=4))
+    for x, y in zip(outs[0][:2], outs[1][:2]):
+        assert torch.equal(x, y) and torch.isfinite(x).all()
+
+
 @pytest.mark.parametrize("name,kw", [("churn", dict(num_steps=5)), ("plain", dict(num_steps=3, s_churn=0.0, sigma_max=5.0))])
 def test_sampler_on_cuda_matches_the_reference(golden, monkeypatch, name, kw):
     """The reference's own samples (fp32, as on the CPU), with the network and the updates on the GPU.  The network's fp32
