@@ -35,6 +35,14 @@ def fused_applies(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype in _CODE and x.ndim == 3 and x.shape[-1] <= MAX_CHANNELS and x.shape[-1] % 8 == 0
 
 
+def _check_shapes(x: torch.Tensor, rows=(), vectors=(), pad: Optional[torch.Tensor] = None) -> None:
+    """The kernels read ``rows`` as (B, N, C) like ``x``, ``vectors`` as (B, C) and ``pad`` as (B, N): nothing is broadcast."""
+    B, N, C = x.shape
+    fits = all(t.shape == x.shape and t.device == x.device for t in rows) and all(t.shape == (B, C) and t.device == x.device for t in vectors)
+    if not fits or (pad is not None and (pad.shape != (B, N) or pad.device != x.device)):
+        raise ValueError(f"expected operands of shapes {(B, N, C)}, {(B, C)} and {(B, N)} on {x.device}")
+
+
 class _LnModulate(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, shift, scale, eps, out_dtype):
@@ -108,6 +116,7 @@ class _GatedResidual(torch.autograd.Function):
 def ln_modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, *, eps: float,
                 out_dtype: torch.dtype = torch.float32) -> torch.Tensor:  # fmt: skip
     """``LayerNorm(x) * (1 + scale[:, None, :]) + shift[:, None, :]`` in ``out_dtype`` (fp32 or bf16)."""
+    _check_shapes(x, vectors=(shift, scale))
     return _LnModulate.apply(x, shift, scale, eps, out_dtype)
 
 
@@ -115,6 +124,7 @@ def gated_residual(x: torch.Tensor, gate: torch.Tensor, a: torch.Tensor,
                    pad_mask: Optional[torch.Tensor] = None) -> torch.Tensor:  # fmt: skip
     """``x + gate[:, None, :] * a`` in ``x``'s dtype; with ``pad_mask`` (B, N) bool, followed by
     ``.masked_fill(pad_mask[..., None], 0)`` in the same pass (forward and backward)."""
+    _check_shapes(x, (a,), (gate,), pad_mask)
     return _GatedResidual.apply(x, gate, a, pad_mask)
 
 
@@ -156,6 +166,7 @@ def gated_ln_modulate(x: torch.Tensor, gate: torch.Tensor, a: torch.Tensor, pad_
     """``y = gated_residual(x, gate, a, pad_mask)`` and ``ln_modulate(y, shift, scale)``; one pass where ``a`` already has
     ``out_dtype`` and the modulation is fp32, the two operators otherwise."""
     if a.dtype == out_dtype and a.dtype in _CODE and all(t.dtype == torch.float32 for t in (gate, shift, scale)):
+        _check_shapes(x, (a,), (gate, shift, scale), pad_mask)
         return _GatedLnModulate.apply(x, gate, a, pad_mask, shift, scale, eps)
     y = gated_residual(x, gate, a, pad_mask)
     return y, ln_modulate(y, shift, scale, eps=eps, out_dtype=out_dtype)

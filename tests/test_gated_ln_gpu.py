@@ -25,3 +25,22 @@ def test_one_pass_equals_two_operators(B, N, C, xd, hd, padded):
     for u, v, t in zip(torch.autograd.grad([y, h], leaves, [gy, gh]), want, leaves):
         tol = 2e-2 if torch.bfloat16 in (xd, hd) else 1e-5  # dx: one rounding of the sum instead of two
         torch.testing.assert_close(u.float(), v.float(), atol=tol * float(v.float().abs().max()), rtol=tol)
+
+
+def test_operands_that_would_need_broadcasting_are_refused():
+    """The kernels read one vector per molecule and one row per token where they expect them."""
+    from matterformer_b200 import fused
+
+    x, v, pad = torch.zeros(3, 4, 16, device="cuda"), torch.zeros(3, 16, device="cuda"), torch.zeros(3, 4, dtype=torch.bool, device="cuda")
+    kw = dict(eps=1e-6, out_dtype=torch.float32)
+    fused.gated_ln_modulate(x, v, x, pad, v, v, **kw)
+    for args in ((x, v[:1], x, pad, v, v), (x, v, x[:1], pad, v, v), (x, v, x, pad[:1], v, v), (x, v, x, pad, v[:, :8], v),
+                 (x, v, x, pad, v, v.cpu())):  # fmt: skip
+        with pytest.raises(ValueError, match="expected operands"):
+            fused.gated_ln_modulate(*args, **kw)
+    for args in ((x, v[:1], v), (x, v, v[0])):
+        with pytest.raises(ValueError, match="expected operands"):
+            fused.ln_modulate(*args, **kw)
+    for args in ((x, v[:2], x), (x, v, x[:, :1]), (x, v, x, pad[:, :1])):
+        with pytest.raises(ValueError, match="expected operands"):
+            fused.gated_residual(*args)
