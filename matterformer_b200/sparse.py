@@ -61,6 +61,13 @@ def _lattice_operand(lattice: torch.Tensor, device: torch.device) -> tuple[torch
     return _as_cell(lattice.detach()).to(device), 1
 
 
+def _check_structures(pos: torch.Tensor, lattice: torch.Tensor) -> None:
+    if pos.ndim != 3 or pos.shape[-1] != 3:
+        raise ValueError(f"pos must have shape (B, N, 3), got {tuple(pos.shape)}")
+    if lattice.shape[0] != pos.shape[0]:
+        raise ValueError(f"lattice must hold one cell per structure ({pos.shape[0]}), got shape {tuple(lattice.shape)}")
+
+
 def cell_grid_dims(cell: torch.Tensor, cutoff: float, max_per_axis: int = 64) -> torch.Tensor:
     """Cells per axis = floor(perpendicular width / cutoff), clamped to [1, max_per_axis]. (B,3) int32."""
     c = cell.double()
@@ -81,6 +88,8 @@ def cell_grid_dims(cell: torch.Tensor, cutoff: float, max_per_axis: int = 64) ->
 def _num_atoms(num_atoms: Optional[torch.Tensor], batch: int, n: int, device) -> torch.Tensor:
     if num_atoms is None:
         return torch.full((batch,), n, device=device, dtype=torch.int32)
+    if num_atoms.numel() != batch:
+        raise ValueError(f"num_atoms must hold one count per structure ({batch}), got shape {tuple(num_atoms.shape)}")
     return num_atoms.to(device=device, dtype=torch.int32).contiguous()
 
 
@@ -111,8 +120,7 @@ def knn_topk(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Optional[torch
     """
     if pos.device.type != "cuda":
         raise RuntimeError("knn_topk requires CUDA tensors")
-    if pos.ndim != 3 or pos.shape[-1] != 3:
-        raise ValueError(f"pos must have shape (B, N, 3), got {tuple(pos.shape)}")
+    _check_structures(pos, lattice)
     if method not in ("cells", "pairs"):
         raise ValueError(f"method must be 'cells' or 'pairs', got {method!r}")
     B, N, _ = pos.shape
@@ -161,6 +169,7 @@ def build_radius_blocks(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Opt
         raise ValueError("only 32-atom tiles are supported")
     if pos.device.type != "cuda":
         raise RuntimeError("build_radius_blocks requires CUDA tensors")
+    _check_structures(pos, lattice)
     B, N, _ = pos.shape
     T = (N + 31) // 32
     dev = pos.device
@@ -297,6 +306,9 @@ def radius_block_sparse_attention(q, k, v, blocks: RadiusBlocks, *, scale: Optio
     scattered back.  Rows of padded atoms (and atoms without any neighbour) return zeros.
     """
     _check_qkv("radius_block_sparse_attention", q, k, v)
+    if blocks.perm.shape != (q.shape[0], q.shape[2]) or blocks.perm.device != q.device:
+        raise ValueError(f"the block list is of {tuple(blocks.perm.shape)} atoms on {blocks.perm.device}, q of "
+                         f"{(q.shape[0], q.shape[2])} on {q.device}")  # fmt: skip
     scale = q.shape[-1] ** -0.5 if scale is None else float(scale)
     if not sorted_inputs:
         idx = blocks.perm.long()[:, None, :, None].expand_as(q)

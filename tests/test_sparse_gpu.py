@@ -382,3 +382,21 @@ def test_local_attention_on_the_packed_projection(B, H, N, D, window):
         mfb.set_sparse_backend(prev)
     assert torch.equal(out.view(B, N, H, D).transpose(1, 2), y)
     assert torch.equal(gx.view(B, N, 3, H, D), torch.stack([t.transpose(1, 2) for t in grads], dim=2))
+
+
+def test_operands_of_another_batch_are_refused():
+    """Counts, cells and block lists are read per structure: one for all, or those of another batch, would be read beyond their end."""
+    lat, frac, _ = _cells(3, 40, seed=1)
+    lat, frac, n = lat.to(DEV), frac.to(DEV), torch.tensor([40, 20, 30], device=DEV)
+    blocks = mfb.build_radius_blocks(frac, lat, n, 4.0)
+    qkv = [torch.zeros(3, 2, 40, 64, device=DEV, dtype=torch.bfloat16) for _ in range(3)]
+    mfb.radius_block_sparse_attention(*qkv, blocks)
+    mfb.local_window_attention(*qkv, n[:, None], window=64)  # (one count each, whatever the shape)
+    for call in (lambda: mfb.knn_topk(frac, lat[:1], n, k=4), lambda: mfb.knn_topk(frac, lat, n[:2], k=4),
+                 lambda: mfb.knn_topk(frac, lat[:1], n, k=4, method="pairs"),
+                 lambda: mfb.build_radius_blocks(frac, lat[:2], n, 4.0), lambda: mfb.build_radius_blocks(frac[0], lat, n, 4.0),
+                 lambda: mfb.build_radius_blocks(frac, lat, n[:1], 4.0), lambda: mfb.local_window_attention(*qkv, n[:1], window=64),
+                 lambda: mfb.radius_block_sparse_attention(*(t[:, :, :30] for t in qkv), blocks),
+                 lambda: mfb.radius_block_sparse_attention(*(torch.cat([t, t]) for t in qkv), blocks)):  # fmt: skip
+        with pytest.raises(ValueError):
+            call()
