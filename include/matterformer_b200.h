@@ -115,7 +115,9 @@ typedef struct MfSimplicialFwdArgs {
   float* out;     /* (B,H,N,D) fp32, written for every row (zeros where invalid) */
   float* lse;     /* (B,H,N)   fp32 natural-log sum of exp over visible pairs */
   void* out_cast; /* optional (B,H,N,D) copy of out in `dtype`; may be NULL */
-  void* workspace; /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0 */
+  /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0.  With the factorized bias above
+   * 32 tokens a call without it is served too, by a kernel that needs none and takes about twice as long. */
+  void* workspace;
   size_t workspace_bytes;
 } MfSimplicialFwdArgs;
 

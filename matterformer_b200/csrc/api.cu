@@ -105,15 +105,17 @@ bool uses_small_kernels(const Args* a) {
   return (a->backend == MF_BACKEND_AUTO || a->backend == MF_BACKEND_TCGEN05_TILES) && a->tokens <= kSmallTokens;
 }
 
-// Larger molecules: the forward pass runs on the warp-level kernel, unless a tcgen05 family is asked for.
-// With the factorized bias there is no other kernel.
+// Larger molecules: with the factorized bias the trilinear tcgen05 kernels (simplicial_tri.cu has both sides' times).  Without it the
+// forward pass runs on the warp-level kernel, unless a tcgen05 family is asked for: 64 molecules of 20-181 atoms take 0.64 ms on
+// the trilinear kernel against 0.89, but 2 molecules 201 us against 105, and the choice may not depend on the batch (a molecule's
+// result does not); the backward pass runs on the row-packed kernel (1.98 against 2.26 ms).
+template <typename Args>
+bool uses_tri_kernels(const Args* a) {
+  return a->tokens > kSmallTokens && has_factorized_bias(a);
+}
 inline bool uses_warp_forward(const MfSimplicialFwdArgs* a) {
   return a->tokens > kSmallTokens && (a->backend == MF_BACKEND_AUTO || has_factorized_bias(a));
 }
-
-// The backward pass does with the factorized bias (with eight warps against twelve, and five products to two, the row-packed
-// tcgen05 kernel is the faster one without it: 1.97 against 3.8 ms for 64 molecules of 20-181 atoms).
-inline bool uses_warp_backward(const MfSimplicialBwdArgs* a) { return a->tokens > kSmallTokens && has_factorized_bias(a); }
 
 // fp32 molecules of at most 64 tokens (two keys per lane would not fit the registers), plain attention, aligned rows.
 template <typename Args>
@@ -144,7 +146,9 @@ extern "C" int mf_feature_flags(void) { return tensor_maps_available() ? MF_FEAT
 extern "C" size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* a) {
   if (!a) return 0;
   int rc;
-  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd") && !uses_small_kernels(a) && !uses_warp_forward(a)) return simplicial_sm100_fwd_workspace_bytes(*a);
+  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd") && !uses_small_kernels(a))
+    return uses_tri_kernels(a)    ? simplicial_tri_fwd_workspace_bytes(*a)
+           : uses_warp_forward(a) ? 0 : simplicial_sm100_fwd_workspace_bytes(*a);
   return 0;
 }
 
@@ -153,7 +157,7 @@ extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a
   int rc;
   if (wants_tcgen05(a, &rc, "mf_simplicial_bwd"))
     return uses_small_kernels(a)   ? 0
-           : uses_warp_backward(a) ? simplicial_warp_bwd_workspace_bytes(*a)
+           : uses_tri_kernels(a)   ? simplicial_tri_bwd_workspace_bytes(*a)
            : a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
   return uses_f32_kernels(a) ? 0 : simplicial_generic_bwd_workspace_bytes(*a);
 }
@@ -197,14 +201,16 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
   const bool tc = wants_tcgen05(a, &rc, "mf_simplicial_fwd");
   if (rc != MF_OK) return rc;
   const size_t need = mf_simplicial_fwd_workspace_bytes(a);
-  if (need > 0 && (!a->workspace || a->workspace_bytes < need)) {
+  const bool scratch = a->workspace && a->workspace_bytes >= need;
+  if (need > 0 && !scratch && !uses_tri_kernels(a)) {
     set_error("mf_simplicial_fwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
   if (!tc) return uses_f32_kernels(a) ? simplicial_f32_fwd(*a, s) : simplicial_generic_fwd(*a, s);
   if (uses_small_kernels(a))
     return a->angle_left || a->message_left ? simplicial_small_res_fwd(*a, s) : simplicial_small_fwd(*a, nullptr, s);
-  if (uses_warp_forward(a)) return simplicial_warp_fwd(*a, s);
+  if (uses_tri_kernels(a) && scratch) return simplicial_tri_fwd(*a, s);
+  if (uses_warp_forward(a)) return simplicial_warp_fwd(*a, s);  // with the bias: callers that give no workspace
   return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
 }
 
@@ -227,7 +233,7 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
   }
   if (!tc) return uses_f32_kernels(a) ? simplicial_f32_bwd(*a, s) : simplicial_generic_bwd(*a, s);
   if (uses_small_kernels(a)) return simplicial_small_bwd(*a, nullptr, s);
-  if (uses_warp_backward(a)) return simplicial_warp_bwd(*a, s);
+  if (uses_tri_kernels(a)) return simplicial_tri_bwd(*a, s);
   return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
 }
 

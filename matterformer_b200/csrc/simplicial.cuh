@@ -33,9 +33,12 @@ int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 
 // warp-level forward kernel for 33 to 192 tokens (simplicial_warp_fwd.cu)
 int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
-// and the backward kernel with the factorized bias (simplicial_warp_bwd.cu)
-int simplicial_warp_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
-size_t simplicial_warp_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
+
+// trilinear tcgen05 kernels for 33 to 192 tokens with the factorized bias (simplicial_tri.cu)
+int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
+int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
+size_t simplicial_tri_fwd_workspace_bytes(const MfSimplicialFwdArgs& a);
+size_t simplicial_tri_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 
 // row-packed tcgen05 kernels (simplicial_rows_fwd.cu, simplicial_rows_bwd.cu); same problems as the kernels above
 int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);

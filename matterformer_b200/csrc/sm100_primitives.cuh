@@ -59,6 +59,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The phase's state as it is (try_wait may hold the thread for a while before it answers "not yet")
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Same test, but the thread may be parked by the hardware for up to `hint_ns` nanoseconds while the phase is
 // incomplete (it is woken when the phase completes).  A parked thread issues nothing, so waiting warps do not
 // take issue slots from the warps that share their scheduler.
@@ -90,6 +105,20 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, lo
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return mbar_wait_for(bar, parity, kWaitLimitCycles);
+}
+
+// True in one lane of the converged warp.  A branch on this predicate, unlike one on the lane number, is known to hold one thread,
+// so the operands of tcgen05.mma in it stay in uniform registers instead of being moved there before every instruction.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one = 0;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "@p mov.u32 %0, 1;\n\t"
+      "}"
+      : "+r"(one));
+  return one != 0;
 }
 
 // ---------------------------------------------------------------------------

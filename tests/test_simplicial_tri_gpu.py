@@ -1,0 +1,67 @@
+"""Trilinear tcgen05 kernels (factorized bias, 33 to 192 tokens): unequal extents, empty molecules, exact maxima, no workspace."""
+import pytest
+import torch
+
+from conftest import bf16_allowance
+from matterformer_b200 import _lib
+from matterformer_b200.simplicial import cuda_simplicial_attention_forward
+from oracle.simplicial_ref import simplicial_forward_backward
+from test_simplicial_gpu import BIAS_NAMES, NAMES, assert_rel, run_cuda_bias
+from test_simplicial_small_gpu import _case
+from test_simplicial_warp_gpu import _with_bias
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(inp, go):
+    out_ref, g_ref = simplicial_forward_backward(inp, go)
+    y, grads = run_cuda_bias(inp, go, dtype=torch.bfloat16, precision="bf16_tc")
+    assert_rel(y, out_ref, 2e-2, "out")  # operands, probabilities and their gradients rounded to 8 bits
+    for n in NAMES + BIAS_NAMES:
+        assert_rel(grads[n], g_ref[n], 2.5e-2, f"d{n}")
+
+
+@pytest.mark.parametrize("N,queries,keys", [(40, 3, 40), (64, 64, 5), (97, 17, 97), (129, 129, 16), (192, 1, 130), (192, 192, 3), (190, 33, 161)])
+def test_unequal_extents(N, queries, keys):
+    """One to eight y per step, one to three chunks of columns (each of 16 to 64), rows of a tile that carry no pair."""
+    inp, go = _case(2, 2, N, seed=N + queries, scale=0.5, lo=N)
+    _with_bias(inp, N)
+    at = torch.arange(N)[None, :]
+    inp.query_valid = (at < queries).repeat(2, 1)
+    inp.pair_key_valid = (at < keys).repeat(2, 1)
+    inp.query_valid[1, 0] = queries > 1  # a hole in front
+    inp.pair_key_valid[1, keys // 2] = keys == 1
+    _check(inp, go)
+
+
+def test_empty_molecules():
+    inp, go = _case(4, 2, 50, seed=1, scale=0.5, lo=30)
+    _with_bias(inp, 1)
+    inp.query_valid[1] = False
+    inp.pair_key_valid[2] = False
+    _check(inp, go)
+
+
+@pytest.mark.parametrize("shift", [1.5, -1.5])
+def test_exact_maxima(shift):
+    """Logits near +-216 leave the range of a softmax with shift 0: the tile is done again with its maxima."""
+    inp, go = _case(2, 2, 70, seed=70, scale=0.2, lo=35, shift=shift)
+    _with_bias(inp, 70)
+    out_ref, g_ref = simplicial_forward_backward(inp, go)
+    tol = bf16_allowance(inp, go, out_ref, g_ref)  # logits this large carry the rounding of their products
+    y, grads = run_cuda_bias(inp, go, dtype=torch.bfloat16, precision="bf16_tc")
+    assert_rel(y, out_ref, tol["out"], "out")
+    for n in NAMES:
+        assert_rel(grads[n], g_ref[n], tol[n], f"d{n}")
+
+
+def test_forward_without_workspace(monkeypatch):
+    """A caller that gives no workspace gets the warp-level kernel."""
+    inp, go = _case(2, 2, 77, seed=77, scale=0.5, lo=38)
+    _with_bias(inp, 77)
+    out_ref, _ = simplicial_forward_backward(inp, go)
+    monkeypatch.setattr(_lib.lib(), "mf_simplicial_fwd_workspace_bytes", lambda ref: 0)
+    out, _, _ = cuda_simplicial_attention_forward(
+        *(getattr(inp, n).bfloat16().cuda() for n in NAMES), query_valid=inp.query_valid.cuda(), pair_key_valid=inp.pair_key_valid.cuda(),
+        pair_valid=None, **{n: getattr(inp, n).cuda() for n in BIAS_NAMES})  # fmt: skip
+    assert_rel(out.float().cpu(), out_ref, 2e-2, "out")
