@@ -40,3 +40,24 @@ def test_knn_from_latents_matches_all_pairs(B, N, k):
     ic, dc = mfb.knn_topk(*args, k=k)
     ip, dp = mfb.knn_topk(*args, k=k, method="pairs")
     assert torch.equal(ic, ip) and torch.equal(dc, dp)
+
+
+def test_equal_distances():
+    """Atoms on a grid: distances that equal the cutoff, and neighbours that only their indices order."""
+    axis = torch.arange(8) / 8.0
+    frac = torch.stack(torch.meshgrid(axis, axis, axis, indexing="ij"), dim=-1).reshape(1, 512, 3)
+    frac = frac[:, torch.randperm(512, generator=torch.Generator().manual_seed(3))]
+    lat = torch.tensor([[16.0, 16.0, 16.0, 1.0, 1.0, 1.0]])
+    lat = torch.cat([lat[:, :3].log(), torch.zeros(1, 3)], dim=1)
+    n = torch.tensor([512])
+    cell = mfb.lattice_latent_to_cell(lat.to(DEV)).cpu()
+    for cutoff in (2.0, 4.0, 6.0, float(torch.tensor(8.0).sqrt()), 8.5):
+        blocks = mfb.build_radius_blocks(frac.to(DEV), lat.to(DEV), n.to(DEV), cutoff)
+        want = geom_ref.cell_sort_blocklist(frac, cell, n, cell_grid_dims(cell, cutoff), cutoff)
+        for got, ref in zip((blocks.perm, blocks.block_count, blocks.block_cols, blocks.block_mask), want):
+            assert torch.equal(got.cpu(), ref)
+    args = (frac.to(DEV), lat.to(DEV), n.to(DEV))
+    for k in (5, 16, 32):
+        ic, dc = mfb.knn_topk(*args, k=k)
+        ip, dp = mfb.knn_topk(*args, k=k, method="pairs")
+        assert torch.equal(ic, ip) and torch.equal(dc, dp)
