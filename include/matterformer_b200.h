@@ -115,8 +115,9 @@ typedef struct MfSimplicialFwdArgs {
   float* out;     /* (B,H,N,D) fp32, written for every row (zeros where invalid) */
   float* lse;     /* (B,H,N)   fp32 natural-log sum of exp over visible pairs */
   void* out_cast; /* optional (B,H,N,D) copy of out in `dtype`; may be NULL */
-  /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0.  With the factorized bias above
-   * 32 tokens a call without it is served too, by a kernel that needs none and takes about twice as long. */
+  /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0.  Tensor-core calls of at most 32 tokens
+   * are served without it too (with it, large batches start with their heavy molecules), and with the factorized bias above 32
+   * tokens (by a kernel that needs none and takes about twice as long). */
   void* workspace;
   size_t workspace_bytes;
 } MfSimplicialFwdArgs;
@@ -150,7 +151,8 @@ typedef struct MfSimplicialBwdArgs {
   void* dv1;
   void* dk2;
   void* dv2;
-  void* workspace; /* mf_simplicial_bwd_workspace_bytes() bytes, 256-byte aligned */
+  /* mf_simplicial_bwd_workspace_bytes() bytes, 256-byte aligned; may be NULL for tensor-core calls of at most 32 tokens */
+  void* workspace;
   size_t workspace_bytes;
   /* Factorized bias of the forward call (all four or none, fp32, same shapes) and the gradients
    * the reference returns for it (triton_simplicial_attention.py:929-1204, outputs du, dv, dw, dgate).

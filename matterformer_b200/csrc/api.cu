@@ -146,17 +146,16 @@ extern "C" int mf_feature_flags(void) { return tensor_maps_available() ? MF_FEAT
 extern "C" size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* a) {
   if (!a) return 0;
   int rc;
-  if (wants_tcgen05(a, &rc, "mf_simplicial_fwd") && !uses_small_kernels(a))
-    return uses_tri_kernels(a)    ? simplicial_tri_fwd_workspace_bytes(*a)
-           : uses_warp_forward(a) ? 0 : simplicial_sm100_fwd_workspace_bytes(*a);
-  return 0;
+  if (!wants_tcgen05(a, &rc, "mf_simplicial_fwd")) return 0;
+  if (uses_small_kernels(a)) return simplicial_small_order_bytes(a->batch, a->heads, false, a->angle_left || a->message_left);
+  return uses_tri_kernels(a) ? simplicial_tri_fwd_workspace_bytes(*a) : uses_warp_forward(a) ? 0 : simplicial_sm100_fwd_workspace_bytes(*a);
 }
 
 extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a) {
   if (!a) return 0;
   int rc;
   if (wants_tcgen05(a, &rc, "mf_simplicial_bwd"))
-    return uses_small_kernels(a)   ? 0
+    return uses_small_kernels(a)   ? simplicial_small_order_bytes(a->batch, a->heads, true, a->angle_left || a->message_left)
            : uses_tri_kernels(a)   ? simplicial_tri_bwd_workspace_bytes(*a)
            : a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd_workspace_bytes(*a) : simplicial_rows_bwd_workspace_bytes(*a);
   return uses_f32_kernels(a) ? 0 : simplicial_generic_bwd_workspace_bytes(*a);
@@ -202,7 +201,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
   if (rc != MF_OK) return rc;
   const size_t need = mf_simplicial_fwd_workspace_bytes(a);
   const bool scratch = a->workspace && a->workspace_bytes >= need;
-  if (need > 0 && !scratch && !uses_tri_kernels(a)) {
+  if (need > 0 && !scratch && !uses_small_kernels(a) && !uses_tri_kernels(a)) {
     set_error("mf_simplicial_fwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
@@ -227,7 +226,7 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
   const bool tc = wants_tcgen05(a, &rc, "mf_simplicial_bwd");
   if (rc != MF_OK) return rc;
   const size_t need = mf_simplicial_bwd_workspace_bytes(a);
-  if (need > 0 && (!a->workspace || a->workspace_bytes < need)) {
+  if (need > 0 && (!a->workspace || a->workspace_bytes < need) && !(tc && uses_small_kernels(a))) {
     set_error("mf_simplicial_bwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }

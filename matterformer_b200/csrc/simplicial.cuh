@@ -30,6 +30,10 @@ constexpr int kSmallTokens = 32;
 int simplicial_small_fwd(const MfSimplicialFwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
 int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream);
 int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);  // with the low-rank residuals
+// Workspace with which a call of them takes heavy molecules first (0 where that does not pay), and the list; all of it is optional
+size_t simplicial_small_order_bytes(int batch, int heads, bool backward, bool residual);
+int simplicial_small_order(const uint8_t* key_valid, int batch, int tokens, void* workspace, size_t workspace_bytes, size_t need,
+                           const int32_t** order, cudaStream_t stream);
 
 // warp-level forward kernel for 33 to 192 tokens (simplicial_warp_fwd.cu)
 int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);

@@ -83,9 +83,13 @@ MfSimplicialBwdArgs as_bwd(const MfSimplicialPackedArgs* a) {
 
 using namespace mf;
 
-// The kernels these calls run on need no workspace; the functions stay for callers that ask.
-extern "C" size_t mf_simplicial_packed_fwd_workspace_bytes(const MfSimplicialPackedArgs*) { return 0; }
-extern "C" size_t mf_simplicial_packed_bwd_workspace_bytes(const MfSimplicialPackedArgs*) { return 0; }
+// The workspace is optional: with it a large batch starts with its heavy molecules.
+extern "C" size_t mf_simplicial_packed_fwd_workspace_bytes(const MfSimplicialPackedArgs* a) {
+  return a && a->batch > 0 && a->heads > 0 ? simplicial_small_order_bytes(a->batch, a->heads, false, false) : 0;
+}
+extern "C" size_t mf_simplicial_packed_bwd_workspace_bytes(const MfSimplicialPackedArgs* a) {
+  return a && a->batch > 0 && a->heads > 0 ? simplicial_small_order_bytes(a->batch, a->heads, true, false) : 0;
+}
 
 extern "C" int mf_simplicial_packed_fwd(const MfSimplicialPackedArgs* a, void* stream) {
   int rc = check_packed(a, "mf_simplicial_packed_fwd", false);

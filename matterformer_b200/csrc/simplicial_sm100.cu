@@ -603,9 +603,12 @@ extern "C" int mf_simplicial_fwd_noalloc(const MfSimplicialFwdArgs* args, void* 
     set_error("mf_simplicial_fwd_noalloc: internal scratch too small for batch %d", (int)a.batch);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }
-  // (kernels that keep no status word leave the one of an earlier call behind)
-  if (mf_simplicial_fwd_workspace_bytes(&a) == 0 && (e = cudaMemsetAsync(scratch, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream))) != cudaSuccess)
-    return cuda_error(e, "mf_simplicial_fwd_noalloc: cudaMemsetAsync");
+  // the kernels that can do without get none: such calls share nothing, and leave no status word behind
+  if (a.backend == MF_BACKEND_AUTO || (a.backend == MF_BACKEND_TCGEN05_TILES && a.tokens <= kSmallTokens)) {
+    a.workspace = nullptr, a.workspace_bytes = 0;
+    if ((e = cudaMemsetAsync(scratch, 0, sizeof(int32_t), static_cast<cudaStream_t>(stream))) != cudaSuccess)
+      return cuda_error(e, "mf_simplicial_fwd_noalloc: cudaMemsetAsync");
+  }
   // Same validation and launch as the allocating entry point; the status word at the start of the scratch is
   // cleared by the first kernel of every call, nothing else has to start at zero.
   return mf_simplicial_fwd(&a, stream);

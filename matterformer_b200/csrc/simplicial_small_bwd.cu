@@ -64,6 +64,7 @@ struct SmallBwdParams {
   __nv_bfloat16* dk2;
   __nv_bfloat16* dv2;
   int H, N;
+  const int32_t* order;  // heavy molecules first, or NULL
   float q_scale;
   RowLayout in, act;
 };
@@ -504,7 +505,7 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
   const bool bias = kBias && (RK == 0 || p.u != nullptr);
   constexpr int kThreads = 32 * kWarps;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int N = p.N, bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
+  const int N = p.N, h = blockIdx.x % p.H, b = p.order ? p.order[blockIdx.x / p.H] : blockIdx.x / p.H, bh = b * p.H + h;
   const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
   const uint32_t qmask = __ballot_sync(0xffffffffu, lane < N && p.query_valid[(size_t)b * N + min(lane, N - 1)] > 0);
   const int n = qmask ? 32 - __clz(kmask) : 0, nq = n ? 32 - __clz(qmask) : 0;
@@ -647,6 +648,9 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
 
 int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layouts, cudaStream_t stream) {
   SmallBwdParams p{};
+  const int rc = simplicial_small_order(a.pair_key_valid, a.batch, a.tokens, a.workspace, a.workspace_bytes,
+                                        simplicial_small_order_bytes(a.batch, a.heads, true, a.angle_left || a.message_left), &p.order, stream);
+  if (rc != MF_OK) return rc;
   p.grad_out = static_cast<const __nv_bfloat16*>(a.grad_out);
   p.q = static_cast<const __nv_bfloat16*>(a.q);
   p.k1 = static_cast<const __nv_bfloat16*>(a.k1);

@@ -37,6 +37,7 @@ struct ResFwdParams {
   float* lse;
   __nv_bfloat16* out_cast;
   int H, N;
+  const int32_t* order;  // heavy molecules first, or NULL
 };
 
 constexpr int kResWarps = 4;
@@ -54,7 +55,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
   ResFwdShared<RK>& sm = *reinterpret_cast<ResFwdShared<RK>*>(smem);
   constexpr int kThreads = 32 * kResWarps, MT = 2, NT = 4;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = lane & 3, row8 = lane >> 2;
-  const int N = p.N, bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
+  const int N = p.N, h = blockIdx.x % p.H, b = p.order ? p.order[blockIdx.x / p.H] : blockIdx.x / p.H, bh = b * p.H + h;
   const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
   const uint32_t qmask = __ballot_sync(0xffffffffu, lane < N && p.query_valid[(size_t)b * N + min(lane, N - 1)] > 0);
   const int n = 32 - __clz(kmask);
@@ -264,6 +265,9 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
 
 int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   ResFwdParams p{};
+  const int rc = simplicial_small_order(a.pair_key_valid, a.batch, a.tokens, a.workspace, a.workspace_bytes,
+                                        simplicial_small_order_bytes(a.batch, a.heads, false, true), &p.order, stream);
+  if (rc != MF_OK) return rc;
   p.q = static_cast<const __nv_bfloat16*>(a.q);
   p.k1 = static_cast<const __nv_bfloat16*>(a.k1);
   p.v1 = static_cast<const __nv_bfloat16*>(a.v1);

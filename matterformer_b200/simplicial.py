@@ -76,6 +76,11 @@ def _remember_status(ws: Optional[torch.Tensor]) -> None:
                                "the outputs of this call are zeros")  # fmt: skip
 
 
+def _keeps_status(a) -> bool:
+    """Whether the call's workspace starts with a status word: the kernels of at most 32 tokens have no device-side waits."""
+    return a.tokens > 32 or a.backend == _lib.MF_BACKEND["tcgen05"]
+
+
 def device_status() -> int:
     """Status word the most recent tensor-core simplicial kernel left in its workspace.
 
@@ -242,7 +247,7 @@ def cuda_simplicial_attention_forward(
     _lib.launch(L.mf_simplicial_fwd, q.device, ref)
     # only the tensor-core kernels keep a status word in their workspace
     if L.mf_simplicial_fwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
-        _remember_status(ws)
+        _remember_status(ws if _keeps_status(a) else None)
     return out, lse, out32
 
 
@@ -352,7 +357,7 @@ def cuda_simplicial_attention_backward(
     _lib.launch(L.mf_simplicial_bwd, q.device, ref)
     # only the tensor-core kernels keep a status word in their workspace
     if L.mf_simplicial_bwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
-        _remember_status(ws)
+        _remember_status(ws if _keeps_status(a) else None)
     if bias is not None:  # the reference returns each bias gradient in the dtype of its operand (:1155-1160)
         bias_grads = [g.to(t.dtype) if g is not None else None for g, t in zip(bias_grads, (u, v_bias, w, gate))]
     if angle is not None:
@@ -447,6 +452,14 @@ class CudaTwoSimplicialAttentionFunction(torch.autograd.Function):
 
 
 
+def _packed_workspace(size, a, like):
+    need = size(ctypes.byref(a))
+    ws = torch.empty(need, device=like.device, dtype=torch.uint8) if need else None
+    if ws is not None:
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    return ws
+
+
 def packed_projection_applies(proj: torch.Tensor, heads: int, head_dim: int) -> bool:
     """Whether :func:`simplicial_attention_packed` serves this projection: CUDA bf16 (B, N, 5*H*64) with at most 32
     tokens."""
@@ -470,6 +483,7 @@ class _PackedSimplicialAttention(torch.autograd.Function):
                                         proj=proj.data_ptr(), query_valid=qv.data_ptr(), pair_key_valid=kv.data_ptr(),
                                         pair_valid=pv.data_ptr() if pv is not None else None, out32=out32.data_ptr(),
                                         lse=lse.data_ptr(), out=out.data_ptr())  # fmt: skip
+        ws = _packed_workspace(_lib.lib().mf_simplicial_packed_fwd_workspace_bytes, a, proj)  # noqa: F841 (kept until the launch)
         _lib.launch(_lib.lib().mf_simplicial_packed_fwd, proj.device, ctypes.byref(a))
         _remember_status(None)
         ctx.save_for_backward(proj, qv, kv, pv, out32, lse)
@@ -489,6 +503,7 @@ class _PackedSimplicialAttention(torch.autograd.Function):
                                         pair_valid=pv.data_ptr() if pv is not None else None, out32=out32.data_ptr(),
                                         lse=lse.data_ptr(), grad_out=grad_out.data_ptr(),
                                         grad_proj=grad_proj.data_ptr())  # fmt: skip
+        ws = _packed_workspace(_lib.lib().mf_simplicial_packed_bwd_workspace_bytes, a, proj)  # noqa: F841
         _lib.launch(_lib.lib().mf_simplicial_packed_bwd, proj.device, ctypes.byref(a))
         _remember_status(None)
         return grad_proj, None, None, None, None, None

@@ -1,0 +1,59 @@
+"""Heavy-first order of the kernels of at most 32 tokens: the results are those of the order given, bit for bit."""
+import ctypes
+
+import pytest
+import torch
+
+from matterformer_b200 import _lib
+from matterformer_b200.simplicial import cuda_simplicial_attention_backward, cuda_simplicial_attention_forward, simplicial_attention_packed
+
+pytestmark = pytest.mark.gpu
+
+
+def _without(monkeypatch):
+    for name in ("fwd", "bwd"):
+        monkeypatch.setattr(_lib.lib(), f"mf_simplicial_{name}_workspace_bytes", lambda ref: 0)
+        monkeypatch.setattr(_lib.lib(), f"mf_simplicial_packed_{name}_workspace_bytes", lambda ref: 0)
+
+
+@pytest.mark.parametrize("B,H,N,rank", [(1025, 4, 7, 0), (600, 8, 32, 0), (129, 4, 20, 8)])
+def test_same_bits_in_either_order(monkeypatch, B, H, N, rank):
+    """Empty molecules, ties, batches beyond the order kernel's block; with the factorized bias and the residuals."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    heads = [randn(B, H, N, 64).bfloat16() for _ in range(5)]
+    go = randn(B, H, N, 64).bfloat16()
+    n = torch.randint(0, N + 1, (B,), generator=g, device="cuda")
+    valid = torch.arange(N, device="cuda")[None] < n[:, None]
+    kw = dict(query_valid=valid, pair_key_valid=valid, pair_valid=None, u=randn(B, H, N, N), v_bias=randn(B, H, N, N), w=randn(B, H, N, N),
+              gate=randn(B, H, N))  # fmt: skip
+    if rank:
+        kw.update(angle_left=randn(B, H, N, N, rank), angle_right=randn(B, H, N, N, rank), angle_gate=randn(B, H, N))
+
+    def run():
+        out, lse, out32 = cuda_simplicial_attention_forward(*heads, **kw)
+        grads = cuda_simplicial_attention_backward(go, *heads, out32, lse, **kw, need_du=True, need_dv_bias=True, need_dw=True, need_dgate=True)
+        return [out, lse, *(t for t in grads if t is not None)]
+
+    a = _lib.MfSimplicialBwdArgs(batch=B, heads=H, tokens=N, head_dim=64, dtype=1, angle_left=go.data_ptr() if rank else None)
+    args = {f: go.data_ptr() for f in ("q", "k1", "v1", "k2", "v2", "grad_out", "out", "dq", "dk1", "dv1", "dk2", "dv2")}
+    for f, v in args.items():
+        setattr(a, f, v)
+    assert _lib.lib().mf_simplicial_bwd_workspace_bytes(ctypes.byref(a)) > 0  # the order is used
+    ordered = run()
+    _without(monkeypatch)
+    assert all(torch.equal(x, y) for x, y in zip(ordered, run()))
+
+
+def test_packed_projection_in_either_order(monkeypatch):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    proj = torch.randn(600, 23, 5 * 8 * 64, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    valid = torch.arange(23, device="cuda")[None] < torch.randint(1, 24, (600,), generator=g, device="cuda")[:, None]
+
+    def run():
+        out = simplicial_attention_packed(proj, heads=8, query_valid=valid, pair_key_valid=valid)
+        return [out, *torch.autograd.grad(out, [proj], torch.ones_like(out))]
+
+    ordered = run()
+    _without(monkeypatch)
+    assert all(torch.equal(x, y) for x, y in zip(ordered, run()))
