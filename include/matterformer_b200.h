@@ -115,9 +115,9 @@ typedef struct MfSimplicialFwdArgs {
   float* out;     /* (B,H,N,D) fp32, written for every row (zeros where invalid) */
   float* lse;     /* (B,H,N)   fp32 natural-log sum of exp over visible pairs */
   void* out_cast; /* optional (B,H,N,D) copy of out in `dtype`; may be NULL */
-  /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0.  Tensor-core calls of at most 32 tokens
-   * are served without it too (with it, large batches start with their heavy molecules), and with the factorized bias above 32
-   * tokens (by a kernel that needs none and takes about twice as long). */
+  /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0.  Calls of the default backend are
+   * served without it too: with it, large batches start with their heavy molecules, and with the factorized bias above 32 tokens
+   * the kernel that needs none takes about twice as long. */
   void* workspace;
   size_t workspace_bytes;
 } MfSimplicialFwdArgs;
@@ -191,7 +191,8 @@ size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* args);
 
 /* Whether a call with these arguments runs on tensor-core kernels (MF_BACKEND_TCGEN05, also where these are the warp-level
  * mma.sync ones) or on CUDA cores (MF_BACKEND_GENERIC).  (No counterpart in the reference.)  Tensor-core kernels that take a
- * workspace leave a status word at its start. */
+ * workspace leave a status word at its start, except the warp-level ones: at most 32 tokens, or a forward call without the bias on
+ * the default backend (they have no device-side waits). */
 int mf_simplicial_fwd_backend(const MfSimplicialFwdArgs* args);
 int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* args);
 /* The gradient of message_basis from MfSimplicialBwdArgs.message_coeff: out[h,r,:] = sum_{b,i} coeff[b,h,i,r] grad_out[b,h,i,:]

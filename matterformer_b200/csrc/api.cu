@@ -148,7 +148,8 @@ extern "C" size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* a
   int rc;
   if (!wants_tcgen05(a, &rc, "mf_simplicial_fwd")) return 0;
   if (uses_small_kernels(a)) return simplicial_small_order_bytes(a->batch, a->heads, false, a->angle_left || a->message_left);
-  return uses_tri_kernels(a) ? simplicial_tri_fwd_workspace_bytes(*a) : uses_warp_forward(a) ? 0 : simplicial_sm100_fwd_workspace_bytes(*a);
+  return uses_tri_kernels(a) ? simplicial_tri_fwd_workspace_bytes(*a) : uses_warp_forward(a) ? simplicial_warp_order_bytes(a->batch, a->heads, a->tokens)
+                                                                           : simplicial_sm100_fwd_workspace_bytes(*a);
 }
 
 extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a) {
@@ -201,7 +202,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
   if (rc != MF_OK) return rc;
   const size_t need = mf_simplicial_fwd_workspace_bytes(a);
   const bool scratch = a->workspace && a->workspace_bytes >= need;
-  if (need > 0 && !scratch && !uses_small_kernels(a) && !uses_tri_kernels(a)) {
+  if (need > 0 && !scratch && !uses_small_kernels(a) && !uses_warp_forward(a)) {
     set_error("mf_simplicial_fwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
   }

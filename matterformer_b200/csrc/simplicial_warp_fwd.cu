@@ -34,6 +34,7 @@ struct WarpFwdParams {
   float* out;
   float* lse;
   __nv_bfloat16* out_cast;
+  const int32_t* order;  // heavy molecules first, or NULL
   int H, N, chunk;  // chunk: queries per CTA
   int even;         // rows of v_bias and w start on 8-byte boundaries
 };
@@ -221,7 +222,7 @@ template <bool kBias>
 __global__ void __launch_bounds__(kFwdThreads, 1) simplicial_warp_fwd_kernel(const __grid_constant__ WarpFwdParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = lane & 3, row8 = lane >> 2;
-  const int N = p.N, bh = blockIdx.y, b = bh / p.H;
+  const int N = p.N, b = p.order ? p.order[blockIdx.y / p.H] : blockIdx.y / p.H, bh = b * p.H + blockIdx.y % p.H;
   WarpFwdHeader& hd = *reinterpret_cast<WarpFwdHeader*>(smem);
   constexpr int kHeader = (sizeof(WarpFwdHeader) + 127) / 128 * 128;
   const uint32_t tile0 = (uint32_t)__cvta_generic_to_shared(smem) + kHeader;
@@ -320,10 +321,81 @@ __global__ void __launch_bounds__(kFwdThreads, 1) simplicial_warp_fwd_kernel(con
   }
 }
 
+// Molecules by the index of their last key, the largest first (the order decides when a molecule runs, not what it computes).
+constexpr int kMostOrdered = 1024;
+__global__ void __launch_bounds__(1024) simplicial_warp_order_kernel(const uint8_t* __restrict__ key_valid, int B, int N, int32_t* order) {
+  __shared__ int last[kMostOrdered], start[kMaxKeys + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, words = (N + 31) >> 5;
+  if (tid < B) last[tid] = 0;
+  if (tid <= kMaxKeys) start[tid] = 0;
+  __syncthreads();
+  constexpr int kAtOnce = 8;  // mask words of a warp that are on their way together
+  for (int i0 = kAtOnce * warp; i0 < B * words; i0 += 32 * kAtOnce) {
+    uint8_t v[kAtOnce];
+#pragma unroll
+    for (int t = 0; t < kAtOnce; ++t) {
+      const int i = min(i0 + t, B * words - 1), b = i / words, k = 32 * (i - b * words) + lane;
+      v[t] = k < N ? __ldg(key_valid + (size_t)b * N + k) : 0;
+    }
+#pragma unroll
+    for (int t = 0; t < kAtOnce; ++t) {
+      const uint32_t m = __ballot_sync(0xffffffffu, v[t] > 0);
+      const int i = min(i0 + t, B * words - 1), b = i / words;
+      if (lane == 0 && m) atomicMax(&last[b], 32 * (i - b * words) + 32 - __clz(m));
+    }
+  }
+  __syncthreads();
+  const int mine = tid < B ? kMaxKeys - last[tid] : 0;
+  if (tid < B) atomicAdd(&start[mine], 1);
+  __syncthreads();
+  if (warp == 0) {  // exclusive sums
+    int before = 0;
+    for (int c = 0; c <= kMaxKeys; c += 32) {
+      const int n = c + lane <= kMaxKeys ? start[c + lane] : 0;
+      int sum = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += x;
+      }
+      if (c + lane <= kMaxKeys) start[c + lane] = before + sum - n;
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+  }
+  __syncthreads();
+  if (tid < B) order[atomicAdd(&start[mine], 1)] = tid;
+}
+
+// Queries per CTA: see simplicial_warp_fwd
+int queries_per_cta(int bh, int tokens) {
+  int chunk = tokens >= 128 ? 24 : tokens > 64 ? 48 : 96;
+  while (chunk > 12 && (long long)bh * ((tokens + chunk - 1) / chunk) < 296) chunk >>= 1;
+  return chunk;
+}
+
 }  // namespace
+
+// Workspace of the list above, which a caller may leave out.  A CTA runs with the square of its molecule's size, so in the order
+// given a launch ends with a few large ones: 8 heads, 20-181 atoms, 64 molecules 893 | 851 us heavy first, 24-192 8 molecules 181 |
+// 140, 20-100 32 134 | 107, 20-160 4 76 | 64, 20-64 64 103 | 85, 10-48 64 60 | 48.  The list takes a launch of 3 us (and nothing is
+// gained where all molecules are of one size), so it is made from a wave and a half of CTAs and about 50 us on.
+size_t simplicial_warp_order_bytes(int batch, int heads, int tokens) {
+  const long long bh = (long long)batch * heads;
+  const int chunk = queries_per_cta((int)bh, tokens);
+  const bool pays = batch > 1 && batch <= kMostOrdered && bh * ((tokens + chunk - 1) / chunk) >= 222 &&
+                    bh * tokens * tokens * tokens >= 30000000ll;
+  return pays ? align_up((size_t)batch * sizeof(int32_t), 256) : 0;
+}
 
 int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   WarpFwdParams p{};
+  const size_t need = a.u ? 0 : simplicial_warp_order_bytes(a.batch, a.heads, a.tokens);
+  if (need > 0 && a.workspace && a.workspace_bytes >= need) {
+    int32_t* order = static_cast<int32_t*>(a.workspace);
+    simplicial_warp_order_kernel<<<1, 1024, 0, stream>>>(a.pair_key_valid, a.batch, a.tokens, order);
+    MF_CHECK_LAUNCH("simplicial_warp_order_kernel");
+    p.order = order;
+  }
   p.q = static_cast<const __nv_bfloat16*>(a.q);
   p.k1 = static_cast<const __nv_bfloat16*>(a.k1);
   p.v1 = static_cast<const __nv_bfloat16*>(a.v1);
@@ -340,8 +412,7 @@ int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   // 128 401 | 384 | 410, 192 1 004 | 977 | 1 035; with the bias 176 | 173 | 166, 387 | 382 | 401, 833 | 831 | 891, 773 | 775 |
   // 839, 2 076 | 2 131 | 2 296.  Halved below two CTAs per SM: 2 molecules of up to 192 tokens, 12 | 24 | 48: 62 | 101 | 183 us.
   const int bh = a.batch * a.heads;
-  int chunk = a.tokens >= 128 ? 24 : a.tokens > 64 ? 48 : 96;
-  while (chunk > 12 && (long long)bh * ((a.tokens + chunk - 1) / chunk) < 296) chunk >>= 1;
+  const int chunk = queries_per_cta(bh, a.tokens);
   p.chunk = chunk;
   const int rows = (a.tokens + 31) & ~31, bytes = (int)((sizeof(WarpFwdHeader) + 127) / 128 * 128) + 4 * rows * kRowBytes;
   auto kernel = a.u ? simplicial_warp_fwd_kernel<true> : simplicial_warp_fwd_kernel<false>;

@@ -79,9 +79,12 @@ void fill_common(Args& a, const std::array<Tensor, kInputs>& t, int precision, i
   a.angle_rank = t[AL].defined() ? t[AL].size(4) : 0, a.message_rank = t[ML].defined() ? t[ML].size(4) : 0;
 }
 
-// Whether the workspace starts with a status word: the warp-level kernels of at most 32 tokens have no device-side waits
-template <typename Args>
-bool keeps_status(const Args& a) { return a.tokens > 32 || a.backend == MF_BACKEND_TCGEN05; }
+// Whether the workspace starts with a status word: the warp-level kernels (at most 32 tokens; forward without the bias) have no
+// device-side waits
+bool keeps_status(const MfSimplicialBwdArgs& a) { return a.tokens > 32 || a.backend == MF_BACKEND_TCGEN05; }
+bool keeps_status(const MfSimplicialFwdArgs& a) {
+  return a.backend == MF_BACKEND_TCGEN05 || (a.tokens > 32 && (a.u || a.backend != MF_BACKEND_AUTO));
+}
 
 struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
   static Variable forward(AutogradContext* ctx, const Tensor& q, const Tensor& k1, const Tensor& v1, const Tensor& k2,

@@ -77,8 +77,11 @@ def _remember_status(ws: Optional[torch.Tensor]) -> None:
 
 
 def _keeps_status(a) -> bool:
-    """Whether the call's workspace starts with a status word: the kernels of at most 32 tokens have no device-side waits."""
-    return a.tokens > 32 or a.backend == _lib.MF_BACKEND["tcgen05"]
+    """Whether the call's workspace starts with a status word: the warp-level kernels (at most 32 tokens; forward without the
+    bias) have no device-side waits."""
+    if a.backend == _lib.MF_BACKEND["tcgen05"] or a.tokens <= 32:
+        return a.backend == _lib.MF_BACKEND["tcgen05"]
+    return isinstance(a, _lib.MfSimplicialBwdArgs) or bool(a.u) or a.backend != _lib.MF_BACKEND["auto"]
 
 
 def device_status() -> int:

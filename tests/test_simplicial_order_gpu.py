@@ -57,3 +57,18 @@ def test_packed_projection_in_either_order(monkeypatch):
     ordered = run()
     _without(monkeypatch)
     assert all(torch.equal(x, y) for x, y in zip(ordered, run()))
+
+
+@pytest.mark.parametrize("B,H,N", [(1024, 2, 33), (40, 8, 64), (9, 8, 131), (8, 8, 192)])
+def test_forward_above_32_tokens_in_either_order(monkeypatch, B, H, N):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    heads = [torch.randn(B, H, N, 64, generator=g, device="cuda").bfloat16() for _ in range(5)]
+    valid = torch.arange(N, device="cuda")[None] < torch.randint(0, N + 1, (B,), generator=g, device="cuda")[:, None]
+    kw = dict(query_valid=valid, pair_key_valid=valid, pair_valid=None)
+    a = _lib.MfSimplicialFwdArgs(batch=B, heads=H, tokens=N, head_dim=64, dtype=1)
+    for f in ("q", "k1", "v1", "k2", "v2", "out"):
+        setattr(a, f, heads[0].data_ptr())
+    assert _lib.lib().mf_simplicial_fwd_workspace_bytes(ctypes.byref(a)) > 0  # the order is used
+    ordered = cuda_simplicial_attention_forward(*heads, **kw)
+    _without(monkeypatch)
+    assert all(torch.equal(x, y) for x, y in zip(ordered, cuda_simplicial_attention_forward(*heads, **kw)))
