@@ -16,8 +16,8 @@
 //
 // Rows are packed as in simplicial_rows.cuh: `groups` consecutive y per step.  Columns go in chunks of at most 64; chunk q
 // belongs to softmax group q & 1, so one group's exponentials run under the other group's products.  The softmax warps do
-// nothing else; the row warps write A and add up T and R (one kind of warp for both, with one chain of waits, took twice as
-// long).  One thread issues every MMA, two warps stage the bias operands of coming steps.  Waits are bounded.
+// nothing else; the row warps write A and add up T and R (one kind of warp for both, with one chain of waits, took 1.4 times
+// as long).  One thread issues every MMA, two warps stage the bias operands of coming steps.  Waits are bounded.
 //
 // The softmax takes shift 0; a tile in which a row's sum leaves 2^-60 .. 2^60 is done again with its exact maxima.
 //
@@ -325,131 +325,131 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
   auto next_mode = [&](bool again) { return __syncthreads_or(again) != 0; };
 
   if (warp >= kIssuerWarp) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<kForward>::kAux));
-  for (int mode = 0; mode < kModes; ++mode) {
-    const int s_first = mode * steps;
-    if (warp == kIssuerWarp) {
-      if (elect_one()) {
-        // ------------------------------------------------------------------ issuer
-        const uint32_t lz = make_desc_lo(smem_u32(smem + kOffZ), 0), lz2 = make_desc_lo(smem_u32(smem + kOffZ2), 0);
-        constexpr uint32_t mn = (kMaxKeys * 128 >> 4) << 16;  // LBO of the MN-major view
-        constexpr uint32_t idesc_t = make_idesc_bf16(kTileM, kD, false, true);
-        const uint32_t idesc_s = make_idesc_bf16(kTileM, 16 * per, false, false);
-        constexpr uint32_t idesc_more = 16u >> 3 << 17;  // 16 columns more
-        const int total = steps * C;
-        // Two streams of chunks, the logits ahead of the sums: step, chunk of the step, its first unit, buffer
-        struct Stream {
-          int S, c, u, buf;
-        };
-        Stream lg{s_first, 0, 0, (int)(mode * total % kBufs)}, sm = lg;
-        uint32_t ph_p = (mode * total / kBufs) & 1;  // phase of bar_p for the buffer sm.buf (flips when the ring wraps)
-        auto advance = [&](Stream& t, int nu) {
-          t.u += nu;
-          if (++t.buf == kBufs) t.buf = 0;
-          if (++t.c == C) t.c = 0, t.u = 0, ++t.S;
-        };
-        auto next_logits = [&]() {
-          if (lg.c == 0) {
-            wait_on(&sh.bar_a[lg.S & 1], lg.S >> 1);
-            tc_fence_after_sync();
-          }
-          const int more = lg.c < extra;
-          const uint32_t idesc = idesc_s + (more ? idesc_more : 0u);
-          const uint32_t a = tmem + (lg.S & 1) * kACols, d = tmem + kColS + lg.buf * kBufCols, z = lg.u * 128;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<kForward>::kAux));
+    for (int mode = 0; mode < kModes; ++mode) {
+      const int s_first = mode * steps;
+      if (warp == kIssuerWarp) {
+        if (elect_one()) {
+          // ------------------------------------------------------------------ issuer
+          const uint32_t lz = make_desc_lo(smem_u32(smem + kOffZ), 0), lz2 = make_desc_lo(smem_u32(smem + kOffZ2), 0);
+          constexpr uint32_t mn = (kMaxKeys * 128 >> 4) << 16;  // LBO of the MN-major view
+          constexpr uint32_t idesc_t = make_idesc_bf16(kTileM, kD, false, true);
+          const uint32_t idesc_s = make_idesc_bf16(kTileM, 16 * per, false, false);
+          constexpr uint32_t idesc_more = 16u >> 3 << 17;  // 16 columns more
+          const int total = steps * C;
+          // Two streams of chunks, the logits ahead of the sums: step, chunk of the step, its first unit, buffer
+          struct Stream {
+            int S, c, u, buf;
+          };
+          Stream lg{s_first, 0, 0, (int)(mode * total % kBufs)}, sm = lg;
+          uint32_t ph_p = (mode * total / kBufs) & 1;  // phase of bar_p for the buffer sm.buf (flips when the ring wraps)
+          auto advance = [&](Stream& t, int nu) {
+            t.u += nu;
+            if (++t.buf == kBufs) t.buf = 0;
+            if (++t.c == C) t.c = 0, t.u = 0, ++t.S;
+          };
+          auto next_logits = [&]() {
+            if (lg.c == 0) {
+              wait_on(&sh.bar_a[lg.S & 1], lg.S >> 1);
+              tc_fence_after_sync();
+            }
+            const int more = lg.c < extra;
+            const uint32_t idesc = idesc_s + (more ? idesc_more : 0u);
+            const uint32_t a = tmem + (lg.S & 1) * kACols, d = tmem + kColS + lg.buf * kBufCols, z = lg.u * 128;
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) umma_ts_lo(d, a + 8 * ks, lz + z + 2 * ks, idesc, ks > 0);
-          if constexpr (!kForward) {
+            for (int ks = 0; ks < 4; ++ks) umma_ts_lo(d, a + 8 * ks, lz + z + 2 * ks, idesc, ks > 0);
+            if constexpr (!kForward) {
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) umma_ts_lo(d + 64, a + 32 + 8 * ks, lz2 + z + 2 * ks, idesc, ks > 0);
-          }
-          umma_commit(&sh.bar_s[lg.buf]);
-          if (lg.c == C - 1) umma_commit(&sh.bar_free[lg.S & 1]);
-          advance(lg, per + more);
-        };
-        // A of step s is built once the row warps have read T of step s - 3: with one chunk a step, three chunks ahead is the limit
-        const int ahead = C == 1 ? min(kBufs, 3) : kBufs;
-        for (int q = 0; q < min(ahead, total); ++q) next_logits();
+              for (int ks = 0; ks < 4; ++ks) umma_ts_lo(d + 64, a + 32 + 8 * ks, lz2 + z + 2 * ks, idesc, ks > 0);
+            }
+            umma_commit(&sh.bar_s[lg.buf]);
+            if (lg.c == C - 1) umma_commit(&sh.bar_free[lg.S & 1]);
+            advance(lg, per + more);
+          };
+          // A of step s is built once the row warps have read T of step s - 3: with one chunk a step, three chunks ahead is the limit
+          const int ahead = C == 1 ? min(kBufs, 3) : kBufs;
+          for (int q = 0; q < min(ahead, total); ++q) next_logits();
 #pragma unroll 1
-        for (int q = 0; q < total; ++q) {
-          wait_on(&sh.bar_p[sm.buf], ph_p);
-          if (sm.c == 0 && sm.S >= kSumBufs) wait_on(&sh.bar_d[(sm.S - kSumBufs) & 1], (sm.S - kSumBufs) >> 1);  // the buffer's last sums have been read
-          tc_fence_after_sync();
-          const int nu = per + (sm.c < extra);
-          const uint32_t a = tmem + kColS + sm.buf * kBufCols, z = sm.u * 128, t = tmem + kColT + (kSumBufs == 2 ? 64 * (sm.S & 1) : 0);
-          const bool more = sm.c > 0;
-#pragma unroll
-          for (int kg = 0; kg < 4; ++kg)
-            if (kg < nu) umma_ts_lo(t, a + (kForward ? 0 : 64) + 8 * kg, ((kForward ? lz2 : lz) | mn) + z + 128 * kg, idesc_t, more || kg > 0);
-          if constexpr (kPass == kDk1 || kPass == kDk2) {
+          for (int q = 0; q < total; ++q) {
+            wait_on(&sh.bar_p[sm.buf], ph_p);
+            if (sm.c == 0 && sm.S >= kSumBufs) wait_on(&sh.bar_d[(sm.S - kSumBufs) & 1], (sm.S - kSumBufs) >> 1);  // the buffer's last sums have been read
+            tc_fence_after_sync();
+            const int nu = per + (sm.c < extra);
+            const uint32_t a = tmem + kColS + sm.buf * kBufCols, z = sm.u * 128, t = tmem + kColT + (kSumBufs == 2 ? 64 * (sm.S & 1) : 0);
+            const bool more = sm.c > 0;
 #pragma unroll
             for (int kg = 0; kg < 4; ++kg)
-              if (kg < nu) umma_ts_lo(tmem + kColR, a + 8 * kg, (lz2 | mn) + z + 128 * kg, idesc_t, more || kg > 0);
-          }
-          if (sm.c == C - 1) umma_commit(&sh.bar_t[sm.S & 1]);
-          if (sm.buf == kBufs - 1) ph_p ^= 1;
-          advance(sm, nu);
-          if (q + ahead < total) next_logits();
-        }
-      }
-      __syncwarp();
-    } else if (warp == kBiasLoader) {
-      // ------------------------------------------------------------------ bias operand of (y, z): w_jk, v_ik, u_ij by pass
-      const float* src = X == 0 ? p.w : X == 1 ? p.v_bias : p.u;
-      const bool vec = X != 1 && !holes && (N & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;  // four columns at a time
-      src += nn;
-      uint32_t in = 0;  // bit t: column lane + 32 t counts
+              if (kg < nu) umma_ts_lo(t, a + (kForward ? 0 : 64) + 8 * kg, ((kForward ? lz2 : lz) | mn) + z + 128 * kg, idesc_t, more || kg > 0);
+            if constexpr (kPass == kDk1 || kPass == kDk2) {
 #pragma unroll
-      for (int t = 0; t < kWords; ++t) {
-        const int z = lane + 32 * t;
-        if (z < nz && valid(Z, z)) in |= 1u << t;
-      }
-      for (int s = 0; s < steps; ++s) {
-        const int S = s_first + s, st = S & (kStages - 1);
-        if (S >= kStages) wait_on(&sh.bar_empty[st], S / kStages - 1);
-        for (int gg = 0; gg < G; ++gg) {
-          const int yy = s * G + gg, y = yy < ny ? sh.ylist[yy] : 0;
-          float* dst = bcol + (st * G + gg) * zpad;
-          if (vec) {
-            for (int z = 4 * lane; z < zpad; z += 128)
-              cp_async16_part(smem_u32(dst + z), src + (size_t)y * N + min(z, nz & ~3), yy < ny ? 4 * min(max(nz - z, 0), 4) : 0);
-          } else {
-            const float* at = src + (X == 1 ? (size_t)lane * N + y : (size_t)y * N + lane);
-            const size_t step = X == 1 ? (size_t)32 * N : 32;
-#pragma unroll
-            for (int t = 0; t < kWords; ++t, at += step)
-              if (lane + 32 * t < zpad) {
-                const bool ok = yy < ny && ((in >> t) & 1u);
-                cp_async_f32(dst + lane + 32 * t, ok ? at : src, ok);
-              }
+              for (int kg = 0; kg < 4; ++kg)
+                if (kg < nu) umma_ts_lo(tmem + kColR, a + 8 * kg, (lz2 | mn) + z + 128 * kg, idesc_t, more || kg > 0);
+            }
+            if (sm.c == C - 1) umma_commit(&sh.bar_t[sm.S & 1]);
+            if (sm.buf == kBufs - 1) ph_p ^= 1;
+            advance(sm, nu);
+            if (q + ahead < total) next_logits();
           }
         }
-        cp_async_arrive(&sh.bar_full[st]);
-      }
-    } else if (warp == kPairLoader) {
-      // ------------------------------------------------------------------ bias operand of (x, y): u_ij, w_jk, v_ik by pass
-      const float* src = X == 0 ? p.u : X == 1 ? p.w : p.v_bias;
-      int rg[4], rx[4];
+        __syncwarp();
+      } else if (warp == kBiasLoader) {
+        // ------------------------------------------------------------------ bias operand of (y, z): w_jk, v_ik, u_ij by pass
+        const float* src = X == 0 ? p.w : X == 1 ? p.v_bias : p.u;
+        const bool vec = X != 1 && !holes && (N & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;  // four columns at a time
+        src += nn;
+        uint32_t in = 0;  // bit t: column lane + 32 t counts
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int row = lane + 32 * t;
-        rg[t] = row / rt, rx[t] = x0 + row - rg[t] * rt;
-        if (rg[t] >= G || rx[t] >= nx || !valid(X, rx[t])) rg[t] = 1 << 20;  // no pair
-      }
-      for (int s = 0; s < steps; ++s) {
-        const int S = s_first + s, st = S & (kStages - 1);
-        if (S >= kStages) wait_on(&sh.bar_empty[st], S / kStages - 1);
+        for (int t = 0; t < kWords; ++t) {
+          const int z = lane + 32 * t;
+          if (z < nz && valid(Z, z)) in |= 1u << t;
+        }
+        for (int s = 0; s < steps; ++s) {
+          const int S = s_first + s, st = S & (kStages - 1);
+          if (S >= kStages) wait_on(&sh.bar_empty[st], S / kStages - 1);
+          for (int gg = 0; gg < G; ++gg) {
+            const int yy = s * G + gg, y = yy < ny ? sh.ylist[yy] : 0;
+            float* dst = bcol + (st * G + gg) * zpad;
+            if (vec) {
+              for (int z = 4 * lane; z < zpad; z += 128)
+                cp_async16_part(smem_u32(dst + z), src + (size_t)y * N + min(z, (nz - 1) & ~3), yy < ny ? 4 * min(max(nz - z, 0), 4) : 0);
+            } else {
+              const float* at = src + (X == 1 ? (size_t)lane * N + y : (size_t)y * N + lane);
+              const size_t step = X == 1 ? (size_t)32 * N : 32;
+#pragma unroll
+              for (int t = 0; t < kWords; ++t, at += step)
+                if (lane + 32 * t < zpad) {
+                  const bool ok = yy < ny && ((in >> t) & 1u);
+                  cp_async_f32(dst + lane + 32 * t, ok ? at : src, ok);
+                }
+            }
+          }
+          cp_async_arrive(&sh.bar_full[st]);
+        }
+      } else if (warp == kPairLoader) {
+        // ------------------------------------------------------------------ bias operand of (x, y): u_ij, w_jk, v_ik by pass
+        const float* src = X == 0 ? p.u : X == 1 ? p.w : p.v_bias;
+        int rg[4], rx[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const int yy = s * G + rg[t];
-          const bool ok = yy < ny;
-          const int y = ok ? sh.ylist[yy] : 0;
-          cp_async_f32(bpair + st * kTileM + lane + 32 * t, ok ? src + nn + (X == 2 ? (size_t)y * N + rx[t] : (size_t)rx[t] * N + y) : src, ok);
+          const int row = lane + 32 * t;
+          rg[t] = row / rt, rx[t] = x0 + row - rg[t] * rt;
+          if (rg[t] >= G || rx[t] >= nx || !valid(X, rx[t])) rg[t] = 1 << 20;  // no pair
         }
-        cp_async_arrive(&sh.bar_full[st]);
+        for (int s = 0; s < steps; ++s) {
+          const int S = s_first + s, st = S & (kStages - 1);
+          if (S >= kStages) wait_on(&sh.bar_empty[st], S / kStages - 1);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const int yy = s * G + rg[t];
+            const bool ok = yy < ny;
+            const int y = ok ? sh.ylist[yy] : 0;
+            cp_async_f32(bpair + st * kTileM + lane + 32 * t, ok ? src + nn + (X == 2 ? (size_t)y * N + rx[t] : (size_t)rx[t] * N + y) : src, ok);
+          }
+          cp_async_arrive(&sh.bar_full[st]);
+        }
       }
+      if (kForward && !next_mode(false)) break;
     }
-    if (kForward && !next_mode(false)) break;
-  }
   } else {
     const int r = tid & 127, grp = (tid >> 7) & 1;  // tile row, group
     const int g = r / rt, ii = r - g * rt, x = x0 + ii, gs = g < G ? g : 0;
@@ -479,160 +479,160 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
         }
       }
       for (int mode = 0; mode < kModes; ++mode) {
-      const int s_first = mode * steps;
-      float l_run = 0.f;
-      float lse = 0.f, delta = 0.f, gate = 0.f, rs = 0.f;
-      float2 rsum = make_float2(0.f, 0.f);
-      bool ok = false, seen = false;
-      const uint32_t* vis = sh.mask[1];
-      const float* colp = bcol;
-      // One unit of 16 columns: P and dS from S and dP
-      auto unit = [&](uint32_t buf, int z, uint32_t (&sv)[16], const uint32_t (&dv)[16]) {
-        float2 t[8];
+        const int s_first = mode * steps;
+        float l_run = 0.f;
+        float lse = 0.f, delta = 0.f, gate = 0.f, rs = 0.f;
+        float2 rsum = make_float2(0.f, 0.f);
+        bool ok = false, seen = false;
+        const uint32_t* vis = sh.mask[1];
+        const float* colp = bcol;
+        // One unit of 16 columns: P and dS from S and dP
+        auto unit = [&](uint32_t buf, int z, uint32_t (&sv)[16], const uint32_t (&dv)[16]) {
+          float2 t[8];
 #pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4) {
-          const float4 xz = btile[((z >> 2) + e4) * pitch + ii], yz = *reinterpret_cast<const float4*>(colp + z + 4 * e4);
-          float4 gz = make_float4(gate, gate, gate, gate);
-          if constexpr (Z == 0) gz = *reinterpret_cast<const float4*>(cols + 2 * kMaxKeys + z + 4 * e4);
-          const float2 xy = make_float2(rs, rs);
+          for (int e4 = 0; e4 < 4; ++e4) {
+            const float4 xz = btile[((z >> 2) + e4) * pitch + ii], yz = *reinterpret_cast<const float4*>(colp + z + 4 * e4);
+            float4 gz = make_float4(gate, gate, gate, gate);
+            if constexpr (Z == 0) gz = *reinterpret_cast<const float4*>(cols + 2 * kMaxKeys + z + 4 * e4);
+            const float2 xy = make_float2(rs, rs);
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const float2 a = half ? make_float2(xz.z, xz.w) : make_float2(xz.x, xz.y);
-            const float2 c = half ? make_float2(yz.z, yz.w) : make_float2(yz.x, yz.y);
-            // (u_ij + v_ik) + w_jk
-            float2& v = t[2 * e4 + half];
-            if constexpr (X == 0) v = add2(add2(xy, a), c);
-            else if constexpr (X == 1) v = add2(add2(a, c), xy);
-            else v = add2(add2(c, xy), a);
-            const int e = 4 * e4 + 2 * half;
-            const float2 y = fma2(half ? make_float2(gz.z, gz.w) : make_float2(gz.x, gz.y), v,
-                                  make_float2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])));
-            sv[e] = __float_as_uint(y.x), sv[e + 1] = __float_as_uint(y.y);
+            for (int half = 0; half < 2; ++half) {
+              const float2 a = half ? make_float2(xz.z, xz.w) : make_float2(xz.x, xz.y);
+              const float2 c = half ? make_float2(yz.z, yz.w) : make_float2(yz.x, yz.y);
+              // (u_ij + v_ik) + w_jk
+              float2& v = t[2 * e4 + half];
+              if constexpr (X == 0) v = add2(add2(xy, a), c);
+              else if constexpr (X == 1) v = add2(add2(a, c), xy);
+              else v = add2(add2(c, xy), a);
+              const int e = 4 * e4 + 2 * half;
+              const float2 y = fma2(half ? make_float2(gz.z, gz.w) : make_float2(gz.x, gz.y), v,
+                                    make_float2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])));
+              sv[e] = __float_as_uint(y.x), sv[e + 1] = __float_as_uint(y.y);
+            }
           }
-        }
-        uint32_t mask = 0xffffu;
-        if constexpr (Z == 0) {
-          mask = seen ? 0xffffu : 0u;
-        } else {
-          if (masks) mask = (vis[z >> 5] >> (z & 16)) & 0xffffu;
-          else if (z + 16 > nz) mask = (1u << (nz - z)) - 1u;
-        }
-        if (!__all_sync(0xffffffffu, mask == 0xffffu)) {
+          uint32_t mask = 0xffffu;
+          if constexpr (Z == 0) {
+            mask = seen ? 0xffffu : 0u;
+          } else {
+            if (masks) mask = (vis[z >> 5] >> (z & 16)) & 0xffffu;
+            else if (z + 16 > nz) mask = (1u << (nz - z)) - 1u;
+          }
+          if (!__all_sync(0xffffffffu, mask == 0xffffu)) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e)
-            if (!((mask >> e) & 1u)) sv[e] = 0xff800000u;  // -infinity
+            for (int e = 0; e < 16; ++e)
+              if (!((mask >> e) & 1u)) sv[e] = 0xff800000u;  // -infinity
+          }
+          if constexpr (kForward) {
+            if (mode == 1) {
+              if (ok) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) m_run = fmaxf(m_run, __uint_as_float(sv[e]));
+              }
+              return;
+            }
+          }
+          uint32_t pk[8], dk[8];
+#pragma unroll
+          for (int e4 = 0; e4 < 4; ++e4) {
+            float4 cl = make_float4(lse, lse, lse, lse), cd = make_float4(delta, delta, delta, delta), cg = cd;
+            if constexpr (Z == 0) {
+              cl = *reinterpret_cast<const float4*>(cols + z + 4 * e4);
+              cd = *reinterpret_cast<const float4*>(cols + kMaxKeys + z + 4 * e4);
+              cg = *reinterpret_cast<const float4*>(cols + 2 * kMaxKeys + z + 4 * e4);
+            }
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              const int e = 4 * e4 + 2 * half;
+              float2 pr = fma2(make_float2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), make_float2(kLog2e, kLog2e),
+                               half ? make_float2(cl.z, cl.w) : make_float2(cl.x, cl.y));
+              pr.x = fast_exp2(pr.x), pr.y = fast_exp2(pr.y);
+              if constexpr (kForward) {
+                rsum = add2(rsum, pr);
+              } else {
+                const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])),
+                                                half ? make_float2(cd.z, cd.w) : make_float2(cd.x, cd.y)));
+                dk[e >> 1] = pack2_bf16(ds.x, ds.y);
+                if constexpr (Z == 0) rsum = fma2(half ? make_float2(cg.z, cg.w) : make_float2(cg.x, cg.y), ds, rsum);
+                else rsum = add2(rsum, ds);
+                if constexpr (X == 0) dgate = fma2(ds, t[e >> 1], dgate);
+              }
+              if constexpr (kPass != kDq) pk[e >> 1] = pack2_bf16(pr.x, pr.y);
+            }
+          }
+          if constexpr (kPass != kDq) tmem_st8(buf, pk);
+          if constexpr (!kForward) tmem_st8(buf + 64, dk);
+        };
+#pragma unroll 1
+        for (int s = 0; s < steps; ++s) {
+          const int S = s_first + s, st = S & (kStages - 1);
+          const int yy = s * G + gs;
+          ok = row_ok && yy < ny;
+          if constexpr (kForward) lse = -shift;
+          else lse = row_lse;
+          delta = row_delta, gate = row_gate;
+          seen = ok;
+          if (Y == 0 || p.pair_valid) {
+            const int y = yy < ny ? (int)sh.ylist[yy] : 0;
+            if constexpr (Y == 0) lse = cols[y], delta = cols[kMaxKeys + y], gate = cols[2 * kMaxKeys + y];
+            if (p.pair_valid) {
+              vis = bits + (Y == 1 ? y : X == 2 ? min(x, kMaxKeys - 1) : 0) * kWords;  // bits over the columns
+              // columns = queries: whether the row's pair of keys counts
+              if constexpr (Z == 0) seen = ok && ((bits[x * kWords + (y >> 5)] >> (y & 31)) & 1u);
+            }
+          }
+          if (!ok) lse = -INFINITY;
+          colp = bcol + (st * G + gs) * zpad;
+          wait_on(&sh.bar_full[st], S / kStages);
+          rs = bpair[st * kTileM + r];
+          rsum = make_float2(0.f, 0.f);
+#pragma unroll 1
+          for (int c = (S * C ^ grp) & 1; c < C; c += 2) {
+            const int Q = S * C + c;
+            wait_on(&sh.bar_s[Q % kBufs], Q / kBufs);
+            if (warp_live) {
+              tc_fence_after_sync();
+              uint32_t buf = trow + kColS + (Q % kBufs) * kBufCols, dst = buf;
+              int z = 16 * chunk_start(c);
+              const int z1 = z + 16 * chunk_units(c);
+#pragma unroll 1
+              for (; z < z1; z += 16, buf += 16, dst += 8) {  // (one copy of the code: the loop has to stay in the instruction caches)
+                uint32_t sv[16], dv[16];
+                tmem_ld16(buf, sv);
+                if constexpr (!kForward) tmem_ld16(buf + 64, dv);
+                tmem_ld_wait();
+                unit(dst, z, sv, dv);
+              }
+              if constexpr (!kForward)
+                if (c + 2 >= C) sums[((S & 3) * 2 + grp) * kTileM + r] = rsum.x + rsum.y;  // the group's last chunk of the step
+              tmem_st_wait();
+            }
+            tc_fence_before_sync();
+            warp_arrive(&sh.bar_p[Q % kBufs]);
+          }
+          if constexpr (kForward) l_run += rsum.x + rsum.y;
+          warp_arrive(&sh.bar_empty[st]);
         }
         if constexpr (kForward) {
-          if (mode == 1) {
-            if (ok) {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) m_run = fmaxf(m_run, __uint_as_float(sv[e]));
+          // the rows' sums (mode 1: maxima) over the two groups and the groups of first keys
+          bool again = false;
+          sums[grp * kTileM + r] = mode == 1 ? m_run : l_run;
+          group_barrier<1>();
+          if (g < G) {
+            float t = mode == 1 ? -INFINITY : 0.f;
+            for (int gg = 0; gg < G; ++gg) {
+              const float a = sums[gg * rt + ii], c = sums[kTileM + gg * rt + ii];
+              t = mode == 1 ? fmaxf(t, fmaxf(a, c)) : t + (a + c);
             }
-            return;
-          }
-        }
-        uint32_t pk[8], dk[8];
-#pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4) {
-          float4 cl = make_float4(lse, lse, lse, lse), cd = make_float4(delta, delta, delta, delta), cg = cd;
-          if constexpr (Z == 0) {
-            cl = *reinterpret_cast<const float4*>(cols + z + 4 * e4);
-            cd = *reinterpret_cast<const float4*>(cols + kMaxKeys + z + 4 * e4);
-            cg = *reinterpret_cast<const float4*>(cols + 2 * kMaxKeys + z + 4 * e4);
-          }
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int e = 4 * e4 + 2 * half;
-            float2 pr = fma2(make_float2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), make_float2(kLog2e, kLog2e),
-                             half ? make_float2(cl.z, cl.w) : make_float2(cl.x, cl.y));
-            pr.x = fast_exp2(pr.x), pr.y = fast_exp2(pr.y);
-            if constexpr (kForward) {
-              rsum = add2(rsum, pr);
+            if (mode == 1) {
+              shift = t > -INFINITY ? t * kLog2e : 0.f;
+              again = true;
             } else {
-              const float2 ds = mul2(pr, add2(make_float2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])),
-                                              half ? make_float2(cd.z, cd.w) : make_float2(cd.x, cd.y)));
-              dk[e >> 1] = pack2_bf16(ds.x, ds.y);
-              if constexpr (Z == 0) rsum = fma2(half ? make_float2(cg.z, cg.w) : make_float2(cg.x, cg.y), ds, rsum);
-              else rsum = add2(rsum, ds);
-              if constexpr (X == 0) dgate = fma2(ds, t[e >> 1], dgate);
+              if (mode == 0) again = row_ok && !bad && !(t >= kSumLow && t <= kSumHigh);
+              if (grp == 0) row_l[r] = t, row_shift[r] = shift;
             }
-            if constexpr (kPass != kDq) pk[e >> 1] = pack2_bf16(pr.x, pr.y);
           }
+          if (!next_mode(again)) break;
         }
-        if constexpr (kPass != kDq) tmem_st8(buf, pk);
-        if constexpr (!kForward) tmem_st8(buf + 64, dk);
-      };
-#pragma unroll 1
-      for (int s = 0; s < steps; ++s) {
-        const int S = s_first + s, st = S & (kStages - 1);
-        const int yy = s * G + gs;
-        ok = row_ok && yy < ny;
-        if constexpr (kForward) lse = -shift;
-        else lse = row_lse;
-        delta = row_delta, gate = row_gate;
-        seen = ok;
-        if (Y == 0 || p.pair_valid) {
-          const int y = yy < ny ? (int)sh.ylist[yy] : 0;
-          if constexpr (Y == 0) lse = cols[y], delta = cols[kMaxKeys + y], gate = cols[2 * kMaxKeys + y];
-          if (p.pair_valid) {
-            vis = bits + (Y == 1 ? y : X == 2 ? min(x, kMaxKeys - 1) : 0) * kWords;  // bits over the columns
-            // columns = queries: whether the row's pair of keys counts
-            if constexpr (Z == 0) seen = ok && ((bits[x * kWords + (y >> 5)] >> (y & 31)) & 1u);
-          }
-        }
-        if (!ok) lse = -INFINITY;
-        colp = bcol + (st * G + gs) * zpad;
-        wait_on(&sh.bar_full[st], S / kStages);
-        rs = bpair[st * kTileM + r];
-        rsum = make_float2(0.f, 0.f);
-#pragma unroll 1
-        for (int c = (S * C ^ grp) & 1; c < C; c += 2) {
-          const int Q = S * C + c;
-          wait_on(&sh.bar_s[Q % kBufs], Q / kBufs);
-          if (warp_live) {
-            tc_fence_after_sync();
-            uint32_t buf = trow + kColS + (Q % kBufs) * kBufCols, dst = buf;
-            int z = 16 * chunk_start(c);
-            const int z1 = z + 16 * chunk_units(c);
-#pragma unroll 1
-            for (; z < z1; z += 16, buf += 16, dst += 8) {  // (one copy of the code: the loop has to stay in the instruction caches)
-              uint32_t sv[16], dv[16];
-              tmem_ld16(buf, sv);
-              if constexpr (!kForward) tmem_ld16(buf + 64, dv);
-              tmem_ld_wait();
-              unit(dst, z, sv, dv);
-            }
-            if constexpr (!kForward)
-              if (c + 2 >= C) sums[((S & 3) * 2 + grp) * kTileM + r] = rsum.x + rsum.y;  // the group's last chunk of the step
-            tmem_st_wait();
-          }
-          tc_fence_before_sync();
-          warp_arrive(&sh.bar_p[Q % kBufs]);
-        }
-        if constexpr (kForward) l_run += rsum.x + rsum.y;
-        warp_arrive(&sh.bar_empty[st]);
-      }
-      if constexpr (kForward) {
-        // the rows' sums (mode 1: maxima) over the two groups and the groups of first keys
-        bool again = false;
-        sums[grp * kTileM + r] = mode == 1 ? m_run : l_run;
-        group_barrier<1>();
-        if (g < G) {
-          float t = mode == 1 ? -INFINITY : 0.f;
-          for (int gg = 0; gg < G; ++gg) {
-            const float a = sums[gg * rt + ii], c = sums[kTileM + gg * rt + ii];
-            t = mode == 1 ? fmaxf(t, fmaxf(a, c)) : t + (a + c);
-          }
-          if (mode == 1) {
-            shift = t > -INFINITY ? t * kLog2e : 0.f;
-            again = true;
-          } else {
-            if (mode == 0) again = row_ok && !bad && !(t >= kSumLow && t <= kSumHigh);
-            if (grp == 0) row_l[r] = t, row_shift[r] = shift;
-          }
-        }
-        if (!next_mode(again)) break;
-      }
       }
       if constexpr (kPass == kDq) {
         // (the row warps read the last steps' sums; these lie beyond them)
