@@ -382,7 +382,7 @@ int queries_per_cta(int bh, int tokens) {
 size_t simplicial_warp_order_bytes(int batch, int heads, int tokens) {
   const long long bh = (long long)batch * heads;
   const int chunk = queries_per_cta((int)bh, tokens);
-  const bool pays = batch > 1 && batch <= kMostOrdered && bh * ((tokens + chunk - 1) / chunk) >= 222 &&
+  const bool pays = batch > 3 && batch <= kMostOrdered && bh * ((tokens + chunk - 1) / chunk) >= 222 &&
                     bh * tokens * tokens * tokens >= 30000000ll;
   return pays ? align_up((size_t)batch * sizeof(int32_t), 256) : 0;
 }
