@@ -59,21 +59,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// The phase's state as it is (try_wait may hold the thread for a while before it answers "not yet")
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // Same test, but the thread may be parked by the hardware for up to `hint_ns` nanoseconds while the phase is
 // incomplete (it is woken when the phase completes).  A parked thread issues nothing, so waiting warps do not
 // take issue slots from the warps that share their scheduler.
