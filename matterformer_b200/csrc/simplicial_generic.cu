@@ -18,6 +18,8 @@
 //
 // Semantics follow simplicial_attention_torch_from_projected
 // (src/matterformer/models/simplicial_attention.py:206-344 of the reference).
+#include <mutex>
+
 #include "common.cuh"
 #include "simplicial.cuh"
 
@@ -521,7 +523,11 @@ int launch_mode_r(const GenericParams& p, int BH, cudaStream_t stream) {
   constexpr int DS = DMAX + 4;
   const size_t smem = (size_t)(4 * 32 * DS + 4 * 2 * DMAX + 4 * p.N + 4 * kResMax) * sizeof(float);
   auto kern = simplicial_generic_kernel<T, DMAX, MODE, kRes>;
+  // the limit follows the call's size: no other host thread may lower it between here and the launch
+  static std::mutex limit_mutex;
+  std::unique_lock<std::mutex> lock(limit_mutex, std::defer_lock);
   if (smem > 48 * 1024) {
+    lock.lock();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_generic)");
   }

@@ -67,7 +67,7 @@ constexpr int kOffSums = kOffCols + 3 * kMaxKeys * 4;           // [4 steps][2][
 constexpr int kOffDgate = kOffSums + 4 * 2 * kTileM * 4;         // [2][128]
 constexpr int kOffTile = kOffDgate + 2 * kTileM * 4;         // bias: operand of (x, z), then that of (y, z) by stages
 static_assert(kOffTile % 128 == 0, "alignment");
-inline int tri_smem_bytes(int tokens) {
+constexpr int tri_smem_bytes(int tokens) {
   // tile: (rows | 1) x columns, stages: groups x columns; rows * groups <= 128, so 129 + kStages rows of floats at most
   return kOffTile + 1024 + kStages * kTileM * 4 + (129 + kStages) * ((tokens + 15) & ~15) * 4;
 }
@@ -933,11 +933,11 @@ int launch_tri(Kernel kernel, const TriParams& p, const TriLayout& l, int batch,
   simplicial_tri_schedule_kernel<<<1, kScheduleThreads, 0, stream>>>(p.query_valid, p.key_valid, batch, p.N, backward,
                                                                      const_cast<BatchInfo*>(p.info), const_cast<int2*>(p.items), p.status);
   MF_CHECK_LAUNCH("simplicial_tri_schedule_kernel");
-  const int bytes = tri_smem_bytes(p.N);
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  // (the limit is one for all sizes: another host thread must not lower it between here and the launch)
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes(kMaxKeys));
   if (e != cudaSuccess) return cuda_error(e, name);
   profile_mark(which, true, stream);
-  kernel<<<(unsigned)l.max_items * p.H, kTriThreads, bytes, stream>>>(p);
+  kernel<<<(unsigned)l.max_items * p.H, kTriThreads, tri_smem_bytes(p.N), stream>>>(p);
   profile_mark(which, false, stream);
   MF_CHECK_LAUNCH(name);
   return MF_OK;

@@ -414,9 +414,11 @@ int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   const int bh = a.batch * a.heads;
   const int chunk = queries_per_cta(bh, a.tokens);
   p.chunk = chunk;
-  const int rows = (a.tokens + 31) & ~31, bytes = (int)((sizeof(WarpFwdHeader) + 127) / 128 * 128) + 4 * rows * kRowBytes;
+  constexpr int header = (int)((sizeof(WarpFwdHeader) + 127) / 128 * 128);
+  const int rows = (a.tokens + 31) & ~31, bytes = header + 4 * rows * kRowBytes;
   auto kernel = a.u ? simplicial_warp_fwd_kernel<true> : simplicial_warp_fwd_kernel<false>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  // (the limit is one for all sizes: another host thread must not lower it between here and the launch)
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, header + 4 * kMaxKeys * kRowBytes);
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_warp_fwd_kernel)");
   profile_mark(MF_PROFILE_SIMPLICIAL_FWD, true, stream);
   kernel<<<dim3((a.tokens + chunk - 1) / chunk, bh), kFwdThreads, bytes, stream>>>(p);
