@@ -190,11 +190,13 @@ size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* args);
 size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* args);
 
 /* Whether a call with these arguments runs on tensor-core kernels (MF_BACKEND_TCGEN05, also where these are the warp-level
- * mma.sync ones) or on CUDA cores (MF_BACKEND_GENERIC).  (No counterpart in the reference.)  Tensor-core kernels that take a
- * workspace leave a status word at its start, except the warp-level ones: at most 32 tokens, or a forward call without the bias on
- * the default backend (they have no device-side waits). */
+ * mma.sync ones) or on CUDA cores (MF_BACKEND_GENERIC).  (No counterpart in the reference.) */
 int mf_simplicial_fwd_backend(const MfSimplicialFwdArgs* args);
 int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* args);
+/* 1 when the call, given the workspace that it asks for, leaves a status word (MF_OK or MF_ERR_DEVICE_TIMEOUT, int32) at the start of
+ * that workspace, 0 when it runs on kernels without device-side waits.  (No counterpart in the reference.) */
+int mf_simplicial_fwd_keeps_status(const MfSimplicialFwdArgs* args);
+int mf_simplicial_bwd_keeps_status(const MfSimplicialBwdArgs* args);
 /* The gradient of message_basis from MfSimplicialBwdArgs.message_coeff: out[h,r,:] = sum_{b,i} coeff[b,h,i,r] grad_out[b,h,i,:]
  * (coeff (B,H,N,R) fp32, grad_out (B,H,N,D) in `dtype`, out (H,R,D) fp32; fixed order of additions). */
 int mf_simplicial_basis_grad(const float* coeff, const void* grad_out, int32_t dtype, int32_t batch, int32_t heads,

@@ -33,6 +33,8 @@ EXPORTED_SYMBOLS = (
     "mf_simplicial_bwd_needs_zeros",
     "mf_simplicial_basis_grad",
     "mf_simplicial_bwd_backend",
+    "mf_simplicial_fwd_keeps_status",
+    "mf_simplicial_bwd_keeps_status",
     "mf_simplicial_row_plan",
     "mf_simplicial_fwd_workspace_bytes",
     "mf_simplicial_bwd_workspace_bytes",
@@ -401,6 +403,10 @@ def lib() -> ctypes.CDLL:
     L.mf_simplicial_fwd_backend.restype = c_int32
     L.mf_simplicial_bwd_backend.argtypes = [POINTER(MfSimplicialBwdArgs)]
     L.mf_simplicial_bwd_backend.restype = c_int32
+    L.mf_simplicial_fwd_keeps_status.argtypes = [POINTER(MfSimplicialFwdArgs)]
+    L.mf_simplicial_fwd_keeps_status.restype = c_int32
+    L.mf_simplicial_bwd_keeps_status.argtypes = [POINTER(MfSimplicialBwdArgs)]
+    L.mf_simplicial_bwd_keeps_status.restype = c_int32
     L.mf_simplicial_bwd_needs_zeros.argtypes = [POINTER(MfSimplicialBwdArgs)]
     L.mf_simplicial_bwd_needs_zeros.restype = c_int32
     L.mf_simplicial_basis_grad.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p,

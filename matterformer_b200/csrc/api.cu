@@ -174,6 +174,19 @@ extern "C" int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* a) {
   return wants_tcgen05(a, &rc, "mf_simplicial_bwd_backend") ? MF_BACKEND_TCGEN05 : MF_BACKEND_GENERIC;
 }
 
+// The kernels of at most 32 tokens, the warp-level forward kernel and the CUDA-core kernels have no device-side waits.
+extern "C" int mf_simplicial_fwd_keeps_status(const MfSimplicialFwdArgs* a) {
+  if (!a) return 0;
+  int rc;
+  return wants_tcgen05(a, &rc, "mf_simplicial_fwd_keeps_status") && !uses_small_kernels(a) && (uses_tri_kernels(a) || !uses_warp_forward(a));
+}
+
+extern "C" int mf_simplicial_bwd_keeps_status(const MfSimplicialBwdArgs* a) {
+  if (!a) return 0;
+  int rc;
+  return wants_tcgen05(a, &rc, "mf_simplicial_bwd_keeps_status") && !uses_small_kernels(a);
+}
+
 extern "C" int mf_simplicial_bwd_needs_zeros(const MfSimplicialBwdArgs* a) {
   if (!a) return 1;
   int rc;

@@ -79,13 +79,6 @@ void fill_common(Args& a, const std::array<Tensor, kInputs>& t, int precision, i
   a.angle_rank = t[AL].defined() ? t[AL].size(4) : 0, a.message_rank = t[ML].defined() ? t[ML].size(4) : 0;
 }
 
-// Whether the workspace starts with a status word: the warp-level kernels (at most 32 tokens; forward without the bias) have no
-// device-side waits
-bool keeps_status(const MfSimplicialBwdArgs& a) { return a.tokens > 32 || a.backend == MF_BACKEND_TCGEN05; }
-bool keeps_status(const MfSimplicialFwdArgs& a) {
-  return a.backend == MF_BACKEND_TCGEN05 || (a.tokens > 32 && (a.u || a.backend != MF_BACKEND_AUTO));
-}
-
 struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
   static Variable forward(AutogradContext* ctx, const Tensor& q, const Tensor& k1, const Tensor& v1, const Tensor& k2,
                           const Tensor& v2, const Tensor& qv, const Tensor& kv, const OptTensor& pv, const OptTensor& u,
@@ -106,7 +99,8 @@ struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
     const Tensor ws = bytes(mf_simplicial_fwd_workspace_bytes(&a), q);
     if (ws.defined()) a.workspace = ws.data_ptr(), a.workspace_bytes = ws.numel();
     check(mf_simplicial_fwd(&a, c10::cuda::getCurrentCUDAStream().stream()));
-    if (mf_simplicial_fwd_backend(&a) == MF_BACKEND_TCGEN05) remember_status(keeps_status(a) && ws.defined() ? OptTensor(ws) : std::nullopt);
+    if (mf_simplicial_fwd_backend(&a) == MF_BACKEND_TCGEN05)
+      remember_status(ws.defined() && mf_simplicial_fwd_keeps_status(&a) ? OptTensor(ws) : std::nullopt);
     ctx->saved_data["precision"] = precision;
     ctx->saved_data["backend"] = backend;
     tensor_list saved(t.begin(), t.end());
@@ -155,7 +149,8 @@ struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
     if (ws.defined()) a.workspace = ws.data_ptr(), a.workspace_bytes = ws.numel();
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     check(mf_simplicial_bwd(&a, stream));
-    if (mf_simplicial_bwd_backend(&a) == MF_BACKEND_TCGEN05) remember_status(keeps_status(a) && ws.defined() ? OptTensor(ws) : std::nullopt);
+    if (mf_simplicial_bwd_backend(&a) == MF_BACKEND_TCGEN05)
+      remember_status(ws.defined() && mf_simplicial_bwd_keeps_status(&a) ? OptTensor(ws) : std::nullopt);
     if (coeff.defined()) {
       g[BASIS] = at::empty_like(t[BASIS]);
       check(mf_simplicial_basis_grad(a.message_coeff, a.grad_out, a.dtype, a.batch, a.heads, a.tokens, a.message_rank, a.head_dim,

@@ -76,14 +76,6 @@ def _remember_status(ws: Optional[torch.Tensor]) -> None:
                                "the outputs of this call are zeros")  # fmt: skip
 
 
-def _keeps_status(a) -> bool:
-    """Whether the call's workspace starts with a status word: the warp-level kernels (at most 32 tokens; forward without the
-    bias) have no device-side waits."""
-    if a.backend == _lib.MF_BACKEND["tcgen05"] or a.tokens <= 32:
-        return a.backend == _lib.MF_BACKEND["tcgen05"]
-    return isinstance(a, _lib.MfSimplicialBwdArgs) or bool(a.u) or a.backend != _lib.MF_BACKEND["auto"]
-
-
 def device_status() -> int:
     """Status word the most recent tensor-core simplicial kernel left in its workspace.
 
@@ -250,7 +242,7 @@ def cuda_simplicial_attention_forward(
     _lib.launch(L.mf_simplicial_fwd, q.device, ref)
     # only the tensor-core kernels keep a status word in their workspace
     if L.mf_simplicial_fwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
-        _remember_status(ws if _keeps_status(a) else None)
+        _remember_status(ws if L.mf_simplicial_fwd_keeps_status(ref) else None)
     return out, lse, out32
 
 
@@ -360,7 +352,7 @@ def cuda_simplicial_attention_backward(
     _lib.launch(L.mf_simplicial_bwd, q.device, ref)
     # only the tensor-core kernels keep a status word in their workspace
     if L.mf_simplicial_bwd_backend(ref) == _lib.MF_BACKEND["tcgen05"]:
-        _remember_status(ws if _keeps_status(a) else None)
+        _remember_status(ws if L.mf_simplicial_bwd_keeps_status(ref) else None)
     if bias is not None:  # the reference returns each bias gradient in the dtype of its operand (:1155-1160)
         bias_grads = [g.to(t.dtype) if g is not None else None for g, t in zip(bias_grads, (u, v_bias, w, gate))]
     if angle is not None:

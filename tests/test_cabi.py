@@ -122,3 +122,21 @@ def test_unaligned_tensors_are_caught_before_any_launch():
     a.query_valid = a.pair_key_valid = ok
     assert L.mf_simplicial_fwd(ctypes.byref(a), None) == _lib.MF_ERR_UNSUPPORTED
     assert "16-byte boundaries" in _lib.last_error()
+
+
+@pytest.mark.parametrize("backend,tokens,bias,dtype,fwd,bwd", [
+    ("auto", 32, False, "bf16", 0, 0), ("auto", 32, True, "bf16", 0, 0), ("auto", 33, False, "bf16", 0, 1),
+    ("auto", 33, True, "f32", 0, 0), ("auto", 193, False, "bf16", 0, 0), ("generic", 64, False, "bf16", 0, 0),
+    ("tcgen05", 20, False, "bf16", 1, 1), ("tcgen05", 33, False, "bf16", 1, 1), ("tcgen05_tiles", 32, True, "bf16", 0, 0),
+    ("tcgen05_tiles", 33, False, "bf16", 1, 1), ("tcgen05_tiles", 192, True, "bf16", 1, 1),
+])  # fmt: skip
+def test_which_calls_leave_a_status_word(backend, tokens, bias, dtype, fwd, bwd):
+    L = _lib.lib()
+    for cls, name, want in ((_lib.MfSimplicialFwdArgs, "fwd", fwd), (_lib.MfSimplicialBwdArgs, "bwd", bwd)):
+        a = cls(batch=64, heads=8, tokens=tokens, head_dim=64, backend=_lib.MF_BACKEND[backend],
+                dtype=_lib.MF_DTYPE_BF16 if dtype == "bf16" else _lib.MF_DTYPE_F32)  # fmt: skip
+        if bias:
+            a.u = a.v_bias = a.w = a.gate = 256  # (never read)
+        assert getattr(L, f"mf_simplicial_{name}_keeps_status")(ctypes.byref(a)) == want
+        if want:  # the workspace that such a call asks for holds the word
+            assert getattr(L, f"mf_simplicial_{name}_workspace_bytes")(ctypes.byref(a)) >= 256
