@@ -43,6 +43,7 @@ EXPORTED_SYMBOLS = (
     "mf_simplicial_fwd_noalloc",
     "mf_simplicial_noalloc_status",
     "mf_selftest_wait_timeout",
+    "mf_selftest_simplicial_give_up",
     "mf_knn_topk",
     "mf_knn_search_grid",
     "mf_knn_cells_workspace_bytes",
@@ -312,6 +313,8 @@ def lib() -> ctypes.CDLL:
     L.mf_simplicial_noalloc_status.restype = c_int32
     L.mf_selftest_wait_timeout.argtypes = [c_void_p, ctypes.c_int64, c_void_p]
     L.mf_selftest_wait_timeout.restype = c_int32
+    L.mf_selftest_simplicial_give_up.argtypes = [POINTER(MfSimplicialFwdArgs), POINTER(MfSimplicialBwdArgs), c_int32, ctypes.c_int64, c_void_p]
+    L.mf_selftest_simplicial_give_up.restype = c_int32
     L.mf_knn_topk.argtypes = [c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p]
     L.mf_knn_topk.restype = c_int32
     L.mf_knn_search_grid.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p]

@@ -250,6 +250,29 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
   return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
 }
 
+extern "C" int mf_selftest_simplicial_give_up(const MfSimplicialFwdArgs* fwd, const MfSimplicialBwdArgs* bwd, int32_t withheld,
+                                              int64_t limit_cycles, void* stream) {
+  const char* name = "mf_selftest_simplicial_give_up";
+  MF_CHECK_ARG((fwd != nullptr) != (bwd != nullptr), "%s: one of the two argument structs", name);
+  MF_CHECK_ARG(withheld >= 0 && withheld < 8, "%s: barrier kind %d not in [0, 8)", name, (int)withheld);
+  MF_CHECK_ARG(limit_cycles >= 1 && limit_cycles <= (1ll << 31), "%s: limit must be in [1, 2^31] clocks", name);
+  const TriWaits waits{(long long)limit_cycles, withheld};
+  auto run = [&](const auto* a, size_t need, auto kernels) {
+    int rc = check_common(a, name);
+    if (rc != MF_OK || (rc = check_bias(a, name)) != MF_OK) return rc;
+    MF_CHECK_ARG(wants_tcgen05(a, &rc, name) && uses_tri_kernels(a) && a->batch > 0 && a->heads > 0 && a->workspace &&
+                     a->workspace_bytes >= need,
+                 "%s: only calls that the trilinear kernels serve, with their workspace", name);
+    return kernels(*a, static_cast<cudaStream_t>(stream), waits);
+  };
+  if (fwd) {
+    MF_CHECK_ARG(fwd->out && fwd->lse, "%s: null output pointer", name);
+    return run(fwd, mf_simplicial_fwd_workspace_bytes(fwd), simplicial_tri_fwd);
+  }
+  MF_CHECK_ARG(bwd->grad_out && bwd->out && bwd->lse && bwd->dq && bwd->dk1 && bwd->dv1 && bwd->dk2 && bwd->dv2, "%s: null pointer", name);
+  return run(bwd, mf_simplicial_bwd_workspace_bytes(bwd), simplicial_tri_bwd);
+}
+
 // ---------------------------------------------------------------------------
 // kernel timing aid
 // ---------------------------------------------------------------------------

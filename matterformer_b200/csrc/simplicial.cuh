@@ -40,8 +40,14 @@ int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 size_t simplicial_warp_order_bytes(int batch, int heads, int tokens);  // without the bias; optional
 
 // trilinear tcgen05 kernels for 33 to 192 tokens with the factorized bias (simplicial_tri.cu)
-int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
-int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
+// Its waits give up after `limit` clocks.  The self-test lets them run out: the barriers of kind `withheld` (0-7) expect one arrival
+// more than there are.
+struct TriWaits {
+  long long limit = 1ll << 31;  // kWaitLimitCycles
+  int withheld = -1;
+};
+int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, TriWaits waits = {});
+int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, TriWaits waits = {});
 size_t simplicial_tri_fwd_workspace_bytes(const MfSimplicialFwdArgs& a);
 size_t simplicial_tri_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 

@@ -120,6 +120,7 @@ struct TriParams {
   const int2* items;              // [0].x = count, then {batch | pass << 16 | tile << 20, rows | tiles << 8}
   int32_t* status;
   int H, N;
+  TriWaits waits;
 };
 
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
@@ -139,7 +140,9 @@ __device__ __forceinline__ void group_barrier() {
 struct TriShared {
   uint64_t bar_a[2], bar_free[2], bar_s[4], bar_p[4], bar_t[2], bar_d[2];
   uint64_t bar_full[kStages], bar_empty[kStages];
+  uint64_t bar_drain;
   uint32_t tmem;
+  int gave_up;               // forward: a wait of any thread has expired
   uint32_t mask[2][kWords];  // valid queries, valid keys
   uint8_t ylist[kMaxKeys];   // the valid y in order
 };
@@ -186,21 +189,24 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
   const int C = (units + 3) >> 2, per = units / C, extra = units % C;  // chunks of a step: per or per + 1 units
 
   if (tid == 0) {
+    auto count = [&](int which, int n) { return (uint32_t)(n + (p.waits.withheld == which)); };  // (see TriWaits)
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh.bar_a[i], kRowWarps);
-      mbar_init(&sh.bar_free[i], 1);
-      mbar_init(&sh.bar_t[i], 1);
-      mbar_init(&sh.bar_d[i], kRowWarps);
+      mbar_init(&sh.bar_a[i], count(0, kRowWarps));
+      mbar_init(&sh.bar_free[i], count(1, 1));
+      mbar_init(&sh.bar_t[i], count(2, 1));
+      mbar_init(&sh.bar_d[i], count(3, kRowWarps));
     }
     for (int i = 0; i < kBufs; ++i) {
-      mbar_init(&sh.bar_s[i], 1);
-      mbar_init(&sh.bar_p[i], 4);
+      mbar_init(&sh.bar_s[i], count(4, 1));
+      mbar_init(&sh.bar_p[i], count(5, 4));
     }
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(&sh.bar_full[i], 64);
-      mbar_init(&sh.bar_empty[i], kExpWarps);
+      mbar_init(&sh.bar_full[i], count(6, 64));
+      mbar_init(&sh.bar_empty[i], count(7, kExpWarps));
     }
+    mbar_init(&sh.bar_drain, 1);
     mbar_fence_init();
+    sh.gave_up = 0;
   }
   if (warp == kIssuerWarp) {
     tmem_alloc(&sh.tmem, kTmemCols);
@@ -315,14 +321,17 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
   const uint32_t tmem = sh.tmem;
   bool bad = false;
   auto wait_on = [&](uint64_t* bar, uint32_t phase) {
-    if (!bad) bad = !mbar_wait(bar, phase & 1u);
+    if (!bad) bad = !mbar_wait_for(bar, phase & 1u, p.waits.limit);
   };
   auto chunk_units = [&](int c) { return per + (c < extra); };
   auto chunk_start = [&](int c) { return c * per + min(c, extra); };  // in units
 
   // Forward: mode 0 with shift 0; if a row's sum is out of range, mode 1 finds the maxima and mode 2 does the tile again.
   constexpr int kModes = kForward ? 3 : 1;
-  auto next_mode = [&](bool again) { return __syncthreads_or(again) != 0; };
+  auto next_mode = [&](bool again) {
+    if (bad) sh.gave_up = 1;
+    return __syncthreads_or(again) != 0;
+  };
 
   if (warp >= kIssuerWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<kForward>::kAux));
@@ -390,6 +399,9 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
             advance(sm, nu);
             if (q + ahead < total) next_logits();
           }
+          // Whoever gave up, no product may be in flight when tensor memory is given back
+          umma_commit(&sh.bar_drain);
+          if (!mbar_wait_for(&sh.bar_drain, mode & 1, p.waits.limit)) bad = true;
         }
         __syncwarp();
       } else if (warp == kBiasLoader) {
@@ -448,6 +460,7 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
           cp_async_arrive(&sh.bar_full[st]);
         }
       }
+      cp_async_wait<0>();  // (nothing is left, unless a consumer gave up)
       if (kForward && !next_mode(false)) break;
     }
   } else {
@@ -642,7 +655,7 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
         if (grp == 0 && g == 0 && x < nx && p.dgate) {
           float t = 0.f;
           for (int gg = 0; gg < G; ++gg) t += xs[gg * rt + r] + xs[kTileM + gg * rt + r];
-          p.dgate[(size_t)bh * N + x] = row_ok && !bad ? t : 0.f;
+          p.dgate[(size_t)bh * N + x] = row_ok ? t : 0.f;
         }
       }
     } else {
@@ -768,6 +781,7 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
       }
       if (g == 0 && x < nx) {
         const float l = kForward ? row_l[r] : 1.f;
+        if constexpr (kForward) bad = bad || sh.gave_up;  // (written before the barrier of next_mode)
         const bool have = row_ok && !bad && l != 0.f;
         const float scale = have ? 1.f / l : 0.f;
         if (kForward || !have) {
@@ -795,7 +809,7 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
 
   tc_fence_before_sync();
   bad = __syncthreads_or(bad) != 0;
-  if (bad && tid == 0) atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
+  if (bad && tid == 0) atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);  // (backward: the gradients are cleared by the last launch)
   if (warp == kIssuerWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
@@ -895,6 +909,20 @@ __global__ void __launch_bounds__(256) simplicial_tri_rows_kernel(const __nv_bfl
   if (lane == 0) lse2[row] = -lse[row] * kLog2e, ndelta[row] = -s;
 }
 
+// When a wait expired anywhere every gradient is written as zeros: a row's sums leave while other roles may still give up, and what
+// the other CTAs have written belongs to the same call.  Else it returns at once.
+struct TriClear {
+  uint32_t* at[9];
+  size_t words[9];
+};
+__global__ void __launch_bounds__(256) simplicial_tri_clear_kernel(const __grid_constant__ TriClear c, const int32_t* __restrict__ status) {
+  if (*status == 0) return;
+#pragma unroll 1
+  for (int t = 0; t < 9; ++t)
+    if (c.at[t])
+      for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < c.words[t]; i += (size_t)gridDim.x * 256) c.at[t][i] = 0u;
+}
+
 struct TriLayout {
   size_t info, items, lse2, ndelta, total;
   int max_items;
@@ -948,9 +976,10 @@ int launch_tri(Kernel kernel, const TriParams& p, const TriLayout& l, int batch,
 size_t simplicial_tri_fwd_workspace_bytes(const MfSimplicialFwdArgs& a) { return tri_layout(a.batch, a.heads, a.tokens, false).total; }
 size_t simplicial_tri_bwd_workspace_bytes(const MfSimplicialBwdArgs& a) { return tri_layout(a.batch, a.heads, a.tokens, true).total; }
 
-int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
+int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, TriWaits waits) {
   const TriLayout l = tri_layout(a.batch, a.heads, a.tokens, false);
   TriParams p{};
+  p.waits = waits;
   fill_params(p, a, l);
   p.other[0] = p.main[0];  // (not read)
   p.out = a.out, p.lse = a.lse, p.out_cast = static_cast<__nv_bfloat16*>(a.out_cast);
@@ -958,9 +987,10 @@ int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
                     "simplicial_tri_fwd_kernel");
 }
 
-int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
+int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, TriWaits waits) {
   const TriLayout l = tri_layout(a.batch, a.heads, a.tokens, true);
   TriParams p{};
+  p.waits = waits;
   fill_params(p, a, l);
   char* ws = static_cast<char*>(a.workspace);
   float* lse2 = reinterpret_cast<float*>(ws + l.lse2);
@@ -974,8 +1004,15 @@ int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   const int rows = a.batch * a.heads * a.tokens;
   simplicial_tri_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p.other[0], a.out, a.lse, a.query_valid, a.heads, a.tokens, rows, lse2, ndelta);
   MF_CHECK_LAUNCH("simplicial_tri_rows_kernel");
-  return launch_tri(simplicial_tri_bwd_kernel, p, l, a.batch, true, MF_PROFILE_SIMPLICIAL_BWD, stream,
-                    "simplicial_tri_bwd_kernel");
+  const int rc = launch_tri(simplicial_tri_bwd_kernel, p, l, a.batch, true, MF_PROFILE_SIMPLICIAL_BWD, stream, "simplicial_tri_bwd_kernel");
+  if (rc != MF_OK) return rc;
+  const size_t n = (size_t)rows;
+  void* grads[9] = {a.dq, a.dk1, a.dv1, a.dk2, a.dv2, a.du, a.dv_bias, a.dw, a.dgate};
+  TriClear c{};
+  for (int t = 0; t < 9; ++t) c.at[t] = static_cast<uint32_t*>(grads[t]), c.words[t] = t < 5 ? n * (kD / 2) : t < 8 ? n * a.tokens : n;
+  simplicial_tri_clear_kernel<<<148, 256, 0, stream>>>(c, p.status);
+  MF_CHECK_LAUNCH("simplicial_tri_clear_kernel");
+  return MF_OK;
 }
 
 }  // namespace mf

@@ -1,0 +1,52 @@
+"""What an expired device-side wait of the trilinear kernels leaves behind: the status, zeros, and a device that goes on."""
+import ctypes
+
+import pytest
+import torch
+
+from matterformer_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+B, H, N = 2, 2, 64  # 32 and 14 steps a tile: more than the stages of the bias operands
+
+
+def _call(cls, **outputs):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    t = {n: rnd(B, H, N, 64).bfloat16() for n in ("q", "k1", "v1", "k2", "v2")}
+    t.update(u=rnd(B, H, N, N), v_bias=rnd(B, H, N, N), w=rnd(B, H, N, N), gate=rnd(B, H, N))
+    valid = (torch.arange(N, device="cuda")[None] < torch.tensor([[N], [40]], device="cuda")).view(torch.uint8)
+    t.update(query_valid=valid, pair_key_valid=valid, **outputs)
+    a = cls(batch=B, heads=H, tokens=N, head_dim=64, dtype=_lib.MF_DTYPE_BF16, backend=_lib.MF_BACKEND["tcgen05_tiles"])
+    for name, x in t.items():
+        setattr(a, name, x.data_ptr())
+    size = "mf_simplicial_fwd_workspace_bytes" if cls is _lib.MfSimplicialFwdArgs else "mf_simplicial_bwd_workspace_bytes"
+    ws = torch.empty(getattr(_lib.lib(), size)(ctypes.byref(a)), dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    return a, t, ws
+
+
+@pytest.mark.parametrize("withheld", range(8))
+@pytest.mark.parametrize("backward", [False, True], ids=["forward", "backward"])
+def test_a_hand_off_that_never_completes(backward, withheld):
+    nan = lambda *s, dtype=torch.float32: torch.full(s, float("nan"), dtype=dtype, device="cuda")  # noqa: E731
+    bf = dict(dtype=torch.bfloat16)
+    if backward:
+        outputs = {n: nan(B, H, N, 64, **bf) for n in ("dq", "dk1", "dv1", "dk2", "dv2")}
+        outputs.update(du=nan(B, H, N, N), dv_bias=nan(B, H, N, N), dw=nan(B, H, N, N), dgate=nan(B, H, N))
+        saved = dict(grad_out=torch.ones(B, H, N, 64, device="cuda", **bf), out=torch.zeros(B, H, N, 64, device="cuda"),
+                     lse=torch.zeros(B, H, N, device="cuda"))  # fmt: skip
+        a, keep, ws = _call(_lib.MfSimplicialBwdArgs, **outputs, **saved)
+    else:
+        outputs = dict(out=nan(B, H, N, 64), out_cast=nan(B, H, N, 64, **bf), lse=nan(B, H, N))
+        a, keep, ws = _call(_lib.MfSimplicialFwdArgs, **outputs)
+    ref, stream = ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _lib.check(_lib.lib().mf_selftest_simplicial_give_up(None if backward else ref, ref if backward else None, withheld, 20_000, stream))
+    assert ws[:4].view(torch.int32).item() == _lib.MF_ERR_DEVICE_TIMEOUT
+    for name, t in outputs.items():
+        assert torch.equal(t, torch.zeros_like(t)), name
+    # the same call with nothing withheld, on the same buffers
+    _lib.check(getattr(_lib.lib(), "mf_simplicial_bwd" if backward else "mf_simplicial_fwd")(ref, stream))
+    assert ws[:4].view(torch.int32).item() == _lib.MF_OK
+    assert all(torch.isfinite(outputs[n]).all() for n in (("dq", "dk1", "dv1", "dk2", "dv2") if backward else outputs))
+    del keep
