@@ -105,14 +105,27 @@ bool uses_small_kernels(const Args* a) {
   return (a->backend == MF_BACKEND_AUTO || a->backend == MF_BACKEND_TCGEN05_TILES) && a->tokens <= kSmallTokens;
 }
 
-// Larger molecules: with the factorized bias the trilinear tcgen05 kernels (simplicial_tri.cu has both sides' times).  Without it the
-// forward pass runs on the warp-level kernel, unless a tcgen05 family is asked for: 64 molecules of 20-181 atoms take 0.64 ms on
-// the trilinear kernel against 0.89, but 2 molecules 201 us against 105, and the choice may not depend on the batch (a molecule's
-// result does not); the backward pass runs on the row-packed kernel (1.98 against 2.26 ms).
+// Larger molecules with the factorized bias: the backward pass runs on the trilinear tcgen05 kernels (simplicial_tri.cu has both sides'
+// times; 1.5 to 4 times as fast from one molecule on).
 template <typename Args>
 bool uses_tri_kernels(const Args* a) {
   return a->tokens > kSmallTokens && has_factorized_bias(a);
 }
+// The forward pass runs on them where a call is long enough.  A tile walks all first keys of its rows whatever the batch, up to
+// 100 tokens in at most 26 steps, from 101 on in up to 128 (tri_plan); the warp-level kernel spreads the queries of a small batch
+// over the chip.  The host does not know how full the batch is, so the lines lie between the two extremes.  8 heads, us, trilinear |
+// warp-level, all molecules full | spread from an eighth of the tokens up: 64 tokens x 4 molecules 53 | 32, 53 | 17; x 16 54 | 77,
+// 54 | 43; x 32 98 | 136, 57 | 92.  96 x 4 54 | 60, 54 | 31; x 12 99 | 150, 60 | 87.  128 x 4 254 | 143, 249 | 68; x 12 255 | 334, 250 | 159; x 32 492 | 892, 255 | 364.  192 x 1
+// 257 | 103; x 6 259 | 557, 257 | 257; x 32 1 479 | 2 814, 580 | 1 078.  On either side a molecule's result does not depend on its
+// batch; the two sides round differently, with the same error.  MF_BACKEND_TCGEN05_TILES stays on one side.
+inline bool uses_tri_forward(const MfSimplicialFwdArgs* a) {
+  if (!uses_tri_kernels(a)) return false;
+  const double heads = (double)a->batch * a->heads, n = a->tokens;
+  return a->backend == MF_BACKEND_TCGEN05_TILES || (n <= 100 ? heads * n >= 6144 : heads * n * n * n >= 150e6);
+}
+// Without the bias the forward pass runs on the warp-level kernel, unless a tcgen05 family is asked for: 64 molecules of 20-181 atoms
+// take 0.64 ms on the trilinear kernel against 0.89, but 2 molecules 201 us against 105, and a molecule's result is to be the same in
+// every batch; the backward pass runs on the row-packed kernel (1.98 against 2.26 ms).
 inline bool uses_warp_forward(const MfSimplicialFwdArgs* a) {
   return a->tokens > kSmallTokens && (a->backend == MF_BACKEND_AUTO || has_factorized_bias(a));
 }
@@ -148,8 +161,9 @@ extern "C" size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* a
   int rc;
   if (!wants_tcgen05(a, &rc, "mf_simplicial_fwd")) return 0;
   if (uses_small_kernels(a)) return simplicial_small_order_bytes(a->batch, a->heads, false, a->angle_left || a->message_left);
-  return uses_tri_kernels(a) ? simplicial_tri_fwd_workspace_bytes(*a) : uses_warp_forward(a) ? simplicial_warp_order_bytes(a->batch, a->heads, a->tokens)
-                                                                           : simplicial_sm100_fwd_workspace_bytes(*a);
+  return uses_tri_forward(a)    ? simplicial_tri_fwd_workspace_bytes(*a)
+         : uses_warp_forward(a) ? simplicial_warp_order_bytes(*a)
+                                : simplicial_sm100_fwd_workspace_bytes(*a);
 }
 
 extern "C" size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* a) {
@@ -178,7 +192,7 @@ extern "C" int mf_simplicial_bwd_backend(const MfSimplicialBwdArgs* a) {
 extern "C" int mf_simplicial_fwd_keeps_status(const MfSimplicialFwdArgs* a) {
   if (!a) return 0;
   int rc;
-  return wants_tcgen05(a, &rc, "mf_simplicial_fwd_keeps_status") && !uses_small_kernels(a) && (uses_tri_kernels(a) || !uses_warp_forward(a));
+  return wants_tcgen05(a, &rc, "mf_simplicial_fwd_keeps_status") && !uses_small_kernels(a) && (uses_tri_forward(a) || !uses_warp_forward(a));
 }
 
 extern "C" int mf_simplicial_bwd_keeps_status(const MfSimplicialBwdArgs* a) {
@@ -222,7 +236,7 @@ extern "C" int mf_simplicial_fwd(const MfSimplicialFwdArgs* a, void* stream) {
   if (!tc) return uses_f32_kernels(a) ? simplicial_f32_fwd(*a, s) : simplicial_generic_fwd(*a, s);
   if (uses_small_kernels(a))
     return a->angle_left || a->message_left ? simplicial_small_res_fwd(*a, s) : simplicial_small_fwd(*a, nullptr, s);
-  if (uses_tri_kernels(a) && scratch) return simplicial_tri_fwd(*a, s);
+  if (uses_tri_forward(a) && scratch) return simplicial_tri_fwd(*a, s);
   if (uses_warp_forward(a)) return simplicial_warp_fwd(*a, s);  // with the bias: callers that give no workspace
   return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_fwd(*a, s) : simplicial_rows_fwd(*a, s);
 }
@@ -267,10 +281,10 @@ extern "C" int mf_selftest_simplicial_give_up(const MfSimplicialFwdArgs* fwd, co
   };
   if (fwd) {
     MF_CHECK_ARG(fwd->out && fwd->lse, "%s: null output pointer", name);
-    return run(fwd, mf_simplicial_fwd_workspace_bytes(fwd), simplicial_tri_fwd);
+    return run(fwd, simplicial_tri_fwd_workspace_bytes(*fwd), simplicial_tri_fwd);
   }
   MF_CHECK_ARG(bwd->grad_out && bwd->out && bwd->lse && bwd->dq && bwd->dk1 && bwd->dv1 && bwd->dk2 && bwd->dv2, "%s: null pointer", name);
-  return run(bwd, mf_simplicial_bwd_workspace_bytes(bwd), simplicial_tri_bwd);
+  return run(bwd, simplicial_tri_bwd_workspace_bytes(*bwd), simplicial_tri_bwd);
 }
 
 // ---------------------------------------------------------------------------

@@ -37,7 +37,7 @@ int simplicial_small_order(const uint8_t* key_valid, int batch, int tokens, void
 
 // warp-level forward kernel for 33 to 192 tokens (simplicial_warp_fwd.cu)
 int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
-size_t simplicial_warp_order_bytes(int batch, int heads, int tokens);  // without the bias; optional
+size_t simplicial_warp_order_bytes(const MfSimplicialFwdArgs& a);  // 0 with the bias; optional
 
 // trilinear tcgen05 kernels for 33 to 192 tokens with the factorized bias (simplicial_tri.cu)
 // Its waits give up after `limit` clocks.  The self-test lets them run out: the barriers of kind `withheld` (0-7) expect one arrival

@@ -379,17 +379,18 @@ int queries_per_cta(int bh, int tokens) {
 // given a launch ends with a few large ones: 8 heads, 20-181 atoms, 64 molecules 893 | 851 us heavy first, 24-192 8 molecules 181 |
 // 140, 20-100 32 134 | 107, 20-160 4 76 | 64, 20-64 64 103 | 85, 10-48 64 60 | 48.  The list takes a launch of 3 us (and nothing is
 // gained where all molecules are of one size), so it is made from a wave and a half of CTAs and about 50 us on.
-size_t simplicial_warp_order_bytes(int batch, int heads, int tokens) {
-  const long long bh = (long long)batch * heads;
+size_t simplicial_warp_order_bytes(const MfSimplicialFwdArgs& a) {
+  const int batch = a.batch, tokens = a.tokens;
+  const long long bh = (long long)batch * a.heads;
   const int chunk = queries_per_cta((int)bh, tokens);
-  const bool pays = batch > 3 && batch <= kMostOrdered && bh * ((tokens + chunk - 1) / chunk) >= 222 &&
+  const bool pays = !a.u && batch > 3 && batch <= kMostOrdered && bh * ((tokens + chunk - 1) / chunk) >= 222 &&
                     bh * tokens * tokens * tokens >= 30000000ll;
   return pays ? align_up((size_t)batch * sizeof(int32_t), 256) : 0;
 }
 
 int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   WarpFwdParams p{};
-  const size_t need = a.u ? 0 : simplicial_warp_order_bytes(a.batch, a.heads, a.tokens);
+  const size_t need = simplicial_warp_order_bytes(a);
   if (need > 0 && a.workspace && a.workspace_bytes >= need) {
     int32_t* order = static_cast<int32_t*>(a.workspace);
     simplicial_warp_order_kernel<<<1, 1024, 0, stream>>>(a.pair_key_valid, a.batch, a.tokens, order);

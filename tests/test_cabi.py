@@ -140,3 +140,19 @@ def test_which_calls_leave_a_status_word(backend, tokens, bias, dtype, fwd, bwd)
         assert getattr(L, f"mf_simplicial_{name}_keeps_status")(ctypes.byref(a)) == want
         if want:  # the workspace that such a call asks for holds the word
             assert getattr(L, f"mf_simplicial_{name}_workspace_bytes")(ctypes.byref(a)) >= 256
+
+
+@pytest.mark.parametrize("batch,tokens,backend,trilinear", [
+    (1, 192, "auto", 0), (2, 192, "auto", 0), (3, 192, "auto", 1), (8, 128, "auto", 0), (9, 128, "auto", 1), (18, 101, "auto", 0),
+    (19, 101, "auto", 1), (7, 100, "auto", 0), (8, 100, "auto", 1), (23, 33, "auto", 0), (24, 33, "auto", 1), (1, 33, "tcgen05_tiles", 1),
+])  # fmt: skip
+def test_short_forward_calls_with_the_bias_stay_on_the_warp_level_kernel(batch, tokens, backend, trilinear):
+    """One to a few molecules took up to five times as long on the trilinear kernel (they have no status word elsewhere)."""
+    L = _lib.lib()
+    f = _lib.MfSimplicialFwdArgs(batch=batch, heads=8, tokens=tokens, head_dim=64, dtype=_lib.MF_DTYPE_BF16, backend=_lib.MF_BACKEND[backend])
+    b = _lib.MfSimplicialBwdArgs(batch=batch, heads=8, tokens=tokens, head_dim=64, dtype=_lib.MF_DTYPE_BF16, backend=_lib.MF_BACKEND[backend])
+    for a in (f, b):
+        a.u = a.v_bias = a.w = a.gate = 256  # (never read)
+    assert L.mf_simplicial_fwd_keeps_status(ctypes.byref(f)) == trilinear
+    assert (L.mf_simplicial_fwd_workspace_bytes(ctypes.byref(f)) > 0) == trilinear
+    assert L.mf_simplicial_bwd_keeps_status(ctypes.byref(b)) == 1

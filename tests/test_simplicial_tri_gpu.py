@@ -4,13 +4,21 @@ import torch
 
 from conftest import bf16_allowance
 from matterformer_b200 import _lib
-from matterformer_b200.simplicial import cuda_simplicial_attention_forward
+from matterformer_b200.simplicial import cuda_simplicial_attention_forward, set_backend
 from oracle.simplicial_ref import simplicial_forward_backward
 from test_simplicial_gpu import BIAS_NAMES, NAMES, assert_rel, run_cuda_bias
 from test_simplicial_small_gpu import _case
 from test_simplicial_warp_gpu import _with_bias
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def trilinear_forward():
+    """The default backend keeps forward calls as short as these on the warp-level kernel."""
+    before = set_backend("tcgen05_tiles")
+    yield
+    set_backend(before)
 
 
 def _check(inp, go):
