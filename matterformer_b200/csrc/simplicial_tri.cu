@@ -597,6 +597,8 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
           colp = bcol + (st * G + gs) * zpad;
           wait_on(&sh.bar_full[st], S / kStages);
           rs = bpair[st * kTileM + r];
+          // an infinite w_jk hides the pair from every query whose lse is not NaN; in the columns of padded queries (gate 0) it would be NaN
+          if constexpr (Z == 0) seen = seen && fabsf(rs) < INFINITY;
           rsum = make_float2(0.f, 0.f);
 #pragma unroll 1
           for (int c = (S * C ^ grp) & 1; c < C; c += 2) {

@@ -4,7 +4,7 @@ import torch
 
 from conftest import bf16_allowance
 from matterformer_b200 import _lib
-from matterformer_b200.simplicial import cuda_simplicial_attention_forward, set_backend
+from matterformer_b200.simplicial import cuda_simplicial_attention_backward, cuda_simplicial_attention_forward, set_backend
 from oracle.simplicial_ref import simplicial_forward_backward
 from test_simplicial_gpu import BIAS_NAMES, NAMES, assert_rel, run_cuda_bias
 from test_simplicial_small_gpu import _case
@@ -61,6 +61,36 @@ def test_exact_maxima(shift):
     assert_rel(y, out_ref, tol["out"], "out")
     for n in NAMES:
         assert_rel(grads[n], g_ref[n], tol[n], f"d{n}")
+
+
+def _run(t, valid, grad, need=(True,) * 4, pair_valid=None):
+    """Forward and backward on device tensors {name: tensor}: every output as a list."""
+    kw = dict(query_valid=valid, pair_key_valid=valid, pair_valid=pair_valid, **{n: t[n] for n in BIAS_NAMES})
+    heads = [t[n] for n in NAMES]
+    out, lse, out32 = cuda_simplicial_attention_forward(*heads, **kw)
+    grads = cuda_simplicial_attention_backward(grad, *heads, out32, lse, **kw, **dict(zip(("need_du", "need_dv_bias", "need_dw", "need_dgate"), need)))
+    return [out, lse, out32, *grads[:9]]
+
+
+@pytest.mark.parametrize("value", [torch.finfo(torch.float32).min, float("-inf")])
+def test_a_bias_that_hides_pairs(value):
+    """The lowest value of the type and minus infinity in w, under a positive gate, hide a pair of keys as the mask does."""
+    inp, go = _case(2, 2, 90, seed=90, scale=0.4, lo=60)
+    _with_bias(inp, 90)
+    inp.gate = inp.gate.abs().clamp(0.05, 0.9)
+    hidden = torch.rand(2, 1, 90, 90, generator=torch.Generator().manual_seed(9)) < 0.3
+    hidden[:, :, 0] = False  # (every query keeps a pair)
+    inp.w = inp.w.masked_fill(hidden, value)
+    out_ref, g_ref = simplicial_forward_backward(inp, go)
+    t = {n: getattr(inp, n).cuda() for n in (*NAMES, *BIAS_NAMES)}  # (the bias in fp32: the lowest value is infinite in bf16)
+    t.update({n: t[n].bfloat16() for n in NAMES})
+    _, _, y, *grads = (x.float().cpu() for x in _run(t, inp.query_valid.cuda(), go.cuda().bfloat16()))
+    assert_rel(y, out_ref, 2e-2, "out")
+    for n, got in zip(NAMES + BIAS_NAMES, grads):
+        if n == "gate" and value == float("-inf"):  # 0 * infinity, as in the torch path
+            assert got[g_ref[n].isfinite()].isfinite().all()
+        else:
+            assert_rel(got, g_ref[n], 2.5e-2, f"d{n}")
 
 
 def test_forward_without_workspace(monkeypatch):
