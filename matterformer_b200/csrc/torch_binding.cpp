@@ -57,6 +57,17 @@ const float* fptr(const Tensor& t) { return t.defined() && t.numel() ? t.const_d
 float* grad_ptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
 Tensor bytes(int64_t n, const Tensor& like) { return n ? at::empty({n}, like.options().dtype(at::kByte)) : Tensor(); }
 
+// The workspace that a call asks for.  On tensor-core kernels without a status word it only holds the list of heavy molecules, which
+// the caller may not want.
+size_t workspace_bytes(const MfSimplicialFwdArgs& a, bool heavy_first) {
+  const bool leave_out = !heavy_first && mf_simplicial_fwd_backend(&a) == MF_BACKEND_TCGEN05 && !mf_simplicial_fwd_keeps_status(&a);
+  return leave_out ? 0 : mf_simplicial_fwd_workspace_bytes(&a);
+}
+size_t workspace_bytes(const MfSimplicialBwdArgs& a, bool heavy_first) {
+  const bool leave_out = !heavy_first && mf_simplicial_bwd_backend(&a) == MF_BACKEND_TCGEN05 && !mf_simplicial_bwd_keeps_status(&a);
+  return leave_out ? 0 : mf_simplicial_bwd_workspace_bytes(&a);
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // 2-simplicial attention
 // ---------------------------------------------------------------------------------------------------------------------
@@ -84,7 +95,7 @@ struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
                           const Tensor& v2, const Tensor& qv, const Tensor& kv, const OptTensor& pv, const OptTensor& u,
                           const OptTensor& v, const OptTensor& w, const OptTensor& gate, const OptTensor& al, const OptTensor& ar,
                           const OptTensor& ag, const OptTensor& ml, const OptTensor& mr, const OptTensor& basis, int64_t precision,
-                          int64_t backend) {
+                          int64_t backend, bool heavy_first) {
     auto or_none = [](const OptTensor& t) { return t ? *t : Tensor(); };
     const std::array<Tensor, kInputs> t = {q, k1, v1, k2, v2, qv, kv, or_none(pv), or_none(u), or_none(v), or_none(w), or_none(gate),
                                            or_none(al), or_none(ar), or_none(ag), or_none(ml), or_none(mr), or_none(basis)};
@@ -96,13 +107,12 @@ struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
     const Tensor out = q.scalar_type() == at::kFloat ? out32 : at::empty_like(q);
     a.out = out32.data_ptr<float>(), a.lse = lse.data_ptr<float>();
     a.out_cast = out.is_same(out32) ? nullptr : out.data_ptr();
-    const Tensor ws = bytes(mf_simplicial_fwd_workspace_bytes(&a), q);
+    const Tensor ws = bytes(workspace_bytes(a, heavy_first), q);
     if (ws.defined()) a.workspace = ws.data_ptr(), a.workspace_bytes = ws.numel();
     check(mf_simplicial_fwd(&a, c10::cuda::getCurrentCUDAStream().stream()));
     if (mf_simplicial_fwd_backend(&a) == MF_BACKEND_TCGEN05)
       remember_status(ws.defined() && mf_simplicial_fwd_keeps_status(&a) ? OptTensor(ws) : std::nullopt);
-    ctx->saved_data["precision"] = precision;
-    ctx->saved_data["backend"] = backend;
+    ctx->saved_data["call"] = precision | backend << 8 | (int64_t)heavy_first << 16;
     tensor_list saved(t.begin(), t.end());
     saved.push_back(out32);
     saved.push_back(lse);
@@ -118,9 +128,10 @@ struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
     const c10::cuda::CUDAGuard guard(q.device());
     const Tensor go = grad_out[0].to(q.scalar_type()).contiguous();
     MfSimplicialBwdArgs a{};
-    fill_common(a, t, ctx->saved_data["precision"].toInt(), ctx->saved_data["backend"].toInt());
+    const int64_t call = ctx->saved_data["call"].toInt();
+    fill_common(a, t, call & 255, call >> 8 & 255);
     a.grad_out = go.const_data_ptr(), a.out = out32.const_data_ptr<float>(), a.lse = lse.const_data_ptr<float>();
-    tensor_list g(kInputs + 2);
+    tensor_list g(kInputs + 3);  // (one for each argument of forward)
     for (int i = Q; i <= V2; ++i) g[i] = at::empty_like(q);
     a.dq = g[Q].data_ptr(), a.dk1 = g[K1].data_ptr(), a.dv1 = g[V1].data_ptr(), a.dk2 = g[K2].data_ptr(), a.dv2 = g[V2].data_ptr();
     // edges of the node are counted over the tensors that were given
@@ -145,7 +156,7 @@ struct SimplicialAttention : torch::autograd::Function<SimplicialAttention> {
         a.message_coeff = coeff.data_ptr<float>();
       }
     }
-    const Tensor ws = bytes(mf_simplicial_bwd_workspace_bytes(&a), q);
+    const Tensor ws = bytes(workspace_bytes(a, call >> 16), q);
     if (ws.defined()) a.workspace = ws.data_ptr(), a.workspace_bytes = ws.numel();
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     check(mf_simplicial_bwd(&a, stream));
@@ -167,7 +178,7 @@ bool ready(const Tensor& t, const Tensor& like, at::ScalarType type, at::IntArra
 std::optional<Tensor> simplicial_attention(const Tensor& q, const Tensor& k1, const Tensor& v1, const Tensor& k2, const Tensor& v2,
                                            const Tensor& qv, const Tensor& kv, const OptTensor& pv, std::vector<OptTensor> bias,
                                            std::vector<OptTensor> angle, std::vector<OptTensor> message, int64_t precision,
-                                           int64_t backend, int64_t max_rank) {
+                                           int64_t backend, int64_t max_rank, bool heavy_first) {
   if (!q.is_cuda() || q.dim() != 4 || dtype_code(q) < 0 || !q.is_contiguous()) return std::nullopt;
   for (const Tensor* t : {&k1, &v1, &k2, &v2})
     if (!ready(*t, q, q.scalar_type(), q.sizes())) return std::nullopt;
@@ -202,7 +213,7 @@ std::optional<Tensor> simplicial_attention(const Tensor& q, const Tensor& k1, co
   }
   bias.resize(4), angle.resize(3), message.resize(3);
   return SimplicialAttention::apply(q, k1, v1, k2, v2, qv, kv, pv, bias[0], bias[1], bias[2], bias[3], angle[0], angle[1], angle[2],
-                                    message[0], message[1], message[2], precision, backend);
+                                    message[0], message[1], message[2], precision, backend, heavy_first);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from matterformer_b200 import _lib
-from matterformer_b200.simplicial import cuda_simplicial_attention_backward, cuda_simplicial_attention_forward, simplicial_attention_packed
+from matterformer_b200.simplicial import cuda_simplicial_attention_backward, cuda_simplicial_attention_forward, simplicial_attention_cuda, simplicial_attention_packed
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +72,35 @@ def test_forward_above_32_tokens_in_either_order(monkeypatch, B, H, N):
     ordered = cuda_simplicial_attention_forward(*heads, **kw)
     _without(monkeypatch)
     assert all(torch.equal(x, y) for x, y in zip(ordered, cuda_simplicial_attention_forward(*heads, **kw)))
+
+
+@pytest.mark.parametrize("N,batch", [(29, 300), (64, 64)])
+def test_a_caller_may_leave_the_list_out(N, batch):
+    """Through the operators on heads and on the packed projection: no launch of a list, the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    heads = [torch.randn(batch, 8, N, 64, generator=g, device="cuda").bfloat16().requires_grad_(True) for _ in range(5)]
+    valid = torch.arange(N, device="cuda")[None] < torch.randint(1, N + 1, (batch,), generator=g, device="cuda")[:, None]
+    proj = torch.randn(batch, N, 5 * 8 * 64, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    kw = dict(query_valid=valid, pair_key_valid=valid)
+
+    def run(heavy_first):
+        out = simplicial_attention_cuda(*heads, **kw, heavy_first=heavy_first)
+        results = [out, *torch.autograd.grad(out, heads, torch.ones_like(out))]
+        if N <= 32:
+            out = simplicial_attention_packed(proj, heads=8, **kw, heavy_first=heavy_first)
+            results += [out, *torch.autograd.grad(out, [proj], torch.ones_like(out))]
+        out, lse, out32 = cuda_simplicial_attention_forward(*heads, **kw, pair_valid=None, heavy_first=heavy_first)
+        grads = cuda_simplicial_attention_backward(out, *heads, out32, lse, **kw, pair_valid=None, heavy_first=heavy_first)
+        return [*results, out, lse, *grads[:5]]
+
+    def lists(heavy_first):
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            results = run(heavy_first)
+            torch.cuda.synchronize()
+        return sum(e.count for e in prof.key_averages() if "_order_kernel" in e.key and "simplicial" in e.key), results
+
+    run(True)
+    made, ordered = lists(True)
+    none, given = lists(False)
+    assert made > 0 and none == 0
+    assert all(torch.equal(a, b) for a, b in zip(ordered, given))
