@@ -1,4 +1,6 @@
 """Trilinear tcgen05 kernels (factorized bias, 33 to 192 tokens): unequal extents, empty molecules, exact maxima, no workspace."""
+from dataclasses import replace
+
 import pytest
 import torch
 
@@ -63,6 +65,21 @@ def test_exact_maxima(shift):
         assert_rel(grads[n], g_ref[n], tol[n], f"d{n}")
 
 
+@pytest.mark.parametrize("shift", [1.5, -1.5])
+def test_bias_gradients_of_sharp_logits(shift):
+    """Each pass forms the logits from products of another pair of the three sets, rounded for itself: the gradients of gate and u come
+    from other roundings than those of w and v.  Allowed is what the torch path in bf16, which rounds the logits too, makes of it."""
+    inp, go = _case(2, 2, 70, seed=70, scale=0.2, lo=35, shift=shift)
+    _with_bias(inp, 70)
+    _, g_ref = simplicial_forward_backward(inp, go)
+    low = replace(inp, **{n: getattr(inp, n).bfloat16() for n in NAMES})
+    _, g_low = simplicial_forward_backward(low, go.bfloat16(), fp32_core=False)
+    _, grads = run_cuda_bias(inp, go, dtype=torch.bfloat16, precision="bf16_tc")
+    for n in BIAS_NAMES:
+        allowed = (g_low[n].float() - g_ref[n]).abs().max() / g_ref[n].abs().max()
+        assert_rel(grads[n], g_ref[n], max(2.5e-2, float(allowed)), f"d{n}")
+
+
 def _run(t, valid, grad, need=(True,) * 4, pair_valid=None):
     """Forward and backward on device tensors {name: tensor}: every output as a list."""
     kw = dict(query_valid=valid, pair_key_valid=valid, pair_valid=pair_valid, **{n: t[n] for n in BIAS_NAMES})
@@ -70,6 +87,29 @@ def _run(t, valid, grad, need=(True,) * 4, pair_valid=None):
     out, lse, out32 = cuda_simplicial_attention_forward(*heads, **kw)
     grads = cuda_simplicial_attention_backward(grad, *heads, out32, lse, **kw, **dict(zip(("need_du", "need_dv_bias", "need_dw", "need_dgate"), need)))
     return [out, lse, out32, *grads[:9]]
+
+
+def _device_case(B, H, N, seed, lo):
+    inp, go = _case(B, H, N, seed=seed, scale=0.4, lo=lo)
+    _with_bias(inp, seed)
+    t = {n: getattr(inp, n).cuda() for n in (*NAMES, *BIAS_NAMES)}
+    t.update({n: t[n].bfloat16() for n in NAMES})
+    return t, inp.query_valid.cuda(), go.cuda().bfloat16()
+
+
+@pytest.mark.parametrize("fill", [float("nan"), float("inf")])
+@pytest.mark.parametrize("N", [50, 132])
+def test_padded_tokens_may_hold_anything(N, fill):
+    """In the rows of the heads and of grad_out, and in every entry of the bias that a padded token has a part in."""
+    t, valid, go = _device_case(3, 2, N, seed=N, lo=N // 3)
+    valid[1, 2] = False  # a hole too: columns are then copied one by one
+    clean = _run(t, valid, go)
+    pad = ~valid[:, None, :]
+    dirty = {n: x.masked_fill(pad[..., None], fill) for n, x in t.items() if x.ndim == 4 and n in NAMES}
+    dirty.update({n: t[n].masked_fill(pad[..., None] | pad[..., None, :], fill) for n in ("u", "v_bias", "w")})
+    dirty["gate"] = t["gate"].masked_fill(pad, fill)
+    for a, b in zip(clean, _run(dirty, valid, go.masked_fill(pad[..., None], fill))):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("value", [torch.finfo(torch.float32).min, float("-inf")])
@@ -91,6 +131,27 @@ def test_a_bias_that_hides_pairs(value):
             assert got[g_ref[n].isfinite()].isfinite().all()
         else:
             assert_rel(got, g_ref[n], 2.5e-2, f"d{n}")
+
+
+@pytest.mark.parametrize("B,H,N,pick", [(5, 2, 192, slice(2, 3)), (1100, 1, 36, slice(1030, 1037))])
+def test_a_molecule_alone_and_in_a_batch(B, H, N, pick):
+    """The same bits, also from a batch of more molecules than the schedule's block has threads."""
+    t, valid, go = _device_case(B, H, N, seed=B, lo=1)
+    valid[B // 2] = False
+    whole = _run(t, valid, go)
+    part = _run({n: x[pick].contiguous() for n, x in t.items()}, valid[pick].contiguous(), go[pick].contiguous())
+    assert all(torch.isfinite(x).all() for x in whole)
+    for a, b in zip(whole, part):
+        assert torch.equal(a[pick], b)
+
+
+def test_each_bias_gradient_alone():
+    t, valid, go = _device_case(2, 2, 77, seed=3, lo=40)
+    whole = _run(t, valid, go)
+    for i in range(4):
+        some = _run(t, valid, go, need=tuple(j == i for j in range(4)))
+        for k, (a, b) in enumerate(zip(whole, some)):
+            assert torch.equal(a, b) if k < 8 or k == 8 + i else b is None
 
 
 def test_forward_without_workspace(monkeypatch):
