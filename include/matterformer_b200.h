@@ -249,9 +249,10 @@ int mf_simplicial_noalloc_status(int32_t* host_status, void* stream);
  * waited to status[1] (two device int32) and returns: the path every tensor-core kernel takes when a hand-off never
  * arrives, exercised without hanging or faulting anything. */
 int mf_selftest_wait_timeout(int32_t* status, int64_t limit_cycles, void* stream);
-/* Self-test of what an expired wait leaves behind: a forward or a backward call (the other pointer NULL) on the trilinear kernels
- * (factorized bias, 33 to 192 tokens, with its workspace) in which one kind of hand-off (`withheld`, 0 to 7) never completes
- * and waits give up after `limit_cycles`.  The call ends with MF_ERR_DEVICE_TIMEOUT in the status word and zeros in its outputs. */
+/* Self-test of what an expired wait leaves behind: a forward or a backward call (the other pointer NULL), with its workspace, in
+ * which one kind of hand-off (`withheld`) never completes and waits give up after `limit_cycles`.  It serves the trilinear kernels
+ * (factorized bias, 33 to 192 tokens; kinds 0 to 7) and the row-packed forward kernel (MF_BACKEND_TCGEN05; 0 to 5).  The call ends
+ * with MF_ERR_DEVICE_TIMEOUT in the status word and zeros in its outputs. */
 int mf_selftest_simplicial_give_up(const MfSimplicialFwdArgs* fwd, const MfSimplicialBwdArgs* bwd, int32_t withheld,
                                    int64_t limit_cycles, void* stream);
 

@@ -268,23 +268,24 @@ extern "C" int mf_selftest_simplicial_give_up(const MfSimplicialFwdArgs* fwd, co
                                               int64_t limit_cycles, void* stream) {
   const char* name = "mf_selftest_simplicial_give_up";
   MF_CHECK_ARG((fwd != nullptr) != (bwd != nullptr), "%s: one of the two argument structs", name);
-  MF_CHECK_ARG(withheld >= 0 && withheld < 8, "%s: barrier kind %d not in [0, 8)", name, (int)withheld);
   MF_CHECK_ARG(limit_cycles >= 1 && limit_cycles <= (1ll << 31), "%s: limit must be in [1, 2^31] clocks", name);
-  const TriWaits waits{(long long)limit_cycles, withheld};
-  auto run = [&](const auto* a, size_t need, auto kernels) {
+  const BoundedWaits waits{(long long)limit_cycles, withheld};
+  auto run = [&](const auto* a, int kinds, size_t need, auto kernels) {
     int rc = check_common(a, name);
     if (rc != MF_OK || (rc = check_bias(a, name)) != MF_OK) return rc;
-    MF_CHECK_ARG(wants_tcgen05(a, &rc, name) && uses_tri_kernels(a) && a->batch > 0 && a->heads > 0 && a->workspace &&
-                     a->workspace_bytes >= need,
-                 "%s: only calls that the trilinear kernels serve, with their workspace", name);
+    const bool served = wants_tcgen05(a, &rc, name) && a->batch > 0 && a->heads > 0 && (uses_tri_kernels(a) || a->backend == MF_BACKEND_TCGEN05);
+    MF_CHECK_ARG(served && a->workspace && a->workspace_bytes >= need, "%s: not a call of these kernels, or no workspace", name);
+    MF_CHECK_ARG(withheld >= 0 && withheld < kinds, "%s: kind of hand-off %d not in [0, %d)", name, (int)withheld, kinds);
     return kernels(*a, static_cast<cudaStream_t>(stream), waits);
   };
   if (fwd) {
     MF_CHECK_ARG(fwd->out && fwd->lse, "%s: null output pointer", name);
-    return run(fwd, simplicial_tri_fwd_workspace_bytes(*fwd), simplicial_tri_fwd);
+    return has_factorized_bias(fwd) ? run(fwd, 8, simplicial_tri_fwd_workspace_bytes(*fwd), simplicial_tri_fwd)
+                                    : run(fwd, 6, simplicial_sm100_fwd_workspace_bytes(*fwd), simplicial_rows_fwd);
   }
   MF_CHECK_ARG(bwd->grad_out && bwd->out && bwd->lse && bwd->dq && bwd->dk1 && bwd->dv1 && bwd->dk2 && bwd->dv2, "%s: null pointer", name);
-  return run(bwd, simplicial_tri_bwd_workspace_bytes(*bwd), simplicial_tri_bwd);
+  MF_CHECK_ARG(has_factorized_bias(bwd), "%s: a backward call needs the bias", name);
+  return run(bwd, 8, simplicial_tri_bwd_workspace_bytes(*bwd), simplicial_tri_bwd);
 }
 
 // ---------------------------------------------------------------------------

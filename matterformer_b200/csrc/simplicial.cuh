@@ -7,6 +7,13 @@
 
 namespace mf {
 
+// Waits of a kernel give up after `limit` clocks.  The self-test lets them run out: the barriers of kind `withheld` (as the kernel
+// numbers them) expect one arrival more than there are.
+struct BoundedWaits {
+  long long limit = 1ll << 31;  // kWaitLimitCycles
+  int withheld = -1;
+};
+
 // fp32 CUDA-core kernels (simplicial_generic.cu)
 int simplicial_generic_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 int simplicial_generic_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
@@ -40,19 +47,13 @@ int simplicial_warp_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
 size_t simplicial_warp_order_bytes(const MfSimplicialFwdArgs& a);  // 0 with the bias; optional
 
 // trilinear tcgen05 kernels for 33 to 192 tokens with the factorized bias (simplicial_tri.cu)
-// Its waits give up after `limit` clocks.  The self-test lets them run out: the barriers of kind `withheld` (0-7) expect one arrival
-// more than there are.
-struct TriWaits {
-  long long limit = 1ll << 31;  // kWaitLimitCycles
-  int withheld = -1;
-};
-int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, TriWaits waits = {});
-int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, TriWaits waits = {});
+int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, BoundedWaits waits = {});
+int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, BoundedWaits waits = {});
 size_t simplicial_tri_fwd_workspace_bytes(const MfSimplicialFwdArgs& a);
 size_t simplicial_tri_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 
 // row-packed tcgen05 kernels (simplicial_rows_fwd.cu, simplicial_rows_bwd.cu); same problems as the kernels above
-int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);
+int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, BoundedWaits waits = {});
 int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
 size_t simplicial_rows_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 

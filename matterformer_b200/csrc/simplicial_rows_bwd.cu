@@ -367,6 +367,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
       issue_sums();
     }
     umma_commit(&bar_fin);
+    if (!mbar_wait(&bar_fin, 0)) bad = true;  // whoever gave up, no product may be in flight when tensor memory is given back
   } else if (warp == 9) {
     // ------------------------------------------------------------------ loader
     // Stages, up to kRowStages steps ahead of the workers, the k1 and v1 rows of each step's first keys (bf16, for
@@ -707,7 +708,10 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
 
   tc_fence_before_sync();
   bad = __syncthreads_or(bad) != 0;
-  if (bad && tid == 0) atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
+  if (bad && tid == 0) {
+    if (p.use_tma) mbar_wait(&bar_kv, 0);  // the copies may be what did not arrive
+    atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
+  }
   if (warp == 0) tmem_dealloc(tmem, kBwdTmemCols);
 }
 

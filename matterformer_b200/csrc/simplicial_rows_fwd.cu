@@ -85,6 +85,7 @@ struct RowsFwdParams {
   int32_t* status;
   int H, N, tiles_max;
   int use_tma;
+  BoundedWaits waits;
   CUtensorMap tm_k2;  // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle
   CUtensorMap tm_v2;
 };
@@ -102,7 +103,7 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
 __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_constant__ RowsFwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t bar_a[2], bar_s[2], bar_p[2], bar_w[2], bar_kv;
+  __shared__ uint64_t bar_a[2], bar_s[2], bar_p[2], bar_w[2], bar_kv, bar_drain;
   __shared__ uint64_t bar_full[kRowStages], bar_empty[kRowStages];  // loader warp <-> row owners
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t kmask[kMaskWords];
@@ -142,17 +143,19 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_
 
   // ---- set-up: barriers, tensor memory, key masks, first-key list, operand tiles
   if (tid == 0) {
+    auto count = [&](int which, int n) { return (uint32_t)(n + (p.waits.withheld == which)); };  // (see BoundedWaits)
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bar_a[i], kWorkerWarps);  // one arrival per row-owner warp
-      mbar_init(&bar_s[i], 1);
-      mbar_init(&bar_p[i], kWorkerWarps);
-      mbar_init(&bar_w[i], 1);
+      mbar_init(&bar_a[i], count(0, kWorkerWarps));  // one arrival per row-owner warp
+      mbar_init(&bar_s[i], count(1, 1));
+      mbar_init(&bar_p[i], count(2, kWorkerWarps));
+      mbar_init(&bar_w[i], count(3, 1));
     }
     for (int i = 0; i < kRowStages; ++i) {
-      mbar_init(&bar_full[i], 1);
-      mbar_init(&bar_empty[i], kWorkerWarps);
+      mbar_init(&bar_full[i], count(4, 1));
+      mbar_init(&bar_empty[i], count(5, kWorkerWarps));
     }
     mbar_init(&bar_kv, 1);
+    mbar_init(&bar_drain, 1);
     mbar_fence_init();
   }
   if (warp == 0) {
@@ -232,7 +235,7 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_
   const uint32_t tmem = tmem_base_s;
 
   auto wait_on = [&](uint64_t* bar, uint32_t ph) {
-    if (!bad) bad = !mbar_wait(bar, ph);
+    if (!bad) bad = !mbar_wait_for(bar, ph, p.waits.limit);
   };
 
   if (warp >= kWorkerWarps) {
@@ -270,6 +273,9 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_
       tc_fence_after_sync();
       issue_pv(s);
     }
+    // Whoever gave up, no product may be in flight when tensor memory is given back
+    umma_commit(&bar_drain);
+    if (!mbar_wait_for(&bar_drain, 0, p.waits.limit)) bad = true;
   } else if (warp == kLoaderWarp) {
     // ------------------------------------------------------------------ loader
     // Stages, up to kRowStages steps ahead, the k1 rows of each step's first keys (bf16, for the operand build) and
@@ -310,6 +316,7 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_
       if (lane == 0) mbar_arrive(&bar_full[stg]);
     }
   }
+    bad = __syncthreads_or(bad) != 0;  // (the row owners' barrier before they store)
   } else {
     // ------------------------------------------------------------------ row owners
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegWorker));
@@ -570,6 +577,7 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_
         l_row = l_all;
       }
     }
+    bad = __syncthreads_or(bad) != 0;  // a wait of any thread that has expired makes the tile's rows zeros
     if (g == 0 && i < n_queries) {
       const bool have = row_ok && l_row > 0.f && !bad;
       const float inv = have ? 1.f / l_row : 0.f;
@@ -595,14 +603,17 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_rows_fwd_kernel(const __grid_
   }
 
   tc_fence_before_sync();
-  bad = __syncthreads_or(bad) != 0;
-  if (bad && tid == 0) atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
+  __syncthreads();
+  if (bad && tid == 0) {
+    if (p.use_tma) mbar_wait(&bar_kv, 0);  // the copies may be what did not arrive
+    atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
+  }
   if (warp == 0) tmem_dealloc(tmem, kFwdTmemCols);
 }
 
 }  // namespace
 
-int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
+int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, BoundedWaits waits) {
   size_t info_off, order_off;
   simplicial_schedule_layout(a.batch, &info_off, &order_off);
   char* ws = static_cast<char*>(a.workspace);
@@ -626,6 +637,7 @@ int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) {
   p.H = a.heads;
   p.N = a.tokens;
   p.tiles_max = cached_max_row_tiles(a.tokens);
+  p.waits = waits;
   p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, a.batch * a.heads) &&
               make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, a.batch * a.heads);
   int rc = launch_schedule(a.query_valid, a.pair_key_valid, a.batch, a.tokens, info, order, p.status, stream);

@@ -120,7 +120,7 @@ struct TriParams {
   const int2* items;              // [0].x = count, then {batch | pass << 16 | tile << 20, rows | tiles << 8}
   int32_t* status;
   int H, N;
-  TriWaits waits;
+  BoundedWaits waits;
 };
 
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
@@ -189,7 +189,7 @@ __device__ __forceinline__ void tri_tile(const TriParams& p, TriShared& sh, uint
   const int C = (units + 3) >> 2, per = units / C, extra = units % C;  // chunks of a step: per or per + 1 units
 
   if (tid == 0) {
-    auto count = [&](int which, int n) { return (uint32_t)(n + (p.waits.withheld == which)); };  // (see TriWaits)
+    auto count = [&](int which, int n) { return (uint32_t)(n + (p.waits.withheld == which)); };  // (see BoundedWaits)
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sh.bar_a[i], count(0, kRowWarps));
       mbar_init(&sh.bar_free[i], count(1, 1));
@@ -978,7 +978,7 @@ int launch_tri(Kernel kernel, const TriParams& p, const TriLayout& l, int batch,
 size_t simplicial_tri_fwd_workspace_bytes(const MfSimplicialFwdArgs& a) { return tri_layout(a.batch, a.heads, a.tokens, false).total; }
 size_t simplicial_tri_bwd_workspace_bytes(const MfSimplicialBwdArgs& a) { return tri_layout(a.batch, a.heads, a.tokens, true).total; }
 
-int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, TriWaits waits) {
+int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, BoundedWaits waits) {
   const TriLayout l = tri_layout(a.batch, a.heads, a.tokens, false);
   TriParams p{};
   p.waits = waits;
@@ -989,7 +989,7 @@ int simplicial_tri_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, TriWai
                     "simplicial_tri_fwd_kernel");
 }
 
-int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, TriWaits waits) {
+int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, BoundedWaits waits) {
   const TriLayout l = tri_layout(a.batch, a.heads, a.tokens, true);
   TriParams p{};
   p.waits = waits;

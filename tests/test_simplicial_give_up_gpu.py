@@ -1,4 +1,4 @@
-"""What an expired device-side wait of the trilinear kernels leaves behind: the status, zeros, and a device that goes on."""
+"""What an expired device-side wait leaves behind: the status, zeros, and a device that goes on."""
 import ctypes
 
 import pytest
@@ -10,14 +10,15 @@ pytestmark = pytest.mark.gpu
 B, H, N = 2, 2, 64  # 32 and 14 steps a tile: more than the stages of the bias operands
 
 
-def _call(cls, **outputs):
+def _call(cls, backend="tcgen05_tiles", **outputs):
     g = torch.Generator(device="cuda").manual_seed(1)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
     t = {n: rnd(B, H, N, 64).bfloat16() for n in ("q", "k1", "v1", "k2", "v2")}
-    t.update(u=rnd(B, H, N, N), v_bias=rnd(B, H, N, N), w=rnd(B, H, N, N), gate=rnd(B, H, N))
+    if backend == "tcgen05_tiles":  # the trilinear kernels
+        t.update(u=rnd(B, H, N, N), v_bias=rnd(B, H, N, N), w=rnd(B, H, N, N), gate=rnd(B, H, N))
     valid = (torch.arange(N, device="cuda")[None] < torch.tensor([[N], [40]], device="cuda")).view(torch.uint8)
     t.update(query_valid=valid, pair_key_valid=valid, **outputs)
-    a = cls(batch=B, heads=H, tokens=N, head_dim=64, dtype=_lib.MF_DTYPE_BF16, backend=_lib.MF_BACKEND["tcgen05_tiles"])
+    a = cls(batch=B, heads=H, tokens=N, head_dim=64, dtype=_lib.MF_DTYPE_BF16, backend=_lib.MF_BACKEND[backend])
     for name, x in t.items():
         setattr(a, name, x.data_ptr())
     size = "mf_simplicial_fwd_workspace_bytes" if cls is _lib.MfSimplicialFwdArgs else "mf_simplicial_bwd_workspace_bytes"
@@ -26,9 +27,10 @@ def _call(cls, **outputs):
     return a, t, ws
 
 
-@pytest.mark.parametrize("withheld", range(8))
-@pytest.mark.parametrize("backward", [False, True], ids=["forward", "backward"])
-def test_a_hand_off_that_never_completes(backward, withheld):
+@pytest.mark.parametrize("kernel,withheld", [*(("forward", i) for i in range(8)), *(("backward", i) for i in range(8)),
+                                             *(("row-packed forward", i) for i in range(6))])  # fmt: skip
+def test_a_hand_off_that_never_completes(kernel, withheld):
+    backward = kernel == "backward"
     nan = lambda *s, dtype=torch.float32: torch.full(s, float("nan"), dtype=dtype, device="cuda")  # noqa: E731
     bf = dict(dtype=torch.bfloat16)
     if backward:
@@ -39,7 +41,7 @@ def test_a_hand_off_that_never_completes(backward, withheld):
         a, keep, ws = _call(_lib.MfSimplicialBwdArgs, **outputs, **saved)
     else:
         outputs = dict(out=nan(B, H, N, 64), out_cast=nan(B, H, N, 64, **bf), lse=nan(B, H, N))
-        a, keep, ws = _call(_lib.MfSimplicialFwdArgs, **outputs)
+        a, keep, ws = _call(_lib.MfSimplicialFwdArgs, "tcgen05" if kernel == "row-packed forward" else "tcgen05_tiles", **outputs)
     ref, stream = ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     _lib.check(_lib.lib().mf_selftest_simplicial_give_up(None if backward else ref, ref if backward else None, withheld, 20_000, stream))
     assert ws[:4].view(torch.int32).item() == _lib.MF_ERR_DEVICE_TIMEOUT
