@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(TcShape<MODE>::kThreads, TcShape<MODE>::kCtasP
   constexpr int kStages = Sh::kStages, kTcThreads = Sh::kThreads, kC = Sh::kCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t bar_own, bar_s[2], bar_p[2], bar_w[2];
+  __shared__ uint64_t bar_own, bar_s[2], bar_p[2], bar_w[2], bar_drain[2];
   __shared__ uint64_t bar_full[kStages], bar_free[kStages];
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t present[kMaxPartTiles];  // per partner tile: bit (owner 32-row block * 2 + partner 32-row block)
@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(TcShape<MODE>::kThreads, TcShape<MODE>::kCtasP
       mbar_init(&bar_s[i], 1);
       mbar_init(&bar_p[i], Sh::kWorkerWarps);  // one arrival per row-owner warp
       mbar_init(&bar_w[i], 1);
+      mbar_init(&bar_drain[i], 1);
     }
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&bar_full[i], 1);
@@ -249,12 +250,17 @@ __global__ void __launch_bounds__(TcShape<MODE>::kThreads, TcShape<MODE>::kCtasP
       tma_load_rows(smem + Sh::kOffOwnA + c * kBoxRows * 128, &p.tm_own_a, row0 + c * kBoxRows, bh, &bar_own);
       if (MODE != T_FWD) tma_load_rows(smem + Sh::kOffOwnB + c * kBoxRows * 128, &p.tm_own_b, row0 + c * kBoxRows, bh, &bar_own);
     }
-    for (int t = 0; t < kStages && t < nsteps; ++t) load_stage(t);
-    for (int t = kStages; t < nsteps; ++t) {  // a stage is free once the products of its previous step have completed
-      wait_on(&bar_free[t % kStages], ((t / kStages) - 1) & 1);
+    int loaded = min(kStages, nsteps);
+    for (int t = 0; t < loaded; ++t) load_stage(t);
+    for (; loaded < nsteps; ++loaded) {  // a stage is free once the products of its previous step have completed
+      wait_on(&bar_free[loaded % kStages], ((loaded / kStages) - 1) & 1);
       if (bad) break;
-      load_stage(t);
+      load_stage(loaded);
     }
+    // whoever gave up, no copy may be in flight when the CTA ends
+    if (!mbar_wait(&bar_own, 0)) bad = true;
+    for (int t = max(0, loaded - kStages); t < loaded; ++t)
+      if (!mbar_wait(&bar_full[t % kStages], (t / kStages) & 1)) bad = true;
   } else if (tid == Sh::kWorkers || tid == Sh::kWorkers + 32) {
     // ------------------------------------------------------------------ MMAs
     // Two issuing threads in warps of different schedulers, so that neither the issue slots of one scheduler nor the
@@ -303,6 +309,10 @@ __global__ void __launch_bounds__(TcShape<MODE>::kThreads, TcShape<MODE>::kCtasP
         umma_commit(&bar_s[buf]);
       }
     }
+    // nor a product when tensor memory is given back
+    uint64_t* drain = &bar_drain[tid != Sh::kWorkers];
+    umma_commit(drain);
+    if (!mbar_wait(drain, 0)) bad = true;
   } else if (tid < Sh::kWorkers) {
     // ------------------------------------------------------------------ row owners
     const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
