@@ -444,6 +444,7 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
         st ^= 1;
       }
       umma_commit(&bar_fin);
+      if (!mbar_wait(&bar_fin, 0)) bad = true;  // whoever gave up, no product may be in flight when tensor memory is given back
     }
   } else {
     // ------------------------------------------------------------------ workers
@@ -561,9 +562,7 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
     // ---- epilogue: the last step's accumulated products are still in flight (the issuer committed bar_fin)
     wait_on(&bar_fin, 0);
     tc_fence_after_sync();
-    if (bad) {
-      atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
-    } else {
+    if (!bad) {
       if (grp == 0 && row < N) {
         float4* dst = reinterpret_cast<float4*>(p.dq_part + (size_t)slab * p.part_stride + base + (size_t)row * kD);
 #pragma unroll
@@ -590,7 +589,11 @@ __global__ void __maxnreg__(168) simplicial_bwd_sm100_kernel(const __grid_consta
   }
 
   tc_fence_before_sync();
-  __syncthreads();
+  bad = __syncthreads_or(bad) != 0;
+  if (bad && tid == 0) {  // any thread's wait: the finalize kernel then clears every gradient
+    if (p.use_tma) mbar_wait(&bar_kv, 0);  // the copies may be what did not arrive
+    atomicExch(p.status, MF_ERR_DEVICE_TIMEOUT);
+  }
   if (warp == 0) tmem_dealloc(tmem, kBwdTmemCols);
 }
 
