@@ -53,12 +53,12 @@ extern "C" {
 #define MF_PRECISION_IEEE_FP32 2
 
 /* Which implementation a simplicial call is allowed to use. */
-#define MF_BACKEND_AUTO 0    /* the fastest: a tensor-core kernel (warp-level mma.sync, or tcgen05 for the backward pass without
-                              * a bias above 32 tokens) when the problem qualifies, else the fp32 CUDA-core kernels */
+#define MF_BACKEND_AUTO 0    /* the fastest: a tensor-core kernel when the problem qualifies (above 32 tokens tcgen05 backward and,
+                              * with the bias, for large forward calls; else warp-level mma.sync), else the CUDA-core kernels */
 #define MF_BACKEND_GENERIC 1 /* always the fp32 CUDA-core kernel */
 #define MF_BACKEND_TCGEN05 2 /* the row-packed tcgen05 kernels or MF_ERR_UNSUPPORTED */
-#define MF_BACKEND_TCGEN05_TILES 3 /* the tcgen05 kernels with one query per tile row; the warp-level mma.sync ones up to 32
-                                    * tokens and with the factorized bias, which those do not serve; or MF_ERR_UNSUPPORTED */
+#define MF_BACKEND_TCGEN05_TILES 3 /* the tcgen05 kernels with one query per tile row, with the factorized bias the trilinear ones;
+                                    * the warp-level mma.sync ones up to 32 tokens; or MF_ERR_UNSUPPORTED */
 
 /* ------------------------------------------------------------------------- */
 /* 2-simplicial attention                                                     */
@@ -116,8 +116,8 @@ typedef struct MfSimplicialFwdArgs {
   float* lse;     /* (B,H,N)   fp32 natural-log sum of exp over visible pairs */
   void* out_cast; /* optional (B,H,N,D) copy of out in `dtype`; may be NULL */
   /* mf_simplicial_fwd_workspace_bytes() bytes, 256-byte aligned; may be NULL when that is 0.  Calls of the default backend are
-   * served without it too: with it, large batches start with their heavy molecules, and with the factorized bias above 32 tokens
-   * the kernel that needs none takes about twice as long. */
+   * served without it too: with it, large batches start with their heavy molecules, and large calls with the factorized bias above
+   * 32 tokens take about half the time. */
   void* workspace;
   size_t workspace_bytes;
 } MfSimplicialFwdArgs;

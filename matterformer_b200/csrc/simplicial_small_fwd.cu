@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(1024) simplicial_small_order_kernel(const uint
 // Where a batch is several waves of CTAs, the last ones to start should be small: molecules of 9-29 atoms x 8 heads, in the order
 // given | heavy first: backward with the bias 128 molecules 131 | 108 us, 256 244 | 199, without 256 159 | 130, 1024 546 | 489; with the
 // residuals 64 243 | 210; forward 1024 141 | 128, 256 with the bias 61 | 58, 64 with the residuals 70 | 55.  The list takes a launch
-// (it is lost where all molecules are of one size): it is made where it pays several times over.
+// (it is lost where all molecules are of one size: 1024 of 29 atoms forward 213 | 219, backward 800 | 807, 256 with the bias backward
+// 310 | 316, which a caller who knows avoids by giving no workspace): it is made where it pays several times over.
 size_t simplicial_small_order_bytes(int batch, int heads, bool backward, bool residual) {
   const long long bh = (long long)batch * heads;
   return bh >= (residual ? 512 : backward ? 1024 : 4096) ? align_up(2 * (size_t)batch * sizeof(int32_t), 256) : 0;

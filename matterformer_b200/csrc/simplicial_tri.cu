@@ -21,10 +21,20 @@
 //
 // The softmax takes shift 0; a tile in which a row's sum leaves 2^-60 .. 2^60 is done again with its exact maxima.
 //
+// Each pass rounds the products of its own pair of operands (q k1, k1 k2 or k2 q) to bf16 before it forms S.  The log-sum-exp comes
+// from the first, so P of the other two is normalised up to that rounding, and dk1, dv1, dw, dk2, dv2, dv belong to logits that
+// differ in their last bits from those of dq, du and dgate.  The errors against 64 bits are those of one rounding (2-3e-3).
+//
+// When a wait expires, the rows of the tile leave as zeros (forward; the failure is shared at the barrier that ends a pass), or a
+// last launch clears every gradient (backward).
+//
 // Bound by the chain of hand-overs of a step (half of the time is left with no MMA and no arithmetic at all) and the softmax
-// warps' instructions; the tensor pipe is busy for a quarter of the time.  64 molecules of 20-181 atoms, 8 heads: forward 0.85 ms,
-// backward 3.6 ms (mma.sync kernels, query by query and first key by first key: 1.84 and 6.09 ms); of 20-64 atoms 0.12 and 0.45
-// ms (0.18 and 0.60).
+// warps' instructions; the tensor pipe is busy for 16 to 20 % of the time.  The backward kernel spills (326 bytes of stores, 432 of
+// loads by ptxas): one register split serves its three passes, whose accumulators differ.  Of the CTAs launched, five per pass,
+// half to four fifths find no tile and return (up to 96 tokens a molecule has at most four, up to 64 at most two).
+// 64 molecules of 20-181 atoms of 192 tokens, 8 heads: forward 0.85 ms, backward 3.6 ms (mma.sync kernels, query by query and first
+// key by first key: 1.82 and 6.09 ms); 64 full ones of 64 tokens 0.19 and 0.68 ms (0.24 and 0.96).  A single molecule of 181: 0.24
+// and 0.42 ms (0.12, which is why short forward calls stay there, and 1.54).
 #include "common.cuh"
 #include "simplicial.cuh"
 #include "simplicial_rows.cuh"

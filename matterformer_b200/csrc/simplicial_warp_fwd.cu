@@ -7,8 +7,9 @@
 // Blocks in which every pair counts take no masks.
 //
 // Bound by the mma.sync pipe, busy 52 % of the time, and the instructions and dependencies around it.  64 molecules of 20-181 atoms,
-// 8 heads: 888 us (1 058 row-packed on tcgen05); 16 molecules of 20-131 atoms 119 (283).  With the bias (26 % busy, the loads of v
-// and w) it serves callers that give no workspace: 1 821 us against 848 of simplicial_tri.cu, which needs one.
+// 8 heads: 851 us, in the order given 893 (1 058 row-packed on tcgen05); 16 molecules of 20-131 atoms 113 (283).  With the bias (26 %
+// busy, the loads of v and w) it serves short calls, see uses_tri_forward(), and callers that give no workspace: 1 821 us for that
+// batch against 848 of simplicial_tri.cu, which needs one.
 #include <type_traits>
 
 #include "common.cuh"
@@ -378,7 +379,8 @@ int queries_per_cta(int bh, int tokens) {
 // Workspace of the list above, which a caller may leave out.  A CTA runs with the square of its molecule's size, so in the order
 // given a launch ends with a few large ones: 8 heads, 20-181 atoms, 64 molecules 893 | 851 us heavy first, 24-192 8 molecules 181 |
 // 140, 20-100 32 134 | 107, 20-160 4 76 | 64, 20-64 64 103 | 85, 10-48 64 60 | 48.  The list takes a launch of 3 us (and nothing is
-// gained where all molecules are of one size), so it is made from a wave and a half of CTAs and about 50 us on.
+// gained where all molecules are of one size: 64 of 64 tokens 153 | 157 us, 8 of 192 396 | 398), so it is made from a wave and a half of
+// CTAs and about 50 us on.
 size_t simplicial_warp_order_bytes(const MfSimplicialFwdArgs& a) {
   const int batch = a.batch, tokens = a.tokens;
   const long long bh = (long long)batch * a.heads;

@@ -73,15 +73,15 @@ def _remember_status(ws: Optional[torch.Tensor]) -> None:
         code = device_status()
         if code != 0:
             raise RuntimeError(f"a device-side wait of the tensor-core simplicial kernel expired (status {code}); "
-                               "the outputs of this call are zeros")  # fmt: skip
+                               "the affected outputs of this call are zeros")  # fmt: skip
 
 
 def device_status() -> int:
     """Status word the most recent tensor-core simplicial kernel left in its workspace.
 
     0 means every bounded device-side wait completed; ``MF_ERR_DEVICE_TIMEOUT`` means a wait
-    expired, the kernel gave up cleanly and the affected outputs are zeros (the backward pass then
-    writes every gradient as zeros).  Reading it synchronises.
+    expired, the kernel gave up cleanly and the affected outputs are zeros (forward the rows of the tile
+    that gave up, backward every gradient).  Reading it synchronises.
     """
     native = _lib.native()
     status = native.last_status() if native is not None else _LAST_STATUS
