@@ -111,13 +111,14 @@ template <typename Args>
 bool uses_tri_kernels(const Args* a) {
   return a->tokens > kSmallTokens && has_factorized_bias(a);
 }
-// The forward pass runs on them where a call is long enough.  A tile walks all first keys of its rows whatever the batch, up to
-// 100 tokens in at most 26 steps, from 101 on in up to 128 (tri_plan); the warp-level kernel spreads the queries of a small batch
-// over the chip.  The host does not know how full the batch is, so the lines lie between the two extremes.  8 heads, us, trilinear |
+// The forward pass runs on them where a call is long enough.  A tile walks all first keys of its rows whatever the batch, up to 100
+// tokens in at most 26 steps, from 101 on in up to 128 (tri_plan); the warp-level kernel spreads the queries of a small batch over
+// the chip.  The host does not know how full the batch is, so the lines lie between the two extremes.  8 heads, us, trilinear |
 // warp-level, all molecules full | spread from an eighth of the tokens up: 64 tokens x 4 molecules 53 | 32, 53 | 17; x 16 54 | 77,
-// 54 | 43; x 32 98 | 136, 57 | 92.  96 x 4 54 | 60, 54 | 31; x 12 99 | 150, 60 | 87.  128 x 4 254 | 143, 249 | 68; x 12 255 | 334, 250 | 159; x 32 492 | 892, 255 | 364.  192 x 1
-// 257 | 103; x 6 259 | 557, 257 | 257; x 32 1 479 | 2 814, 580 | 1 078.  On either side a molecule's result does not depend on its
-// batch; the two sides round differently, with the same error.  MF_BACKEND_TCGEN05_TILES stays on one side.
+// 54 | 43; x 32 98 | 136, 57 | 92.  96 x 4 54 | 60, 54 | 31; x 12 99 | 150, 60 | 87.  128 x 4 254 | 143, 249 | 68; x 12 255 | 334,
+// 250 | 159; x 32 492 | 892, 255 | 364.  192 x 1 257 | 103; x 6 259 | 557, 257 | 257; x 32 1 479 | 2 814, 580 | 1 078.  On either
+// side a molecule's result does not depend on its batch; the two sides round differently, with the same error.
+// MF_BACKEND_TCGEN05_TILES stays on one side.
 inline bool uses_tri_forward(const MfSimplicialFwdArgs* a) {
   if (!uses_tri_kernels(a)) return false;
   const double heads = (double)a->batch * a->heads, n = a->tokens;
