@@ -17,6 +17,8 @@
 //
 // Structures with a coordinate outside [0,1) (where the reference's 27 offsets of the unwrapped
 // coordinates are not the nearest images) are searched exhaustively.
+#include <type_traits>
+
 #include "common.cuh"
 #include "geometry.cuh"
 
@@ -225,34 +227,69 @@ __global__ void __launch_bounds__(1024) knn_setup_kernel(const float* __restrict
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Warp-cooperative search.  One warp serves one bin of the grid: the atoms of the 3 x 3 x 3 bins around it are the
-// candidates of every query atom in the bin, so they are gathered once into shared memory (own bin first, then the
-// face, edge and corner neighbours, so that the list of the k best tightens early).  For one query at a time the 32
-// lanes evaluate 32 candidates, and the k best live in a list spread over the lanes (lane t holds entry t, sorted by
-// (d2, index)): a candidate that beats the last entry is broadcast and every lane either keeps its entry, takes the
-// candidate, or takes its left neighbour's entry.  Queries whose k-th distance does not prove the first shell
-// complete, structures searched exhaustively and neighbourhoods larger than the shared-memory list fall back to
-// scanning bins straight from global memory with the same list logic.  The result does not depend on the order of
-// candidates, so it is the same, bit for bit, as the one-thread-per-query search.
+// Warp-cooperative search.  One warp serves one bin of the grid: the atoms of the 3 x 3 x 3 bins around it are the candidates of
+// every query atom in the bin, so they are gathered once into shared memory.  The k best live in a list spread over the lanes
+// (lane t holds entry t, sorted by (d2, index)).  Two queries are searched together: distances of 64 candidates, two per lane
+// and instruction; those within the first shell's reach are compacted, sorted across the lanes and become the list.  Queries
+// whose k-th distance does not prove the first shell complete, structures searched exhaustively and neighbourhoods larger than
+// the shared-memory list fall back to scanning bins straight from global memory, 32 candidates at a time: a candidate that
+// beats the last entry is broadcast and every lane either keeps its entry, takes the candidate, or takes its left neighbour's
+// entry.  Small structures without a first shell (fewer than three bins along an axis, or three along each) are searched as
+// one list of all their atoms.  The result does not depend on the order of candidates, so it is the same, bit for bit, as the
+// one-thread-per-query search.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kWarpCand = 384;  // candidates per warp in shared memory (a 27-bin neighbourhood holds about 216)
+constexpr int kPairSurv = 128;  // survivors per query of the paired search
 
-__constant__ int8_t kShellOrder[27][3] = {
-    {0, 0, 0},
-    {-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0}, {0, 0, -1}, {0, 0, 1},
-    {-1, -1, 0}, {-1, 1, 0}, {1, -1, 0}, {1, 1, 0}, {-1, 0, -1}, {-1, 0, 1}, {1, 0, -1}, {1, 0, 1},
-    {0, -1, -1}, {0, -1, 1}, {0, 1, -1}, {0, 1, 1},
-    {-1, -1, -1}, {-1, -1, 1}, {-1, 1, -1}, {-1, 1, 1}, {1, -1, -1}, {1, -1, 1}, {1, 1, -1}, {1, 1, 1}};
+// Shared memory of one warp.  The paired search reads its candidates two at a time per coordinate and keeps the image offset
+// of each (ox and oy as the upper halves of their fp32 patterns in one word, oz); the other searches hold float4 candidates.
+struct alignas(16) KnnWarpMem {
+  union {
+    float4 cand[kWarpCand];
+    struct {
+      float nx[kWarpCand], ny[kWarpCand], nz[kWarpCand];  // negated coordinates
+      int id[kWarpCand];
+    };
+  };
+  uint32_t oxy[kWarpCand];
+  float oz[kWarpCand];
+  float2 surv[2][kPairSurv];  // (d2, index bits) of the candidates within the first shell's reach
+};
+
+// Two fp32 operations in one instruction, each rounded as its scalar form is.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
 
 template <int KMAX>
-__global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__ cell,
+__global__ void __launch_bounds__(128, 5) knn_warp_kernel(const float* __restrict__ cell,
                                                        const int32_t* __restrict__ num_atoms,
                                                        const int32_t* __restrict__ grid_dims,
                                                        const float* __restrict__ bounds, int n_max, int k,
                                                        int include_self, KnnWorkspace w, int32_t* __restrict__ idx,
                                                        float* __restrict__ dist2) {
-  __shared__ float4 cand_s[4][kWarpCand];
-  __shared__ float2 surv_s[4][kWarpCand];  // (d2, index bits) of the candidates within the first shell's reach
+  __shared__ KnnWarpMem mem_s[4];
   const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gx = grid_dims[3 * b], gy = grid_dims[3 * b + 1], gz = grid_dims[3 * b + 2];
   const int n = min(num_atoms[b], n_max);
@@ -272,54 +309,84 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
   const bool exhaustive = w.flags[b] != 0;
   const int cz = bin % gz, cy = (bin / gz) % gy, cx = bin / (gy * gz);
   const int need = min(k, include_self ? n : n - 1);  // neighbours that exist
-  float4* cand = cand_s[warp];
-  float2* surv = surv_s[warp];
+  KnnWarpMem& mem = mem_s[warp];
 
   // ---- the first shell's candidates, gathered once for all queries of the bin
-  const bool ordered = !exhaustive && gx >= 3 && gy >= 3 && gz >= 3;
-  const bool covers_all = exhaustive || (gx <= 3 && gy <= 3 && gz <= 3);
+  const bool covers = exhaustive || (gx <= 3 && gy <= 3 && gz <= 3);
+  // From three bins per axis on, every neighbour bin is reached once, and whether that is across the cell boundary decides the
+  // image.  Rounding the fractional delta finds another image only where the delta exceeds 0.5, and then both images are
+  // beyond the reach: from one third of the cell's width on along that axis.
+  bool paired = !covers && gx >= 3 && gy >= 3 && gz >= 3;
   int n_cand = 0;
-  bool in_smem = ordered;
-  bool inner = false;  // no neighbour bin is reached across the cell boundary: the zero image is the rounded one
-  if (!ordered && n <= kWarpCand) {
-    // a structure that fits the list: all its atoms, instead of a search bin by bin with a handful of atoms each
-    for (int e = lane; e < n; e += 32) cand[e] = __ldg(sorted + e);
-    n_cand = n;
-    in_smem = true;
-    __syncwarp();
-  }
-  const bool covers = covers_all || (!ordered && in_smem);
-  if (ordered) {
-    inner = gx >= 5 && gy >= 5 && gz >= 5 && cx > 0 && cx < gx - 1 && cy > 0 && cy < gy - 1 && cz > 0 && cz < gz - 1;
-    // lane t < 27 looks up the extent of neighbour bin t; one prefix sum places every bin's atoms in the list, and the
-    // copies of the 27 bins are independent loads (two round trips to memory instead of one per bin)
-    int e0 = 0, cnt = 0;
-    if (lane < 27) {
-      const int bx = (cx + kShellOrder[lane][0] + gx) % gx, by = (cy + kShellOrder[lane][1] + gy) % gy,
-                bz = (cz + kShellOrder[lane][2] + gz) % gz;
-      const int ob = (bx * gy + by) * gz + bz;
-      e0 = start[ob];
-      cnt = start[ob + 1] - e0;
+  if (paired) {
+    // The bins of a column along z lie one behind the other: nine columns, of one stretch or (where z wraps) two.  Lane t < 9
+    // looks up column t; the loads of three columns are in flight together.
+    const int zb = cz == 0 ? gz - 1 : 0, zlo = max(cz - 1, 0), zhi = min(cz + 1, gz - 1);
+    const bool zwrap = cz == 0 || cz == gz - 1;
+    const float ozb = cz == 0 ? 1.f : -1.f;
+    int e0 = 0, c0 = 0, e1 = 0, c1 = 0;
+    if (lane < 9) {
+      const int x = cx + lane / 3 - 1, y = cy + lane % 3 - 1;
+      const int col = ((x < 0 ? gx - 1 : (x >= gx ? 0 : x)) * gy + (y < 0 ? gy - 1 : (y >= gy ? 0 : y))) * gz;
+      e0 = start[col + zlo];
+      c0 = start[col + zhi + 1] - e0;
+      if (zwrap) {
+        e1 = start[col + zb];
+        c1 = start[col + zb + 1] - e1;
+      }
     }
-    int off = cnt;
+    int off = c0 + c1;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < 16; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, off, o);
       if (lane >= o) off += v;
     }
-    n_cand = __shfl_sync(0xffffffffu, off, 31);
-    off -= cnt;
-    if (n_cand > kWarpCand) {
-      in_smem = false;
-    } else {
-      for (int t = 0; t < 27; ++t) {
-        const int e0_t = __shfl_sync(0xffffffffu, e0, t), c_t = __shfl_sync(0xffffffffu, cnt, t),
-                  o_t = __shfl_sync(0xffffffffu, off, t);
-        for (int e = lane; e < c_t; e += 32) cand[o_t + e] = __ldg(sorted + e0_t + e);
+    n_cand = __shfl_sync(0xffffffffu, off, 8);
+    off -= c0 + c1;
+    paired = n_cand <= kWarpCand;
+    if (paired) {
+#pragma unroll 1
+      for (int t0 = 0; t0 < 9; t0 += 3) {
+        float4 v[3];
+        int at[3], size[3], s0[3], s1[3], first[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          at[u] = __shfl_sync(0xffffffffu, off, t0 + u);
+          s0[u] = __shfl_sync(0xffffffffu, e0, t0 + u);
+          s1[u] = __shfl_sync(0xffffffffu, e1, t0 + u);
+          first[u] = __shfl_sync(0xffffffffu, c0, t0 + u);
+          size[u] = first[u] + __shfl_sync(0xffffffffu, c1, t0 + u);
+          if (lane < size[u]) v[u] = __ldg(sorted + (lane < first[u] ? s0[u] + lane : s1[u] + lane - first[u]));
+        }
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          const int x = cx + (t0 + u) / 3 - 1, y = cy + (t0 + u) % 3 - 1;
+          const float ox = x < 0 ? 1.f : (x >= gx ? -1.f : 0.f), oy = y < 0 ? 1.f : (y >= gy ? -1.f : 0.f);
+          const uint32_t oxy = __float_as_uint(ox) | (__float_as_uint(oy) >> 16);
+          for (int e = lane; e < size[u]; e += 32) {
+            if (e >= 32) v[u] = __ldg(sorted + (e < first[u] ? s0[u] + e : s1[u] + e - first[u]));
+            mem.nx[at[u] + e] = -v[u].x;
+            mem.ny[at[u] + e] = -v[u].y;
+            mem.nz[at[u] + e] = -v[u].z;
+            mem.id[at[u] + e] = __float_as_int(v[u].w);
+            mem.oxy[at[u] + e] = oxy;
+            mem.oz[at[u] + e] = e < first[u] ? 0.f : ozb;
+          }
+        }
+      }
+      for (int e = n_cand + lane; e < (n_cand + 63) / 64 * 64; e += 32) {  // (NaN is within no distance)
+        mem.nx[e] = __int_as_float(0x7fffffff);
+        mem.ny[e] = mem.nz[e] = 0.f;
+        mem.id[e] = -1;
+        mem.oxy[e] = 0;
+        mem.oz[e] = 0.f;
       }
     }
-    __syncwarp();
   }
+  const bool listed = !paired && n <= kWarpCand;  // all atoms of a small structure
+  if (listed)
+    for (int e = lane; e < n; e += 32) mem.cand[e] = __ldg(sorted + e);
+  __syncwarp();
 
   // the list of the k best, entry t on lane t
   // entries are 64-bit keys, the bits of d2 (never negative) above the index: one comparison orders by (d2, index)
@@ -340,13 +407,6 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
     if (ok && (include_self || __float_as_int(o.w) != my_id)) {
       if (!exhaustive) {
         const float dx = __fsub_rn(me.x, o.x), dy = __fsub_rn(me.y, o.y), dz = __fsub_rn(me.z, o.z);
-        if (inner) {  // |delta| < 0.5 on every axis: (0, 0, 0) is the offset the comparisons below would find
-          const float rx = __fmaf_rn(dz, c.l20, __fmaf_rn(dy, c.l10, __fmul_rn(dx, c.l00)));
-          const float ry = __fmaf_rn(dz, c.l21, __fmul_rn(dy, c.l11)), rz = __fmul_rn(dz, c.l22);
-          d2 = __fmaf_rn(rz, rz, __fmaf_rn(ry, ry, __fmul_rn(rx, rx)));
-          if (d2 >= fast_limit2 && far_kept >= fast_limit2) d2 = min_image_d2(me.x, me.y, me.z, o.x, o.y, o.z, c);
-          return d2;
-        }
         // -rint(delta) for |delta| < 1 (ties at +-0.5 go to 0), by comparison: cheaper than three conversions
         const float ox = dx > 0.5f ? -1.f : (dx < -0.5f ? 1.f : 0.f), oy = dy > 0.5f ? -1.f : (dy < -0.5f ? 1.f : 0.f),
                     oz = dz > 0.5f ? -1.f : (dz < -0.5f ? 1.f : 0.f);
@@ -381,110 +441,200 @@ __global__ void __launch_bounds__(128) knn_warp_kernel(const float* __restrict__
     insert_batch(distance(o, ok, fminf(worst, keep_below)), __float_as_int(o.w));
   };
   // the lanes' 32 entries sorted ascending across the warp (bitonic network, 15 exchanges)
-  auto sort_lanes = [&]() {
-#pragma unroll
+  auto sort_lanes = [&](unsigned long long& v) {
+#pragma unroll 1
     for (int k2 = 2; k2 <= 32; k2 <<= 1) {
-#pragma unroll
+#pragma unroll 1
       for (int j = k2 >> 1; j > 0; j >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, v, j);
         const bool keep_min = ((lane & j) == 0) == ((lane & k2) == 0);
-        if ((other < key) == keep_min) key = other;
+        if ((other < v) == keep_min) v = other;
       }
     }
   };
-  // all atoms of the bins within s of the query's bin, straight from global memory
+  // All atoms of the bins within s of the query's bin, straight from global memory.  The bins of a column along z are one
+  // stretch of the sorted atoms (two where the run wraps): 32 columns are looked up at a time and walked as one list, the next
+  // 32 atoms on their way while the current ones are compared.  Few queries come here, but a warp that does is on its own:
+  // bin by bin (125 round trips to memory at s = 2) one of them took longer than the whole search of the others.
   auto scan_shell = [&](int s) {
     const int nx = exhaustive ? gx : min(2 * s + 1, gx);
     const int ny = exhaustive ? gy : min(2 * s + 1, gy);
     const int nz = exhaustive ? gz : min(2 * s + 1, gz);
-    for (int ix = 0; ix < nx; ++ix) {
-      const int bx = ((cx - s + ix) % gx + gx) % gx;
-      for (int iy = 0; iy < ny; ++iy) {
-        const int by = ((cy - s + iy) % gy + gy) % gy;
-        for (int iz = 0; iz < nz; ++iz) {
-          const int bz = ((cz - s + iz) % gz + gz) % gz;
-          const int ob = (bx * gy + by) * gz + bz;
-          const int e0 = start[ob], e1 = start[ob + 1];
-          for (int e = e0; e < e1; e += 32) {
-            const bool ok = e + lane < e1;
-            consider(ok ? __ldg(sorted + e + lane) : make_float4(0.f, 0.f, 0.f, 0.f), ok);
-          }
-        }
+    const int z0 = nz == gz ? 0 : (cz - s + gz) % gz, over = max(z0 + nz - gz, 0);
+    for (int t0 = 0; t0 < nx * ny; t0 += 32) {
+      int e0 = 0, c0 = 0, e1 = 0, c1 = 0;
+      if (t0 + lane < nx * ny) {
+        const int bx = ((cx - s + (t0 + lane) / ny) % gx + gx) % gx, by = ((cy - s + (t0 + lane) % ny) % gy + gy) % gy;
+        const int col = (bx * gy + by) * gz;
+        e0 = start[col + z0];
+        c0 = start[col + z0 + nz - over] - e0;
+        e1 = start[col];
+        c1 = start[col + over] - e1;
+      }
+      int end = c0 + c1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, end, 31);
+      auto load = [&](int p) {  // the p-th atom of these columns
+        int t = 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          if (__shfl_sync(0xffffffffu, end, t + o - 1) <= p) t += o;
+        t = min(t, 31);  // (beyond the last one: not loaded)
+        const int f0 = __shfl_sync(0xffffffffu, e0, t), n0 = __shfl_sync(0xffffffffu, c0, t), f1 = __shfl_sync(0xffffffffu, e1, t);
+        const int r = p - (__shfl_sync(0xffffffffu, end, t) - n0 - __shfl_sync(0xffffffffu, c1, t));
+        return p < total ? __ldg(sorted + (r < n0 ? f0 + r : f1 + r - n0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      };
+      float4 next = load(lane);
+      for (int p = lane; p - lane < total; p += 32) {
+        const float4 o = next;
+        next = load(p + 32);
+        consider(o, p < total);
       }
     }
     return nx == gx && ny == gy && nz == gz;  // every bin was visited
   };
 
   const int s_max = max(max(gx, gy), gz);
-  for (int q = q0; q < q1; q += parts) {
-    me = __ldg(sorted + q);
-    my_id = __float_as_int(me.w);
-    key = kNone;
-    int s = 1;
-    bool all_bins;
-    keep_below = (covers || s_max <= 1) ? INFINITY : h * h * (1.f - 2e-5f);
-    if (in_smem && !ordered) {
-      // the first 32 atoms sorted in one go, the others inserted while they beat the last entry (which also spares most of
-      // the far ones the 27-image search)
-      const float4 o = lane < n_cand ? cand[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float d2 = distance(o, lane < n_cand, INFINITY);
-      if (d2 < INFINITY) key = key_of(d2, __float_as_int(o.w));
-      sort_lanes();
-      if (lane >= KMAX) key = kNone;
-      for (int c0 = 32; c0 < n_cand; c0 += 32) {
-        const bool ok = c0 + lane < n_cand;
-        consider(ok ? cand[c0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f), ok);
-      }
-      all_bins = true;
-    } else if (in_smem) {
-      // first every candidate's distance, keeping those within the shell's reach; then the first 32 survivors are
-      // sorted across the lanes in one go and become the list, the rest (few) are inserted one at a time
-      int m = 0;
-      for (int c0 = 0; c0 < n_cand; c0 += 32) {
-        const bool ok = c0 + lane < n_cand;
-        const float4 o = ok ? cand[c0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float d2 = distance(o, ok, keep_below);
-        const bool keep = d2 < keep_below;  // also drops the INF of lanes without a candidate
-        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-        if (keep) surv[m + __popc(bal & ((1u << lane) - 1u))] = make_float2(d2, o.w);
-        m += __popc(bal);
+  const float reach2 = h * h * (1.f - 2e-5f);
+  const uint32_t below = (1u << lane) - 1u;
+  // Every step below is written once (no unrolled copies, one place that scans a shell, one that finishes a row): with the same
+  // steps inlined in several places half of every warp's cycles went into waiting for an instruction.  32 cells of 4 096 atoms,
+  // k = 16, this kernel: one query at a time 247 us; with shells beyond the first scanned as stretches 198; two queries at a
+  // time, inlined 237; as it stands 155 (2.5 instructions per clock and SM; at four CTAs per SM instead of five 156).
+#pragma unroll 1
+  for (int q = q0; q < q1; q += 2 * parts) {
+    const int qs[2] = {q, q + parts < q1 ? q + parts : q};
+    const float4 p0 = __ldg(sorted + qs[0]), p1 = __ldg(sorted + qs[1]);
+    uint32_t word0 = 0, word1 = 0;
+    int m0 = 0, m1 = 0;
+    if (paired) {
+      // two candidates of 64 per lane and instruction; both queries read them once
+      const F2 qx[2] = {pack2(p0.x, p0.x), pack2(p1.x, p1.x)}, qy[2] = {pack2(p0.y, p0.y), pack2(p1.y, p1.y)},
+               qz[2] = {pack2(p0.z, p0.z), pack2(p1.z, p1.z)};
+      const int self[2] = {include_self ? -1 : __float_as_int(p0.w), include_self ? -1 : __float_as_int(p1.w)};
+      int m[2] = {0, 0};
+      const F2 l00 = pack2(c.l00, c.l00), l10 = pack2(c.l10, c.l10), l11 = pack2(c.l11, c.l11), l20 = pack2(c.l20, c.l20),
+               l21 = pack2(c.l21, c.l21), l22 = pack2(c.l22, c.l22);
+#pragma unroll 1
+      for (int e = 2 * lane; e - 2 * lane < n_cand; e += 64) {
+        const F2 nx = *reinterpret_cast<const F2*>(mem.nx + e), ny = *reinterpret_cast<const F2*>(mem.ny + e),
+                 nz = *reinterpret_cast<const F2*>(mem.nz + e), oz = *reinterpret_cast<const F2*>(mem.oz + e);
+        const int2 id = *reinterpret_cast<const int2*>(mem.id + e);
+        const uint2 w2 = *reinterpret_cast<const uint2*>(mem.oxy + e);
+        const F2 ox = pack2(__uint_as_float(w2.x & 0xffff0000u), __uint_as_float(w2.y & 0xffff0000u)),
+                 oy = pack2(__uint_as_float(w2.x << 16), __uint_as_float(w2.y << 16));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const F2 ax = add2(add2(qx[u], nx), ox), ay = add2(add2(qy[u], ny), oy), az = add2(add2(qz[u], nz), oz);
+          const F2 rx = fma2(az, l20, fma2(ay, l10, mul2(ax, l00))), ry = fma2(az, l21, mul2(ay, l11)), rz = mul2(az, l22);
+          float d0, d1;
+          unpack2(fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))), d0, d1);
+          const bool k0 = d0 < reach2 && id.x != self[u], k1 = d1 < reach2 && id.y != self[u];
+          const uint32_t b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
+          const int s0 = m[u] + __popc(b0 & below), mid = m[u] + __popc(b0), s1 = mid + __popc(b1 & below);
+          if (k0 && s0 < kPairSurv) mem.surv[u][s0] = make_float2(d0, __int_as_float(id.x));
+          if (k1 && s1 < kPairSurv) mem.surv[u][s1] = make_float2(d1, __int_as_float(id.y));
+          m[u] = mid + __popc(b1);
+        }
       }
       __syncwarp();
-      if (lane < m) {
-        const float2 sv = surv[lane];
-        key = key_of(sv.x, __float_as_int(sv.y));
+      // The first 32 survivors sorted by one 32-bit word each: the upper 27 bits of d2 and the slot.
+      m0 = m[0], m1 = m[1];
+      word0 = lane < m0 ? (__float_as_uint(mem.surv[0][lane].x) & ~31u) | lane : 0xffffffe0u | lane;
+      word1 = lane < m1 ? (__float_as_uint(mem.surv[1][lane].x) & ~31u) | lane : 0xffffffe0u | lane;
+#pragma unroll
+      for (int k2 = 2; k2 <= 32; k2 <<= 1) {
+#pragma unroll
+        for (int j = k2 >> 1; j > 0; j >>= 1) {
+          const bool keep_min = ((lane & j) == 0) == ((lane & k2) == 0);
+          const uint32_t other0 = __shfl_xor_sync(0xffffffffu, word0, j), other1 = __shfl_xor_sync(0xffffffffu, word1, j);
+          word0 = keep_min ? min(word0, other0) : max(word0, other0);
+          word1 = keep_min ? min(word1, other1) : max(word1, other1);
+        }
       }
-      sort_lanes();
-      if (lane >= KMAX) key = kNone;
-      for (int c0 = 32; c0 < m; c0 += 32) {
-        const bool ok = c0 + lane < m;
-        const float2 sv = ok ? surv[c0 + lane] : make_float2(INFINITY, __int_as_float(0x7fffffff));
-        insert_batch(sv.x, __float_as_int(sv.y));
-      }
-      __syncwarp();  // the survivor buffer is rewritten for the next query
-      all_bins = covers_all;
-    } else {
-      all_bins = scan_shell(1);
     }
-    // complete when the needed neighbours are known and the farthest of them is inside the searched shell
-    while (!all_bins && !exhaustive) {
-      const float reach = (float)s * h;
-      const float kth = need >= 1 ? dist_of(__shfl_sync(0xffffffffu, key, need - 1)) : 0.f;
-      if (kth < reach * reach * (1.f - 2e-5f) || s >= s_max) break;
-      ++s;
+#pragma unroll 1
+    for (int u = 0; u < (qs[1] == q ? 1 : 2); ++u) {
+      me = u == 0 ? p0 : p1;
+      my_id = __float_as_int(me.w);
       key = kNone;
-      {  // the reach of the new shell, unless it is the last one (every bin, or the largest half-width)
-        const bool last = (2 * s + 1 >= gx && 2 * s + 1 >= gy && 2 * s + 1 >= gz) || s >= s_max;
-        const float reach_s = (float)s * h;
-        keep_below = last ? INFINITY : reach_s * reach_s * (1.f - 2e-5f);
+      const int m = u == 0 ? m0 : m1;
+      int s = 0;  // half-width of the shell searched so far
+      bool all_bins = false;
+      if (listed) {
+        // the first 32 atoms sorted in one go, the others inserted while they beat the last entry (which also spares most of
+        // the far ones the 27-image search)
+        keep_below = INFINITY;
+        const float4 o = lane < n ? mem.cand[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float d2 = distance(o, lane < n, INFINITY);
+        if (d2 < INFINITY) key = key_of(d2, __float_as_int(o.w));
+        sort_lanes(key);
+        if (lane >= KMAX) key = kNone;
+#pragma unroll 1
+        for (int c0 = 32; c0 < n; c0 += 32) {
+          const bool ok = c0 + lane < n;
+          consider(ok ? mem.cand[c0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f), ok);
+        }
+        all_bins = true;
+      } else if (paired && m <= kPairSurv) {
+        keep_below = reach2;
+        const float2* list = mem.surv[u];
+        const float2 sv = lane < m ? list[(u == 0 ? word0 : word1) & 31] : make_float2(INFINITY, __int_as_float(0x7fffffff));
+        key = key_of(sv.x, __float_as_int(sv.y));
+        // where the words leave two of them out of order (they agree to 2^-18, or in d2 altogether) the full keys are sorted
+        const unsigned long long next = __shfl_down_sync(0xffffffffu, key, 1);
+        if (__any_sync(0xffffffffu, lane < 31 && next < key)) sort_lanes(key);
+        if (lane >= KMAX) key = kNone;
+#pragma unroll 1
+        for (int c0 = 32; c0 < m; c0 += 32) {
+          const bool ok = c0 + lane < m;
+          const float2 o = ok ? list[c0 + lane] : make_float2(INFINITY, __int_as_float(0x7fffffff));
+          unsigned long long mine = key_of(o.x, __float_as_int(o.y));
+          const unsigned long long last = __shfl_sync(0xffffffffu, key, KMAX - 1);
+          if (__popc(__ballot_sync(0xffffffffu, mine < last)) <= 10) {
+            insert_batch(o.x, __float_as_int(o.y));
+            continue;
+          }
+          // many of them: sorted too, and the two lists merged
+          sort_lanes(mine);
+          const unsigned long long r = __shfl_sync(0xffffffffu, mine, (KMAX - 1 - lane) & 31);
+          if (lane < KMAX && r < key) key = r;
+#pragma unroll 1
+          for (int j = KMAX / 2; j > 0; j >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
+            if ((other < key) == ((lane & j) == 0)) key = other;
+          }
+        }
+        s = 1;
       }
-      all_bins = scan_shell(s);
+      // complete when the needed neighbours are known and the farthest of them is inside the searched shell
+#pragma unroll 1
+      while (!all_bins) {
+        if (s > 0) {
+          const float reach = (float)s * h;
+          const float kth = need >= 1 ? dist_of(__shfl_sync(0xffffffffu, key, need - 1)) : 0.f;
+          if (exhaustive || kth < reach * reach * (1.f - 2e-5f) || s >= s_max) break;
+        }
+        ++s;
+        key = kNone;
+        {  // the reach of the shell, unless it is the last one (every bin, or the largest half-width)
+          const bool last = exhaustive || (2 * s + 1 >= gx && 2 * s + 1 >= gy && 2 * s + 1 >= gz) || s >= s_max;
+          const float reach_s = (float)s * h;
+          keep_below = last ? INFINITY : reach_s * reach_s * (1.f - 2e-5f);
+        }
+        all_bins = scan_shell(s);
+      }
+      if (lane < k) {
+        const bool have = dist_of(key) < INFINITY;
+        idx[((size_t)b * n_max + my_id) * k + lane] = have ? (int)(unsigned)key : -1;
+        if (dist2) dist2[((size_t)b * n_max + my_id) * k + lane] = have ? dist_of(key) : INFINITY;
+      }
     }
-    if (lane < k) {
-      const bool have = dist_of(key) < INFINITY;
-      idx[((size_t)b * n_max + my_id) * k + lane] = have ? (int)(unsigned)key : -1;
-      if (dist2) dist2[((size_t)b * n_max + my_id) * k + lane] = have ? dist_of(key) : INFINITY;
-    }
+    __syncwarp();  // the survivors are rewritten for the next pair
   }
   __syncwarp();  // the shared-memory list is refilled for the next bin
   }

@@ -61,3 +61,24 @@ def test_equal_distances():
         ic, dc = mfb.knn_topk(*args, k=k)
         ip, dp = mfb.knn_topk(*args, k=k, method="pairs")
         assert torch.equal(ic, ip) and torch.equal(dc, dp)
+
+
+@pytest.mark.parametrize("k", [1, 8, 16, 17, 32])
+@pytest.mark.parametrize("edges,N", [((13.0, 17.5, 60.0), 1300), ((14.0, 14.0, 14.0), 260), ((18.0, 18.0, 18.0), 577),
+                                     ((9.0, 30.0, 30.0), 900), ((40.0, 40.0, 40.0), 385)])  # fmt: skip
+def test_knn_search_paths_match_all_pairs(edges, N, k):
+    """Three, four and more bins per axis (one pass over the neighbour bins, with and without crossing the boundary), fewer than
+    three, lists of all atoms; half of the atoms of one structure in a corner: more candidates and survivors than the shared
+    lists hold there, several shells elsewhere."""
+    g = torch.Generator().manual_seed(N + k)
+    lat = torch.tensor(edges).log().repeat(3, 1)
+    lat = torch.cat([lat, torch.tensor([[0.0, 0.0, 0.0], [0.3, -0.2, 0.1], [0.0, 0.0, 0.0]])], dim=1)
+    frac = torch.rand(3, N, 3, generator=g)
+    frac[2, : N // 2] *= 0.2
+    frac[1, 1] = frac[1, 0]  # two atoms in one place
+    n = torch.tensor([N, N - 5, N])
+    args = (frac.to(DEV), lat.to(DEV), n.to(DEV))
+    for include_self in (False, True):
+        ic, dc = mfb.knn_topk(*args, k=k, include_self=include_self)
+        ip, dp = mfb.knn_topk(*args, k=k, include_self=include_self, method="pairs")
+        assert torch.equal(ic, ip) and torch.equal(dc, dp)
