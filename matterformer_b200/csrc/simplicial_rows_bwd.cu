@@ -1,8 +1,9 @@
 // Backward pass of 2-simplicial attention on the Blackwell tensor cores, row-packed.
 //
-// One CTA owns one (batch, head) and one slab of at most 128 keys of the second key set (index k).  Every row
+// One CTA owns one (batch, head) and a slab of at most 128 keys of the second key set (index k).  Every row
 // of its 128-row tile carries its own (query i, first key j) pair (see simplicial_rows.cuh); the CTA walks over
-// all query ranges of the molecule and, inside a range, over groups of first keys.  Per step, with
+// all query ranges of the molecule and, inside a range, over groups of first keys.  Molecules of more than 128 keys
+// are cut into three such parts, two of them with the key sets exchanged (see Part).  Per step, with
 //   A1[r,:] = q[i_r,:] o k1[j_r,:]   and   A2[r,:] = dO[i_r,:] o v1[j_r,:]     (rewritten into shared memory)
 // seven GEMMs run on tcgen05 with fp32 accumulators in tensor memory:
 //   S   = A1 . K2^T            logits (recomputed)
@@ -18,8 +19,8 @@
 // memory as bf16 and a GEMM against a 0/1 selector sums the rows of each group (M = 128 output columns,
 // N = 16 groups, K = 128 rows), so the column sums of a step cost one narrow MMA instead of a shuffle tree.
 //
-// dK2 / dV2 leave the CTA as final bf16 rows (no other CTA contributes to them).  dq and dk1 / dv1 are written
-// as fp32 partials per key slab and summed in a fixed order by the finalize kernel; within a CTA dk1 / dv1
+// dK2 / dV2 of the first 128 keys leave the CTA as final bf16 rows (no other CTA contributes to them).  Everything
+// else is written as fp32 partials per part and summed in a fixed order by the finalize kernel; within a CTA dk1 / dv1
 // partials are accumulated over the query ranges by plain read-modify-write of addresses only this CTA
 // touches.  There are no floating-point atomics: gradients are bit-identical from run to run.
 //
@@ -80,26 +81,38 @@ struct RowsBwdParams {
   const uint8_t* query_valid;
   const uint8_t* key_valid;
   const uint8_t* pair_valid;
-  __nv_bfloat16* dk2;  // final
-  __nv_bfloat16* dv2;  // final
-  float* dq_part;      // [slab] x (BH, N, 64) fp32
-  float* dk1_part;     // [slab]
-  float* dv1_part;     // [slab]
+  __nv_bfloat16* dk2;  // keys [0, 128): final
+  __nv_bfloat16* dv2;
+  float* dq_part;      // [part] x (BH, N, 64) fp32
+  float* dk1_part;     // two planes: part 0, parts 1 and 2
+  float* dv1_part;
+  float* dk2_part;     // parts 1 and 2: planes of (BH, N - 128, 64) for the keys from 128 on
+  float* dv2_part;
   const BatchInfo* info;
   const int32_t* order;
   int32_t* status;
-  int H, N, slabs_max;
-  size_t part_stride;  // elements per partial plane
+  int H, N, BH;
+  size_t part_stride, part2_stride;  // elements per plane
   int use_tma;
-  CUtensorMap tm_k2;   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle
-  CUtensorMap tm_v2;
+  CUtensorMap tm_k[2];   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle: second keys, first keys
+  CUtensorMap tm_v[2];
 };
 
-// Key slabs of a molecule: equal widths, multiples of 32 so that mask words line up with 32-column chunks.
-__host__ __device__ inline int slab_count(int n_keys) { return (n_keys + kSlab - 1) / kSlab; }
-__host__ __device__ inline int slab_width(int n_keys) {
-  const int s = slab_count(n_keys);
-  return s > 0 ? (((n_keys + s - 1) / s + 31) & ~31) : 0;
+// Parts of a molecule.  Part 0 has the first 128 second keys as columns and walks every first key.  The pairs left, those of the
+// second keys from 128 on, are walked by these instead: the logits are symmetric in the two key sets, so parts 1 and 2 exchange
+// them, with the first keys as columns (128 and the rest).  A molecule of n > 128 atoms takes n + 2 (n - 128) first keys' worth of
+// steps (the last n - 128 of them at most 64 columns wide); two slabs of its second keys, each walking all first keys, took 2 n.
+// 64 molecules of 20-181 atoms, 8 heads: 1 929 -> 1 620 us.
+constexpr int kParts = 3;
+struct Part {
+  bool exchanged;
+  int col0, cols;  // keys that are columns
+  int walk0;       // first key walked
+};
+__device__ __forceinline__ Part part_of(int index, int n_keys) {
+  if (index == 0) return Part{false, 0, min(n_keys, kSlab), 0};
+  if (n_keys <= kSlab) return Part{true, 0, 0, 0};
+  return index == 1 ? Part{true, 0, kSlab, kSlab} : Part{true, kSlab, n_keys - kSlab, kSlab};
 }
 
 __global__ void delta_rows_kernel(const __nv_bfloat16* __restrict__ grad_out, const float* __restrict__ out,
@@ -127,28 +140,34 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
   __shared__ uint64_t bar_kv;                                   // bulk tensor copies of the K2 / V2 slab
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t kmask[kMaskWords];
-  __shared__ uint8_t jlist[kMaxKeys];
+  __shared__ uint8_t valid_keys[kMaxKeys];
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool is_worker = tid < 256;
   const int grp = (tid >> 7) & 1;  // 0: q side, 1: dO side
   const int r = tid & 127;         // row of the tile
-  const int per_b = p.H * p.slabs_max;
-  const int b = p.order[blockIdx.x / per_b];
-  const int rem = blockIdx.x % per_b;
-  const int h = rem / p.slabs_max, slab = rem % p.slabs_max;
+  // heavy molecules first, and of all molecules part 0 (the longest) before the others
+  const int rest = (int)blockIdx.x - p.BH;
+  const int part = rest < 0 ? 0 : 1 + (rest & 1), item = rest < 0 ? (int)blockIdx.x : rest >> 1;
+  const int b = p.order[item / p.H], h = item % p.H;
   const int N = p.N;
   const int bh = b * p.H + h;
   const size_t base = (size_t)bh * N * kD;
   const int n_keys = p.info[b].n_keys;
   const int n_queries = p.info[b].n_queries;
-  const int nj = p.info[b].reserved0;  // valid first keys
+  const Part own = part_of(part, n_keys);
+  const int k0 = own.col0, nk_slab = own.cols;  // columns: keys [k0, k0 + nk_slab) of the one set
+  if (nk_slab <= 0) return;                     // the finalize kernel writes the zeros
+  // keys of the other set that are walked: the valid ones from walk0 on
+  int before = 0;
+  if (own.walk0 > 0)
+    for (int k = threadIdx.x & 31; k < own.walk0; k += 32) before += p.key_valid[(size_t)b * N + k] > 0;
+  before = __reduce_add_sync(0xffffffffu, before);
+  const int nj = p.info[b].reserved0 - before;
   const RowPlan plan = plan_rows(n_queries, nj);
-  if (plan.tiles == 0 || slab >= slab_count(n_keys)) return;  // the finalize kernel writes the zeros
-  const int slab_w = slab_width(n_keys);
-  const int k0 = slab * slab_w;                     // first key of the slab (multiple of 32)
-  const int nk_slab = min(slab_w, n_keys - k0);     // keys in the slab
-  if (nk_slab <= 0) return;
+  if (plan.tiles == 0) return;
+  const __nv_bfloat16 *walk_k = own.exchanged ? p.k2 : p.k1, *walk_v = own.exchanged ? p.v2 : p.v1;
+  const __nv_bfloat16 *col_k = own.exchanged ? p.k1 : p.k2, *col_v = own.exchanged ? p.v1 : p.v2;
   // MMA N of the logit GEMMs: whole 32-column chunks, so that every column a worker reads has been written (keys
   // beyond the slab's last have zero K2 / V2 rows)
   const int nk_pad = (nk_slab + 31) & ~31;
@@ -183,11 +202,12 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
     kmask[tid] = w;
   }
   __syncthreads();
-  if (tid < kMaxKeys && ((kmask[tid >> 5] >> (tid & 31)) & 1u)) {  // compacted list of the valid first keys
+  if (tid < kMaxKeys && ((kmask[tid >> 5] >> (tid & 31)) & 1u)) {  // compacted list of the valid keys
     int pos = __popc(kmask[tid >> 5] & ((1u << (tid & 31)) - 1u));
     for (int c = 0; c < (tid >> 5); ++c) pos += __popc(kmask[c]);
-    jlist[pos] = (uint8_t)tid;
+    valid_keys[pos] = (uint8_t)tid;
   }
+  const uint8_t* const jlist = valid_keys + before;
   auto key_live = [&](int rr) {  // slab row rr holds a key that takes part
     const int k = k0 + rr;
     return rr < nk_slab && ((kmask[k >> 5] >> (k & 31)) & 1u);
@@ -202,7 +222,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         w = 0;
         for (int e = 0; e < 32; ++e) {
           const int k = c * 32 + e;
-          if (k < n_keys && pv[(size_t)j * N + k] > 0) w |= 1u << e;
+          if (k < n_keys && pv[own.exchanged ? (size_t)k * N + j : (size_t)j * N + k] > 0) w |= 1u << e;
         }
       }
       pvbits_w[idx] = w;
@@ -213,8 +233,8 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
       if (tid == 0) {
         mbar_arrive_expect_tx(&bar_kv, (uint32_t)(kSlab / kTmaBoxRows) * 2u * kTmaBoxRows * 128u);
         for (int c = 0; c < kSlab / kTmaBoxRows; ++c) {
-          tma_load_rows(smem + kOffK2 + c * kTmaBoxRows * 128, &p.tm_k2, k0 + c * kTmaBoxRows, bh, &bar_kv);
-          tma_load_rows(smem + kOffV2 + c * kTmaBoxRows * 128, &p.tm_v2, k0 + c * kTmaBoxRows, bh, &bar_kv);
+          tma_load_rows(smem + kOffK2 + c * kTmaBoxRows * 128, &p.tm_k[own.exchanged], k0 + c * kTmaBoxRows, bh, &bar_kv);
+          tma_load_rows(smem + kOffV2 + c * kTmaBoxRows * 128, &p.tm_v[own.exchanged], k0 + c * kTmaBoxRows, bh, &bar_kv);
         }
       }
     } else {
@@ -222,8 +242,8 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         const int rr = idx >> 3, c = idx & 7;
         uint4 vk = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
         if (key_live(rr)) {
-          vk = __ldg(reinterpret_cast<const uint4*>(p.k2 + base + (size_t)(k0 + rr) * kD) + c);
-          vv = __ldg(reinterpret_cast<const uint4*>(p.v2 + base + (size_t)(k0 + rr) * kD) + c);
+          vk = __ldg(reinterpret_cast<const uint4*>(col_k + base + (size_t)(k0 + rr) * kD) + c);
+          vv = __ldg(reinterpret_cast<const uint4*>(col_v + base + (size_t)(k0 + rr) * kD) + c);
         }
         const uint32_t off = rr * 128 + ((c ^ (rr & 7)) << 4);
         *reinterpret_cast<uint4*>(smem + kOffK2 + off) = vk;
@@ -387,7 +407,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
           const int jj = s * G + gg;
           v[q] = make_uint4(0, 0, 0, 0);
           if (gg < G && jj < nj)
-            v[q] = __ldg(reinterpret_cast<const uint4*>((which == 0 ? p.k1 : p.v1) + base + (size_t)jlist[jj] * kD) + part);
+            v[q] = __ldg(reinterpret_cast<const uint4*>((which == 0 ? walk_k : walk_v) + base + (size_t)jlist[jj] * kD) + part);
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -430,7 +450,10 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
     const bool live_x = warp_live && 32 * grp < nk_x;
     const bool live_y = warp_live && 32 * grp < nk_y;
     // partial column sums of this thread's output column (readers: the 128 threads of the q side)
-    float* part_col = (r < 64 ? p.dk1_part : p.dv1_part) + (size_t)slab * p.part_stride + base + (r & 63);
+    float* part_col = (own.exchanged ? (r < 64 ? p.dk2_part : p.dv2_part) + (size_t)(part - 1) * p.part2_stride +
+                                           (long long)bh * (N - kSlab) * kD - kSlab * kD
+                                     : (r < 64 ? p.dk1_part : p.dv1_part) + base) +
+                      (r & 63);
 
     uint32_t xreg[32];
     float dq_acc[32];  // dq columns [32 grp, 32 grp + 32) of this thread's row: the two groups share the accumulation
@@ -639,7 +662,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
       // ---- end of the range: last column sums, then dq of the range (rows of one query summed over the groups)
       prefetch_sums(t, steps - 1);
       commit_sums(steps - 1);  // also: every product issued so far has completed
-      float* dq_dst = p.dq_part + (size_t)slab * p.part_stride + base;
+      float* dq_dst = p.dq_part + (size_t)part * p.part_stride + base;
       if (G == 1) {
         if (slot_ok && i < n_queries) {
           float4* dst = reinterpret_cast<float4*>(dq_dst + (size_t)i * kD + 32 * grp);
@@ -677,11 +700,13 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         named_barrier(1, 256);  // the next range's operands overwrite the staging area
       }
     }
-    // ---- epilogue: accumulators: lane r of tensor memory = key k0 + r; group 0 stores dK2, group 1 dV2
+    // ---- epilogue: accumulators: lane r of tensor memory = key k0 + r; group 0 stores dK2, group 1 dV2 (of exchanged key
+    // sets: partial dK1 and dV1)
     wait_on(&bar_fin, 0);
     tc_fence_after_sync();
     {
       __nv_bfloat16* dst = (grp == 0 ? p.dk2 : p.dv2) + base + (size_t)(k0 + r) * kD;
+      float* dst32 = (grp == 0 ? p.dk1_part : p.dv1_part) + p.part_stride + base + (size_t)(k0 + r) * kD;
       const bool store = !bad && r < nk_slab;
       const bool live = key_live(r);
 #pragma unroll
@@ -689,7 +714,11 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         uint32_t w[32];
         tmem_ld32(tmem_row + (grp == 0 ? kColDK2 : kColDV2) + 32 * half, w);  // whole warps: the load is warp-wide
         tmem_ld_wait();
-        if (store) {
+        if (store && own.exchanged) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            reinterpret_cast<uint4*>(dst32 + 32 * half)[c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+        } else if (store) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint4 v = make_uint4(0, 0, 0, 0);  // an invalid key's row is exactly zero
@@ -731,7 +760,7 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
   const int n_keys = p.info[b].n_keys, n_queries = p.info[b].n_queries, nj = p.info[b].reserved0;
   const bool failed = p.status[0] != 0;
   const bool active = n_queries > 0 && nj > 0 && !failed;
-  const int nsl = slab_count(n_keys);
+  const bool parted = n_keys > kSlab;
   const size_t off = ((size_t)bh * p.N + row) * kD + 4 * d4;
   const bool q_ok = active && row < n_queries && p.query_valid[(size_t)b * p.N + row] > 0;
   const bool k_ok = active && row < n_keys && p.key_valid[(size_t)b * p.N + row] > 0;
@@ -749,41 +778,53 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
   };
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
   if (q_ok)
-    for (int s = 0; s < nsl; ++s) add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)s * p.part_stride + off));
+    for (int s = 0; s < (parted ? kParts : 1); ++s) add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)s * p.part_stride + off));
   store4(dq + off, a);
   float4 k1v = make_float4(0.f, 0.f, 0.f, 0.f), v1v = k1v;
   if (k_ok)
-    for (int s = 0; s < nsl; ++s) {
+    for (int s = 0; s < (parted ? 2 : 1); ++s) {
       add4(k1v, *reinterpret_cast<const float4*>(p.dk1_part + (size_t)s * p.part_stride + off));
       add4(v1v, *reinterpret_cast<const float4*>(p.dv1_part + (size_t)s * p.part_stride + off));
     }
   store4(dk1 + off, k1v);
   store4(dv1 + off, v1v);
-  if (!(active && row < n_keys)) {
-    store4(p.dk2 + off, make_float4(0.f, 0.f, 0.f, 0.f));
-    store4(p.dv2 + off, make_float4(0.f, 0.f, 0.f, 0.f));
+  if (row >= kSlab || !(active && row < n_keys)) {  // (the others were stored by part 0)
+    float4 k2v = make_float4(0.f, 0.f, 0.f, 0.f), v2v = k2v;
+    if (k_ok)
+      for (int s = 0; s < 2; ++s) {
+        const size_t off2 = (size_t)s * p.part2_stride + ((size_t)bh * (p.N - kSlab) + row - kSlab) * kD + 4 * d4;
+        add4(k2v, *reinterpret_cast<const float4*>(p.dk2_part + off2));
+        add4(v2v, *reinterpret_cast<const float4*>(p.dv2_part + off2));
+      }
+    store4(p.dk2 + off, k2v);
+    store4(p.dv2 + off, v2v);
   }
 }
 
 struct RowsBwdLayout {
-  size_t info, order, delta, dq, dk1, dv1, total;
-  int slabs_max;
-  size_t part;  // bytes per partial plane
+  size_t info, order, delta, dq, dk1, dv1, dk2, dv2, total;
+  int parts;
+  size_t part, part2;  // bytes per partial plane
 };
 
 RowsBwdLayout rows_bwd_layout(int B, int H, int N) {
   RowsBwdLayout l{};
-  l.slabs_max = (N + kSlab - 1) / kSlab;
+  l.parts = N > kSlab ? kParts : 1;
   l.part = align_up((size_t)B * H * N * kD * sizeof(float), 256);
+  l.part2 = N > kSlab ? align_up((size_t)B * H * (N - kSlab) * kD * sizeof(float), 256) : 0;
+  const size_t planes = l.parts > 1 ? 2 : 1;
   size_t off = simplicial_schedule_layout(B, &l.info, &l.order);
-  l.delta = off;
-  off += align_up((size_t)B * H * N * sizeof(float), 256);
-  l.dq = off;
-  off += l.part * l.slabs_max;
-  l.dk1 = off;
-  off += l.part * l.slabs_max;
-  l.dv1 = off;
-  off += l.part * l.slabs_max;
+  auto take = [&off](size_t bytes) {
+    const size_t at = off;
+    off += bytes;
+    return at;
+  };
+  l.delta = take(align_up((size_t)B * H * N * sizeof(float), 256));
+  l.dq = take(l.part * l.parts);
+  l.dk1 = take(l.part * planes);
+  l.dv1 = take(l.part * planes);
+  l.dk2 = take(l.part2 * 2);
+  l.dv2 = take(l.part2 * 2);
   l.total = off;
   return l;
 }
@@ -812,7 +853,8 @@ int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   p.dk2 = static_cast<__nv_bfloat16*>(a.dk2);
   p.dv2 = static_cast<__nv_bfloat16*>(a.dv2);
   p.status = reinterpret_cast<int32_t*>(ws);
-  p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, BH) && make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, BH);
+  p.use_tma = make_rows_tensor_map(&p.tm_k[0], a.k2, a.tokens, BH) && make_rows_tensor_map(&p.tm_v[0], a.v2, a.tokens, BH) &&
+              make_rows_tensor_map(&p.tm_k[1], a.k1, a.tokens, BH) && make_rows_tensor_map(&p.tm_v[1], a.v1, a.tokens, BH);
   BatchInfo* info = reinterpret_cast<BatchInfo*>(ws + l.info);
   int32_t* order = reinterpret_cast<int32_t*>(ws + l.order);
   float* delta = reinterpret_cast<float*>(ws + l.delta);
@@ -822,10 +864,13 @@ int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   p.dq_part = reinterpret_cast<float*>(ws + l.dq);
   p.dk1_part = reinterpret_cast<float*>(ws + l.dk1);
   p.dv1_part = reinterpret_cast<float*>(ws + l.dv1);
+  p.dk2_part = reinterpret_cast<float*>(ws + l.dk2);
+  p.dv2_part = reinterpret_cast<float*>(ws + l.dv2);
   p.H = a.heads;
   p.N = a.tokens;
-  p.slabs_max = l.slabs_max;
+  p.BH = BH;
   p.part_stride = l.part / sizeof(float);
+  p.part2_stride = l.part2 / sizeof(float);
 
   int rc = launch_schedule(a.query_valid, a.pair_key_valid, a.batch, a.tokens, info, order, p.status, stream);
   if (rc != MF_OK) return rc;
@@ -836,7 +881,7 @@ int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(simplicial_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_rows_bwd_kernel)");
   }
-  const long long blocks = (long long)BH * p.slabs_max;
+  const long long blocks = (long long)BH * l.parts;
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
   simplicial_rows_bwd_kernel<<<(unsigned)blocks, kBwdThreads, kSmemAlloc, stream>>>(p);
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, false, stream);

@@ -94,6 +94,17 @@ def test_rows_kernels_with_mask_holes(N, lo, hi, holes):
     _check(inp, go)
 
 
+@pytest.mark.parametrize("N,beyond", [(129, 1), (161, 1), (161, 20), (192, 33), (192, 64)])
+def test_rows_backward_parts(N, beyond):
+    """More than 128 keys: the pairs beyond the 128th second key are walked with the key sets exchanged.  Few and many keys beyond,
+    holes on both sides of it, a pair mask that is not symmetric; another molecule of the batch has no such part."""
+    inp, go = _case(2, 2, N, seed=9000 + N + beyond, lo=N, hi=N, pair_holes=True, key_holes=True)
+    inp.pair_key_valid[0, 128:] = False
+    inp.pair_key_valid[0, N - 1 - torch.randperm(N - 128)[:beyond]] = True
+    inp.pair_key_valid[1, 100:] = False
+    _check(inp, go)
+
+
 def test_rows_kernels_peaked_softmax():
     """Scaled-up queries make the softmax sharp: the running maximum moves and rows of one query that sit in
     different groups end with different maxima, which the final merge has to reconcile."""
