@@ -1,8 +1,9 @@
-// The differentiable operators' host path in C++: argument checks, allocations, launch and the autograd node.
+// The operators' host path in C++: argument checks, allocations, launch and, where there is one, the autograd node.
 //
 // A call on small tensors is bound by the host.  Through a Python autograd function and ctypes a forward + backward pass of
 // simplicial attention on one small molecule took 171 us of which the kernels are 15; the backward node additionally
-// competes for the interpreter lock with the thread that waits for it.  These functions serve calls whose operands are
+// competes for the interpreter lock with the thread that waits for it.  A block list (two launches of 17 us together) took 27 us
+// that way and takes 20.  These functions serve calls whose operands are
 // ready as they are (contiguous, on one device, of the types the kernels take) and return None for every other call, which
 // then takes the Python path with its conversions and error messages.
 #include <c10/cuda/CUDAGuard.h>
@@ -280,11 +281,58 @@ std::optional<Tensor> sparse_attention(const Tensor& q, const Tensor& k, const T
   return SparseAttention::apply(q, k, v, n, count, cols, mask, window, scale, backend);
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Neighbour lists and block lists
+// ---------------------------------------------------------------------------------------------------------------------
+// Positions (B, N, 3), latents (B, 6) or cells (B, 3, 3) and, if given, counts of the types and on the device that the kernels take.
+bool structures_ready(const Tensor& pos, const Tensor& lattice, const OptTensor& n) {
+  if (!pos.is_cuda() || pos.dim() != 3 || pos.size(2) != 3 || pos.numel() == 0 || !ready(pos, pos, at::kFloat, pos.sizes())) return false;
+  const int64_t B = pos.size(0);
+  if (!ready(lattice, pos, at::kFloat, {B, 6}) && !ready(lattice, pos, at::kFloat, {B, 3, 3})) return false;
+  return !n || (n->numel() == B && ready(*n, pos, at::kInt, n->sizes()));
+}
+Tensor counts(const OptTensor& n, const Tensor& pos, const at::TensorOptions& ints) {
+  return n ? *n : at::full({pos.size(0)}, pos.size(1), ints);
+}
+
+// perm, block_count, block_cols, block_mask, num_atoms
+std::optional<std::array<Tensor, 5>> radius_blocks(const Tensor& pos, const Tensor& lattice, const OptTensor& num_atoms, double cutoff) {
+  if (!structures_ready(pos, lattice, num_atoms)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(pos.device());
+  const int64_t B = pos.size(0), N = pos.size(1), T = (N + 31) / 32;
+  const auto ints = at::TensorOptions(pos.device()).dtype(at::kInt);
+  const Tensor n = counts(num_atoms, pos, ints);
+  const Tensor perm = at::empty({B, N}, ints), count = at::empty({B, T}, ints), cols = at::empty({B, T, T}, ints);
+  const Tensor mask = at::empty({B, T, T, 32}, ints), ws = bytes(mf_radius_blocks_workspace_bytes(B, N), pos);
+  check(mf_radius_blocks(pos.const_data_ptr<float>(), lattice.const_data_ptr<float>(), lattice.dim() == 3, n.const_data_ptr<int32_t>(), B, N,
+                         cutoff, perm.data_ptr<int32_t>(), count.data_ptr<int32_t>(), cols.data_ptr<int32_t>(),
+                         reinterpret_cast<uint32_t*>(mask.data_ptr<int32_t>()), ws.data_ptr(), ws.numel(),
+                         c10::cuda::getCurrentCUDAStream().stream()));
+  return std::array<Tensor, 5>{perm, count, cols, mask, n};
+}
+
+std::optional<std::array<Tensor, 2>> knn_topk(const Tensor& pos, const Tensor& lattice, const OptTensor& num_atoms, int64_t k,
+                                              bool include_self) {
+  if (k < 1 || k > 32 || !structures_ready(pos, lattice, num_atoms)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(pos.device());
+  const int64_t B = pos.size(0), N = pos.size(1);
+  const auto ints = at::TensorOptions(pos.device()).dtype(at::kInt);
+  const Tensor n = counts(num_atoms, pos, ints);
+  const Tensor idx = at::empty({B, N, k}, ints), d2 = at::empty({B, N, k}, ints.dtype(at::kFloat));
+  const Tensor ws = bytes(mf_knn_cells_workspace_bytes(B, N), pos);
+  check(mf_knn_topk_lattice(pos.const_data_ptr<float>(), lattice.const_data_ptr<float>(), lattice.dim() == 3, n.const_data_ptr<int32_t>(), B,
+                            N, k, include_self, idx.data_ptr<int32_t>(), d2.data_ptr<float>(), ws.data_ptr(), ws.numel(),
+                            c10::cuda::getCurrentCUDAStream().stream()));
+  return std::array<Tensor, 2>{idx, d2};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("simplicial_attention", &simplicial_attention);
   m.def("sparse_attention", &sparse_attention);
+  m.def("radius_blocks", &radius_blocks);
+  m.def("knn_topk", &knn_topk);
   m.def("remember_status", &remember_status);
   m.def("last_status", &last_status);
 }

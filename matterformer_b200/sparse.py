@@ -123,6 +123,11 @@ def knn_topk(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Optional[torch
     _check_structures(pos, lattice)
     if method not in ("cells", "pairs"):
         raise ValueError(f"method must be 'cells' or 'pairs', got {method!r}")
+    native = _lib.native()
+    if native is not None and method == "cells" and type(k) is int:  # operands that are ready as they are: one call into C++
+        out = native.knn_topk(pos, lattice, num_atoms, k, bool(include_self))
+        if out is not None:
+            return tuple(out)
     B, N, _ = pos.shape
     frac = pos.float().contiguous()
     na = _num_atoms(num_atoms, B, N, pos.device)
@@ -170,6 +175,11 @@ def build_radius_blocks(pos: torch.Tensor, lattice: torch.Tensor, num_atoms: Opt
     if pos.device.type != "cuda":
         raise RuntimeError("build_radius_blocks requires CUDA tensors")
     _check_structures(pos, lattice)
+    native = _lib.native()
+    if native is not None and grid_dims is None:  # operands that are ready as they are: one call into C++
+        out = native.radius_blocks(pos, lattice, num_atoms, float(cutoff))
+        if out is not None:
+            return RadiusBlocks(*out, cutoff=float(cutoff))
     B, N, _ = pos.shape
     T = (N + 31) // 32
     dev = pos.device

@@ -68,3 +68,31 @@ def test_operands_that_need_converting_take_the_python_path():
     assert torch.equal(a, b)
     with pytest.raises(ValueError, match="k1 must match q"):
         mfb.simplicial_attention_cuda(t[0], t[1][:, :1], *t[2:], query_valid=valid, pair_key_valid=valid)
+
+
+@pytest.mark.parametrize("counts", [None, torch.int32, torch.int64])
+@pytest.mark.parametrize("form", ["latent", "cell", "strided"])
+def test_neighbour_and_block_lists(counts, form, monkeypatch):
+    """Operands that the C++ functions take as they are and operands that need converting: the bits of the Python path."""
+    g = torch.Generator("cuda").manual_seed(5)
+    pos = torch.rand(3, 3, 70, generator=g, device="cuda").transpose(1, 2)
+    pos = pos if form == "strided" else pos.contiguous()
+    lattice = torch.tensor([2.3, 2.4, 2.5, 0.1, -0.05, 0.2], device="cuda").repeat(3, 1)
+    lattice = mfb.lattice_latent_to_cell(lattice) if form == "cell" else lattice
+    n = counts and torch.tensor([70, 41, 1], device="cuda", dtype=counts)
+    results = []
+    for native in (_lib.native(), None):
+        monkeypatch.setattr(_lib, "_NATIVE", [native])
+        b = mfb.build_radius_blocks(pos, lattice, n, 4.0)
+        results.append([b.perm, b.block_count, b.block_cols, b.block_mask, b.num_atoms, *mfb.knn_topk(pos, lattice, n, k=7),
+                        *mfb.knn_topk(pos, lattice, n, k=3, include_self=True)])  # fmt: skip
+    for a, c in zip(*results):
+        assert a.dtype == c.dtype and torch.equal(a, c)
+    monkeypatch.undo()
+    for bad in (0, 33):
+        with pytest.raises(ValueError, match="k must be in"):
+            mfb.knn_topk(pos, lattice, n, k=bad)
+    with pytest.raises(ValueError, match="cutoff must be non-negative"):
+        mfb.build_radius_blocks(pos, lattice, n, -1.0)
+    with pytest.raises(ValueError, match="one count per structure"):
+        mfb.build_radius_blocks(pos, lattice, torch.ones(2, device="cuda", dtype=torch.int32), 4.0)
