@@ -45,6 +45,23 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
       }                                                                                                      \
   } while (0)
 
+// ---- launches that begin while the kernel before them ends ------------------------
+// A kernel launched with launch_dependent may begin as soon as every CTA of the kernel before it in the stream has said so
+// (launch_dependents) or has ended; it calls wait_for_previous before it touches memory, which returns when that kernel has ended and
+// its writes can be seen.  What the launch itself takes is hidden that way, also between the nodes of a captured graph.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = smem, config.stream = stream;
+  config.attrs = &attribute, config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+
 // ---- device: index checks of debug builds ----------------------------------------
 // Built with -DMF_DEBUG_BOUNDS (MF_DEBUG_BOUNDS=1 python -m matterformer_b200.build), the table and bitmap lookups
 // of the tensor-core kernels check their index first: one outside [0, limit) is recorded in the kernel's status word

@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(128) knn_kernel(const float* __restrict__ frac
 // cell sort and block list: two launches
 //
 // Bound by launches and the host: 8 structures of 300-500 atoms took 443 us as 54 launches (the cell and the grid as chains
-// of element-wise operations, keys, ranks, one CTA per pair of tiles, compaction) of 132 us on the device, and take 27 us
-// as two.
+// of element-wise operations, keys, ranks, one CTA per pair of tiles, compaction) of 132 us on the device, and take 12.5 us as two,
+// the second of which is launched while the first one runs.
 // ---------------------------------------------------------------------------
 // What the second kernel needs of a structure: its cell and the perpendicular widths.
 struct StructureInfo {
@@ -120,8 +120,16 @@ __global__ void __launch_bounds__(1024) cell_rank_kernel(const float* __restrict
   __shared__ int32_t keys[kRankTile];
   __shared__ float sc[9];
   __shared__ int grid[3];
-  const int b = blockIdx.y, tid = threadIdx.x, n = min(num_atoms[b], n_max);
+  const int b = blockIdx.y, tid = threadIdx.x;
   const int i0 = blockIdx.x * kRankAtoms;
+  launch_dependents();
+  // the first positions are on their way while one warp works out the grid
+  float first[2][3];
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int x = 0; x < 3; ++x) first[t][x] = tid + 1024 * t < n_max ? frac[((size_t)b * n_max + tid + 1024 * t) * 3 + x] : 0.f;
+  const int n = min(num_atoms[b], n_max);
   if (tid < 32) {
     if (lattice) {
       if (tid == 0) cell_from_latent(lattice + (size_t)b * 6, sc);
@@ -139,17 +147,21 @@ __global__ void __launch_bounds__(1024) cell_rank_kernel(const float* __restrict
   }
   __syncthreads();
   const int gx = grid[0], gy = grid[1], gz = grid[2];
-  auto key_of = [&](int i) {
-    const float* p = frac + ((size_t)b * n_max + i) * 3;
-    return (cell_coord(p[0], gx) * gy + cell_coord(p[1], gy)) * gz + cell_coord(p[2], gz);
-  };
+  auto key_at = [&](const float* p) { return (cell_coord(p[0], gx) * gy + cell_coord(p[1], gy)) * gz + cell_coord(p[2], gz); };
+  auto key_of = [&](int i) { return key_at(frac + ((size_t)b * n_max + i) * 3); };
   const int i = i0 + (tid >> 4), part = tid & 15;
   const int ki = i < n ? key_of(i) : 0;
   int rank = 0;
   for (int j0 = 0; j0 < n && i0 < n; j0 += kRankTile) {
     const int cnt = min(kRankTile, n - j0);
     __syncthreads();
-    for (int t = tid; t < cnt; t += 1024) keys[t] = key_of(j0 + t);
+    if (j0 == 0) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+        if (tid + 1024 * t < cnt) keys[tid + 1024 * t] = key_at(first[t]);
+    } else {
+      for (int t = tid; t < cnt; t += 1024) keys[t] = key_of(j0 + t);
+    }
     __syncthreads();
 #pragma unroll 4
     for (int t = part; t < cnt; t += 16) rank += keys[t] < ki + (j0 + t < i ? 1 : 0);  // ties: the lower index first
@@ -169,20 +181,8 @@ __device__ __forceinline__ float squared_cutoff(float cutoff) {
 }
 
 // Whether one of the 27 images of the pair is within the cutoff: the images that min_image_d2 would minimise over, less
-// those that lie farther than the cutoff by their distance along one axis alone.  That bound carries a margin for the
-// rounding of the distances it stands for, so the answer is the same bit.
-// Where the cutoff is below half of each width, at most one image per axis passes the bound, the nearest; in wider cells (most)
-// a pair then takes one distance instead of up to 27.  8 structures of 300-500 atoms, cutoff 6 Angstrom: 21 us with the loop for
-// every pair.
-__device__ __forceinline__ bool within_cutoff(float xi, float yi, float zi, float xj, float yj, float zj, const Cell& c,
-                                              const float* width, float cutoff, float cutoff2, float margin) {
-  const float dx = __fsub_rn(xi, xj), dy = __fsub_rn(yi, yj), dz = __fsub_rn(zi, zj);
-  const float limit = fmaf(margin, fabsf(dx) + fabsf(dy) + fabsf(dz) + 3.f, cutoff * 1.0001f);
-  if (limit < 0.4999f * fminf(fminf(width[0], width[1]), width[2])) {
-    const float ox = fminf(fmaxf(-rintf(dx), -1.f), 1.f), oy = fminf(fmaxf(-rintf(dy), -1.f), 1.f), oz = fminf(fmaxf(-rintf(dz), -1.f), 1.f);
-    return fabsf(__fadd_rn(dx, ox)) * width[0] <= limit && fabsf(__fadd_rn(dy, oy)) * width[1] <= limit &&
-           fabsf(__fadd_rn(dz, oz)) * width[2] <= limit && image_d2(dx, dy, dz, ox, oy, oz, c) <= cutoff2;
-  }
+// those that lie farther than `limit` by their distance along one axis alone.
+__device__ __forceinline__ bool within_cutoff(float dx, float dy, float dz, const Cell& c, const float* width, float limit, float cutoff2) {
   bool hit = false;
 #pragma unroll 1
   for (int ox = -1; ox <= 1; ++ox) {
@@ -203,56 +203,99 @@ __device__ __forceinline__ bool within_cutoff(float xi, float yi, float zi, floa
   return hit;
 }
 
-// One CTA per row tile I; warp r = row of the tile, lane = column of the column tile J.  The active column tiles are
+// The offset of -1, 0 or 1 that brings a fractional difference nearest to zero, added to it.
+__device__ __forceinline__ float2 nearest_image(float2 d) {
+  return add2(d, make_float2(fabsf(d.x) > 0.5f ? copysignf(1.f, -d.x) : 0.f, fabsf(d.y) > 0.5f ? copysignf(1.f, -d.y) : 0.f));
+}
+
+// One CTA per row tile I; a warp takes column tiles, a lane the row I*32 + lane of the bitmap.  The active column tiles are
 // collected in shared memory and listed at the end.
-constexpr int kBlockAtoms = 1024;  // one for every thread of a CTA
-__global__ void __launch_bounds__(kBlockAtoms) block_list_kernel(const float* __restrict__ frac, const StructureInfo* __restrict__ info,
+//
+// Bound by instructions once the first loads are in.  What decides how many images of a pair have to be looked at is a bound on
+// its distance along each axis: the cutoff with a margin for the rounding of the distances that it stands for, which grows
+// with the coordinates and is taken once for a pair of tiles.  Where it is below half of each width, at most one image per axis
+// passes, the nearest, and is evaluated without a test, two columns at a time: the same bits as the minimum over 27.  8 structures
+// of 300-500 atoms, cutoff 6 Angstrom: 21 us with the loop over images for every pair, 12.4 us with a bound per pair and a column
+// per lane, 6.0 us now; 16 of 512-1 024 atoms 66.6 -> 24.8 us.
+constexpr int kListWarps = 16;
+constexpr int kListAtoms = 1024;  // columns in shared memory at a time
+__global__ void __launch_bounds__(32 * kListWarps) block_list_kernel(const float* __restrict__ frac, const StructureInfo* __restrict__ info,
                                                           const int32_t* __restrict__ num_atoms, const int32_t* __restrict__ perm,
                                                           int n_max, int tiles, float cutoff, uint32_t* __restrict__ block_mask,
                                                           int32_t* __restrict__ block_count, int32_t* __restrict__ block_cols) {
   extern __shared__ uint32_t active[];  // bit J
-  __shared__ float px[kBlockAtoms], py[kBlockAtoms], pz[kBlockAtoms];  // sorted atoms, kBlockAtoms at a time
+  __shared__ __align__(16) float px[kListAtoms], py[kListAtoms], pz[kListAtoms];  // minus the coordinates of sorted atoms
+  __shared__ float reach[kListAtoms / 32];                                        // largest |x| + |y| + |z| of a column tile
   const int I = blockIdx.x, b = blockIdx.y;
-  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = min(num_atoms[b], n_max);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* pos = frac + (size_t)b * n_max * 3;
   const int32_t* pb = perm + (size_t)b * n_max;
   const int words = (tiles + 31) / 32;
-  for (int t = threadIdx.x; t < words; t += 1024) active[t] = 0u;
+  for (int t = threadIdx.x; t < words; t += 32 * kListWarps) active[t] = 0u;
+  const float cutoff2 = squared_cutoff(cutoff);
+  wait_for_previous();
+  const int n = min(num_atoms[b], n_max);
   const Cell c = load_cell(info[b].cell);
   const float width[3] = {info[b].width[0], info[b].width[1], info[b].width[2]};
   float sum = 0.f;
 #pragma unroll
   for (int t = 0; t < 9; ++t) sum += fabsf(info[b].cell[t]);
-  const float margin = 4e-6f * sum, cutoff2 = squared_cutoff(cutoff);
-  const int si = 32 * I + r;
+  const float margin = 4e-6f * sum, half_width = 0.4999f * fminf(fminf(width[0], width[1]), width[2]);
+  const int si = 32 * I + lane;
   float xi = 0.f, yi = 0.f, zi = 0.f;
   if (si < n) {
     const int ai = pb[si];
     xi = pos[3 * ai], yi = pos[3 * ai + 1], zi = pos[3 * ai + 2];
   }
-  uint32_t* mask = block_mask + ((size_t)b * tiles + I) * tiles * 32 + r;
-  for (int J = 0; J < tiles; ++J) {
-    const int sj = 32 * J + lane, at = sj % kBlockAtoms;
-    if (32 * J % kBlockAtoms == 0) {
-      __syncthreads();
-      const int t = 32 * J + threadIdx.x;
-      if (t < n) {
-        const int aj = pb[t];
-        px[threadIdx.x] = pos[3 * aj], py[threadIdx.x] = pos[3 * aj + 1], pz[threadIdx.x] = pos[3 * aj + 2];
+  const float row_reach = warp_max(fabsf(xi) + fabsf(yi) + fabsf(zi));
+  const float2 x2 = make_float2(xi, xi), y2 = make_float2(yi, yi), z2 = make_float2(zi, zi);
+  const float2 l00 = make_float2(c.l00, c.l00), l10 = make_float2(c.l10, c.l10), l11 = make_float2(c.l11, c.l11),
+               l20 = make_float2(c.l20, c.l20), l21 = make_float2(c.l21, c.l21), l22 = make_float2(c.l22, c.l22);
+  uint32_t* mask = block_mask + ((size_t)b * tiles + I) * tiles * 32 + lane;
+  for (int J0 = 0; J0 < tiles; J0 += kListAtoms / 32) {
+    __syncthreads();
+    for (int t = warp; t < min(kListAtoms / 32, tiles - J0); t += kListWarps) {
+      const int sj = 32 * (J0 + t) + lane;
+      float x = 0.f, y = 0.f, z = 0.f;
+      if (sj < n) {
+        const int aj = pb[sj];
+        x = pos[3 * aj], y = pos[3 * aj + 1], z = pos[3 * aj + 2];
       }
-      __syncthreads();
+      px[32 * t + lane] = -x, py[32 * t + lane] = -y, pz[32 * t + lane] = -z;
+      const float far = warp_max(fabsf(x) + fabsf(y) + fabsf(z));
+      if (lane == 0) reach[t] = far;
     }
-    const float xj = px[at], yj = py[at], zj = pz[at];
-    const bool hit = si < n && sj < n && within_cutoff(xi, yi, zi, xj, yj, zj, c, width, cutoff, cutoff2, margin);
-    const uint32_t word = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) {
-      mask[(size_t)J * 32] = word;
-      if (word) atomicOr(&active[J >> 5], 1u << (J & 31));
+    __syncthreads();
+    for (int t = warp; t < min(kListAtoms / 32, tiles - J0); t += kListWarps) {
+      const int left = n - 32 * (J0 + t);
+      const float limit = fmaf(margin, 1.0001f * (row_reach + reach[t]) + 3.f, cutoff * 1.0001f);
+      uint32_t word = 0u;
+      if (left <= 0 || 32 * I >= n) {
+        // nothing but padding
+      } else if (limit < half_width) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 ax = nearest_image(add2(x2, *reinterpret_cast<const float2*>(&px[32 * t + j])));
+          const float2 ay = nearest_image(add2(y2, *reinterpret_cast<const float2*>(&py[32 * t + j])));
+          const float2 az = nearest_image(add2(z2, *reinterpret_cast<const float2*>(&pz[32 * t + j])));
+          const float2 rx = fma2(az, l20, fma2(ay, l10, mul2(ax, l00))), ry = fma2(az, l21, mul2(ay, l11)), rz = mul2(az, l22);
+          const float2 d2 = fma2(rz, rz, fma2(ry, ry, mul2(rx, rx)));
+          if (d2.x <= cutoff2) word |= 1u << j;
+          if (d2.y <= cutoff2) word |= 2u << j;
+        }
+      } else {
+        for (int j = 0; j < min(left, 32); ++j)
+          if (within_cutoff(__fadd_rn(xi, px[32 * t + j]), __fadd_rn(yi, py[32 * t + j]), __fadd_rn(zi, pz[32 * t + j]), c, width, limit, cutoff2))
+            word |= 1u << j;
+      }
+      if (si >= n) word = 0u;
+      if (left < 32) word &= left > 0 ? (1u << left) - 1u : 0u;
+      mask[(size_t)(J0 + t) * 32] = word;
+      if (__any_sync(0xffffffffu, word != 0u) && lane == 0) atomicOr(&active[(J0 + t) >> 5], 1u << ((J0 + t) & 31));
     }
   }
   __syncthreads();
-  if (r == 0) {
+  if (warp == 0) {
     int32_t* cols = block_cols + ((size_t)b * tiles + I) * tiles;
     int count = 0;
     for (int w = 0; w < words; ++w) {
@@ -291,9 +334,9 @@ int radius_blocks(const float* frac, const float* lattice, const float* cell, co
     const cudaError_t e = cudaFuncSetAttribute(block_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(block_list_kernel)");
   }
-  block_list_kernel<<<dim3(tiles, batch), 1024, words, s>>>(frac, info, num_atoms, perm, n_max, tiles, (float)cutoff, block_mask,
-                                                            block_count, block_cols);
-  MF_CHECK_LAUNCH("block_list_kernel");
+  const cudaError_t e = launch_dependent(block_list_kernel, dim3(tiles, batch), dim3(32 * kListWarps), words, s, frac, info, num_atoms, perm,
+                                         n_max, tiles, (float)cutoff, block_mask, block_count, block_cols);
+  if (e != cudaSuccess) return cuda_error(e, "block_list_kernel");
   return MF_OK;
 }
 

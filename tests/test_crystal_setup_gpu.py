@@ -19,7 +19,7 @@ def _crystals(B, N, seed, lo=8.0, hi=20.0, spread=1.0):
     return lat, torch.rand(B, N, 3, generator=g) * spread - (spread - 1) / 2, n
 
 
-@pytest.mark.parametrize("B,N,cutoff,spread", [(3, 1, 3.0, 1.0), (2, 64, 3.0, 3.0), (2, 65, 9.0, 1.0), (1, 1025, 4.0, 1.0),
+@pytest.mark.parametrize("B,N,cutoff,spread", [(3, 1, 3.0, 1.0), (2, 64, 3.0, 3.0), (2, 65, 9.0, 1.0), (6, 200, 4.5, 1.0), (1, 1025, 4.0, 1.0),
                                                (1, 2049, 2.0, 2.0)])  # fmt: skip
 def test_block_list_from_latents_bit_exact(B, N, cutoff, spread):
     """Atoms per CTA and key-tile edges, cells smaller and larger than the cutoff, coordinates outside [0, 1)."""
