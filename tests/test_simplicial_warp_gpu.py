@@ -100,3 +100,21 @@ def test_bf16_residuals_against_oracle(N, ra, rm, factorized):
     for n in names:  # (a lone token has exact zeros: judge them on the scale of the others)
         err = float((grads[n].float().cpu() - g_ref[n]).abs().max())
         assert err <= max(3e-2 * float(g_ref[n].abs().max()), 1e-2 * largest), f"d{n}: {err}"
+
+
+@pytest.mark.parametrize("B,N,R,D,dtype", [(1, 1, 1, 64, torch.float32), (7, 9, 16, 64, torch.bfloat16), (41, 25, 17, 64, torch.float16),
+                                           (3, 171, 32, 128, torch.bfloat16), (10, 103, 8, 32, torch.float32)])  # fmt: skip
+def test_basis_gradient_sums(B, N, R, D, dtype):
+    """Rows around a round of the cluster (1024, and 512 for wide heads), ranks and channels that do not fill their lanes.  Each sum has
+    B N products of fp32 factors: the largest error is B N 2^-24 of the sum of absolute values."""
+    from matterformer_b200 import _lib
+    H = 3
+    g = torch.Generator("cuda").manual_seed(B)
+    c = torch.randn(B, H, N, R, generator=g, device="cuda")
+    go = torch.randn(B, H, N, D, generator=g, device="cuda").to(dtype)
+    out = torch.empty(H, R, D, device="cuda")
+    code = {torch.float32: _lib.MF_DTYPE_F32, torch.bfloat16: _lib.MF_DTYPE_BF16, torch.float16: _lib.MF_DTYPE_F16}[dtype]
+    _lib.launch(_lib.lib().mf_simplicial_basis_grad, out.device, c.data_ptr(), go.data_ptr(), code, B, H, N, R, D, out.data_ptr())
+    want = torch.einsum("bhir,bhid->hrd", c.double(), go.double())
+    bound = B * N * 2.0**-24 * torch.einsum("bhir,bhid->hrd", c.double().abs(), go.double().abs())
+    assert ((out.double() - want).abs() <= bound + 1e-30).all()
