@@ -73,8 +73,7 @@ constexpr int kAccStride = kD + 4;  // fp32 rows of the gradient stage
 
 template <bool kBias, int RK = 0, int kWarps = 1>
 struct SmallBwdShared {
-  __align__(128) uint8_t tile[6][kSmallTile];  // q, k1, v1, k2, v2, grad_out
-  __nv_bfloat16 dq[kSmallRows][kD];
+  __align__(128) uint8_t tile[6][kSmallTile];  // q (a row becomes dq once its warp is done with it), k1, v1, k2, v2, grad_out
   union {
     float acc[2][kSmallRows][kAccStride];      // sums of the side just walked: first-key and second-key gradient
     float4 dw[4][8][32];                       // K side walk: the warps' dw_jk as the fragments of the logits hold it
@@ -82,6 +81,7 @@ struct SmallBwdShared {
   float lse2[kSmallRows], delta[kSmallRows];
   uint32_t visible[kSmallRows];                // bit k of word j: the pair (j, k) counts
   float4 w[kBias ? 8 : 1][32];                 // bias w_jk as the fragments of the logits hold it
+  float u[kBias ? kSmallRows : 1][kSmallRows], v[kBias ? kSmallRows : 1][kSmallRows], gate[kBias ? kSmallRows : 1];
   // RK > 0: rm^-1/2 dO_i . basis_r, and the residual factors of the query that each warp works on
   float dc[RK ? kSmallRows : 1][RK ? 16 * RK : 1];
   __align__(128) uint8_t factor[RK ? kWarps : 1][4][RK ? 2 * RankTile<RK ? RK : 1>::kTile : 16];
@@ -171,10 +171,7 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, Shared& 
     }
     float ul = 0.f, vl = 0.f, g = 0.f;  // bias: u_i,lane, v_i,lane
     if (bias) {
-      const size_t at = ((size_t)bh * p.N + i) * p.N + lane;
-      ul = lane < n ? p.u[at] : 0.f;
-      vl = lane < n ? p.v_bias[at] : 0.f;
-      g = p.gate[(size_t)bh * p.N + i];
+      ul = sm.u[i][lane], vl = sm.v[i][lane], g = sm.gate[i];
       float ur[MT][2];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
@@ -426,8 +423,9 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, Shared& 
     if constexpr (kKeySide) {
       quad_sum8(dq, lane);
       const int d0 = (4 * (quad & 1) + 2 * (quad >> 1)) * 8 + row8;
-      sm.dq[i][d0] = __float2bfloat16_rn(dq[0] * p.q_scale);
-      sm.dq[i][d0 + 8] = __float2bfloat16_rn(dq[1] * p.q_scale);
+      __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(sm.tile[0]);
+      row[row_chunk(0, i, d0 >> 3) / 2 + (d0 & 7)] = __float2bfloat16_rn(dq[0] * p.q_scale);
+      row[row_chunk(0, i, (d0 >> 3) + 1) / 2 + (d0 & 7)] = __float2bfloat16_rn(dq[1] * p.q_scale);
     }
   }
 
@@ -524,6 +522,23 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
         cp_async16(row_chunk(t0 + t * kSmallTile, r, c), src[t] + (t == 5 ? p.act : p.in).at(b, h, ok ? r : 0) + c * 8, ok);
       }
     }
+    // the bias along with the tiles, so that no query of a walk waits for its rows (256 molecules of 9-29 atoms 193 -> 186 us, 512 of
+    // 10-32 408 -> 389)
+    if (bias) {
+      for (int idx = tid; idx < nq * kSmallRows; idx += kThreads) {
+        const int x = idx >> 5, y = idx & 31;
+        const size_t at = ((size_t)bh * N + x) * N + min(y, n - 1);
+        cp_async4(&sm.u[x][y], p.u + at, y < n);
+        cp_async4(&sm.v[x][y], p.v_bias + at, y < n);
+      }
+      for (int x = tid; x < nq; x += kThreads) cp_async4(&sm.gate[x], p.gate + (size_t)bh * N + x, true);
+      for (int idx = tid; idx < 4 * 8 * 32; idx += kThreads) {
+        const int f = idx >> 7, ln = (idx >> 2) & 31, e = idx & 3;
+        const int j = (f >> 2) * 16 + 8 * (e >> 1) + (ln >> 2), k = (f & 3) * 8 + 2 * (ln & 3) + (e & 1);
+        const bool ok = j < n && k < n;
+        cp_async4(reinterpret_cast<float*>(&sm.w[f][ln]) + e, p.w + (size_t)bh * N * N + (ok ? j * N + k : 0), ok);
+      }
+    }
     cp_async_commit();
   }
   bool hole = (kmask & (kmask + 1)) != 0u;
@@ -536,22 +551,9 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
     }
     if (lane == 0) sm.visible[j] = word;
   }
-  for (int idx = tid; idx < kSmallRows * kD / 8; idx += kThreads) reinterpret_cast<float4*>(sm.dq)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
   if constexpr (RK > 0) {
     for (int idx = tid; idx < (int)sizeof(sm.factor) / 16; idx += kThreads)
       reinterpret_cast<float4*>(sm.factor)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  if (bias) {
-    for (int idx = tid; idx < 8 * 32; idx += kThreads) {
-      const int f = idx >> 5, ln = idx & 31, j = (f >> 2) * 16 + (ln >> 2), k = (f & 3) * 8 + 2 * (ln & 3);
-      const float* w = p.w + (size_t)bh * N * N;
-      float4 v;
-      v.x = (j < n && k < n) ? w[j * N + k] : 0.f;
-      v.y = (j < n && k + 1 < n) ? w[j * N + k + 1] : 0.f;
-      v.z = (j + 8 < n && k < n) ? w[(j + 8) * N + k] : 0.f;
-      v.w = (j + 8 < n && k + 1 < n) ? w[(j + 8) * N + k + 1] : 0.f;
-      sm.w[f][ln] = v;
-    }
   }
   // delta_i = dO_i . out_i, eight lanes per query
   for (int idx = tid; idx < ((8 * nq + 31) & ~31); idx += kThreads) {
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
   for (int idx = tid; idx < (n > 0 ? 1 : 5) * 8 * N; idx += kThreads) {
     const int t = idx / (8 * N), rem = idx - t * 8 * N, r = rem >> 3, c = rem & 7;
     *reinterpret_cast<uint4*>(dst[t] + p.in.at(b, h, r) + 8 * c) =
-        t == 0 ? *reinterpret_cast<const uint4*>(&sm.dq[r][8 * c]) : make_uint4(0u, 0u, 0u, 0u);
+        t == 0 && r < nq && ((qmask >> r) & 1u) ? *reinterpret_cast<const uint4*>(sm.tile[0] + row_chunk(0, r, c)) : make_uint4(0u, 0u, 0u, 0u);
   }
   if constexpr (RK > 0) {  // residual gradients of queries that no warp took
     float* rows[6] = {p.dal, p.dar, p.dml, p.dmr, p.dagate, p.mcoef};

@@ -45,6 +45,10 @@ __device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gptr,
   const int bytes = valid ? 16 : 0;  // zero-fill when the source row does not exist
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr), "l"(gptr), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async4(float* smem, const float* gptr, bool valid) {
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at), "l"(gptr), "r"(valid ? 4 : 0) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
