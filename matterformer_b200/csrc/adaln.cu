@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
                                                                          float eps, TH* __restrict__ h,
                                                                          float* __restrict__ mean_out,
                                                                          float* __restrict__ rstd_out,
-                                                                         GatedInput<TX, TH> in = {}) {
+                                                                         GatedInput<TX, TH> in) {
+  wait_for_previous();
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* sh = shift + (size_t)b * C;
   const float* sc = scale + (size_t)b * C;
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_bwd_kernel(const T
                                                                          float* __restrict__ dscale,
                                                                          const TX* __restrict__ add) {
   extern __shared__ __align__(16) float part[];  // [kAdaWarps][C]
+  wait_for_previous();
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* sc = scale + (size_t)b * C;
   const int nvec = C >> 3;
@@ -278,6 +280,7 @@ template <typename TX, typename TA>
 __global__ void gated_residual_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gate,
                                           const TA* __restrict__ a, const uint8_t* __restrict__ pad, int N, int C,
                                           long long total, TX* __restrict__ y) {
+  wait_for_previous();
   const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (i >= total) return;
   const int c = (int)(i % C);
@@ -304,6 +307,7 @@ __global__ void __launch_bounds__(kAdaWarps * 32) gated_residual_bwd_kernel(cons
                                                                             TA* __restrict__ da, TX* __restrict__ dx,
                                                                             float* __restrict__ dgate) {
   extern __shared__ __align__(16) float part[];  // [kAdaWarps][C]
+  wait_for_previous();
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* gt = gate + (size_t)b * C;
   const int nvec = C >> 3;
@@ -410,9 +414,9 @@ extern "C" int mf_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* s
   const dim3 grid = rows_grid(batch, tokens);
   MF_ADA_DISPATCH(x_dtype, h_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
-                             (ln_modulate_fwd_kernel<TX, TH, VEC><<<grid, kAdaWarps * 32, 0, s>>>(
-                                 static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
-                                 rstd))));
+                             launch_dependent(ln_modulate_fwd_kernel<TX, TH, VEC>, grid, dim3(kAdaWarps * 32), 0, s,
+                                              static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
+                                              rstd, GatedInput<TX, TH>{})));
   MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
   return MF_OK;
 }
@@ -430,9 +434,9 @@ extern "C" int mf_gated_ln_modulate_fwd(const void* x, int32_t x_dtype, const fl
   const dim3 grid = rows_grid(batch, tokens);
   MF_ADA_DISPATCH(x_dtype, h_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
-                             (ln_modulate_fwd_kernel<TX, TH, VEC, true><<<grid, kAdaWarps * 32, 0, s>>>(
-                                 static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
-                                 rstd, GatedInput<TX, TH>{gate, static_cast<const TH*>(a), pad, static_cast<TX*>(y)}))));
+                             launch_dependent(ln_modulate_fwd_kernel<TX, TH, VEC, true>, grid, dim3(kAdaWarps * 32), 0, s,
+                                              static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
+                                              rstd, GatedInput<TX, TH>{gate, static_cast<const TH*>(a), pad, static_cast<TX*>(y)})));
   MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
   return MF_OK;
 }
@@ -451,7 +455,7 @@ extern "C" int mf_ln_modulate_add_bwd(const void* dh, int32_t dh_dtype, const vo
   MF_ADA_DISPATCH(x_dtype, dh_dtype, TX, TH,
                   MF_ADA_VEC(channels, VEC,
                              auto kernel = add ? ln_modulate_bwd_kernel<TX, TH, VEC, true> : ln_modulate_bwd_kernel<TX, TH, VEC, false>;
-                             kernel<<<batch, kAdaWarps * 32, smem, s>>>(
+                             launch_dependent(kernel, dim3(batch), dim3(kAdaWarps * 32), smem, s,
                                  static_cast<const TH*>(dh), static_cast<const TX*>(x), scale, mean, rstd, tokens, channels,
                                  static_cast<TX*>(dx), dshift, dscale, static_cast<const TX*>(add))));
   MF_CHECK_LAUNCH("ln_modulate_bwd_kernel");
@@ -478,9 +482,8 @@ extern "C" int mf_gated_residual_fwd(const void* x, int32_t x_dtype, const float
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned blocks = (unsigned)((total / 8 + 255) / 256);
   MF_ADA_DISPATCH(x_dtype, a_dtype, TX, TA,
-                  (gated_residual_fwd_kernel<TX, TA><<<blocks, 256, 0, s>>>(
-                      static_cast<const TX*>(x), gate, static_cast<const TA*>(a), pad, tokens, channels, total,
-                      static_cast<TX*>(y))));
+                  launch_dependent(gated_residual_fwd_kernel<TX, TA>, dim3(blocks), dim3(256), 0, s, static_cast<const TX*>(x), gate,
+                                   static_cast<const TA*>(a), pad, tokens, channels, total, static_cast<TX*>(y)));
   MF_CHECK_LAUNCH("gated_residual_fwd_kernel");
   return MF_OK;
 }
@@ -498,9 +501,9 @@ extern "C" int mf_gated_residual_bwd(const void* dy, int32_t dy_dtype, const flo
   const size_t smem = (size_t)kAdaWarps * channels * sizeof(float);
   MF_ADA_DISPATCH(dy_dtype, a_dtype, TX, TA,
                   MF_ADA_VEC(channels, VEC,
-                             (gated_residual_bwd_kernel<TX, TA, VEC><<<batch, kAdaWarps * 32, smem, s>>>(
-                                 static_cast<const TX*>(dy), gate, static_cast<const TA*>(a), pad, tokens, channels,
-                                 static_cast<TA*>(da), static_cast<TX*>(dx), dgate))));
+                             launch_dependent(gated_residual_bwd_kernel<TX, TA, VEC>, dim3(batch), dim3(kAdaWarps * 32), smem, s,
+                                              static_cast<const TX*>(dy), gate, static_cast<const TA*>(a), pad, tokens, channels,
+                                              static_cast<TA*>(da), static_cast<TX*>(dx), dgate)));
   MF_CHECK_LAUNCH("gated_residual_bwd_kernel");
   return MF_OK;
 }

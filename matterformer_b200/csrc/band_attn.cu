@@ -111,6 +111,7 @@ __device__ __forceinline__ void store_rows(__nv_bfloat16* dst, long long stride,
 template <int W, int kRows>
 __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 128 ? 2 : 4) : (kRows == 128 ? 3 : 6)) band_fwd_kernel(const __grid_constant__ BandParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
+  wait_for_previous();
   constexpr bool kDense = W == 0;
   constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = kDense ? kRows / 16 : W / 16 + 1;
   constexpr int kTv = kHalo * kRowBytes, kTq = 2 * kTv;
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
 template <int W, int kRows>
 __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 128 ? 1 : 2) : (W == 128 ? 2 : 3)) band_bwd_kernel(const __grid_constant__ BandParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
+  wait_for_previous();
   constexpr bool kDense = W == 0;
   constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = kDense ? kRows / 16 : W / 16 + 1;
   constexpr int kTk = kHalo * kRowBytes, kTv = 2 * kTk, kTg = 3 * kTk;  // q, k, v, grad_out
@@ -367,7 +369,7 @@ int launch_band(const BandParams& p, int BH, bool backward, cudaStream_t s) {
   auto kernel = backward ? band_bwd_kernel<W, kRows> : band_fwd_kernel<W, kRows>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(band_attn_kernel)");
-  kernel<<<dim3((p.N + kRows - 1) / kRows, BH), kRows * 2, bytes, s>>>(p);
+  launch_dependent(kernel, dim3((p.N + kRows - 1) / kRows, BH), dim3(kRows * 2), bytes, s, p);
   MF_CHECK_LAUNCH("band_attn_kernel");
   return MF_OK;
 }

@@ -86,6 +86,7 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
 
 template <typename T>
 __global__ void gelu_tanh_fwd_kernel(const T* __restrict__ x, long long n, T* __restrict__ y) {
+  wait_for_previous();
   const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (i >= n) return;
   float v[8];
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_sums_band_kernel(const T* 
                                                                       T* __restrict__ dx, long long rows, int C,
                                                                       long long rows_per_band, float* __restrict__ part) {
   __shared__ float red[kWarps][kColsPerBlock];
+  wait_for_previous();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * kColsPerBlock + 8 * lane;
   const long long r0 = (long long)blockIdx.y * rows_per_band;
@@ -166,6 +168,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_sums_band_kernel(const T* 
 __global__ void __launch_bounds__(256) column_sums_final_kernel(const float* __restrict__ part, int bands, int C,
                                                                 float* __restrict__ out) {
   __shared__ float red[8][32];
+  wait_for_previous();
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + x;
   float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
@@ -229,13 +232,13 @@ extern "C" int mf_column_sums(const void* x, int32_t dtype, int64_t rows, int32_
   const long long rows_per_band = (rows + bands - 1) / bands;
   const dim3 grid((cols + kColsPerBlock - 1) / kColsPerBlock, bands);
   if (dtype == MF_DTYPE_BF16)
-    column_sums_band_kernel<__nv_bfloat16, false><<<grid, kWarps * 32, 0, s>>>(static_cast<const __nv_bfloat16*>(x), nullptr,
-                                                                               nullptr, rows, cols, rows_per_band, part);
+    launch_dependent(column_sums_band_kernel<__nv_bfloat16, false>, grid, dim3(kWarps * 32), 0, s, static_cast<const __nv_bfloat16*>(x),
+                     nullptr, nullptr, rows, cols, rows_per_band, part);
   else
-    column_sums_band_kernel<float, false><<<grid, kWarps * 32, 0, s>>>(static_cast<const float*>(x), nullptr, nullptr, rows,
-                                                                       cols, rows_per_band, part);
+    launch_dependent(column_sums_band_kernel<float, false>, grid, dim3(kWarps * 32), 0, s, static_cast<const float*>(x), nullptr, nullptr,
+                     rows, cols, rows_per_band, part);
   MF_CHECK_LAUNCH("column_sums_band_kernel");
-  column_sums_final_kernel<<<(cols + 31) / 32, 256, 0, s>>>(part, bands, cols, out);
+  launch_dependent(column_sums_final_kernel, dim3((cols + 31) / 32), dim3(256), 0, s, part, bands, cols, out);
   MF_CHECK_LAUNCH("column_sums_final_kernel");
   return MF_OK;
 }
@@ -250,10 +253,10 @@ extern "C" int mf_gelu_tanh_fwd(const void* x, int32_t dtype, int64_t n, void* y
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned blocks = (unsigned)((n / 8 + 255) / 256);
   if (dtype == MF_DTYPE_BF16)
-    gelu_tanh_fwd_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), n,
-                                                                static_cast<__nv_bfloat16*>(y));
+    launch_dependent(gelu_tanh_fwd_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, s, static_cast<const __nv_bfloat16*>(x), n,
+                     static_cast<__nv_bfloat16*>(y));
   else
-    gelu_tanh_fwd_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), n, static_cast<float*>(y));
+    launch_dependent(gelu_tanh_fwd_kernel<float>, dim3(blocks), dim3(256), 0, s, static_cast<const float*>(x), n, static_cast<float*>(y));
   MF_CHECK_LAUNCH("gelu_tanh_fwd_kernel");
   return MF_OK;
 }
@@ -281,14 +284,13 @@ extern "C" int mf_gelu_tanh_bwd(const void* x, const void* dy, int32_t dtype, in
   const long long rows_per_band = (rows + bands - 1) / bands;
   const dim3 grid((cols + kColsPerBlock - 1) / kColsPerBlock, bands);
   if (dtype == MF_DTYPE_BF16)
-    column_sums_band_kernel<__nv_bfloat16, true><<<grid, kWarps * 32, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), rows,
-        cols, rows_per_band, part);
+    launch_dependent(column_sums_band_kernel<__nv_bfloat16, true>, grid, dim3(kWarps * 32), 0, s, static_cast<const __nv_bfloat16*>(x),
+                     static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), rows, cols, rows_per_band, part);
   else
-    column_sums_band_kernel<float, true><<<grid, kWarps * 32, 0, s>>>(static_cast<const float*>(x), static_cast<const float*>(dy),
-                                                                      static_cast<float*>(dx), rows, cols, rows_per_band, part);
+    launch_dependent(column_sums_band_kernel<float, true>, grid, dim3(kWarps * 32), 0, s, static_cast<const float*>(x),
+                     static_cast<const float*>(dy), static_cast<float*>(dx), rows, cols, rows_per_band, part);
   MF_CHECK_LAUNCH("column_sums_band_kernel");
-  column_sums_final_kernel<<<(cols + 31) / 32, 256, 0, s>>>(part, bands, cols, column_sums);
+  launch_dependent(column_sums_final_kernel, dim3((cols + 31) / 32), dim3(256), 0, s, part, bands, cols, column_sums);
   MF_CHECK_LAUNCH("column_sums_final_kernel");
   return MF_OK;
 }

@@ -17,6 +17,7 @@ __device__ __forceinline__ float masked_sum_at(const MfMaskedSumArgs& p, float a
 }
 
 __global__ void __launch_bounds__(kSumThreads) masked_sum_kernel(const __grid_constant__ MfMaskedSumArgs p) {
+  wait_for_previous();
   const int b = blockIdx.x, tid = threadIdx.x, N = p.tokens, C = p.channels;
   const float a = p.a ? p.a[b] : p.a_value, c = p.c ? p.c[b] : p.c_value;
   const uint8_t* pad = p.pad + (size_t)b * N;
@@ -62,7 +63,7 @@ extern "C" int mf_masked_sum(const MfMaskedSumArgs* p, void* stream) {
   MF_CHECK_ARG((long long)p->tokens * p->channels < (1ll << 31), "mf_masked_sum: molecule too large");
   if (p->batch == 0 || p->tokens == 0 || p->channels == 0) return MF_OK;
   MF_CHECK_ARG(p->x && p->pad && p->out && (!p->p || p->q) && (!p->z || p->y), "mf_masked_sum: null pointer argument");
-  masked_sum_kernel<<<p->batch, kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(*p);
+  launch_dependent(masked_sum_kernel, dim3(p->batch), dim3(kSumThreads), 0, static_cast<cudaStream_t>(stream), *p);
   MF_CHECK_LAUNCH("masked_sum_kernel");
   return MF_OK;
 }

@@ -87,6 +87,7 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadParams p) {
   constexpr int U = MODE == kBackwardRows ? 1 : 2;  // partners per step of the walk
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  wait_for_previous();
   PairShared& sm = *reinterpret_cast<PairShared*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = p.tokens;
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
 
 // out_i = raw_i - mean over the molecule's real atoms; zero on padding.  One warp per molecule.
 __global__ void pair_head_center_kernel(float* out, const uint8_t* valid, int batch, int tokens) {
+  wait_for_previous();
   const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (b >= batch) return;
   float* o = out + (size_t)b * tokens * 3;
@@ -395,7 +397,7 @@ int grid_size_dtype(int dtype, long long items, int* blocks) {
 
 template <typename T, int MODE>
 int launch(const PairHeadParams& p, int blocks, cudaStream_t s) {
-  pair_head_kernel<T, MODE><<<blocks, kWarps * 32, sizeof(PairShared), s>>>(p);
+  launch_dependent(pair_head_kernel<T, MODE>, dim3(blocks), dim3(kWarps * 32), sizeof(PairShared), s, p);
   MF_CHECK_LAUNCH("pair_head_kernel");
   return MF_OK;
 }
@@ -449,7 +451,7 @@ extern "C" int mf_pair_head_fwd(const MfPairHeadArgs* a, void* stream) {
   p.rows_per_item = rows;
   rc = launch_dtype<kForward>(a->dtype, p, blocks, s);
   if (rc != MF_OK) return rc;
-  pair_head_center_kernel<<<(a->batch + 7) / 8, 256, 0, s>>>(a->out, a->valid, a->batch, a->tokens);
+  launch_dependent(pair_head_center_kernel, dim3((a->batch + 7) / 8), dim3(256), 0, s, a->out, a->valid, a->batch, a->tokens);
   MF_CHECK_LAUNCH("pair_head_center_kernel");
   return MF_OK;
 }

@@ -500,6 +500,7 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
   extern __shared__ __align__(128) uint8_t smem[];
   using Shared = SmallBwdShared<kBias, RK, kWarps>;
   Shared& sm = *reinterpret_cast<Shared*>(smem);
+  wait_for_previous();
   const bool bias = kBias && (RK == 0 || p.u != nullptr);
   constexpr int kThreads = 32 * kWarps;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -693,7 +694,7 @@ int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layout
   do {                                                                                                                 \
     constexpr int bytes = (int)sizeof(SmallBwdShared<BIAS, RK, S>);                                                        \
     e = cudaFuncSetAttribute(simplicial_small_bwd_kernel<BIAS, RK, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
-    if (e == cudaSuccess) simplicial_small_bwd_kernel<BIAS, RK, S><<<bh, 32 * S, bytes, stream>>>(p);                      \
+    if (e == cudaSuccess) launch_dependent(simplicial_small_bwd_kernel<BIAS, RK, S>, dim3(bh), dim3(32 * S), bytes, stream, p);                      \
   } while (0)
   if (a.angle_left || a.message_left) {
     if (max(p.ra, p.rm) <= 16) MF_LAUNCH(true, 1, 4);

@@ -275,6 +275,7 @@ __device__ __forceinline__ void small_fwd_rows(const SmallFwdParams& p, SmallFwd
 template <bool kBias, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, kBias ? 12 / kWarps : (kWarps == 4 ? 4 : 14 / kWarps)) simplicial_small_fwd_kernel(const __grid_constant__ SmallFwdParams p) {
   __shared__ SmallFwdShared<kBias> sm;
+  wait_for_previous();
   const int tid = threadIdx.x, lane = tid & 31;
   const int N = p.N, h = blockIdx.x % p.H, b = p.order ? p.order[blockIdx.x / p.H] : blockIdx.x / p.H, bh = b * p.H + h;
   const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBias ? 12 / kWarps : (kWarps == 
 __global__ void __launch_bounds__(1024) simplicial_small_order_kernel(const uint8_t* __restrict__ key_valid, int B, int N, int32_t* keys,
                                                                      int32_t* order) {
   __shared__ int start[kSmallRows + 1];
+  wait_for_previous();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid <= kSmallRows) start[tid] = 0;
   __syncthreads();
@@ -390,7 +392,7 @@ int simplicial_small_order(const uint8_t* key_valid, int batch, int tokens, void
   *order = nullptr;
   if (need == 0 || !workspace || workspace_bytes < need) return MF_OK;  // (a caller may leave it out)
   int32_t* keys = static_cast<int32_t*>(workspace);
-  simplicial_small_order_kernel<<<1, 1024, 0, stream>>>(key_valid, batch, tokens, keys, keys + batch);
+  launch_dependent(simplicial_small_order_kernel, dim3(1), dim3(1024), 0, stream, key_valid, batch, tokens, keys, keys + batch);
   MF_CHECK_LAUNCH("simplicial_small_order_kernel");
   *order = keys + batch;
   return MF_OK;
@@ -427,7 +429,7 @@ int simplicial_small_fwd(const MfSimplicialFwdArgs& a, const TileLayouts* layout
   // 148; with the bias 23.9 | 23.3, 57.2 | 56.9, 119 | 123, 222 | 239.
   const int warps = bh >= 4096 ? 2 : 4;
   profile_mark(MF_PROFILE_SIMPLICIAL_FWD, true, stream);
-#define MF_LAUNCH(BIAS, W) simplicial_small_fwd_kernel<BIAS, W><<<bh, 32 * W, 0, stream>>>(p)
+#define MF_LAUNCH(BIAS, W) launch_dependent(simplicial_small_fwd_kernel<BIAS, W>, dim3(bh), dim3(32 * W), 0, stream, p)
   if (a.u) {
     if (warps == 2) MF_LAUNCH(true, 2);
     else MF_LAUNCH(true, 4);
