@@ -471,6 +471,47 @@ int mf_ln_modulate_add_bwd(const void* dh, int32_t dh_dtype, const void* x, int3
                            int32_t channels, void* dx, float* dshift, float* dscale, void* stream);
 
 /*
+ * The same with a norm that has no modulation and is kept in fp32 (the trunk's output norm): a in a_dtype, h fp32.
+ */
+int mf_gated_layer_norm_fwd(const void* x, int32_t x_dtype, const float* gate, const void* a, int32_t a_dtype, const uint8_t* pad,
+                            int32_t batch, int32_t tokens, int32_t channels, float eps, void* y, float* h, float* mean, float* rstd,
+                            void* stream);
+/* h = LayerNorm(x) * weight + bias over (rows, C), in h_dtype; mean and rstd (rows) fp32 are what the backward calls above take. */
+int mf_layer_norm_fwd(const void* x, int32_t x_dtype, const float* weight, const float* bias, int32_t rows, int32_t channels, float eps,
+                      int32_t h_dtype, void* h, float* mean, float* rstd, void* stream);
+
+/* ------------------------------------------------------------------------- */
+/* Around the trunk: a few numbers per molecule, one launch each              */
+/* ------------------------------------------------------------------------- */
+/*
+ * From noise levels sigma (B) fp32: scalings (3,B) = sd^2 / (sigma^2 + sd^2), sigma sd / sqrt(sigma^2 + sd^2),
+ * 1 / sqrt(sigma^2 + sd^2) (EDMPreconditioner, tasks/edm.py:34-81) and noise (B) = log(max(sigma, 1e-8)) / 4
+ * (models/qm9.py:509-565); either may be NULL.
+ */
+int mf_edm_scalings(const float* sigma, int32_t batch, double sigma_data, float* scalings, float* noise, void* stream);
+/* out (B, 4 half) = [cos, sin, cos, sin](2 pi t f), f_i = 10000^(-i/half): TimeEmbedder of one level given twice, models/embeddings.py:9-44. */
+int mf_time_embedding(const float* t, int32_t batch, int32_t half, int32_t dtype, void* out, void* stream);
+/* valid (B,N) = 1 where pad is 0, else 0; counts (B) = their sums. */
+int mf_pad_counts(const uint8_t* pad, int32_t batch, int32_t tokens, uint8_t* valid, int32_t* counts, void* stream);
+/*
+ * Token projection of the model, models/qm9.py:509-565: out (B,N,C) bf16 = W [x, noise_b] + bias with inputs and parameters rounded to
+ * bf16 and fp32 sums, zeros where pad is set.  x (B,N,inputs-1) fp32, weight (C,inputs) and bias (C) fp32, inputs <= 8, C a multiple
+ * of 64 up to 1024.  The backward call takes dy (B,N,C) bf16 and writes grads: C * inputs of the weight, then C of the bias, summed in
+ * a fixed order; padded rows count for nothing.
+ */
+int mf_token_projection_fwd(const float* x, const float* noise, const uint8_t* pad, const float* weight, const float* bias, int32_t batch,
+                            int32_t tokens, int32_t inputs, int32_t channels, void* out, void* stream);
+size_t mf_token_projection_bwd_workspace_bytes(int32_t batch, int32_t tokens, int32_t inputs, int32_t channels);
+int mf_token_projection_bwd(const void* dy, const float* x, const float* noise, const uint8_t* pad, int32_t batch, int32_t tokens,
+                            int32_t inputs, int32_t channels, float* grads, void* workspace, size_t workspace_bytes, void* stream);
+/*
+ * Modulation vectors, transformer.py:242-244: mod (B, groups*C) bf16 <-> groups fp32 matrices (B,C).  The split writes (groups,B,C);
+ * the merge reads `groups` pointers on the host (NULL: zeros) and rounds to bf16.  groups <= 128, C a multiple of 8 up to 4096.
+ */
+int mf_split_modulation(const void* mod, int32_t batch, int32_t groups, int32_t channels, float* out, void* stream);
+int mf_merge_modulation(const float* const* grads, int32_t batch, int32_t groups, int32_t channels, void* out, void* stream);
+
+/*
  * y = x + gate[b,:] * a, the gated residual of AdaLNBlock.forward, transformer.py:308-316.  x, y (B,N,C) fp32 or bf16
  * (x_dtype), gate fp32 (B,C), a fp32 or bf16 (a_dtype).  `pad` (NULL or (B,N) bytes, non-zero = padded token) folds in
  * the `x.masked_fill(pad_mask[..., None], 0)` that the trunk applies before the next block (transformer.py, the loop

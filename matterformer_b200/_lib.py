@@ -68,6 +68,16 @@ EXPORTED_SYMBOLS = (
     "mf_ln_modulate_bwd",
     "mf_gated_ln_modulate_fwd",
     "mf_ln_modulate_add_bwd",
+    "mf_gated_layer_norm_fwd",
+    "mf_layer_norm_fwd",
+    "mf_edm_scalings",
+    "mf_time_embedding",
+    "mf_pad_counts",
+    "mf_token_projection_fwd",
+    "mf_token_projection_bwd_workspace_bytes",
+    "mf_token_projection_bwd",
+    "mf_split_modulation",
+    "mf_merge_modulation",
     "mf_masked_sum",
     "mf_gated_residual_fwd",
     "mf_gated_residual_bwd",
@@ -367,6 +377,22 @@ def lib() -> ctypes.CDLL:
     L.mf_gated_residual_bwd.argtypes = [c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int32,
                                         c_int32, c_void_p, c_void_p, c_void_p, c_void_p]  # fmt: skip
     L.mf_gated_residual_bwd.restype = c_int32
+    for fn, types in (
+        (L.mf_gated_layer_norm_fwd, [c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int32, c_int32, c_float, c_void_p,
+                                     c_void_p, c_void_p, c_void_p, c_void_p]),
+        (L.mf_layer_norm_fwd, [c_void_p, c_int32, c_void_p, c_void_p, c_int32, c_int32, c_float, c_int32, c_void_p, c_void_p, c_void_p,
+                               c_void_p]),
+        (L.mf_edm_scalings, [c_void_p, c_int32, c_double, c_void_p, c_void_p, c_void_p]),
+        (L.mf_time_embedding, [c_void_p, c_int32, c_int32, c_int32, c_void_p, c_void_p]),
+        (L.mf_pad_counts, [c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_void_p]),
+        (L.mf_token_projection_fwd, [c_void_p] * 5 + [c_int32] * 4 + [c_void_p] * 2),
+        (L.mf_token_projection_bwd, [c_void_p] * 4 + [c_int32] * 4 + [c_void_p] * 2 + [c_size_t, c_void_p]),
+        (L.mf_split_modulation, [c_void_p, c_int32, c_int32, c_int32, c_void_p, c_void_p]),
+        (L.mf_merge_modulation, [c_void_p, c_int32, c_int32, c_int32, c_void_p, c_void_p]),
+    ):  # fmt: skip
+        fn.argtypes, fn.restype = types, c_int32
+    L.mf_token_projection_bwd_workspace_bytes.argtypes = [c_int32] * 4
+    L.mf_token_projection_bwd_workspace_bytes.restype = c_size_t
     L.mf_column_sums_workspace_bytes.argtypes = [ctypes.c_int64, c_int32]
     L.mf_column_sums_workspace_bytes.restype = c_size_t
     L.mf_column_sums.argtypes = [c_void_p, c_int32, ctypes.c_int64, c_int32, c_void_p, c_void_p, c_size_t, c_void_p]

@@ -84,14 +84,15 @@ struct GatedInput {
 
 // kGated: one pass for the gated residual and the norm behind it.  Bound by a row's chain of loads and reductions (3.9 TB/s):
 // 33 -> 31 us for 29 696 rows of 512 in bf16; for 1 856 rows 5.4 -> 3.6 us, the launch it saves.
-template <typename TX, typename TH, int VEC, bool kGated = false>
+// shift and scale may be absent; `one` + scale_b multiplies the row (1 for a modulation, 0 where scale is an affine norm's weight).
+template <typename TX, typename TH, int VEC, bool kGated = false, typename TA = TH>
 __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const TX* __restrict__ x,
                                                                          const float* __restrict__ shift,
                                                                          const float* __restrict__ scale, int N, int C,
                                                                          float eps, TH* __restrict__ h,
                                                                          float* __restrict__ mean_out,
                                                                          float* __restrict__ rstd_out,
-                                                                         GatedInput<TX, TH> in) {
+                                                                         GatedInput<TX, TA> in, float one) {
   wait_for_previous();
   const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* sh = shift + (size_t)b * C;
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
         ld8<TX>(xr + 8 * v, xv[t]);
         if constexpr (kGated) {
           float av[8], gv[8];
-          ld8<TH>(in.a + row * C + 8 * v, av);
+          ld8<TA>(in.a + row * C + 8 * v, av);
           ld8<float>(in.gate + (size_t)b * C + 8 * v, gv);
           const bool hidden = in.pad && in.pad[row];
 #pragma unroll
@@ -121,8 +122,13 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
           }
           st8<TX>(in.y + row * C + 8 * v, xv[t]);
         }
-        ld8<float>(sc + 8 * v, scv[t]);
-        ld8<float>(sh + 8 * v, shv[t]);
+        if (scale) {
+          ld8<float>(sc + 8 * v, scv[t]);
+          ld8<float>(sh + 8 * v, shv[t]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) scv[t][e] = shv[t][e] = 0.f;
+        }
 #pragma unroll
         for (int e = 0; e < 8; ++e) s += xv[t][e];
       }
@@ -146,7 +152,7 @@ __global__ void __launch_bounds__(kAdaWarps * 32) ln_modulate_fwd_kernel(const T
       if (v < nvec) {
         float out[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) out[e] = fmaf((xv[t][e] - mean) * rstd, 1.f + scv[t][e], shv[t][e]);
+        for (int e = 0; e < 8; ++e) out[e] = fmaf((xv[t][e] - mean) * rstd, one + scv[t][e], shv[t][e]);
         st8<TH>(h + row * C + 8 * v, out);
       }
     }
@@ -416,7 +422,7 @@ extern "C" int mf_ln_modulate_fwd(const void* x, int32_t x_dtype, const float* s
                   MF_ADA_VEC(channels, VEC,
                              launch_dependent(ln_modulate_fwd_kernel<TX, TH, VEC>, grid, dim3(kAdaWarps * 32), 0, s,
                                               static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
-                                              rstd, GatedInput<TX, TH>{})));
+                                              rstd, GatedInput<TX, TH>{}, 1.f)));
   MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
   return MF_OK;
 }
@@ -436,7 +442,45 @@ extern "C" int mf_gated_ln_modulate_fwd(const void* x, int32_t x_dtype, const fl
                   MF_ADA_VEC(channels, VEC,
                              launch_dependent(ln_modulate_fwd_kernel<TX, TH, VEC, true>, grid, dim3(kAdaWarps * 32), 0, s,
                                               static_cast<const TX*>(x), shift, scale, tokens, channels, eps, static_cast<TH*>(h), mean,
-                                              rstd, GatedInput<TX, TH>{gate, static_cast<const TH*>(a), pad, static_cast<TX*>(y)})));
+                                              rstd, GatedInput<TX, TH>{gate, static_cast<const TH*>(a), pad, static_cast<TX*>(y)}, 1.f)));
+  MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
+  return MF_OK;
+}
+
+// The last gated residual of a stack and the norm behind it, which has no modulation and is kept in fp32.
+extern "C" int mf_gated_layer_norm_fwd(const void* x, int32_t x_dtype, const float* gate, const void* a, int32_t a_dtype, const uint8_t* pad,
+                                       int32_t batch, int32_t tokens, int32_t channels, float eps, void* y, float* h, float* mean, float* rstd,
+                                       void* stream) {
+  int rc = check_sizes("mf_gated_layer_norm_fwd", batch, tokens, channels, a_dtype);
+  if (rc == MF_OK) rc = check_sizes("mf_gated_layer_norm_fwd", batch, tokens, channels, x_dtype);
+  if (rc != MF_OK) return rc;
+  if (batch == 0 || tokens == 0) return MF_OK;
+  MF_CHECK_ARG(x && gate && a && y && h && mean && rstd, "mf_gated_layer_norm_fwd: null pointer argument");
+  MF_CHECK_ALIGNED("mf_gated_layer_norm_fwd", x, gate, a, y, h);
+  MF_ADA_DISPATCH(x_dtype, a_dtype, TX, TA,
+                  MF_ADA_VEC(channels, VEC,
+                             launch_dependent(ln_modulate_fwd_kernel<TX, float, VEC, true, TA>, rows_grid(batch, tokens), dim3(kAdaWarps * 32), 0,
+                                              static_cast<cudaStream_t>(stream), static_cast<const TX*>(x), nullptr, nullptr, tokens, channels,
+                                              eps, h, mean, rstd,
+                                              GatedInput<TX, TA>{gate, static_cast<const TA*>(a), pad, static_cast<TX*>(y)}, 1.f)));
+  MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
+  return MF_OK;
+}
+
+// An affine LayerNorm over rows, its result in h's type.
+extern "C" int mf_layer_norm_fwd(const void* x, int32_t x_dtype, const float* weight, const float* bias, int32_t rows, int32_t channels,
+                                 float eps, int32_t h_dtype, void* h, float* mean, float* rstd, void* stream) {
+  int rc = check_sizes("mf_layer_norm_fwd", 1, rows, channels, h_dtype);
+  if (rc == MF_OK) rc = check_sizes("mf_layer_norm_fwd", 1, rows, channels, x_dtype);
+  if (rc != MF_OK) return rc;
+  if (rows == 0) return MF_OK;
+  MF_CHECK_ARG(x && weight && bias && h && mean && rstd, "mf_layer_norm_fwd: null pointer argument");
+  MF_CHECK_ALIGNED("mf_layer_norm_fwd", x, weight, bias, h);
+  MF_ADA_DISPATCH(x_dtype, h_dtype, TX, TH,
+                  MF_ADA_VEC(channels, VEC,
+                             launch_dependent(ln_modulate_fwd_kernel<TX, TH, VEC>, rows_grid(1, rows), dim3(kAdaWarps * 32), 0,
+                                              static_cast<cudaStream_t>(stream), static_cast<const TX*>(x), bias, weight, rows, channels, eps,
+                                              static_cast<TH*>(h), mean, rstd, GatedInput<TX, TH>{}, 0.f)));
   MF_CHECK_LAUNCH("ln_modulate_fwd_kernel");
   return MF_OK;
 }

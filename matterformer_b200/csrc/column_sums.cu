@@ -203,6 +203,12 @@ int bands_for(long long rows, int cols) {
 }
 
 }  // namespace
+
+int add_bands(const float* part, int bands, int cols, float* out, cudaStream_t stream) {
+  launch_dependent(column_sums_final_kernel, dim3((cols + 31) / 32), dim3(256), 0, stream, part, bands, cols, out);
+  MF_CHECK_LAUNCH("column_sums_final_kernel");
+  return MF_OK;
+}
 }  // namespace mf
 
 using namespace mf;
@@ -238,9 +244,7 @@ extern "C" int mf_column_sums(const void* x, int32_t dtype, int64_t rows, int32_
     launch_dependent(column_sums_band_kernel<float, false>, grid, dim3(kWarps * 32), 0, s, static_cast<const float*>(x), nullptr, nullptr,
                      rows, cols, rows_per_band, part);
   MF_CHECK_LAUNCH("column_sums_band_kernel");
-  launch_dependent(column_sums_final_kernel, dim3((cols + 31) / 32), dim3(256), 0, s, part, bands, cols, out);
-  MF_CHECK_LAUNCH("column_sums_final_kernel");
-  return MF_OK;
+  return add_bands(part, bands, cols, out, s);
 }
 
 extern "C" int mf_gelu_tanh_fwd(const void* x, int32_t dtype, int64_t n, void* y, void* stream) {
@@ -290,7 +294,5 @@ extern "C" int mf_gelu_tanh_bwd(const void* x, const void* dy, int32_t dtype, in
     launch_dependent(column_sums_band_kernel<float, true>, grid, dim3(kWarps * 32), 0, s, static_cast<const float*>(x),
                      static_cast<const float*>(dy), static_cast<float*>(dx), rows, cols, rows_per_band, part);
   MF_CHECK_LAUNCH("column_sums_band_kernel");
-  launch_dependent(column_sums_final_kernel, dim3((cols + 31) / 32), dim3(256), 0, s, part, bands, cols, column_sums);
-  MF_CHECK_LAUNCH("column_sums_final_kernel");
-  return MF_OK;
+  return add_bands(part, bands, cols, column_sums, s);
 }

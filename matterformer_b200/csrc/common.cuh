@@ -160,4 +160,6 @@ __device__ __forceinline__ float warp_sum(float v) {
 namespace mf {
 // Kernel timing aid (see mf_profile_enable): record an event on `stream` before/after a main kernel.
 void profile_mark(int which, bool begin, cudaStream_t stream);
+// out[c] = sum over the bands of part[band][c], in band order (column_sums.cu).
+int add_bands(const float* part, int bands, int cols, float* out, cudaStream_t stream);
 }  // namespace mf

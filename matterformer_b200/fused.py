@@ -463,3 +463,152 @@ def masked_sum(pad_mask: torch.Tensor, x: torch.Tensor, *, a=1.0, y: Optional[to
     if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, y, z)):
         return _MaskedSum.apply(pad_mask, x, a, y, z, c, center)
     return masked_update(pad_mask, x, a, y, z, c, center=center)
+
+
+def edm_scalings(sigma: torch.Tensor, sigma_data: float):
+    """``c_skip, c_out, c_in`` of the EDM preconditioner (tasks/edm.py:34-81) for CUDA fp32 noise levels (B,); no autograd."""
+    out = torch.empty((3, sigma.shape[0]), device=sigma.device, dtype=torch.float32)
+    _lib.launch(_lib.lib().mf_edm_scalings, sigma.device, sigma.data_ptr(), sigma.shape[0], float(sigma_data), out.data_ptr(), None)
+    return out.unbind(0)
+
+
+def noise_channel(sigma: torch.Tensor) -> torch.Tensor:
+    """``log(max(sigma, 1e-8)) / 4`` for CUDA fp32 noise levels (B,); no autograd."""
+    out = torch.empty_like(sigma)
+    _lib.launch(_lib.lib().mf_edm_scalings, sigma.device, sigma.data_ptr(), sigma.shape[0], 1.0, None, out.data_ptr())
+    return out
+
+
+def per_molecule_applies(t: torch.Tensor) -> bool:
+    """What the one-launch forms of the conditioning take: a contiguous CUDA fp32 vector without gradient."""
+    return t.is_cuda and t.ndim == 1 and t.dtype == torch.float32 and t.is_contiguous() and not t.requires_grad
+
+
+def time_embedding(t: torch.Tensor, half: int, dtype: torch.dtype) -> torch.Tensor:
+    """``[cos, sin, cos, sin](2 pi t f)``: what ``TimeEmbedder`` feeds its MLP when both its levels are ``t`` (B,); no autograd."""
+    out = torch.empty((t.shape[0], 4 * half), device=t.device, dtype=dtype)
+    _lib.launch(_lib.lib().mf_time_embedding, t.device, t.data_ptr(), t.shape[0], half, _CODE[dtype], out.data_ptr())
+    return out
+
+
+def valid_and_counts(pad_mask: torch.Tensor):
+    """``~pad_mask`` and its row sums in int32, for a CUDA bool (B, N) mask."""
+    pad = pad_mask.contiguous()
+    B, N = pad.shape
+    valid, counts = torch.empty_like(pad), torch.empty(B, device=pad.device, dtype=torch.int32)
+    _lib.launch(_lib.lib().mf_pad_counts, pad.device, pad.data_ptr(), B, N, valid.data_ptr(), counts.data_ptr())
+    return valid, counts
+
+
+def token_projection_applies(x: torch.Tensor, noise: torch.Tensor, pad_mask: torch.Tensor, weight: torch.Tensor,
+                             bias: Optional[torch.Tensor]) -> bool:  # fmt: skip
+    return (x.is_cuda and x.ndim == 3 and x.dtype == torch.float32 and not x.requires_grad and x.shape[2] < 8 and per_molecule_applies(noise)
+            and noise.shape[0] == x.shape[0] and pad_mask.dtype == torch.bool and pad_mask.shape == x.shape[:2] and bias is not None
+            and weight.dtype == bias.dtype == torch.float32 and weight.shape[1] == x.shape[2] + 1 and weight.shape[0] % 64 == 0
+            and 64 <= weight.shape[0] <= 1024 and all(t.device == x.device for t in (noise, pad_mask, weight, bias)))  # fmt: skip
+
+
+class _TokenProjection(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, noise, pad_mask, weight, bias):
+        x, pad = x.contiguous(), _bytes(pad_mask)
+        w, b = weight.detach().contiguous(), bias.detach().contiguous()
+        B, N, C = *x.shape[:2], w.shape[0]
+        out = torch.empty((B, N, C), device=x.device, dtype=torch.bfloat16)
+        _lib.launch(_lib.lib().mf_token_projection_fwd, x.device, x.data_ptr(), noise.data_ptr(), pad.data_ptr(), w.data_ptr(), b.data_ptr(),
+                    B, N, w.shape[1], C, out.data_ptr())  # fmt: skip
+        ctx.save_for_backward(x, noise, pad)
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, noise, pad = ctx.saved_tensors
+        dy = dy.to(torch.bfloat16).contiguous()
+        (B, N, C), K = dy.shape, x.shape[2] + 1
+        L = _lib.lib()
+        need = L.mf_token_projection_bwd_workspace_bytes(B, N, K, C)
+        ws = torch.empty(max(need, 16), device=dy.device, dtype=torch.uint8)
+        grads = torch.empty(C * (K + 1), device=dy.device, dtype=torch.float32)
+        _lib.launch(L.mf_token_projection_bwd, dy.device, dy.data_ptr(), x.data_ptr(), noise.data_ptr(), pad.data_ptr(), B, N, K, C,
+                    grads.data_ptr(), ws.data_ptr(), need)  # fmt: skip
+        return None, None, None, grads[: C * K].view(C, K), grads[C * K :]
+
+
+def token_projection(x: torch.Tensor, noise: torch.Tensor, pad_mask: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+    """The model's first Linear in bf16 on ``cat[x, noise]`` per token, padded rows cleared, without the concatenation; see
+    :func:`token_projection_applies`.  Gradients flow to ``weight`` and ``bias``."""
+    return _TokenProjection.apply(x, noise, pad_mask, weight, bias)
+
+
+class _GatedLayerNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, gate, a, pad, eps):
+        x, a, gate = x.contiguous(), a.contiguous(), gate.contiguous()
+        pad = _bytes(pad) if pad is not None else None
+        B, N, C = x.shape
+        y, h = torch.empty_like(x), torch.empty((B, N, C), device=x.device, dtype=torch.float32)
+        mean = torch.empty((B, N), device=x.device, dtype=torch.float32)
+        rstd = torch.empty_like(mean)
+        _lib.launch(_lib.lib().mf_gated_layer_norm_fwd, x.device, x.data_ptr(), _CODE[x.dtype], gate.data_ptr(), a.data_ptr(), _CODE[a.dtype],
+                    pad.data_ptr() if pad is not None else None, B, N, C, float(eps), y.data_ptr(), h.data_ptr(), mean.data_ptr(),
+                    rstd.data_ptr())  # fmt: skip
+        ctx.save_for_backward(gate, a, pad, y, mean, rstd)
+        return h
+
+    @staticmethod
+    def backward(ctx, dh):
+        gate, a, pad, y, mean, rstd = ctx.saved_tensors
+        B, N, C = y.shape
+        dh = dh.float().contiguous()
+        total, da = torch.empty_like(y), torch.empty_like(a)
+        dx = torch.empty_like(y) if pad is not None else None
+        sums = torch.empty((3, B, C), device=y.device, dtype=torch.float32)
+        zeros = torch.zeros((B, C), device=y.device, dtype=torch.float32)
+        _lib.launch(_lib.lib().mf_ln_modulate_bwd, y.device, dh.data_ptr(), _CODE[dh.dtype], y.data_ptr(), _CODE[y.dtype], zeros.data_ptr(),
+                    mean.data_ptr(), rstd.data_ptr(), B, N, C, total.data_ptr(), sums[1].data_ptr(), sums[2].data_ptr())  # fmt: skip
+        _lib.launch(_lib.lib().mf_gated_residual_bwd, y.device, total.data_ptr(), _CODE[total.dtype], gate.data_ptr(), a.data_ptr(),
+                    _CODE[a.dtype], pad.data_ptr() if pad is not None else None, B, N, C, da.data_ptr(),
+                    dx.data_ptr() if dx is not None else None, sums.data_ptr())  # fmt: skip
+        return total if dx is None else dx, sums[0], da, None, None
+
+
+def gated_layer_norm(x: torch.Tensor, gate: torch.Tensor, a: torch.Tensor, pad_mask: Optional[torch.Tensor], eps: float) -> torch.Tensor:
+    """``LayerNorm(gated_residual(x, gate, a, pad_mask))`` without affine parameters, in fp32; ``gate`` is fp32.  Padded rows come out as
+    zeros."""
+    if gate.dtype != torch.float32 or a.dtype not in _CODE:
+        gate, a = gate.float(), a if a.dtype in _CODE else a.float()
+    _check_shapes(x, (a,), (gate,), pad_mask)
+    return _GatedLayerNorm.apply(x, gate, a, pad_mask, eps)
+
+
+class _LayerNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps, out_dtype):
+        x, w, b = x.contiguous(), weight.detach().float().contiguous(), bias.detach().float().contiguous()
+        B, N, C = x.shape
+        h = torch.empty((B, N, C), device=x.device, dtype=out_dtype)
+        mean = torch.empty((B, N), device=x.device, dtype=torch.float32)
+        rstd = torch.empty_like(mean)
+        _lib.launch(_lib.lib().mf_layer_norm_fwd, x.device, x.data_ptr(), _CODE[x.dtype], w.data_ptr(), b.data_ptr(), B * N, C, float(eps),
+                    _CODE[out_dtype], h.data_ptr(), mean.data_ptr(), rstd.data_ptr())  # fmt: skip
+        ctx.dtypes = (weight.dtype, bias.dtype)
+        ctx.save_for_backward(x, w, mean, rstd)
+        return h
+
+    @staticmethod
+    def backward(ctx, dh):
+        x, w, mean, rstd = ctx.saved_tensors
+        B, N, C = x.shape
+        dh = (dh if dh.dtype in _CODE else dh.float()).contiguous()
+        dx = torch.empty_like(x)
+        sums = torch.empty((2, B, C), device=x.device, dtype=torch.float32)
+        scale = (w - 1.0).expand(B, C).contiguous()
+        _lib.launch(_lib.lib().mf_ln_modulate_bwd, x.device, dh.data_ptr(), _CODE[dh.dtype], x.data_ptr(), _CODE[x.dtype], scale.data_ptr(),
+                    mean.data_ptr(), rstd.data_ptr(), B, N, C, dx.data_ptr(), sums[0].data_ptr(), sums[1].data_ptr())  # fmt: skip
+        db, dw = sums.sum(1)
+        return dx, dw.to(ctx.dtypes[0]), db.to(ctx.dtypes[1]), None, None
+
+
+def affine_layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float, out_dtype: torch.dtype) -> torch.Tensor:
+    """``F.layer_norm`` over the channels of a (B, N, C) residual stream (see :func:`fused_applies`) in ``out_dtype``."""
+    return _LayerNorm.apply(x, weight, bias, eps, out_dtype)

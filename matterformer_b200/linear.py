@@ -21,7 +21,8 @@ from typing import Iterable, Optional, Sequence
 import torch
 import torch.nn.functional as F
 
-from .fused import column_sums, column_sums_applies, gelu_tanh_applies, gelu_tanh_backward, gelu_tanh_forward
+from . import _lib
+from .fused import _ptr_array, column_sums, column_sums_applies, gelu_tanh_applies, gelu_tanh_backward, gelu_tanh_forward
 
 _COPY = "_mf_bf16_copy"  # attribute on a parameter given to refresh_bf16_copies: (bf16 tensor, version it was made from)
 
@@ -160,6 +161,12 @@ def refresh_bf16_copies(params: Iterable[torch.Tensor], *, force: bool = False) 
             torch._foreach_copy_(stale_dst, stale_src)
 
 
+def _modulation_kernels_apply(mod: torch.Tensor, groups: int) -> bool:
+    """A contiguous CUDA bf16 (B, groups * C) matrix of vectors that the split and merge kernels take."""
+    C = mod.shape[1] // groups
+    return mod.is_cuda and mod.dtype == torch.bfloat16 and mod.is_contiguous() and groups <= 128 and C % 8 == 0 and 8 <= C <= 4096
+
+
 class _StackedModulation(torch.autograd.Function):
     """The adaptive-LayerNorm modulations of all layers from the one conditioning vector they share: one GEMM forward, three
     products backward, instead of those per layer.  ``params``: the layers' weights, then their biases."""
@@ -170,7 +177,10 @@ class _StackedModulation(torch.autograd.Function):
             mod = F.linear(x, weights, biases)
         B, C = x.shape[0], mod.shape[1] // (6 * layers)
         out = torch.empty((6 * layers, B, C), device=x.device, dtype=torch.float32)
-        out.copy_(mod.view(B, 6 * layers, C).transpose(0, 1))
+        if _modulation_kernels_apply(mod, 6 * layers):
+            _lib.launch(_lib.lib().mf_split_modulation, x.device, mod.data_ptr(), B, 6 * layers, C, out.data_ptr())
+        else:
+            out.copy_(mod.view(B, 6 * layers, C).transpose(0, 1))
         ctx.save_for_backward(x, weights)
         ctx.layers = layers
         return tuple(out.unbind(0))
@@ -179,8 +189,13 @@ class _StackedModulation(torch.autograd.Function):
     def backward(ctx, *grads):
         x, weights = ctx.saved_tensors
         like = next(g for g in grads if g is not None)
-        g = torch.stack([t if t is not None else torch.zeros_like(like) for t in grads], dim=1)  # (B, 6 L, C) fp32
-        g = g.reshape(g.shape[0], -1).to(torch.bfloat16)
+        B, C = like.shape
+        g = torch.empty((B, len(grads) * C), device=x.device, dtype=torch.bfloat16)
+        if _modulation_kernels_apply(g, len(grads)) and all(t is None or (t.dtype == torch.float32 and t.data_ptr() % 16 == 0) for t in grads):
+            parts = [t.contiguous() if t is not None else None for t in grads]
+            _lib.launch(_lib.lib().mf_merge_modulation, x.device, _ptr_array(parts), B, len(parts), C, g.data_ptr())
+        else:
+            g.copy_(torch.stack([t if t is not None else torch.zeros_like(like) for t in grads], dim=1).reshape(B, -1))  # (B, 6 L, C)
         with torch.autocast("cuda", enabled=False):
             dx = torch.mm(g, weights) if ctx.needs_input_grad[0] else None
             dw = _mm_f32(g.t(), x)
@@ -279,3 +294,40 @@ def linear_gelu_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch
     if x.dtype != torch.bfloat16:
         x = x.to(torch.bfloat16)
     return _LinearGeluBf16.apply(x.contiguous(), weight, bias)
+
+
+class _PairLinear(torch.autograd.Function):
+    """The two d-wide column blocks of a pair MLP's first Linear, applied once per atom."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias):
+        d = x.shape[-1]
+        w16, b16 = bf16_copy(weight), bf16_copy(bias)
+        x = x.to(torch.bfloat16)
+        ctx.save_for_backward(x, w16)
+        ctx.columns = weight.shape[1]
+        with torch.autocast("cuda", enabled=False):
+            return F.linear(x, w16[:, :d]), F.linear(x, w16[:, d : 2 * d], b16)
+
+    @staticmethod
+    def backward(ctx, da, db):
+        x, w16 = ctx.saved_tensors
+        d = x.shape[-1]
+        x2 = x.reshape(-1, d)
+        da, db = (g.reshape(-1, g.shape[-1]).to(torch.bfloat16).contiguous() for g in (da, db))
+        dx = dw = sums = None
+        with torch.autocast("cuda", enabled=False):
+            if ctx.needs_input_grad[0]:  # in fp32, as the sum of the two products' fp32 results
+                dx = _mm_f32(da, w16[:, :d]).add_(_mm_f32(db, w16[:, d : 2 * d])).view(x.shape)
+            if ctx.needs_input_grad[1]:
+                dw = torch.zeros((da.shape[1], ctx.columns), device=x.device, dtype=torch.float32)
+                dw[:, :d] = _mm_f32(da.t(), x2)
+                dw[:, d : 2 * d] = _mm_f32(db.t(), x2)
+            if ctx.needs_input_grad[2]:
+                sums = column_sums(db) if column_sums_applies(db) else db.sum(0, dtype=torch.float32)
+        return dx, dw, sums
+
+
+def pair_linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor):
+    """``F.linear(x, weight[:, :d])`` and ``F.linear(x, weight[:, d:2d], bias)`` in bf16 on fp32 parameters, x (B, N, d) fp32 or bf16."""
+    return _PairLinear.apply(x, weight, bias)

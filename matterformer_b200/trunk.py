@@ -28,9 +28,9 @@ import torch.nn.functional as F
 from torch import nn
 
 from . import fused
-from .fused import (fused_applies, gated_ln_modulate, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
+from .fused import (fused_applies, gated_layer_norm, gated_ln_modulate, gated_residual, heads_layout_applies, ln_modulate, merge_heads, split_heads,
                     split_modulation)
-from .linear import bf16_copies, linear_bf16, linear_bf16_applies, linear_gelu_bf16, stacked_modulation
+from .linear import bf16_copies, linear_bf16, linear_bf16_applies, linear_gelu_bf16, pair_linear_bf16, stacked_modulation
 from .simplicial import (normalize_simplicial_precision, packed_projection_applies, simplicial_attention_cuda,
                          simplicial_attention_packed)  # fmt: skip
 
@@ -291,20 +291,27 @@ class Mlp(nn.Module):
         return linear_bf16(linear_gelu_bf16(x, self.fc1.weight, self.fc1.bias), self.fc2.weight, self.fc2.bias)
 
 
-def layer_norm(x: torch.Tensor, norm: nn.LayerNorm) -> torch.Tensor:
-    """``norm(x)`` for a (B, N, C) CUDA tensor through the fused LayerNorm-modulate kernels (ATen's backward for an
-    affine LayerNorm of this width is ten times slower than its forward): the affine weight and bias become the
-    modulation ``scale = weight - 1``, ``shift = bias`` of every molecule, and their gradients come back through the
-    broadcast.  Other tensors take ``norm`` itself."""
+def layer_norm(x: torch.Tensor, norm: nn.LayerNorm, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    """``norm(x)`` for a (B, N, C) CUDA tensor through the fused LayerNorm kernels (ATen's backward for an affine LayerNorm of
+    this width is ten times slower than its forward), in ``out_dtype``.  Other tensors take ``norm`` itself, in whatever type it
+    returns."""
     if not (fused_applies(x) and x.dtype == torch.float32 and norm.normalized_shape == (x.shape[-1],)):
         return norm(x)
+    if norm.elementwise_affine and norm.bias is not None:
+        return fused.affine_layer_norm(x, norm.weight, norm.bias, norm.eps, out_dtype)
     B, C = x.shape[0], x.shape[-1]
-    if norm.elementwise_affine:
-        scale = (norm.weight.float() - 1.0).expand(B, C)
-        shift = (norm.bias.float() if norm.bias is not None else torch.zeros_like(norm.weight, dtype=torch.float32)).expand(B, C)
-    else:
-        scale = shift = torch.zeros((B, C), device=x.device, dtype=torch.float32)
-    return ln_modulate(x, shift, scale, eps=norm.eps, out_dtype=torch.float32)
+    shift = torch.zeros((B, C), device=x.device, dtype=torch.float32)
+    scale = (norm.weight.float() - 1.0).expand(B, C) if norm.elementwise_affine else shift
+    return ln_modulate(x, shift, scale, eps=norm.eps, out_dtype=out_dtype)
+
+
+def _bf16_autocast(x: torch.Tensor) -> bool:
+    return x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
+
+
+def _unhooked(*modules: nn.Module) -> bool:
+    """Modules whose call may be replaced by what they compute."""
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in modules)
 
 
 def _modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
@@ -342,7 +349,8 @@ class AdaLNBlock(nn.Module):
         ``modulation``: the six modulation tensors, formed by the trunk for all its blocks at once; ``num_atoms``: counts of
         real tokens for the attention layer, ``padding_is_suffix``: whether they come first in every row.  ``following``:
         (shift, scale, eps) of the norm that opens the next block; the block then returns its output and that norm's, formed in
-        one pass, and the next block takes the latter as ``h``."""
+        one pass, and the next block takes the latter as ``h``.  (None, None, eps): the norm is the stack's output norm, which has no
+        modulation and is kept in fp32; only its output is returned."""
         fused = self.fused_elementwise and fused_applies(x)
         mod = None if modulation is not None else linear_bf16(cond_act if cond_act is not None else self.ada_ln[0](cond_emb), self.ada_ln[-1].weight,
                           self.ada_ln[-1].bias)  # fmt: skip
@@ -368,6 +376,8 @@ class AdaLNBlock(nn.Module):
             pad = pad_mask if zero_padding else None
             if following is not None:
                 shift, scale, eps = following
+                if shift is None:
+                    return gated_layer_norm(x, gate_m, self.mlp(h), pad, eps)
                 return gated_ln_modulate(x, gate_m, self.mlp(h), pad, shift, scale, eps=eps, out_dtype=h_dtype)
             return gated_residual(x, gate_m, self.mlp(h), pad)
         x = x + gate_a[:, None, :] * attn_out
@@ -405,35 +415,41 @@ class TransformerTrunk(nn.Module):
         return out
 
     def forward(self, x: torch.Tensor, cond_emb: torch.Tensor, *, pad_mask: Optional[torch.Tensor] = None,
-                sparse_plan: Optional[SparseAttentionPlan] = None) -> torch.Tensor:  # fmt: skip
+                sparse_plan: Optional[SparseAttentionPlan] = None, padding_cleared: bool = False) -> torch.Tensor:  # fmt: skip
         """``sparse_plan`` (see :func:`plan_sparse_attention`) makes every MHA layer attend over the plan's
-        neighbourhoods instead of all tokens: the periodic-crystal mode of the trunk."""
+        neighbourhoods instead of all tokens: the periodic-crystal mode of the trunk.  ``padding_cleared``: the rows of ``x`` that
+        ``pad_mask`` marks are zeros already."""
         bf16 = x.is_cuda and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") == torch.bfloat16
         layers = [block.ada_ln[-1] for block in self.blocks]
         stacked = bf16 and fused_applies(x) and cond_emb.ndim == 2 and all(
             block.fused_elementwise and m.weight.dtype == torch.float32 and m.bias is not None for block, m in zip(self.blocks, layers)
         )
         if not (bf16 or (x.is_cuda and x.dtype == torch.bfloat16)):
-            return self._forward(x, cond_emb, pad_mask, sparse_plan, None)
+            return self._forward(x, cond_emb, pad_mask, sparse_plan, None, padding_cleared)
         # the bf16 copies the blocks' Linear layers compute with: all of them in one multi-tensor copy
         stacks = ([m.weight for m in layers], [m.bias for m in layers]) if stacked else ()
         with bf16_copies(self._linear_parameters(), stacks) as made:
-            return self._forward(x, cond_emb, pad_mask, sparse_plan, made if stacked else None)
+            return self._forward(x, cond_emb, pad_mask, sparse_plan, made if stacked else None, padding_cleared)
 
-    def _forward(self, x, cond_emb, pad_mask, sparse_plan, modulation_copies):
+    def _forward(self, x, cond_emb, pad_mask, sparse_plan, modulation_copies, padding_cleared):
         """``modulation_copies``: stacked bf16 weights and biases of the modulation layers, where one GEMM serves them all."""
         b, n, _ = x.shape
         if pad_mask is not None:
             pad_mask = pad_mask.bool()
         stacked = modulation_copies is not None
-        sim_mask = SimplicialAttentionMask.from_key_padding_mask(pad_mask, batch_size=b, num_tokens=n, device=x.device)
+        num_atoms = None
+        if x.is_cuda and pad_mask is not None and pad_mask.device == x.device and pad_mask.shape == (b, n):
+            valid, num_atoms = fused.valid_and_counts(pad_mask)
+            sim_mask = SimplicialAttentionMask(valid, valid)
+        else:
+            sim_mask = SimplicialAttentionMask.from_key_padding_mask(pad_mask, batch_size=b, num_tokens=n, device=x.device)
         if self.emit_pair_valid and not x.is_cuda:  # (the kernels take the padding from the key mask: the same pairs)
             v = sim_mask.pair_key_valid
             sim_mask = SimplicialAttentionMask(sim_mask.query_valid, v, v[:, :, None] & v[:, None, :])
         # the reference clears the padded rows before every block (transformer.py, the loop of TransformerTrunk.forward);
         # here every block hands its output over already cleared (one pass with its last gated residual), which is
         # the same for every block but the last, whose padded rows are cleared once more after the output norm anyway
-        if pad_mask is not None:
+        if pad_mask is not None and not padding_cleared:
             x = x.masked_fill(pad_mask[..., None], 0.0)
         # every block starts its modulation with the same SiLU(cond_emb): formed (and cast for the bf16 Linear) once
         cond_act = F.silu(cond_emb)
@@ -444,18 +460,23 @@ class TransformerTrunk(nn.Module):
             layers = [block.ada_ln[-1] for block in self.blocks]
             modulation = stacked_modulation(cond_act, *modulation_copies, [m.weight for m in layers] + [m.bias for m in layers],
                                             len(layers))  # fmt: skip
-        num_atoms = (~pad_mask).sum(dim=1).to(torch.int32) if x.is_cuda and pad_mask is not None else None
         mha = [block.attn for block in self.blocks if isinstance(block.attn, RegularAttention)]
         reads = sparse_plan is None and any(attn._core_fits(x, pad_mask) for attn in mha)
         suffix = _padding_is_suffix(self, pad_mask) if reads else None  # one read-back for all layers
-        h = None
+        h, norm = None, self.norm_out
+        last = len(self.blocks) - 1
+        # the output norm in one pass with the last block's output (its padded rows are zeros, which the norm leaves as they are)
+        closing = stacked and last >= 0 and type(norm) is nn.LayerNorm and not norm.elementwise_affine and norm.normalized_shape == (x.shape[-1],) and \
+            _unhooked(norm, *self.blocks[last:])  # fmt: skip
         for i, (block, six) in enumerate(zip(self.blocks, modulation)):
-            chain = stacked and i + 1 < len(self.blocks)  # the next block's first norm in one pass with this one's output
-            following = (*modulation[i + 1][:2], self.blocks[i + 1].norm1.eps) if chain else None
+            chain = stacked and i < last  # the next block's first norm in one pass with this one's output
+            following = (*modulation[i + 1][:2], self.blocks[i + 1].norm1.eps) if chain else (None, None, norm.eps) if closing else None
             x = block(x, cond_emb, pad_mask=pad_mask, simplicial_attention_mask=sim_mask, sparse_plan=sparse_plan,
                       zero_padding=pad_mask is not None, cond_act=cond_act, modulation=six, num_atoms=num_atoms, h=h,
                       following=following, padding_is_suffix=suffix)  # fmt: skip
             x, h = x if chain else (x, None)
+        if closing:
+            return x
         x = layer_norm(x, self.norm_out)
         if pad_mask is not None:
             x = x.masked_fill(pad_mask[..., None], 0.0)
@@ -481,6 +502,9 @@ class TimeEmbedder(nn.Module):
         return torch.cat([torch.cos(args), torch.sin(args)], dim=-1)
 
     def forward(self, t_global: torch.Tensor, t_atomic: torch.Tensor) -> torch.Tensor:
+        if t_global is t_atomic and fused.per_molecule_applies(t_global):  # one launch instead of some twenty
+            return _two_layers(self.mlp, fused.time_embedding(t_global, self.freq_dim // 2,
+                                                              torch.bfloat16 if _bf16_autocast(t_global) else torch.float32))  # fmt: skip
         return _two_layers(self.mlp, torch.cat([self._embed(t_global), self._embed(t_atomic)], dim=-1))
 
 
@@ -532,8 +556,11 @@ class EDMModel(nn.Module):
         kernel_fits = trunk_out.is_cuda and trunk_out.dtype in (torch.float32, torch.bfloat16)
         if kernel_fits and tuple(w0[:, 2 * d :].shape) == (fused.PAIR_HIDDEN, fused.PAIR_RBF) and not coords.requires_grad:
             # per-atom halves of the first Linear (two GEMMs), everything per pair in one kernel
-            a = F.linear(trunk_out, w0[:, :d])
-            b = F.linear(trunk_out, w0[:, d : 2 * d], b0)
+            if _bf16_autocast(trunk_out) and w0.dtype == torch.float32 and w0.shape[1] % 8 == 0 and d % 8 == 0:
+                a, b = pair_linear_bf16(trunk_out, w0, b0)
+            else:
+                a = F.linear(trunk_out, w0[:, :d])
+                b = F.linear(trunk_out, w0[:, d : 2 * d], b0)
             return fused.equivariant_pair_head(a, b, coords, ~pad_mask, w0[:, 2 * d :], self.pair_head[2].weight,
                                                self.pair_head[2].bias, self._pair_rbf_centers, self._pair_rbf_gamma_value)  # fmt: skip
         return self._coord_delta_torch(trunk_out, coords, pad_mask)
@@ -566,19 +593,26 @@ class EDMModel(nn.Module):
     def forward(self, atom_noisy, coords_noisy, pad_mask, sigma, lattice=None):
         if sigma.ndim == 2:
             sigma = sigma[:, 0]
-        sigma_cond = torch.log(sigma.clamp_min(1e-8)) / 4.0
+        sigma_cond = fused.noise_channel(sigma) if fused.per_molecule_applies(sigma) else torch.log(sigma.clamp_min(1e-8)) / 4.0
         if not linear_bf16_applies(atom_noisy, self.atom_proj.weight):
             return self._forward(atom_noisy, coords_noisy, pad_mask, sigma_cond)
         layers = [self.atom_proj, self.conditioning.mlp[0], self.conditioning.mlp[2], self.atom_head[1], self.atom_head[3]]
+        layers.append(self.pair_head[0])
         with bf16_copies(p for m in layers for p in (m.weight, m.bias)):  # (the trunk makes its own)
             return self._forward(atom_noisy, coords_noisy, pad_mask, sigma_cond)
 
     def _forward(self, atom_noisy, coords_noisy, pad_mask, sigma_cond):
-        feat = sigma_cond[:, None, None].expand(-1, atom_noisy.shape[1], 1).masked_fill(pad_mask[..., None], 0.0)
-        tokens = linear_bf16(torch.cat([atom_noisy, feat], dim=-1), self.atom_proj.weight, self.atom_proj.bias)
+        proj, low = self.atom_proj, _bf16_autocast(atom_noisy)
+        whole = low and fused.token_projection_applies(atom_noisy, sigma_cond, pad_mask, proj.weight, proj.bias)
+        if whole:
+            tokens = fused.token_projection(atom_noisy, sigma_cond, pad_mask, proj.weight, proj.bias)
+        else:
+            feat = sigma_cond[:, None, None].expand(-1, atom_noisy.shape[1], 1).masked_fill(pad_mask[..., None], 0.0)
+            tokens = linear_bf16(torch.cat([atom_noisy, feat], dim=-1), proj.weight, proj.bias)
         cond = self.conditioning(sigma_cond, sigma_cond)
-        trunk_out = self.trunk(tokens, cond, pad_mask=pad_mask)
-        atom_delta = _two_layers(self.atom_head[1:], layer_norm(trunk_out, self.atom_head[0])).masked_fill(pad_mask[..., None], 0.0)
+        trunk_out = self.trunk(tokens, cond, pad_mask=pad_mask, **({"padding_cleared": True} if whole and type(self.trunk) is TransformerTrunk else {}))
+        normed = layer_norm(trunk_out, self.atom_head[0], torch.bfloat16 if low else torch.float32)
+        atom_delta = _two_layers(self.atom_head[1:], normed).masked_fill(pad_mask[..., None], 0.0)
         return atom_delta, self._coord_delta(trunk_out, coords_noisy, pad_mask)
 
 
@@ -595,9 +629,12 @@ class EDMPreconditioner(nn.Module):
             sigma = sigma[:, 0]
         sigma = sigma.float()
         sd2 = self.sigma_data**2
-        c_skip = sd2 / (sigma.square() + sd2)
-        c_out = sigma * self.sigma_data / torch.sqrt(sigma.square() + sd2)
-        c_in = 1.0 / torch.sqrt(sd2 + sigma.square())
+        if fused.per_molecule_applies(sigma):
+            c_skip, c_out, c_in = fused.edm_scalings(sigma, self.sigma_data)
+        else:
+            c_skip = sd2 / (sigma.square() + sd2)
+            c_out = sigma * self.sigma_data / torch.sqrt(sigma.square() + sd2)
+            c_in = 1.0 / torch.sqrt(sd2 + sigma.square())
         atom_in = atom_noisy * c_in[:, None, None]
         fits = not sigma.requires_grad and fused.masked_sum_applies(coords_noisy, pad_mask) and \
             fused.masked_sum_applies(atom_noisy, pad_mask)  # fmt: skip
