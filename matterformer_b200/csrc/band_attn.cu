@@ -13,11 +13,16 @@
 // a warp sees two chunks, and nothing but the structure's end is masked.  1 024 molecules of 9 - 29 tokens x 8
 // heads: forward 37 -> 25 us, backward 104 -> 53 us (two launches of the 32-row walk before).
 //
-// What bounds it: the L1 / shared-memory path, 62 % (forward) and 69 % (backward) of its throughput (operand fragments, at 16
-// rows per warp), while a CTA's loads overlap only with the other CTAs of the SM.  32 cells of 4096 tokens x 8 heads, window 64: forward 144 us, backward 382 us (HBM
-// floors 82 and 164 us), against 219 and 311 + 322 us for the 32-row walk with its three passes.
+// What bounds it: issue slots and the L1 / shared-memory path (operand fragments, at 16 rows per warp), while a CTA's loads overlap only
+// with the other CTAs of the SM.  The 128-row tiles arrive by bulk tensor copies: as 16-byte copies of the threads they took a
+// quarter of the forward kernel's instructions and a share of the L1 path; 64-row tiles, which serve calls of a few microseconds,
+// keep those (a map is encoded on the host for each call).  Interior chunks take no masks and two elements an instruction.  32 cells of
+// 4096 tokens x 8 heads, window 64: forward 144 -> 117 us, backward 381 -> 335 us (HBM floors 82 and 164 us); window 32 125 -> 102 and
+// 342 -> 255, window 128 207 -> 167 and 779 -> 698.  The 32-row walk with its three passes: 219 and 311 + 322 us at window 64.
 #include "common.cuh"
 #include "simplicial_warp.cuh"
+#include "sm100_primitives.cuh"
+#include "tensor_map.cuh"
 
 namespace mf {
 namespace {
@@ -37,6 +42,39 @@ struct BandParams {
   float scale;
   RowLayout in, act;  // rows of q, k, v and their gradients; rows of out and grad_out
 };
+
+__device__ int32_t g_band_status = 0;  // MF_ERR_DEVICE_TIMEOUT after an expired wait
+
+// The wide tiles bring their rows by bulk tensor copies, which zero what lies outside [0, N): forward k, v, q, backward q, k, v, dO.
+struct BandMaps {
+  CUtensorMap m[4];
+};
+struct NoMaps {};
+template <int kRows>
+using MapsOf = std::conditional_t<kRows == 128, BandMaps, NoMaps>;
+
+// Waits for the copies on `bar` and clears the rows of `tiles` tiles that lie in [n, N) (they may hold NaN).  False: the wait expired,
+// for every thread alike.
+template <int kThreads, int kTiles>
+__device__ __forceinline__ bool tiles_arrived(uint64_t* bar, uint8_t* smem, const int (&at)[kTiles], const int (&first)[kTiles],
+                                              const int (&rows)[kTiles], int n) {
+  bool ok = mbar_wait(bar, 0);
+  if (!ok) ok = mbar_wait(bar, 0);  // the copies write to this CTA: give them once more as long
+  if (__syncthreads_or(!ok)) {
+    if (threadIdx.x == 0) atomicExch(&g_band_status, MF_ERR_DEVICE_TIMEOUT);
+    return false;
+  }
+  bool edge = false;
+#pragma unroll
+  for (int t = 0; t < kTiles; ++t) {
+    if (first[t] + rows[t] <= n) continue;
+    edge = true;
+    for (int idx = threadIdx.x + 8 * max(n - first[t], 0); idx < 8 * rows[t]; idx += kThreads)
+      *reinterpret_cast<uint4*>(smem + at[t] + 16 * idx) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (edge) __syncthreads();  // (the same for all threads)
+  return true;
+}
 
 // rows [first, first + rows) of one head into a swizzled tile; rows outside [0, n) become zeros
 template <int kThreads>
@@ -109,8 +147,8 @@ __device__ __forceinline__ void store_rows(__nv_bfloat16* dst, long long stride,
 }
 
 template <int W, int kRows>
-__global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 128 ? 2 : 4) : (kRows == 128 ? 3 : 6)) band_fwd_kernel(const __grid_constant__ BandParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
+__global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 128 ? 2 : 4) : (kRows == 128 ? 3 : 6)) band_fwd_kernel(const __grid_constant__ BandParams p, const __grid_constant__ MapsOf<kRows> maps) {
+  extern __shared__ __align__(1024) uint8_t smem[];
   wait_for_previous();
   constexpr bool kDense = W == 0;
   constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = kDense ? kRows / 16 : W / 16 + 1;
@@ -121,12 +159,26 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
   const uint32_t tile = (uint32_t)__cvta_generic_to_shared(smem);
   const long long in0 = p.in.at(b, h, 0), act0 = p.act.at(b, h, 0);
   if (t0 < n) {
-    load_band<kThreads>(tile, p.k + in0, p.in.token, t0 - kHalf, kHalo, n);
-    load_band<kThreads>(tile + kTq, p.q + in0, p.in.token, t0, kRows, n);
-    load_band<kThreads>(tile + kTv, p.v + in0, p.in.token, t0 - kHalf, kHalo, n);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
+    if constexpr (kRows == 128) {
+      uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kTq + kRows * kRowBytes);
+      if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+        mbar_arrive_expect_tx(bar, (2 * kHalo + kRows) * kRowBytes);
+        tma_load_strided_rows(tile, &maps.m[0], t0 - kHalf, h, b, bar);
+        tma_load_strided_rows(tile + kTq, &maps.m[2], t0, h, b, bar);
+        tma_load_strided_rows(tile + kTv, &maps.m[1], t0 - kHalf, h, b, bar);
+      }
+      __syncthreads();
+      if (!tiles_arrived<kThreads, 3>(bar, smem, {0, kTv, kTq}, {t0 - kHalf, t0 - kHalf, t0}, {kHalo, kHalo, kRows}, n)) return;
+    } else {
+      load_band<kThreads>(tile, p.k + in0, p.in.token, t0 - kHalf, kHalo, n);
+      load_band<kThreads>(tile + kTq, p.q + in0, p.in.token, t0, kRows, n);
+      load_band<kThreads>(tile + kTv, p.v + in0, p.in.token, t0 - kHalf, kHalo, n);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+    }
   }
   const int i0 = t0 + warp * 16, row = i0 + row8;  // the lane's rows: row and row + 8
   if (i0 >= N) return;
@@ -143,21 +195,20 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) load_a(q[ks], fb, kTq + mine, 0, ks);
     const float sc2 = p.scale * kLog2e;
-    // hidden pairs of chunk c: the two triangles, and keys outside the structure
-    auto logits = [&](float(&s)[2][4], int c) {
-      chunk_product(s, q, fb, c * 16 * kRowBytes);
+    // sets the hidden pairs of chunk c: the two triangles, and keys outside the structure
+    auto hide = [&](float(&s)[2][4], int c, float value) {
       const int key0 = kDense ? 16 * c : i0 - kHalf + 16 * c;
       const bool ends = key0 < 0 || key0 + 16 > n;
+      if (!ends && (kDense || (c != 0 && c != kChunks - 1))) return;
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
-          bool seen = true;
-          if (!kDense && c == 0) seen = rel >= r;
-          if (!kDense && c == kChunks - 1) seen = rel < r;
-          if (ends) seen = seen && key0 + rel >= 0 && key0 + rel < n;
-          s[nt][e] = seen ? s[nt][e] * sc2 : -INFINITY;
+          bool seen = key0 + rel >= 0 && key0 + rel < n;
+          if (!kDense && c == 0) seen = seen && rel >= r;
+          if (!kDense && c == kChunks - 1) seen = seen && rel < r;
+          if (!seen) s[nt][e] = value;
         }
     };
     for (bool exact = false;; exact = true) {
@@ -166,7 +217,12 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
 #pragma unroll 1
         for (int c = 0; c < kChunks; ++c) {
           float s[2][4];
-          logits(s, c);
+          chunk_product(s, q, fb, c * 16 * kRowBytes);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[nt][e] *= sc2;
+          hide(s, c, -INFINITY);
 #pragma unroll
           for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -184,20 +240,23 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
           for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
       }
       float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      const float2 factor = make_float2(sc2, sc2);
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
         float s[2][4];
-        logits(s, c);
+        chunk_product(s, q, fb, c * 16 * kRowBytes);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            float2 x = add2(make_float2(s[nt][2 * hh], s[nt][2 * hh + 1]), make_float2(-shift[hh], -shift[hh]));
-            x.x = fast_exp2(x.x);
-            x.y = fast_exp2(x.y);
-            l2[hh] = add2(l2[hh], x);
-            s[nt][2 * hh] = x.x, s[nt][2 * hh + 1] = x.y;
+            const float2 x = fma2(make_float2(s[nt][2 * hh], s[nt][2 * hh + 1]), factor, make_float2(-shift[hh], -shift[hh]));
+            s[nt][2 * hh] = fast_exp2(x.x), s[nt][2 * hh + 1] = fast_exp2(x.y);
           }
+        hide(s, c, 0.f);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) l2[hh] = add2(l2[hh], make_float2(s[nt][2 * hh], s[nt][2 * hh + 1]));
         uint32_t pk[4];
         pack_chunk(pk, s);
         chunk_accumulate(o, pk, fb, kTv + c * 16 * kRowBytes);
@@ -223,26 +282,37 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
 }
 
 template <int W, int kRows>
-__global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 128 ? 1 : 2) : (W == 128 ? 2 : 3)) band_bwd_kernel(const __grid_constant__ BandParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
+__global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 128 ? 1 : 2) : (W == 128 ? 2 : 3)) band_bwd_kernel(const __grid_constant__ BandParams p, const __grid_constant__ MapsOf<kRows> maps) {
+  extern __shared__ __align__(1024) uint8_t smem[];
   wait_for_previous();
   constexpr bool kDense = W == 0;
   constexpr int kHalf = W / 2, kHalo = kRows + W, kThreads = kRows * 2, kChunks = kDense ? kRows / 16 : W / 16 + 1;
   constexpr int kTk = kHalo * kRowBytes, kTv = 2 * kTk, kTg = 3 * kTk;  // q, k, v, grad_out
   float* lse = reinterpret_cast<float*>(smem + 4 * kTk);  // of the halo rows, in the log2 domain
   float* delta = lse + kHalo;
+  [[maybe_unused]] uint64_t* bar = reinterpret_cast<uint64_t*>(delta + kHalo);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2;
   const int t0 = blockIdx.x * kRows, first = t0 - kHalf, bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H, N = p.N;
   const int n = min(p.num_atoms[b], N);
   const uint32_t tile = (uint32_t)__cvta_generic_to_shared(smem);
   const long long in0 = p.in.at(b, h, 0), act0 = p.act.at(b, h, 0);
   if (t0 < n) {
-    load_band<kThreads>(tile + kTg, p.grad_out + act0, p.act.token, first, kHalo, n);
-    load_band<kThreads>(tile, p.q + in0, p.in.token, first, kHalo, n);
-    load_band<kThreads>(tile + kTk, p.k + in0, p.in.token, first, kHalo, n);
-    load_band<kThreads>(tile + kTv, p.v + in0, p.in.token, first, kHalo, n);
-    cp_async_commit();
-    // delta of the halo rows, eight lanes per row (their own loads of dO, while the copies are in flight), all loads first
+    if constexpr (kRows == 128) {
+      if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+        mbar_arrive_expect_tx(bar, 4 * kHalo * kRowBytes);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) tma_load_strided_rows(tile + t * kTk, &maps.m[t], first, h, b, bar);
+      }
+    } else {
+      load_band<kThreads>(tile + kTg, p.grad_out + act0, p.act.token, first, kHalo, n);
+      load_band<kThreads>(tile, p.q + in0, p.in.token, first, kHalo, n);
+      load_band<kThreads>(tile + kTk, p.k + in0, p.in.token, first, kHalo, n);
+      load_band<kThreads>(tile + kTv, p.v + in0, p.in.token, first, kHalo, n);
+      cp_async_commit();
+    }
+    // delta of the halo rows, eight lanes per row, all loads first (of dO their own ones, or the tile once it is there)
     constexpr int kSteps = kHalo * 8 / kThreads;
     static_assert(kHalo * 8 % kThreads == 0, "whole steps");
     uint4 x[kSteps], g[kSteps];
@@ -255,9 +325,15 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
       ls[t] = INFINITY;  // no weight for rows outside the structure
       if (row >= 0 && row < n) {
         x[t] = *reinterpret_cast<const uint4*>(p.out + act0 + row * p.act.token + c * 8);
-        g[t] = *reinterpret_cast<const uint4*>(p.grad_out + act0 + row * p.act.token + c * 8);
+        if constexpr (kRows != 128) g[t] = *reinterpret_cast<const uint4*>(p.grad_out + act0 + row * p.act.token + c * 8);
         if (c == 0) ls[t] = p.lse[(size_t)bh * N + row] * kLog2e;
       }
+    }
+    if constexpr (kRows == 128) {
+      __syncthreads();  // the barrier exists
+      if (!tiles_arrived<kThreads, 4>(bar, smem, {0, kTk, kTv, kTg}, {first, first, first, first}, {kHalo, kHalo, kHalo, kHalo}, n)) return;
+#pragma unroll
+      for (int t = 0; t < kSteps; ++t) g[t] = *reinterpret_cast<const uint4*>(smem + row_chunk(kTg, r0 + t * (kThreads / 8), c));
     }
 #pragma unroll
     for (int t = 0; t < kSteps; ++t) {
@@ -273,7 +349,7 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
         lse[r0 + t * (kThreads / 8)] = ls[t];
       }
     }
-    cp_async_wait<0>();
+    if constexpr (kRows != 128) cp_async_wait<0>();
     __syncthreads();
   }
   const int i0 = t0 + warp * 16, row = i0 + row8;
@@ -282,7 +358,7 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
   const FragBase fb(tile + (kDense ? 0 : warp * 16 * kRowBytes), lane);
   const int mine = kDense ? warp * 16 * kRowBytes : 0;
   const int own = kHalf * kRowBytes + mine;  // the warp's rows inside the halo
-  const float sc2 = p.scale * kLog2e;
+  const float2 factor = make_float2(p.scale * kLog2e, p.scale * kLog2e);
   uint32_t a[4][4], g[4][4];
   float acc0[8][4], acc1[8][4];
 #pragma unroll
@@ -303,21 +379,24 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
+        for (int hh = 0; hh < 2; ++hh) {
+          const float lr = hh ? lb : la, dr = hh ? db : da;
+          const float2 x = fma2(make_float2(s[nt][2 * hh], s[nt][2 * hh + 1]), factor, make_float2(-lr, -lr));
           // a logit of 0 against zero rows may give a huge weight where the row's log-sum-exp is very negative: bounded, so
           // that it stays finite and 0 . weight = 0
-          float pr = fast_exp2(fminf(fmaf(s[nt][e], sc2, -(e < 2 ? la : lb)), 100.f));
-          if (!kDense && c == 0 && rel < r) pr = 0.f;
-          if (!kDense && c == kChunks - 1 && rel >= r) pr = 0.f;
-          s[nt][e] = pr * (dp[nt][e] - (e < 2 ? da : db)) * p.scale;
+          float2 pr = make_float2(fast_exp2(fminf(x.x, 100.f)), fast_exp2(fminf(x.y, 100.f)));
+          const int r = row8 + 8 * hh, rel = nt * 8 + 2 * quad;
+          if (!kDense && c == 0) pr.x = rel < r ? 0.f : pr.x, pr.y = rel + 1 < r ? 0.f : pr.y;
+          if (!kDense && c == kChunks - 1) pr.x = rel >= r ? 0.f : pr.x, pr.y = rel + 1 >= r ? 0.f : pr.y;
+          pr = mul2(pr, add2(make_float2(dp[nt][2 * hh], dp[nt][2 * hh + 1]), make_float2(-dr, -dr)));
+          s[nt][2 * hh] = pr.x, s[nt][2 * hh + 1] = pr.y;  // (the scale comes with the sums)
         }
       uint32_t pk[4];
       pack_chunk(pk, s);
       chunk_accumulate(acc0, pk, fb, kTk + at);
     }
   }
-  store_rows(p.dq + in0, p.in.token, acc0, row, N, row < n ? 1.f : 0.f, row + 8 < n ? 1.f : 0.f);
+  store_rows(p.dq + in0, p.in.token, acc0, row, N, row < n ? p.scale : 0.f, row + 8 < n ? p.scale : 0.f);
 #pragma unroll
   for (int t = 0; t < 8; ++t)
 #pragma unroll
@@ -336,13 +415,15 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
         const int q0 = ((kDense ? 0 : warp) + c) * 16 + nt * 8 + 2 * quad;
         const float2 l = *reinterpret_cast<const float2*>(&lse[q0]), d = *reinterpret_cast<const float2*>(&delta[q0]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int r = row8 + 8 * (e >> 1), rel = nt * 8 + 2 * quad + (e & 1);
-          float pr = fast_exp2(fmaf(s[nt][e], sc2, -((e & 1) ? l.y : l.x)));
-          if (!kDense && c == 0 && rel <= r) pr = 0.f;
-          if (!kDense && c == kChunks - 1 && rel > r) pr = 0.f;
-          s[nt][e] = pr;
-          dp[nt][e] = pr * (dp[nt][e] - ((e & 1) ? d.y : d.x)) * p.scale;
+        for (int hh = 0; hh < 2; ++hh) {
+          const float2 x = fma2(make_float2(s[nt][2 * hh], s[nt][2 * hh + 1]), factor, make_float2(-l.x, -l.y));
+          float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+          const int r = row8 + 8 * hh, rel = nt * 8 + 2 * quad;
+          if (!kDense && c == 0) pr.x = rel <= r ? 0.f : pr.x, pr.y = rel + 1 <= r ? 0.f : pr.y;
+          if (!kDense && c == kChunks - 1) pr.x = rel > r ? 0.f : pr.x, pr.y = rel + 1 > r ? 0.f : pr.y;
+          s[nt][2 * hh] = pr.x, s[nt][2 * hh + 1] = pr.y;
+          pr = mul2(pr, add2(make_float2(dp[nt][2 * hh], dp[nt][2 * hh + 1]), make_float2(-d.x, -d.y)));
+          dp[nt][2 * hh] = pr.x, dp[nt][2 * hh + 1] = pr.y;
         }
       }
       uint32_t pk[4];
@@ -358,20 +439,38 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
 #pragma unroll
     for (int e = 0; e < 4; ++e)
       if (!(e < 2 ? lo : hi)) acc0[t][e] = acc1[t][e] = 0.f;
-  store_rows(p.dk + in0, p.in.token, acc0, row, N, 1.f, 1.f);
+  store_rows(p.dk + in0, p.in.token, acc0, row, N, p.scale, p.scale);
   store_rows(p.dv + in0, p.in.token, acc1, row, N, 1.f, 1.f);
 }
 
+// *done: whether the launch was made; tiles of 128 rows need maps of their tensors.
 template <int W, int kRows>
-int launch_band(const BandParams& p, int BH, bool backward, cudaStream_t s) {
+int launch_band(const BandParams& p, int B, bool backward, cudaStream_t s, bool* done = nullptr) {
   constexpr int halo = (kRows + W) * kRowBytes;
-  const int bytes = backward ? 4 * halo + (kRows + W) * 8 : 2 * halo + kRows * kRowBytes;
+  const int bytes = 16 + (backward ? 4 * halo + (kRows + W) * 8 : 2 * halo + kRows * kRowBytes);
+  MapsOf<kRows> maps{};
+  if constexpr (kRows == 128) {
+    const __nv_bfloat16* src[4] = {backward ? p.q : p.k, backward ? p.k : p.v, backward ? p.v : p.q, backward ? p.grad_out : nullptr};
+    *done = true;
+    for (int t = 0; t < (backward ? 4 : 3); ++t) {
+      const RowLayout& l = t == 3 ? p.act : p.in;
+      *done = *done && make_strided_rows_tensor_map(&maps.m[t], src[t], p.N, {p.H, B}, l.token, {l.head, l.batch},
+                                                    !backward && t == 2 ? kRows : kRows + W);
+    }
+    if (!*done) return MF_OK;
+  }
   auto kernel = backward ? band_bwd_kernel<W, kRows> : band_fwd_kernel<W, kRows>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(band_attn_kernel)");
-  launch_dependent(kernel, dim3((p.N + kRows - 1) / kRows, BH), dim3(kRows * 2), bytes, s, p);
+  launch_dependent(kernel, dim3((p.N + kRows - 1) / kRows, B * p.H), dim3(kRows * 2), bytes, s, p, maps);
   MF_CHECK_LAUNCH("band_attn_kernel");
   return MF_OK;
+}
+template <int W>
+int launch_either(const BandParams& p, int B, bool wide, bool backward, cudaStream_t s) {
+  bool done = false;
+  const int rc = wide ? launch_band<W, 128>(p, B, backward, s, &done) : MF_OK;
+  return rc != MF_OK || done ? rc : launch_band<W, 64>(p, B, backward, s);
 }
 
 }  // namespace
@@ -405,17 +504,23 @@ int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward
   p.H = a.heads, p.N = a.tokens, p.scale = a.scale;
   p.in = layouts ? layouts[0] : contiguous_rows(a.heads, a.tokens);
   p.act = layouts ? layouts[1] : contiguous_rows(a.heads, a.tokens);
-  const int BH = a.batch * a.heads;
-  if (a.tokens <= kDenseTokens) return launch_band<0, kDenseTokens>(p, BH, backward, stream);
+  if (a.tokens <= kDenseTokens) return launch_band<0, kDenseTokens>(p, a.batch, backward, stream);
   // 128-row tiles re-read half as much halo; 64-row ones spread a call over twice as many CTAs, which pays while the wide ones
   // would not cover the chip.  Forward + backward at window 64, 64 | 128 rows: 8 structures of 128 tokens (64 wide tiles) 14.7 |
   // 16.3 us, 128 tiles 17.3 | 16.4, 256 tiles 29.1 | 22.5, 576 tiles 50.4 | 42.2; windows 32 and 128 turn at the same place.
-  const bool wide = (long long)BH * ((a.tokens + 127) / 128) >= 128;
+  const bool wide = (long long)a.batch * a.heads * ((a.tokens + 127) / 128) >= 128;
   switch (a.window) {
-    case 32: return wide ? launch_band<32, 128>(p, BH, backward, stream) : launch_band<32, 64>(p, BH, backward, stream);
-    case 64: return wide ? launch_band<64, 128>(p, BH, backward, stream) : launch_band<64, 64>(p, BH, backward, stream);
-    default: return wide ? launch_band<128, 128>(p, BH, backward, stream) : launch_band<128, 64>(p, BH, backward, stream);
+    case 32: return launch_either<32>(p, a.batch, wide, backward, stream);
+    case 64: return launch_either<64>(p, a.batch, wide, backward, stream);
+    default: return launch_either<128>(p, a.batch, wide, backward, stream);
   }
+}
+
+int band_attn_status(int32_t* host_status, cudaStream_t stream) {
+  cudaError_t e = cudaMemcpyFromSymbolAsync(host_status, g_band_status, sizeof(int32_t), 0, cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return cuda_error(e, "band attention status read-back");
+  return MF_OK;
 }
 
 }  // namespace mf

@@ -395,7 +395,8 @@ extern "C" int mf_local_attn_bwd(const MfSparseAttnArgs* a, void* stream) {
 }
 extern "C" int mf_sparse_attn_status(int32_t* host_status, void* stream) {
   MF_CHECK_ARG(host_status != nullptr, "mf_sparse_attn_status: null pointer");
-  return sparse_attn_sm100_status(host_status, static_cast<cudaStream_t>(stream));
+  const int rc = sparse_attn_sm100_status(host_status, static_cast<cudaStream_t>(stream));
+  return rc != MF_OK || *host_status != 0 ? rc : band_attn_status(host_status, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -33,18 +33,20 @@ bool tensor_maps_available() { return encoder() != nullptr; }
 static thread_local int g_last_encode_result = 0;
 int last_tensor_map_result() { return g_last_encode_result; }
 
-bool make_rows_tensor_map(CUtensorMap* map, const void* base, int rows_per_matrix, int matrices, int box_rows) {
+namespace {
+// `rank` dimensions from the innermost, 64 bf16 elements wide; strides in bytes of dimensions 1, 2, ...
+bool encode_rows(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, int box_rows) {
   EncodeTiledFn fn = encoder();
   g_last_encode_result = -1;  // refused before the driver was asked
-  if (!fn || !base || rows_per_matrix <= 0 || matrices <= 0 || box_rows <= 0 || box_rows > 256 || box_rows % 8) return false;
+  if (!fn || !base || box_rows <= 0 || box_rows > 256 || box_rows % 8) return false;
+  for (int i = 1; i < rank; ++i)
+    if (dims[i] == 0 || strides[i - 1] % 16) return false;
   if (reinterpret_cast<uintptr_t>(base) & 15u) return false;  // the copy engine needs a 16-byte aligned base
-  const cuuint64_t dims[3] = {64, (cuuint64_t)rows_per_matrix, (cuuint64_t)matrices};
-  const cuuint64_t strides[2] = {128, (cuuint64_t)rows_per_matrix * 128};  // bytes, dimensions 1 and 2
-  const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
-  const cuuint32_t elem_strides[3] = {1, 1, 1};
+  const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
+  const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
   CUtensorMap tmp;
   auto encode = [&]() {
-    return fn(&tmp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem_strides,
+    return fn(&tmp, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, elem_strides,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
@@ -60,6 +62,22 @@ bool make_rows_tensor_map(CUtensorMap* map, const void* base, int rows_per_matri
   if (r != CUDA_SUCCESS) return false;
   *map = tmp;
   return true;
+}
+}  // namespace
+
+bool make_rows_tensor_map(CUtensorMap* map, const void* base, int rows_per_matrix, int matrices, int box_rows) {
+  if (rows_per_matrix < 0 || matrices < 0) return false;
+  const cuuint64_t dims[3] = {64, (cuuint64_t)rows_per_matrix, (cuuint64_t)matrices};
+  const cuuint64_t strides[2] = {128, (cuuint64_t)rows_per_matrix * 128};  // bytes, dimensions 1 and 2
+  return encode_rows(map, base, 3, dims, strides, box_rows);
+}
+
+bool make_strided_rows_tensor_map(CUtensorMap* map, const void* base, int rows, const int (&matrices)[2], long long row_stride,
+                                  const long long (&matrix_strides)[2], int box_rows) {
+  if (rows < 0 || matrices[0] < 0 || matrices[1] < 0) return false;
+  const cuuint64_t dims[4] = {64, (cuuint64_t)rows, (cuuint64_t)matrices[0], (cuuint64_t)matrices[1]};
+  const cuuint64_t strides[3] = {(cuuint64_t)row_stride * 2, (cuuint64_t)matrix_strides[0] * 2, (cuuint64_t)matrix_strides[1] * 2};
+  return encode_rows(map, base, 4, dims, strides, box_rows);
 }
 
 }  // namespace mf

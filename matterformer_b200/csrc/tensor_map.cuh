@@ -20,6 +20,10 @@ constexpr int kTmaBoxRows = 32;
 // entry point is missing or the tensor does not meet the alignment rules; callers then use plain loads.
 // `box_rows` rows per copy (a multiple of 8, at most 256); the simplicial kernels use kTmaBoxRows.
 bool make_rows_tensor_map(CUtensorMap* map, const void* base, int rows_per_matrix, int matrices, int box_rows = 32);
+// The same for rows of 64 elements of `matrices[1]` x `matrices[0]` matrices whose rows and matrices lie at any stride (in elements,
+// multiples of 8): a map {64, rows, matrices[0], matrices[1]}.
+bool make_strided_rows_tensor_map(CUtensorMap* map, const void* base, int rows, const int (&matrices)[2], long long row_stride,
+                                  const long long (&matrix_strides)[2], int box_rows);
 // Result of the calling thread's last make_rows_tensor_map: the driver's code (0 = success), or -1 when the
 // arguments were refused before the driver was asked.
 int last_tensor_map_result();
@@ -40,6 +44,13 @@ __device__ __forceinline__ void tma_load_rows(void* smem_dst, const CUtensorMap*
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
       ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)),
       "l"(map), "r"(0), "r"(row0), "r"(mat), "r"((uint32_t)__cvta_generic_to_shared(bar))
+      : "memory");
+}
+// The same through a map of make_strided_rows_tensor_map.
+__device__ __forceinline__ void tma_load_strided_rows(uint32_t smem_dst, const CUtensorMap* map, int row0, int mat0, int mat1, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(smem_dst), "l"(map), "r"(0), "r"(row0), "r"(mat0), "r"(mat1), "r"((uint32_t)__cvta_generic_to_shared(bar))
       : "memory");
 }
 #endif
