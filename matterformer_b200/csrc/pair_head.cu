@@ -96,19 +96,24 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
   const bool one_chunk = N <= kChunk;  // then the partners are staged once per work item
 
   // the lane's slice of the parameters
-  float wr[kPer][kRbf], wo[kPer];
+  // (two neighbouring basis functions to a register pair: products and gradients take both in one instruction)
+  float2 wr[kPer][kRbf / 2];
+  float wo[kPer];
 #pragma unroll
   for (int m = 0; m < kPer; ++m) {
     wo[m] = p.w_out[lane + 32 * m];
 #pragma unroll
-    for (int r = 0; r < kRbf; ++r) wr[m][r] = p.w_rbf[(lane + 32 * m) * kRbf + r];
+    for (int r = 0; r < kRbf / 4; ++r) {
+      const float4 x = reinterpret_cast<const float4*>(p.w_rbf + (lane + 32 * m) * kRbf)[r];
+      wr[m][2 * r] = make_float2(x.x, x.y), wr[m][2 * r + 1] = make_float2(x.z, x.w);
+    }
   }
   const float b_out = p.b_out[0];
   const T* own_src = static_cast<const T*>(MODE == kBackwardCols ? p.b : p.a);
   const T* partner_src = static_cast<const T*>(MODE == kBackwardCols ? p.a : p.b);
 
   // parameter gradients of everything this CTA works on (owner = i pass only)
-  float g_wr[MODE == kBackwardRows ? kPer : 1][MODE == kBackwardRows ? kRbf : 1] = {};
+  float2 g_wr[MODE == kBackwardRows ? kPer : 1][MODE == kBackwardRows ? kRbf / 2 : 1] = {};
   float g_wo[kPer] = {};
   float g_bo = 0.f;
 
@@ -222,7 +227,8 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
           }
           const int t_end = min(32, steps_end - s0);
           for (int tt = 0; tt < t_end; tt += U) {
-            float rb[U][kRbf], d[U][3], dw[U], keep[U], wsum[U];
+            float2 rb[U][kRbf / 2];
+            float d[U][3], dw[U], keep[U], wsum[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
               const float4 q = sm.pxyz[s0 + tt + u];
@@ -231,7 +237,7 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
 #pragma unroll
               for (int r = 0; r < kRbf; r += 4) {
                 const float4 e = *reinterpret_cast<const float4*>(&sm.rbf[warp][(tt + u) * kRbfStride + r]);
-                rb[u][r] = e.x, rb[u][r + 1] = e.y, rb[u][r + 2] = e.z, rb[u][r + 3] = e.w;
+                rb[u][r / 2] = make_float2(e.x, e.y), rb[u][r / 2 + 1] = make_float2(e.z, e.w);
               }
               // x_i - x_j with i the first index of the pair
               const float sgn = MODE == kBackwardCols ? -1.f : 1.f;
@@ -247,9 +253,10 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
             for (int m = 0; m < kPer; ++m) {
 #pragma unroll
               for (int u = 0; u < U; ++u) {
-                float pre = own[m] + sm.part[s0 + tt + u][lane + 32 * m];
+                float2 pre2 = make_float2(own[m] + sm.part[s0 + tt + u][lane + 32 * m], 0.f);
 #pragma unroll
-                for (int r = 0; r < kRbf; ++r) pre = fmaf(wr[m][r], rb[u][r], pre);
+                for (int r = 0; r < kRbf / 2; ++r) pre2 = fma2(wr[m][r], rb[u][r], pre2);
+                const float pre = pre2.x + pre2.y;
                 const float sig = __fdividef(1.f, 1.f + __expf(-pre));
                 if (MODE == kForward) {
                   wsum[u] = fmaf(wo[m], pre * sig, wsum[u]);
@@ -259,7 +266,7 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
                   if constexpr (MODE == kBackwardRows) {
                     g_wo[m] = fmaf(dw[u], pre * sig, g_wo[m]);
 #pragma unroll
-                    for (int r = 0; r < kRbf; ++r) g_wr[m][r] = fmaf(dh, rb[u][r], g_wr[m][r]);
+                    for (int r = 0; r < kRbf / 2; ++r) g_wr[m][r] = fma2(make_float2(dh, dh), rb[u][r], g_wr[m][r]);
                   }
                 }
               }
@@ -301,7 +308,10 @@ __global__ void __launch_bounds__(kWarps * 32) pair_head_kernel(const PairHeadPa
         for (int m = 0; m < kPer; ++m) {
           const int c = lane + 32 * m;
 #pragma unroll
-          for (int r = 0; r < kRbf; ++r) red[c * kRbf + r] = (w ? red[c * kRbf + r] : 0.f) + g_wr[m][r];
+          for (int r = 0; r < kRbf / 2; ++r) {
+            float2& o = *reinterpret_cast<float2*>(&red[c * kRbf + 2 * r]);
+            o = add2(w ? o : make_float2(0.f, 0.f), g_wr[m][r]);
+          }
           red[kHid * kRbf + c] = (w ? red[kHid * kRbf + c] : 0.f) + g_wo[m];
         }
         if (lane == 0) red[kHid * kRbf + kHid] = (w ? red[kHid * kRbf + kHid] : 0.f) + g_bo;
