@@ -5,7 +5,9 @@
 // products like the attention itself, so this kernel walks query by query (the kernel without residuals walks over first
 // keys, where the factors would be different for every row).  A warp takes a query: 32 x 32 logits in registers, factors
 // staged in its own shared memory as hi + lo bf16 (see RankTile), exact maximum, P as the B operand of W^T = V2^T P^T and
-// of T^T = MR^T P^T, c_ir = sum_j ML_jr T_jr.
+// of T^T = MR^T P^T, c_ir = sum_j ML_jr T_jr.  The bias and the basis of the head come to shared memory with the tiles: loaded where
+// a query needs them they were most of its instructions (64 molecules of 9-29 atoms with the bias at rank 16 60 -> 50 us, 32 of 10-32 at
+// rank 32 75 -> 58).  One variant of the walk for all sizes: narrower ones for small molecules took that back (see simplicial_small_bwd.cu).
 #include "common.cuh"
 #include "simplicial.cuh"
 #include "simplicial_warp.cuh"
@@ -47,41 +49,18 @@ struct ResFwdShared {
   __align__(128) uint8_t tile[5][kSmallTile];                            // q, k1, v1, k2, v2
   __align__(128) uint8_t factor[kResWarps][4][2 * RankTile<RK>::kTile];  // L, R, ML, MR of the warp's query
   uint32_t visible[kSmallRows];
+  // bias: w_jk as the fragments of the logits hold it, u_ij, v_ik and the gate
+  float4 w[8][32];
+  float u[kSmallRows][kSmallRows], v[kSmallRows][kSmallRows], gate[kSmallRows];
+  float basis[16 * RK][kD];  // of the head, zeros beyond the rank
 };
 
-template <int RK>
-__global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_kernel(const __grid_constant__ ResFwdParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
-  ResFwdShared<RK>& sm = *reinterpret_cast<ResFwdShared<RK>*>(smem);
-  constexpr int kThreads = 32 * kResWarps, MT = 2, NT = 4;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = lane & 3, row8 = lane >> 2;
-  const int N = p.N, h = blockIdx.x % p.H, b = p.order ? p.order[blockIdx.x / p.H] : blockIdx.x / p.H, bh = b * p.H + h;
-  const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
-  const uint32_t qmask = __ballot_sync(0xffffffffu, lane < N && p.query_valid[(size_t)b * N + min(lane, N - 1)] > 0);
-  const int n = 32 - __clz(kmask);
-  const RowLayout rows{(long long)p.H * N * kD, (long long)N * kD, kD};
-  {
-    const __nv_bfloat16* src[5] = {p.q, p.k1, p.v1, p.k2, p.v2};
-    const uint32_t t0 = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
-#pragma unroll
-    for (int t = 0; t < 5; ++t)
-      for (int idx = tid; idx < 8 * kSmallRows; idx += kThreads) {
-        const int r = idx >> 3, c = idx & 7;
-        const bool ok = ((t == 0 ? qmask : kmask) >> r) & 1u;
-        cp_async16(row_chunk(t0 + t * kSmallTile, r, c), src[t] + rows.at(b, h, ok ? r : 0) + c * 8, ok);
-      }
-    cp_async_commit();
-  }
-  for (int idx = tid; idx < (int)sizeof(sm.factor) / 16; idx += kThreads) reinterpret_cast<float4*>(sm.factor)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int j = warp; j < kSmallRows; j += kResWarps) {
-    uint32_t word = (j < N && ((kmask >> j) & 1u)) ? kmask : 0u;
-    if (p.pair_valid && word != 0u)
-      word &= __ballot_sync(0xffffffffu, lane < N && p.pair_valid[((size_t)b * N + j) * N + min(lane, N - 1)] > 0);
-    if (lane == 0) sm.visible[j] = word;
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-
+// The queries of a warp.
+template <int MT, int NT, int RK>
+__device__ __forceinline__ void res_fwd_queries(const ResFwdParams& p, ResFwdShared<RK>& sm, int bh, int n, uint32_t kmask,
+                                                uint32_t qmask) {
+  constexpr int KS = (NT + 1) / 2;  // 16-key steps of the products over the second keys
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2, N = p.N;
   const uint32_t qt = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
   const FragBase fb(qt, lane);
   constexpr int kTk1 = kSmallTile, kTv1 = 2 * kSmallTile, kTk2 = 3 * kSmallTile, kTv2 = 4 * kSmallTile;
@@ -120,19 +99,22 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
         pair_product<MT, NT>(s, fb, kTk1, kTk2, qf);
       }
       if (p.u) {
-        const size_t row = qi * N + lane;
-        const float ul = lane < n ? p.u[row] : 0.f, vl = lane < n ? p.v_bias[row] : 0.f, g = p.gate[qi];
+        const float g = sm.gate[i];
+        float ur[MT][2];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+        for (int mt = 0; mt < MT; ++mt) ur[mt][0] = sm.u[i][mt * 16 + row8], ur[mt][1] = sm.u[i][mt * 16 + 8 + row8];
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < NT; ++nt) {
+          const float2 v = *reinterpret_cast<const float2*>(&sm.v[i][nt * 8 + 2 * quad]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int j = mt * 16 + (e >> 1) * 8 + row8, k = nt * 8 + 2 * quad + (e & 1);
-              const float uv = __shfl_sync(0xffffffffu, ul, j) + __shfl_sync(0xffffffffu, vl, k);
-              const float w = (j < n && k < n) ? p.w[((size_t)bh * N + j) * N + k] : 0.f;
-              s[mt][nt][e] = fmaf(g, uv + w, s[mt][nt][e]);
-            }
+          for (int mt = 0; mt < MT; ++mt) {
+            const float4 w = sm.w[mt * 4 + nt][lane];
+            s[mt][nt][0] = fmaf(g, (ur[mt][0] + v.x) + w.x, s[mt][nt][0]);
+            s[mt][nt][1] = fmaf(g, (ur[mt][0] + v.y) + w.y, s[mt][nt][1]);
+            s[mt][nt][2] = fmaf(g, (ur[mt][1] + v.x) + w.z, s[mt][nt][2]);
+            s[mt][nt][3] = fmaf(g, (ur[mt][1] + v.y) + w.w, s[mt][nt][3]);
+          }
+        }
       }
       if (p.al) {
         float ad[MT][NT][4];
@@ -163,13 +145,17 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
       m = warp_max(m);
       have = m > -INFINITY;
       const float m2 = have ? m * kLog2e : 0.f;
-      uint32_t pk[MT][NT][2];
+      uint32_t pk[MT][2 * KS][2];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < 2 * KS; ++nt)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
+            if (nt >= NT) {
+              pk[mt][nt][hh] = 0u;
+              continue;
+            }
             const float a = fast_exp2(fmaf(s[mt][nt][2 * hh], kLog2e, -m2)), c = fast_exp2(fmaf(s[mt][nt][2 * hh + 1], kLog2e, -m2));
             l += a + c;
             pk[mt][nt][hh] = pack2_bf16(a, c);
@@ -179,7 +165,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
       for (int dt = 0; dt < 4; ++dt) {
         float w[2 * MT][4];
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
+        for (int ks = 0; ks < KS; ++ks) {
           uint32_t a[4];
           load_t(a, fb, kTv2, dt, ks);
 #pragma unroll
@@ -209,7 +195,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
 #pragma unroll
         for (int rk = 0; rk < RK; ++rk) {
           float t[2 * MT][4], lo = 0.f, hi = 0.f;
-          rank_sums<MT, NT, RK>(t, mright, pk, rk, lane);
+          rank_sums<MT, 2 * KS, RK>(t, mright, pk, rk, lane);
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
             uint32_t mh[4], mo[4];
@@ -241,12 +227,8 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
 #pragma unroll
         for (int r8 = 0; r8 < 8; ++r8) {
           const float c = __shfl_sync(0xffffffffu, coef[e], 4 * r8) * scale;
-          const int r = 8 * e + r8;
-          if (r < p.rm) {
-            const float* bs = p.basis + ((size_t)h * p.rm + r) * kD + d0;
-            x0 = fmaf(c, bs[0], x0);
-            x1 = fmaf(c, bs[8], x1);
-          }
+          x0 = fmaf(c, sm.basis[8 * e + r8][d0], x0);
+          x1 = fmaf(c, sm.basis[8 * e + r8][d0 + 8], x1);
         }
     }
     const float inv = have ? 1.f / l : 0.f;
@@ -259,6 +241,62 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
     }
     if (lane == 0) p.lse[qi] = have ? m + logf(l) : 0.f;
   }
+}
+
+template <int RK>
+__global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_kernel(const __grid_constant__ ResFwdParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  ResFwdShared<RK>& sm = *reinterpret_cast<ResFwdShared<RK>*>(smem);
+  wait_for_previous();
+  constexpr int kThreads = 32 * kResWarps;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int N = p.N, h = blockIdx.x % p.H, b = p.order ? p.order[blockIdx.x / p.H] : blockIdx.x / p.H, bh = b * p.H + h;
+  const uint32_t kmask = __ballot_sync(0xffffffffu, lane < N && p.key_valid[(size_t)b * N + min(lane, N - 1)] > 0);
+  const uint32_t qmask = __ballot_sync(0xffffffffu, lane < N && p.query_valid[(size_t)b * N + min(lane, N - 1)] > 0);
+  const int n = 32 - __clz(kmask);
+  const RowLayout rows{(long long)p.H * N * kD, (long long)N * kD, kD};
+  {
+    const __nv_bfloat16* src[5] = {p.q, p.k1, p.v1, p.k2, p.v2};
+    const uint32_t t0 = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
+#pragma unroll
+    for (int t = 0; t < 5; ++t)
+      for (int idx = tid; idx < 8 * kSmallRows; idx += kThreads) {
+        const int r = idx >> 3, c = idx & 7;
+        const bool ok = ((t == 0 ? qmask : kmask) >> r) & 1u;
+        cp_async16(row_chunk(t0 + t * kSmallTile, r, c), src[t] + rows.at(b, h, ok ? r : 0) + c * 8, ok);
+      }
+    if (p.ml)
+      for (int idx = tid; idx < 16 * RK * kD; idx += kThreads) {
+        const int r = idx / kD;
+        cp_async4(&sm.basis[r][idx % kD], p.basis + ((size_t)h * p.rm + min(r, p.rm - 1)) * kD + idx % kD, r < p.rm);
+      }
+    if (p.u && n > 0) {
+      for (int idx = tid; idx < N * kSmallRows; idx += kThreads) {
+        const int x = idx >> 5, y = idx & 31;
+        const size_t at = ((size_t)bh * N + x) * N + min(y, n - 1);
+        cp_async4(&sm.u[x][y], p.u + at, y < n);
+        cp_async4(&sm.v[x][y], p.v_bias + at, y < n);
+      }
+      for (int x = tid; x < N; x += kThreads) cp_async4(&sm.gate[x], p.gate + (size_t)bh * N + x, true);
+      for (int idx = tid; idx < 4 * 8 * 32; idx += kThreads) {
+        const int f = idx >> 7, ln = (idx >> 2) & 31, e = idx & 3;
+        const int j = (f >> 2) * 16 + 8 * (e >> 1) + (ln >> 2), k = (f & 3) * 8 + 2 * (ln & 3) + (e & 1);
+        const bool ok = j < n && k < n;
+        cp_async4(reinterpret_cast<float*>(&sm.w[f][ln]) + e, p.w + (size_t)bh * N * N + (ok ? j * N + k : 0), ok);
+      }
+    }
+    cp_async_commit();
+  }
+  for (int idx = tid; idx < (int)sizeof(sm.factor) / 16; idx += kThreads) reinterpret_cast<float4*>(sm.factor)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j = warp; j < kSmallRows; j += kResWarps) {
+    uint32_t word = (j < N && ((kmask >> j) & 1u)) ? kmask : 0u;
+    if (p.pair_valid && word != 0u)
+      word &= __ballot_sync(0xffffffffu, lane < N && p.pair_valid[((size_t)b * N + j) * N + min(lane, N - 1)] > 0);
+    if (lane == 0) sm.visible[j] = word;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  res_fwd_queries<2, 4, RK>(p, sm, bh, n, kmask, qmask);
 }
 
 }  // namespace
@@ -282,7 +320,7 @@ int simplicial_small_res_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream) 
   p.H = a.heads, p.N = a.tokens;
   auto launch = [&](auto kernel, int bytes) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) kernel<<<a.batch * a.heads, 32 * kResWarps, bytes, stream>>>(p);
+    if (e == cudaSuccess) launch_dependent(kernel, dim3(a.batch * a.heads), dim3(32 * kResWarps), bytes, stream, p);
     return e;
   };
   profile_mark(MF_PROFILE_SIMPLICIAL_FWD, true, stream);
