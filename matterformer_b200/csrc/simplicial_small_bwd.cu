@@ -357,7 +357,7 @@ __device__ __forceinline__ void small_bwd_side(const SmallBwdParams& p, Shared& 
                   if (k < p.N && r < rank) gr[(qi * p.N + k) * rank + r] = (kKeySide ? ga : sm.dc[i][r]) * c[kt][t8][e];
                 }
           }
-          if (kKeySide) {
+          if constexpr (kKeySide) {
             gate_sum += lo + hi;
           } else {
             quad_reduce(lo);
@@ -495,7 +495,10 @@ __device__ __forceinline__ void small_bwd_walks(const SmallBwdParams& p, Shared&
   store_rows(p.dk1, p.dk2);
 }
 
-template <bool kBias, int RK, int kWarps>
+// kSizes: the variants for molecules beyond 16 keys that the kernel holds, 1 = up to 24, 2 = up to 32.  (Three variants on an SM at a time
+// strain its instruction cache; without the bias that costs more than the narrower one saves.  9-29 atoms, both | the wider one alone:
+// 64 molecules 60.8 | 57.6 us, 1 024 492 | 480, with the bias 256 187 | 192.)
+template <bool kBias, int RK, int kWarps, int kSizes>
 __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_kernel(const __grid_constant__ SmallBwdParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   using Shared = SmallBwdShared<kBias, RK, kWarps>;
@@ -606,10 +609,14 @@ __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) simplicial_small_bwd_
       }
       __syncthreads();
     }
+    // one variant for all sizes: four of them on an SM at a time do not fit its instruction cache (64 molecules of 9-29 atoms at rank 16
+    // 174 us with one, 227 with a variant for each size class)
     if (n > 0) small_bwd_walks<2, 4, true, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
   } else if (n > 0) {
     if (hole) small_bwd_walks<2, 4, true, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
     else if (n <= 16) small_bwd_walks<1, 2, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else if constexpr (kSizes == 1) small_bwd_walks<2, 3, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
+    else if constexpr (kSizes == 2) small_bwd_walks<2, 4, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
     else if (n <= 24) small_bwd_walks<2, 3, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
     else small_bwd_walks<2, 4, false, kBias, RK, kWarps>(p, sm, b, h, n, kmask, qmask);
   }
@@ -690,21 +697,25 @@ int simplicial_small_bwd(const MfSimplicialBwdArgs& a, const TileLayouts* layout
   const int warps = bh >= 1024 ? 2 : 4;
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
   cudaError_t e = cudaSuccess;
-#define MF_LAUNCH(BIAS, RK, S)                                                                                             \
+#define MF_LAUNCH(BIAS, RK, S, SIZES)                                                                                      \
   do {                                                                                                                 \
     constexpr int bytes = (int)sizeof(SmallBwdShared<BIAS, RK, S>);                                                        \
-    e = cudaFuncSetAttribute(simplicial_small_bwd_kernel<BIAS, RK, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
-    if (e == cudaSuccess) launch_dependent(simplicial_small_bwd_kernel<BIAS, RK, S>, dim3(bh), dim3(32 * S), bytes, stream, p);                      \
+    auto kernel = simplicial_small_bwd_kernel<BIAS, RK, S, SIZES>;                                                         \
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);                                  \
+    if (e == cudaSuccess) launch_dependent(kernel, dim3(bh), dim3(32 * S), bytes, stream, p);                              \
   } while (0)
   if (a.angle_left || a.message_left) {
-    if (max(p.ra, p.rm) <= 16) MF_LAUNCH(true, 1, 4);
-    else MF_LAUNCH(true, 2, 4);
+    if (max(p.ra, p.rm) <= 16) MF_LAUNCH(true, 1, 4, 2);
+    else MF_LAUNCH(true, 2, 4, 2);
   } else if (a.u) {
-    if (warps == 2) MF_LAUNCH(true, 0, 2);
-    else MF_LAUNCH(true, 0, 4);
+    if (warps == 2) MF_LAUNCH(true, 0, 2, 3);
+    else MF_LAUNCH(true, 0, 4, 3);
+  } else if (a.tokens <= 24) {
+    if (warps == 2) MF_LAUNCH(false, 0, 2, 1);
+    else MF_LAUNCH(false, 0, 4, 1);
   } else {
-    if (warps == 2) MF_LAUNCH(false, 0, 2);
-    else MF_LAUNCH(false, 0, 4);
+    if (warps == 2) MF_LAUNCH(false, 0, 2, 2);
+    else MF_LAUNCH(false, 0, 4, 2);
   }
 #undef MF_LAUNCH
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_small_bwd_kernel)");
