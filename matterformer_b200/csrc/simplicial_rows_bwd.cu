@@ -19,8 +19,8 @@
 // memory as bf16 and a GEMM against a 0/1 selector sums the rows of each group (M = 128 output columns,
 // N = 16 groups, K = 128 rows), so the column sums of a step cost one narrow MMA instead of a shuffle tree.
 //
-// dK2 / dV2 of the first 128 keys leave the CTA as final bf16 rows (no other CTA contributes to them).  Everything
-// else is written as fp32 partials per part and summed in a fixed order by the finalize kernel; within a CTA dk1 / dv1
+// Small batches walk in several pieces per part (see Pieces).  dK2 / dV2 of the first 128 keys leave the CTA as final bf16 rows where
+// one piece walks them all (no other CTA contributes to them).  Everything else is written as fp32 partials and summed in a fixed order by the finalize kernel; within a CTA dk1 / dv1
 // partials are accumulated over the query ranges by plain read-modify-write of addresses only this CTA
 // touches.  There are no floating-point atomics: gradients are bit-identical from run to run.
 //
@@ -30,6 +30,8 @@
 // global load.  The element-wise pass handles the slab as two halves of 64 logit columns so that U and W of the
 // first half are issued while the second is still being processed.  Hand-offs are mbarriers (one elected lane
 // per warp arrives); every wait is bounded and an expired wait is reported through the status word.
+#include <algorithm>
+
 #include "common.cuh"
 #include "simplicial.cuh"
 #include "simplicial_rows.cuh"
@@ -81,18 +83,21 @@ struct RowsBwdParams {
   const uint8_t* query_valid;
   const uint8_t* key_valid;
   const uint8_t* pair_valid;
-  __nv_bfloat16* dk2;  // keys [0, 128): final
+  __nv_bfloat16* dk2;  // keys [0, 128): final where part 0 is one piece
   __nv_bfloat16* dv2;
-  float* dq_part;      // [part] x (BH, N, 64) fp32
-  float* dk1_part;     // two planes: part 0, parts 1 and 2
+  float* dq_part;      // a plane of (BH, N, 64) fp32 for each piece of each part
+  float* dk1_part;     // planes: part 0; the pieces of parts 1 and 2
   float* dv1_part;
+  float* dk2_low;      // pieces of part 0 (where there are several): planes of (BH, min(N, 128), 64)
+  float* dv2_low;
   float* dk2_part;     // parts 1 and 2: planes of (BH, N - 128, 64) for the keys from 128 on
   float* dv2_part;
   const BatchInfo* info;
   const int32_t* order;
   int32_t* status;
   int H, N, BH;
-  size_t part_stride, part2_stride;  // elements per plane
+  size_t part_stride, part2_stride, low_stride;  // elements per plane
+  int pieces, pieces12;                          // of part 0; of parts 1 and 2
   int use_tma;
   CUtensorMap tm_k[2];   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle: second keys, first keys
   CUtensorMap tm_v[2];
@@ -115,8 +120,45 @@ __device__ __forceinline__ Part part_of(int index, int n_keys) {
   return index == 1 ? Part{true, 0, kSlab, kSlab} : Part{true, kSlab, n_keys - kSlab, kSlab};
 }
 
+// A part walks its first keys in one piece where the molecules fill the chip several times over, and in several, a CTA each, where they
+// do not: a CTA by itself takes the walk's full length however few others there are, and the largest molecule of a batch decides.
+// A piece costs its set-up and fp32 planes for the sums that run over the walk.
+struct Pieces {
+  int first, others;  // of part 0; of parts 1 and 2, by the share of the keys that they walk
+};
+// The number with the shortest estimate: the longer of one piece (the largest molecule: kPieceUs for its set-up and the beginnings and
+// ends of its query ranges, and its share of a walk of kWalkUs N^2, both from measured times) and all of them on kSms SMs, the batch at
+// half of its largest molecule's work (sizes spread from an eighth up 0.38, all full 1; the host does not know).  A molecule or two
+// cannot fill a second wave with small pieces: it counts by itself.  Powers of two, so that batches near each other share a number: on
+// one side of a line a molecule's bits do not depend on its batch.  8 heads, n / 3 to n atoms, the kernel in us, one piece | this:
+// 40 tokens, 1, 4, 16 molecules 51 | 17, 51 | 25, 52 | 52; 96 235 | 47, 235 | 71, 241 | 146; 128 401 | 43, 401 | 110, 408 | 235; 181 (three
+// parts in one piece each 880) 163, 295, 671.
+inline Pieces pieces_of(int BH, int N) {
+  constexpr float kPieceUs = 30.f, kWalkUs = 0.0245f, kShare = 0.5f, kSms = 148.f;
+  const float walk = kWalkUs * N * N, rest = N > kSlab ? walk * (N - kSlab) / N : 0.f;
+  Pieces best{1, 1};
+  float least = INFINITY;
+  for (int pieces = 1; pieces <= 16; pieces *= 2) {
+    const int others = N > kSlab ? std::max(1, (int)(pieces * (N - kSlab) / (float)N + 0.5f)) : 0;
+    const float all = BH * ((pieces + 2 * others) * kPieceUs + kShare * (walk + 2.f * rest)) / kSms;
+    float piece = kPieceUs + walk / pieces;
+    const int waves = (BH * (pieces + 2 * others) + (int)kSms - 1) / (int)kSms;
+    if (BH <= 16 && waves > 1) piece *= waves * (N > kSlab ? 0.78f : 0.6f);
+    const float time = std::max(piece, all);
+    if (time < 0.97f * least) least = time, best = Pieces{pieces, std::max(1, others)};
+  }
+  return best;
+}
+// walked keys of a piece, and how many pieces have any
+__host__ __device__ __forceinline__ int piece_keys(int walked, int pieces) { return (walked + pieces - 1) / pieces; }
+__device__ __forceinline__ int pieces_used(int walked, int pieces) {
+  const int each = piece_keys(walked, pieces);
+  return each > 0 ? (walked + each - 1) / each : 0;
+}
+
 __global__ void delta_rows_kernel(const __nv_bfloat16* __restrict__ grad_out, const float* __restrict__ out,
                                   float* __restrict__ delta, int rows) {
+  wait_for_previous();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -131,6 +173,8 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// kParted: the batch has room for molecules of more than 128 keys.
+template <bool kParted>
 __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constant__ RowsBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -140,30 +184,29 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
   __shared__ uint64_t bar_kv;                                   // bulk tensor copies of the K2 / V2 slab
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t kmask[kMaskWords];
-  __shared__ uint8_t valid_keys[kMaxKeys];
+  __shared__ uint8_t jlist[kMaxKeys];
 
+  wait_for_previous();
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool is_worker = tid < 256;
   const int grp = (tid >> 7) & 1;  // 0: q side, 1: dO side
   const int r = tid & 127;         // row of the tile
   // heavy molecules first, and of all molecules part 0 (the longest) before the others
-  const int rest = (int)blockIdx.x - p.BH;
-  const int part = rest < 0 ? 0 : 1 + (rest & 1), item = rest < 0 ? (int)blockIdx.x : rest >> 1;
+  const int rest = kParted ? (int)blockIdx.x - p.BH * p.pieces : -1;
+  const int part = rest < 0 ? 0 : 1 + (rest & 1), pieces = rest < 0 ? p.pieces : p.pieces12;
+  const int at = rest < 0 ? (int)blockIdx.x : rest >> 1, item = at / pieces, piece = at - item * pieces;
   const int b = p.order[item / p.H], h = item % p.H;
   const int N = p.N;
   const int bh = b * p.H + h;
   const size_t base = (size_t)bh * N * kD;
   const int n_keys = p.info[b].n_keys;
   const int n_queries = p.info[b].n_queries;
-  const Part own = part_of(part, n_keys);
+  const Part own = kParted ? part_of(part, n_keys) : Part{false, 0, n_keys, 0};
   const int k0 = own.col0, nk_slab = own.cols;  // columns: keys [k0, k0 + nk_slab) of the one set
   if (nk_slab <= 0) return;                     // the finalize kernel writes the zeros
-  // keys of the other set that are walked: the valid ones from walk0 on
-  int before = 0;
-  if (own.walk0 > 0)
-    for (int k = threadIdx.x & 31; k < own.walk0; k += 32) before += p.key_valid[(size_t)b * N + k] > 0;
-  before = __reduce_add_sync(0xffffffffu, before);
-  const int nj = p.info[b].reserved0 - before;
+  // keys of the other set that are walked: this piece of the valid ones from walk0 on
+  const int skipped = own.walk0 > 0 ? p.info[b].reserved1 : 0, walked = p.info[b].reserved0 - skipped, each = piece_keys(walked, pieces);
+  const int before = skipped + piece * each, nj = min(each, walked - piece * each);
   const RowPlan plan = plan_rows(n_queries, nj);
   if (plan.tiles == 0) return;
   const __nv_bfloat16 *walk_k = own.exchanged ? p.k2 : p.k1, *walk_v = own.exchanged ? p.v2 : p.v1;
@@ -202,12 +245,11 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
     kmask[tid] = w;
   }
   __syncthreads();
-  if (tid < kMaxKeys && ((kmask[tid >> 5] >> (tid & 31)) & 1u)) {  // compacted list of the valid keys
+  if (tid < kMaxKeys && ((kmask[tid >> 5] >> (tid & 31)) & 1u)) {  // compacted list of the valid keys that are walked
     int pos = __popc(kmask[tid >> 5] & ((1u << (tid & 31)) - 1u));
     for (int c = 0; c < (tid >> 5); ++c) pos += __popc(kmask[c]);
-    valid_keys[pos] = (uint8_t)tid;
+    if (pos >= before && pos < before + nj) jlist[pos - before] = (uint8_t)tid;
   }
-  const uint8_t* const jlist = valid_keys + before;
   auto key_live = [&](int rr) {  // slab row rr holds a key that takes part
     const int k = k0 + rr;
     return rr < nk_slab && ((kmask[k >> 5] >> (k & 31)) & 1u);
@@ -662,7 +704,8 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
       // ---- end of the range: last column sums, then dq of the range (rows of one query summed over the groups)
       prefetch_sums(t, steps - 1);
       commit_sums(steps - 1);  // also: every product issued so far has completed
-      float* dq_dst = p.dq_part + (size_t)part * p.part_stride + base;
+      const int plane = part == 0 ? piece : p.pieces + (part - 1) * p.pieces12 + piece;
+      float* dq_dst = p.dq_part + (size_t)plane * p.part_stride + base;
       if (G == 1) {
         if (slot_ok && i < n_queries) {
           float4* dst = reinterpret_cast<float4*>(dq_dst + (size_t)i * kD + 32 * grp);
@@ -706,7 +749,9 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
     tc_fence_after_sync();
     {
       __nv_bfloat16* dst = (grp == 0 ? p.dk2 : p.dv2) + base + (size_t)(k0 + r) * kD;
-      float* dst32 = (grp == 0 ? p.dk1_part : p.dv1_part) + p.part_stride + base + (size_t)(k0 + r) * kD;
+      const bool partial = own.exchanged || p.pieces > 1;
+      float* dst32 = own.exchanged ? (grp == 0 ? p.dk1_part : p.dv1_part) + (1 + piece) * p.part_stride + base + (size_t)(k0 + r) * kD
+                                   : (grp == 0 ? p.dk2_low : p.dv2_low) + piece * p.low_stride + ((size_t)bh * min(N, kSlab) + r) * kD;
       const bool store = !bad && r < nk_slab;
       const bool live = key_live(r);
 #pragma unroll
@@ -714,7 +759,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         uint32_t w[32];
         tmem_ld32(tmem_row + (grp == 0 ? kColDK2 : kColDV2) + 32 * half, w);  // whole warps: the load is warp-wide
         tmem_ld_wait();
-        if (store && own.exchanged) {
+        if (store && partial) {
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             reinterpret_cast<uint4*>(dst32 + 32 * half)[c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
@@ -750,6 +795,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
 __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat16* __restrict__ dq,
                                                     __nv_bfloat16* __restrict__ dk1, __nv_bfloat16* __restrict__ dv1,
                                                     int BH) {
+  wait_for_previous();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // one thread per 4 elements
   const long long total = (long long)BH * p.N * (kD / 4);
   if (idx >= total) return;
@@ -761,6 +807,8 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
   const bool failed = p.status[0] != 0;
   const bool active = n_queries > 0 && nj > 0 && !failed;
   const bool parted = n_keys > kSlab;
+  const int used = p.pieces > 1 ? pieces_used(nj, p.pieces) : 1;
+  const int used12 = !parted ? 0 : p.pieces12 > 1 ? pieces_used(nj - p.info[b].reserved1, p.pieces12) : 1;
   const size_t off = ((size_t)bh * p.N + row) * kD + 4 * d4;
   const bool q_ok = active && row < n_queries && p.query_valid[(size_t)b * p.N + row] > 0;
   const bool k_ok = active && row < n_keys && p.key_valid[(size_t)b * p.N + row] > 0;
@@ -777,20 +825,30 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
     *reinterpret_cast<uint2*>(dst) = o;
   };
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (q_ok)
-    for (int s = 0; s < (parted ? kParts : 1); ++s) add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)s * p.part_stride + off));
+  if (q_ok) {
+    auto plane = [&](int s) { add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)s * p.part_stride + off)); };
+    for (int s = 0; s < used; ++s) plane(s);
+    for (int part = 0; part < 2; ++part)
+      for (int s = 0; s < used12; ++s) plane(p.pieces + part * p.pieces12 + s);
+  }
   store4(dq + off, a);
   float4 k1v = make_float4(0.f, 0.f, 0.f, 0.f), v1v = k1v;
   if (k_ok)
-    for (int s = 0; s < (parted ? 2 : 1); ++s) {
+    for (int s = 0; s < 1 + used12; ++s) {
       add4(k1v, *reinterpret_cast<const float4*>(p.dk1_part + (size_t)s * p.part_stride + off));
       add4(v1v, *reinterpret_cast<const float4*>(p.dv1_part + (size_t)s * p.part_stride + off));
     }
   store4(dk1 + off, k1v);
   store4(dv1 + off, v1v);
-  if (row >= kSlab || !(active && row < n_keys)) {  // (the others were stored by part 0)
+  if (row >= kSlab || p.pieces > 1 || !(active && row < n_keys)) {  // (the others were stored by part 0)
     float4 k2v = make_float4(0.f, 0.f, 0.f, 0.f), v2v = k2v;
-    if (k_ok)
+    if (k_ok && row < kSlab)
+      for (int s = 0; s < used; ++s) {
+        const size_t low = s * p.low_stride + ((size_t)bh * min(p.N, kSlab) + row) * kD + 4 * d4;
+        add4(k2v, *reinterpret_cast<const float4*>(p.dk2_low + low));
+        add4(v2v, *reinterpret_cast<const float4*>(p.dv2_low + low));
+      }
+    else if (k_ok)
       for (int s = 0; s < 2; ++s) {
         const size_t off2 = (size_t)s * p.part2_stride + ((size_t)bh * (p.N - kSlab) + row - kSlab) * kD + 4 * d4;
         add4(k2v, *reinterpret_cast<const float4*>(p.dk2_part + off2));
@@ -802,17 +860,20 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
 }
 
 struct RowsBwdLayout {
-  size_t info, order, delta, dq, dk1, dv1, dk2, dv2, total;
-  int parts;
-  size_t part, part2;  // bytes per partial plane
+  size_t info, order, delta, dq, dk1, dv1, dk2, dv2, dk2_low, dv2_low, total;
+  Pieces pieces;
+  int ctas;                 // per (batch, head): one for each piece of each part
+  size_t part, part2, low;  // bytes per partial plane
 };
 
 RowsBwdLayout rows_bwd_layout(int B, int H, int N) {
   RowsBwdLayout l{};
-  l.parts = N > kSlab ? kParts : 1;
+  l.pieces = pieces_of(B * H, N);
+  l.ctas = l.pieces.first + (N > kSlab ? (kParts - 1) * l.pieces.others : 0);
   l.part = align_up((size_t)B * H * N * kD * sizeof(float), 256);
   l.part2 = N > kSlab ? align_up((size_t)B * H * (N - kSlab) * kD * sizeof(float), 256) : 0;
-  const size_t planes = l.parts > 1 ? 2 : 1;
+  l.low = l.pieces.first > 1 ? align_up((size_t)B * H * (N < kSlab ? N : kSlab) * kD * sizeof(float), 256) : 0;
+  const size_t planes = N > kSlab ? 1 + l.pieces.others : 1;
   size_t off = simplicial_schedule_layout(B, &l.info, &l.order);
   auto take = [&off](size_t bytes) {
     const size_t at = off;
@@ -820,11 +881,13 @@ RowsBwdLayout rows_bwd_layout(int B, int H, int N) {
     return at;
   };
   l.delta = take(align_up((size_t)B * H * N * sizeof(float), 256));
-  l.dq = take(l.part * l.parts);
+  l.dq = take(l.part * l.ctas);
   l.dk1 = take(l.part * planes);
   l.dv1 = take(l.part * planes);
   l.dk2 = take(l.part2 * 2);
   l.dv2 = take(l.part2 * 2);
+  l.dk2_low = take(l.low * l.pieces.first);
+  l.dv2_low = take(l.low * l.pieces.first);
   l.total = off;
   return l;
 }
@@ -866,29 +929,34 @@ int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   p.dv1_part = reinterpret_cast<float*>(ws + l.dv1);
   p.dk2_part = reinterpret_cast<float*>(ws + l.dk2);
   p.dv2_part = reinterpret_cast<float*>(ws + l.dv2);
+  p.dk2_low = reinterpret_cast<float*>(ws + l.dk2_low);
+  p.dv2_low = reinterpret_cast<float*>(ws + l.dv2_low);
+  p.pieces = l.pieces.first, p.pieces12 = l.pieces.others;
   p.H = a.heads;
   p.N = a.tokens;
   p.BH = BH;
   p.part_stride = l.part / sizeof(float);
   p.part2_stride = l.part2 / sizeof(float);
+  p.low_stride = l.low / sizeof(float);
 
   int rc = launch_schedule(a.query_valid, a.pair_key_valid, a.batch, a.tokens, info, order, p.status, stream);
   if (rc != MF_OK) return rc;
   const int rows = BH * a.tokens;
-  delta_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p.grad_out, a.out, delta, rows);
+  launch_dependent(delta_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, p.grad_out, a.out, delta, rows);
   MF_CHECK_LAUNCH("delta_rows_kernel");
+  auto kernel = a.tokens > kSlab ? simplicial_rows_bwd_kernel<true> : simplicial_rows_bwd_kernel<false>;
   {
-    cudaError_t e = cudaFuncSetAttribute(simplicial_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_rows_bwd_kernel)");
   }
-  const long long blocks = (long long)BH * l.parts;
+  const long long blocks = (long long)BH * l.ctas;
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
-  simplicial_rows_bwd_kernel<<<(unsigned)blocks, kBwdThreads, kSmemAlloc, stream>>>(p);
+  launch_dependent(kernel, dim3((unsigned)blocks), dim3(kBwdThreads), kSmemAlloc, stream, p);
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, false, stream);
   MF_CHECK_LAUNCH("simplicial_rows_bwd_kernel");
   const long long total4 = (long long)rows * (kD / 4);
-  simplicial_rows_bwd_finalize_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, stream>>>(
-      p, static_cast<__nv_bfloat16*>(a.dq), static_cast<__nv_bfloat16*>(a.dk1), static_cast<__nv_bfloat16*>(a.dv1), BH);
+  launch_dependent(simplicial_rows_bwd_finalize_kernel, dim3((unsigned)((total4 + 255) / 256)), dim3(256), 0, stream, p,
+                   static_cast<__nv_bfloat16*>(a.dq), static_cast<__nv_bfloat16*>(a.dk1), static_cast<__nv_bfloat16*>(a.dv1), BH);
   MF_CHECK_LAUNCH("simplicial_rows_bwd_finalize_kernel");
   return MF_OK;
 }

@@ -39,15 +39,17 @@ constexpr int kColW = 192;
 // one warp per batch element: the last valid key / query index + 1
 __global__ void extent_kernel(const uint8_t* __restrict__ query_valid, const uint8_t* __restrict__ key_valid, int B,
                               int N, BatchInfo* __restrict__ info, int32_t* __restrict__ status) {
+  wait_for_previous();
   if (blockIdx.x == 0 && threadIdx.x < 64) status[threadIdx.x] = 0;  // the 256-byte status block
   const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (b >= B) return;
-  int nk = 0, nq = 0, cnt = 0;
+  int nk = 0, nq = 0, cnt = 0, low = 0;
   for (int t = lane; t < N; t += 32) {
     if (key_valid[(size_t)b * N + t]) {
       nk = t + 1;
       ++cnt;
+      low += t < 128;
     }
     if (query_valid[(size_t)b * N + t]) nq = t + 1;
   }
@@ -56,18 +58,20 @@ __global__ void extent_kernel(const uint8_t* __restrict__ query_valid, const uin
     nk = max(nk, __shfl_xor_sync(0xffffffffu, nk, o));
     nq = max(nq, __shfl_xor_sync(0xffffffffu, nq, o));
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    low += __shfl_xor_sync(0xffffffffu, low, o);
   }
   if (lane == 0) {
     info[b].n_keys = nk;
     info[b].n_queries = nq;
     info[b].reserved0 = cnt;  // number of valid keys
-    info[b].reserved1 = 0;
+    info[b].reserved1 = low;
   }
 }
 
 // rank by cost (descending), ties by index: a stable, deterministic order; one warp per batch element, its lanes
 // striding over the elements it is compared with
 __global__ void order_kernel(const BatchInfo* __restrict__ info, int B, int32_t* __restrict__ order) {
+  wait_for_previous();
   const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (b >= B) return;  // uniform per warp
   auto cost = [&](int i) {
@@ -479,9 +483,9 @@ int cached_max_row_tiles(int tokens) {
 
 int launch_schedule(const uint8_t* query_valid, const uint8_t* key_valid, int B, int N, BatchInfo* info,
                     int32_t* order, int32_t* status, cudaStream_t stream) {
-  extent_kernel<<<(B + 7) / 8, 256, 0, stream>>>(query_valid, key_valid, B, N, info, status);
+  launch_dependent(extent_kernel, dim3((B + 7) / 8), dim3(256), 0, stream, query_valid, key_valid, B, N, info, status);
   MF_CHECK_LAUNCH("extent_kernel");
-  order_kernel<<<(B + 7) / 8, 256, 0, stream>>>(info, B, order);
+  launch_dependent(order_kernel, dim3((B + 7) / 8), dim3(256), 0, stream, info, B, order);
   MF_CHECK_LAUNCH("order_kernel");
   return MF_OK;
 }

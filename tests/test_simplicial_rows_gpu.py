@@ -174,3 +174,27 @@ def test_row_plan_matches_what_the_kernel_does():
     assert torch.equal(o1, out[2:3])
     for n in NAMES:
         assert torch.equal(g1[n], grads[n][2:3])
+
+
+@pytest.mark.parametrize("N,repeats", [(33, (1, 20, 120)), (70, (1, 5, 30)), (130, (1, 8, 60)), (150, (1, 3, 12, 100))])
+def test_walks_in_pieces(N, repeats):
+    """The same four molecules (one without a valid token, one with a single one, holes) in batches of every number of pieces: the
+    oracle's gradients each time, and the same bits for every copy within a batch.  More pieces than walked keys, pieces of one key."""
+    inp, go = _case(4, 1, N, seed=N, key_holes=True, query_holes=True, pair_holes=True, lo=N // 3)
+    for m in (inp.query_valid, inp.pair_key_valid):
+        m[1] = False
+        m[2] = torch.arange(N) == 5
+        m[3, N - 1] = True
+    out_ref, g_ref = simplicial_forward_backward(inp, go)
+    allow = bf16_allowance(inp, go, out_ref, g_ref)
+    floor = 1e-2 * max(g.abs().max().item() for g in g_ref.values())
+    for r in repeats:
+        many = SimplicialInputs(**{n: getattr(inp, n).repeat(r, 1, 1, 1) for n in NAMES}, query_valid=inp.query_valid.repeat(r, 1),
+                                pair_key_valid=inp.pair_key_valid.repeat(r, 1), pair_valid=inp.pair_valid.repeat(r, 1, 1))  # fmt: skip
+        _, _, grads = _run(many, go.repeat(r, 1, 1, 1), "auto")
+        for n in NAMES:
+            g = grads[n].view(r, *g_ref[n].shape)
+            assert (g == g[:1]).all(), (r, n)
+            err = _rel(g[0], g_ref[n], floor)
+            assert err <= allow[n], f"{r} d{n}: {err:.3e} > {allow[n]:.3e}"
+            assert g[0, 1].abs().max() == 0
