@@ -35,6 +35,8 @@
 // 64 molecules of 20-181 atoms of 192 tokens, 8 heads: forward 0.85 ms, backward 3.6 ms (mma.sync kernels, query by query and first
 // key by first key: 1.82 and 6.09 ms); 64 full ones of 64 tokens 0.19 and 0.68 ms (0.24 and 0.96).  A single molecule of 181: 0.24
 // and 0.42 ms (0.12, which is why short forward calls stay there, and 1.54).
+#include <algorithm>
+
 #include "common.cuh"
 #include "simplicial.cuh"
 #include "simplicial_rows.cuh"
@@ -83,24 +85,31 @@ constexpr int tri_smem_bytes(int tokens) {
 }
 
 // The split of a molecule into tiles of (x, y) rows, as plan_rows() of simplicial_rows.cuh, but a tile costs kTileCost steps
-// besides its own (loads, the pipeline's first and last step).  It depends on the molecule alone, so that its results do not depend
-// on the batch it is in.  More than five tiles for the sake of fuller rows save nothing: 64 molecules of 20-181 atoms, steps + 5 per tile at most 8 | 6 |
+// besides its own (loads, the pipeline's first and last step).  It depends on the molecule alone, but for `spread`, so that its results
+// do not depend on the batch it is in.  More than five tiles for the sake of fuller rows save nothing: 64 molecules of 20-181 atoms, steps + 5 per tile at most 8 | 6 |
 // 4 | 3 tiles: 60.5 | 60.5 | 61.3 | 63.8 thousand.
-constexpr int kTileCost = 4, kMostTiles = 5;
+// `spread`: in a call of few heads and more than 100 tokens, where tiles of one first key a step (rows of more than 64 x) leave most of the
+// chip idle for as long as the longest of them takes, up to that many tiles are taken for the sake of shorter ones.
+constexpr int kTileCost = 4, kMostTiles = 5, kSpreadTiles = 6;
 struct TriPlan {
   int tiles, rows;
 };
-__device__ inline TriPlan tri_plan(int nx, int ny) {
+__device__ inline TriPlan tri_plan(int nx, int ny, int spread) {
   TriPlan best{0, 0};
-  int best_cost = 0;
+  int best_cost = 0, best_steps = 0;
   if (nx <= 0 || ny <= 0) return best;
 #pragma unroll 1
   for (int t = 1; t <= kMostTiles; ++t) {
     const int rows = (nx + t - 1) / t;
     if (rows > kTileM) continue;
     const int tiles = (nx + rows - 1) / rows, groups = min(kTileM / rows, kMaxGroups);
-    const int cost = tiles * ((ny + groups - 1) / groups + kTileCost);
-    if (best.tiles == 0 || cost < best_cost) best = TriPlan{tiles, rows}, best_cost = cost;
+    const int steps = (ny + groups - 1) / groups, cost = tiles * (steps + kTileCost);
+    if (best.tiles == 0 || cost < best_cost) best = TriPlan{tiles, rows}, best_cost = cost, best_steps = steps;
+  }
+#pragma unroll 1
+  for (int t = best.tiles + 1; t <= spread; ++t) {
+    const int rows = (nx + t - 1) / t, tiles = (nx + rows - 1) / rows, steps = (ny + min(kTileM / rows, kMaxGroups) - 1) / min(kTileM / rows, kMaxGroups);
+    if (steps < best_steps) best = TriPlan{tiles, rows}, best_steps = steps;
   }
   return best;
 }
@@ -829,6 +838,7 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_tri_fwd_kernel(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (an address made from an integer would be a generic one)
   __shared__ TriShared sh;
+  wait_for_previous();
   const int at = blockIdx.x / p.H;
   if (at >= p.items[0].x) return;
   tri_tile<kFwd>(p, sh, smem, p.items[1 + at], blockIdx.x % p.H);
@@ -838,6 +848,7 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_tri_bwd_kernel(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (an address made from an integer would be a generic one)
   __shared__ TriShared sh;
+  wait_for_previous();
   const int at = blockIdx.x / p.H, h = blockIdx.x % p.H;
   if (at >= p.items[0].x) return;
   const int2 item = p.items[1 + at];
@@ -852,8 +863,9 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_tri_bwd_kernel(const __grid_c
 constexpr int kScheduleThreads = 1024;
 __global__ void __launch_bounds__(kScheduleThreads) simplicial_tri_schedule_kernel(const uint8_t* __restrict__ query_valid,
                                                                                   const uint8_t* __restrict__ key_valid, int B, int N,
-                                                                                  int backward, BatchInfo* info, int2* items,
-                                                                                  int32_t* status) {
+                                                                                  int backward, int spread, BatchInfo* info,
+                                                                                  int2* items, int32_t* status) {
+  wait_for_previous();
   __shared__ int start[kMaxKeys + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid < 64) status[tid] = 0;
@@ -861,15 +873,9 @@ __global__ void __launch_bounds__(kScheduleThreads) simplicial_tri_schedule_kern
   __syncthreads();
   auto plan = [&](const BatchInfo& m, int pass) {
     const bool any = m.reserved0 > 0 && m.reserved1 > 0;
-    return tri_plan(pass == kDq || pass == kFwd ? m.n_queries : m.n_keys, any ? pass == kDk2 ? m.reserved1 : m.reserved0 : 0);
+    return tri_plan(pass == kDq || pass == kFwd ? m.n_queries : m.n_keys, any ? pass == kDk2 ? m.reserved1 : m.reserved0 : 0, spread);
   };
   const int first = backward ? kDq : kFwd, last = backward ? kDk2 : kFwd;
-  auto all_tiles = [&](const BatchInfo& m) {  // at least one each: it clears the rows that nothing covers
-    int n = 0;
-#pragma unroll 1
-    for (int pass = first; pass <= last; ++pass) n += max(plan(m, pass).tiles, 1);
-    return n;
-  };
   auto bucket = [&](const BatchInfo& m) { return kMaxKeys - (m.n_keys + m.n_queries) / 2; };
   for (int b = warp; b < B; b += kScheduleThreads / 32) {
     int nk = 0, nq = 0, ck = 0, cq = 0;
@@ -879,31 +885,39 @@ __global__ void __launch_bounds__(kScheduleThreads) simplicial_tri_schedule_kern
     }
     nk = __reduce_max_sync(0xffffffffu, nk), nq = __reduce_max_sync(0xffffffffu, nq);
     ck = __reduce_add_sync(0xffffffffu, ck), cq = __reduce_add_sync(0xffffffffu, cq);
+    const BatchInfo m{nk, nq, ck, cq};
+    const int tiles = __reduce_add_sync(0xffffffffu, first + lane <= last ? max(plan(m, first + lane).tiles, 1) : 0);
     if (lane == 0) {
-      const BatchInfo m{nk, nq, ck, cq};
       info[b] = m;
-      atomicAdd(&start[bucket(m)], all_tiles(m));
+      atomicAdd(&start[bucket(m)], tiles);
     }
   }
   __syncthreads();
-  if (tid == 0) {
-    int at = 0;
-    for (int t = 0; t <= kMaxKeys; ++t) {
-      const int n = start[t];
-      start[t] = at;
-      at += n;
+  if (warp == 0) {  // exclusive sums
+    int before = 0;
+    for (int c = 0; c <= kMaxKeys; c += 32) {
+      const int n = c + lane <= kMaxKeys ? start[c + lane] : 0;
+      int sum = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += x;
+      }
+      if (c + lane <= kMaxKeys) start[c + lane] = before + sum - n;
+      before += __shfl_sync(0xffffffffu, sum, 31);
     }
-    items[0] = make_int2(at, 0);
+    if (lane == 0) items[0] = make_int2(before, 0);
   }
-  __syncthreads();
-  for (int b = tid; b < B; b += kScheduleThreads) {
+  __syncthreads();  // (and each warp reads the extents that it wrote)
+  for (int b = warp; b < B; b += kScheduleThreads / 32) {  // a lane per pass; at least one tile each: it clears the rows that nothing covers
     const BatchInfo m = info[b];
-    int at = 1 + atomicAdd(&start[bucket(m)], all_tiles(m));
-#pragma unroll 1
-    for (int pass = first; pass <= last; ++pass) {
-      const TriPlan pl = plan(m, pass);
-      for (int t = 0; t < max(pl.tiles, 1); ++t) items[at++] = make_int2(b | pass << 16 | t << 20, pl.rows | pl.tiles << 8);
-    }
+    const bool mine = first + lane <= last;
+    const TriPlan pl = mine ? plan(m, first + lane) : TriPlan{0, 0};
+    const int tiles = mine ? max(pl.tiles, 1) : 0, t0 = __shfl_sync(0xffffffffu, tiles, 0), t1 = __shfl_sync(0xffffffffu, tiles, 1);
+    const int all = __reduce_add_sync(0xffffffffu, tiles);
+    int at = lane == 0 ? 1 + atomicAdd(&start[bucket(m)], all) : 0;
+    at = __shfl_sync(0xffffffffu, at, 0) + (lane > 0 ? t0 : 0) + (lane > 1 ? t1 : 0);
+    for (int t = 0; t < tiles; ++t) items[at + t] = make_int2(b | (first + lane) << 16 | t << 20, pl.rows | pl.tiles << 8);
   }
 }
 
@@ -912,6 +926,7 @@ __global__ void __launch_bounds__(256) simplicial_tri_rows_kernel(const __nv_bfl
                                                                  const float* __restrict__ lse, const uint8_t* __restrict__ query_valid,
                                                                  int H, int N, int rows, float* __restrict__ lse2,
                                                                  float* __restrict__ ndelta) {
+  wait_for_previous();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   if (query_valid[(size_t)(row / (H * N)) * N + row % N] == 0) return;
@@ -928,6 +943,7 @@ struct TriClear {
   size_t words[9];
 };
 __global__ void __launch_bounds__(256) simplicial_tri_clear_kernel(const __grid_constant__ TriClear c, const int32_t* __restrict__ status) {
+  wait_for_previous();
   if (*status == 0) return;
 #pragma unroll 1
   for (int t = 0; t < 9; ++t)
@@ -937,13 +953,21 @@ __global__ void __launch_bounds__(256) simplicial_tri_clear_kernel(const __grid_
 
 struct TriLayout {
   size_t info, items, lse2, ndelta, total;
-  int max_items;
+  int max_items, spread;
 };
+// Tiles that each molecule and pass may take for the sake of short ones: as many as about one and a half waves hold.  8 heads, backward,
+// n / 3 to n atoms, us without | with: 101 tokens, 1, 4, 16 molecules 251 | 56, 254 | 95, 278 | 280; 128
+// 340 | 88, 330 | 174, 515 | 440; 181 398 | 215, 642 | 530, 1 589 | 1 493.
+int spread_tiles(int batch, int heads, int tokens, int passes) {
+  const long long items = (long long)batch * heads * passes;
+  return tokens <= 100 || items <= 0 || items >= 222 ? 0 : (int)std::min<long long>(kSpreadTiles, (222 + items - 1) / items);
+}
 TriLayout tri_layout(int batch, int heads, int tokens, bool backward) {
   TriLayout l{};
   size_t off = kStatusBytes;
   l.info = off, off = align_up(off + (size_t)batch * sizeof(BatchInfo), 256);
-  l.max_items = batch * kMostTiles * (backward ? 3 : 1);
+  l.spread = spread_tiles(batch, heads, tokens, backward ? 3 : 1);
+  l.max_items = batch * std::max(kMostTiles, l.spread) * (backward ? 3 : 1);
   l.items = off, off = align_up(off + (1 + (size_t)l.max_items) * sizeof(int2), 256);
   if (backward) {
     const size_t rows = align_up((size_t)batch * heads * tokens * sizeof(float), 256);
@@ -970,14 +994,14 @@ void fill_params(TriParams& p, const Args& a, const TriLayout& l) {
 
 template <typename Kernel>
 int launch_tri(Kernel kernel, const TriParams& p, const TriLayout& l, int batch, bool backward, int which, cudaStream_t stream, const char* name) {
-  simplicial_tri_schedule_kernel<<<1, kScheduleThreads, 0, stream>>>(p.query_valid, p.key_valid, batch, p.N, backward,
-                                                                     const_cast<BatchInfo*>(p.info), const_cast<int2*>(p.items), p.status);
+  launch_dependent(simplicial_tri_schedule_kernel, dim3(1), dim3(kScheduleThreads), 0, stream, p.query_valid, p.key_valid, batch, p.N,
+                   backward, l.spread, const_cast<BatchInfo*>(p.info), const_cast<int2*>(p.items), p.status);
   MF_CHECK_LAUNCH("simplicial_tri_schedule_kernel");
   // (the limit is one for all sizes: another host thread must not lower it between here and the launch)
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes(kMaxKeys));
   if (e != cudaSuccess) return cuda_error(e, name);
   profile_mark(which, true, stream);
-  kernel<<<(unsigned)l.max_items * p.H, kTriThreads, tri_smem_bytes(p.N), stream>>>(p);
+  launch_dependent(kernel, dim3((unsigned)l.max_items * p.H), dim3(kTriThreads), tri_smem_bytes(p.N), stream, p);
   profile_mark(which, false, stream);
   MF_CHECK_LAUNCH(name);
   return MF_OK;
@@ -1014,7 +1038,8 @@ int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, Bounde
   p.grad_other[1] = static_cast<__nv_bfloat16*>(a.dv1), p.grad_other[2] = static_cast<__nv_bfloat16*>(a.dv2);
   p.du = a.du, p.dv_bias = a.dv_bias, p.dw = a.dw, p.dgate = a.dgate;
   const int rows = a.batch * a.heads * a.tokens;
-  simplicial_tri_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p.other[0], a.out, a.lse, a.query_valid, a.heads, a.tokens, rows, lse2, ndelta);
+  launch_dependent(simplicial_tri_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, p.other[0], a.out, a.lse, a.query_valid, a.heads,
+                   a.tokens, rows, lse2, ndelta);
   MF_CHECK_LAUNCH("simplicial_tri_rows_kernel");
   const int rc = launch_tri(simplicial_tri_bwd_kernel, p, l, a.batch, true, MF_PROFILE_SIMPLICIAL_BWD, stream, "simplicial_tri_bwd_kernel");
   if (rc != MF_OK) return rc;
@@ -1022,7 +1047,7 @@ int simplicial_tri_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream, Bounde
   void* grads[9] = {a.dq, a.dk1, a.dv1, a.dk2, a.dv2, a.du, a.dv_bias, a.dw, a.dgate};
   TriClear c{};
   for (int t = 0; t < 9; ++t) c.at[t] = static_cast<uint32_t*>(grads[t]), c.words[t] = t < 5 ? n * (kD / 2) : t < 8 ? n * a.tokens : n;
-  simplicial_tri_clear_kernel<<<148, 256, 0, stream>>>(c, p.status);
+  launch_dependent(simplicial_tri_clear_kernel, dim3(148), dim3(256), 0, stream, c, p.status);
   MF_CHECK_LAUNCH("simplicial_tri_clear_kernel");
   return MF_OK;
 }

@@ -164,3 +164,24 @@ def test_forward_without_workspace(monkeypatch):
         *(getattr(inp, n).bfloat16().cuda() for n in NAMES), query_valid=inp.query_valid.cuda(), pair_key_valid=inp.pair_key_valid.cuda(),
         pair_valid=None, **{n: getattr(inp, n).cuda() for n in BIAS_NAMES})  # fmt: skip
     assert_rel(out.float().cpu(), out_ref, 2e-2, "out")
+
+
+@pytest.mark.parametrize("B,H,N", [(1, 1, 101), (2, 9, 128), (6, 8, 140), (13, 8, 110), (28, 8, 103)])
+def test_spread_tiles_against_oracle(B, H, N):
+    """Six tiles, fewer and none besides the usual ones, forward on either side of its line: molecules of 1, 65, 101 and N atoms (the others
+    repeat them), against the oracle."""
+    inp, go = _case(4, H, N, seed=N, scale=0.5, lo=1)
+    for i, n in enumerate((N, 101, 65, 1)):
+        inp.query_valid[i] = inp.pair_key_valid[i] = torch.arange(N) < n
+    _with_bias(inp, N)
+    out_ref, g_ref = simplicial_forward_backward(inp, go)
+    pick = torch.arange(B) % 4
+    t = {n: getattr(inp, n)[pick].cuda() for n in (*NAMES, *BIAS_NAMES)}
+    t.update({n: t[n].bfloat16() for n in NAMES})
+    _, _, y, *grads = (x.float().cpu() for x in _run(t, inp.query_valid[pick].cuda(), go[pick].cuda().bfloat16()))
+    keep = min(B, 4)
+    assert_rel(y[:keep], out_ref[:keep], 2e-2, "out")
+    for n, got in zip(NAMES + BIAS_NAMES, grads):
+        assert_rel(got[:keep], g_ref[n][:keep], 2.5e-2, f"d{n}")
+        if B > 4:
+            assert torch.equal(got[4:8], got[: min(4, B - 4)])
