@@ -111,19 +111,20 @@ template <typename Args>
 bool uses_tri_kernels(const Args* a) {
   return a->tokens > kSmallTokens && has_factorized_bias(a);
 }
-// The forward pass runs on them where a call is long enough.  A tile walks all first keys of its rows whatever the batch, in at most 26
-// steps up to 100 tokens and, where few molecules leave room for more tiles (spread_tiles), in at most 50 above; the warp-level kernel
-// spreads the queries of a small batch over the chip.  The host does not know how full the batch is, so the lines lie between the two
-// extremes.  8 heads, us, trilinear | warp-level, all molecules full; sizes spread (from an eighth of the tokens up at 64 and 96,
-// from a third above): 64 tokens x 4 molecules 53 | 32; 53 | 17, x 16 54 | 77; 54 | 43, x 32 98 | 136; 57 | 92.  96 x 4 54 | 60; 54 | 31,
-// x 12 99 | 150; 60 | 87.  101 x 1 44 | 45; 44 | 45, x 4 80 | 91; 44 | 46.  128 x 1 65 | 50; 65 | 50, x 2 66 | 97; 65 | 51, x 4 121 | 145;
-// 66 | 82, x 8 146 | 252; 80 | 156.  160 x 1 104 | 76; 105 | 76, x 2 107 | 150; 106 | 88, x 4 200 | 268; 108 | 133.  192 x 1 136 | 106, x 2
-// 139 | 207; 138 | 122.  On either side a molecule's result does not depend on its batch but for the tiles it is spread over; the two
-// sides round differently, with the same error.  MF_BACKEND_TCGEN05_TILES stays on one side.
+// The forward pass runs on them where a call is long enough.  A tile walks all first keys of its rows whatever the batch, up to 100
+// tokens in at most 26 steps, from 101 on in up to 128 (tri_plan); the warp-level kernel spreads the queries of a small batch over
+// the chip.  The host does not know how full the batch is, so the lines lie between the two extremes.  8 heads, us, trilinear |
+// warp-level, all molecules full | spread from an eighth of the tokens up: 64 tokens x 4 molecules 53 | 32, 53 | 17; x 16 54 | 77,
+// 54 | 43; x 32 98 | 136, 57 | 92.  96 x 4 54 | 60, 54 | 31; x 12 99 | 150, 60 | 87.  128 x 4 254 | 143, 249 | 68; x 12 255 | 334,
+// 250 | 159; x 32 492 | 892, 255 | 364.  192 x 1 257 | 103; x 6 259 | 557, 257 | 257; x 32 1 479 | 2 814, 580 | 1 078.  On either
+// side a molecule's result does not depend on its batch; the two sides round differently, with the same error.
+// MF_BACKEND_TCGEN05_TILES stays on one side.  (Measured before calls of few molecules were spread over more tiles, see spread_tiles;
+// with that the trilinear kernel wins above 100 tokens from two to four molecules on: 128 x 4 121 | 145 full, 66 | 82 spread, x 8 146 |
+// 252, 80 | 156.  The lines are kept: moving them changes which kernel, and which rounding, a call gets.)
 inline bool uses_tri_forward(const MfSimplicialFwdArgs* a) {
   if (!uses_tri_kernels(a)) return false;
   const double heads = (double)a->batch * a->heads, n = a->tokens;
-  return a->backend == MF_BACKEND_TCGEN05_TILES || (n <= 100 ? heads * n >= 6144 : heads >= 16);
+  return a->backend == MF_BACKEND_TCGEN05_TILES || (n <= 100 ? heads * n >= 6144 : heads * n * n * n >= 150e6);
 }
 // Without the bias the forward pass runs on the warp-level kernel, unless a tcgen05 family is asked for: 64 molecules of 20-181 atoms
 // take 0.64 ms on the trilinear kernel against 0.89, but 2 molecules 201 us against 105, and a molecule's result is to be the same in
