@@ -19,8 +19,8 @@ import torch
 
 
 def simplicial_tile_steps(num_atoms: int) -> int:
-    """Bound on the tile-steps of the backward kernel for one molecule and one head, exact up to 128 atoms (above, the kernel takes a
-    sixth to a half fewer; the forward needs at most as many)."""
+    """Tile-steps of the backward kernel for one molecule and one head (the forward needs at most as many) in a batch that fills the chip.
+    A small batch walks a molecule in several pieces, whose steps are rounded up one by one."""
     from . import _lib
 
     if num_atoms <= 0:

@@ -2,8 +2,7 @@
 //
 // One CTA owns one (batch, head) and a slab of at most 128 keys of the second key set (index k).  Every row
 // of its 128-row tile carries its own (query i, first key j) pair (see simplicial_rows.cuh); the CTA walks over
-// all query ranges of the molecule and, inside a range, over groups of first keys.  Molecules of more than 128 keys
-// are cut into three such parts, two of them with the key sets exchanged (see Part).  Per step, with
+// all query ranges of the molecule and, inside a range, over groups of first keys.  Per step, with
 //   A1[r,:] = q[i_r,:] o k1[j_r,:]   and   A2[r,:] = dO[i_r,:] o v1[j_r,:]     (rewritten into shared memory)
 // seven GEMMs run on tcgen05 with fp32 accumulators in tensor memory:
 //   S   = A1 . K2^T            logits (recomputed)
@@ -19,10 +18,17 @@
 // memory as bf16 and a GEMM against a 0/1 selector sums the rows of each group (M = 128 output columns,
 // N = 16 groups, K = 128 rows), so the column sums of a step cost one narrow MMA instead of a shuffle tree.
 //
-// Small batches walk in several pieces per part (see Pieces).  dK2 / dV2 of the first 128 keys leave the CTA as final bf16 rows where
-// one piece walks them all (no other CTA contributes to them).  Everything else is written as fp32 partials and summed in a fixed order by the finalize kernel; within a CTA dk1 / dv1
-// partials are accumulated over the query ranges by plain read-modify-write of addresses only this CTA
-// touches.  There are no floating-point atomics: gradients are bit-identical from run to run.
+// Small batches walk a slab in several pieces, a CTA each (see pieces_of).  Where there is one, dK2 / dV2 leave the CTA as final bf16
+// rows (no other CTA contributes to them).  dq and dk1 / dv1, and dK2 / dV2 of several pieces, are written as fp32 partials and summed
+// in a fixed order by the finalize kernel; within a CTA dk1 / dv1 partials are accumulated over the query ranges by plain
+// read-modify-write of addresses only this CTA touches.  There are no floating-point atomics: gradients are bit-identical from run to
+// run.
+//
+// Both slabs of a molecule of more than 128 keys walk all its first keys, n steps' worth each.  Exchanging the key sets for the second
+// keys from 128 on would take n + 2 (n - 128) instead of 2 n (64 molecules of 20-181 atoms, 8 heads: 1 620 us against 1 929), but
+// their dK2 and dV2 would be sums of products rounded to bf16 (3.7e-3 and 3.4e-3 from the exact ones against 3.3e-3 and 2.9e-3 at 181
+// atoms), and their probabilities, from q o k2 instead of the q o k1 that lse is formed from, would not add up to 1: with logits of a
+// standard deviation of 8, 3.7e-2 and 3.8e-2 against 2.4e-2 and 1.0e-2.
 //
 // Threads: 384.  Warps 0-3 hold the q rows (build A1, drain U), warps 4-7 the dO rows (build A2, drain W); both
 // form P and dS, each on every other 32-column chunk; one thread of warp 8 issues every tcgen05.mma; warp 9
@@ -83,69 +89,51 @@ struct RowsBwdParams {
   const uint8_t* query_valid;
   const uint8_t* key_valid;
   const uint8_t* pair_valid;
-  __nv_bfloat16* dk2;  // keys [0, 128): final where part 0 is one piece
+  __nv_bfloat16* dk2;  // final where a slab is walked in one piece
   __nv_bfloat16* dv2;
-  float* dq_part;      // a plane of (BH, N, 64) fp32 for each piece of each part
-  float* dk1_part;     // planes: part 0; the pieces of parts 1 and 2
+  float* dq_part;      // a plane of (BH, N, 64) fp32 for each piece of each slab
+  float* dk1_part;     // a plane for each slab
   float* dv1_part;
-  float* dk2_low;      // pieces of part 0 (where there are several): planes of (BH, min(N, 128), 64)
-  float* dv2_low;
-  float* dk2_part;     // parts 1 and 2: planes of (BH, N - 128, 64) for the keys from 128 on
+  float* dk2_part;     // a plane for each piece, where there are several
   float* dv2_part;
   const BatchInfo* info;
   const int32_t* order;
   int32_t* status;
-  int H, N, BH;
-  size_t part_stride, part2_stride, low_stride;  // elements per plane
-  int pieces, pieces12;                          // of part 0; of parts 1 and 2
+  int H, N, slabs_max, pieces;
+  size_t part_stride;  // elements per plane
   int use_tma;
-  CUtensorMap tm_k[2];   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle: second keys, first keys
-  CUtensorMap tm_v[2];
+  CUtensorMap tm_k2;   // (B*H, N, 64) bf16, boxes of 32 rows, 128-byte swizzle
+  CUtensorMap tm_v2;
 };
 
-// Parts of a molecule.  Part 0 has the first 128 second keys as columns and walks every first key.  The pairs left, those of the
-// second keys from 128 on, are walked by these instead: the logits are symmetric in the two key sets, so parts 1 and 2 exchange
-// them, with the first keys as columns (128 and the rest).  A molecule of n > 128 atoms takes n + 2 (n - 128) first keys' worth of
-// steps (the last n - 128 of them at most 64 columns wide); two slabs of its second keys, each walking all first keys, took 2 n.
-// 64 molecules of 20-181 atoms, 8 heads: 1 929 -> 1 620 us.
-constexpr int kParts = 3;
-struct Part {
-  bool exchanged;
-  int col0, cols;  // keys that are columns
-  int walk0;       // first key walked
-};
-__device__ __forceinline__ Part part_of(int index, int n_keys) {
-  if (index == 0) return Part{false, 0, min(n_keys, kSlab), 0};
-  if (n_keys <= kSlab) return Part{true, 0, 0, 0};
-  return index == 1 ? Part{true, 0, kSlab, kSlab} : Part{true, kSlab, n_keys - kSlab, kSlab};
+// Key slabs of a molecule: equal widths, multiples of 32 so that mask words line up with 32-column chunks.
+__host__ __device__ inline int slab_count(int n_keys) { return (n_keys + kSlab - 1) / kSlab; }
+__host__ __device__ inline int slab_width(int n_keys) {
+  const int s = slab_count(n_keys);
+  return s > 0 ? (((n_keys + s - 1) / s + 31) & ~31) : 0;
 }
 
-// A part walks its first keys in one piece where the molecules fill the chip several times over, and in several, a CTA each, where they
-// do not: a CTA by itself takes the walk's full length however few others there are, and the largest molecule of a batch decides.
-// A piece costs its set-up and fp32 planes for the sums that run over the walk.
-struct Pieces {
-  int first, others;  // of part 0; of parts 1 and 2, by the share of the keys that they walk
-};
+// A slab's walk goes in one piece where the molecules fill the chip several times over, and in several, a CTA each, where they do not: a
+// CTA by itself takes the walk's full length however few others there are, and the largest molecule of a batch decides.  A piece
+// costs its set-up and fp32 planes for the sums that run over the walk.
 // The number with the shortest estimate: the longer of one piece (the largest molecule: kPieceUs for its set-up and the beginnings and
 // ends of its query ranges, and its share of a walk of kWalkUs N^2, both from measured times) and all of them on kSms SMs, the batch at
 // half of its largest molecule's work (sizes spread from an eighth up 0.38, all full 1; the host does not know).  A molecule or two
 // cannot fill a second wave with small pieces: it counts by itself.  Powers of two, so that batches near each other share a number: on
-// one side of a line a molecule's bits do not depend on its batch.  8 heads, n / 3 to n atoms, the kernel in us, one piece | this:
-// 40 tokens, 1, 4, 16 molecules 51 | 17, 51 | 25, 52 | 52; 96 235 | 47, 235 | 71, 241 | 146; 128 401 | 43, 401 | 110, 408 | 235; 181 (three
-// parts in one piece each 880) 163, 295, 671.
-inline Pieces pieces_of(int BH, int N) {
+// one side of a line a molecule's bits do not depend on its batch.
+inline int pieces_of(int BH, int N) {
   constexpr float kPieceUs = 30.f, kWalkUs = 0.0245f, kShare = 0.5f, kSms = 148.f;
-  const float walk = kWalkUs * N * N, rest = N > kSlab ? walk * (N - kSlab) / N : 0.f;
-  Pieces best{1, 1};
+  const int slabs = slab_count(N);
+  const float walk = kWalkUs * N * N;
+  int best = 1;
   float least = INFINITY;
   for (int pieces = 1; pieces <= 16; pieces *= 2) {
-    const int others = N > kSlab ? std::max(1, (int)(pieces * (N - kSlab) / (float)N + 0.5f)) : 0;
-    const float all = BH * ((pieces + 2 * others) * kPieceUs + kShare * (walk + 2.f * rest)) / kSms;
+    const float all = BH * slabs * (pieces * kPieceUs + kShare * walk) / kSms;
     float piece = kPieceUs + walk / pieces;
-    const int waves = (BH * (pieces + 2 * others) + (int)kSms - 1) / (int)kSms;
-    if (BH <= 16 && waves > 1) piece *= waves * (N > kSlab ? 0.78f : 0.6f);
+    const int waves = (BH * slabs * pieces + (int)kSms - 1) / (int)kSms;
+    if (BH <= 16 && waves > 1) piece *= 0.6f * waves;
     const float time = std::max(piece, all);
-    if (time < 0.97f * least) least = time, best = Pieces{pieces, std::max(1, others)};
+    if (time < 0.97f * least) least = time, best = pieces;
   }
   return best;
 }
@@ -173,8 +161,6 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// kParted: the batch has room for molecules of more than 128 keys.
-template <bool kParted>
 __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constant__ RowsBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -191,26 +177,23 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
   const bool is_worker = tid < 256;
   const int grp = (tid >> 7) & 1;  // 0: q side, 1: dO side
   const int r = tid & 127;         // row of the tile
-  // heavy molecules first, and of all molecules part 0 (the longest) before the others
-  const int rest = kParted ? (int)blockIdx.x - p.BH * p.pieces : -1;
-  const int part = rest < 0 ? 0 : 1 + (rest & 1), pieces = rest < 0 ? p.pieces : p.pieces12;
-  const int at = rest < 0 ? (int)blockIdx.x : rest >> 1, item = at / pieces, piece = at - item * pieces;
-  const int b = p.order[item / p.H], h = item % p.H;
+  const int per_b = p.H * p.slabs_max * p.pieces;
+  const int b = p.order[blockIdx.x / per_b];
+  const int rem = blockIdx.x % per_b;
+  const int h = rem / (p.slabs_max * p.pieces), slab = rem / p.pieces % p.slabs_max, piece = rem % p.pieces;
   const int N = p.N;
   const int bh = b * p.H + h;
   const size_t base = (size_t)bh * N * kD;
   const int n_keys = p.info[b].n_keys;
   const int n_queries = p.info[b].n_queries;
-  const Part own = kParted ? part_of(part, n_keys) : Part{false, 0, n_keys, 0};
-  const int k0 = own.col0, nk_slab = own.cols;  // columns: keys [k0, k0 + nk_slab) of the one set
-  if (nk_slab <= 0) return;                     // the finalize kernel writes the zeros
-  // keys of the other set that are walked: this piece of the valid ones from walk0 on
-  const int skipped = own.walk0 > 0 ? p.info[b].reserved1 : 0, walked = p.info[b].reserved0 - skipped, each = piece_keys(walked, pieces);
-  const int before = skipped + piece * each, nj = min(each, walked - piece * each);
+  // first keys that are walked: this piece of the valid ones
+  const int valid = p.info[b].reserved0, each = piece_keys(valid, p.pieces), before = piece * each, nj = min(each, valid - before);
   const RowPlan plan = plan_rows(n_queries, nj);
-  if (plan.tiles == 0) return;
-  const __nv_bfloat16 *walk_k = own.exchanged ? p.k2 : p.k1, *walk_v = own.exchanged ? p.v2 : p.v1;
-  const __nv_bfloat16 *col_k = own.exchanged ? p.k1 : p.k2, *col_v = own.exchanged ? p.v1 : p.v2;
+  if (plan.tiles == 0 || slab >= slab_count(n_keys)) return;  // the finalize kernel writes the zeros
+  const int slab_w = slab_width(n_keys);
+  const int k0 = slab * slab_w;                     // first key of the slab (multiple of 32)
+  const int nk_slab = min(slab_w, n_keys - k0);     // keys in the slab
+  if (nk_slab <= 0) return;
   // MMA N of the logit GEMMs: whole 32-column chunks, so that every column a worker reads has been written (keys
   // beyond the slab's last have zero K2 / V2 rows)
   const int nk_pad = (nk_slab + 31) & ~31;
@@ -245,7 +228,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
     kmask[tid] = w;
   }
   __syncthreads();
-  if (tid < kMaxKeys && ((kmask[tid >> 5] >> (tid & 31)) & 1u)) {  // compacted list of the valid keys that are walked
+  if (tid < kMaxKeys && ((kmask[tid >> 5] >> (tid & 31)) & 1u)) {  // compacted list of the valid first keys that are walked
     int pos = __popc(kmask[tid >> 5] & ((1u << (tid & 31)) - 1u));
     for (int c = 0; c < (tid >> 5); ++c) pos += __popc(kmask[c]);
     if (pos >= before && pos < before + nj) jlist[pos - before] = (uint8_t)tid;
@@ -264,7 +247,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         w = 0;
         for (int e = 0; e < 32; ++e) {
           const int k = c * 32 + e;
-          if (k < n_keys && pv[own.exchanged ? (size_t)k * N + j : (size_t)j * N + k] > 0) w |= 1u << e;
+          if (k < n_keys && pv[(size_t)j * N + k] > 0) w |= 1u << e;
         }
       }
       pvbits_w[idx] = w;
@@ -275,8 +258,8 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
       if (tid == 0) {
         mbar_arrive_expect_tx(&bar_kv, (uint32_t)(kSlab / kTmaBoxRows) * 2u * kTmaBoxRows * 128u);
         for (int c = 0; c < kSlab / kTmaBoxRows; ++c) {
-          tma_load_rows(smem + kOffK2 + c * kTmaBoxRows * 128, &p.tm_k[own.exchanged], k0 + c * kTmaBoxRows, bh, &bar_kv);
-          tma_load_rows(smem + kOffV2 + c * kTmaBoxRows * 128, &p.tm_v[own.exchanged], k0 + c * kTmaBoxRows, bh, &bar_kv);
+          tma_load_rows(smem + kOffK2 + c * kTmaBoxRows * 128, &p.tm_k2, k0 + c * kTmaBoxRows, bh, &bar_kv);
+          tma_load_rows(smem + kOffV2 + c * kTmaBoxRows * 128, &p.tm_v2, k0 + c * kTmaBoxRows, bh, &bar_kv);
         }
       }
     } else {
@@ -284,8 +267,8 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         const int rr = idx >> 3, c = idx & 7;
         uint4 vk = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
         if (key_live(rr)) {
-          vk = __ldg(reinterpret_cast<const uint4*>(col_k + base + (size_t)(k0 + rr) * kD) + c);
-          vv = __ldg(reinterpret_cast<const uint4*>(col_v + base + (size_t)(k0 + rr) * kD) + c);
+          vk = __ldg(reinterpret_cast<const uint4*>(p.k2 + base + (size_t)(k0 + rr) * kD) + c);
+          vv = __ldg(reinterpret_cast<const uint4*>(p.v2 + base + (size_t)(k0 + rr) * kD) + c);
         }
         const uint32_t off = rr * 128 + ((c ^ (rr & 7)) << 4);
         *reinterpret_cast<uint4*>(smem + kOffK2 + off) = vk;
@@ -449,7 +432,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
           const int jj = s * G + gg;
           v[q] = make_uint4(0, 0, 0, 0);
           if (gg < G && jj < nj)
-            v[q] = __ldg(reinterpret_cast<const uint4*>((which == 0 ? walk_k : walk_v) + base + (size_t)jlist[jj] * kD) + part);
+            v[q] = __ldg(reinterpret_cast<const uint4*>((which == 0 ? p.k1 : p.v1) + base + (size_t)jlist[jj] * kD) + part);
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -492,10 +475,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
     const bool live_x = warp_live && 32 * grp < nk_x;
     const bool live_y = warp_live && 32 * grp < nk_y;
     // partial column sums of this thread's output column (readers: the 128 threads of the q side)
-    float* part_col = (own.exchanged ? (r < 64 ? p.dk2_part : p.dv2_part) + (size_t)(part - 1) * p.part2_stride +
-                                           (long long)bh * (N - kSlab) * kD - kSlab * kD
-                                     : (r < 64 ? p.dk1_part : p.dv1_part) + base) +
-                      (r & 63);
+    float* part_col = (r < 64 ? p.dk1_part : p.dv1_part) + (size_t)slab * p.part_stride + base + (r & 63);
 
     uint32_t xreg[32];
     float dq_acc[32];  // dq columns [32 grp, 32 grp + 32) of this thread's row: the two groups share the accumulation
@@ -704,8 +684,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
       // ---- end of the range: last column sums, then dq of the range (rows of one query summed over the groups)
       prefetch_sums(t, steps - 1);
       commit_sums(steps - 1);  // also: every product issued so far has completed
-      const int plane = part == 0 ? piece : p.pieces + (part - 1) * p.pieces12 + piece;
-      float* dq_dst = p.dq_part + (size_t)plane * p.part_stride + base;
+      float* dq_dst = p.dq_part + (size_t)(slab * p.pieces + piece) * p.part_stride + base;
       if (G == 1) {
         if (slot_ok && i < n_queries) {
           float4* dst = reinterpret_cast<float4*>(dq_dst + (size_t)i * kD + 32 * grp);
@@ -743,15 +722,12 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         named_barrier(1, 256);  // the next range's operands overwrite the staging area
       }
     }
-    // ---- epilogue: accumulators: lane r of tensor memory = key k0 + r; group 0 stores dK2, group 1 dV2 (of exchanged key
-    // sets: partial dK1 and dV1)
+    // ---- epilogue: accumulators: lane r of tensor memory = key k0 + r; group 0 stores dK2, group 1 dV2
     wait_on(&bar_fin, 0);
     tc_fence_after_sync();
     {
       __nv_bfloat16* dst = (grp == 0 ? p.dk2 : p.dv2) + base + (size_t)(k0 + r) * kD;
-      const bool partial = own.exchanged || p.pieces > 1;
-      float* dst32 = own.exchanged ? (grp == 0 ? p.dk1_part : p.dv1_part) + (1 + piece) * p.part_stride + base + (size_t)(k0 + r) * kD
-                                   : (grp == 0 ? p.dk2_low : p.dv2_low) + piece * p.low_stride + ((size_t)bh * min(N, kSlab) + r) * kD;
+      float* dst32 = (grp == 0 ? p.dk2_part : p.dv2_part) + (size_t)piece * p.part_stride + base + (size_t)(k0 + r) * kD;
       const bool store = !bad && r < nk_slab;
       const bool live = key_live(r);
 #pragma unroll
@@ -759,7 +735,7 @@ __global__ void __maxnreg__(168) simplicial_rows_bwd_kernel(const __grid_constan
         uint32_t w[32];
         tmem_ld32(tmem_row + (grp == 0 ? kColDK2 : kColDV2) + 32 * half, w);  // whole warps: the load is warp-wide
         tmem_ld_wait();
-        if (store && partial) {
+        if (store && p.pieces > 1) {
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             reinterpret_cast<uint4*>(dst32 + 32 * half)[c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
@@ -806,9 +782,7 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
   const int n_keys = p.info[b].n_keys, n_queries = p.info[b].n_queries, nj = p.info[b].reserved0;
   const bool failed = p.status[0] != 0;
   const bool active = n_queries > 0 && nj > 0 && !failed;
-  const bool parted = n_keys > kSlab;
-  const int used = p.pieces > 1 ? pieces_used(nj, p.pieces) : 1;
-  const int used12 = !parted ? 0 : p.pieces12 > 1 ? pieces_used(nj - p.info[b].reserved1, p.pieces12) : 1;
+  const int nsl = slab_count(n_keys), used = p.pieces > 1 ? pieces_used(nj, p.pieces) : 1;
   const size_t off = ((size_t)bh * p.N + row) * kD + 4 * d4;
   const bool q_ok = active && row < n_queries && p.query_valid[(size_t)b * p.N + row] > 0;
   const bool k_ok = active && row < n_keys && p.key_valid[(size_t)b * p.N + row] > 0;
@@ -825,34 +799,24 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
     *reinterpret_cast<uint2*>(dst) = o;
   };
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (q_ok) {
-    auto plane = [&](int s) { add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)s * p.part_stride + off)); };
-    for (int s = 0; s < used; ++s) plane(s);
-    for (int part = 0; part < 2; ++part)
-      for (int s = 0; s < used12; ++s) plane(p.pieces + part * p.pieces12 + s);
-  }
+  if (q_ok)
+    for (int s = 0; s < nsl; ++s)
+      for (int t = 0; t < used; ++t) add4(a, *reinterpret_cast<const float4*>(p.dq_part + (size_t)(s * p.pieces + t) * p.part_stride + off));
   store4(dq + off, a);
   float4 k1v = make_float4(0.f, 0.f, 0.f, 0.f), v1v = k1v;
   if (k_ok)
-    for (int s = 0; s < 1 + used12; ++s) {
+    for (int s = 0; s < nsl; ++s) {
       add4(k1v, *reinterpret_cast<const float4*>(p.dk1_part + (size_t)s * p.part_stride + off));
       add4(v1v, *reinterpret_cast<const float4*>(p.dv1_part + (size_t)s * p.part_stride + off));
     }
   store4(dk1 + off, k1v);
   store4(dv1 + off, v1v);
-  if (row >= kSlab || p.pieces > 1 || !(active && row < n_keys)) {  // (the others were stored by part 0)
+  if (p.pieces > 1 || !(active && row < n_keys)) {  // (the others were stored by their slab)
     float4 k2v = make_float4(0.f, 0.f, 0.f, 0.f), v2v = k2v;
-    if (k_ok && row < kSlab)
-      for (int s = 0; s < used; ++s) {
-        const size_t low = s * p.low_stride + ((size_t)bh * min(p.N, kSlab) + row) * kD + 4 * d4;
-        add4(k2v, *reinterpret_cast<const float4*>(p.dk2_low + low));
-        add4(v2v, *reinterpret_cast<const float4*>(p.dv2_low + low));
-      }
-    else if (k_ok)
-      for (int s = 0; s < 2; ++s) {
-        const size_t off2 = (size_t)s * p.part2_stride + ((size_t)bh * (p.N - kSlab) + row - kSlab) * kD + 4 * d4;
-        add4(k2v, *reinterpret_cast<const float4*>(p.dk2_part + off2));
-        add4(v2v, *reinterpret_cast<const float4*>(p.dv2_part + off2));
+    if (k_ok)
+      for (int t = 0; t < used; ++t) {
+        add4(k2v, *reinterpret_cast<const float4*>(p.dk2_part + (size_t)t * p.part_stride + off));
+        add4(v2v, *reinterpret_cast<const float4*>(p.dv2_part + (size_t)t * p.part_stride + off));
       }
     store4(p.dk2 + off, k2v);
     store4(p.dv2 + off, v2v);
@@ -860,20 +824,16 @@ __global__ void simplicial_rows_bwd_finalize_kernel(RowsBwdParams p, __nv_bfloat
 }
 
 struct RowsBwdLayout {
-  size_t info, order, delta, dq, dk1, dv1, dk2, dv2, dk2_low, dv2_low, total;
-  Pieces pieces;
-  int ctas;                 // per (batch, head): one for each piece of each part
-  size_t part, part2, low;  // bytes per partial plane
+  size_t info, order, delta, dq, dk1, dv1, dk2, dv2, total;
+  int slabs_max, pieces;
+  size_t part;  // bytes per partial plane
 };
 
-RowsBwdLayout rows_bwd_layout(int B, int H, int N) {
+RowsBwdLayout rows_bwd_layout(int B, int H, int N, int pieces) {
   RowsBwdLayout l{};
-  l.pieces = pieces_of(B * H, N);
-  l.ctas = l.pieces.first + (N > kSlab ? (kParts - 1) * l.pieces.others : 0);
+  l.slabs_max = slab_count(N);
+  l.pieces = pieces;
   l.part = align_up((size_t)B * H * N * kD * sizeof(float), 256);
-  l.part2 = N > kSlab ? align_up((size_t)B * H * (N - kSlab) * kD * sizeof(float), 256) : 0;
-  l.low = l.pieces.first > 1 ? align_up((size_t)B * H * (N < kSlab ? N : kSlab) * kD * sizeof(float), 256) : 0;
-  const size_t planes = N > kSlab ? 1 + l.pieces.others : 1;
   size_t off = simplicial_schedule_layout(B, &l.info, &l.order);
   auto take = [&off](size_t bytes) {
     const size_t at = off;
@@ -881,16 +841,15 @@ RowsBwdLayout rows_bwd_layout(int B, int H, int N) {
     return at;
   };
   l.delta = take(align_up((size_t)B * H * N * sizeof(float), 256));
-  l.dq = take(l.part * l.ctas);
-  l.dk1 = take(l.part * planes);
-  l.dv1 = take(l.part * planes);
-  l.dk2 = take(l.part2 * 2);
-  l.dv2 = take(l.part2 * 2);
-  l.dk2_low = take(l.low * l.pieces.first);
-  l.dv2_low = take(l.low * l.pieces.first);
+  l.dq = take(l.part * l.slabs_max * pieces);
+  l.dk1 = take(l.part * l.slabs_max);
+  l.dv1 = take(l.part * l.slabs_max);
+  l.dk2 = take(pieces > 1 ? l.part * pieces : 0);
+  l.dv2 = take(pieces > 1 ? l.part * pieces : 0);
   l.total = off;
   return l;
 }
+RowsBwdLayout rows_bwd_layout(int B, int H, int N) { return rows_bwd_layout(B, H, N, pieces_of(B * H, N)); }
 
 }  // namespace
 
@@ -916,8 +875,7 @@ int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   p.dk2 = static_cast<__nv_bfloat16*>(a.dk2);
   p.dv2 = static_cast<__nv_bfloat16*>(a.dv2);
   p.status = reinterpret_cast<int32_t*>(ws);
-  p.use_tma = make_rows_tensor_map(&p.tm_k[0], a.k2, a.tokens, BH) && make_rows_tensor_map(&p.tm_v[0], a.v2, a.tokens, BH) &&
-              make_rows_tensor_map(&p.tm_k[1], a.k1, a.tokens, BH) && make_rows_tensor_map(&p.tm_v[1], a.v1, a.tokens, BH);
+  p.use_tma = make_rows_tensor_map(&p.tm_k2, a.k2, a.tokens, BH) && make_rows_tensor_map(&p.tm_v2, a.v2, a.tokens, BH);
   BatchInfo* info = reinterpret_cast<BatchInfo*>(ws + l.info);
   int32_t* order = reinterpret_cast<int32_t*>(ws + l.order);
   float* delta = reinterpret_cast<float*>(ws + l.delta);
@@ -929,29 +887,24 @@ int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
   p.dv1_part = reinterpret_cast<float*>(ws + l.dv1);
   p.dk2_part = reinterpret_cast<float*>(ws + l.dk2);
   p.dv2_part = reinterpret_cast<float*>(ws + l.dv2);
-  p.dk2_low = reinterpret_cast<float*>(ws + l.dk2_low);
-  p.dv2_low = reinterpret_cast<float*>(ws + l.dv2_low);
-  p.pieces = l.pieces.first, p.pieces12 = l.pieces.others;
+  p.pieces = l.pieces;
   p.H = a.heads;
   p.N = a.tokens;
-  p.BH = BH;
+  p.slabs_max = l.slabs_max;
   p.part_stride = l.part / sizeof(float);
-  p.part2_stride = l.part2 / sizeof(float);
-  p.low_stride = l.low / sizeof(float);
 
   int rc = launch_schedule(a.query_valid, a.pair_key_valid, a.batch, a.tokens, info, order, p.status, stream);
   if (rc != MF_OK) return rc;
   const int rows = BH * a.tokens;
   launch_dependent(delta_rows_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, p.grad_out, a.out, delta, rows);
   MF_CHECK_LAUNCH("delta_rows_kernel");
-  auto kernel = a.tokens > kSlab ? simplicial_rows_bwd_kernel<true> : simplicial_rows_bwd_kernel<false>;
   {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
+    cudaError_t e = cudaFuncSetAttribute(simplicial_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(simplicial_rows_bwd_kernel)");
   }
-  const long long blocks = (long long)BH * l.ctas;
+  const long long blocks = (long long)BH * l.slabs_max * l.pieces;
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, true, stream);
-  launch_dependent(kernel, dim3((unsigned)blocks), dim3(kBwdThreads), kSmemAlloc, stream, p);
+  launch_dependent(simplicial_rows_bwd_kernel, dim3((unsigned)blocks), dim3(kBwdThreads), kSmemAlloc, stream, p);
   profile_mark(MF_PROFILE_SIMPLICIAL_BWD, false, stream);
   MF_CHECK_LAUNCH("simplicial_rows_bwd_kernel");
   const long long total4 = (long long)rows * (kD / 4);

@@ -44,12 +44,11 @@ __global__ void extent_kernel(const uint8_t* __restrict__ query_valid, const uin
   const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (b >= B) return;
-  int nk = 0, nq = 0, cnt = 0, low = 0;
+  int nk = 0, nq = 0, cnt = 0;
   for (int t = lane; t < N; t += 32) {
     if (key_valid[(size_t)b * N + t]) {
       nk = t + 1;
       ++cnt;
-      low += t < 128;
     }
     if (query_valid[(size_t)b * N + t]) nq = t + 1;
   }
@@ -58,13 +57,12 @@ __global__ void extent_kernel(const uint8_t* __restrict__ query_valid, const uin
     nk = max(nk, __shfl_xor_sync(0xffffffffu, nk, o));
     nq = max(nq, __shfl_xor_sync(0xffffffffu, nq, o));
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    low += __shfl_xor_sync(0xffffffffu, low, o);
   }
   if (lane == 0) {
     info[b].n_keys = nk;
     info[b].n_queries = nq;
     info[b].reserved0 = cnt;  // number of valid keys
-    info[b].reserved1 = low;
+    info[b].reserved1 = 0;
   }
 }
 

@@ -18,7 +18,7 @@ struct BatchInfo {
   int32_t n_keys;     // 1 + index of the last valid key (0 when none)
   int32_t n_queries;  // 1 + index of the last valid query
   int32_t reserved0;  // number of valid keys
-  int32_t reserved1;  // row-packed and tile kernels: number of valid keys among the first 128
+  int32_t reserved1;
 };
 
 // Where row `token` of head `head` of batch element `batch` starts, in elements: (B,H,N,64) contiguous by default;
