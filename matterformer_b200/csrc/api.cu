@@ -112,15 +112,14 @@ bool uses_tri_kernels(const Args* a) {
   return a->tokens > kSmallTokens && has_factorized_bias(a);
 }
 // The forward pass runs on them where a call is long enough.  A tile walks all first keys of its rows whatever the batch, up to 100
-// tokens in at most 26 steps, from 101 on in up to 128 (tri_plan); the warp-level kernel spreads the queries of a small batch over
+// tokens in at most 32 steps, from 101 on in up to 64 (tri_plan); the warp-level kernel spreads the queries of a small batch over
 // the chip.  The host does not know how full the batch is, so the lines lie between the two extremes.  8 heads, us, trilinear |
-// warp-level, all molecules full | spread from an eighth of the tokens up: 64 tokens x 4 molecules 53 | 32, 53 | 17; x 16 54 | 77,
-// 54 | 43; x 32 98 | 136, 57 | 92.  96 x 4 54 | 60, 54 | 31; x 12 99 | 150, 60 | 87.  128 x 4 254 | 143, 249 | 68; x 12 255 | 334,
-// 250 | 159; x 32 492 | 892, 255 | 364.  192 x 1 257 | 103; x 6 259 | 557, 257 | 257; x 32 1 479 | 2 814, 580 | 1 078.  On either
-// side a molecule's result does not depend on its batch; the two sides round differently, with the same error.
-// MF_BACKEND_TCGEN05_TILES stays on one side.  (Measured before calls of few molecules were spread over more tiles, see spread_tiles;
-// with that the trilinear kernel wins above 100 tokens from two to four molecules on: 128 x 4 121 | 145 full, 66 | 82 spread, x 8 146 |
-// 252, 80 | 156.  The lines are kept: moving them changes which kernel, and which rounding, a call gets.)
+// warp-level, all molecules full | spread, up to 96 tokens from an eighth of the tokens up, above from a third: 64 tokens x 4 molecules
+// 53 | 32, 53 | 17; x 16 54 | 77, 54 | 43; x 32 98 | 136, 57 | 92.  96 x 4 54 | 60, 54 | 31; x 12 99 | 150, 60 | 87.  128 x 1 144 | 50; x 4
+// 146 | 145, 142 | 82; x 8 148 | 252, 144 | 156.  192 x 1 144 | 106; x 2 146 | 207, 144 | 122.  (Above 100 tokens the line, from nine
+// molecules of 128 or three of 192 on, dates from longer tiles, of up to 128 steps; it is kept, because moving it changes which rounding a
+// call gets.)  On either side a molecule's result does not depend on its batch; the two sides round differently, with the same error.
+// MF_BACKEND_TCGEN05_TILES stays on one side.
 inline bool uses_tri_forward(const MfSimplicialFwdArgs* a) {
   if (!uses_tri_kernels(a)) return false;
   const double heads = (double)a->batch * a->heads, n = a->tokens;

@@ -30,12 +30,12 @@
 //
 // Bound by the chain of hand-overs of a step (half of the time is left with no MMA and no arithmetic at all) and the softmax
 // warps' instructions; the tensor pipe is busy for 16 to 20 % of the time.  The backward kernel spills (326 bytes of stores, 432 of
-// loads by ptxas): one register split serves its three passes, whose accumulators differ.  Of the CTAs launched, five per pass,
-// half to four fifths find no tile and return (up to 96 tokens a molecule has at most four, up to 64 at most two).
-// 64 molecules of 20-181 atoms of 192 tokens, 8 heads: forward 0.85 ms, backward 3.6 ms (mma.sync kernels, query by query and first
-// key by first key: 1.82 and 6.09 ms); 64 full ones of 64 tokens 0.19 and 0.68 ms (0.24 and 0.96).  A single molecule of 181: 0.24
-// and 0.42 ms (0.12, which is why short forward calls stay there, and 1.54).
-#include <algorithm>
+// loads by ptxas): one register split serves its three passes, whose accumulators differ.  Of the CTAs launched, six per pass, half
+// to five sixths find no tile and return (up to 96 tokens a molecule has at most four, up to 64 at most two).
+// 64 molecules of 20-181 atoms of 192 tokens, 8 heads: forward 0.86 ms, backward 3.65 ms (mma.sync kernels, query by query and first
+// key by first key: 1.82 and 6.09 ms); 64 full ones of 64 tokens 0.19 and 0.68 ms (0.24 and 0.96).  A single molecule of 181: 0.14
+// and 0.23 ms (0.12, which is why short forward calls stay there, and 1.54).
+#include <climits>
 
 #include "common.cuh"
 #include "simplicial.cuh"
@@ -85,31 +85,37 @@ constexpr int tri_smem_bytes(int tokens) {
 }
 
 // The split of a molecule into tiles of (x, y) rows, as plan_rows() of simplicial_rows.cuh, but a tile costs kTileCost steps
-// besides its own (loads, the pipeline's first and last step).  It depends on the molecule alone, but for `spread`, so that its results
-// do not depend on the batch it is in.  More than five tiles for the sake of fuller rows save nothing: 64 molecules of 20-181 atoms, steps + 5 per tile at most 8 | 6 |
-// 4 | 3 tiles: 60.5 | 60.5 | 61.3 | 63.8 thousand.
-// `spread`: in a call of few heads and more than 100 tokens, where tiles of one first key a step (rows of more than 64 x) leave most of the
-// chip idle for as long as the longest of them takes, up to that many tiles are taken for the sake of shorter ones.
-constexpr int kTileCost = 4, kMostTiles = 5, kSpreadTiles = 6;
+// besides its own (loads, the pipeline's first and last step).  More than five tiles for the sake of fuller rows save nothing: 64
+// molecules of 20-181 atoms, steps + 5 per tile at most 8 | 6 | 4 | 3 tiles: 60.5 | 60.5 | 61.3 | 63.8 thousand.
+// A call lasts at least as long as its longest tile, and beyond kShortWalk x the cheapest split may have tiles of one first key a step
+// (rows of more than 64 x), 100 to 128 steps long, or of two, up to 96.  There the split with the fewest steps is taken of those, of up to
+// six tiles, whose cost is within kSlack hundredths of the lowest.  Backward, 8 heads, us, slack 0 | 7 | 10: 1 molecule of 101 atoms 278 |
+// 96 | 78, of 128 345 | 190 | 117, of 181 417 | 229 | 231; 4 of 43-128 343 | 190 | 164, of 60-181 454 | 375 | 375; 64 of 128 3 305 | 3 307 |
+// 3 515, of 181 10 357 | 11 009 | 11 015; 64 of 20-181 atoms of 192 tokens, forward + backward, 4 436 | 4 519 | 4 532.
+// The split depends on the molecule alone, so that its results do not depend on the batch it is in: more tiles for small batches only
+// would cost the large ones nothing.
+constexpr int kTileCost = 4, kMostTiles = 6, kShortWalk = 100, kSlack = 7;
 struct TriPlan {
   int tiles, rows;
 };
-__device__ inline TriPlan tri_plan(int nx, int ny, int spread) {
+__device__ inline TriPlan tri_plan(int nx, int ny) {
   TriPlan best{0, 0};
-  int best_cost = 0, best_steps = 0;
   if (nx <= 0 || ny <= 0) return best;
+  const int most = nx > kShortWalk ? kMostTiles : kMostTiles - 1, slack = nx > kShortWalk ? kSlack : 0;
+  int limit = INT_MAX, best_cost = 0, best_steps = 0;
 #pragma unroll 1
-  for (int t = 1; t <= kMostTiles; ++t) {
-    const int rows = (nx + t - 1) / t;
-    if (rows > kTileM) continue;
-    const int tiles = (nx + rows - 1) / rows, groups = min(kTileM / rows, kMaxGroups);
-    const int steps = (ny + groups - 1) / groups, cost = tiles * (steps + kTileCost);
-    if (best.tiles == 0 || cost < best_cost) best = TriPlan{tiles, rows}, best_cost = cost, best_steps = steps;
-  }
+  for (int choice = 0; choice < 2; ++choice) {  // the lowest cost, then the fewest steps within its slack
 #pragma unroll 1
-  for (int t = best.tiles + 1; t <= spread; ++t) {
-    const int rows = (nx + t - 1) / t, tiles = (nx + rows - 1) / rows, steps = (ny + min(kTileM / rows, kMaxGroups) - 1) / min(kTileM / rows, kMaxGroups);
-    if (steps < best_steps) best = TriPlan{tiles, rows}, best_steps = steps;
+    for (int t = 1; t <= most; ++t) {
+      const int rows = (nx + t - 1) / t;
+      if (rows > kTileM) continue;
+      const int tiles = (nx + rows - 1) / rows, groups = min(kTileM / rows, kMaxGroups), steps = (ny + groups - 1) / groups;
+      const int cost = tiles * (steps + kTileCost);
+      const bool better = best.tiles == 0 || (choice == 0 ? cost < best_cost : steps < best_steps && 100 * cost <= limit);
+      if (better) best = TriPlan{tiles, rows}, best_cost = cost, best_steps = steps;
+    }
+    if (slack == 0) break;
+    limit = (100 + slack) * best_cost;
   }
   return best;
 }
@@ -863,8 +869,8 @@ __global__ void __maxnreg__(kRegLaunch) simplicial_tri_bwd_kernel(const __grid_c
 constexpr int kScheduleThreads = 1024;
 __global__ void __launch_bounds__(kScheduleThreads) simplicial_tri_schedule_kernel(const uint8_t* __restrict__ query_valid,
                                                                                   const uint8_t* __restrict__ key_valid, int B, int N,
-                                                                                  int backward, int spread, BatchInfo* info,
-                                                                                  int2* items, int32_t* status) {
+                                                                                  int backward, BatchInfo* info, int2* items,
+                                                                                  int32_t* status) {
   wait_for_previous();
   __shared__ int start[kMaxKeys + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -873,7 +879,7 @@ __global__ void __launch_bounds__(kScheduleThreads) simplicial_tri_schedule_kern
   __syncthreads();
   auto plan = [&](const BatchInfo& m, int pass) {
     const bool any = m.reserved0 > 0 && m.reserved1 > 0;
-    return tri_plan(pass == kDq || pass == kFwd ? m.n_queries : m.n_keys, any ? pass == kDk2 ? m.reserved1 : m.reserved0 : 0, spread);
+    return tri_plan(pass == kDq || pass == kFwd ? m.n_queries : m.n_keys, any ? pass == kDk2 ? m.reserved1 : m.reserved0 : 0);
   };
   const int first = backward ? kDq : kFwd, last = backward ? kDk2 : kFwd;
   auto bucket = [&](const BatchInfo& m) { return kMaxKeys - (m.n_keys + m.n_queries) / 2; };
@@ -953,21 +959,13 @@ __global__ void __launch_bounds__(256) simplicial_tri_clear_kernel(const __grid_
 
 struct TriLayout {
   size_t info, items, lse2, ndelta, total;
-  int max_items, spread;
+  int max_items;
 };
-// Tiles that each molecule and pass may take for the sake of short ones: as many as about one and a half waves hold.  8 heads, backward,
-// n / 3 to n atoms, us without | with: 101 tokens, 1, 4, 16 molecules 251 | 56, 254 | 95, 278 | 280; 128
-// 340 | 88, 330 | 174, 515 | 440; 181 398 | 215, 642 | 530, 1 589 | 1 493.
-int spread_tiles(int batch, int heads, int tokens, int passes) {
-  const long long items = (long long)batch * heads * passes;
-  return tokens <= 100 || items <= 0 || items >= 222 ? 0 : (int)std::min<long long>(kSpreadTiles, (222 + items - 1) / items);
-}
 TriLayout tri_layout(int batch, int heads, int tokens, bool backward) {
   TriLayout l{};
   size_t off = kStatusBytes;
   l.info = off, off = align_up(off + (size_t)batch * sizeof(BatchInfo), 256);
-  l.spread = spread_tiles(batch, heads, tokens, backward ? 3 : 1);
-  l.max_items = batch * std::max(kMostTiles, l.spread) * (backward ? 3 : 1);
+  l.max_items = batch * kMostTiles * (backward ? 3 : 1);
   l.items = off, off = align_up(off + (1 + (size_t)l.max_items) * sizeof(int2), 256);
   if (backward) {
     const size_t rows = align_up((size_t)batch * heads * tokens * sizeof(float), 256);
@@ -995,7 +993,7 @@ void fill_params(TriParams& p, const Args& a, const TriLayout& l) {
 template <typename Kernel>
 int launch_tri(Kernel kernel, const TriParams& p, const TriLayout& l, int batch, bool backward, int which, cudaStream_t stream, const char* name) {
   launch_dependent(simplicial_tri_schedule_kernel, dim3(1), dim3(kScheduleThreads), 0, stream, p.query_valid, p.key_valid, batch, p.N,
-                   backward, l.spread, const_cast<BatchInfo*>(p.info), const_cast<int2*>(p.items), p.status);
+                   backward, const_cast<BatchInfo*>(p.info), const_cast<int2*>(p.items), p.status);
   MF_CHECK_LAUNCH("simplicial_tri_schedule_kernel");
   // (the limit is one for all sizes: another host thread must not lower it between here and the launch)
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes(kMaxKeys));

@@ -185,3 +185,18 @@ def test_spread_tiles_against_oracle(B, H, N):
         assert_rel(got[:keep], g_ref[n][:keep], 2.5e-2, f"d{n}")
         if B > 4:
             assert torch.equal(got[4:8], got[: min(4, B - 4)])
+
+
+@pytest.mark.parametrize("B,N", [(2, 128), (9, 128), (20, 128), (28, 128), (4, 192), (8, 192), (14, 110)])
+def test_a_molecule_alone_and_in_batches_of_many_sizes(B, N):
+    """The split into tiles depends on the molecule alone: the same bits from a call that leaves most of the chip idle and from one that
+    fills it, for molecules of N, 101 and 65 atoms."""
+    t, valid, go = _device_case(B, 8, N, seed=B + N, lo=N)
+    if B > 2:
+        valid[1] = torch.arange(N, device="cuda") < 101
+        valid[2] = torch.arange(N, device="cuda") < 65
+    whole = _run(t, valid, go)
+    for i in range(min(B, 3)):
+        part = _run({n: x[i : i + 1].contiguous() for n, x in t.items()}, valid[i : i + 1].contiguous(), go[i : i + 1].contiguous())
+        for a, b in zip(whole, part):
+            assert torch.equal(a[i : i + 1], b)
