@@ -114,26 +114,32 @@ __host__ __device__ inline int slab_width(int n_keys) {
 }
 
 // A slab's walk goes in one piece where the molecules fill the chip several times over, and in several, a CTA each, where they do not: a
-// CTA by itself takes the walk's full length however few others there are, and the largest molecule of a batch decides.  A piece
-// costs its set-up and fp32 planes for the sums that run over the walk.
-// The number with the shortest estimate: the longer of one piece (the largest molecule: kPieceUs for its set-up and the beginnings and
-// ends of its query ranges, and its share of a walk of kWalkUs N^2, both from measured times) and all of them on kSms SMs, the batch at
-// half of its largest molecule's work (sizes spread from an eighth up 0.38, all full 1; the host does not know).  A molecule or two
-// cannot fill a second wave with small pieces: it counts by itself.  Powers of two, so that batches near each other share a number: on
-// one side of a line a molecule's bits do not depend on its batch.
+// CTA by itself takes the walk's full length however few others there are, and the largest molecule of a batch decides.
+//
+// The host knows no sizes but the padded one, so the number is the one with the shortest estimate summed over two batches: one whose
+// molecules are all full, ceil(CTAs / kSms) rounds of full pieces, one CTA to an SM; and one whose sizes are spread from an eighth up,
+// whose walks are 0.38 of a full one on average (the mean of x^2), all of them packed onto the SMs, or the largest piece where that is
+// longer.  A full walk is kWalkUs N^2, a piece costs kPieceUs besides its share (set-up, the beginnings and ends of its query ranges),
+// a call kCallUs for its other kernels; all three fitted to the times below.  A number has to be 5 % faster than half of it, for its fp32
+// planes.  Powers of two, so that batches near each other share a number: a molecule's bits depend on it.
+//
+// 8 heads, the call in us, 1 | 2 | 4 | 8 | 16 pieces, all full (spread), [this]: 128 tokens, 1 molecule 424 | 229 | 133 | 86 | 66 [16]; 4
+// 422 | 231 | 137 | 154 | 184 (418 | 227 | 133 | 98 | 129) [8]; 16 432 | 453 | 483 | 490 | 614 (424 | 234 | 239 | 303 | 424) [2].  181
+// tokens, 4 845 | 455 | 479 | 539 | 563 (842 | 451 | 250 | 217 | 238) [4]; 32 3 345 | 3 089 | 3 263 | 3 727 | 4 222 (1 146 | 1 113 | 1 240 |
+// 1 469 | 1 898) [2]; 64 5 864 | 6 119 | 6 470 | 7 362 | 8 416 (1 998 | 2 143 | 2 404 | 2 856 | 3 747) [1].  Over 40-192 tokens x 1-64
+// molecules, both batches together, the choice takes 1.6 % longer than the best of the five on average, and nowhere longer than one piece.
 inline int pieces_of(int BH, int N) {
-  constexpr float kPieceUs = 30.f, kWalkUs = 0.0245f, kShare = 0.5f, kSms = 148.f;
-  const int slabs = slab_count(N);
+  constexpr float kCallUs = 15.f, kPieceUs = 18.f, kWalkUs = 0.0245f, kSpread = 0.38f;
+  constexpr int kSms = 148;
   const float walk = kWalkUs * N * N;
   int best = 1;
   float least = INFINITY;
   for (int pieces = 1; pieces <= 16; pieces *= 2) {
-    const float all = BH * slabs * (pieces * kPieceUs + kShare * walk) / kSms;
-    float piece = kPieceUs + walk / pieces;
-    const int waves = (BH * slabs * pieces + (int)kSms - 1) / (int)kSms;
-    if (BH <= 16 && waves > 1) piece *= 0.6f * waves;
-    const float time = std::max(piece, all);
-    if (time < 0.97f * least) least = time, best = pieces;
+    const long long ctas = (long long)BH * slab_count(N) * pieces;
+    const float piece = kPieceUs + walk / pieces, full = (float)((ctas + kSms - 1) / kSms) * piece;
+    const float spread = std::max(piece, ctas * (kPieceUs + kSpread * walk / pieces) / kSms);
+    const float time = 2.f * kCallUs + full + spread;
+    if (time < 0.95f * least) least = time, best = pieces;
   }
   return best;
 }
