@@ -185,7 +185,9 @@ typedef struct MfSimplicialBwdArgs {
   float* message_coeff;
 } MfSimplicialBwdArgs;
 
-/* Bytes of scratch the calls below need for these sizes (0 is possible). */
+/* Bytes of scratch for the calls below with these sizes (0 is possible).  What a batch asks for serves smaller batches of the same
+ * molecules' size too, although the backward call may ask for more for a smaller batch: with less than that it walks a molecule
+ * in fewer pieces (without the bias, above 32 tokens; the gradients' last bits depend on the number of pieces, and so on the batch). */
 size_t mf_simplicial_fwd_workspace_bytes(const MfSimplicialFwdArgs* args);
 size_t mf_simplicial_bwd_workspace_bytes(const MfSimplicialBwdArgs* args);
 

@@ -255,7 +255,8 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool tc = wants_tcgen05(a, &rc, "mf_simplicial_bwd");
   if (rc != MF_OK) return rc;
-  const size_t need = mf_simplicial_bwd_workspace_bytes(a);
+  const bool rows = tc && !uses_small_kernels(a) && !uses_tri_kernels(a) && a->backend != MF_BACKEND_TCGEN05_TILES;
+  const size_t need = rows ? simplicial_rows_bwd_least_bytes(*a) : mf_simplicial_bwd_workspace_bytes(a);
   if (need > 0 && (!a->workspace || a->workspace_bytes < need) && !(tc && uses_small_kernels(a))) {
     set_error("mf_simplicial_bwd: workspace of %zu bytes needed, %zu given", need, a->workspace_bytes);
     return MF_ERR_WORKSPACE_TOO_SMALL;
@@ -263,7 +264,7 @@ extern "C" int mf_simplicial_bwd(const MfSimplicialBwdArgs* a, void* stream) {
   if (!tc) return uses_f32_kernels(a) ? simplicial_f32_bwd(*a, s) : simplicial_generic_bwd(*a, s);
   if (uses_small_kernels(a)) return simplicial_small_bwd(*a, nullptr, s);
   if (uses_tri_kernels(a)) return simplicial_tri_bwd(*a, s);
-  return a->backend == MF_BACKEND_TCGEN05_TILES ? simplicial_sm100_bwd(*a, s) : simplicial_rows_bwd(*a, s);
+  return rows ? simplicial_rows_bwd(*a, s) : simplicial_sm100_bwd(*a, s);
 }
 
 extern "C" int mf_selftest_simplicial_give_up(const MfSimplicialFwdArgs* fwd, const MfSimplicialBwdArgs* bwd, int32_t withheld,

@@ -56,5 +56,6 @@ size_t simplicial_tri_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
 int simplicial_rows_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream, BoundedWaits waits = {});
 int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream);
 size_t simplicial_rows_bwd_workspace_bytes(const MfSimplicialBwdArgs& a);
+size_t simplicial_rows_bwd_least_bytes(const MfSimplicialBwdArgs& a);  // with less the call is refused
 
 }  // namespace mf

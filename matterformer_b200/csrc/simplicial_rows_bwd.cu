@@ -121,7 +121,7 @@ __host__ __device__ inline int slab_width(int n_keys) {
 // whose walks are 0.38 of a full one on average (the mean of x^2), all of them packed onto the SMs, or the largest piece where that is
 // longer.  A full walk is kWalkUs N^2, a piece costs kPieceUs besides its share (set-up, the beginnings and ends of its query ranges),
 // a call kCallUs for its other kernels; all three fitted to the times below.  A number has to be 5 % faster than half of it, for its fp32
-// planes.  Powers of two, so that batches near each other share a number: a molecule's bits depend on it.
+// planes.  Powers of two: the last bits of a molecule's gradients depend on the number, so there are few.
 //
 // 8 heads, the call in us, 1 | 2 | 4 | 8 | 16 pieces, all full (spread), [this]: 128 tokens, 1 molecule 424 | 229 | 133 | 86 | 66 [16]; 4
 // 422 | 231 | 137 | 154 | 184 (418 | 227 | 133 | 98 | 129) [8]; 16 432 | 453 | 483 | 490 | 614 (424 | 234 | 239 | 303 | 424) [2].  181
@@ -855,16 +855,23 @@ RowsBwdLayout rows_bwd_layout(int B, int H, int N, int pieces) {
   l.total = off;
   return l;
 }
-RowsBwdLayout rows_bwd_layout(int B, int H, int N) { return rows_bwd_layout(B, H, N, pieces_of(B * H, N)); }
+// The preferred number of pieces, or the largest that fits `bytes`: a smaller batch may prefer more pieces than a larger one and
+// need more scratch, but what the larger one needs always holds one piece of it.
+RowsBwdLayout rows_bwd_layout_within(int B, int H, int N, size_t bytes) {
+  RowsBwdLayout l = rows_bwd_layout(B, H, N, pieces_of(B * H, N));
+  while (l.pieces > 1 && l.total > bytes) l = rows_bwd_layout(B, H, N, l.pieces / 2);
+  return l;
+}
 
 }  // namespace
 
 size_t simplicial_rows_bwd_workspace_bytes(const MfSimplicialBwdArgs& a) {
-  return rows_bwd_layout(a.batch, a.heads, a.tokens).total;
+  return rows_bwd_layout(a.batch, a.heads, a.tokens, pieces_of(a.batch * a.heads, a.tokens)).total;
 }
+size_t simplicial_rows_bwd_least_bytes(const MfSimplicialBwdArgs& a) { return rows_bwd_layout(a.batch, a.heads, a.tokens, 1).total; }
 
 int simplicial_rows_bwd(const MfSimplicialBwdArgs& a, cudaStream_t stream) {
-  const RowsBwdLayout l = rows_bwd_layout(a.batch, a.heads, a.tokens);
+  const RowsBwdLayout l = rows_bwd_layout_within(a.batch, a.heads, a.tokens, a.workspace_bytes);
   char* ws = static_cast<char*>(a.workspace);
   const int BH = a.batch * a.heads;
   RowsBwdParams p{};

@@ -5,6 +5,8 @@ key slabs), masks with holes on queries, keys and pairs, and the benchmark batch
 Tolerance: bf16 results within 2e-2 of the oracle's largest value, or no worse than the error the reference's
 own bf16 torch path makes against its fp32 core on the same inputs (src/matterformer/models/
 simplicial_attention.py:251-297), whichever is larger (conftest.bf16_allowance)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -218,3 +220,40 @@ def test_gradients_of_all_second_keys_are_as_exact(scale):
         size = ref.square()
         low, high = (error[..., s, :].mean().div(size[..., s, :].mean()).sqrt().item() for s in (slice(0, 128), slice(128, 181)))
         assert high < (1.08 if scale < 1 else 1.16) * low, f"d{n}: {high:.3e} from key 128 on, {low:.3e} before"
+
+
+def _scratch(batch, N):
+    a = _lib.MfSimplicialBwdArgs(batch=batch, heads=8, tokens=N, head_dim=64, dtype=_lib.MF_DTYPE_BF16)
+    return _lib.lib().mf_simplicial_bwd_workspace_bytes(ctypes.byref(a))
+
+
+@pytest.mark.parametrize("N,large,small", [(128, 20, 19), (128, 7, 6), (150, 17, 16), (192, 4, 3), (40, 10, 9)])
+def test_scratch_of_a_larger_batch_serves_a_smaller_one(N, large, small):
+    """A smaller batch prefers more pieces and asks for more scratch; with what the larger one asks for it takes fewer.  Half of what one
+    piece needs is refused."""
+    L = _lib.lib()
+    g = torch.Generator(device=DEV).manual_seed(N)
+    t = {n: torch.randn(small, 8, N, 64, generator=g, device=DEV).div(8).bfloat16() for n in (*NAMES, "grad_out")}
+    valid = torch.arange(N, device=DEV)[None] < torch.randint(N // 2, N + 1, (small, 1), generator=g, device=DEV)
+    out, lse, out32 = mfb.cuda_simplicial_attention_forward(*(t[n] for n in NAMES), query_valid=valid, pair_key_valid=valid, pair_valid=None)
+    assert _scratch(large, N) < _scratch(small, N)
+
+    def call(scratch):
+        a = _lib.MfSimplicialBwdArgs(batch=small, heads=8, tokens=N, head_dim=64, dtype=_lib.MF_DTYPE_BF16)
+        grads = {f"d{n}": torch.full_like(t[n], float("nan")) for n in NAMES}
+        ws = torch.empty(scratch, dtype=torch.uint8, device=DEV)
+        mask = valid.view(torch.uint8)
+        for name, x in {**t, **grads, "out": out32, "lse": lse, "query_valid": mask, "pair_key_valid": mask, "workspace": ws}.items():
+            setattr(a, name, x.data_ptr())
+        a.workspace_bytes = scratch
+        code = L.mf_simplicial_bwd(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        return code, grads, ws[:4].view(torch.int32).item() if code == _lib.MF_OK else None
+
+    code, want, status = call(_scratch(small, N))
+    assert (code, status) == (_lib.MF_OK, 0)
+    code, got, status = call(_scratch(large, N))
+    assert (code, status) == (_lib.MF_OK, 0)
+    for n in NAMES:  # the same up to the order of fp32 sums and one rounding
+        assert _rel(got[f"d{n}"].float(), want[f"d{n}"].float()) <= 1e-2
+    one_piece = _scratch(1000, N) // 1000 * small  # (a thousand molecules walk in one piece)
+    assert call(one_piece // 2)[0] == _lib.MF_ERR_WORKSPACE_TOO_SMALL
