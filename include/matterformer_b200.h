@@ -419,11 +419,16 @@ int mf_local_attn_packed_fwd(const MfLocalAttnPackedArgs* args, void* stream);
 int mf_local_attn_packed_bwd(const MfLocalAttnPackedArgs* args, void* stream);
 
 /*
- * Status word of the tcgen05 sparse-attention kernels (no counterpart in the reference): 0, or
- * MF_ERR_DEVICE_TIMEOUT once a bounded device-side wait has expired (the outputs of that call are then
- * undefined).  Waits for `stream`, copies four bytes, allocates nothing.
+ * Status word of the sparse-attention kernels with device-side waits, tcgen05 and 128-row band tiles (no counterpart in the
+ * reference): 0, or MF_ERR_DEVICE_TIMEOUT from the first bounded wait that has expired on (the outputs of that call are then
+ * undefined on tcgen05; of band tiles, the rows of the tile are zeros).  Waits for `stream`, copies four bytes, allocates nothing.
  */
 int mf_sparse_attn_status(int32_t* host_status, void* stream);
+/* Self-test of what an expired wait of the 128-row band tiles leaves behind (no counterpart in the reference): a local-window call,
+ * forward or backward, whose tiles never arrive for the kernel; waits give up after `limit_cycles`, and after about a second more for
+ * copies in flight.  Leaves zeros in the outputs and MF_ERR_DEVICE_TIMEOUT in *host_status, and clears the status word of these
+ * kernels.  bf16, head_dim 64, windows of 32, 64 or 128, at least 128 tiles (batch * heads * ceil(tokens / 128)). */
+int mf_selftest_band_give_up(const MfSparseAttnArgs* args, int32_t backward, int64_t limit_cycles, int32_t* host_status, void* stream);
 
 /* ------------------------------------------------------------------------- */
 /* Errors                                                                     */

@@ -58,6 +58,7 @@ EXPORTED_SYMBOLS = (
     "mf_local_attn_fwd",
     "mf_local_attn_bwd",
     "mf_sparse_attn_status",
+    "mf_selftest_band_give_up",
     "mf_local_attn_packed_bwd_workspace_bytes",
     "mf_local_attn_packed_fwd",
     "mf_local_attn_packed_bwd",
@@ -421,6 +422,8 @@ def lib() -> ctypes.CDLL:
         fn.restype = c_int32
     L.mf_sparse_attn_status.argtypes = [POINTER(c_int32), c_void_p]
     L.mf_sparse_attn_status.restype = c_int32
+    L.mf_selftest_band_give_up.argtypes = [POINTER(MfSparseAttnArgs), c_int32, ctypes.c_int64, POINTER(c_int32), c_void_p]
+    L.mf_selftest_band_give_up.restype = c_int32
     L.mf_pair_head_bwd_workspace_bytes.argtypes = [POINTER(MfPairHeadArgs)]
     L.mf_pair_head_bwd_workspace_bytes.restype = c_size_t
     L.mf_masked_sum.argtypes = [POINTER(MfMaskedSumArgs), c_void_p]

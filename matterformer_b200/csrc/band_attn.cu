@@ -41,6 +41,7 @@ struct BandParams {
   int H, N;
   float scale;
   RowLayout in, act;  // rows of q, k, v and their gradients; rows of out and grad_out
+  BoundedWaits waits; // of the tiles that arrive by bulk copies (kind 0)
 };
 
 __device__ int32_t g_band_status = 0;  // MF_ERR_DEVICE_TIMEOUT after an expired wait
@@ -54,12 +55,12 @@ template <int kRows>
 using MapsOf = std::conditional_t<kRows == 128, BandMaps, NoMaps>;
 
 // Waits for the copies on `bar` and clears the rows of `tiles` tiles that lie in [n, N) (they may hold NaN).  False: the wait expired,
-// for every thread alike.
+// for every thread alike; the CTA then writes zeros (clear_rows) and ends.
 template <int kThreads, int kTiles>
 __device__ __forceinline__ bool tiles_arrived(uint64_t* bar, uint8_t* smem, const int (&at)[kTiles], const int (&first)[kTiles],
-                                              const int (&rows)[kTiles], int n) {
-  bool ok = mbar_wait(bar, 0);
-  if (!ok) ok = mbar_wait(bar, 0);  // the copies write to this CTA: give them once more as long
+                                              const int (&rows)[kTiles], int n, const BoundedWaits& waits) {
+  bool ok = mbar_wait_for(bar, 0, waits.limit);
+  if (!ok) ok = mbar_wait(bar, 0);  // the copies write to this CTA: none is in flight when it gives up
   if (__syncthreads_or(!ok)) {
     if (threadIdx.x == 0) atomicExch(&g_band_status, MF_ERR_DEVICE_TIMEOUT);
     return false;
@@ -74,6 +75,13 @@ __device__ __forceinline__ bool tiles_arrived(uint64_t* bar, uint8_t* smem, cons
   }
   if (edge) __syncthreads();  // (the same for all threads)
   return true;
+}
+
+// rows [first, first + rows) of one head that lie below N
+template <int kThreads>
+__device__ __forceinline__ void clear_rows(__nv_bfloat16* dst, long long stride, int first, int rows, int N) {
+  for (int idx = threadIdx.x; idx < 8 * min(rows, N - first); idx += kThreads)
+    *reinterpret_cast<uint4*>(dst + (first + (idx >> 3)) * stride + (idx & 7) * 8) = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // rows [first, first + rows) of one head into a swizzled tile; rows outside [0, n) become zeros
@@ -162,7 +170,7 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
     if constexpr (kRows == 128) {
       uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kTq + kRows * kRowBytes);
       if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+        mbar_init(bar, 1 + (p.waits.withheld == 0));
         mbar_fence_init();
         mbar_arrive_expect_tx(bar, (2 * kHalo + kRows) * kRowBytes);
         tma_load_strided_rows(tile, &maps.m[0], t0 - kHalf, h, b, bar);
@@ -170,7 +178,11 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 12 : W == 128 ? (kRows == 
         tma_load_strided_rows(tile + kTv, &maps.m[1], t0 - kHalf, h, b, bar);
       }
       __syncthreads();
-      if (!tiles_arrived<kThreads, 3>(bar, smem, {0, kTv, kTq}, {t0 - kHalf, t0 - kHalf, t0}, {kHalo, kHalo, kRows}, n)) return;
+      if (!tiles_arrived<kThreads, 3>(bar, smem, {0, kTv, kTq}, {t0 - kHalf, t0 - kHalf, t0}, {kHalo, kHalo, kRows}, n, p.waits)) {
+        clear_rows<kThreads>(p.out + act0, p.act.token, t0, kRows, N);
+        for (int i = threadIdx.x; i < min(kRows, N - t0); i += kThreads) p.lse[(size_t)bh * N + t0 + i] = 0.f;
+        return;
+      }
     } else {
       load_band<kThreads>(tile, p.k + in0, p.in.token, t0 - kHalf, kHalo, n);
       load_band<kThreads>(tile + kTq, p.q + in0, p.in.token, t0, kRows, n);
@@ -299,7 +311,7 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
   if (t0 < n) {
     if constexpr (kRows == 128) {
       if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+        mbar_init(bar, 1 + (p.waits.withheld == 0));
         mbar_fence_init();
         mbar_arrive_expect_tx(bar, 4 * kHalo * kRowBytes);
 #pragma unroll
@@ -331,7 +343,12 @@ __global__ void __launch_bounds__(kRows * 2, W == 0 ? 6 : kRows == 128 ? (W == 1
     }
     if constexpr (kRows == 128) {
       __syncthreads();  // the barrier exists
-      if (!tiles_arrived<kThreads, 4>(bar, smem, {0, kTk, kTv, kTg}, {first, first, first, first}, {kHalo, kHalo, kHalo, kHalo}, n)) return;
+      if (!tiles_arrived<kThreads, 4>(bar, smem, {0, kTk, kTv, kTg}, {first, first, first, first}, {kHalo, kHalo, kHalo, kHalo}, n, p.waits)) {
+        clear_rows<kThreads>(p.dq + in0, p.in.token, t0, kRows, N);
+        clear_rows<kThreads>(p.dk + in0, p.in.token, t0, kRows, N);
+        clear_rows<kThreads>(p.dv + in0, p.in.token, t0, kRows, N);
+        return;
+      }
 #pragma unroll
       for (int t = 0; t < kSteps; ++t) g[t] = *reinterpret_cast<const uint4*>(smem + row_chunk(kTg, r0 + t * (kThreads / 8), c));
     }
@@ -489,8 +506,16 @@ bool band_attn_applies(const MfSparseAttnArgs& a) {
   return a.window == 32 || a.window == 64;
 }
 
-int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream) {
+// 128-row tiles re-read half as much halo; 64-row ones spread a call over twice as many CTAs, which pays while the wide ones
+// would not cover the chip.  Forward + backward at window 64, 64 | 128 rows: 8 structures of 128 tokens (64 wide tiles) 14.7 |
+// 16.3 us, 128 tiles 17.3 | 16.4, 256 tiles 29.1 | 22.5, 576 tiles 50.4 | 42.2; windows 32 and 128 turn at the same place.
+bool band_attn_wide(const MfSparseAttnArgs& a) {
+  return a.tokens > kDenseTokens && (long long)a.batch * a.heads * ((a.tokens + 127) / 128) >= 128;
+}
+
+int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream, BoundedWaits waits) {
   BandParams p{};
+  p.waits = waits;
   p.q = static_cast<const __nv_bfloat16*>(a.q);
   p.k = static_cast<const __nv_bfloat16*>(a.k);
   p.v = static_cast<const __nv_bfloat16*>(a.v);
@@ -505,10 +530,7 @@ int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward
   p.in = layouts ? layouts[0] : contiguous_rows(a.heads, a.tokens);
   p.act = layouts ? layouts[1] : contiguous_rows(a.heads, a.tokens);
   if (a.tokens <= kDenseTokens) return launch_band<0, kDenseTokens>(p, a.batch, backward, stream);
-  // 128-row tiles re-read half as much halo; 64-row ones spread a call over twice as many CTAs, which pays while the wide ones
-  // would not cover the chip.  Forward + backward at window 64, 64 | 128 rows: 8 structures of 128 tokens (64 wide tiles) 14.7 |
-  // 16.3 us, 128 tiles 17.3 | 16.4, 256 tiles 29.1 | 22.5, 576 tiles 50.4 | 42.2; windows 32 and 128 turn at the same place.
-  const bool wide = (long long)a.batch * a.heads * ((a.tokens + 127) / 128) >= 128;
+  const bool wide = band_attn_wide(a);
   switch (a.window) {
     case 32: return launch_either<32>(p, a.batch, wide, backward, stream);
     case 64: return launch_either<64>(p, a.batch, wide, backward, stream);
@@ -516,9 +538,12 @@ int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward
   }
 }
 
-int band_attn_status(int32_t* host_status, cudaStream_t stream) {
+int band_attn_status(int32_t* host_status, cudaStream_t stream, bool clear) {
   cudaError_t e = cudaMemcpyFromSymbolAsync(host_status, g_band_status, sizeof(int32_t), 0, cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  constexpr int32_t kNone = MF_OK;
+  if (e == cudaSuccess && clear) e = cudaMemcpyToSymbolAsync(g_band_status, &kNone, sizeof(int32_t), 0, cudaMemcpyHostToDevice, stream);
+  if (e == cudaSuccess && clear) e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_error(e, "band attention status read-back");
   return MF_OK;
 }

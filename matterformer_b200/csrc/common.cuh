@@ -45,6 +45,13 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
       }                                                                                                      \
   } while (0)
 
+// Waits of a kernel give up after `limit` clocks.  The self-test lets them run out: the barriers of kind `withheld` (as the kernel
+// numbers them) expect one arrival more than there are.
+struct BoundedWaits {
+  long long limit = 1ll << 31;  // kWaitLimitCycles
+  int withheld = -1;
+};
+
 // ---- launches that begin while the kernel before them ends ------------------------
 // A kernel launched with launch_dependent may begin as soon as every CTA of the kernel before it in the stream has said so
 // (launch_dependents) or has ended; it calls wait_for_previous before it touches memory, which returns when that kernel has ended and

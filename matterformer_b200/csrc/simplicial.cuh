@@ -4,15 +4,9 @@
 #include <cuda_runtime.h>
 
 #include "../../include/matterformer_b200.h"
+#include "common.cuh"
 
 namespace mf {
-
-// Waits of a kernel give up after `limit` clocks.  The self-test lets them run out: the barriers of kind `withheld` (as the kernel
-// numbers them) expect one arrival more than there are.
-struct BoundedWaits {
-  long long limit = 1ll << 31;  // kWaitLimitCycles
-  int withheld = -1;
-};
 
 // fp32 CUDA-core kernels (simplicial_generic.cu)
 int simplicial_generic_fwd(const MfSimplicialFwdArgs& a, cudaStream_t stream);

@@ -399,6 +399,21 @@ extern "C" int mf_sparse_attn_status(int32_t* host_status, void* stream) {
   return rc != MF_OK || *host_status != 0 ? rc : band_attn_status(host_status, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int mf_selftest_band_give_up(const MfSparseAttnArgs* a, int32_t backward, int64_t limit_cycles, int32_t* host_status,
+                                        void* stream) {
+  const char* name = "mf_selftest_band_give_up";
+  MF_CHECK_ARG(a && host_status, "%s: null argument", name);
+  MF_CHECK_ARG(limit_cycles >= 1 && limit_cycles <= (1ll << 31), "%s: limit must be in [1, 2^31] clocks", name);
+  MF_CHECK_ARG(a->q && a->k && a->v && a->num_atoms && a->out && a->lse && (!backward || (a->grad_out && a->dq && a->dk && a->dv)),
+               "%s: null tensor pointer", name);
+  MF_CHECK_ALIGNED(name, a->q, a->k, a->v, a->out, a->grad_out, a->dq, a->dk, a->dv);
+  MF_CHECK_ARG(a->batch > 0 && a->heads > 0 && (long long)a->batch * a->heads <= 65535 && band_attn_applies(*a) && band_attn_wide(*a),
+               "%s: not a call of the 128-row band tiles", name);
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int rc = band_attn(*a, nullptr, backward != 0, s, BoundedWaits{(long long)limit_cycles, 0});
+  return rc != MF_OK ? rc : band_attn_status(host_status, s, true);
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Band attention on the packed projection of an attention layer: q, k, v are read inside the (B,N,3,H,D) output of
 // the layer's input GEMM and out is written as (B,N,H*D), so the head split before and the merge after the core

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "../../include/matterformer_b200.h"
+#include "common.cuh"
 
 namespace mf {
 
@@ -20,8 +21,9 @@ int local_attn_mma_layouts(const MfSparseAttnArgs& a, const RowLayout& in, const
 
 // Bands of 32, 64 or 128 tokens at head_dim 64 (band_attn.cu); `layouts` as above, or null for contiguous rows.
 bool band_attn_applies(const MfSparseAttnArgs& a);
-int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream);
-int band_attn_status(int32_t* host_status, cudaStream_t stream);  // as sparse_attn_sm100_status
+bool band_attn_wide(const MfSparseAttnArgs& a);  // in tiles of 128 rows
+int band_attn(const MfSparseAttnArgs& a, const RowLayout* layouts, bool backward, cudaStream_t stream, BoundedWaits waits = {});
+int band_attn_status(int32_t* host_status, cudaStream_t stream, bool clear = false);  // as sparse_attn_sm100_status
 
 // ---- warp-level tensor-core helpers (m16n8k16, bf16 operands, fp32 accumulate) ---------------------------
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem_addr) {

@@ -220,8 +220,8 @@ def set_sparse_backend(name: str) -> str:
 
 
 def sparse_device_status(device=None) -> int:
-    """Status word of the tcgen05 sparse-attention kernels on the current stream (0, or the code of an expired
-    device-side wait).  Synchronises the stream."""
+    """Status word of the sparse-attention kernels with device-side waits (tcgen05, 128-row band tiles): 0, or the code of an expired
+    wait (the rows of such a band tile are zeros, the outputs of a tcgen05 call undefined).  Synchronises the current stream."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     out = ctypes.c_int32(0)
     with torch.cuda.device(dev):

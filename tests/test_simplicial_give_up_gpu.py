@@ -52,3 +52,33 @@ def test_a_hand_off_that_never_completes(kernel, withheld):
     assert ws[:4].view(torch.int32).item() == _lib.MF_OK
     assert all(torch.isfinite(outputs[n]).all() for n in (("dq", "dk1", "dv1", "dk2", "dv2") if backward else outputs))
     del keep
+
+
+@pytest.mark.parametrize("window", [32, 64, 128])
+@pytest.mark.parametrize("backward", [False, True])
+def test_band_tiles_that_never_arrive(window, backward):
+    B, H, N = 16, 4, 200
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    rows = {n: torch.ones(B, H, N, 64, **bf) for n in ("q", "k", "v", "grad_out")}
+    nan = {n: torch.full((B, H, N, 64), float("nan"), **bf) for n in (("dq", "dk", "dv") if backward else ("out",))}
+    if backward:
+        rows["out"] = torch.ones(B, H, N, 64, **bf)
+    lse = torch.full((B, H, N), 0.0 if backward else float("nan"), device="cuda")
+    n = torch.full((B,), N, dtype=torch.int32, device="cuda")
+    n[1], n[2] = 0, 100
+    ws = torch.empty(1 << 20, dtype=torch.uint8, device="cuda")
+    a = _lib.MfSparseAttnArgs(batch=B, heads=H, tokens=N, head_dim=64, dtype=_lib.MF_DTYPE_BF16, window=window, scale=0.125)
+    for name, x in {**rows, **nan, "lse": lse, "num_atoms": n, "workspace": ws}.items():
+        setattr(a, name, x.data_ptr())
+    a.workspace_bytes = ws.numel()
+    ref, stream, status = ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_int32(0)
+    _lib.check(_lib.lib().mf_selftest_band_give_up(ref, int(backward), 20_000, ctypes.byref(status), stream))
+    assert status.value == _lib.MF_ERR_DEVICE_TIMEOUT
+    for name, t in (*nan.items(), *(() if backward else (("lse", lse),))):
+        assert torch.equal(t, torch.zeros_like(t)), name
+    # the same call with tiles that arrive, on the same buffers
+    _lib.check(getattr(_lib.lib(), "mf_local_attn_bwd" if backward else "mf_local_attn_fwd")(ref, stream))
+    _lib.check(_lib.lib().mf_sparse_attn_status(ctypes.byref(status), stream))
+    assert status.value == _lib.MF_OK
+    assert all(torch.isfinite(t).all() for t in nan.values())
+    assert backward or (nan["out"][0].float() - 1).abs().max() < 2**-7  # a mean of ones with weights rounded to bf16
