@@ -13,6 +13,7 @@ import ctypes
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -479,9 +480,18 @@ def noise_channel(sigma: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def watched(*tensors: torch.Tensor) -> bool:
+    """Something follows the torch operations on these tensors (a transform of ``torch.func``, forward-mode differentiation, tracing,
+    compilation) and would not see a kernel launched past it: plain operations have to do."""
+    if (torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0
+            or torch._C._functorch.peek_interpreter_stack() is not None):  # fmt: skip
+        return True
+    return forward_ad._current_level >= 0 and any(forward_ad.unpack_dual(t).tangent is not None for t in tensors)
+
+
 def per_molecule_applies(t: torch.Tensor) -> bool:
-    """What the one-launch forms of the conditioning take: a contiguous CUDA fp32 vector without gradient."""
-    return t.is_cuda and t.ndim == 1 and t.dtype == torch.float32 and t.is_contiguous() and not t.requires_grad
+    """What the one-launch forms of the conditioning take: a contiguous CUDA fp32 vector without gradient that nothing watches."""
+    return t.is_cuda and t.ndim == 1 and t.dtype == torch.float32 and t.is_contiguous() and not t.requires_grad and not watched(t)
 
 
 def time_embedding(t: torch.Tensor, half: int, dtype: torch.dtype) -> torch.Tensor:
@@ -502,7 +512,8 @@ def valid_and_counts(pad_mask: torch.Tensor):
 
 def token_projection_applies(x: torch.Tensor, noise: torch.Tensor, pad_mask: torch.Tensor, weight: torch.Tensor,
                              bias: Optional[torch.Tensor]) -> bool:  # fmt: skip
-    return (x.is_cuda and x.ndim == 3 and x.dtype == torch.float32 and not x.requires_grad and x.shape[2] < 8 and per_molecule_applies(noise)
+    return (x.is_cuda and x.ndim == 3 and x.dtype == torch.float32 and not x.requires_grad and x.shape[2] < 8 and not watched(x)
+            and per_molecule_applies(noise)
             and noise.shape[0] == x.shape[0] and pad_mask.dtype == torch.bool and pad_mask.shape == x.shape[:2] and bias is not None
             and weight.dtype == bias.dtype == torch.float32 and weight.shape[1] == x.shape[2] + 1 and weight.shape[0] % 64 == 0
             and 64 <= weight.shape[0] <= 1024 and all(t.device == x.device for t in (noise, pad_mask, weight, bias)))  # fmt: skip
