@@ -603,17 +603,18 @@ class _LayerNorm(torch.autograd.Function):
         _lib.launch(_lib.lib().mf_layer_norm_fwd, x.device, x.data_ptr(), _CODE[x.dtype], w.data_ptr(), b.data_ptr(), B * N, C, float(eps),
                     _CODE[out_dtype], h.data_ptr(), mean.data_ptr(), rstd.data_ptr())  # fmt: skip
         ctx.dtypes = (weight.dtype, bias.dtype)
-        ctx.save_for_backward(x, w, mean, rstd)
+        # (values of its own: the weight may change before the backward pass)
+        ctx.save_for_backward(x, w - 1.0 if any(ctx.needs_input_grad) else None, mean, rstd)
         return h
 
     @staticmethod
     def backward(ctx, dh):
-        x, w, mean, rstd = ctx.saved_tensors
+        x, w1, mean, rstd = ctx.saved_tensors
         B, N, C = x.shape
         dh = (dh if dh.dtype in _CODE else dh.float()).contiguous()
         dx = torch.empty_like(x)
         sums = torch.empty((2, B, C), device=x.device, dtype=torch.float32)
-        scale = (w - 1.0).expand(B, C).contiguous()
+        scale = w1.expand(B, C).contiguous()
         _lib.launch(_lib.lib().mf_ln_modulate_bwd, x.device, dh.data_ptr(), _CODE[dh.dtype], x.data_ptr(), _CODE[x.dtype], scale.data_ptr(),
                     mean.data_ptr(), rstd.data_ptr(), B, N, C, dx.data_ptr(), sums[0].data_ptr(), sums[1].data_ptr())  # fmt: skip
         db, dw = sums.sum(1)

@@ -7,6 +7,7 @@ import torch.nn.functional as F
 
 from matterformer_b200 import fused
 from matterformer_b200.linear import _StackedModulation, pair_linear_bf16
+from matterformer_b200.trunk import layer_norm
 
 pytestmark = pytest.mark.gpu
 EPS16 = 2.0**-7  # spacing of bf16 at 1 (seven fraction bits); a rounded value is within half of it, relatively
@@ -126,3 +127,16 @@ def test_pair_linear():
         assert (y.double() - r).abs().max() <= EPS16 * r.abs().max()
     for y, r in zip(torch.autograd.grad(got, (x, w, b), (da, db)), torch.autograd.grad(want, (x, w, b), (da.double(), db.double()))):
         assert (y.double() - r.double()).abs().max() <= EPS16 * r.abs().max()
+
+
+def test_a_norm_whose_weight_changes_before_the_backward_pass():
+    """The gradient is that of the weight that the forward pass used."""
+    g = torch.Generator("cuda").manual_seed(2)
+    x, norm, dh = _rand(g, 3, 7, 64).requires_grad_(True), torch.nn.LayerNorm(64).cuda(), _rand(g, 3, 7, 64)
+    torch.nn.init.normal_(norm.weight)
+    wants = torch.autograd.grad(layer_norm(x, norm), (x, norm.weight, norm.bias), dh)
+    h = layer_norm(x, norm)
+    with torch.no_grad():
+        norm.weight.mul_(1.5)
+    for got, want in zip(torch.autograd.grad(h, (x, norm.weight, norm.bias), dh), wants):
+        assert torch.equal(got, want)
