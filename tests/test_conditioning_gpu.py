@@ -7,7 +7,7 @@ import torch.nn.functional as F
 
 from matterformer_b200 import fused
 from matterformer_b200.linear import _StackedModulation, pair_linear_bf16
-from matterformer_b200.trunk import layer_norm
+from matterformer_b200.trunk import AdaLNBlock, TransformerTrunk, layer_norm
 
 pytestmark = pytest.mark.gpu
 EPS16 = 2.0**-7  # spacing of bf16 at 1 (seven fraction bits); a rounded value is within half of it, relatively
@@ -140,3 +140,31 @@ def test_a_norm_whose_weight_changes_before_the_backward_pass():
         norm.weight.mul_(1.5)
     for got, want in zip(torch.autograd.grad(h, (x, norm.weight, norm.bias), dh), wants):
         assert torch.equal(got, want)
+
+
+def _trunk_case():
+    torch.manual_seed(1)
+    trunk = TransformerTrunk(64, 1, ["mha", "mha"]).cuda()
+    for block in trunk.blocks:
+        torch.nn.init.normal_(block.ada_ln[-1].weight, std=0.1)
+        torch.nn.init.normal_(block.ada_ln[-1].bias, std=0.5)
+    x, cond = torch.randn(2, 24, 64, device="cuda"), torch.randn(2, 64, device="cuda")
+    return trunk, x, cond, torch.arange(24, device="cuda")[None] >= torch.tensor([[24], [10]], device="cuda")
+
+
+class _Weighted(AdaLNBlock):
+    def forward(self, *args, **kwargs):
+        return super().forward(*args, **kwargs) * torch.linspace(0.5, 2.0, 64, device="cuda")
+
+
+def test_a_last_block_of_another_class():
+    """What a derived last block makes of its output comes before the output norm: as in a trunk whose norm is applied by hand."""
+    trunk, x, cond, pad = _trunk_case()
+    trunk.blocks[1].__class__ = _Weighted
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+        got, norm = trunk(x, cond, pad_mask=pad), trunk.norm_out
+        trunk.norm_out = torch.nn.Identity()
+        trunk.norm_out.normalized_shape = ()
+        before = trunk(x, cond, pad_mask=pad)
+    want = norm(before).masked_fill(pad[..., None], 0.0)
+    assert (got - want).abs().max() <= 1e-5 * want.abs().max()
