@@ -465,10 +465,10 @@ class TransformerTrunk(nn.Module):
         suffix = _padding_is_suffix(self, pad_mask) if reads else None  # one read-back for all layers
         h, norm = None, self.norm_out
         last = len(self.blocks) - 1
-        # the output norm in one pass with the last block's output (its padded rows are zeros, which the norm leaves as they are)
+        # the output norm in one pass with the last block's output (its padded rows are zeros, which a norm with an eps leaves as they are)
         # and nothing but the block itself stands between the two
         closing = stacked and last >= 0 and type(self.blocks[last]) is AdaLNBlock and type(norm) is nn.LayerNorm and not norm.elementwise_affine and norm.normalized_shape == (x.shape[-1],) and \
-            _unhooked(norm, *self.blocks[last:])  # fmt: skip
+            norm.eps > 0 and _unhooked(norm, *self.blocks[last:])  # fmt: skip
         for i, (block, six) in enumerate(zip(self.blocks, modulation)):
             chain = stacked and i < last  # the next block's first norm in one pass with this one's output
             following = (*modulation[i + 1][:2], self.blocks[i + 1].norm1.eps) if chain else (None, None, norm.eps) if closing else None

@@ -168,3 +168,15 @@ def test_a_last_block_of_another_class():
         before = trunk(x, cond, pad_mask=pad)
     want = norm(before).masked_fill(pad[..., None], 0.0)
     assert (got - want).abs().max() <= 1e-5 * want.abs().max()
+
+
+def test_an_output_norm_without_eps():
+    """Padded rows come out as zeros, and no NaN of theirs reaches a gradient."""
+    trunk, x, cond, pad = _trunk_case()
+    trunk.norm_out.eps = 0.0
+    x.requires_grad_(True)
+    with torch.autocast("cuda", torch.bfloat16):
+        out = trunk(x, cond, pad_mask=pad)
+    assert (out[pad] == 0).all() and torch.isfinite(out).all()
+    grads = torch.autograd.grad(out.square().sum() + out.sum(), [x, *(b.mlp.fc1.weight for b in trunk.blocks)])
+    assert all(torch.isfinite(t[~pad] if t is grads[0] else t).all() for t in grads)
