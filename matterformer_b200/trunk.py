@@ -557,7 +557,7 @@ class EDMModel(nn.Module):
         kernel_fits = trunk_out.is_cuda and trunk_out.dtype in (torch.float32, torch.bfloat16)
         if kernel_fits and tuple(w0[:, 2 * d :].shape) == (fused.PAIR_HIDDEN, fused.PAIR_RBF) and not coords.requires_grad:
             # per-atom halves of the first Linear (two GEMMs), everything per pair in one kernel
-            if _bf16_autocast(trunk_out) and w0.dtype == torch.float32 and w0.shape[1] % 8 == 0 and d % 8 == 0:
+            if _bf16_autocast(trunk_out) and b0 is not None and w0.dtype == b0.dtype == torch.float32 and w0.shape[1] % 8 == 0 and d % 8 == 0:
                 a, b = pair_linear_bf16(trunk_out, w0, b0)
             else:
                 a = F.linear(trunk_out, w0[:, :d])
@@ -598,7 +598,8 @@ class EDMModel(nn.Module):
         if not linear_bf16_applies(atom_noisy, self.atom_proj.weight):
             return self._forward(atom_noisy, coords_noisy, pad_mask, sigma_cond)
         layers = [self.atom_proj, self.conditioning.mlp[0], self.conditioning.mlp[2], self.atom_head[1], self.atom_head[3]]
-        layers.append(self.pair_head[0])
+        if self.pair_head[0].bias is not None:
+            layers.append(self.pair_head[0])
         with bf16_copies(p for m in layers for p in (m.weight, m.bias)):  # (the trunk makes its own)
             return self._forward(atom_noisy, coords_noisy, pad_mask, sigma_cond)
 

@@ -6,6 +6,7 @@ import torch
 import torch.nn.functional as F
 
 from matterformer_b200 import fused
+from matterformer_b200.dp import build_edm_net
 from matterformer_b200.linear import _StackedModulation, pair_linear_bf16
 from matterformer_b200.trunk import AdaLNBlock, TransformerTrunk, layer_norm
 
@@ -180,3 +181,23 @@ def test_an_output_norm_without_eps():
     assert (out[pad] == 0).all() and torch.isfinite(out).all()
     grads = torch.autograd.grad(out.square().sum() + out.sum(), [x, *(b.mlp.fc1.weight for b in trunk.blocks)])
     assert all(torch.isfinite(t[~pad] if t is grads[0] else t).all() for t in grads)
+
+
+def test_a_pair_head_without_a_bias():
+    """A first Linear without a bias is one whose bias is zero.  The halves are rounded to bf16 once either way, their products summed in
+    fp32: two spacings of bf16."""
+    net = build_edm_net(seed=0).cuda()
+    head = net.model.pair_head
+    torch.nn.init.normal_(head[2].weight)
+    torch.nn.init.zeros_(head[0].bias)
+    g = torch.Generator("cuda").manual_seed(3)
+    atoms, coords, pad = _rand(g, 2, 9, 6), _rand(g, 2, 9, 3), torch.zeros(2, 9, dtype=torch.bool, device="cuda")
+
+    def call():
+        with torch.no_grad(), torch.autocast("cuda", torch.bfloat16):
+            return net(atoms, coords, pad, torch.ones(2, device="cuda"))
+
+    want = call()
+    head[0].bias = None
+    for got, ref in zip(call(), want):
+        assert (got - ref).abs().max() <= 2 * EPS16 * ref.abs().max()
