@@ -631,7 +631,7 @@ class EDMPreconditioner(nn.Module):
             sigma = sigma[:, 0]
         sigma = sigma.float()
         sd2 = self.sigma_data**2
-        if fused.per_molecule_applies(sigma):
+        if type(self.sigma_data) is float and fused.per_molecule_applies(sigma):  # (a tensor put there may have a gradient)
             c_skip, c_out, c_in = fused.edm_scalings(sigma, self.sigma_data)
         else:
             c_skip = sd2 / (sigma.square() + sd2)

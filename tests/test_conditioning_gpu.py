@@ -201,3 +201,20 @@ def test_a_pair_head_without_a_bias():
     head[0].bias = None
     for got, ref in zip(call(), want):
         assert (got - ref).abs().max() <= 2 * EPS16 * ref.abs().max()
+
+
+def test_a_data_scale_that_is_learned():
+    """A tensor in the place of the number, as a program may put one there, keeps its gradient: that of the scalings written out."""
+    from matterformer_b200.trunk import EDMPreconditioner
+
+    g = torch.Generator("cuda").manual_seed(4)
+    pre = EDMPreconditioner(lambda a, c, pad, sigma, lattice=None: (a * 0.5, c * 0.5))
+    atoms, coords, pad = _rand(g, 3, 4, 6).double(), _rand(g, 3, 4, 3).double(), torch.zeros(3, 4, dtype=torch.bool, device="cuda")
+    sigma, scale = torch.tensor([0.5, 1.0, 2.0], device="cuda"), torch.tensor(1.5, device="cuda", requires_grad=True)
+    pre.sigma_data = scale
+    got = torch.autograd.grad(pre(atoms, coords, pad, sigma)[0].sum(), scale)[0]
+    s = sigma.double()[:, None, None]
+    d = scale.detach().double().requires_grad_(True)
+    written = d**2 / (s**2 + d**2) * atoms + s * d / (s**2 + d**2) * 0.5 * atoms
+    want = torch.autograd.grad(written.sum(), d)[0]
+    assert abs(got.item() - want.item()) <= 1e-5 * abs(want.item())
