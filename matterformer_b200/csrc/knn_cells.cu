@@ -17,8 +17,6 @@
 //
 // Structures with a coordinate outside [0,1) (where the reference's 27 offsets of the unwrapped
 // coordinates are not the nearest images) are searched exhaustively.
-#include <type_traits>
-
 #include "common.cuh"
 #include "geometry.cuh"
 
@@ -238,7 +236,9 @@ __global__ void __launch_bounds__(1024) knn_setup_kernel(const float* __restrict
 // one list of all their atoms.  The result does not depend on the order of candidates, so it is the same, bit for bit, as the
 // one-thread-per-query search.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kWarpCand = 384;  // candidates per warp in shared memory (a 27-bin neighbourhood holds about 216)
+// Candidates per warp in shared memory.  A 27-bin neighbourhood holds 27 bins of at least 1.25^3 3 k / 4 pi atoms, 201 at k = 16; from k of
+// about 31 on (403 at 32) it does not fit, and every query of such a search scans global memory.
+constexpr int kWarpCand = 384;
 constexpr int kPairSurv = 128;  // survivors per query of the paired search
 
 // Shared memory of one warp.  The paired search reads its candidates two at a time per coordinate and keeps the image offset

@@ -56,10 +56,10 @@ struct ResFwdShared {
 };
 
 // The queries of a warp.
-template <int MT, int NT, int RK>
+template <int RK>
 __device__ __forceinline__ void res_fwd_queries(const ResFwdParams& p, ResFwdShared<RK>& sm, int bh, int n, uint32_t kmask,
                                                 uint32_t qmask) {
-  constexpr int KS = (NT + 1) / 2;  // 16-key steps of the products over the second keys
+  constexpr int MT = 2, NT = 4, KS = NT / 2;  // 16-row and 8-column tiles of the logits, 16-key steps over the second keys
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3, row8 = lane >> 2, N = p.N;
   const uint32_t qt = (uint32_t)__cvta_generic_to_shared(sm.tile[0]);
   const FragBase fb(qt, lane);
@@ -145,17 +145,13 @@ __device__ __forceinline__ void res_fwd_queries(const ResFwdParams& p, ResFwdSha
       m = warp_max(m);
       have = m > -INFINITY;
       const float m2 = have ? m * kLog2e : 0.f;
-      uint32_t pk[MT][2 * KS][2];
+      uint32_t pk[MT][NT][2];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 2 * KS; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            if (nt >= NT) {
-              pk[mt][nt][hh] = 0u;
-              continue;
-            }
             const float a = fast_exp2(fmaf(s[mt][nt][2 * hh], kLog2e, -m2)), c = fast_exp2(fmaf(s[mt][nt][2 * hh + 1], kLog2e, -m2));
             l += a + c;
             pk[mt][nt][hh] = pack2_bf16(a, c);
@@ -195,7 +191,7 @@ __device__ __forceinline__ void res_fwd_queries(const ResFwdParams& p, ResFwdSha
 #pragma unroll
         for (int rk = 0; rk < RK; ++rk) {
           float t[2 * MT][4], lo = 0.f, hi = 0.f;
-          rank_sums<MT, 2 * KS, RK>(t, mright, pk, rk, lane);
+          rank_sums<MT, NT, RK>(t, mright, pk, rk, lane);
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
             uint32_t mh[4], mo[4];
@@ -296,7 +292,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 2) simplicial_small_res_fwd_ke
   }
   cp_async_wait<0>();
   __syncthreads();
-  res_fwd_queries<2, 4, RK>(p, sm, bh, n, kmask, qmask);
+  res_fwd_queries<RK>(p, sm, bh, n, kmask, qmask);
 }
 
 }  // namespace
