@@ -91,7 +91,7 @@ constexpr int tri_smem_bytes(int tokens) {
 // (rows of more than 64 x), 100 to 128 steps long, or of two, up to 96.  There the split with the fewest steps is taken of those, of up to
 // six tiles, whose cost is within kSlack hundredths of the lowest.  Backward, 8 heads, us, slack 0 | 7 | 10: 1 molecule of 101 atoms 278 |
 // 96 | 78, of 128 345 | 190 | 117, of 181 417 | 229 | 231; 4 of 43-128 343 | 190 | 164, of 60-181 454 | 375 | 375; 64 of 128 3 305 | 3 307 |
-// 3 515, of 181 10 357 | 11 009 | 11 015; 64 of 20-181 atoms of 192 tokens, forward + backward, 4 436 | 4 519 | 4 532.
+// 3 515, of 181 10 357 | 11 009 | 11 015; 64 of 20-181 atoms of 192 tokens, forward + backward, 4 436 | 4 511 | 4 525.
 // The split depends on the molecule alone, so that its results do not depend on the batch it is in: more tiles for small batches only
 // would cost the large ones nothing.
 constexpr int kTileCost = 4, kMostTiles = 6, kShortWalk = 100, kSlack = 7;
@@ -102,21 +102,23 @@ __device__ inline TriPlan tri_plan(int nx, int ny) {
   TriPlan best{0, 0};
   if (nx <= 0 || ny <= 0) return best;
   const int most = nx > kShortWalk ? kMostTiles : kMostTiles - 1, slack = nx > kShortWalk ? kSlack : 0;
-  int limit = INT_MAX, best_cost = 0, best_steps = 0;
-#pragma unroll 1
-  for (int choice = 0; choice < 2; ++choice) {  // the lowest cost, then the fewest steps within its slack
-#pragma unroll 1
-    for (int t = 1; t <= most; ++t) {
-      const int rows = (nx + t - 1) / t;
-      if (rows > kTileM) continue;
-      const int tiles = (nx + rows - 1) / rows, groups = min(kTileM / rows, kMaxGroups), steps = (ny + groups - 1) / groups;
-      const int cost = tiles * (steps + kTileCost);
-      const bool better = best.tiles == 0 || (choice == 0 ? cost < best_cost : steps < best_steps && 100 * cost <= limit);
-      if (better) best = TriPlan{tiles, rows}, best_cost = cost, best_steps = steps;
-    }
-    if (slack == 0) break;
-    limit = (100 + slack) * best_cost;
+  int cost[kMostTiles], steps[kMostTiles], lowest = INT_MAX;
+#pragma unroll
+  for (int t = 0; t < kMostTiles; ++t) {  // t + 1 tiles or fewer
+    const int rows = (nx + t) / (t + 1), groups = min(kTileM / rows, kMaxGroups);
+    cost[t] = INT_MAX, steps[t] = 0;
+    if (rows > kTileM || t >= most) continue;
+    steps[t] = (ny + groups - 1) / groups;
+    cost[t] = (nx + rows - 1) / rows * (steps[t] + kTileCost);
+    lowest = min(lowest, cost[t]);
   }
+  const int limit = (100 + slack) * lowest / 100;
+  int fewest = INT_MAX, chosen = 0;
+#pragma unroll
+  for (int t = 0; t < kMostTiles; ++t)
+    if (cost[t] <= limit && (slack > 0 ? steps[t] < fewest : fewest == INT_MAX)) fewest = steps[t], chosen = t + 1;
+  best.rows = (nx + chosen - 1) / chosen;
+  best.tiles = (nx + best.rows - 1) / best.rows;
   return best;
 }
 
