@@ -210,7 +210,8 @@ int mf_simplicial_bwd_needs_zeros(const MfSimplicialBwdArgs* args);
 /* How the row-packed tensor-core kernels lay a molecule with `n_queries` queries (1 + index of the last valid
  * one) and `valid_keys` valid keys onto 128-row tiles: plan[0] = query ranges, plan[1] = queries per range,
  * plan[2] = first keys handled per step, plan[3] = steps per range (all 0 when either count is 0).  Host-only
- * arithmetic, the same function the kernels evaluate; exported so that callers can size and balance batches by
+ * arithmetic, the same function the kernels evaluate (the backward kernel for each piece of the keys that it walks: all
+ * of them at once in batches that fill the chip); exported so that callers can size and balance batches by
  * attention cost (ranges * steps tile-steps per molecule and head).  (No counterpart in the reference.) */
 int mf_simplicial_row_plan(int32_t n_queries, int32_t valid_keys, int32_t plan[4]);
 

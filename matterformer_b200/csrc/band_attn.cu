@@ -17,8 +17,8 @@
 // with the other CTAs of the SM.  The 128-row tiles arrive by bulk tensor copies: as 16-byte copies of the threads they took a
 // quarter of the forward kernel's instructions and a share of the L1 path; 64-row tiles, which serve calls of a few microseconds,
 // keep those (a map is encoded on the host for each call).  Interior chunks take no masks and two elements an instruction.  32 cells of
-// 4096 tokens x 8 heads, window 64: forward 144 -> 117 us, backward 381 -> 335 us (HBM floors 82 and 164 us); window 32 125 -> 102 and
-// 342 -> 255, window 128 207 -> 167 and 779 -> 698.  The 32-row walk with its three passes: 219 and 311 + 322 us at window 64.
+// 4096 tokens x 8 heads, window 64: forward 144 -> 117 us, backward 381 -> 317 us (HBM floors 82 and 164 us); window 32 125 -> 102 and
+// 342 -> 248, window 128 207 -> 167 and 779 -> 681.  The 32-row walk with its three passes: 219 and 311 + 322 us at window 64.
 #include "common.cuh"
 #include "simplicial_warp.cuh"
 #include "sm100_primitives.cuh"
